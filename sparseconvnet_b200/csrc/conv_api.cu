@@ -1,6 +1,7 @@
 // C-ABI entry points of the three convolution operators: rulebook lookup (built on first use
 // and cached, like the reference's Metadata), shape checks, kernel choice.
 #include <stdlib.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -52,6 +53,30 @@ int conv_forward_rows_thin(const float *in, long long n_in, float *out, long lon
 int conv_forward_rows_scatter(const float *in, long long n_in, float *out, long long n_out, const float *weight,
                               const float *bias, const float *bn_scale, const float *bn_shift, float leak,
                               const int *child_of, int K, int cin, int cout, int *flags, cudaStream_t stream);
+
+bool conv_tile_supported(const float *in, const float *in_b, int planes_a, const float *out, const float *bias, int K,
+                         int cin, int cout, int groups);
+int conv_forward_tile(const float *in, long long n_in, float *out, long long n_out, const float *weight,
+                      const float *bias, const float *bn_scale, const float *bn_shift, float leak, const int *table,
+                      const RowOrder &ord, int K, int cin, int cout, int precision, int *flags, cudaStream_t stream,
+                      const float *pre_scale, const float *pre_shift, float pre_leak, const float *in_b, int planes_a);
+
+// Is an environment variable of the library set at all?  (One pass over the environment instead of one per knob.)
+static bool any_knob() {
+  for (char **e = ::environ; e && *e; ++e)
+    if ((*e)[0] == 'S' && (*e)[1] == 'C' && (*e)[2] == 'N' && (*e)[3] == '_') return true;
+  return false;
+}
+// SCN_CONV_TILE=0 turns the tile kernel off, and so does every knob that selects or tunes one of the other kernels.
+static bool tile_enabled(bool narrow) {
+  if (!any_knob()) return true;
+  if (getenv("SCN_CONV_TILE")) return atoi(getenv("SCN_CONV_TILE")) != 0;
+  for (const char *k : {"SCN_TC_PERSISTENT", "SCN_TC_SPLIT", "SCN_TC_COPY", "SCN_TC_KC", "SCN_TC_STAGES", "SCN_X3_MIN_COUT",
+                        "SCN_WIDE_MIN_ROWS", "SCN_CONV_WIDE"})
+    if (getenv(k)) return false;
+  if (getenv("SCN_X3_FORM") && getenv("SCN_X3_FORM")[0] == 't') return false;
+  return !(narrow && getenv("SCN_X3_ROWS"));
+}
 
 int split_mode_of_env(int dflt) {
   const char *e = getenv("SCN_X3_FORM");
@@ -299,6 +324,10 @@ int conv_forward_dispatch(const float *in, long long rows_in, float *out, long l
 // `disjoint` additionally promises that every output row HAS a rule: the caller clears it when the
 // fine grid may hold rows that are in no map (earlier duplicates under input mode 0), whose output
 // the scatter form would leave unwritten while the gather form and the reference give them the bias.
+static long long tile_min_rows() {
+  const char *e = any_knob() ? getenv("SCN_TILE_MIN_ROWS") : nullptr;
+  return e ? atoll(e) : 1;
+}
 static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float *in, float *out,
                     const float *weight, const float *bias, int n_in_planes, int n_out_planes, int groups,
                     int precision, cudaStream_t stream, double *macs, bool disjoint = false,
@@ -317,15 +346,6 @@ static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float
   long long rows_in = transposed ? rb.n_out : rb.n_in;
   long long rows_out = transposed ? rb.n_in : rb.n_out;
   const int *table = rb.nbr;
-  // the transposed layer with one rule per output row runs from its input side, on the table as built
-  const bool scatter = transposed && disjoint && precision == SCN_PRECISION_TF32X3 && rows_in > 0 &&
-                       !(getenv("SCN_X3_ROWS") && atoi(getenv("SCN_X3_ROWS")) == 0) &&
-                       !(getenv("SCN_ROWS_SCATTER") && atoi(getenv("SCN_ROWS_SCATTER")) == 0) &&
-                       conv_rows_supported(in, out, weight, bias, rb.n_offsets, cin, cout, groups);
-  if (transposed && !scatter) {
-    SCN_TRY(rulebook_transposed(rb, stream));
-    table = rb.tnbr;
-  }
   if (rows_out > 0) {
     SCN_REQUIRE(out && (in || rows_in == 0), SCN_ERR_BAD_ARG, "null features");
     if (!md->flags_dev) {
@@ -333,7 +353,25 @@ static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float
       SCN_CUDA_CHECK(cudaMemsetAsync(md->flags_dev, 0, sizeof(int), stream));
     }
   }
-  if (rows_out > 0 && scatter) {
+  // tensor cores over mask-sorted tiles: every bf16-class shape it takes
+  const bool tile = precision != SCN_PRECISION_FP32 && rows_out >= tile_min_rows() && tile_enabled(cout <= 64) &&
+                    conv_tile_supported(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups);
+  // the transposed layer with one rule per output row runs from its input side, on the table as built
+  const bool scatter = !tile && transposed && disjoint && precision == SCN_PRECISION_TF32X3 && rows_in > 0 &&
+                       !(getenv("SCN_X3_ROWS") && atoi(getenv("SCN_X3_ROWS")) == 0) &&
+                       !(getenv("SCN_ROWS_SCATTER") && atoi(getenv("SCN_ROWS_SCATTER")) == 0) &&
+                       conv_rows_supported(in, out, weight, bias, rb.n_offsets, cin, cout, groups);
+  if (transposed && !scatter) {
+    SCN_TRY(rulebook_transposed(rb, stream));
+    table = rb.tnbr;
+  }
+  if (tile) {
+    RowOrder &ord = transposed ? rb.torder : rb.order;
+    SCN_TRY(rulebook_row_order(rb, table, rows_out, ord, stream));
+    SCN_TRY(conv_forward_tile(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, table, ord, rb.n_offsets,
+                              cin, cout, precision, md->flags_dev, stream, pre_scale, pre_shift, pre_leak, in_b, planes_a));
+    g_last_kernel = cout <= 64 ? SCN_KERNEL_CONV_ROWS : rows_out <= 148 * 256 ? SCN_KERNEL_CONV_TC : SCN_KERNEL_CONV_WIDE;
+  } else if (rows_out > 0 && scatter) {
     SCN_TRY(conv_forward_rows_scatter(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, rb.nbr,
                                       rb.n_offsets, cin, cout, md->flags_dev, stream));
     g_last_kernel = SCN_KERNEL_CONV_ROWS;

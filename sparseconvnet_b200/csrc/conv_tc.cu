@@ -607,8 +607,8 @@ __global__ void k_sum_partials(const float4 *__restrict__ partial, int n_split, 
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
-// set by scn_test_drop_barrier_arrival, consumed by the next conv_forward_tc of the calling thread
-static thread_local int g_drop_arrival = 0;
+// set by scn_test_drop_barrier_arrival, consumed by the next k_conv_tile or k_conv_tc launch of the calling thread
+thread_local int g_drop_arrival = 0;
 
 static int tc_mode_of(int precision) {
   switch (precision) {

@@ -1,0 +1,780 @@
+// Sparse convolution on tcgen05 tensor cores over mask-sorted row tiles: the kernel of the bf16 modes (the
+// fp32-class three-term form and the single-pass one).
+//
+// Same mathematics as the other convolution kernels (the reference's per-offset gather / GEMM / scatter-add is
+// CPU/Convolution.cpp:137-148, CUDA/Convolution.cu:57-233): output stationary, each output row written once,
+//     D[128 rows x planes] += G_k[128 rows x 32 planes] * W_k[32 planes x planes]
+// with the gathered input rows as the MMA's A operand (M = 128 TMEM lanes = rows of the tile) and the weights as
+// its B operand (N = output planes).
+//
+// What this form is built on:
+//   * Tiles are packed from rows that have the same set of filter offsets (row_order.cu), so a tile of 128 rows
+//     runs 9 to 12 steps of 27 instead of 22 to 25 and nearly every row of a step holds a rule.
+//   * A tcgen05.mma takes max(56, N / 2) cycles for 128 rows (scn_tc_probe_mma).  With up to 64 output planes
+//     the slab [W_h | W_m] is one operand of 2 x planes columns: h (W_h | W_m) is ONE instruction whose two
+//     column ranges are the large and one small term, m W_h goes to the small range, the epilogue adds the two:
+//     2 instructions per 16 planes instead of 3.
+//   * What bounds it is the gather: 128 bytes per row and 32-plane step (16 + 16 bits per value) through 16-byte
+//     cp.async at about 32 bytes per cycle and SM, 512 cycles per step against 224 cycles of tensor work for 32
+//     output planes, 304 for 96.
+//
+// Roles (15 warps, one CTA per SM, persistent).  A step is one filter offset of one tile and SP input planes; the
+// steps of a CTA are numbered through all its tiles and step n uses stage n % n_stages of one ring.
+//   scheduler   publishes a slot per (tile, filter offset with a rule): the input row of every tile row, brought in by
+//               4-byte cp.async so that it never waits for them; up to kSlots offsets ahead
+//   producers   8 warps, warp w takes steps w, w + 8, ...: all 128 rows of the step by 16-byte cp.async pieces
+//               straight into the swizzled operand layout, zero fill where a row has no rule; the barrier arrival
+//               happens when a lane's copies have landed.  (One warp per step: with a step spread over all warps its
+//               chain of waits and address arithmetic, longer than its copies take, was the time of the step: 1 500
+//               cycles against the 512 the copies need.)
+//   weights     one thread: one bulk copy per step
+//   MMA         one thread
+//   epilogue    4 warps: tcgen05.ld -> bias -> optional BatchNorm scale / shift / leaky ReLU -> 16-byte stores,
+//               one thread per row (a row's columns are contiguous)
+//
+// With fewer tiles than SMs the offsets of a tile are divided over n_split items whose partial sums are added in a
+// fixed order (k_tile_sum).
+//
+// Every wait is bounded; on expiry the role raises the abort flag, everybody leaves, tensor memory is freed and
+// the host sees FLAG_TC_TIMEOUT through scn_md_poll_errors.
+#include <stdlib.h>
+
+#include <algorithm>
+#include <atomic>
+
+#include "metadata.cuh"
+#include "tc_ptx.cuh"
+
+namespace scn {
+
+namespace {
+
+constexpr int kRows = kOrderTile;  // rows of a tile = MMA M
+constexpr int kProdWarps = 8;
+constexpr int kEpi0 = kProdWarps, kMma = kProdWarps + 4, kWgt = kMma + 1, kSched = kMma + 2;
+constexpr int kThreads = (kProdWarps + 7) * 32;
+constexpr int kSlots = 16;      // offsets the scheduler runs ahead
+constexpr int kMaxStages = 12;
+
+struct TileParams {
+  const unsigned char *in_split;  // split rows: per slice [SP h | SP m] (three-term) or [SP h]
+  long long row_bytes;
+  long long n_in;
+  float *out;       // n_split == 1: [n_out][cout]; else partial sums [n_split][n_tiles * 128][cout]
+  long long n_out;
+  int cout, coutp;  // coutp: output planes rounded up to 16 (the operand image's)
+  const unsigned char *wprep;
+  const float *bias, *bn_scale, *bn_shift;
+  float leak;
+  const int *nbr;
+  const int *order;
+  const unsigned *tile_bits;
+  int words;
+  int K, n_slices;
+  int n_stages, tmem_cols;
+  long long n_tiles, n_items;
+  int n_split;
+  int drop;         // test hook: leave out one barrier arrival of the first CTA
+  int *flags;
+};
+
+template <int TERMS, int SP>
+struct TileShape {
+  static constexpr int PARTS = TERMS == 3 ? 2 : 1;
+  static constexpr int PP = SP * 2 * PARTS / 16;      // 16-byte pieces per row and step
+  static constexpr int RPI = 32 / PP;                 // rows per copy instruction of a warp
+  static constexpr int NI = kRows / RPI;              // copy instructions per step
+  static constexpr unsigned ROW = PP * 16;            // bytes of a row in a stage: 128 or 64
+  static constexpr unsigned A_BYTES = kRows * ROW;
+  static_assert(PP == 8 || PP == 4, "a row of a step is 128 or 64 bytes");
+  // where the entry of tile row r is kept in a slot: the NI rows of a lane follow one another
+  __device__ static constexpr int entry(int r) { return (r % RPI) * NI + r / RPI; }
+};
+
+// Operand descriptor of a stage of gathered rows: K-major, 128- or 64-byte swizzle (a row's 16-byte chunk c is stored
+// at chunk c ^ (r & 7), or c ^ ((r >> 1) & 3)), 8-row groups back to back.  `offset`: bytes along the row.
+// Whole rows being contiguous is what makes the gather fast: a row arrives as full 128-byte writes.  With the pieces
+// spread over core matrices 2 KB apart every 16 bytes were a write of their own: 1 700 cycles per 16 KB step.
+template <unsigned ROW>
+__device__ __forceinline__ unsigned long long rows_desc(unsigned addr, unsigned offset) {
+  unsigned long long d = 0;
+  d |= (unsigned long long)(((addr + offset) >> 4) & 0x3FFF);
+  d |= 1ull << 16;
+  d |= (unsigned long long)((ROW * 8) >> 4) << 32;
+  d |= 1ull << 46;
+  d |= (unsigned long long)(ROW == 128 ? 2 : 4) << 61;
+  return d;
+}
+
+// control block behind the ring
+struct Ctl {
+  unsigned long long full[kMaxStages], empty[kMaxStages];  // rows and weights landed; MMAs done
+  unsigned long long s_full[kSlots], s_empty[kSlots], acc_full[4], acc_empty[4];
+  int slot_k[kSlots];  // filter offset of the slot; -1: no more work
+  unsigned tmem;
+  int abort;
+};
+
+// what a tile row past the end of the matrix reads as its rulebook entry
+__device__ const int d_no_rule = -1;
+
+__host__ __device__ inline unsigned tile_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(kRows >> 4) << 24);
+}
+
+__device__ __forceinline__ void cp_async4(unsigned dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(unsigned long long *bar) {  // when this thread's copies have landed
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  unsigned r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+// mbar_wait for a whole warp whose control flow has to stay uniform
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long *bar, unsigned parity) {
+  const unsigned addr = smem_u32(bar);
+  for (unsigned it = 0; it < kWaitLimit; ++it) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (__all_sync(0xffffffffu, done != 0)) return true;
+  }
+  return false;
+}
+// D[128 x N] (+)= A * B; descriptors as (low, high) words
+__device__ __forceinline__ void mma_bf16(unsigned d, unsigned a_lo, unsigned a_hi, unsigned b_lo, unsigned b_hi,
+                                         unsigned idesc, unsigned accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+      "setp.ne.b32 p, %6, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void mma_bf16_acc(unsigned d, unsigned a_lo, unsigned a_hi, unsigned b_lo, unsigned b_hi,
+                                             unsigned idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+      "setp.eq.u32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16_nowait(unsigned taddr, unsigned (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+      "[%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// bits `lo` .. `hi` - 1 of the set bits of a 128-bit mask, counted from bit 0 (the offsets of one part of a split)
+__device__ __forceinline__ void keep_range(unsigned (&m)[4], int lo, int hi) {
+  int seen = 0;
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    unsigned keep = 0;
+    for (unsigned u = m[w]; u; u &= u - 1, ++seen)
+      if (seen >= lo && seen < hi) keep |= u & (0u - u);
+    m[w] = keep;
+  }
+}
+
+// filter offsets of an item: those of its tile, or its share of them when the offsets are divided
+__device__ __forceinline__ int item_offsets(const TileParams &P, long long item) {
+  if (item >= P.n_items) return 0;
+  const long long t = item / P.n_split;
+  int total = 0;
+  for (int w = 0; w < P.words; ++w) total += __popc(__ldg(P.tile_bits + t * P.words + w));
+  if (P.n_split == 1) return total;
+  const int part = (int)(item - t * P.n_split);
+  return total * (part + 1) / P.n_split - total * part / P.n_split;
+}
+
+template <int TERMS, int SP>
+__global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
+  using Shape = TileShape<TERMS, SP>;
+  constexpr int PP = Shape::PP, RPI = Shape::RPI, NI = Shape::NI, PARTS = Shape::PARTS;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const unsigned w_part = (unsigned)P.coutp * SP * 2;  // one bf16 weight slab
+  const unsigned w_bytes = w_part * PARTS;
+  const unsigned stage_bytes = Shape::A_BYTES + ((w_bytes + 1023u) & ~1023u);  // the swizzle pattern repeats every 1 KB
+  const unsigned smem0 = smem_u32(smem);
+  unsigned char *tail = smem + (size_t)P.n_stages * stage_bytes;
+  int *entries = reinterpret_cast<int *>(tail);  // [kSlots][128] input row of every tile row, or -1
+  Ctl &C = *reinterpret_cast<Ctl *>(tail + sizeof(int) * kSlots * kRows);
+  const bool joint = TERMS == 3 && P.coutp <= 64;  // [W_h | W_m] as one operand
+  const int dcols = ((joint ? 2 : 1) * P.coutp + 31) & ~31;
+  const int n_acc = min(4, P.tmem_cols / dcols);
+
+  if (tid == 0) {
+    for (int i = 0; i < P.n_stages; ++i) {
+      mbar_init(&C.full[i], 32 + 1);  // the producing warp's lanes and the weights
+      mbar_init(&C.empty[i], 1);
+    }
+    for (int i = 0; i < kSlots; ++i) {
+      mbar_init(&C.s_full[i], 32 + 1);             // the scheduler's copies, and its lane 0 for the words beside them
+      mbar_init(&C.s_empty[i], P.n_slices + 1);    // a producer warp per slice, and the weights
+    }
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(&C.acc_full[i], 1);
+      mbar_init(&C.acc_empty[i], 4);
+    }
+    C.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kMma) tmem_alloc(&C.tmem, (unsigned)P.tmem_cols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const unsigned tmem = C.tmem;
+  volatile int *abort = &C.abort;
+  const long long my_items = (P.n_items - blockIdx.x + gridDim.x - 1) / gridDim.x;  // (the grid has at most n_items CTAs)
+
+  if (warp < kProdWarps) {
+    // ==================================== producers =============================================
+    const int j = lane % PP, q = lane / PP;  // this lane's piece, and the first of its rows q, q + RPI, ...
+    const unsigned chunk = (unsigned)(PP == 8 ? j ^ q : j ^ ((q >> 1) & 3)) * 16 + (unsigned)q * Shape::ROW;
+    // No more warps than stages: a warp at step n has seen the consumption of step n - active - n_stages, and its wait
+    // below can tell step n - n_stages from the one a round earlier only if that one is not later than this.
+    const int active = min(kProdWarps, P.n_stages);
+    const int d_slot = active / P.n_slices, d_slice = active % P.n_slices;
+    const int d_round = active / P.n_stages, d_st = active % P.n_stages;
+    int slot = warp / P.n_slices, slice = warp % P.n_slices;
+    int round = warp / P.n_stages, st = warp % P.n_stages;
+    bool ok = true, bad = false;
+    while (warp < active) {
+      const int si = slot % kSlots;
+      if (!mbar_wait(&C.s_full[si], (slot / kSlots) & 1)) {
+        ok = false;
+        break;
+      }
+      if (C.slot_k[si] < 0 || *abort) break;
+      const int4 *ent = reinterpret_cast<const int4 *>(entries + si * kRows + q * NI);
+      if (!mbar_wait(&C.empty[st], (round + 1) & 1)) {  // (the first round passes)
+        ok = false;
+        break;
+      }
+      const unsigned dst = smem0 + (unsigned)st * stage_bytes + chunk;
+      const unsigned char *col = P.in_split + slice * (SP * 2 * PARTS) + j * 16;
+#pragma unroll
+      for (int i = 0; i < NI; i += 4) {
+        const int4 e4 = ent[i / 4];
+        const int v[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool hit = (unsigned)v[e] < (unsigned)P.n_in;
+          bad |= v[e] >= (int)P.n_in;
+          // (eight pieces: rows four apart alternate between the two halves of the swizzle pattern)
+          cp_async16((PP == 8 && (e & 1) ? dst ^ 64u : dst) + (i + e) * RPI * Shape::ROW,
+                     col + (size_t)(unsigned)(hit ? v[e] : 0) * P.row_bytes, hit ? 16u : 0u);
+        }
+      }
+      cp_async_arrive(&C.full[st]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&C.s_empty[si]);
+      slot += d_slot, slice += d_slice;
+      if (slice >= P.n_slices) slice -= P.n_slices, ++slot;
+      round += d_round, st += d_st;
+      if (st >= P.n_stages) st -= P.n_stages, ++round;
+    }
+    if (bad) atomicOr(P.flags, FLAG_BAD_ROW);
+    asm volatile("cp.async.wait_all;" ::: "memory");  // they must land before the CTA's shared memory goes away
+    if (!ok) *abort = 1;
+  } else if (warp == kWgt) {
+    // ==================================== weights ===============================================
+    if (lane == 0) {
+      int st = 0, par = 1;
+      long long filled = 0;
+      bool ok = true;
+      for (int slot = 0; ok; ++slot) {
+        const int si = slot % kSlots;
+        if (!mbar_wait(&C.s_full[si], (slot / kSlots) & 1)) {
+          ok = false;
+          break;
+        }
+        const int k = C.slot_k[si];
+        mbar_arrive(&C.s_empty[si]);
+        if (k < 0) break;
+        const unsigned char *src = P.wprep + (size_t)k * P.n_slices * w_bytes;
+        for (int s = 0; s < P.n_slices; ++s) {
+          if (!mbar_wait(&C.empty[st], par) || *abort) {
+            ok = false;
+            break;
+          }
+          if (!(P.drop && blockIdx.x == 0 && filled == 0)) {
+            mbar_expect_tx(&C.full[st], w_bytes);
+            bulk_copy_g2s(smem0 + (unsigned)st * stage_bytes + Shape::A_BYTES, src + (size_t)s * w_bytes, w_bytes, &C.full[st]);
+          }
+          ++filled;
+          if (++st == P.n_stages) st = 0, par ^= 1;
+        }
+      }
+      if (!ok) {  // slabs in flight must land before the CTA's shared memory goes away
+        *abort = 1;
+        for (int i = 0; i < P.n_stages; ++i) {
+          const long long uses = (filled + P.n_stages - 1 - i) / P.n_stages;
+          if (uses > 0) mbar_wait(&C.full[i], (unsigned)((uses - 1) & 1));
+        }
+      }
+    }
+  } else if (warp == kMma) {
+    // ==================================== MMA issue =============================================
+    // The whole warp runs the loop and one elected lane issues: with warp-uniform control flow and operands (votes and
+    // reductions instead of loaded flags) the descriptors stay in uniform registers.  Issued from inside a lane == 0
+    // branch every instruction cost 200 to 260 cycles of moves and address arithmetic, four to eight times its own.
+    const unsigned id_all = tile_idesc(joint ? 2 * P.coutp : P.coutp), id_one = tile_idesc(P.coutp);
+    const unsigned long long a_desc = rows_desc<Shape::ROW>(smem0, 0);
+    const unsigned long long w_desc = smem_desc(smem0 + Shape::A_BYTES, 128, SP / 8 * 128);
+    const unsigned a_hi = (unsigned)(a_desc >> 32), w_hi = (unsigned)(w_desc >> 32);
+    const unsigned a0 = (unsigned)a_desc, w0 = (unsigned)w_desc;
+    const unsigned stage_step = stage_bytes >> 4, wm_step = w_part >> 4;
+    const int items = (int)my_items, n_stages = P.n_stages, coutp = P.coutp;
+    int st = 0, par = 0, buf = 0, buf_par = 1;
+    unsigned at = 0, d = tmem;
+    bool ok = true;
+    const bool leader = elect_one();
+    int offsets_next = item_offsets(P, blockIdx.x);
+    for (int i = 0; i < items && ok; ++i) {
+      const int steps = __reduce_max_sync(0xffffffffu, max(1, offsets_next)) * P.n_slices;
+      offsets_next = item_offsets(P, blockIdx.x + (long long)(i + 1) * gridDim.x);
+      // the item's accumulator must have been drained
+      if (!mbar_wait_warp(&C.acc_empty[buf], buf_par) || __any_sync(0xffffffffu, *abort != 0)) {
+        ok = false;
+        break;
+      }
+      for (int s = 0; s < steps; ++s) {
+        if (!mbar_wait_warp(&C.full[st], par)) {
+          ok = false;
+          break;
+        }
+        if (leader) {
+          // order the copied rows (acquired through the barrier) before the tensor core's async-proxy reads; done
+          // here, not by the producers: their fence would wait for the copies they have just started
+          fence_proxy_async_smem();
+          tc_fence_after();
+#pragma unroll
+          for (int jj = 0; jj < SP / 16; ++jj) {
+            const unsigned ah = a0 + at + jj * 2, am = ah + SP / 8, wh = w0 + at + jj * 16;
+            if (jj == 0) mma_bf16(d, ah, a_hi, wh, w_hi, joint ? id_all : id_one, (unsigned)s);
+            else mma_bf16_acc(d, ah, a_hi, wh, w_hi, joint ? id_all : id_one);
+            if (TERMS == 3) {
+              if (joint) {
+                mma_bf16_acc(d + coutp, am, a_hi, wh, w_hi, id_one);
+              } else {
+                mma_bf16_acc(d, ah, a_hi, wh + wm_step, w_hi, id_one);
+                mma_bf16_acc(d, am, a_hi, wh, w_hi, id_one);
+              }
+            }
+          }
+          tc_commit(&C.empty[st]);
+          if (s == steps - 1) tc_commit(&C.acc_full[buf]);
+        }
+        __syncwarp();
+        at += stage_step;
+        if (++st == n_stages) st = 0, par ^= 1, at = 0;
+      }
+      d += dcols;
+      if (++buf == n_acc) buf = 0, buf_par ^= 1, d = tmem;
+    }
+    if (!ok) *abort = 1;
+  } else if (warp == kSched) {
+    // ==================================== scheduler =============================================
+    int slot = 0;
+    bool ok = true;
+    const int words = P.words;
+    const unsigned entries0 = smem_u32(entries) + 4 * Shape::entry(4 * lane);
+    // lane holds rows 4 lane .. 4 lane + 3 of a tile; the next item's are fetched one item ahead
+    int4 o_next;
+    unsigned b_next[4];
+    auto fetch = [&](long long item) {
+      const long long t = item / P.n_split;
+      const bool in = item < P.n_items;
+      o_next = in ? __ldg(reinterpret_cast<const int4 *>(P.order + t * kRows) + lane) : make_int4(-1, -1, -1, -1);
+#pragma unroll
+      for (int w = 0; w < 4; ++w) b_next[w] = in && w < words ? __ldg(P.tile_bits + t * words + w) : 0u;
+    };
+    fetch(blockIdx.x);
+    for (long long it = 0; it < my_items && ok; ++it) {
+      const long long item = blockIdx.x + it * gridDim.x;
+      const int o[4] = {o_next.x, o_next.y, o_next.z, o_next.w};
+      unsigned u[4];
+#pragma unroll
+      for (int w = 0; w < 4; ++w) u[w] = b_next[w];
+      fetch(item + gridDim.x);
+      if (P.n_split > 1) {
+        const int total = __popc(u[0]) + __popc(u[1]) + __popc(u[2]) + __popc(u[3]), part = (int)(item % P.n_split);
+        keep_range(u, total * part / P.n_split, total * (part + 1) / P.n_split);
+      }
+      // a tile (or part) without any rule still gets one step: its rows are all zero fill and so is its sum
+      const bool none = (u[0] | u[1] | u[2] | u[3]) == 0;
+      if (none) u[0] = 1u;
+      const int *p[4];
+      bool row[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        row[e] = o[e] >= 0 && !none;
+        p[e] = row[e] ? P.nbr + o[e] : &d_no_rule;
+      }
+      const bool whole = __all_sync(0xffffffffu, row[0] && row[1] && row[2] && row[3]);
+#pragma unroll 1
+      for (int w = 0; w < words && ok; ++w) {
+        unsigned m = u[0];
+        u[0] = u[1], u[1] = u[2], u[2] = u[3], u[3] = 0;
+        while (m) {
+          const int k = w * 32 + __ffs(m) - 1;
+          m &= m - 1;
+          const int si = slot % kSlots;
+          if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1) || *abort) {
+            ok = false;
+            break;
+          }
+          const unsigned dst = entries0 + si * (kRows * 4);
+          const long long col = (long long)k * P.n_out;
+          if (whole) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) cp_async4(dst + 4 * (Shape::entry(4 * lane + e) - Shape::entry(4 * lane)), p[e] + col);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              cp_async4(dst + 4 * (Shape::entry(4 * lane + e) - Shape::entry(4 * lane)), p[e] + (row[e] ? col : 0));
+          }
+          cp_async_arrive(&C.s_full[si]);
+          if (lane == 0) {
+            C.slot_k[si] = k;
+            mbar_arrive(&C.s_full[si]);
+          }
+          ++slot;
+        }
+      }
+    }
+    // every producer warp finds its next step in a slot that ends it
+    for (int i = 0; i <= (kProdWarps + P.n_slices - 1) / P.n_slices && ok; ++i, ++slot) {
+      const int si = slot % kSlots;
+      if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1)) {
+        ok = false;
+        break;
+      }
+      cp_async_arrive(&C.s_full[si]);
+      if (lane == 0) {
+        C.slot_k[si] = -1;
+        mbar_arrive(&C.s_full[si]);
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (!ok) *abort = 1;
+  } else {
+    // ==================================== epilogue ==============================================
+    const int quad = warp & 3;
+    const int nc = P.cout;
+    int buf = 0, buf_par = 0;
+    for (long long it = 0; it < my_items; ++it) {
+      const long long item = blockIdx.x + it * gridDim.x, t = item / P.n_split;
+      const int part = (int)(item % P.n_split);
+      const int orow = __ldg(P.order + t * kRows + quad * 32 + lane);
+      int got = 1;
+      if (lane == 0) got = (!*abort && mbar_wait(&C.acc_full[buf], buf_par)) ? 1 : 0;
+      got = __shfl_sync(0xffffffffu, got, 0);
+      if (!got) {
+        *abort = 1;
+        break;
+      }
+      tc_fence_after();
+      float *dst = P.n_split > 1 ? P.out + ((long long)part * P.n_tiles * kRows + t * kRows + quad * 32 + lane) * nc
+                                 : P.out + (long long)orow * nc;
+      const unsigned base = tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(buf * dcols);
+      for (int c0 = 0; c0 < nc; c0 += 16) {
+        unsigned a[16], b[16];
+        tmem_ld16_nowait(base + c0, a);
+        if (joint) tmem_ld16_nowait(base + P.coutp + c0, b);
+        tmem_wait_ld();
+        if (orow >= 0) {  // (no early way out of this iteration: the loads above need the whole warp)
+#pragma unroll
+          for (int e = 0; e < 16; e += 4) {
+            if (c0 + e >= nc) break;
+            float4 v;
+            v.x = __uint_as_float(a[e]), v.y = __uint_as_float(a[e + 1]), v.z = __uint_as_float(a[e + 2]), v.w = __uint_as_float(a[e + 3]);
+            if (joint) {
+              v.x += __uint_as_float(b[e]), v.y += __uint_as_float(b[e + 1]);
+              v.z += __uint_as_float(b[e + 2]), v.w += __uint_as_float(b[e + 3]);
+            }
+            if (P.n_split == 1) {
+              if (P.bias) {
+                const float4 b4 = __ldg(reinterpret_cast<const float4 *>(P.bias + c0 + e));
+                v.x += b4.x, v.y += b4.y, v.z += b4.z, v.w += b4.w;
+              }
+              if (P.bn_scale) {  // separate multiply and add, as the stand-alone BatchNorm kernel rounds them
+                const float4 sc = __ldg(reinterpret_cast<const float4 *>(P.bn_scale + c0 + e));
+                const float4 sh = __ldg(reinterpret_cast<const float4 *>(P.bn_shift + c0 + e));
+                v.x = __fadd_rn(__fmul_rn(v.x, sc.x), sh.x), v.y = __fadd_rn(__fmul_rn(v.y, sc.y), sh.y);
+                v.z = __fadd_rn(__fmul_rn(v.z, sc.z), sh.z), v.w = __fadd_rn(__fmul_rn(v.w, sc.w), sh.w);
+                v.x *= v.x > 0.f ? 1.f : P.leak, v.y *= v.y > 0.f ? 1.f : P.leak;
+                v.z *= v.z > 0.f ? 1.f : P.leak, v.w *= v.w > 0.f ? 1.f : P.leak;
+              }
+            }
+            *reinterpret_cast<float4 *>(dst + c0 + e) = v;
+          }
+        }
+        __syncwarp();
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&C.acc_empty[buf]);
+      if (++buf == n_acc) buf = 0, buf_par ^= 1;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (*abort && tid == 0) atomicOr(P.flags, FLAG_TC_TIMEOUT);
+  if (warp == kMma) tmem_dealloc(tmem, (unsigned)P.tmem_cols);
+}
+
+// partial [n_split][n_tiles * 128][cout] -> out: the parts of a row added in order, then bias and BatchNorm
+__global__ void __launch_bounds__(256)
+k_tile_sum(const float4 *__restrict__ partial, int n_split, long long n_pos, int cout4, const int *__restrict__ order,
+           const float *__restrict__ bias, const float *__restrict__ bn_scale, const float *__restrict__ bn_shift,
+           float leak, float4 *__restrict__ out) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_pos * cout4) return;
+  const int c = (int)(i % cout4);
+  const int r = __ldg(order + i / cout4);
+  if (r < 0) return;
+  float4 q = __ldg(partial + i);
+  for (int p = 1; p < n_split; ++p) {
+    const float4 a = __ldg(partial + (long long)p * n_pos * cout4 + i);
+    q.x += a.x, q.y += a.y, q.z += a.z, q.w += a.w;
+  }
+  if (bias) {
+    const float4 b4 = __ldg(reinterpret_cast<const float4 *>(bias) + c);
+    q.x += b4.x, q.y += b4.y, q.z += b4.z, q.w += b4.w;
+  }
+  if (bn_scale) {
+    const float4 sc = __ldg(reinterpret_cast<const float4 *>(bn_scale) + c), sh = __ldg(reinterpret_cast<const float4 *>(bn_shift) + c);
+    q.x = __fadd_rn(__fmul_rn(q.x, sc.x), sh.x), q.y = __fadd_rn(__fmul_rn(q.y, sc.y), sh.y);
+    q.z = __fadd_rn(__fmul_rn(q.z, sc.z), sh.z), q.w = __fadd_rn(__fmul_rn(q.w, sc.w), sh.w);
+    q.x *= q.x > 0.f ? 1.f : leak, q.y *= q.y > 0.f ? 1.f : leak;
+    q.z *= q.z > 0.f ? 1.f : leak, q.w *= q.w > 0.f ? 1.f : leak;
+  }
+  out[(long long)r * cout4 + c] = q;
+}
+
+// in [n][cin] fp32 (or the column-wise concatenation [in (planes_a) | in_b], read where the two lie) -> per row and
+// slice of SP planes [SP h | SP m], h = bf16(x), m = bf16(x - h); PARTS 1: only h.  Planes past cin are zero.  One
+// thread per 8 planes.  pre_scale / pre_shift: x first goes through an eval-mode BatchNorm and its leaky ReLU, with
+// the roundings of the stand-alone operator.  Bound by HBM: 32 bytes in, 16 x PARTS out per thread.
+template <int PARTS>
+__global__ void __launch_bounds__(256)
+k_tile_split(const float *__restrict__ in, unsigned char *__restrict__ out, long long n_pieces, int cin, int ppr, int SP,
+             const float *__restrict__ pre_scale, const float *__restrict__ pre_shift, float pre_leak,
+             const float *__restrict__ in_b, int planes_a) {
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= n_pieces) return;
+  const long long row = idx / ppr;
+  const int piece = (int)(idx - row * ppr), c = piece * 8, slice = c / SP, j = (c % SP) / 8;
+  float x[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) x[e] = 0.f;
+  if (c < cin) {
+    const float *src = !in_b ? in + row * cin + c
+                             : (c < planes_a ? in + row * planes_a + c : in_b + row * (cin - planes_a) + (c - planes_a));
+    const float4 a = __ldg(reinterpret_cast<const float4 *>(src)), b = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+    x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+    if (pre_scale) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float y = __fadd_rn(__fmul_rn(x[e], __ldg(pre_scale + c + e)), __ldg(pre_shift + c + e));
+        x[e] = y * (y > 0.f ? 1.f : pre_leak);
+      }
+    }
+  }
+  uint4 h, m;
+  split_bf16_pair(x[0], x[1], h.x, m.x);
+  split_bf16_pair(x[2], x[3], h.y, m.y);
+  split_bf16_pair(x[4], x[5], h.z, m.z);
+  split_bf16_pair(x[6], x[7], h.w, m.w);
+  unsigned char *q = out + (row * (ppr * 8 / SP) + slice) * (size_t)(SP * 2 * PARTS) + j * 16;
+  *reinterpret_cast<uint4 *>(q) = h;
+  if (PARTS == 2) *reinterpret_cast<uint4 *>(q + SP * 2) = m;
+}
+
+// W [K][cin][cout] -> [K][slice][part][coutp x SP] bf16 in the K-major core-matrix layout of the MMA's B operand
+__global__ void k_tile_weights(const float *__restrict__ w, unsigned char *__restrict__ out, int K, int cin, int cout,
+                               int coutp, int n_slices, int SP, int parts) {
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int cp = n_slices * SP;
+  if (idx >= (long long)K * cp * coutp) return;
+  const int n = (int)(idx % coutp), c = (int)((idx / coutp) % cp), k = (int)(idx / ((long long)coutp * cp));
+  const float v = (c < cin && n < cout) ? w[((long long)k * cin + c) * cout + n] : 0.f;
+  const int slice = c / SP, kk = c % SP;
+  const size_t tile = (size_t)coutp * SP * 2;
+  const size_t off = (size_t)(n / 8) * (SP / 8) * 128 + (size_t)(kk / 8) * 128 + (n % 8) * 16 + (kk % 8) * 2;
+  unsigned char *base = out + ((size_t)k * n_slices + slice) * parts * tile;
+  const __nv_bfloat16 h = __float2bfloat16_rn(v);
+  *reinterpret_cast<__nv_bfloat16 *>(base + off) = h;
+  if (parts == 2) *reinterpret_cast<__nv_bfloat16 *>(base + tile + off) = __float2bfloat16_rn(v - __bfloat162float(h));
+}
+
+constexpr size_t kSmemBudget = 226 * 1024;
+
+// planes per step: as wide as the row allows (fewer steps, longer contiguous reads) without padding it further than
+// to a multiple of 16 (32 with single parts)
+int slice_planes(int terms, int cin) {
+  const int c = (cin + 15) / 16 * 16;
+  if (terms == 1) return c % 64 == 0 ? 64 : 32;
+  return c % 32 == 0 ? 32 : 16;
+}
+
+template <int TERMS, int SP>
+int launch_tile(TileParams &P, int n_sm, int dev, cudaStream_t stream) {
+  using Shape = TileShape<TERMS, SP>;
+  static std::atomic<bool> configured[64];
+  auto kernel = k_conv_tile<TERMS, SP>;
+  if (!configured[dev].load()) {
+    SCN_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    configured[dev].store(true);
+  }
+  const size_t stage = Shape::A_BYTES + ((size_t)P.coutp * SP * 2 * Shape::PARTS + 1023) / 1024 * 1024;
+  const size_t fixed = sizeof(int) * kSlots * kRows + sizeof(Ctl);
+  const int dcols = ((TERMS == 3 && P.coutp <= 64 ? 2 : 1) * P.coutp + 31) & ~31;
+  // Two CTAs per SM, each with half of the shared memory and of the TMEM columns, where that leaves four stages and two
+  // accumulators: one CTA's issue overhead and epilogue run beside the other's tensor instructions.
+  int ctas = dcols * 2 <= 256 && (kSmemBudget / 2 - fixed) / stage >= 4 ? 2 : 1;
+  if (const char *e = getenv("SCN_TILE_CTAS")) ctas = atoi(e) == 2 && dcols <= 256 && (kSmemBudget / 2 - fixed) / stage >= 2 ? 2 : 1;
+  const size_t smem = kSmemBudget / ctas / 1024 * 1024;
+  P.tmem_cols = 512 / ctas;
+  P.n_stages = (int)std::min<size_t>(kMaxStages, (smem - fixed) / stage);
+  SCN_REQUIRE(P.n_stages >= 2, SCN_ERR_UNSUPPORTED, "tile kernel: %d output planes do not fit shared memory", P.cout);
+  P.n_items = P.n_tiles * P.n_split;
+  SCN_LAUNCH(kernel, (unsigned)std::min<long long>(P.n_items, (long long)n_sm * ctas), kThreads, smem, stream, P);
+  SCN_CUDA_CHECK(cudaGetLastError());
+  return SCN_OK;
+}
+
+}  // namespace
+
+extern thread_local int g_drop_arrival;  // test hook (conv_tc.cu)
+
+bool conv_tile_supported(const float *in, const float *in_b, int planes_a, const float *out, const float *bias, int K,
+                         int cin, int cout, int groups) {
+  return groups == 1 && K <= kOrderMaxOffsets && cin % 8 == 0 && cin >= 8 && cout % 8 == 0 && cout >= 8 && cout <= 256 &&
+         (!in_b || planes_a % 8 == 0) && ((uintptr_t)in | (uintptr_t)in_b | (uintptr_t)out | (uintptr_t)bias) % 16 == 0;
+}
+
+// Into how many parts a tile's offsets are divided: the smallest estimate of (waves of items) x (steps of an item),
+// plus, with more than one part, the partial sums' traffic and the second launch.  In SM cycles; a step is bound by its
+// 16 KB of gathered rows at 32 bytes per cycle or by its weight slab, an item also costs the fill and drain of the rings.
+static int split_parts(long long n_tiles, int K, int n_slices, double step_cycles, int cout, int n_sm) {
+  const double offsets = n_tiles >= 2 * n_sm ? 0.5 * K : 0.75 * K;  // sorted tiles of a large level meet fewer
+  double best = 0;
+  int best_s = 1;
+  for (int s = 1; s <= 16 && s <= K; ++s) {
+    const double waves = (double)ceil_div(n_tiles * s, n_sm);
+    double t = waves * (offsets / s * n_slices * step_cycles + 2500.0);
+    if (s > 1) t += 6000.0 + (s + 1.0) * n_tiles * kRows * cout * 4.0 / 3400.0;
+    if (s == 1 || t < 0.95 * best) best = t, best_s = s;
+  }
+  return best_s;
+}
+
+// out [n_out, cout] = act((bias + sum_k in[table[k][.]] @ W[k]) * bn_scale + bn_shift), the input optionally a join and
+// behind a BatchNorm of its own (see k_tile_split).  `ord`: the packing of the table's rows.
+int conv_forward_tile(const float *in, long long n_in, float *out, long long n_out, const float *weight,
+                      const float *bias, const float *bn_scale, const float *bn_shift, float leak, const int *table,
+                      const RowOrder &ord, int K, int cin, int cout, int precision, int *flags, cudaStream_t stream,
+                      const float *pre_scale, const float *pre_shift, float pre_leak, const float *in_b, int planes_a) {
+  if (n_out == 0) return SCN_OK;
+  SCN_REQUIRE(n_in < (1ll << 31) && n_out < (1ll << 31), SCN_ERR_UNSUPPORTED, "row count above 2^31");
+  const int terms = precision == SCN_PRECISION_BF16 ? 1 : 3, parts = terms == 3 ? 2 : 1;
+  const int SP = slice_planes(terms, cin), n_slices = (cin + SP - 1) / SP, cinp = n_slices * SP;
+  const int coutp = (cout + 15) / 16 * 16;
+  int dev = 0;
+  SCN_CUDA_CHECK(cudaGetDevice(&dev));
+  SCN_REQUIRE(dev >= 0 && dev < 64, SCN_ERR_UNSUPPORTED, "device index %d unsupported", dev);
+  static std::atomic<int> sm_count[64];
+  int n_sm = sm_count[dev].load();
+  if (!n_sm) {
+    SCN_CUDA_CHECK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+    sm_count[dev].store(n_sm);
+  }
+
+  WeightImage wi;
+  bool build = true;
+  SCN_TRY(weight_image_get(WIMG_TILE, K, cin, cout, SP * 4 + parts, (size_t)K * cinp * coutp * 2 * parts, stream, &wi, &build));
+  if (build)
+    SCN_LAUNCH(k_tile_weights, (unsigned)ceil_div((long long)K * cinp * coutp, 256), 256, 0, stream, weight,
+               (unsigned char *)wi.ptr, K, cin, cout, coutp, n_slices, SP, parts);
+
+  // the input rows as bf16 parts, made once per call: a row is gathered by up to K output rows
+  unsigned char *split = nullptr;
+  const long long rows_in = std::max<long long>(n_in, 1);
+  SCN_TRY(device_alloc((void **)&split, (size_t)rows_in * cinp * 2 * parts, stream));
+  if (n_in > 0) {
+    const int ppr = cinp / 8;
+    const long long n_pieces = n_in * ppr;
+    if (parts == 2)
+      SCN_LAUNCH(k_tile_split<2>, (unsigned)ceil_div(n_pieces, 256), 256, 0, stream, in, split, n_pieces, cin, ppr, SP, pre_scale, pre_shift, pre_leak, in_b, planes_a);
+    else
+      SCN_LAUNCH(k_tile_split<1>, (unsigned)ceil_div(n_pieces, 256), 256, 0, stream, in, split, n_pieces, cin, ppr, SP, pre_scale, pre_shift, pre_leak, in_b, planes_a);
+  }
+
+  TileParams P{};
+  P.in_split = split;
+  P.row_bytes = (long long)cinp * 2 * parts;
+  P.n_in = n_in;
+  P.out = out;
+  P.n_out = n_out;
+  P.cout = cout;
+  P.coutp = coutp;
+  P.wprep = (const unsigned char *)wi.ptr;
+  P.bias = bias;
+  P.bn_scale = bn_scale;
+  P.bn_shift = bn_shift;
+  P.leak = bn_scale ? leak : 1.f;
+  P.nbr = table;
+  P.order = ord.order;
+  P.tile_bits = ord.tile_bits;
+  P.words = ord.words;
+  P.K = K;
+  P.n_slices = n_slices;
+  P.n_tiles = ord.n_tiles;
+  P.flags = flags;
+  P.drop = g_drop_arrival;
+  g_drop_arrival = 0;
+  const double w_bytes = (double)coutp * SP * 2 * parts, a_bytes = kRows * SP * 2.0 * parts;
+  const char *e = getenv("SCN_TILE_SPLIT");
+  P.n_split = e ? std::max(1, atoi(e)) : split_parts(P.n_tiles, K, n_slices, (a_bytes + w_bytes) / 32.0, cout, n_sm);
+  float *partial = nullptr;
+  int rc = SCN_OK;
+  if (P.n_split > 1) {
+    rc = device_alloc((void **)&partial, (size_t)P.n_split * P.n_tiles * kRows * cout * sizeof(float), stream);
+    P.out = partial;
+  }
+  if (rc == SCN_OK) {
+    if (terms == 3)
+      rc = SP == 32 ? launch_tile<3, 32>(P, n_sm, dev, stream) : launch_tile<3, 16>(P, n_sm, dev, stream);
+    else
+      rc = SP == 64 ? launch_tile<1, 64>(P, n_sm, dev, stream) : launch_tile<1, 32>(P, n_sm, dev, stream);
+  }
+  if (rc == SCN_OK && P.n_split > 1) {
+    const long long n_pos = P.n_tiles * kRows;
+    SCN_LAUNCH(k_tile_sum, (unsigned)ceil_div(n_pos * (cout / 4), 256), 256, 0, stream, (const float4 *)partial, P.n_split, n_pos, cout / 4, ord.order, bias, bn_scale, bn_shift, leak, (float4 *)out);
+    if (cudaGetLastError() != cudaSuccess) {
+      set_error("tile kernel: launch failed");
+      rc = SCN_ERR_CUDA;
+    }
+  }
+  device_free(partial, stream);
+  device_free(split, stream);
+  const int rf = weight_image_put(wi, stream);
+  return rc != SCN_OK ? rc : rf;
+}
+
+}  // namespace scn

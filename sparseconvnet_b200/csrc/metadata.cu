@@ -95,6 +95,8 @@ static void free_rulebook(Rulebook &r, cudaStream_t stream) {
   device_free(r.nbr, stream);
   device_free(r.tnbr, stream);
   device_free(r.counts_dev, stream);
+  free_row_order(r.order, stream);
+  free_row_order(r.torder, stream);
   r = Rulebook{};
 }
 
@@ -613,6 +615,8 @@ int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
   long long n = g->n_active;
   SCN_REQUIRE(K * std::max<long long>(n, 1) < (1ll << 40), SCN_ERR_UNSUPPORTED, "rulebook too large");
   rb.n_offsets = (int)K;
+  rb.dim = md->dim;
+  for (int d = 0; d < md->dim; ++d) rb.filter[d] = filter_size[d];
   rb.n_in = rb.n_out = n;
   SCN_TRY(device_alloc((void **)&rb.nbr, sizeof(int) * (size_t)(K * std::max<long long>(n, 1)), stream));
   SCN_TRY(device_alloc((void **)&rb.counts_dev, sizeof(unsigned long long) * (size_t)K, stream));
@@ -834,6 +838,8 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
   gout.n_active = n_out;
   SCN_TRY(device_alloc((void **)&gout.row_keys, sizeof(unsigned long long) * (size_t)std::max<long long>(n_out, 1), stream));
   rb.n_offsets = (int)K;
+  rb.dim = md->dim;
+  for (int d = 0; d < md->dim; ++d) rb.filter[d] = filter_size[d];
   rb.n_in = n_in;
   rb.n_out = n_out;
   size_t nbr_bytes = sizeof(int) * (size_t)(K * std::max<long long>(n_out, 1));
@@ -1037,6 +1043,8 @@ static int chain_collect(scn_metadata *md, long long n_in, long long batch_size,
       lv.gout.n_active = n_out;
       lv.gout.batch_size = batch_size;
       lv.rb.n_offsets = (int)lv.K;
+      lv.rb.dim = dim;
+      for (int d = 0; d < dim; ++d) lv.rb.filter[d] = filter[d];
       lv.rb.n_in = n_in;
       lv.rb.n_out = n_out;
       lv.rb.built = true;

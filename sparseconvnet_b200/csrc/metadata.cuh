@@ -43,11 +43,26 @@ struct CountTicket {
 void count_ticket_release(CountTicket *t);
 int count_ticket_total(CountTicket *t, long long *total);  // waits for the event only
 
+// The packing of a table's output rows into tensor-core tiles (row_order.cu): order[p] = output row at position
+// p, -1 past the end (padded to whole tiles); tile_bits[t][words] = filter offsets for which any of the 128 rows
+// of tile t has a rule.
+constexpr int kOrderTile = 128;
+constexpr int kOrderMaxOffsets = 128;
+struct RowOrder {
+  int *order = nullptr;
+  unsigned *tile_bits = nullptr;
+  int words = 1;  // 32-bit words per tile: 1 up to 32 offsets, else 4
+  long long n_tiles = 0;
+};
+
 struct Rulebook {
   int n_offsets = 0;  // filter volume K
+  int dim = 0;
+  int64_t filter[kMaxDim] = {0};
   long long n_in = 0, n_out = 0;
   int *nbr = nullptr;
   int *tnbr = nullptr;                       // built on first use
+  RowOrder order, torder;                    // of nbr and of tnbr; built on first use
   unsigned long long *counts_dev = nullptr;  // [K] rules per offset
   std::vector<long long> counts_host;        // filled on first request (waits for the stream)
   long long total_rules = -1;
@@ -60,6 +75,9 @@ int rulebook_counts(Rulebook &rb, cudaStream_t stream);         // fills counts_
 // waiting if the copy has already landed.  total_rules stays -1 while the copy is in flight.
 int rulebook_counts_async(Rulebook &rb, cudaStream_t stream);
 int rulebook_transposed(Rulebook &rb, cudaStream_t stream);     // builds tnbr if missing
+// builds the packing order of the table [K][n] (nbr or tnbr of `rb`) if missing
+int rulebook_row_order(const Rulebook &rb, const int *table, long long n, RowOrder &ord, cudaStream_t stream);
+void free_row_order(RowOrder &o, cudaStream_t stream);
 
 struct PendingChain;  // metadata.cu: levels of a strided chain whose kernels run on the side stream
 

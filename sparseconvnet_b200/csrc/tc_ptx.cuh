@@ -30,7 +30,7 @@ int prepare_weights(const float *w, unsigned char *out, int K, int cin, int cout
 // thread has a non-zero weight token set (scn_set_weight_token), an image is looked up under
 // (device, token, layout, shape) and built only when it is not there; with token 0 it is scratch of the
 // call.  `needs_build` says whether the caller has to launch its preparation kernel.
-enum WeightImageKind : int { WIMG_ROWS = 1, WIMG_ROWS_B3, WIMG_ROWS_THIN, WIMG_TC };
+enum WeightImageKind : int { WIMG_ROWS = 1, WIMG_ROWS_B3, WIMG_ROWS_THIN, WIMG_TC, WIMG_TILE };
 struct WeightImage {
   void *ptr = nullptr;
   bool cached = false;

@@ -1,0 +1,95 @@
+"""k_conv_tile and the row order it packs its tiles by, against the fp32 kernels (themselves checked against the
+reference's results in test_gpu_parity.py).
+
+Tolerances relative to the largest output: the three-term form drops m m' and what h + m leaves of x, 2^-17 of a product
+each, so 2^-16 of the largest sum of |products|, which stays below 4 of the largest output for these random sums: 1e-4
+(the fp32 bar).  One bf16 product: 2^-8 per product, averaging to 1e-2."""
+import numpy as np
+import pytest
+import torch
+
+from tests import helpers
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"tf32x3": helpers.FP32_TOL, "tf32": helpers.FP32_TOL, "bf16": helpers.TC_TOL}
+
+
+def _points(n, dim, size, seed):
+    rng = np.random.default_rng(seed)
+    pts = rng.integers(0, size, (n, dim))
+    if n > 200:  # a wavy surface: masks repeat as they do on scans
+        pts[:, dim - 1] = size // 2 + size // 5 * np.sin(pts[:, 0] / 6.0) + rng.integers(0, 2, n)
+    pts = np.unique(pts, axis=0)[rng.permutation(len(np.unique(pts, axis=0)))]
+    return np.concatenate([pts, rng.integers(0, 2, (len(pts), 1))], axis=1)
+
+
+def _compare(layers, coords, dim, size, cin, precision, cuda, mode=3):
+    import sparseconvnet_b200 as scn
+    rng = np.random.default_rng(cin)
+    feats = torch.from_numpy(rng.standard_normal((coords.shape[0], cin)).astype(np.float32)).to(cuda)
+    try:
+        with torch.no_grad():
+            x = scn.InputLayer(dim, size, mode=mode)([torch.from_numpy(coords), feats])
+            for layer in layers:
+                scn.set_precision("fp32")
+                want = layer.to(cuda)(x)
+                scn.set_precision(precision)
+                got = layer(x)
+                again = layer(x)
+                x.metadata.poll_errors()
+                assert got.features.shape == want.features.shape
+                assert torch.equal(got.features, again.features), "not the same twice"
+                e = helpers.rel_err(got.features.cpu().numpy(), want.features.cpu().numpy())
+                assert e <= TOL[precision], (layer, precision, coords.shape[0], e)
+                x = want
+    finally:
+        scn.set_precision("fp32")
+
+
+@pytest.mark.parametrize("precision", ["tf32x3", "bf16", "tf32"])
+@pytest.mark.parametrize("cin,cout", [(32, 32), (16, 16), (8, 24), (24, 40), (48, 64), (64, 72), (96, 96), (80, 160),
+                                      (128, 256), (320, 8)])
+def test_plane_counts(cin, cout, precision, cuda):
+    import sparseconvnet_b200 as scn
+    torch.manual_seed(cin + cout)
+    sc = scn.SubmanifoldConvolution(3, cin, cout, 3, True)
+    sc.bias.data.normal_()
+    _compare([sc], _points(9001, 3, 72, 1), 3, 72, cin, precision, cuda)
+
+
+@pytest.mark.parametrize("n", [1, 2, 127, 128, 129, 257, 4095, 4097, 60001])
+@pytest.mark.parametrize("cin,cout", [(32, 32), (64, 96)])
+def test_row_counts(n, cin, cout, cuda):
+    import sparseconvnet_b200 as scn
+    torch.manual_seed(n)
+    layers = [scn.SubmanifoldConvolution(3, cin, cout, 3, False), scn.Convolution(3, cout, 64, 2, 2, True),
+              scn.SubmanifoldConvolution(3, 64, 64, 3, False), scn.Deconvolution(3, 64, 32, 2, 2, False)]
+    _compare(layers, _points(n, 3, 160, n), 3, 160, cin, "tf32x3", cuda, mode=0 if n < 300 else 3)
+
+
+@pytest.mark.parametrize("dim,filter_size,stride", [(1, 3, 2), (2, 3, 2), (2, 5, 3), (3, 1, 1), (4, 3, 2), (3, 5, 2)])
+def test_filters(dim, filter_size, stride, cuda):
+    """1 to 125 filter offsets: one to five sort digits, one and four mask words, keys that join offsets."""
+    import sparseconvnet_b200 as scn
+    size = {1: 4001, 2: 182, 3: 63, 4: 23}[dim]
+    size = (size - filter_size) // stride * stride + filter_size
+    torch.manual_seed(dim)
+    layers = [scn.SubmanifoldConvolution(dim, 32, 48, filter_size, False)]
+    if filter_size > 1:
+        layers += [scn.Convolution(dim, 48, 32, filter_size, stride, False), scn.Deconvolution(dim, 32, 16, filter_size, stride, False)]
+    pts = _points(14000, dim, size, dim)
+    pts[:, :dim] = np.clip(pts[:, :dim], 0, size - 1)
+    _compare(layers, pts, dim, size, 32, "tf32x3", cuda)
+
+
+@pytest.mark.parametrize("split", ["1", "2", "5", "16"])
+@pytest.mark.parametrize("precision", ["tf32x3", "bf16"])
+@pytest.mark.parametrize("n", [700, 30000])
+def test_splits(split, precision, n, cuda, monkeypatch):
+    import sparseconvnet_b200 as scn
+    monkeypatch.setenv("SCN_TILE_SPLIT", split)
+    torch.manual_seed(n)
+    layers = [scn.SubmanifoldConvolution(3, 64, 64, 3, True), scn.SubmanifoldConvolution(3, 64, 128, 3, False),
+              scn.Convolution(3, 128, 96, 2, 2, False)]
+    _compare(layers, _points(n, 3, 120, 7), 3, 120, 64, precision, cuda)
