@@ -324,10 +324,34 @@ int conv_forward_dispatch(const float *in, long long rows_in, float *out, long l
 // `disjoint` additionally promises that every output row HAS a rule: the caller clears it when the
 // fine grid may hold rows that are in no map (earlier duplicates under input mode 0), whose output
 // the scatter form would leave unwritten while the gather form and the reference give them the bias.
-static long long tile_min_rows() {
-  const char *e = any_knob() ? getenv("SCN_TILE_MIN_ROWS") : nullptr;
-  return e ? atoll(e) : 1;
+// Does the convolution of a rulebook table run on mask-sorted tensor-core tiles?  Every bf16-class shape the kernel takes.
+static bool tile_takes(const float *in, const float *in_b, int planes_a, const float *out, const float *bias, int K, int cin,
+                       int cout, int groups, int precision, long long rows_out) {
+  return precision != SCN_PRECISION_FP32 && rows_out > 0 && tile_enabled(cout <= 64) &&
+         conv_tile_supported(in, in_b, planes_a, out, bias, K, cin, cout, groups);
 }
+
+// out [rows_out, groups * cout] = bias + sum_k in[table[k][.]] @ W[k] for a table of `rb` (nbr with rb.order, tnbr with
+// rb.torder): on mask-sorted tiles where they apply, otherwise whichever kernel conv_forward_dispatch picks.  Shared by the
+// forward operators and the input-gradient pass of the backward ones.
+int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, long long rows_in, float *out,
+                       long long rows_out, const float *weight, const float *bias, int cin, int cout, int groups,
+                       int precision, int *flags, cudaStream_t stream, const float *bn_scale, const float *bn_shift,
+                       float leak, const float *pre_scale, const float *pre_shift, float pre_leak, const float *in_b,
+                       int planes_a) {
+  const int *table = transposed_table ? rb.tnbr : rb.nbr;
+  if (tile_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, precision, rows_out)) {
+    RowOrder &ord = transposed_table ? rb.torder : rb.order;
+    SCN_TRY(rulebook_row_order(rb, table, rows_out, ord, stream));
+    SCN_TRY(conv_forward_tile(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, table, ord, rb.n_offsets,
+                              cin, cout, precision, flags, stream, pre_scale, pre_shift, pre_leak, in_b, planes_a));
+    g_last_kernel = cout <= 64 ? SCN_KERNEL_CONV_ROWS : rows_out <= 148 * 256 ? SCN_KERNEL_CONV_TC : SCN_KERNEL_CONV_WIDE;
+    return SCN_OK;
+  }
+  return conv_forward_dispatch(in, rows_in, out, rows_out, weight, bias, table, rb.n_offsets, cin, cout, groups, precision,
+                               flags, stream, bn_scale, bn_shift, leak, pre_scale, pre_shift, pre_leak, in_b, planes_a);
+}
+
 static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float *in, float *out,
                     const float *weight, const float *bias, int n_in_planes, int n_out_planes, int groups,
                     int precision, cudaStream_t stream, double *macs, bool disjoint = false,
@@ -345,7 +369,6 @@ static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float
   int cin = n_in_planes / groups, cout = n_out_planes / groups;
   long long rows_in = transposed ? rb.n_out : rb.n_in;
   long long rows_out = transposed ? rb.n_in : rb.n_out;
-  const int *table = rb.nbr;
   if (rows_out > 0) {
     SCN_REQUIRE(out && (in || rows_in == 0), SCN_ERR_BAD_ARG, "null features");
     if (!md->flags_dev) {
@@ -353,32 +376,21 @@ static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float
       SCN_CUDA_CHECK(cudaMemsetAsync(md->flags_dev, 0, sizeof(int), stream));
     }
   }
-  // tensor cores over mask-sorted tiles: every bf16-class shape it takes
-  const bool tile = precision != SCN_PRECISION_FP32 && rows_out >= tile_min_rows() && tile_enabled(cout <= 64) &&
-                    conv_tile_supported(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups);
+  const bool tile = tile_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, precision, rows_out);
   // the transposed layer with one rule per output row runs from its input side, on the table as built
   const bool scatter = !tile && transposed && disjoint && precision == SCN_PRECISION_TF32X3 && rows_in > 0 &&
                        !(getenv("SCN_X3_ROWS") && atoi(getenv("SCN_X3_ROWS")) == 0) &&
                        !(getenv("SCN_ROWS_SCATTER") && atoi(getenv("SCN_ROWS_SCATTER")) == 0) &&
                        conv_rows_supported(in, out, weight, bias, rb.n_offsets, cin, cout, groups);
-  if (transposed && !scatter) {
-    SCN_TRY(rulebook_transposed(rb, stream));
-    table = rb.tnbr;
-  }
-  if (tile) {
-    RowOrder &ord = transposed ? rb.torder : rb.order;
-    SCN_TRY(rulebook_row_order(rb, table, rows_out, ord, stream));
-    SCN_TRY(conv_forward_tile(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, table, ord, rb.n_offsets,
-                              cin, cout, precision, md->flags_dev, stream, pre_scale, pre_shift, pre_leak, in_b, planes_a));
-    g_last_kernel = cout <= 64 ? SCN_KERNEL_CONV_ROWS : rows_out <= 148 * 256 ? SCN_KERNEL_CONV_TC : SCN_KERNEL_CONV_WIDE;
-  } else if (rows_out > 0 && scatter) {
+  if (transposed && !scatter) SCN_TRY(rulebook_transposed(rb, stream));
+  if (rows_out > 0 && scatter) {
     SCN_TRY(conv_forward_rows_scatter(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, rb.nbr,
                                       rb.n_offsets, cin, cout, md->flags_dev, stream));
     g_last_kernel = SCN_KERNEL_CONV_ROWS;
   } else if (rows_out > 0) {
-    SCN_TRY(conv_forward_dispatch(in, rows_in, out, rows_out, weight, bias, table, rb.n_offsets, cin, cout, groups,
-                                  precision, md->flags_dev, stream, bn_scale, bn_shift, leak, pre_scale, pre_shift,
-                                  pre_leak, in_b, planes_a));
+    SCN_TRY(conv_forward_table(rb, transposed, in, rows_in, out, rows_out, weight, bias, cin, cout, groups, precision,
+                               md->flags_dev, stream, bn_scale, bn_shift, leak, pre_scale, pre_shift, pre_leak, in_b,
+                               planes_a));
   }
   if (macs) {  // the reference's return value: rules x ip x op x groups (CPU/Convolution.cpp:141)
     if (g_deferred_counts.load()) {

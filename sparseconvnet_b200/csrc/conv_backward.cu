@@ -21,25 +21,26 @@
 namespace scn {
 
 extern std::atomic<int> g_backward_precision;
-int conv_forward_dispatch(const float *in, long long rows_in, float *out, long long rows_out, const float *weight,
-                          const float *bias, const int *table, int K, int cin, int cout, int groups, int precision,
-                          int *flags, cudaStream_t stream, const float *bn_scale = nullptr,
-                          const float *bn_shift = nullptr, float leak = 1.f, const float *pre_scale = nullptr,
-                          const float *pre_shift = nullptr, float pre_leak = 1.f, const float *in_b = nullptr,
-                          int planes_a = 0);
+int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, long long rows_in, float *out,
+                       long long rows_out, const float *weight, const float *bias, int cin, int cout, int groups,
+                       int precision, int *flags, cudaStream_t stream, const float *bn_scale = nullptr,
+                       const float *bn_shift = nullptr, float leak = 1.f, const float *pre_scale = nullptr,
+                       const float *pre_shift = nullptr, float pre_leak = 1.f, const float *in_b = nullptr,
+                       int planes_a = 0);
 int conv_forward_simt(const float *in, long long n_in, float *out, long long n_out, const float *weight,
                       const float *bias, const int *table, int K, int cin, int cout, int groups, int *flags,
                       cudaStream_t stream);
 
-// W [K][groups][cin][cout] -> [K][groups][cout][cin]
+// W [K][groups][cin][cout] -> [K][groups][cout][cin]; mirror_groups > 0 (the number of groups): offset k goes to K - 1 - k
 __global__ void k_transpose_weight(const float *__restrict__ w, float *__restrict__ wt, long long n_mats, int cin,
-                                   int cout) {
+                                   int cout, int mirror_groups) {
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long per = (long long)cin * cout;
   if (idx >= n_mats * per) return;
   const long long m = idx / per;
   const int c = (int)((idx % per) / cout), n = (int)(idx % cout);
-  wt[m * per + (long long)n * cin + c] = w[idx];
+  const long long to = mirror_groups ? n_mats - (m / mirror_groups + 1) * mirror_groups + m % mirror_groups : m;
+  wt[to * per + (long long)n * cin + c] = w[idx];
 }
 
 // partial[chunk][k][g][c][n] = sum over the chunk's rulebook entries j of offset k of
@@ -334,14 +335,14 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
   if (d_in) {
     float *wt = nullptr;
     SCN_TRY(device_alloc((void **)&wt, sizeof(float) * (size_t)w_elems, stream));
-    SCN_LAUNCH(k_transpose_weight, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, weight, wt, (long long)K * groups, cin, cout);
-    const int *table = rb.nbr;  // Deconvolution: coarse row <- fine rows
-    if (!transposed) {
-      SCN_TRY(rulebook_transposed(rb, stream));
-      table = rb.tnbr;
-    }
-    SCN_TRY(conv_forward_dispatch(d_out, rows_out, d_in, rows_in, wt, nullptr, table, K, cout, cin, groups,
-                                  g_backward_precision.load(), md->flags_dev, stream));
+    // Deconvolution: coarse row <- fine rows, the table as built.  A submanifold rulebook of odd filter sizes is its own
+    // transposed one with the offsets in reverse, so that its table and row order serve the backward pass as well.
+    const bool mirrored = !transposed && rb.symmetric;
+    SCN_LAUNCH(k_transpose_weight, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, weight, wt, (long long)K * groups, cin, cout, mirrored ? groups : 0);
+    const bool use_tnbr = !transposed && !mirrored;
+    if (use_tnbr) SCN_TRY(rulebook_transposed(rb, stream));
+    SCN_TRY(conv_forward_table(rb, use_tnbr, d_out, rows_out, d_in, rows_in, wt, nullptr, cout, cin, groups,
+                               g_backward_precision.load(), md->flags_dev, stream));
     SCN_TRY(device_free(wt, stream));
   }
   return SCN_OK;

@@ -48,6 +48,7 @@ int count_ticket_total(CountTicket *t, long long *total);  // waits for the even
 // of tile t has a rule.
 constexpr int kOrderTile = 128;
 constexpr int kOrderMaxOffsets = 128;
+inline int mask_words(int K) { return K <= 32 ? 1 : 4; }
 struct RowOrder {
   int *order = nullptr;
   unsigned *tile_bits = nullptr;
@@ -63,11 +64,15 @@ struct Rulebook {
   int *nbr = nullptr;
   int *tnbr = nullptr;                       // built on first use
   RowOrder order, torder;                    // of nbr and of tnbr; built on first use
+  // offsets with a rule of every output row of nbr, mask_words(K) words each (submanifold rulebooks up to
+  // kOrderMaxOffsets offsets; null otherwise)
+  unsigned *masks = nullptr;
   unsigned long long *counts_dev = nullptr;  // [K] rules per offset
   std::vector<long long> counts_host;        // filled on first request (waits for the stream)
   long long total_rules = -1;
   CountTicket *ticket = nullptr;             // counts in flight (rulebook_counts_async)
   bool built = false;
+  bool symmetric = false;  // submanifold with odd filter sizes: tnbr[k] is nbr[K - 1 - k]
 };
 
 int rulebook_counts(Rulebook &rb, cudaStream_t stream);         // fills counts_host/total_rules (waits)

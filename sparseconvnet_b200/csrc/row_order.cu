@@ -12,8 +12,9 @@
 //   shells and planes (267 k rows)   26.5 -> 13.8     4-D moving shells, 81 offsets      71.8 -> 35.2
 //   stride-2 transposed layers (8 offsets, one rule per row): -> 1
 //
-// Steps: k_order_keys (mask -> sort key of up to 64 bits), then one stable counting pass per digit of at most
-// nine bits (k_order_count, k_order_scatter), then k_order_tiles (the union of the masks of every 128 rows).
+// Steps: k_order_keys (mask -> sort key, and the digit counts of the first pass), then one stable counting pass per
+// digit of at most nine bits (k_order_scatter, with k_order_count between two passes), then k_order_tiles (the union
+// of the masks of every 128 rows).
 #include <stdlib.h>
 
 #include <algorithm>
@@ -25,91 +26,112 @@ namespace {
 
 constexpr int kTile = kOrderTile;
 constexpr int kMaxDigit = 512;  // nine bits
-constexpr int kCountThreads = 512, kScatterThreads = 512;
+constexpr int kThreads = 1024, kWarps = kThreads / 32;
 
+template <typename KEY>
 struct KeyBits {
-  unsigned char pos[kOrderMaxOffsets];  // bit of the sort key that offset k sets; 255: none
+  KEY bit[sizeof(KEY) == 4 ? 32 : kOrderMaxOffsets];  // what an offset with a rule sets in the sort key
 };
 
-// One thread per output row: which offsets have a rule, and the sort key made of them.
-template <typename KEY, int WORDS>
-__global__ void __launch_bounds__(256)
-k_order_keys(const int *__restrict__ nbr, long long n, int K, KeyBits B, KEY *__restrict__ keys,
-             unsigned *__restrict__ masks) {
-  const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  KEY key = 0;
-  unsigned m[WORDS];
-#pragma unroll
-  for (int w = 0; w < WORDS; ++w) m[w] = 0;
-#pragma unroll
-  for (int w = 0; w < WORDS; ++w) {
-    if (w * 32 >= K) break;
-#pragma unroll 8
-    for (int b = 0; b < 32; ++b) {
-      const int k = w * 32 + b;
-      if (k < K && __ldg(nbr + (long long)k * n + r) >= 0) {
-        m[w] |= 1u << b;
-        if (B.pos[k] != 255) key |= (KEY)1 << B.pos[k];
-      }
-    }
+// One more row with digit d in the block's counts: most rows of a surface share a handful of masks, so one update per
+// distinct digit in the warp.
+__device__ __forceinline__ void count_digit(int *h, int d) {
+  const unsigned peers = __match_any_sync(__activemask(), d);
+  if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&h[d], __popc(peers));
+}
+__device__ __forceinline__ void store_counts(const int *h, int R, int *block_count, int *total) {
+  for (int i = threadIdx.x; i < R; i += kThreads) {
+    block_count[(long long)blockIdx.x * R + i] = h[i];
+    if (h[i]) atomicAdd(&total[i], h[i]);
   }
-  keys[r] = key;
+}
+
+// Which offsets of a row have a rule (read from the table unless the rulebook's builder has left them in `known`), and
+// the sort key made of them.
+template <typename KEY, int WORDS>
+__global__ void __launch_bounds__(kThreads)
+k_order_keys(const int *__restrict__ nbr, const unsigned *__restrict__ known, long long n, int K, KeyBits<KEY> B,
+             int rows_per_block, int R, KEY *__restrict__ keys, unsigned *__restrict__ masks,
+             int *__restrict__ block_count, int *__restrict__ total) {
+  __shared__ int h[kMaxDigit];
+  for (int i = threadIdx.x; i < R; i += kThreads) h[i] = 0;
+  __syncthreads();
+  const long long r0 = (long long)blockIdx.x * rows_per_block, r1 = min(n, r0 + rows_per_block);
+  for (long long r = r0 + threadIdx.x; r < r1; r += kThreads) {
+    KEY key = 0;
 #pragma unroll
-  for (int w = 0; w < WORDS; ++w) masks[r * WORDS + w] = m[w];
+    for (int w = 0; w < WORDS; ++w) {
+      unsigned m = 0;
+      if (known) {
+        m = __ldg(known + r * WORDS + w);
+      } else {
+#pragma unroll 1
+        for (int b0 = 0; b0 < 32 && w * 32 + b0 < K; b0 += 8) {
+          int v[8];
+#pragma unroll
+          for (int b = 0; b < 8; ++b) v[b] = w * 32 + b0 + b < K ? __ldg(nbr + (long long)(w * 32 + b0 + b) * n + r) : -1;
+#pragma unroll
+          for (int b = 0; b < 8; ++b) m |= v[b] >= 0 ? 1u << (b0 + b) : 0u;
+        }
+        masks[r * WORDS + w] = m;
+      }
+#pragma unroll
+      for (int b = 0; b < 32; ++b)
+        if (m >> b & 1u) key |= B.bit[w * 32 + b];
+    }
+    keys[r] = key;
+    count_digit(h, (int)key & (R - 1));
+  }
+  __syncthreads();
+  store_counts(h, R, block_count, total);
 }
 
 // Digit counts of every block's rows (block_count [blocks][R]) and of all rows (total [R], zeroed before).
 template <typename KEY>
-__global__ void __launch_bounds__(kCountThreads)
+__global__ void __launch_bounds__(kThreads)
 k_order_count(const KEY *__restrict__ keys, long long n, int rows_per_block, int shift, int R,
               int *__restrict__ block_count, int *__restrict__ total) {
   __shared__ int h[kMaxDigit];
-  for (int i = threadIdx.x; i < R; i += blockDim.x) h[i] = 0;
+  for (int i = threadIdx.x; i < R; i += kThreads) h[i] = 0;
   __syncthreads();
   const long long r0 = (long long)blockIdx.x * rows_per_block, r1 = min(n, r0 + rows_per_block);
-  for (long long r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-    const int d = (int)(keys[r] >> shift) & (R - 1);
-    // most rows of a surface share a handful of masks: one update per distinct digit in the warp
-    const unsigned peers = __match_any_sync(__activemask(), d);
-    if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&h[d], __popc(peers));
-  }
+  for (long long r = r0 + threadIdx.x; r < r1; r += kThreads) count_digit(h, (int)(keys[r] >> shift) & (R - 1));
   __syncthreads();
-  for (int i = threadIdx.x; i < R; i += blockDim.x) {
-    block_count[(long long)blockIdx.x * R + i] = h[i];
-    if (h[i]) atomicAdd(&total[i], h[i]);
-  }
+  store_counts(h, R, block_count, total);
 }
 
 // Stable scatter of a block's rows by one digit.  A block's first position of digit d is (rows of smaller
 // digits) + (rows of digit d in the blocks before it), both read from the counts; within the block the warps
 // own consecutive segments.  rows_in null: the row of position i is i.
 template <typename KEY>
-__global__ void __launch_bounds__(kScatterThreads)
+__global__ void __launch_bounds__(kThreads)
 k_order_scatter(const KEY *__restrict__ keys, const int *__restrict__ rows_in, long long n, int rows_per_block,
                 int shift, int R, const int *__restrict__ block_count, const int *__restrict__ total,
                 KEY *__restrict__ keys_out, int *__restrict__ rows_out) {
-  constexpr int kWarps = kScatterThreads / 32;
-  __shared__ int cnt[kWarps][kMaxDigit];  // then: next position of digit d for warp w
+  __shared__ unsigned short cnt[kWarps][kMaxDigit];  // rows of digit d in warp w's segment, then in the warps before it
+  __shared__ int base[kMaxDigit], part[kMaxDigit];   // (a block has fewer than 65536 rows)
   __shared__ int warp_sum[kWarps];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < kWarps * kMaxDigit; i += kScatterThreads) (&cnt[0][0])[i] = 0;
+  for (int i = tid; i < kWarps * kMaxDigit / 2; i += kThreads) reinterpret_cast<unsigned *>(&cnt[0][0])[i] = 0;
   __syncthreads();
   const int seg = rows_per_block / kWarps;  // a multiple of 32
   const long long s0 = (long long)blockIdx.x * rows_per_block + (long long)warp * seg;
   const long long s1 = min(n, s0 + seg);
   for (long long r = s0 + lane; r < s1; r += 32) {
+    const unsigned act = __activemask();
     const int d = (int)(keys[r] >> shift) & (R - 1);
-    const unsigned peers = __match_any_sync(__activemask(), d);
-    if (lane == __ffs(peers) - 1) cnt[warp][d] += __popc(peers);
-    __syncwarp(__activemask());
+    const unsigned peers = __match_any_sync(act, d);
+    if (lane == __ffs(peers) - 1) cnt[warp][d] += (unsigned short)__popc(peers);
+    __syncwarp(act);
   }
-  // thread d: rows of digit d in the blocks before this one, and the exclusive scan of the totals
+  // rows of digit d in the blocks before this one: two threads per digit, every other block each
+  const int d = tid & (kMaxDigit - 1), half = tid / kMaxDigit;
   int before = 0, tot = 0;
-  if (tid < R) {
-    tot = total[tid];
-#pragma unroll 8
-    for (int b = 0; b < (int)blockIdx.x; ++b) before += block_count[(long long)b * R + tid];
+  if (d < R) {
+#pragma unroll 16
+    for (int b = half; b < (int)blockIdx.x; b += 2) before += __ldg(block_count + (long long)b * R + d);
+    if (half == 0) tot = total[d];
+    else part[d] = before;
   }
   int incl = tot;
 #pragma unroll
@@ -119,28 +141,60 @@ k_order_scatter(const KEY *__restrict__ keys, const int *__restrict__ rows_in, l
   }
   if (lane == 31) warp_sum[warp] = incl;
   __syncthreads();
-  int base = incl - tot + before;
-  for (int w = 0; w < warp; ++w) base += warp_sum[w];
-  if (tid < R) {
+  if (half == 0 && d < R) {
+    int at = incl - tot + before + part[d];
+    for (int w = 0; w < warp; ++w) at += warp_sum[w];
+    base[d] = at;
+    unsigned run = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-      const int c = cnt[w][tid];
-      cnt[w][tid] = base;
-      base += c;
+      const unsigned c = cnt[w][d];
+      cnt[w][d] = (unsigned short)run;
+      run += c;
     }
   }
   __syncthreads();
   for (long long r = s0 + lane; r < s1; r += 32) {
     const unsigned act = __activemask();
     const KEY key = keys[r];
-    const int d = (int)(key >> shift) & (R - 1);
-    const unsigned peers = __match_any_sync(act, d);
-    const int pos = cnt[warp][d] + __popc(peers & ((1u << lane) - 1u));
+    const int dg = (int)(key >> shift) & (R - 1);
+    const unsigned peers = __match_any_sync(act, dg);
+    const int pos = base[dg] + cnt[warp][dg] + __popc(peers & ((1u << lane) - 1u));
     __syncwarp(act);
-    if (lane == __ffs(peers) - 1) cnt[warp][d] += __popc(peers);
+    if (lane == __ffs(peers) - 1) cnt[warp][dg] += (unsigned short)__popc(peers);
     __syncwarp(act);
     if (keys_out) keys_out[pos] = key;
     rows_out[pos] = rows_in ? rows_in[r] : (int)r;
+  }
+}
+
+// Levels too small to sort: the identity order and its tiles in one launch, one warp per tile.
+template <int WORDS>
+__global__ void __launch_bounds__(256)
+k_order_plain(const int *__restrict__ nbr, long long n, int K, int *__restrict__ order, unsigned *__restrict__ tile_bits,
+              long long n_tiles) {
+  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (t >= n_tiles) return;
+#pragma unroll
+  for (int i = 0; i < kTile / 32; ++i) {
+    const long long p = t * kTile + i * 32 + lane;
+    order[p] = p < n ? (int)p : -1;
+  }
+#pragma unroll
+  for (int w = 0; w < WORDS; ++w) {
+    unsigned bits = 0;
+#pragma unroll 4
+    for (int b = 0; b < 32 && w * 32 + b < K; ++b) {
+      bool any = false;
+#pragma unroll
+      for (int i = 0; i < kTile / 32; ++i) {
+        const long long p = t * kTile + i * 32 + lane;
+        any |= p < n && __ldg(nbr + (long long)(w * 32 + b) * n + p) >= 0;
+      }
+      if (__any_sync(0xffffffffu, any)) bits |= 1u << b;
+    }
+    if (lane == 0) tile_bits[t * WORDS + w] = bits;
   }
 }
 
@@ -174,37 +228,52 @@ k_order_tiles(int *__restrict__ order, long long n, long long n_padded, const un
   }
 }
 
-__global__ void k_order_identity(int *order, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) order[i] = (int)i;
-}
-
-// Which key bit an offset sets.  Up to 32 offsets: one bit each, the first offset the highest (ordering by the
-// leading offsets first keeps masks that differ in the trailing ones together: 9.5 offsets per tile of 128 rows
-// on rooms; by how close an offset's frequency is to one half: 9.7).  More offsets: a 4-D filter of size 3 puts
-// the offsets of the earlier and later time slice first, OR-ed over one spatial dimension, then the slice of the
-// site itself in full (45 bits: 35.2 offsets per tile; all 81 bits in filter order: 40.8).  Other large filters:
-// OR-ed over groups of consecutive offsets.
-int key_bits(int dim, const int64_t *filter, int K, KeyBits &B) {
-  for (int k = 0; k < kOrderMaxOffsets; ++k) B.pos[k] = 255;
+// Which key bits the offsets set (pos[k], 255 for none), and how many bits there are.  Fewer bits cost fewer passes,
+// and below about 65 000 rows a coarser key also packs better, because full masks are hardly ever repeated.  Offsets
+// per tile of 128 rows on rooms of 405 k / 119 k / 37 k / 15 k rows, 27 offsets (in coordinate order 22.4 / 23.9 /
+// 23.8 / 25.6):
+//   27 bits, the first offset highest               9.48   9.88  10.3  17.3   three passes
+//   the 12 edges, then the 6 faces                   9.70  10.2   11.4  18.1   two
+//   OR-ed over the middle dimension (9 bits)        13.0   12.8   11.3  14.4   one
+// A 4-D filter of size 3 puts the offsets of the earlier and later time slice first, OR-ed over one spatial dimension,
+// then the slice of the site itself in full (45 bits: 35.2 offsets per tile of moving shells; all 81 bits in filter
+// order: 40.8), or OR-ed as well (27 bits: 38.2).  Other large filters: groups of consecutive offsets.
+int key_bits(const Rulebook &rb, int K, long long n, unsigned char *pos) {
+  for (int k = 0; k < kOrderMaxOffsets; ++k) pos[k] = 255;
+  bool three = rb.dim >= 3;
+  for (int d = 0; d < rb.dim; ++d) three &= rb.filter[d] == 3;
+  if (rb.dim == 3 && three && n < 65536) {
+    for (int k = 0; k < 27; ++k) pos[k] = (unsigned char)(8 - ((k / 9) * 3 + k % 3));
+    return 9;
+  }
+  if (rb.dim == 3 && three && n < 524288) {
+    int edges = 0, faces = 0;
+    for (int k = 0; k < 27; ++k) {
+      const int far = (k % 3 != 1) + (k / 3 % 3 != 1) + (k / 9 != 1);
+      if (far == 2) pos[k] = (unsigned char)(17 - edges++);
+      if (far == 1) pos[k] = (unsigned char)(5 - faces++);
+    }
+    return 18;
+  }
   if (K <= 32) {
-    for (int k = 0; k < K; ++k) B.pos[k] = (unsigned char)(K - 1 - k);
+    for (int k = 0; k < K; ++k) pos[k] = (unsigned char)(K - 1 - k);
     return K;
   }
-  if (dim == 4 && filter && filter[0] == 3 && filter[1] == 3 && filter[2] == 3 && filter[3] == 3) {
+  if (rb.dim == 4 && three) {
+    const bool full = n >= 262144;
     for (int k = 0; k < 81; ++k) {
       const int t = k % 3, z = (k / 3) % 3, y = (k / 9) % 3, x = k / 27;
       int rank;  // 0 = highest bit
       if (t == 1)
-        rank = 18 + (x * 3 + y) * 3 + z;
+        rank = 18 + (full ? (x * 3 + y) * 3 + z : x * 3 + z);
       else
         rank = (t == 0 ? 0 : 9) + x * 3 + z;
-      B.pos[k] = (unsigned char)(44 - rank);
+      pos[k] = (unsigned char)((full ? 44 : 26) - rank);
     }
-    return 45;
+    return full ? 45 : 27;
   }
-  const int group = (K + 44) / 45, bits = (K + group - 1) / group;
-  for (int k = 0; k < K; ++k) B.pos[k] = (unsigned char)(bits - 1 - k / group);
+  const int most = n >= 262144 ? 45 : 27, group = (K + most - 1) / most, bits = (K + group - 1) / group;
+  for (int k = 0; k < K; ++k) pos[k] = (unsigned char)(bits - 1 - k / group);
   return bits;
 }
 
@@ -224,40 +293,38 @@ struct Scratch {  // freed on every way out
 };
 
 template <typename KEY, int WORDS>
-int build(const int *table, long long n, int K, const KeyBits &B, int bits, RowOrder &ord, bool sort, cudaStream_t stream) {
+int build(const int *table, const unsigned *known, long long n, int K, const unsigned char *pos, int bits, RowOrder &ord, cudaStream_t stream) {
   Scratch tmp(stream);
   unsigned *masks = nullptr;
   KEY *keys[2] = {nullptr, nullptr};
   int *rows = nullptr, *counts = nullptr, *totals = nullptr;
-  SCN_TRY(tmp.get((void **)&masks, sizeof(unsigned) * WORDS * (size_t)n));
+  const int passes = (bits + 8) / 9, digit = (bits + passes - 1) / passes, R = 1 << digit;
+  // Rows per block: a multiple of the warps' 32-row chunks; one block per SM at most, because a block adds up the counts
+  // of the blocks before it itself
+  const long long rpb = std::min<long long>(ceil_div(ceil_div(n, 148), kThreads), 63) * kThreads;
+  const int blocks = (int)ceil_div(n, rpb);
+  KeyBits<KEY> B{};
+  for (int k = 0; k < K; ++k) B.bit[k] = pos[k] == 255 ? (KEY)0 : (KEY)1 << pos[k];
+  if (!known) SCN_TRY(tmp.get((void **)&masks, sizeof(unsigned) * WORDS * (size_t)n));
   SCN_TRY(tmp.get((void **)&keys[0], sizeof(KEY) * (size_t)n));
-  SCN_LAUNCH((k_order_keys<KEY, WORDS>), (unsigned)ceil_div(n, 256), 256, 0, stream, table, n, K, B, keys[0], masks);
-  if (!sort) {
-    SCN_LAUNCH(k_order_identity, (unsigned)ceil_div(n, 256), 256, 0, stream, ord.order, n);
-  } else {
-    const int passes = (bits + 8) / 9, digit = (bits + passes - 1) / passes, R = 1 << digit;
-    // Rows per block: a multiple of the warps' 32-row chunks; at most about 200 blocks, because a block adds up the
-    // counts of the blocks before it itself
-    long long rpb = ceil_div(ceil_div(n, 200), kScatterThreads) * kScatterThreads;
-    const int blocks = (int)ceil_div(n, rpb);
-    SCN_TRY(tmp.get((void **)&counts, sizeof(int) * (size_t)blocks * R));
-    SCN_TRY(tmp.get((void **)&totals, sizeof(int) * (size_t)passes * R));
-    SCN_CUDA_CHECK(cudaMemsetAsync(totals, 0, sizeof(int) * (size_t)passes * R, stream));
-    if (passes > 1) {
-      SCN_TRY(tmp.get((void **)&keys[1], sizeof(KEY) * (size_t)n));
-      SCN_TRY(tmp.get((void **)&rows, sizeof(int) * (size_t)n));
-    }
-    // the row arrays alternate so that the last pass writes ord.order
-    const int *src = nullptr;
-    for (int p = 0; p < passes; ++p) {
-      int *dst = ((passes - 1 - p) & 1) ? rows : ord.order;
-      KEY *kin = keys[p & 1], *kout = p + 1 < passes ? keys[(p + 1) & 1] : nullptr;
-      SCN_LAUNCH((k_order_count<KEY>), blocks, kCountThreads, 0, stream, kin, n, (int)rpb, p * digit, R, counts, totals + (size_t)p * R);
-      SCN_LAUNCH((k_order_scatter<KEY>), blocks, kScatterThreads, 0, stream, kin, src, n, (int)rpb, p * digit, R, counts, totals + (size_t)p * R, kout, dst);
-      src = dst;
-    }
+  SCN_TRY(tmp.get((void **)&counts, sizeof(int) * (size_t)blocks * R));
+  SCN_TRY(tmp.get((void **)&totals, sizeof(int) * (size_t)passes * R));
+  if (passes > 1) {
+    SCN_TRY(tmp.get((void **)&keys[1], sizeof(KEY) * (size_t)n));
+    SCN_TRY(tmp.get((void **)&rows, sizeof(int) * (size_t)n));
   }
-  SCN_LAUNCH((k_order_tiles<WORDS>), (unsigned)ceil_div(ord.n_tiles * 32, 256), 256, 0, stream, ord.order, n, ord.n_tiles * kTile, masks, ord.tile_bits, ord.n_tiles);
+  SCN_CUDA_CHECK(cudaMemsetAsync(totals, 0, sizeof(int) * (size_t)passes * R, stream));
+  SCN_LAUNCH((k_order_keys<KEY, WORDS>), blocks, kThreads, 0, stream, table, known, n, K, B, (int)rpb, R, keys[0], masks, counts, totals);
+  const int *src = nullptr;
+  for (int p = 0; p < passes; ++p) {
+    int *dst = ((passes - 1 - p) & 1) ? rows : ord.order;  // alternating so that the last pass writes ord.order
+    KEY *kin = keys[p & 1], *kout = p + 1 < passes ? keys[(p + 1) & 1] : nullptr;
+    if (p > 0)
+      SCN_LAUNCH((k_order_count<KEY>), blocks, kThreads, 0, stream, kin, n, (int)rpb, p * digit, R, counts, totals + (size_t)p * R);
+    SCN_LAUNCH((k_order_scatter<KEY>), blocks, kThreads, 0, stream, kin, src, n, (int)rpb, p * digit, R, counts, totals + (size_t)p * R, kout, dst);
+    src = dst;
+  }
+  SCN_LAUNCH((k_order_tiles<WORDS>), (unsigned)ceil_div(ord.n_tiles * 32, 256), 256, 0, stream, ord.order, n, ord.n_tiles * kTile, known ? known : masks, ord.tile_bits, ord.n_tiles);
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }
@@ -275,18 +342,31 @@ int rulebook_row_order(const Rulebook &rb, const int *table, long long n, RowOrd
   if (ord.order || n == 0) return SCN_OK;
   const int K = rb.n_offsets;
   SCN_REQUIRE(K >= 1 && K <= kOrderMaxOffsets && n < (1ll << 31), SCN_ERR_UNSUPPORTED, "row order: %d offsets", K);
-  KeyBits B;
-  const int bits = key_bits(rb.dim, rb.filter, K, B);
   RowOrder o;
   o.words = K <= 32 ? 1 : 4;
   o.n_tiles = ceil_div(n, kTile);
   int st = device_alloc((void **)&o.order, sizeof(int) * (size_t)o.n_tiles * kTile, stream);
   if (st == SCN_OK) st = device_alloc((void **)&o.tile_bits, sizeof(unsigned) * (size_t)o.words * o.n_tiles, stream);
-  // one tile per SM or fewer: nothing to gain from the order
-  const bool sort = n >= 4096 && !(getenv("SCN_ROW_ORDER") && atoi(getenv("SCN_ROW_ORDER")) == 0);
-  if (st == SCN_OK)
-    st = K <= 32 ? build<unsigned, 1>(table, n, K, B, bits, o, sort, stream)
-                 : build<unsigned long long, 4>(table, n, K, B, bits, o, sort, stream);
+  // Small levels are bound by latency whatever the order, and the sort takes as long as one of their layers.
+  long long least = 8192;
+  if (const char *e = getenv("SCN_ORDER_MIN_ROWS")) least = atoll(e);
+  if (st == SCN_OK && n < least) {
+    const unsigned grid = (unsigned)ceil_div(o.n_tiles * 32, 256);
+    if (K <= 32)
+      SCN_LAUNCH(k_order_plain<1>, grid, 256, 0, stream, table, n, K, o.order, o.tile_bits, o.n_tiles);
+    else
+      SCN_LAUNCH(k_order_plain<4>, grid, 256, 0, stream, table, n, K, o.order, o.tile_bits, o.n_tiles);
+    if (cudaGetLastError() != cudaSuccess) {
+      set_error("row order: launch failed");
+      st = SCN_ERR_CUDA;
+    }
+  } else if (st == SCN_OK) {
+    unsigned char pos[kOrderMaxOffsets];
+    const int bits = key_bits(rb, K, n, pos);
+    const unsigned *known = table == rb.nbr ? rb.masks : nullptr;
+    st = K <= 32 ? build<unsigned, 1>(table, known, n, K, pos, bits, o, stream)
+                 : build<unsigned long long, 4>(table, known, n, K, pos, bits, o, stream);
+  }
   if (st != SCN_OK) {
     free_row_order(o, stream);
     return st;
