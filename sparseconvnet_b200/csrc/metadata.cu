@@ -148,6 +148,82 @@ static void mailbox_release(int *slot) {
   P.free_slots.push_back(slot);
 }
 
+// ---- rule counts: pinned chunks are pooled per device and never given back to the driver -----------------------
+namespace {
+constexpr int kTicketValues = 256;  // filter volumes up to 256 offsets
+struct TicketPool {
+  std::mutex mu;
+  std::vector<unsigned long long *> chunks[64];  // kTicketValues values each
+  std::vector<CountTicket *> dropped[64];        // released before the device had written their counts (or just now)
+};
+TicketPool &ticket_pool() {
+  static TicketPool *p = new TicketPool();  // leaked on purpose: tickets may be released at exit
+  return *p;
+}
+}  // namespace
+
+static bool counts_landed(const CountTicket *t);
+
+// A ticket for a rulebook that is about to be built (none above kTicketValues offsets).
+static int count_ticket_new(Rulebook &rb) {
+  if (rb.ticket || rb.n_offsets > kTicketValues) return SCN_OK;
+  int dev = 0;
+  SCN_CUDA_CHECK(cudaGetDevice(&dev));
+  SCN_REQUIRE(dev < 64, SCN_ERR_UNSUPPORTED, "device %d", dev);
+  unsigned long long *host = nullptr;
+  CountTicket *t = nullptr;
+  TicketPool &P = ticket_pool();
+  {
+    std::lock_guard<std::mutex> lock(P.mu);
+    auto &dropped = P.dropped[dev];
+    for (size_t i = 0; i < dropped.size() && !host; ++i)
+      if (counts_landed(dropped[i])) {
+        t = dropped[i];
+        host = (unsigned long long *)t->host;
+        dropped[i] = dropped.back();
+        dropped.pop_back();
+      }
+    if (!host && !P.chunks[dev].empty()) {
+      host = P.chunks[dev].back();
+      P.chunks[dev].pop_back();
+    }
+    if (!host) {  // a slab of 256 chunks (512 KB of pinned memory) at a time
+      unsigned long long *slab = nullptr;
+      if (cudaHostAlloc((void **)&slab, sizeof(unsigned long long) * kTicketValues * 256,
+                        cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        SCN_REQUIRE(false, SCN_ERR_CUDA, "pinned allocation failed");
+      }
+      host = slab;
+      for (int i = 1; i < 256; ++i) P.chunks[dev].push_back(slab + (size_t)i * kTicketValues);
+    }
+  }
+  unsigned long long *host_dev = t ? t->dev : nullptr;
+  if (!t) {
+    t = new CountTicket();
+    if (cudaHostGetDevicePointer((void **)&host_dev, host, 0) != cudaSuccess) {
+      cudaGetLastError();
+      delete t;
+      std::lock_guard<std::mutex> lock(P.mu);
+      P.chunks[dev].push_back(host);
+      SCN_REQUIRE(false, SCN_ERR_CUDA, "pinned memory is not mapped");
+    }
+  }
+  t->host = host;
+  t->dev = host_dev;
+  t->n = rb.n_offsets;
+  t->device = dev;
+  t->refs.store(1);
+  for (int k = 0; k < t->n; ++k) t->host[k] = kCountPending;
+  rb.ticket = t;
+  return SCN_OK;
+}
+static unsigned long long *ticket_dev(const Rulebook &rb) { return rb.ticket ? rb.ticket->dev : nullptr; }
+static void count_ticket_zero(Rulebook &rb) {  // nothing will be launched: no rules
+  if (rb.ticket)
+    for (int k = 0; k < rb.ticket->n; ++k) rb.ticket->host[k] = 0;
+}
+
 __global__ void k_post_scalars(int *flags_dev, const int *scalars_dev, volatile int *mailbox) {
   mailbox[0] = *flags_dev;
   *flags_dev = 0;
@@ -526,6 +602,21 @@ struct FilterDesc {
   int tmax;
 };
 
+// Called by every block of a rulebook builder after it has added to the rule counts: the block that finishes last hands
+// them to the host (counts_host: pinned, device-mapped; null: nobody wants them).  counts[K] counts finished blocks.
+__device__ __forceinline__ void post_counts(unsigned long long *counts, int K, volatile unsigned long long *counts_host) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&counts[K], 1ull) == (unsigned long long)gridDim.x * gridDim.y - 1;
+  }
+  __syncthreads();
+  if (!last || !counts_host) return;
+  for (int k = threadIdx.x; k < K; k += blockDim.x) counts_host[k] = atomicAdd(&counts[k], 0ull);
+  __threadfence_system();
+}
+
 // One thread per output site, looping over this block's range of filter offsets.  Offset k
 // (row-major over the filter, last dimension fastest, RectangularRegions.h:30-38) looks at
 // input = output + delta_k with delta = k_d - f_d / 2 (SubmanifoldConvolutionRules.h:15-19).
@@ -534,7 +625,8 @@ struct FilterDesc {
 __global__ void __launch_bounds__(256)
 k_submanifold_rules(KeyLayout L, HashTable T, const unsigned long long *__restrict__ row_keys,
                     long long n, int K, FilterDesc F, int k_chunk, int *__restrict__ nbr,
-                    unsigned long long *counts, int mirrored, unsigned *__restrict__ masks, int mask_words) {
+                    unsigned long long *counts, int mirrored, unsigned *__restrict__ masks, int mask_words,
+                    volatile unsigned long long *counts_host) {
   extern __shared__ long long sh_raw[];
   long long *sh_keydelta = sh_raw;                         // [k_chunk]
   int *sh_count = (int *)(sh_keydelta + k_chunk);          // [k_chunk]
@@ -604,6 +696,21 @@ k_submanifold_rules(KeyLayout L, HashTable T, const unsigned long long *__restri
       atomicAdd(&counts[kk], (unsigned long long)sh_count[kk - k0]);
       if (mirrored && kk < K / 2) atomicAdd(&counts[K - 1 - kk], (unsigned long long)sh_count[kk - k0]);
     }
+  post_counts(counts, K, counts_host);
+}
+
+// What a submanifold rulebook starts from, in one launch: counts and masks zero, the mirrored half of the table empty.
+__global__ void __launch_bounds__(256)
+k_rules_init(unsigned long long *counts, int n_counts, unsigned *masks, long long n_masks, int *nbr, long long n_nbr) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  for (long long j = i; j < n_counts; j += step) counts[j] = 0;
+  for (long long j = i; j < n_masks; j += step) masks[j] = 0;
+  if ((uintptr_t)nbr % 16 == 0) {
+    for (long long j = i; j < n_nbr / 4; j += step) reinterpret_cast<int4 *>(nbr)[j] = make_int4(-1, -1, -1, -1);
+    for (long long j = n_nbr / 4 * 4 + i; j < n_nbr; j += step) nbr[j] = -1;
+  } else {
+    for (long long j = i; j < n_nbr; j += step) nbr[j] = -1;
+  }
 }
 
 int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
@@ -639,27 +746,27 @@ int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
   }
   rb.n_in = rb.n_out = n;
   SCN_TRY(device_alloc((void **)&rb.nbr, sizeof(int) * (size_t)(K * std::max<long long>(n, 1)), stream));
-  SCN_TRY(device_alloc((void **)&rb.counts_dev, sizeof(unsigned long long) * (size_t)K, stream));
-  SCN_CUDA_CHECK(cudaMemsetAsync(rb.counts_dev, 0, sizeof(unsigned long long) * (size_t)K, stream));
-  if (n > 0) {
+  SCN_TRY(device_alloc((void **)&rb.counts_dev, sizeof(unsigned long long) * (size_t)(K + 1), stream));
+  SCN_TRY(count_ticket_new(rb));
+  if (n == 0) {
+    SCN_CUDA_CHECK(cudaMemsetAsync(rb.counts_dev, 0, sizeof(unsigned long long) * (size_t)(K + 1), stream));
+    count_ticket_zero(rb);
+  } else {
     const int threads = 256;
     long long bx = ceil_div(n, threads);
     bool mirrored = K > 1 && !(getenv("SCN_RULES_MIRROR") && atoi(getenv("SCN_RULES_MIRROR")) == 0);
     for (int d = 0; d < md->dim; ++d) mirrored &= (filter_size[d] % 2 == 1);
     const long long k_end = mirrored ? K / 2 + 1 : K;  // offsets that are looked up
     const int words = mask_words((int)K);
-    if (K <= kOrderMaxOffsets) {
-      SCN_TRY(device_alloc((void **)&rb.masks, sizeof(unsigned) * words * (size_t)n, stream));
-      SCN_CUDA_CHECK(cudaMemsetAsync(rb.masks, 0, sizeof(unsigned) * words * (size_t)n, stream));
-    }
-    if (mirrored)  // the mirrored half starts out empty
-      SCN_CUDA_CHECK(cudaMemsetAsync(rb.nbr + k_end * n, 0xFF, sizeof(int) * (size_t)((K - k_end) * n), stream));
+    if (K <= kOrderMaxOffsets) SCN_TRY(device_alloc((void **)&rb.masks, sizeof(unsigned) * words * (size_t)n, stream));
+    const long long n_back = mirrored ? (K - k_end) * n : 0;
+    SCN_LAUNCH(k_rules_init, (unsigned)std::min<long long>(148 * 8, ceil_div(std::max(n_back / 4, n * words), 256)), 256, 0, stream, rb.counts_dev, (int)K + 1, rb.masks, rb.masks ? n * words : 0, rb.nbr + k_end * n, n_back);
     // enough blocks to fill the machine even for few sites: split the offsets over grid.y
     long long want_y = std::max<long long>(1, std::min<long long>(k_end, ceil_div(148 * 16, bx)));
     int k_chunk = (int)ceil_div(k_end, want_y);
     int gy = (int)ceil_div(k_end, k_chunk);
     size_t smem = (size_t)k_chunk * (sizeof(long long) + sizeof(int) + md->dim);
-    SCN_LAUNCH(k_submanifold_rules, dim3((unsigned)bx, (unsigned)gy), threads, smem, stream, g->layout, g->table, g->row_keys, n, (int)K, F, k_chunk, rb.nbr, rb.counts_dev, mirrored ? 1 : 0, rb.masks, words);
+    SCN_LAUNCH(k_submanifold_rules, dim3((unsigned)bx, (unsigned)gy), threads, smem, stream, g->layout, g->table, g->row_keys, n, (int)K, F, k_chunk, rb.nbr, rb.counts_dev, mirrored ? 1 : 0, rb.masks, words, ticket_dev(rb));
     SCN_CUDA_CHECK(cudaGetLastError());
   }
   rb.built = true;
@@ -742,11 +849,11 @@ __global__ void k_strided_insert(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Ha
   slot_of[id] = __shfl_sync(peers, s_out, leader);
 }
 
-__global__ void k_strided_fill(KeyLayout Lin, FilterDesc F, const Slot *__restrict__ slots,
-                               const unsigned long long *__restrict__ in_keys,
-                               const int *__restrict__ slot_of, long long n_in, long long n_out,
-                               const int *__restrict__ n_out_dev, long long capacity,
-                               int *__restrict__ nbr, unsigned long long *counts) {
+__device__ __forceinline__ void strided_fill_one(const KeyLayout &Lin, const FilterDesc &F, const Slot *__restrict__ slots,
+                                                 const unsigned long long *__restrict__ in_keys,
+                                                 const int *__restrict__ slot_of, long long n_in, long long n_out,
+                                                 const int *__restrict__ n_out_dev, long long capacity,
+                                                 int *__restrict__ nbr, unsigned long long *counts) {
   long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= n_in * F.tmax) return;
   int s = slot_of[id];
@@ -769,6 +876,16 @@ __global__ void k_strided_fill(KeyLayout Lin, FilterDesc F, const Slot *__restri
   // one counter update per distinct offset in the warp
   unsigned peers = __match_any_sync(__activemask(), k);
   if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&counts[k], (unsigned long long)__popc(peers));
+}
+
+__global__ void k_strided_fill(KeyLayout Lin, FilterDesc F, const Slot *__restrict__ slots,
+                               const unsigned long long *__restrict__ in_keys,
+                               const int *__restrict__ slot_of, long long n_in, long long n_out,
+                               const int *__restrict__ n_out_dev, long long capacity,
+                               int *__restrict__ nbr, unsigned long long *counts, int K,
+                               volatile unsigned long long *counts_host) {
+  strided_fill_one(Lin, F, slots, in_keys, slot_of, n_in, n_out, n_out_dev, capacity, nbr, counts);
+  post_counts(counts, K, counts_host);
 }
 
 int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int64_t *output_size,
@@ -870,13 +987,15 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
   size_t nbr_bytes = sizeof(int) * (size_t)(K * std::max<long long>(n_out, 1));
   SCN_TRY(device_alloc((void **)&rb.nbr, nbr_bytes, stream));
   SCN_CUDA_CHECK(cudaMemsetAsync(rb.nbr, 0xFF, nbr_bytes, stream));
-  SCN_TRY(device_alloc((void **)&rb.counts_dev, sizeof(unsigned long long) * (size_t)K, stream));
-  SCN_CUDA_CHECK(cudaMemsetAsync(rb.counts_dev, 0, sizeof(unsigned long long) * (size_t)K, stream));
+  SCN_TRY(device_alloc((void **)&rb.counts_dev, sizeof(unsigned long long) * (size_t)(K + 1), stream));
+  SCN_CUDA_CHECK(cudaMemsetAsync(rb.counts_dev, 0, sizeof(unsigned long long) * (size_t)(K + 1), stream));
+  SCN_TRY(count_ticket_new(rb));
+  if (n_ids == 0) count_ticket_zero(rb);
   if (n_ids > 0) {
     unsigned blocks = (unsigned)ceil_div(n_ids, threads);
     const long long n_slots = 2 * (long long)gout.table.n_buckets;
     SCN_LAUNCH(k_number_slots, (unsigned)ceil_div(n_slots, threads), threads, 0, stream, gout.table.slots, n_slots, rank, n_out, md->flags_dev, gout.row_keys);
-    SCN_LAUNCH(k_strided_fill, blocks, threads, 0, stream, gin->layout, F, gout.table.slots, gin->row_keys, slot_of, n_in, n_out, nullptr, n_out, rb.nbr, rb.counts_dev);
+    SCN_LAUNCH(k_strided_fill, blocks, threads, 0, stream, gin->layout, F, gout.table.slots, gin->row_keys, slot_of, n_in, n_out, nullptr, n_out, rb.nbr, rb.counts_dev, (int)K, ticket_dev(rb));
     SCN_CUDA_CHECK(cudaGetLastError());
   }
   device_free(slot_of, stream);
@@ -950,7 +1069,10 @@ static int chain_allocate(std::vector<ChainLevel> &plan, cudaStream_t alloc_stre
     SCN_TRY(device_alloc((void **)&lv.gout.table.slots, slots * sizeof(Slot), alloc_stream));
     SCN_TRY(device_alloc((void **)&lv.gout.row_keys, sizeof(unsigned long long) * cap, alloc_stream));
     SCN_TRY(device_alloc((void **)&lv.rb.nbr, sizeof(int) * (size_t)lv.K * cap, alloc_stream));
-    SCN_TRY(device_alloc((void **)&lv.rb.counts_dev, sizeof(unsigned long long) * (size_t)lv.K, alloc_stream));
+    SCN_TRY(device_alloc((void **)&lv.rb.counts_dev, sizeof(unsigned long long) * (size_t)(lv.K + 1), alloc_stream));
+    lv.rb.n_offsets = (int)lv.K;
+    SCN_TRY(count_ticket_new(lv.rb));
+    if (lv.bound_in == 0) count_ticket_zero(lv.rb);
   }
   return SCN_OK;
 }
@@ -967,7 +1089,7 @@ static int chain_enqueue(scn_metadata *md, const Grid *gin, std::vector<ChainLev
     // key = all ones (free), row = -1, aux = 0xFFFFFFFF
     SCN_CUDA_CHECK(cudaMemsetAsync(lv.gout.table.slots, 0xFF, 2 * lv.gout.table.n_buckets * sizeof(Slot), stream));
     SCN_CUDA_CHECK(cudaMemsetAsync(lv.rb.nbr, 0xFF, sizeof(int) * (size_t)lv.K * cap, stream));
-    SCN_CUDA_CHECK(cudaMemsetAsync(lv.rb.counts_dev, 0, sizeof(unsigned long long) * (size_t)lv.K, stream));
+    SCN_CUDA_CHECK(cudaMemsetAsync(lv.rb.counts_dev, 0, sizeof(unsigned long long) * (size_t)(lv.K + 1), stream));
     if (lv.bound_in > 0) {
       const long long n_ids = lv.bound_in * lv.F.tmax;  // (site, output it may feed) candidates
       const unsigned blocks = (unsigned)ceil_div(n_ids, threads);
@@ -977,7 +1099,7 @@ static int chain_enqueue(scn_metadata *md, const Grid *gin, std::vector<ChainLev
       SCN_TRY(exclusive_scan_i32(lv.flag, lv.rank, n_ids, n_out_dev, stream, lv.scan));
       const long long n_slots = 2 * (long long)lv.gout.table.n_buckets;
       SCN_LAUNCH(k_number_slots, (unsigned)ceil_div(n_slots, threads), threads, 0, stream, lv.gout.table.slots, n_slots, lv.rank, lv.cap_out, level_flags, lv.gout.row_keys);
-      SCN_LAUNCH(k_strided_fill, blocks, threads, 0, stream, Lin, lv.F, lv.gout.table.slots, in_keys, lv.slot_of, lv.bound_in, 0ll, n_out_dev, lv.cap_out, lv.rb.nbr, lv.rb.counts_dev);
+      SCN_LAUNCH(k_strided_fill, blocks, threads, 0, stream, Lin, lv.F, lv.gout.table.slots, in_keys, lv.slot_of, lv.bound_in, 0ll, n_out_dev, lv.cap_out, lv.rb.nbr, lv.rb.counts_dev, (int)lv.K, ticket_dev(lv.rb));
       SCN_CUDA_CHECK(cudaGetLastError());
     }
     in_keys = lv.gout.row_keys;
@@ -1284,101 +1406,36 @@ int start_strided_chain(scn_metadata *md, const int64_t *input_size, const int64
 // rulebook views
 // ------------------------------------------------------------------------------------------
 
-// ---- rule counts: pinned chunks and events are pooled per device, never given back to the driver
-namespace {
-struct TicketPool {
-  std::mutex mu;
-  std::vector<unsigned long long *> chunks[64];  // kRMaxCounts values each
-  std::vector<cudaEvent_t> events[64];
-};
-constexpr int kTicketValues = 256;  // filter volumes up to 256 offsets
-TicketPool &ticket_pool() {
-  static TicketPool *p = new TicketPool();  // leaked on purpose: tickets may be released at exit
-  return *p;
-}
-}  // namespace
-
-__global__ void k_post_counts(const unsigned long long *__restrict__ counts, volatile unsigned long long *host, int n) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) host[i] = counts[i];
-  __threadfence_system();
+static bool counts_landed(const CountTicket *t) {
+  for (int k = 0; k < t->n; ++k)
+    if (t->host[k] == kCountPending) return false;
+  return true;
 }
 
-static int count_ticket_start(Rulebook &rb, cudaStream_t stream) {
-  if (rb.ticket) return SCN_OK;
-  SCN_REQUIRE(rb.n_offsets <= kTicketValues, SCN_ERR_UNSUPPORTED, "%d filter offsets", rb.n_offsets);
-  int dev = 0;
-  SCN_CUDA_CHECK(cudaGetDevice(&dev));
-  SCN_REQUIRE(dev < 64, SCN_ERR_UNSUPPORTED, "device %d", dev);
-  CountTicket *t = new CountTicket();
-  t->n = rb.n_offsets;
-  t->device = dev;
-  {
-    TicketPool &P = ticket_pool();
-    std::lock_guard<std::mutex> lock(P.mu);
-    if (!P.chunks[dev].empty()) {
-      t->host = P.chunks[dev].back();
-      P.chunks[dev].pop_back();
-    }
-    if (!P.events[dev].empty()) {
-      t->event = P.events[dev].back();
-      P.events[dev].pop_back();
-    }
-  }
-  if (!t->host) {  // a slab of 256 chunks (512 KB of pinned memory) at a time
-    unsigned long long *slab = nullptr;
-    if (cudaHostAlloc((void **)&slab, sizeof(unsigned long long) * kTicketValues * 256,
-                      cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
-      cudaGetLastError();
-      delete t;
-      SCN_REQUIRE(false, SCN_ERR_CUDA, "pinned allocation failed");
-    }
-    t->host = slab;
-    TicketPool &P = ticket_pool();
-    std::lock_guard<std::mutex> lock(P.mu);
-    for (int i = 1; i < 256; ++i) P.chunks[dev].push_back(slab + (size_t)i * kTicketValues);
-  }
-  if (!t->event && cudaEventCreateWithFlags(&t->event, cudaEventDisableTiming) != cudaSuccess) {
-    cudaGetLastError();
-    t->event = nullptr;
-    count_ticket_release(t);
-    SCN_REQUIRE(false, SCN_ERR_CUDA, "event creation failed");
-  }
-  // posted by a kernel into mapped host memory, not copied: a copy on this stream would hold the stream's next
-  // kernels until the copy engine has finished whatever the application is copying (see the mailboxes above)
-  unsigned long long *host_dev = nullptr;
-  cudaError_t e = cudaHostGetDevicePointer((void **)&host_dev, t->host, 0);
-  if (e == cudaSuccess) {
-    SCN_LAUNCH(k_post_counts, 1, 256, 0, stream, rb.counts_dev, host_dev, rb.n_offsets);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = cudaEventRecord(t->event, stream);
-  if (e != cudaSuccess) {
-    // the rulebook gets the ticket only once its event has been recorded: a later wait on a
-    // never-recorded event would return at once and sum whatever the chunk held
-    cudaEventDestroy(t->event);  // possibly half-recorded: not returned to the pool
-    t->event = nullptr;
-    count_ticket_release(t);
-    SCN_CUDA_CHECK(e);
-  }
-  rb.ticket = t;
+// Waits until the device has written a ticket's counts: a short look, then for the whole device (the kernel that writes
+// them was enqueued before the ticket was handed out, on a stream that may be gone by now).
+static int counts_wait(CountTicket *t) {
+  if (counts_landed(t)) return SCN_OK;  // an answer that already landed is no wait
+  note_host_wait();
+  int current = -1;
+  SCN_CUDA_CHECK(cudaGetDevice(&current));
+  if (current != t->device) SCN_CUDA_CHECK(cudaSetDevice(t->device));
+  const cudaError_t e = cudaDeviceSynchronize();
+  if (current != t->device) cudaSetDevice(current);
+  SCN_CUDA_CHECK(e);
+  SCN_REQUIRE(counts_landed(t), SCN_ERR_CUDA, "rule counts were not written");
   return SCN_OK;
 }
 
 void count_ticket_release(CountTicket *t) {
   if (!t || t->refs.fetch_sub(1) != 1) return;
-  if (t->event) cudaEventSynchronize(t->event);  // the copy must not land in a chunk that was handed on
   TicketPool &P = ticket_pool();
-  {
-    std::lock_guard<std::mutex> lock(P.mu);
-    if (t->host) P.chunks[t->device].push_back(t->host);
-    if (t->event) P.events[t->device].push_back(t->event);
-  }
-  delete t;
+  std::lock_guard<std::mutex> lock(P.mu);
+  P.dropped[t->device].push_back(t);  // its chunk is handed on once the device has written to it
 }
 
 int count_ticket_total(CountTicket *t, long long *total) {
-  if (cudaEventQuery(t->event) != cudaSuccess) note_host_wait();  // an answer that already landed is no wait
-  SCN_CUDA_CHECK(cudaEventSynchronize(t->event));
+  SCN_TRY(counts_wait(t));
   long long s = 0;
   for (int k = 0; k < t->n; ++k) s += (long long)t->host[k];
   *total = s;
@@ -1386,7 +1443,8 @@ int count_ticket_total(CountTicket *t, long long *total) {
 }
 
 static void counts_from_ticket(Rulebook &rb) {
-  rb.counts_host.assign(rb.ticket->host, rb.ticket->host + rb.n_offsets);
+  rb.counts_host.assign(rb.n_offsets, 0);
+  for (int k = 0; k < rb.n_offsets; ++k) rb.counts_host[k] = (long long)rb.ticket->host[k];
   long long t = 0;
   for (auto c : rb.counts_host) t += c;
   rb.total_rules = t;
@@ -1408,23 +1466,15 @@ static int rulebook_counts_blocking(Rulebook &rb, cudaStream_t stream) {
 
 int rulebook_counts_async(Rulebook &rb, cudaStream_t stream) {
   if (rb.total_rules >= 0) return SCN_OK;
-  if (rb.n_offsets > kTicketValues) return rulebook_counts_blocking(rb, stream);
-  SCN_TRY(count_ticket_start(rb, stream));
-  cudaError_t q = cudaEventQuery(rb.ticket->event);
-  if (q == cudaSuccess) {
-    counts_from_ticket(rb);
-  } else if (q != cudaErrorNotReady) {
-    SCN_CUDA_CHECK(q);
-  }
+  if (!rb.ticket) return rulebook_counts_blocking(rb, stream);
+  if (counts_landed(rb.ticket)) counts_from_ticket(rb);
   return SCN_OK;
 }
 
 int rulebook_counts(Rulebook &rb, cudaStream_t stream) {
   if (rb.total_rules >= 0) return SCN_OK;
-  if (rb.n_offsets > kTicketValues) return rulebook_counts_blocking(rb, stream);
-  SCN_TRY(count_ticket_start(rb, stream));
-  note_host_wait();
-  SCN_CUDA_CHECK(cudaEventSynchronize(rb.ticket->event));
+  if (!rb.ticket) return rulebook_counts_blocking(rb, stream);
+  SCN_TRY(counts_wait(rb.ticket));
   counts_from_ticket(rb);
   return SCN_OK;
 }

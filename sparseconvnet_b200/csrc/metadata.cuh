@@ -29,19 +29,20 @@ struct Grid {
 //     tnbr[k * n_in + i] = output row fed by input row i through offset k, or -1
 // used by Deconvolution (the reference swaps the two rule columns, CPU/Deconvolution.cpp:35-37);
 // it is valid because every (offset, input row) also has at most one rule.
-// A rulebook's per-offset rule counts on their way to the host: an asynchronous copy into pinned
-// memory and the event recorded behind it.  The multiply-add count the reference's operators
-// return needs these totals (CPU/Convolution.cpp:141), and waiting for them where the operator is
-// called would leave the GPU idle once per rulebook; a caller that can take the number later is
-// handed the ticket instead.  Reference counted: the ticket outlives its rulebook and metadata.
+// A rulebook's per-offset rule counts on their way to the host: the last block of the kernel that builds the rulebook
+// writes them into pinned, device-mapped memory.  The multiply-add count the reference's operators return needs these
+// totals (CPU/Convolution.cpp:141), and waiting for them where the operator is called would leave the GPU idle once
+// per rulebook; a caller that can take the number later is handed the ticket instead.  Reference counted: the ticket
+// outlives its rulebook and metadata.
 struct CountTicket {
-  unsigned long long *host = nullptr;  // [n] pinned
-  cudaEvent_t event = nullptr;
+  volatile unsigned long long *host = nullptr;  // [n] pinned; kCountPending until the device has written the value
+  unsigned long long *dev = nullptr;            // the same memory as the device sees it
   int n = 0, device = 0;
   std::atomic<int> refs{1};
 };
+constexpr unsigned long long kCountPending = ~0ull;
 void count_ticket_release(CountTicket *t);
-int count_ticket_total(CountTicket *t, long long *total);  // waits for the event only
+int count_ticket_total(CountTicket *t, long long *total);  // waits for the values
 
 // The packing of a table's output rows into tensor-core tiles (row_order.cu): order[p] = output row at position
 // p, -1 past the end (padded to whole tiles); tile_bits[t][words] = filter offsets for which any of the 128 rows
@@ -67,17 +68,16 @@ struct Rulebook {
   // offsets with a rule of every output row of nbr, mask_words(K) words each (submanifold rulebooks up to
   // kOrderMaxOffsets offsets; null otherwise)
   unsigned *masks = nullptr;
-  unsigned long long *counts_dev = nullptr;  // [K] rules per offset
+  unsigned long long *counts_dev = nullptr;  // [K] rules per offset, then the builder's count of finished blocks
   std::vector<long long> counts_host;        // filled on first request (waits for the stream)
   long long total_rules = -1;
-  CountTicket *ticket = nullptr;             // counts in flight (rulebook_counts_async)
+  CountTicket *ticket = nullptr;             // counts in flight (null above kTicketValues offsets)
   bool built = false;
   bool symmetric = false;  // submanifold with odd filter sizes: tnbr[k] is nbr[K - 1 - k]
 };
 
 int rulebook_counts(Rulebook &rb, cudaStream_t stream);         // fills counts_host/total_rules (waits)
-// Starts the copy of the counts if it has not been started; fills counts_host/total_rules without
-// waiting if the copy has already landed.  total_rules stays -1 while the copy is in flight.
+// Fills counts_host/total_rules without waiting if the counts have landed; total_rules stays -1 while they are in flight.
 int rulebook_counts_async(Rulebook &rb, cudaStream_t stream);
 int rulebook_transposed(Rulebook &rb, cudaStream_t stream);     // builds tnbr if missing
 // builds the packing order of the table [K][n] (nbr or tnbr of `rb`) if missing
