@@ -16,6 +16,9 @@ import torch
 
 from . import _lib
 from ._lib import check, lib, sizes
+from . import _binding  # the operator calls as native functions (csrc/binding.cpp); fails loudly if it is missing
+
+_binding.set_check(check)
 
 class DeferredCount(object):
     """Multiply-add count of a convolution whose rule totals were still on their way to the host
@@ -117,6 +120,11 @@ class _FlopCounter(object):
 
 flop_counter = _FlopCounter()
 check(lib.scn_set_deferred_counts(1))
+
+
+def _macs(m):
+    """What a native convolution call returned as its multiply-add count: a float, or (ticket, factor)."""
+    return DeferredCount(*m) if type(m) is tuple else m
 
 
 def _macs_result(m, macs):
@@ -317,6 +325,7 @@ class _Metadata(object):
     def __init__(self):
         self._h = C.c_void_p()
         check(lib.scn_md_create(self.dimension, C.byref(self._h)))
+        self.handle = self._h.value    # for the native calls
         self.device = None
         self.chain_looked_for = False  # containers.Sequential: has a container looked for an encoder to prefetch?
         self.chain_started = False     # ... and started one (SCN.strided_chain_start)
@@ -339,9 +348,7 @@ class _Metadata(object):
             check(lib.scn_md_poll_errors(self._h, _stream()))
 
     def getNActive(self, spatial_size):
-        n = C.c_int64()
-        check(lib.scn_md_n_active(self._h, sizes(spatial_size), C.byref(n)))
-        return n.value
+        return _binding.active_sites(self.handle, spatial_size)
 
     def getBatchSize(self, spatial_size):
         n = C.c_int64()
@@ -532,26 +539,18 @@ def batchnorm_fold(running_mean, running_var, weight, bias, eps):
 
 
 def SubmanifoldConvolution_updateOutput(inputSize, filterSize, m, input_features, output_features,
-                                        weight, bias, epilogue=None):
-    """sparseconvnet.h:101-104.  `epilogue` (not in the reference): see batchnorm_fold."""
+                                        weight, bias, epilogue=None, token=0):
+    """sparseconvnet.h:101-104.  `epilogue` (not in the reference): see batchnorm_fold.  `token`: see weight_token."""
+    if Profile.active is None:  # the convolution entry finds or builds the rulebook itself
+        return _macs(_binding.submanifold_convolution(m.handle, inputSize, filterSize, input_features, output_features,
+                                                      weight, bias, epilogue, _precision, token))
     f, w, b, groups, cin, cout = _conv_args(input_features, weight, bias)
     macs = C.c_double()
-    with _on_device(f.device):
+    with _on_device(f.device), weight_token(token):
         n = m.getNActive(inputSize)
         if f.size(0) != n:
             raise RuntimeError("features have %d rows, metadata has %d active sites" % (f.size(0), n))
         output_features.resize_(n, groups * cout)
-        if Profile.active is None:  # the convolution entry finds or builds the rulebook itself
-            if epilogue is None:
-                check(lib.scn_submanifold_convolution_forward(
-                    m._h, sizes(inputSize), sizes(filterSize), _ptr(f), _ptr(output_features), _ptr(w), _ptr(b),
-                    groups * cin, groups * cout, groups, _precision, _stream(), C.byref(macs)))
-            else:
-                sc, sh, leak = _epilogue_args(epilogue, f, groups * cout)
-                check(lib.scn_submanifold_convolution_bn_forward(
-                    m._h, sizes(inputSize), sizes(filterSize), _ptr(f), _ptr(output_features), _ptr(w), _ptr(b),
-                    sc, sh, leak, groups * cin, groups * cout, groups, _precision, _stream(), C.byref(macs)))
-            return _macs_result(m, macs)
         # profiled: the rulebook call on its own, so that its time and bytes are not the convolution's
         with _timed("rules_submanifold", dict(sites=n, offsets=w.size(0), dim=m.dimension)) as info:
             builds = lib.scn_rulebook_build_count()
@@ -604,13 +603,16 @@ def strided_chain(m, inputSize, filterSize, filterStride, levels, device):
 
 
 def SubmanifoldConvolution_joined(inputSize, filterSize, m, inputs, output_features, weight, bias, prologue=None,
-                                  epilogue=None):
+                                  epilogue=None, token=0):
     """SubmanifoldConvolution of the column-wise concatenation of two feature matrices over the same sites (a
     JoinTable in front of the layer), optionally through an eval-mode BatchNorm in between (`prologue`) and with the
     one behind in its store (`epilogue`): scn_submanifold_convolution_joined_forward.  Not in the reference.
     Returns None when the shapes are not ones the call takes (the caller then joins first)."""
     if len(inputs) != 2 or weight.size(1) != 1:
         return None
+    if Profile.active is None:
+        return _macs(_binding.submanifold_joined(m.handle, inputSize, filterSize, inputs[0], inputs[1], output_features,
+                                                 weight, bias, prologue, epilogue, _precision, token))
     fa, fb = (_features(f, "input_features") for f in inputs)
     ca, cb = fa.size(1), fb.size(1)
     if fa.size(0) != fb.size(0) or ca % 8 or cb % 4 or fa.device != fb.device or weight.size(2) != ca + cb:
@@ -619,7 +621,7 @@ def SubmanifoldConvolution_joined(inputSize, filterSize, m, inputs, output_featu
     b = _optional(bias, fa, "bias")
     n, cout = fa.size(0), w.size(3)
     macs = C.c_double()
-    with _on_device(fa.device):
+    with _on_device(fa.device), weight_token(token):
         if n != m.getNActive(inputSize):
             raise RuntimeError("features have %d rows, metadata has %d active sites" % (n, m.getNActive(inputSize)))
         output_features.resize_(n, cout)
@@ -651,13 +653,16 @@ def strided_chain_start(m, inputSize, filterSize, filterStride, levels, device):
 
 
 def Convolution_updateOutput(inputSize, outputSize, filterSize, filterStride, m, input_features,
-                             output_features, weight, bias, epilogue=None, prologue=None):
+                             output_features, weight, bias, epilogue=None, prologue=None, token=0):
     """sparseconvnet.h:87-92.  `epilogue` (not in the reference): see batchnorm_fold.  `prologue` (not in the
     reference): the same triple for an eval-mode BatchNorm in FRONT of the layer (scn_convolution_bn_bn_forward)."""
+    if Profile.active is None:
+        return _macs(_binding.convolution(m.handle, inputSize, outputSize, filterSize, filterStride, input_features,
+                                          output_features, weight, bias, epilogue, prologue, _precision, token))
     f, w, b, groups, cin, cout = _conv_args(input_features, weight, bias)
     macs = C.c_double()
     n_out = C.c_int64()
-    with _on_device(f.device):
+    with _on_device(f.device), weight_token(token):
         if f.size(0) != m.getNActive(inputSize):
             raise RuntimeError("features have %d rows, metadata has %d active sites"
                                % (f.size(0), m.getNActive(inputSize)))
@@ -699,11 +704,14 @@ def Convolution_updateOutput(inputSize, outputSize, filterSize, filterStride, m,
 
 
 def Deconvolution_updateOutput(inputSize, outputSize, filterSize, filterStride, m, input_features,
-                               output_features, weight, bias, epilogue=None):
+                               output_features, weight, bias, epilogue=None, token=0):
     """sparseconvnet.h:149-154.  `epilogue` (not in the reference): see batchnorm_fold."""
+    if Profile.active is None:
+        return _macs(_binding.deconvolution(m.handle, inputSize, outputSize, filterSize, filterStride, input_features,
+                                            output_features, weight, bias, epilogue, _precision, token))
     f, w, b, groups, cin, cout = _conv_args(input_features, weight, bias)
     macs = C.c_double()
-    with _on_device(f.device):
+    with _on_device(f.device), weight_token(token):
         # same rulebook as the Convolution that made `inputSize` out of `outputSize`
         check(lib.scn_md_strided_rulebook(m._h, sizes(outputSize), sizes(inputSize), sizes(filterSize),
                                           sizes(filterStride), _stream(), None, None))
@@ -737,6 +745,9 @@ def BatchNormalization_updateOutput(input_features, output_features, saveMean, s
                                     runningVar, weight, bias, eps, momentum, train, leakiness):
     """sparseconvnet.h:22-26.  Accepts a column slice of a wider matrix (row stride > planes),
     as the reference does (CPU/BatchNormalization.cpp:9-10)."""
+    if Profile.active is None:
+        return _binding.batchnorm_forward(input_features, output_features, saveMean, saveInvStd, runningMean, runningVar,
+                                          weight, bias, eps, momentum, train, leakiness)
     f = input_features
     if not f.is_cuda or f.dtype != torch.float32 or f.dim() != 2 or (f.numel() and f.stride(1) != 1):
         raise RuntimeError("input_features must be a CUDA float32 matrix with unit column stride")
@@ -781,105 +792,52 @@ def batchnorm_concat(inputs, running_mean, running_var, weight, bias, eps, leaki
     return out
 
 
-def _conv_backward_args(input_features, d_input_features, d_output_features, weight, d_weight, d_bias):
-    f, w, _, groups, cin, cout = _conv_args(input_features, weight, torch.empty(0))
-    go = _features(d_output_features, "d_output_features")
-    dw = _features(d_weight, "d_weight")
-    if dw.shape != w.shape:
-        raise RuntimeError("d_weight must have the shape of weight")
-    db = _features(d_bias, "d_bias") if d_bias is not None and d_bias.numel() else None
-    d_input_features.resize_(f.size(0), groups * cin)
-    return f, w, go, dw, db, groups, cin, cout
-
-
 def SubmanifoldConvolution_backward(inputSize, filterSize, m, input_features, d_input_features,
                                     d_output_features, weight, d_weight, d_bias):
     """sparseconvnet.h:106-114.  fp32; gradients are overwritten."""
-    f, w, go, dw, db, groups, cin, cout = _conv_backward_args(input_features, d_input_features,
-                                                             d_output_features, weight, d_weight, d_bias)
-    with _on_device(f.device):
-        check(lib.scn_submanifold_convolution_backward(
-            m._h, sizes(inputSize), sizes(filterSize), _ptr(f), _ptr(d_input_features), _ptr(go), _ptr(w),
-            _ptr(dw), _ptr(db), groups * cin, groups * cout, groups, _stream()))
+    _binding.convolution_backward(0, m.handle, inputSize, None, filterSize, None, input_features, d_input_features,
+                                  d_output_features, weight, d_weight, d_bias)
 
 
 def Convolution_backward(inputSize, outputSize, filterSize, filterStride, m, input_features, d_input_features,
                          d_output_features, weight, d_weight, d_bias):
     """sparseconvnet.h:94-104."""
-    f, w, go, dw, db, groups, cin, cout = _conv_backward_args(input_features, d_input_features,
-                                                             d_output_features, weight, d_weight, d_bias)
-    with _on_device(f.device):
-        check(lib.scn_convolution_backward(
-            m._h, sizes(inputSize), sizes(outputSize), sizes(filterSize), sizes(filterStride), _ptr(f),
-            _ptr(d_input_features), _ptr(go), _ptr(w), _ptr(dw), _ptr(db), groups * cin, groups * cout, groups,
-            _stream()))
+    _binding.convolution_backward(1, m.handle, inputSize, outputSize, filterSize, filterStride, input_features,
+                                  d_input_features, d_output_features, weight, d_weight, d_bias)
 
 
 def Deconvolution_backward(inputSize, outputSize, filterSize, filterStride, m, input_features, d_input_features,
                            d_output_features, weight, d_weight, d_bias):
     """sparseconvnet.h:156-166."""
-    f, w, go, dw, db, groups, cin, cout = _conv_backward_args(input_features, d_input_features,
-                                                             d_output_features, weight, d_weight, d_bias)
-    with _on_device(f.device):
-        check(lib.scn_deconvolution_backward(
-            m._h, sizes(inputSize), sizes(outputSize), sizes(filterSize), sizes(filterStride), _ptr(f),
-            _ptr(d_input_features), _ptr(go), _ptr(w), _ptr(dw), _ptr(db), groups * cin, groups * cout, groups,
-            _stream()))
+    _binding.convolution_backward(2, m.handle, inputSize, outputSize, filterSize, filterStride, input_features,
+                                  d_input_features, d_output_features, weight, d_weight, d_bias)
 
 
 def MaxPooling_updateOutput(inputSize, outputSize, poolSize, poolStride, m, input_features,
                             output_features, nFeaturesToDrop):
     """sparseconvnet.h:198-201."""
-    f = _features(input_features, "input_features")
-    n_out = C.c_int64()
-    with _on_device(f.device):
-        check(lib.scn_md_strided_rulebook(m._h, sizes(inputSize), sizes(outputSize), sizes(poolSize),
-                                          sizes(poolStride), _stream(), C.byref(n_out), None))
-        output_features.resize_(n_out.value, f.size(1) - int(nFeaturesToDrop))
-        check(lib.scn_max_pooling_forward(
-            m._h, sizes(inputSize), sizes(outputSize), sizes(poolSize), sizes(poolStride), _ptr(f),
-            _ptr(output_features), f.size(1), int(nFeaturesToDrop), _stream()))
+    _binding.pooling_forward(0, m.handle, inputSize, outputSize, poolSize, poolStride, input_features, output_features,
+                             nFeaturesToDrop)
 
 
 def AveragePooling_updateOutput(inputSize, outputSize, poolSize, poolStride, m, input_features,
                                 output_features, nFeaturesToDrop):
     """sparseconvnet.h (AveragePooling_updateOutput), CPU/AveragePooling.cpp:38-61."""
-    f = _features(input_features, "input_features")
-    n_out = C.c_int64()
-    with _on_device(f.device):
-        check(lib.scn_md_strided_rulebook(m._h, sizes(inputSize), sizes(outputSize), sizes(poolSize),
-                                          sizes(poolStride), _stream(), C.byref(n_out), None))
-        output_features.resize_(n_out.value, f.size(1) - int(nFeaturesToDrop))
-        check(lib.scn_average_pooling_forward(
-            m._h, sizes(inputSize), sizes(outputSize), sizes(poolSize), sizes(poolStride), _ptr(f),
-            _ptr(output_features), f.size(1), int(nFeaturesToDrop), _stream()))
+    _binding.pooling_forward(1, m.handle, inputSize, outputSize, poolSize, poolStride, input_features, output_features,
+                             nFeaturesToDrop)
 
 
 def UnPooling_updateOutput(inputSize, outputSize, poolSize, poolStride, m, input_features, output_features,
                            nFeaturesToDrop):
     """sparseconvnet.h (UnPooling_updateOutput), CPU/UnPooling.cpp:35-59: inputSize is the coarse scale,
     outputSize the fine one (its grid must exist already)."""
-    f = _features(input_features, "input_features")
-    with _on_device(f.device):
-        output_features.resize_(m.getNActive(outputSize), f.size(1) - int(nFeaturesToDrop))
-        check(lib.scn_unpooling_forward(
-            m._h, sizes(inputSize), sizes(outputSize), sizes(poolSize), sizes(poolStride), _ptr(f),
-            _ptr(output_features), f.size(1), int(nFeaturesToDrop), _stream()))
+    _binding.pooling_forward(2, m.handle, inputSize, outputSize, poolSize, poolStride, input_features, output_features,
+                             nFeaturesToDrop)
 
 
 def SparseToDense_updateOutput(inputSize, m, input_features, output_features, nPlanes):
     """sparseconvnet.h:220-222.  Output [batch, nPlanes, *inputSize]."""
-    f = _features(input_features, "input_features")
-    with _on_device(f.device):
-        shape = [m.getBatchSize(inputSize), int(nPlanes)] + [int(v) for v in inputSize]
-        output_features.resize_(*shape)
-        if f.dim() == 2:
-            if f.size(1) != nPlanes:
-                raise RuntimeError("features have %d planes, nPlanes is %d" % (f.size(1), nPlanes))
-            check(lib.scn_sparse_to_dense_forward(m._h, sizes(inputSize), _ptr(f), _ptr(output_features),
-                                                  int(nPlanes), _stream()))
-        else:
-            output_features.zero_()
+    _binding.sparse_to_dense(m.handle, inputSize, input_features, output_features, nPlanes)
 
 
 def rows_affine_supported(features, weight):
@@ -935,15 +893,8 @@ def NetworkInNetwork_updateOutput(input_features, output_features, weight, bias)
 def BatchNormalization_backward(input_features, d_input_features, output_features, d_output_features, saveMean,
                                 saveInvStd, runningMean, runningVar, weight, bias, d_weight, d_bias, leakiness):
     """sparseconvnet.h:28-38.  d_output_features is left untouched (the reference scales it in place)."""
-    f = input_features
-    n, c = f.size(0), f.size(1)
-    d_input_features.resize_(n, c)
-    w = _optional(weight, f, "weight")
-    with _on_device(f.device):
-        check(lib.scn_batchnorm_backward(
-            _ptr(f), _ptr(d_input_features), _ptr(output_features), _ptr(d_output_features), n, c,
-            f.stride(0) if n else c, output_features.stride(0) if n else c, _ptr(saveMean), _ptr(saveInvStd),
-            _ptr(w), _ptr(d_weight), _ptr(d_bias), float(leakiness), _stream()))
+    _binding.batchnorm_backward(input_features, d_input_features, output_features, d_output_features, saveMean,
+                                saveInvStd, weight, d_weight, d_bias, leakiness)
 
 
 def _sum_over_ranks(t, group):
@@ -1030,34 +981,22 @@ def OutputLayer_updateGradInput(m, d_input_features, d_output_features):
 def MaxPooling_updateGradInput(inputSize, outputSize, poolSize, poolStride, m, input_features, d_input_features,
                                output_features, d_output_features, nFeaturesToDrop):
     """sparseconvnet.h:203-212."""
-    f = _features(input_features, "input_features")
-    d_input_features.resize_(f.size(0), f.size(1))
-    with _on_device(f.device):
-        check(lib.scn_max_pooling_backward(
-            m._h, sizes(inputSize), sizes(outputSize), sizes(poolSize), sizes(poolStride), _ptr(f),
-            _ptr(d_input_features), _ptr(_features(output_features, "output_features")),
-            _ptr(_features(d_output_features, "d_output_features")), f.size(1), int(nFeaturesToDrop), _stream()))
+    _binding.pooling_backward(0, m.handle, inputSize, outputSize, poolSize, poolStride, input_features, d_input_features,
+                              output_features, d_output_features, input_features.size(1), nFeaturesToDrop)
 
 
 def AveragePooling_updateGradInput(inputSize, outputSize, poolSize, poolStride, m, input_features,
                                    d_input_features, d_output_features, nFeaturesToDrop):
     """sparseconvnet.h:81-92."""
-    f = _features(input_features, "input_features")
-    d_input_features.resize_(f.size(0), f.size(1))
-    with _on_device(f.device):
-        check(lib.scn_average_pooling_backward(
-            m._h, sizes(inputSize), sizes(outputSize), sizes(poolSize), sizes(poolStride), _ptr(d_input_features),
-            _ptr(_features(d_output_features, "d_output_features")), f.size(1), int(nFeaturesToDrop), _stream()))
+    _binding.pooling_backward(1, m.handle, inputSize, outputSize, poolSize, poolStride, input_features, d_input_features,
+                              None, d_output_features, input_features.size(1), nFeaturesToDrop)
 
 
 def UnPooling_updateGradInput(inputSize, outputSize, poolSize, poolStride, m, d_input_features, d_output_features,
                               nFeaturesToDrop):
     """sparseconvnet.h:235-242: d_input_features must already have the input's shape."""
-    go = _features(d_output_features, "d_output_features")
-    with _on_device(go.device):
-        check(lib.scn_unpooling_backward(
-            m._h, sizes(inputSize), sizes(outputSize), sizes(poolSize), sizes(poolStride), _ptr(d_input_features),
-            _ptr(go), d_input_features.size(1), int(nFeaturesToDrop), _stream()))
+    _binding.pooling_backward(2, m.handle, inputSize, outputSize, poolSize, poolStride, None, d_input_features,
+                              None, d_output_features, d_input_features.size(1), nFeaturesToDrop)
 
 
 def SparseToDense_updateGradInput(inputSize, m, input_features, d_input_features, d_output_features):

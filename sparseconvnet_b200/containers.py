@@ -192,7 +192,10 @@ class AddTable(torch.nn.Sequential):
 
     def forward(self, input):
         output = SparseConvNetTensor(metadata=input[0].metadata, spatial_size=input[0].spatial_size)
-        output.features = sum([i.features for i in input])
+        features = input[0].features
+        for i in input[1:]:
+            features = features + i.features
+        output.features = features
         return output
 
     def input_spatial_size(self, out_size):

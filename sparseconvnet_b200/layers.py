@@ -182,7 +182,7 @@ class _ConvBase(Module):
         whenever the weight tensor is written (version counter) or moved (data pointer)."""
         if not _ConvBase.cache_weight_images:
             return 0
-        w = self.weight
+        w = self._parameters["weight"]
         key = (w.data_ptr(), w._version)
         if getattr(self, "_wkey", None) != key:
             old = getattr(self, "_wtoken", 0)
@@ -193,6 +193,13 @@ class _ConvBase(Module):
             self._wkey = key
             self._wfinal = weakref.finalize(self, SCN.release_weight_token, self._wtoken)
         return self._wtoken
+
+    def _run(self, call, output, *args):
+        """A native convolution call that makes its own output tensor (inference; profiled passes and gradients take the
+        functions of SCN.py)."""
+        output.features, macs = call(*args)
+        self._count(SCN._macs(macs), output.features)
+        return output
 
     def _count(self, macs, output_features):
         SCN.flop_counter.add(macs)
@@ -207,20 +214,26 @@ class SubmanifoldConvolution(_ConvBase):
     def forward(self, input, bn=None):
         """`bn` (used by Sequential): an eval-mode BatchNormalization that follows this layer and is
         applied in the convolution's store instead of as a pass of its own."""
-        assert input.features.nelement() == 0 or input.features.size(1) == self.nIn, (self.nIn, self.nOut, input)
+        features, params = input.features, self._parameters
+        weight, bias = params["weight"], params.get("bias")
+        assert features.nelement() == 0 or features.size(1) == self.nIn, (self.nIn, self.nOut, input)
         output = SparseConvNetTensor(metadata=input.metadata, spatial_size=input.spatial_size)
-        bias = optional_tensor(self, "bias")
-        if autograd.needs_grad(input.features, self.weight, bias):
+        if autograd.needs_grad(features, weight, bias):
             assert bn is None
+            bias = optional_tensor(self, "bias")
             output.features, macs = autograd.convolution(
-                autograd.SUBMANIFOLD, input.features, self.weight, bias.to(self.weight.device), input.metadata,
+                autograd.SUBMANIFOLD, features, weight, bias.to(weight.device), input.metadata,
                 input.spatial_size, None, self.filter_size, None)
+        elif SCN.Profile.active is None:
+            return self._run(SCN._binding.submanifold_convolution, output, input.metadata.handle, input.spatial_size,
+                             self.filter_size, features.contiguous(), None, weight, bias,
+                             bn.folded() if bn is not None else None, SCN._precision, self._weight_token())
         else:
-            output.features = input.features.new_empty(0)
-            with SCN.weight_token(self._weight_token()):
-                macs = SCN.SubmanifoldConvolution_updateOutput(
-                    input.spatial_size, self.filter_size, input.metadata, input.features.detach().contiguous(),
-                    output.features, self.weight, bias, epilogue=bn.folded() if bn is not None else None)
+            output.features = features.new_empty(0)
+            macs = SCN.SubmanifoldConvolution_updateOutput(
+                input.spatial_size, self.filter_size, input.metadata, features.detach().contiguous(),
+                output.features, weight, bias, epilogue=bn.folded() if bn is not None else None,
+                token=self._weight_token())
         self._count(macs, output.features)
         return output
 
@@ -230,12 +243,11 @@ class SubmanifoldConvolution(_ConvBase):
         the normalised copy being built as tensors of their own.  None when the shapes do not allow it."""
         output = SparseConvNetTensor(metadata=inputs[0].metadata, spatial_size=inputs[0].spatial_size)
         output.features = inputs[0].features.new_empty(0)
-        with SCN.weight_token(self._weight_token()):
-            macs = SCN.SubmanifoldConvolution_joined(
-                inputs[0].spatial_size, self.filter_size, inputs[0].metadata,
-                [i.features.detach().contiguous() for i in inputs], output.features, self.weight,
-                optional_tensor(self, "bias"), prologue=pre_bn.folded() if pre_bn is not None else None,
-                epilogue=bn.folded() if bn is not None else None)
+        macs = SCN.SubmanifoldConvolution_joined(
+            inputs[0].spatial_size, self.filter_size, inputs[0].metadata,
+            [i.features.detach().contiguous() for i in inputs], output.features, self._parameters["weight"],
+            self._parameters.get("bias"), prologue=pre_bn.folded() if pre_bn is not None else None,
+            epilogue=bn.folded() if bn is not None else None, token=self._weight_token())
         if macs is None:
             return None
         self._count(macs, output.features)
@@ -267,28 +279,33 @@ class Convolution(_ConvBase):
     def forward(self, input, bn=None, pre_bn=None):
         """`bn` / `pre_bn` (used by Sequential): eval-mode BatchNormalizations behind / in front of this layer that
         are applied inside the convolution call instead of as passes of their own."""
-        assert input.features.nelement() == 0 or input.features.size(1) == self.nIn
-        out_size = torch.div(input.spatial_size - self.filter_size, self.filter_stride, rounding_mode="trunc") + 1
-        assert ((out_size - 1) * self.filter_stride + self.filter_size == input.spatial_size).all(), \
-            (input.spatial_size, out_size, self.filter_size, self.filter_stride)
+        features, params = input.features, self._parameters
+        weight, bias = params["weight"], params.get("bias")
+        assert features.nelement() == 0 or features.size(1) == self.nIn
+        out_size = SCN._binding.strided_size(input.spatial_size, self.filter_size, self.filter_stride)
+        assert out_size is not None, (input.spatial_size, self.filter_size, self.filter_stride)
         output = SparseConvNetTensor(metadata=input.metadata, spatial_size=out_size)
-        bias = optional_tensor(self, "bias")
-        if self.levels_below > 1 and input.features.is_cuda:
+        if self.levels_below > 1 and features.is_cuda:
             SCN.strided_chain(input.metadata, input.spatial_size, self.filter_size, self.filter_stride,
-                              self.levels_below, input.features.device)
-        if autograd.needs_grad(input.features, self.weight, bias):
+                              self.levels_below, features.device)
+        if autograd.needs_grad(features, weight, bias):
             assert bn is None and pre_bn is None  # (the fused forms are inference-only; Sequential checks the same)
+            bias = optional_tensor(self, "bias")
             output.features, macs = autograd.convolution(
-                autograd.STRIDED, input.features, self.weight, bias.to(self.weight.device), input.metadata,
+                autograd.STRIDED, features, weight, bias.to(weight.device), input.metadata,
                 input.spatial_size, out_size, self.filter_size, self.filter_stride)
+        elif SCN.Profile.active is None:
+            return self._run(SCN._binding.convolution, output, input.metadata.handle, input.spatial_size, out_size,
+                             self.filter_size, self.filter_stride, features.contiguous(), None, weight, bias,
+                             bn.folded() if bn is not None else None, pre_bn.folded() if pre_bn is not None else None,
+                             SCN._precision, self._weight_token())
         else:
-            output.features = input.features.new_empty(0)
-            with SCN.weight_token(self._weight_token()):
-                macs = SCN.Convolution_updateOutput(
-                    input.spatial_size, out_size, self.filter_size, self.filter_stride, input.metadata,
-                    input.features.detach().contiguous(), output.features, self.weight, bias,
-                    epilogue=bn.folded() if bn is not None else None,
-                    prologue=pre_bn.folded() if pre_bn is not None else None)
+            output.features = features.new_empty(0)
+            macs = SCN.Convolution_updateOutput(
+                input.spatial_size, out_size, self.filter_size, self.filter_stride, input.metadata,
+                features.detach().contiguous(), output.features, weight, bias,
+                epilogue=bn.folded() if bn is not None else None,
+                prologue=pre_bn.folded() if pre_bn is not None else None, token=self._weight_token())
         self._count(macs, output.features)
         return output
 
@@ -307,21 +324,26 @@ class Deconvolution(_ConvBase):
         self.filter_stride = to_long_tensor(dimension, filter_stride)
 
     def forward(self, input, bn=None):
-        assert input.features.nelement() == 0 or input.features.size(1) == self.nIn
-        out_size = (input.spatial_size - 1) * self.filter_stride + self.filter_size
+        features, params = input.features, self._parameters
+        weight, bias = params["weight"], params.get("bias")
+        assert features.nelement() == 0 or features.size(1) == self.nIn
+        out_size = SCN._binding.transposed_size(input.spatial_size, self.filter_size, self.filter_stride)
         output = SparseConvNetTensor(metadata=input.metadata, spatial_size=out_size)
-        bias = optional_tensor(self, "bias")
-        if autograd.needs_grad(input.features, self.weight, bias):
+        if autograd.needs_grad(features, weight, bias):
+            bias = optional_tensor(self, "bias")
             output.features, macs = autograd.convolution(
-                autograd.TRANSPOSED, input.features, self.weight, bias.to(self.weight.device), input.metadata,
+                autograd.TRANSPOSED, features, weight, bias.to(weight.device), input.metadata,
                 input.spatial_size, out_size, self.filter_size, self.filter_stride)
+        elif SCN.Profile.active is None:
+            return self._run(SCN._binding.deconvolution, output, input.metadata.handle, input.spatial_size, out_size,
+                             self.filter_size, self.filter_stride, features.contiguous(), None, weight, bias,
+                             bn.folded() if bn is not None else None, SCN._precision, self._weight_token())
         else:
-            output.features = input.features.new_empty(0)
-            with SCN.weight_token(self._weight_token()):
-                macs = SCN.Deconvolution_updateOutput(
-                    input.spatial_size, out_size, self.filter_size, self.filter_stride, input.metadata,
-                    input.features.detach().contiguous(), output.features, self.weight, bias,
-                    epilogue=bn.folded() if bn is not None else None)
+            output.features = features.new_empty(0)
+            macs = SCN.Deconvolution_updateOutput(
+                input.spatial_size, out_size, self.filter_size, self.filter_stride, input.metadata,
+                features.detach().contiguous(), output.features, weight, bias,
+                epilogue=bn.folded() if bn is not None else None, token=self._weight_token())
         self._count(macs, output.features)
         return output
 
@@ -354,23 +376,24 @@ class BatchNormalization(Module):
     def folded(self):
         """(scale, shift, leakiness) of this layer in eval mode, for a convolution that applies it in its
         store.  Kept until a parameter or running statistic changes (tensor version counters)."""
-        tensors = (self.running_mean, self.running_var, getattr(self, "weight", None), getattr(self, "bias", None))
-        key = tuple((t.data_ptr(), t._version) if t is not None else None for t in tensors) + (self.eps,)
-        cached = getattr(self, "_folded", None)
-        if cached is None or cached[0] != key:
+        buffers, params = self._buffers, self._parameters
+        key = SCN._binding.versions(buffers["running_mean"], buffers["running_var"], params.get("weight"),
+                                    params.get("bias"))
+        cached = self.__dict__.get("_folded")
+        if cached is None or cached[0] != key or cached[1] != self.eps:
             scale, shift = SCN.batchnorm_fold(self.running_mean, self.running_var, optional_tensor(self, "weight"),
                                               optional_tensor(self, "bias"), self.eps)
-            cached = (key, scale, shift)
-            self._folded = cached
-        return cached[1], cached[2], self.leakiness
+            cached = self._folded = (key, self.eps, scale, shift)
+        return cached[2], cached[3], self.leakiness
 
     def fusable(self, features):
         """True when a preceding convolution may apply this layer in its store: eval mode, no gradients
         wanted, statistics on the features' device."""
-        return (not self.training and not autograd.needs_grad(features, optional_tensor(self, "weight"),
-                                                              optional_tensor(self, "bias"))
-                and self.running_mean.is_cuda and self.running_mean.device == features.device
-                and not self._forward_hooks and not self._forward_pre_hooks)
+        if self.training or self._forward_hooks or self._forward_pre_hooks:
+            return False
+        mean, params = self._buffers["running_mean"], self._parameters
+        return (mean.is_cuda and mean.device == features.device
+                and not autograd.needs_grad(features, params.get("weight"), params.get("bias")))
 
     def forward_joined(self, inputs):
         """This layer (eval mode) applied to the concatenation of `inputs` (what a JoinTable in front of
@@ -419,13 +442,13 @@ class BatchNormalization(Module):
                                                  self.running_var, self.eps, self.momentum, self.training,
                                                  self.leakiness)
             return output
-        output.features = input.features.new_empty(0)
-        save_mean = input.features.new_empty(self.nPlanes)
-        save_invstd = input.features.new_empty(self.nPlanes)
+        features = input.features.detach()
+        output.features = features.new_empty(0)
+        save_mean = features.new_empty(self.nPlanes)
+        save_invstd = features.new_empty(self.nPlanes)
         SCN.BatchNormalization_updateOutput(
-            input.features.detach(), output.features, save_mean, save_invstd, self.running_mean,
-            self.running_var, optional_tensor(self, "weight"), optional_tensor(self, "bias"), self.eps,
-            self.momentum, self.training, self.leakiness)
+            features, output.features, save_mean, save_invstd, self.running_mean, self.running_var, weight, bias,
+            self.eps, self.momentum, self.training, self.leakiness)
         return output
 
     def input_spatial_size(self, out_size):
@@ -465,17 +488,16 @@ class MaxPooling(Module):
         self.nFeaturesToDrop = nFeaturesToDrop
 
     def forward(self, input):
-        out_size = torch.div(input.spatial_size - self.pool_size, self.pool_stride, rounding_mode="trunc") + 1
-        assert ((out_size - 1) * self.pool_stride + self.pool_size == input.spatial_size).all()
+        out_size = SCN._binding.strided_size(input.spatial_size, self.pool_size, self.pool_stride)
+        assert out_size is not None, (input.spatial_size, self.pool_size, self.pool_stride)
         output = SparseConvNetTensor(metadata=input.metadata, spatial_size=out_size)
         if autograd.needs_grad(input.features):
             output.features = autograd.pooling("max", input.features, input.metadata, input.spatial_size, out_size,
                                                self.pool_size, self.pool_stride, self.nFeaturesToDrop)
             return output
-        output.features = input.features.new_empty(0)
-        SCN.MaxPooling_updateOutput(input.spatial_size, out_size, self.pool_size, self.pool_stride,
-                                    input.metadata, input.features.detach().contiguous(), output.features,
-                                    self.nFeaturesToDrop)
+        output.features = SCN._binding.pooling_forward(
+            0, input.metadata.handle, input.spatial_size, out_size, self.pool_size, self.pool_stride,
+            input.features.detach().contiguous(), None, self.nFeaturesToDrop)
         return output
 
     def input_spatial_size(self, out_size):
@@ -497,17 +519,16 @@ class AveragePooling(Module):
         self.nFeaturesToDrop = nFeaturesToDrop
 
     def forward(self, input):
-        out_size = torch.div(input.spatial_size - self.pool_size, self.pool_stride, rounding_mode="trunc") + 1
-        assert ((out_size - 1) * self.pool_stride + self.pool_size == input.spatial_size).all()
+        out_size = SCN._binding.strided_size(input.spatial_size, self.pool_size, self.pool_stride)
+        assert out_size is not None, (input.spatial_size, self.pool_size, self.pool_stride)
         output = SparseConvNetTensor(metadata=input.metadata, spatial_size=out_size)
         if autograd.needs_grad(input.features):
             output.features = autograd.pooling("avg", input.features, input.metadata, input.spatial_size, out_size,
                                                self.pool_size, self.pool_stride, self.nFeaturesToDrop)
             return output
-        output.features = input.features.new_empty(0)
-        SCN.AveragePooling_updateOutput(input.spatial_size, out_size, self.pool_size, self.pool_stride,
-                                        input.metadata, input.features.detach().contiguous(), output.features,
-                                        self.nFeaturesToDrop)
+        output.features = SCN._binding.pooling_forward(
+            1, input.metadata.handle, input.spatial_size, out_size, self.pool_size, self.pool_stride,
+            input.features.detach().contiguous(), None, self.nFeaturesToDrop)
         return output
 
     def input_spatial_size(self, out_size):
@@ -529,16 +550,15 @@ class UnPooling(Module):
         self.nFeaturesToDrop = nFeaturesToDrop
 
     def forward(self, input):
-        out_size = (input.spatial_size - 1) * self.pool_stride + self.pool_size
+        out_size = SCN._binding.transposed_size(input.spatial_size, self.pool_size, self.pool_stride)
         output = SparseConvNetTensor(metadata=input.metadata, spatial_size=out_size)
         if autograd.needs_grad(input.features):
             output.features = autograd.pooling("unpool", input.features, input.metadata, input.spatial_size, out_size,
                                                self.pool_size, self.pool_stride, self.nFeaturesToDrop)
             return output
-        output.features = input.features.new_empty(0)
-        SCN.UnPooling_updateOutput(input.spatial_size, out_size, self.pool_size, self.pool_stride,
-                                   input.metadata, input.features.detach().contiguous(), output.features,
-                                   self.nFeaturesToDrop)
+        output.features = SCN._binding.pooling_forward(
+            2, input.metadata.handle, input.spatial_size, out_size, self.pool_size, self.pool_stride,
+            input.features.detach().contiguous(), None, self.nFeaturesToDrop)
         return output
 
     def input_spatial_size(self, out_size):
@@ -559,10 +579,8 @@ class SparseToDense(Module):
     def forward(self, input):
         if autograd.needs_grad(input.features):
             return autograd.sparse_to_dense(input.features, input.metadata, input.spatial_size, self.nPlanes)
-        output = input.features.new_empty(0)
-        SCN.SparseToDense_updateOutput(input.spatial_size, input.metadata,
-                                       input.features.detach().contiguous(), output, self.nPlanes)
-        return output
+        return SCN._binding.sparse_to_dense(input.metadata.handle, input.spatial_size,
+                                            input.features.detach().contiguous(), None, self.nPlanes)
 
     def input_spatial_size(self, out_size):
         return out_size
