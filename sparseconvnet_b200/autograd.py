@@ -41,7 +41,7 @@ class _Convolution(torch.autograd.Function):
         features, weight, bias = ctx.saved_tensors
         kind, metadata, in_size, out_size, filter_size, filter_stride = ctx.args
         grad_out = grad_out.contiguous()
-        d_in = grad_out.new_empty(0)
+        d_in = grad_out.new_empty(0) if ctx.needs_input_grad[0] else None
         d_w = torch.empty_like(weight)
         d_b = torch.empty_like(bias) if bias.numel() else None
         w = weight.detach()

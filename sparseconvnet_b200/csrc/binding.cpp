@@ -362,8 +362,9 @@ SCN_FN(convolution_backward) {
   const int kind = (int)PyLong_AsLong(a[0]);
   scn_metadata *md = md_of(a[1]);
   const Sizes in_size(a[2]), out_size(kind == 0 ? a[2] : a[3]), filter(a[4]), stride(kind == 0 ? a[4] : a[5]);
-  const at::Tensor &f = features(a[6], "input_features"), &df = tensor(a[7], "d_input_features");
-  const at::Tensor &go = features(a[8], "d_output_features");
+  const at::Tensor &f = features(a[6], "input_features"), &go = features(a[8], "d_output_features");
+  const bool want_input = a[7] != Py_None;  // (the gradient of a network's input features is not wanted)
+  float *df = nullptr;
   const Weight w(a[9], f);
   const int nin = w.groups * w.cin, nout = w.groups * w.cout;
   if (f.numel() && f.size(1) != nin) fail("features have %d planes, weight expects %d", (int)f.size(1), nin);
@@ -371,13 +372,17 @@ SCN_FN(convolution_backward) {
   if (dw.sizes() != w.w.sizes()) fail("d_weight must have the shape of weight");
   float *db = a[11] == Py_None || tensor(a[11], "d_bias").numel() == 0 ? nullptr : ptr(features(a[11], "d_bias"));
   const OnDevice on(f);
-  size_to(df, {f.size(0), nin});
+  if (want_input) {
+    const at::Tensor &t = tensor(a[7], "d_input_features");
+    size_to(t, {f.size(0), nin});
+    df = ptr(t);
+  }
   if (kind == 0)
-    SCN_CALL(scn_submanifold_convolution_backward(md, in_size.p, filter.p, ptr(f), ptr(df), ptr(go), ptr(w.w), ptr(dw), db, nin,
+    SCN_CALL(scn_submanifold_convolution_backward(md, in_size.p, filter.p, ptr(f), df, ptr(go), ptr(w.w), ptr(dw), db, nin,
                                                nout, w.groups, on.stream));
   else
     SCN_CALL((kind == 1 ? scn_convolution_backward : scn_deconvolution_backward)(
-        md, in_size.p, out_size.p, filter.p, stride.p, ptr(f), ptr(df), ptr(go), ptr(w.w), ptr(dw), db, nin, nout, w.groups,
+        md, in_size.p, out_size.p, filter.p, stride.p, ptr(f), df, ptr(go), ptr(w.w), ptr(dw), db, nin, nout, w.groups,
         on.stream));
   Py_RETURN_NONE;
   SCN_END

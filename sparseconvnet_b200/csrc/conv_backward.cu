@@ -17,6 +17,7 @@
 #include <atomic>
 
 #include "metadata.cuh"
+#include "tc_ptx.cuh"
 
 namespace scn {
 
@@ -108,14 +109,26 @@ k_conv_dweight(const float *__restrict__ in, int ld_in, long long n_in_rows, con
     }
 }
 
-// The same partial sums on the warp-level tensor path, for groups = 1 and plane counts that are
-// multiples of 32: grid = (chunks, K, c-tiles * n-tiles), four warps.  Each warp takes a contiguous
-// quarter of the chunk's rulebook entries, keeps only the entries that hold a rule (a third of them
-// on surface data: the FMA kernel above multiplies the empty ones as zeros), and accumulates the
-// 32 x 32 tile  in^T [32 x 8 rules] x d_out [8 rules x 32]  per block of eight rules with
-// mma.sync.m16n8k8 on the hi/lo split of both operands (hi x hi + hi x lo + lo x hi, fp32
-// accumulate: fp32-class accuracy).  The four warps' tiles are added in warp order, so the result
-// does not depend on timing.
+// out[i] = sum over chunks, in order, of partial[chunk][i]
+__global__ void k_sum_chunks(const float *__restrict__ partial, int chunks, long long n, float *__restrict__ out) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float acc = 0.f;
+  for (int c = 0; c < chunks; ++c) acc += partial[(long long)c * n + i];
+  out[i] = acc;
+}
+
+// The same partial sums on the warp-level tensor path (groups = 1, any plane counts): a CTA owns one offset, one chunk
+// of its rulebook column and a tile of 32 WM x 32 WN weights.  It keeps only the entries that hold a rule (a third of
+// them on surface data), in a list in shared memory, and walks the list in steps of 32 or 64 rules: the rules' input and
+// output rows travel with cp.async through a ring of stages, then each warp multiplies
+// in^T [32 x 8 rules] x d_out [8 rules x 32] per block of eight rules with mma.sync.m16n8k8 on the hi/lo split of both
+// operands (hi x hi + hi x lo + lo x hi, fp32 accumulate: fp32-class accuracy).  With few 32 x 32 tiles several warps
+// share the blocks of a step and their sums are added in warp order, so the result does not depend on timing.  Plane
+// counts that are no multiple of the tile are padded with zeros in the stage only.
+//
+// Bound by the tensor instructions (three passes of tf32: 92 TFLOP/s).  Reading every fragment value of every rule
+// straight from the matrices, once per 32 x 32 tile, was bound by the loads.
 __device__ __forceinline__ void dw_mma(float (&d)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
   asm volatile(
       "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -126,122 +139,230 @@ __device__ __forceinline__ void dw_split(float x, unsigned &hi, unsigned &lo) {
   hi = __float_as_uint(x) & 0xFFFFE000u;
   lo = __float_as_uint(x - __uint_as_float(hi));
 }
+__device__ __forceinline__ void dw_copy4(unsigned dst, const float *src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4u : 0u) : "memory");
+}
 
-__global__ void __launch_bounds__(128)
+// WM x WN warps side by side, each with 16 MT x 32 weights (MT 1: layers of at most 16 input planes)
+template <int WM, int WN, int MT>
+struct DwShape {
+  static constexpr int M = 16 * MT * WM, N = 32 * WN;
+  static constexpr int SHARE = WM * WN == 1 ? 4 : WM * WN <= 3 ? 2 : 1;  // warps that share a 32 x 32 tile
+  static constexpr int THREADS = 32 * WM * WN * SHARE;
+  static constexpr int STEP = SHARE == 4 ? 64 : 32, STAGES = 3;
+  static constexpr int LOADS = 8, LIST = LOADS * THREADS;  // entries looked at in one go
+  static constexpr int SA = M + 8, SB = N + 8;  // row strides: rules t and planes g of a fragment fall on different banks
+  static constexpr int STAGE = STEP * (SA + SB);
+  static constexpr int TILE = 32 * 33;          // a warp's result, in the stages' memory
+  static constexpr size_t SMEM = sizeof(float) * STAGES * STAGE + sizeof(int2) * LIST;
+  static_assert(STAGES * STAGE >= (THREADS / 32) * TILE, "the warps' results do not fit the stages");
+};
+
+template <int WM, int WN, int MT>
+__global__ void __launch_bounds__(DwShape<WM, WN, MT>::THREADS)
 k_conv_dweight_mma(const float *__restrict__ in, int ld_in, long long n_in_rows, const float *__restrict__ dout,
                    int ld_out, long long n_out_rows, const int *__restrict__ nbr, long long n_entries, int swap,
-                   int cin, int cout, long long chunk_rows, float *__restrict__ partial, int *flags) {
+                   int cin, int cout, int vec_in, int vec_out, long long chunk_rows, float *__restrict__ partial, int *flags) {
+  using S = DwShape<WM, WN, MT>;
   constexpr unsigned kFull = 0xffffffffu;
-  __shared__ int q_in[4][64], q_out[4][64];  // per warp: rules waiting for a block of eight
-  __shared__ float tile[4][32][33];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  constexpr int kWarps = S::THREADS / 32;
+  extern __shared__ __align__(16) unsigned char dw_smem[];
+  float *stages = reinterpret_cast<float *>(dw_smem);
+  int2 *list = reinterpret_cast<int2 *>(stages + S::STAGES * S::STAGE);
+  __shared__ int counts[S::LOADS][kWarps];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int k = blockIdx.y;
-  const int tiles_n = cout / 32;
-  const int c0 = (blockIdx.z / tiles_n) * 32, n0 = (blockIdx.z % tiles_n) * 32;
-  const long long j0 = (long long)blockIdx.x * chunk_rows;
-  const long long j1 = min(n_entries, j0 + chunk_rows);
-  const long long per_warp = ((j1 - j0 + 3) / 4 + 31) / 32 * 32;
-  const long long w0 = min(j1, j0 + warp * per_warp), w1 = min(j1, w0 + per_warp);
+  const int tiles_n = (cout + S::N - 1) / S::N;
+  const int c0 = ((int)blockIdx.z / tiles_n) * S::M, n0 = ((int)blockIdx.z % tiles_n) * S::N;
+  const int mw = warp % WM, nw = (warp / WM) % WN, share = warp / (WM * WN);
+  const long long j0 = (long long)blockIdx.x * chunk_rows, j1 = min(n_entries, j0 + chunk_rows);
   const int *col = nbr + (long long)k * n_entries;
+  // planes of the tile that exist; rows that are copied value by value leave the others the zeros they start as
+  const int cols_in = min(S::M, cin - c0), cols_out = min(S::N, cout - n0);
+  if (!vec_in || !vec_out) {
+    for (int i = tid; i < S::STAGES * S::STAGE; i += S::THREADS) stages[i] = 0.f;
+    __syncthreads();
+  }
 
-  float d[2][4][4];
+  float d[MT][4][4];
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
+  for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) d[mt][nt][0] = d[mt][nt][1] = d[mt][nt][2] = d[mt][nt][3] = 0.f;
 
-  // one block of eight rules starting at queue position `head`; `count` (< 8 only at the end) are real
-  auto block = [&](int head, int count) {
-    const int p0 = (head + t) & 63, p1 = (head + t + 4) & 63;
-    const bool ok0 = t < count, ok1 = t + 4 < count;
-    const long long ri0 = ok0 ? q_in[warp][p0] : 0, ri1 = ok1 ? q_in[warp][p1] : 0;
-    const long long ro0 = ok0 ? q_out[warp][p0] : 0, ro1 = ok1 ? q_out[warp][p1] : 0;
-    const float *a0p = in + ri0 * ld_in + c0 + g, *a1p = in + ri1 * ld_in + c0 + g;
-    const float *b0p = dout + ro0 * ld_out + n0 + g, *b1p = dout + ro1 * ld_out + n0 + g;
-    float av[2][4], bv[4][2];
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {  // A[m = plane][k = rule]: a0 (g, t), a1 (g + 8, t), a2 (g, t + 4), a3 (g + 8, t + 4)
-      av[mt][0] = ok0 ? __ldg(a0p + mt * 16) : 0.f;
-      av[mt][1] = ok0 ? __ldg(a0p + mt * 16 + 8) : 0.f;
-      av[mt][2] = ok1 ? __ldg(a1p + mt * 16) : 0.f;
-      av[mt][3] = ok1 ? __ldg(a1p + mt * 16 + 8) : 0.f;
-    }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {  // B[k = rule][n = plane]: b0 (t, g), b1 (t + 4, g)
-      bv[nt][0] = ok0 ? __ldg(b0p + nt * 8) : 0.f;
-      bv[nt][1] = ok1 ? __ldg(b1p + nt * 8) : 0.f;
-    }
-    unsigned ah[2][4], al[2][4], bh[4][2], bl[4][2];
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) dw_split(av[mt][e], ah[mt][e], al[mt][e]);
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      dw_split(bv[nt][0], bh[nt][0], bl[nt][0]);
-      dw_split(bv[nt][1], bh[nt][1], bl[nt][1]);
-    }
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) dw_mma(d[mt][nt], al[mt], bh[nt]);
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) dw_mma(d[mt][nt], ah[mt], bl[nt]);
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) dw_mma(d[mt][nt], ah[mt], bh[nt]);
-  };
-
-  int head = 0, tail = 0;  // queue positions (not wrapped)
-  for (long long jb = w0; jb < w1; jb += 32) {
-    const long long j = jb + lane;
-    int ri = -1, ro = -1;
-    if (j < w1) {
-      const int a = __ldg(col + j);
-      if (a >= 0) {
-        ri = swap ? (int)j : a;
-        ro = swap ? a : (int)j;
-        if (ri >= n_in_rows || ro >= n_out_rows) {
-          atomicOr(flags, FLAG_BAD_ROW);
-          ri = ro = -1;
+  // the rows of step `s` of a list of `n` rules into stage `s % STAGES`; one cp.async group per call
+  auto issue = [&](int s, int n) {
+    float *a = stages + (s % S::STAGES) * S::STAGE, *b = a + S::STEP * S::SA;
+    if (s * S::STEP < n) {
+      if (vec_in) {
+#pragma unroll 4
+        for (int i = tid; i < S::STEP * (S::M / 4); i += S::THREADS) {
+          const int r = i / (S::M / 4), c = (i % (S::M / 4)) * 4, e = s * S::STEP + r;
+          const bool ok = e < n && c < cols_in;
+          cp_async16(smem_u32(a + r * S::SA + c), ok ? in + (long long)list[e].x * ld_in + c0 + c : in, ok ? 16u : 0u);
+        }
+      } else {
+        for (int i = tid; i < S::STEP * cols_in; i += S::THREADS) {
+          const int r = i / cols_in, c = i - r * cols_in, e = s * S::STEP + r;
+          dw_copy4(smem_u32(a + r * S::SA + c), e < n ? in + (long long)list[e].x * ld_in + c0 + c : in, e < n);
+        }
+      }
+      if (vec_out) {
+#pragma unroll 4
+        for (int i = tid; i < S::STEP * (S::N / 4); i += S::THREADS) {
+          const int r = i / (S::N / 4), c = (i % (S::N / 4)) * 4, e = s * S::STEP + r;
+          const bool ok = e < n && c < cols_out;
+          cp_async16(smem_u32(b + r * S::SB + c), ok ? dout + (long long)list[e].y * ld_out + n0 + c : dout, ok ? 16u : 0u);
+        }
+      } else {
+        for (int i = tid; i < S::STEP * cols_out; i += S::THREADS) {
+          const int r = i / cols_out, c = i - r * cols_out, e = s * S::STEP + r;
+          dw_copy4(smem_u32(b + r * S::SB + c), e < n ? dout + (long long)list[e].y * ld_out + n0 + c : dout, e < n);
         }
       }
     }
-    const unsigned m = __ballot_sync(kFull, ri >= 0);
-    if (ri >= 0) {
-      const int p = (tail + __popc(m & ((1u << lane) - 1u))) & 63;
-      q_in[warp][p] = ri;
-      q_out[warp][p] = ro;
-    }
-    tail += __popc(m);
-    __syncwarp();
-    while (tail - head >= 8) {
-      block(head, 8);
-      head += 8;
-    }
-    __syncwarp();  // the blocks' reads of the queue come before the next group's writes
-  }
-  if (tail > head) block(head, tail - head);
+    cp_async_commit();
+  };
 
-  // ---- the four warps' tiles, added in warp order ------------------------------------------------
+  for (long long jb = j0; jb < j1; jb += S::LIST) {
+    // ---- the rules among the next LIST entries, in entry order -----------------------------------------------------
+    int v[S::LOADS];
+    unsigned m[S::LOADS];
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
+    for (int u = 0; u < S::LOADS; ++u) {
+      const long long j = jb + u * S::THREADS + tid;
+      v[u] = j < j1 ? __ldg(col + j) : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < S::LOADS; ++u) {
+      if (v[u] >= (swap ? n_out_rows : n_in_rows)) {
+        atomicOr(flags, FLAG_BAD_ROW);
+        v[u] = -1;
+      }
+      m[u] = __ballot_sync(kFull, v[u] >= 0);
+      if (lane == 0) counts[u][warp] = __popc(m[u]);
+    }
+    __syncthreads();
+    int n = 0;
+#pragma unroll
+    for (int u = 0; u < S::LOADS; ++u) {
+      int at = n;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        if (w < warp) at += counts[u][w];
+        n += counts[u][w];
+      }
+      const int j = (int)(jb + u * S::THREADS + tid);
+      if (v[u] >= 0) list[at + __popc(m[u] & ((1u << lane) - 1u))] = swap ? make_int2(j, v[u]) : make_int2(v[u], j);
+    }
+    __syncthreads();
+    // ---- the list in steps -------------------------------------------------------------------------------------------
+    const int steps = (n + S::STEP - 1) / S::STEP;
+#pragma unroll
+    for (int s = 0; s < S::STAGES - 1; ++s) issue(s, n);
+    for (int s = 0; s < steps; ++s) {
+      cp_async_wait<S::STAGES - 2>();
+      __syncthreads();  // the step has landed for everybody, and the step before is consumed
+      issue(s + S::STAGES - 1, n);
+      const float *a = stages + (s % S::STAGES) * S::STAGE + mw * 16 * MT, *b = stages + (s % S::STAGES) * S::STAGE + S::STEP * S::SA + nw * 32;
+#pragma unroll
+      for (int kb = 0; kb < S::STEP / 8 / S::SHARE; ++kb) {
+        const int r0 = (kb * S::SHARE + share) * 8 + t;
+        const float *a0 = a + r0 * S::SA + g, *a1 = a0 + 4 * S::SA, *b0 = b + r0 * S::SB + g, *b1 = b0 + 4 * S::SB;
+        unsigned ah[MT][4], al[MT][4], bh[4][2], bl[4][2];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {  // A[m = plane][k = rule]: a0 (g, t), a1 (g + 8, t), a2 (g, t + 4), a3 (g + 8, t + 4)
+          dw_split(a0[mt * 16], ah[mt][0], al[mt][0]);
+          dw_split(a0[mt * 16 + 8], ah[mt][1], al[mt][1]);
+          dw_split(a1[mt * 16], ah[mt][2], al[mt][2]);
+          dw_split(a1[mt * 16 + 8], ah[mt][3], al[mt][3]);
+        }
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {  // B[k = rule][n = plane]: b0 (t, g), b1 (t + 4, g)
+          dw_split(b0[nt * 8], bh[nt][0], bl[nt][0]);
+          dw_split(b1[nt * 8], bh[nt][1], bl[nt][1]);
+        }
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) dw_mma(d[mt][nt], al[mt], bh[nt]);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) dw_mma(d[mt][nt], ah[mt], bl[nt]);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) dw_mma(d[mt][nt], ah[mt], bh[nt]);
+      }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+  }
+
+  // ---- the warps' tiles; those of warps that shared one are added in warp order ------------------------------------
+  float *tile = stages + warp * S::TILE;
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {  // d0 (g, 2t), d1 (g, 2t + 1), d2 (g + 8, 2t), d3 (g + 8, 2t + 1)
-      tile[warp][mt * 16 + g][nt * 8 + 2 * t] = d[mt][nt][0];
-      tile[warp][mt * 16 + g][nt * 8 + 2 * t + 1] = d[mt][nt][1];
-      tile[warp][mt * 16 + g + 8][nt * 8 + 2 * t] = d[mt][nt][2];
-      tile[warp][mt * 16 + g + 8][nt * 8 + 2 * t + 1] = d[mt][nt][3];
+      float *q = tile + (mt * 16 + g) * 33 + nt * 8 + 2 * t;
+      q[0] = d[mt][nt][0];
+      q[1] = d[mt][nt][1];
+      q[8 * 33] = d[mt][nt][2];
+      q[8 * 33 + 1] = d[mt][nt][3];
     }
   __syncthreads();
   float *dst = partial + ((long long)blockIdx.x * gridDim.y + k) * cin * cout;
-  for (int i = threadIdx.x; i < 32 * 32; i += 128) {
-    const int c = i >> 5, n = i & 31;
-    dst[(long long)(c0 + c) * cout + n0 + n] = ((tile[0][c][n] + tile[1][c][n]) + tile[2][c][n]) + tile[3][c][n];
+  for (int i = tid; i < S::M * S::N; i += S::THREADS) {
+    const int c = i / S::N, n = i % S::N;
+    if (c0 + c >= cin || n0 + n >= cout) continue;
+    const float *q = stages + (c / (16 * MT) + (n / 32) * WM) * S::TILE + c % (16 * MT) * 33 + n % 32;  // share 0 of the tile
+    float v = q[0];
+#pragma unroll
+    for (int w = 1; w < S::SHARE; ++w) v += q[w * WM * WN * S::TILE];
+    dst[(long long)(c0 + c) * cout + n0 + n] = v;
   }
+}
+
+template <int WM, int WN, int MT = 2>
+static int launch_dweight(const float *in, int ld_in, long long n_in_rows, const float *dout, int ld_out,
+                          long long n_out_rows, const int *nbr, long long n_entries, int swap, int K, int cin, int cout,
+                          float *d_weight, int *flags, cudaStream_t stream) {
+  using S = DwShape<WM, WN, MT>;
+  static std::atomic<bool> configured[64];
+  int dev = 0;
+  SCN_CUDA_CHECK(cudaGetDevice(&dev));
+  SCN_REQUIRE(dev >= 0 && dev < 64, SCN_ERR_UNSUPPORTED, "device index %d unsupported", dev);
+  SCN_REQUIRE(n_entries < (1ll << 31), SCN_ERR_UNSUPPORTED, "%lld rulebook entries", n_entries);
+  if (!configured[dev].load()) {
+    SCN_CUDA_CHECK(cudaFuncSetAttribute(k_conv_dweight_mma<WM, WN, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
+    configured[dev].store(true);
+  }
+  // about four waves of the CTAs the SMs hold, in chunks of whole lists
+  const int tiles = (int)(ceil_div(cin, S::M) * ceil_div(cout, S::N));
+  const int per_sm = std::max(1, (int)(220 * 1024 / S::SMEM));
+  const int chunks = (int)std::max<long long>(1, std::min<long long>(ceil_div(148 * 4 * per_sm, (long long)K * tiles), n_entries / S::LIST));
+  const long long chunk_rows = ceil_div(ceil_div(n_entries, chunks), S::LIST) * S::LIST;
+  const int grid_x = (int)ceil_div(n_entries, chunk_rows);
+  const long long w_elems = (long long)K * cin * cout;
+  float *partial = d_weight;
+  if (grid_x > 1) SCN_TRY(device_alloc((void **)&partial, sizeof(float) * (size_t)grid_x * w_elems, stream));
+  const int vec_in = cin % 4 == 0 && ld_in % 4 == 0 && (uintptr_t)in % 16 == 0;
+  const int vec_out = cout % 4 == 0 && ld_out % 4 == 0 && (uintptr_t)dout % 16 == 0;
+  SCN_LAUNCH((k_conv_dweight_mma<WM, WN, MT>), dim3((unsigned)grid_x, (unsigned)K, (unsigned)tiles), S::THREADS, S::SMEM, stream, in, ld_in, n_in_rows, dout, ld_out, n_out_rows, nbr, n_entries, swap, cin, cout, vec_in, vec_out, chunk_rows, partial, flags);
+  if (grid_x > 1) {
+    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, grid_x, w_elems, d_weight);
+    SCN_TRY(device_free(partial, stream));
+  }
+  SCN_CUDA_CHECK(cudaGetLastError());
+  return SCN_OK;
+}
+
+// 32-plane tiles per side: one CTA tile up to 96 planes, beyond that whichever of 64 and 96 pads less
+static int dweight_side(int planes) {
+  if (planes <= 96) return (planes + 31) / 32;
+  return ceil_div(planes, 96) * 96 < ceil_div(planes, 64) * 64 ? 3 : 2;
 }
 
 // partial[chunk][p] = sum over the chunk's rows of x[row][p]; grid = (plane tiles of 32, chunks)
@@ -263,15 +384,6 @@ k_column_sums(const float *__restrict__ x, long long n_rows, int planes, long lo
     for (int i = 0; i < 8; ++i) t += sh[i][lane];
     partial[(long long)blockIdx.y * planes + p] = t;
   }
-}
-
-// out[i] = sum over chunks, in order, of partial[chunk][i]
-__global__ void k_sum_chunks(const float *__restrict__ partial, int chunks, long long n, float *__restrict__ out) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float acc = 0.f;
-  for (int c = 0; c < chunks; ++c) acc += partial[(long long)c * n + i];
-  out[i] = acc;
 }
 
 static int n_chunks(long long rows) { return (int)std::max<long long>(1, std::min<long long>(64, rows / 4096)); }
@@ -316,19 +428,26 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
   // ---- d_weight -----------------------------------------------------------------------------------
   {
     const long long n_entries = rb.n_out;  // nbr is [K][rb.n_out]
-    const int chunks = n_chunks(n_entries);
-    const long long chunk_rows = ceil_div(ceil_div(n_entries, chunks), 32) * 32;
-    float *partial = nullptr;
-    SCN_TRY(device_alloc((void **)&partial, sizeof(float) * (size_t)chunks * w_elems, stream));
-    const int tiles = groups * (int)ceil_div(cin, 32) * (int)ceil_div(cout, 32);
     const bool fma_only = getenv("SCN_DWEIGHT_FMA") && atoi(getenv("SCN_DWEIGHT_FMA")) != 0;
-    if (groups == 1 && cin % 32 == 0 && cout % 32 == 0 && !fma_only)
-      SCN_LAUNCH(k_conv_dweight_mma, dim3((unsigned)chunks, (unsigned)K, (unsigned)tiles), 128, 0, stream, in, n_in_planes, rows_in, d_out, n_out_planes, rows_out, rb.nbr, n_entries, transposed ? 1 : 0, cin, cout, chunk_rows, partial, md->flags_dev);
-    else
+    if (groups == 1 && !fma_only) {
+      decltype(&launch_dweight<1, 1>) const by_side[3][3] = {{launch_dweight<1, 1>, launch_dweight<1, 2>, launch_dweight<1, 3>},
+                                                             {launch_dweight<2, 1>, launch_dweight<2, 2>, launch_dweight<2, 3>},
+                                                             {launch_dweight<3, 1>, launch_dweight<3, 2>, launch_dweight<3, 3>}};
+      auto launch = by_side[dweight_side(cin) - 1][dweight_side(cout) - 1];
+      if (cin <= 16) launch = cout <= 32 ? launch_dweight<1, 1, 1> : cout <= 64 ? launch_dweight<1, 2, 1> : launch_dweight<1, 3, 1>;
+      SCN_TRY(launch(in, n_in_planes, rows_in, d_out, n_out_planes, rows_out, rb.nbr, n_entries, transposed ? 1 : 0, K, cin,
+                     cout, d_weight, md->flags_dev, stream));
+    } else {
+      const int chunks = n_chunks(n_entries);
+      const long long chunk_rows = ceil_div(ceil_div(n_entries, chunks), 32) * 32;
+      float *partial = nullptr;
+      SCN_TRY(device_alloc((void **)&partial, sizeof(float) * (size_t)chunks * w_elems, stream));
+      const int tiles = groups * (int)ceil_div(cin, 32) * (int)ceil_div(cout, 32);
       SCN_LAUNCH(k_conv_dweight, dim3((unsigned)chunks, (unsigned)K, (unsigned)tiles), 256, 0, stream, in, n_in_planes, rows_in, d_out, n_out_planes, rows_out, rb.nbr, n_entries, transposed ? 1 : 0, cin, cout, groups, chunk_rows, partial, md->flags_dev);
-    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, chunks, w_elems, d_weight);
-    SCN_CUDA_CHECK(cudaGetLastError());
-    SCN_TRY(device_free(partial, stream));
+      SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, chunks, w_elems, d_weight);
+      SCN_CUDA_CHECK(cudaGetLastError());
+      SCN_TRY(device_free(partial, stream));
+    }
   }
 
   // ---- d_input ------------------------------------------------------------------------------------

@@ -225,16 +225,32 @@ k_bn_back_sums(const float *__restrict__ in, const float *__restrict__ out, cons
   }
 }
 
-__global__ void k_bn_back_finalize(const double *__restrict__ partial, int chunks, int C, long long n_rows,
-                                   const float *__restrict__ invstd, float *__restrict__ d_weight,
-                                   float *__restrict__ d_bias, float *__restrict__ coef /* [2][C] */) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  double s = 0.0, q = 0.0;
-  for (int i = 0; i < chunks; ++i) {
+// the chunk sums of plane c, added by one warp in a fixed order (lane l takes chunks l, l + 32, ..., then the lanes)
+__device__ __forceinline__ void bn_back_total(const double *__restrict__ partial, int chunks, int C, int c, double &s, double &q) {
+  const int lane = threadIdx.x & 31;
+  s = q = 0.0;
+  for (int i = lane; i < chunks; i += 32) {
     s += partial[((long long)i * 2 + 0) * C + c];
     q += partial[((long long)i * 2 + 1) * C + c];
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    q += __shfl_xor_sync(0xffffffffu, q, o);
+  }
+}
+
+// one warp per plane (a thread per plane that walked up to 1024 chunks on its own took 57 us, as long as the passes over
+// the rows)
+__global__ void __launch_bounds__(256)
+k_bn_back_finalize(const double *__restrict__ partial, int chunks, int C, long long n_rows,
+                   const float *__restrict__ invstd, float *__restrict__ d_weight, float *__restrict__ d_bias,
+                   float *__restrict__ coef /* [2][C] */) {
+  const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (c >= C) return;
+  double s, q;
+  bn_back_total(partial, chunks, C, c, s, q);
+  if ((threadIdx.x & 31) != 0) return;
   const float is = invstd[c];
   if (d_bias) d_bias[c] = (float)s;
   if (d_weight) d_weight[c] = (float)q * is;
@@ -244,14 +260,13 @@ __global__ void k_bn_back_finalize(const double *__restrict__ partial, int chunk
 
 // The two-phase form of the backward pass (rows spread over several devices): the chunk sums of one device
 // added in their fixed order ...
-__global__ void k_bn_back_reduce(const double *__restrict__ partial, int chunks, int C, double *__restrict__ sums) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256)
+k_bn_back_reduce(const double *__restrict__ partial, int chunks, int C, double *__restrict__ sums) {
+  const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (c >= C) return;
-  double s = 0.0, q = 0.0;
-  for (int i = 0; i < chunks; ++i) {
-    s += partial[((long long)i * 2 + 0) * C + c];
-    q += partial[((long long)i * 2 + 1) * C + c];
-  }
+  double s, q;
+  bn_back_total(partial, chunks, C, c, s, q);
+  if ((threadIdx.x & 31) != 0) return;
   sums[c] = s;
   sums[C + c] = q;
 }
@@ -286,6 +301,38 @@ k_bn_back_apply(const float *__restrict__ in, float *__restrict__ d_in, const fl
   if (!(out[r * out_stride + c] > 0.f)) d *= leak;
   const float x = in[r * in_stride + c] - mean[c];
   d_in[r * in_stride + c] = (d - coef[c] - x * coef[C + c]) * invstd[c] * (weight ? weight[c] : 1.f);
+}
+
+// the same for dense rows of a multiple of four planes (16-byte aligned, fewer than 2^32 values)
+__global__ void __launch_bounds__(256)
+k_bn_back_apply4(const float4 *__restrict__ in, float4 *__restrict__ d_in, const float4 *__restrict__ out,
+                 const float4 *__restrict__ d_out, unsigned n4, unsigned C4, const float *__restrict__ mean,
+                 const float *__restrict__ invstd, const float *__restrict__ weight, const float *__restrict__ coef, float leak) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n4) return;
+  const int c = (int)(i % C4) * 4, C = (int)C4 * 4;
+  const float4 dv = __ldg(d_out + i), ov = __ldg(out + i), xv = __ldg(in + i);
+  const float d0[4] = {dv.x, dv.y, dv.z, dv.w}, o[4] = {ov.x, ov.y, ov.z, ov.w}, x0[4] = {xv.x, xv.y, xv.z, xv.w};
+  float r[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float d = d0[e];
+    if (!(o[e] > 0.f)) d *= leak;
+    const float x = x0[e] - __ldg(mean + c + e);
+    r[e] = (d - __ldg(coef + c + e) - x * __ldg(coef + C + c + e)) * __ldg(invstd + c + e) * (weight ? __ldg(weight + c + e) : 1.f);
+  }
+  d_in[i] = make_float4(r[0], r[1], r[2], r[3]);
+}
+
+static void launch_bn_back_apply(const float *in, float *d_in, const float *out, const float *d_out, long long n_rows, int C,
+                                 long long in_stride, long long out_stride, const float *mean, const float *invstd,
+                                 const float *weight, const float *coef, float leak, cudaStream_t stream) {
+  const long long n = n_rows * C;
+  if (C % 4 == 0 && in_stride == C && out_stride == C && n < (1ll << 32) &&
+      ((uintptr_t)in | (uintptr_t)d_in | (uintptr_t)out | (uintptr_t)d_out) % 16 == 0)
+    SCN_LAUNCH(k_bn_back_apply4, (unsigned)ceil_div(n / 4, 256), 256, 0, stream, (const float4 *)in, (float4 *)d_in, (const float4 *)out, (const float4 *)d_out, (unsigned)(n / 4), (unsigned)(C / 4), mean, invstd, weight, coef, leak);
+  else
+    SCN_LAUNCH(k_bn_back_apply, (unsigned)ceil_div(n, 256), 256, 0, stream, in, d_in, out, d_out, n_rows, C, in_stride, out_stride, mean, invstd, weight, coef, leak);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -714,8 +761,8 @@ int scn_batchnorm_backward(const float *in_features, float *d_in_features, const
   SCN_TRY(device_alloc((void **)&partial, sizeof(double) * 2 * (size_t)chunks * n_planes, stream));
   SCN_TRY(device_alloc((void **)&coef, sizeof(float) * 2 * (size_t)n_planes, stream));
   SCN_LAUNCH(k_bn_back_sums, dim3((unsigned)ceil_div(n_planes, 32), (unsigned)chunks), 256, 0, stream, in_features, out_features, d_out_features, n_rows, n_planes, in_stride, out_stride, save_mean, (float)leakiness, chunk_rows, partial);
-  SCN_LAUNCH(k_bn_back_finalize, (unsigned)ceil_div(n_planes, 128), 128, 0, stream, partial, chunks, n_planes, n_rows, save_invstd, d_weight, d_bias, coef);
-  SCN_LAUNCH(k_bn_back_apply, (unsigned)ceil_div(n_rows * n_planes, 256), 256, 0, stream, in_features, d_in_features, out_features, d_out_features, n_rows, n_planes, in_stride, out_stride, save_mean, save_invstd, weight, coef, (float)leakiness);
+  SCN_LAUNCH(k_bn_back_finalize, (unsigned)ceil_div(n_planes, 8), 256, 0, stream, partial, chunks, n_planes, n_rows, save_invstd, d_weight, d_bias, coef);
+  launch_bn_back_apply(in_features, d_in_features, out_features, d_out_features, n_rows, n_planes, in_stride, out_stride, save_mean, save_invstd, weight, coef, (float)leakiness, stream);
   SCN_CUDA_CHECK(cudaGetLastError());
   SCN_TRY(device_free(partial, stream));
   SCN_TRY(device_free(coef, stream));
@@ -789,7 +836,7 @@ int scn_batchnorm_backward_sums(const float *in_features, const float *out_featu
   double *partial = nullptr;
   SCN_TRY(device_alloc((void **)&partial, sizeof(double) * 2 * (size_t)chunks * n_planes, stream));
   SCN_LAUNCH(k_bn_back_sums, dim3((unsigned)ceil_div(n_planes, 32), (unsigned)chunks), 256, 0, stream, in_features, out_features, d_out_features, (long long)n_rows, n_planes, (long long)in_stride, (long long)out_stride, save_mean, (float)leakiness, chunk_rows, partial);
-  SCN_LAUNCH(k_bn_back_reduce, (unsigned)ceil_div(n_planes, 128), 128, 0, stream, partial, chunks, n_planes, sums);
+  SCN_LAUNCH(k_bn_back_reduce, (unsigned)ceil_div(n_planes, 8), 256, 0, stream, partial, chunks, n_planes, sums);
   const cudaError_t err = cudaGetLastError();
   SCN_TRY(device_free(partial, stream));
   SCN_CUDA_CHECK(err);
@@ -816,7 +863,7 @@ int scn_batchnorm_backward_sums_apply(const float *in_features, float *d_in_feat
       device_free(coef, stream);
       SCN_REQUIRE(false, SCN_ERR_BAD_ARG, "null features");
     }
-    SCN_LAUNCH(k_bn_back_apply, (unsigned)ceil_div(n_rows * n_planes, 256), 256, 0, stream, in_features, d_in_features, out_features, d_out_features, (long long)n_rows, n_planes, (long long)in_stride, (long long)out_stride, save_mean, save_invstd, weight, coef, (float)leakiness);
+    launch_bn_back_apply(in_features, d_in_features, out_features, d_out_features, (long long)n_rows, n_planes, (long long)in_stride, (long long)out_stride, save_mean, save_invstd, weight, coef, (float)leakiness, stream);
   }
   const cudaError_t err = cudaGetLastError();
   SCN_TRY(device_free(coef, stream));

@@ -1,0 +1,52 @@
+"""Weight gradients of the convolutions (k_conv_dweight_mma) against a float64 product over the exported rulebook.
+
+Tolerance: three tf32 products of the hi / lo split drop lo x lo and the low bits of lo, 2^-21 of a product, and n fp32
+additions of random sign add 2^-24 sqrt(n) of the running sum: below 1e-5 of the largest entry for the row counts here;
+1e-4 is the fp32 bar of the package."""
+import numpy as np
+import pytest
+import torch
+
+from tests import helpers
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("cin,cout", [(1, 8), (3, 32), (8, 16), (24, 20), (32, 33), (31, 64), (64, 96), (96, 64), (96, 96),
+                                      (100, 160), (192, 96), (33, 1)])
+@pytest.mark.parametrize("n,size", [(40, 12), (6000, 40), (30001, 96)])
+def test_weight_gradient(n, size, cin, cout, cuda):
+    import sparseconvnet_b200 as scn
+    rng = np.random.default_rng(n + cin)
+    pts = rng.integers(0, size, (n, 3))
+    pts[:, 2] = size // 2 + size // 5 * np.sin(pts[:, 0] / 6.0) + rng.integers(0, 2, n)
+    x = scn.InputLayer(3, size, mode=4)([torch.from_numpy(pts), torch.zeros(n, 1, device=cuda)])
+    up_size = torch.LongTensor([size // 2] * 3)
+    torch.manual_seed(cin)
+    for layer in (scn.SubmanifoldConvolution(3, cin, cout, 3, True), scn.Convolution(3, cin, cout, 2, 2, False),
+                  scn.Deconvolution(3, cin, cout, 2, 2, False)):
+        layer.to(cuda)
+        md, filt = x.metadata, [2, 2, 2]
+        if isinstance(layer, scn.Deconvolution):
+            rows, spatial = md.getNActive(up_size), up_size
+        else:
+            rows, spatial = x.features.size(0), x.spatial_size
+        f = torch.randn(rows, cin, device=cuda, requires_grad=True)
+        y = layer(scn.SparseConvNetTensor(f, md, spatial))
+        g = torch.randn_like(y.features)
+        y.features.backward(g)
+        if isinstance(layer, scn.SubmanifoldConvolution):
+            rules = md.rulebook(0, x.spatial_size, [3, 3, 3])
+        else:
+            rules = md.rulebook(1, x.spatial_size, filt, filt)
+        if isinstance(layer, scn.Deconvolution):
+            rules = [r.flip(1) for r in rules]
+        fd, gd = f.detach().double(), g.double()
+        want = torch.stack([fd[r[:, 0].long()].t() @ gd[r[:, 1].long()] for r in rules])
+        e = helpers.rel_err(layer.weight.grad[:, 0].double().cpu().numpy(), want.cpu().numpy())
+        assert e <= helpers.FP32_TOL, (layer, e)
+        want = torch.zeros(rows, cin, dtype=torch.float64, device=cuda)
+        for r, w in zip(rules, layer.weight.detach().double()[:, 0]):
+            want.index_add_(0, r[:, 0].long(), gd[r[:, 1].long()] @ w.t())
+        e = helpers.rel_err(f.grad.double().cpu().numpy(), want.cpu().numpy())
+        assert e <= helpers.FP32_TOL, (layer, "input gradient", e)
