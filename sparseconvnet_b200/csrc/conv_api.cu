@@ -61,6 +61,13 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
                       const RowOrder &ord, int K, int cin, int cout, int precision, int *flags, cudaStream_t stream,
                       const float *pre_scale, const float *pre_shift, float pre_leak, const float *in_b, int planes_a);
 
+bool conv_fma_supported(const float *in, const float *out, const float *weight, const float *bias, int K, int cin, int cout,
+                        int groups);
+bool conv_fma_wants_order(long long n_out);
+int conv_forward_fma(const float *in, long long n_in, float *out, long long n_out, const float *weight, const float *bias,
+                     const float *bn_scale, const float *bn_shift, float leak, const int *table, const RowOrder *ord, int K,
+                     int cin, int cout, int *flags, cudaStream_t stream);
+
 // Is an environment variable of the library set at all?  (One pass over the environment instead of one per knob.)
 static bool any_knob() {
   for (char **e = ::environ; e && *e; ++e)
@@ -214,6 +221,31 @@ __global__ void k_bn_fold(const float *__restrict__ mean, const float *__restric
   shift[c] = __fadd_rn(__fmul_rn(-mean[c], w), beta ? beta[c] : 0.f);
 }
 
+// For kernels that read their input as it is: a join (in_b: the input is [in (planes_a) | in_b], groups == 1) and / or an
+// eval-mode BatchNorm in front are written to a scratch matrix first, which then is the input (*copy, the caller frees it).
+static int prepared_input(const float **in, long long rows_in, int cin, int groups, const float *pre_scale,
+                          const float *pre_shift, float pre_leak, const float *in_b, int planes_a, float **copy,
+                          cudaStream_t stream) {
+  if (rows_in == 0 || (!in_b && !pre_scale)) return SCN_OK;
+  const long long total = rows_in * (long long)cin * groups;
+  if (in_b)
+    SCN_REQUIRE(groups == 1 && planes_a % 4 == 0 && (cin - planes_a) % 4 == 0 && (uintptr_t)*in % 16 == 0 &&
+                    (uintptr_t)in_b % 16 == 0,
+                SCN_ERR_UNSUPPORTED, "joined input: plane counts must be multiples of four");
+  SCN_TRY(device_alloc((void **)copy, sizeof(float) * (size_t)total, stream));
+  if (in_b) {
+    SCN_LAUNCH(k_scale_shift_act_join_to, (unsigned)std::min<long long>(ceil_div(total / 4, 256), 148 * 16), 256, 0, stream,
+               *in, planes_a, in_b, cin - planes_a, *copy, rows_in, pre_scale, pre_shift, pre_leak);
+  } else {
+    const int vec = (cin * groups) % 4 == 0 && (uintptr_t)*in % 16 == 0 && (uintptr_t)pre_scale % 16 == 0 &&
+                    (uintptr_t)pre_shift % 16 == 0;
+    SCN_LAUNCH(k_scale_shift_act_to, (unsigned)std::min<long long>(ceil_div(total / (vec ? 4 : 1), 256), 148 * 16), 256, 0,
+               stream, *in, *copy, rows_in, cin * groups, pre_scale, pre_shift, pre_leak, vec);
+  }
+  *in = *copy;
+  return SCN_OK;
+}
+
 // pre_scale / pre_shift / pre_leak (optional): an eval-mode BatchNorm and its leaky ReLU in FRONT of the
 // convolution, in[r][p] <- act(in[r][p] * pre_scale[p] + pre_shift[p]).  The tcgen05 kernels that split their input
 // rows before the launch apply it in that pass; for every other kernel it is applied into a scratch copy of the
@@ -250,28 +282,9 @@ int conv_forward_dispatch(const float *in, long long rows_in, float *out, long l
   const bool to_tc = tensor && !to_wide && !to_tma && conv_tc_supported(cin, cout, groups, precision);
   float *pre_copy = nullptr;
   const bool splits = to_wide || (to_tc && conv_tc_splits_rows(precision, cin, rows_in, rows_out));
-  if (in_b && rows_in > 0 && !splits) {
-    // a joined input (in_b: the input is [in (planes_a) | in_b]; groups == 1) for a kernel without a split pass:
-    // the concatenation, normalised if a BatchNorm comes with it, is written to a scratch matrix first
-    SCN_REQUIRE(groups == 1 && planes_a % 4 == 0 && (cin - planes_a) % 4 == 0 && (uintptr_t)in % 16 == 0 &&
-                    (uintptr_t)in_b % 16 == 0,
-                SCN_ERR_UNSUPPORTED, "joined input: plane counts must be multiples of four");
-    const long long total = rows_in * (long long)cin;
-    SCN_TRY(device_alloc((void **)&pre_copy, sizeof(float) * (size_t)total, stream));
-    SCN_LAUNCH(k_scale_shift_act_join_to, (unsigned)std::min<long long>(ceil_div(total / 4, 256), 148 * 16), 256, 0, stream,
-               in, planes_a, in_b, cin - planes_a, pre_copy, rows_in, pre_scale, pre_shift, pre_leak);
-    in = pre_copy;
+  if (!splits && rows_in > 0) {
+    SCN_TRY(prepared_input(&in, rows_in, cin, groups, pre_scale, pre_shift, pre_leak, in_b, planes_a, &pre_copy, stream));
     in_b = nullptr;
-    pre_scale = pre_shift = nullptr;
-  }
-  if (pre_scale && rows_in > 0 && !splits) {
-    const long long total = rows_in * (long long)cin * groups;
-    SCN_TRY(device_alloc((void **)&pre_copy, sizeof(float) * (size_t)total, stream));
-    const int vec = (cin * groups) % 4 == 0 && (uintptr_t)in % 16 == 0 && (uintptr_t)pre_scale % 16 == 0 &&
-                    (uintptr_t)pre_shift % 16 == 0;
-    SCN_LAUNCH(k_scale_shift_act_to, (unsigned)std::min<long long>(ceil_div(total / (vec ? 4 : 1), 256), 148 * 16), 256, 0,
-               stream, in, pre_copy, rows_in, cin * groups, pre_scale, pre_shift, pre_leak, vec);
-    in = pre_copy;
     pre_scale = pre_shift = nullptr;
   }
   const int status = [&]() -> int {
@@ -348,8 +361,28 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
     g_last_kernel = cout <= 64 ? SCN_KERNEL_CONV_ROWS : rows_out <= 148 * 256 ? SCN_KERNEL_CONV_TC : SCN_KERNEL_CONV_WIDE;
     return SCN_OK;
   }
-  return conv_forward_dispatch(in, rows_in, out, rows_out, weight, bias, table, rb.n_offsets, cin, cout, groups, precision,
-                               flags, stream, bn_scale, bn_shift, leak, pre_scale, pre_shift, pre_leak, in_b, planes_a);
+  // fp32: the same tiles on the FMA pipe (first layers of at most four input planes keep their own kernel), unless a
+  // BatchNorm or a join in front has to be applied to a copy of the input first
+  const bool fma = precision == SCN_PRECISION_FP32 && rows_out > 0 && cin > 4 &&
+                   conv_fma_supported(in, out, weight, bias, rb.n_offsets, cin, cout, groups) &&
+                   !(any_knob() && getenv("SCN_SIMT_BLOCK") && atoi(getenv("SCN_SIMT_BLOCK")) != 0);
+  if (!fma)
+    return conv_forward_dispatch(in, rows_in, out, rows_out, weight, bias, table, rb.n_offsets, cin, cout, groups, precision,
+                                 flags, stream, bn_scale, bn_shift, leak, pre_scale, pre_shift, pre_leak, in_b, planes_a);
+  float *pre_copy = nullptr;
+  SCN_TRY(prepared_input(&in, rows_in, cin, groups, pre_scale, pre_shift, pre_leak, in_b, planes_a, &pre_copy, stream));
+  RowOrder *ord = nullptr;
+  int rc = SCN_OK;
+  if (conv_fma_wants_order(rows_out)) {
+    ord = transposed_table ? &rb.torder : &rb.order;
+    rc = rulebook_row_order(rb, table, rows_out, *ord, stream);
+  }
+  if (rc == SCN_OK)
+    rc = conv_forward_fma(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, table, ord, rb.n_offsets, cin,
+                          cout, flags, stream);
+  device_free(pre_copy, stream);
+  g_last_kernel = SCN_KERNEL_CONV_SIMT;
+  return rc;
 }
 
 static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float *in, float *out,

@@ -540,13 +540,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
 // partial [n_split][n_tiles * 128][cout] -> out: the parts of a row added in order, then bias and BatchNorm
 __global__ void __launch_bounds__(256)
 k_tile_sum(const float4 *__restrict__ partial, int n_split, long long n_pos, int cout4, const int *__restrict__ order,
-           const float *__restrict__ bias, const float *__restrict__ bn_scale, const float *__restrict__ bn_shift,
+           long long n_out, const float *__restrict__ bias, const float *__restrict__ bn_scale, const float *__restrict__ bn_shift,
            float leak, float4 *__restrict__ out) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_pos * cout4) return;
   const int c = (int)(i % cout4);
-  const int r = __ldg(order + i / cout4);
-  if (r < 0) return;
+  const long long r = order ? __ldg(order + i / cout4) : i / cout4;
+  if (r < 0 || r >= n_out) return;
   float4 q = __ldg(partial + i);
   for (int p = 1; p < n_split; ++p) {
     const float4 a = __ldg(partial + (long long)p * n_pos * cout4 + i);
@@ -563,7 +563,7 @@ k_tile_sum(const float4 *__restrict__ partial, int n_split, long long n_pos, int
     q.x *= q.x > 0.f ? 1.f : leak, q.y *= q.y > 0.f ? 1.f : leak;
     q.z *= q.z > 0.f ? 1.f : leak, q.w *= q.w > 0.f ? 1.f : leak;
   }
-  out[(long long)r * cout4 + c] = q;
+  out[r * cout4 + c] = q;
 }
 
 // in [n][cin] fp32 (or the column-wise concatenation [in (planes_a) | in_b], read where the two lie) -> per row and
@@ -659,6 +659,16 @@ int launch_tile(TileParams &P, int n_sm, int dev, cudaStream_t stream) {
 }
 
 }  // namespace
+
+// out = act((bias + the parts of partial [n_split][n_pos][cout], in order) * bn_scale + bn_shift); position p is row
+// order[p] (order null: row p)
+int sum_partial_tiles(const float *partial, int n_split, long long n_pos, int cout, const int *order, long long n_out,
+                      const float *bias, const float *bn_scale, const float *bn_shift, float leak, float *out,
+                      cudaStream_t stream) {
+  SCN_LAUNCH(k_tile_sum, (unsigned)ceil_div(n_pos * (cout / 4), 256), 256, 0, stream, (const float4 *)partial, n_split, n_pos, cout / 4, order, n_out, bias, bn_scale, bn_shift, leak, (float4 *)out);
+  SCN_CUDA_CHECK(cudaGetLastError());
+  return SCN_OK;
+}
 
 extern thread_local int g_drop_arrival;  // test hook (conv_tc.cu)
 
@@ -763,14 +773,8 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
     else
       rc = SP == 64 ? launch_tile<1, 64>(P, n_sm, dev, stream) : launch_tile<1, 32>(P, n_sm, dev, stream);
   }
-  if (rc == SCN_OK && P.n_split > 1) {
-    const long long n_pos = P.n_tiles * kRows;
-    SCN_LAUNCH(k_tile_sum, (unsigned)ceil_div(n_pos * (cout / 4), 256), 256, 0, stream, (const float4 *)partial, P.n_split, n_pos, cout / 4, ord.order, bias, bn_scale, bn_shift, leak, (float4 *)out);
-    if (cudaGetLastError() != cudaSuccess) {
-      set_error("tile kernel: launch failed");
-      rc = SCN_ERR_CUDA;
-    }
-  }
+  if (rc == SCN_OK && P.n_split > 1)
+    rc = sum_partial_tiles(partial, P.n_split, P.n_tiles * kRows, cout, ord.order, n_out, bias, bn_scale, bn_shift, leak, out, stream);
   device_free(partial, stream);
   device_free(split, stream);
   const int rf = weight_image_put(wi, stream);

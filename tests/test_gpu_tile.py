@@ -93,3 +93,36 @@ def test_splits(split, precision, n, cuda, monkeypatch):
     layers = [scn.SubmanifoldConvolution(3, 64, 64, 3, True), scn.SubmanifoldConvolution(3, 64, 128, 3, False),
               scn.Convolution(3, 128, 96, 2, 2, False)]
     _compare(layers, _points(n, 3, 120, 7), 3, 120, 64, precision, cuda)
+
+
+@pytest.mark.parametrize("cin,cout", [(8, 8), (12, 16), (24, 32), (32, 36), (36, 64), (64, 96), (100, 160), (64, 224)])
+@pytest.mark.parametrize("n,split", [(1, None), (31, None), (900, "3"), (8191, None), (8200, "7"), (60001, None)])
+def test_fp32_tiles(n, split, cin, cout, cuda, monkeypatch):
+    """k_conv_fma (fp32) against a float64 product over the exported rulebook: packed and unpacked rows, both tile heights,
+    every plane tile, with and without divided offsets.  Sums of at most 27 x 100 fp32 products: 2700 x 2^-24 of the
+    largest sum of magnitudes at the very worst, 2^-24 sqrt(2700) in practice; 1e-5."""
+    import sparseconvnet_b200 as scn
+    if split:
+        monkeypatch.setenv("SCN_FMA_SPLIT", split)
+    coords = _points(n, 3, 160, n)
+    x = scn.InputLayer(3, 160, mode=0)([torch.from_numpy(coords), torch.zeros(len(coords), 1, device=cuda)])
+    torch.manual_seed(cin)
+    layers = [(scn.SubmanifoldConvolution(3, cin, cout, 3, True), 0, [3, 3, 3], None, x.spatial_size),
+              (scn.Convolution(3, cin, cout, 2, 2, True), 1, [2, 2, 2], [2, 2, 2], x.spatial_size),
+              (scn.Deconvolution(3, cin, cout, 2, 2, False), 1, [2, 2, 2], [2, 2, 2], torch.LongTensor([80, 80, 80]))]
+    with torch.no_grad():
+        for layer, kind, filt, stride, spatial in layers:
+            layer.to(cuda)
+            if hasattr(layer, "bias"):
+                layer.bias.normal_()
+            f = torch.randn(x.metadata.getNActive(spatial), cin, device=cuda)
+            y = layer(scn.SparseConvNetTensor(f, x.metadata, spatial)).features
+            want = torch.zeros(y.shape, dtype=torch.float64, device=cuda)
+            if hasattr(layer, "bias"):
+                want += layer.bias.double()
+            for r, w in zip(x.metadata.rulebook(kind, x.spatial_size, filt, stride), layer.weight.double()[:, 0]):
+                r = r.long() if not isinstance(layer, scn.Deconvolution) else r.long().flip(1)
+                want.index_add_(0, r[:, 1], f.double()[r[:, 0]] @ w)
+            e = helpers.rel_err(y.double().cpu().numpy(), want.cpu().numpy())
+            assert e <= 1e-5, (layer, e)
+            x.metadata.poll_errors()
