@@ -57,7 +57,7 @@ int conv_forward_rows_scatter(const float *in, long long n_in, float *out, long 
 bool conv_tile_supported(const float *in, const float *in_b, int planes_a, const float *out, const float *bias, int K,
                          int cin, int cout, int groups);
 int conv_forward_tile(const float *in, long long n_in, float *out, long long n_out, const float *weight,
-                      const float *bias, const float *bn_scale, const float *bn_shift, float leak, const int *table,
+                      const float *bias, const float *bn_scale, const float *bn_shift, float leak,
                       const RowOrder &ord, int K, int cin, int cout, int precision, int *flags, cudaStream_t stream,
                       const float *pre_scale, const float *pre_shift, float pre_leak, const float *in_b, int planes_a);
 
@@ -356,7 +356,7 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
   if (tile_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, precision, rows_out)) {
     RowOrder &ord = transposed_table ? rb.torder : rb.order;
     SCN_TRY(rulebook_row_order(rb, table, rows_out, ord, stream));
-    SCN_TRY(conv_forward_tile(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, table, ord, rb.n_offsets,
+    SCN_TRY(conv_forward_tile(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, ord, rb.n_offsets,
                               cin, cout, precision, flags, stream, pre_scale, pre_shift, pre_leak, in_b, planes_a));
     g_last_kernel = cout <= 64 ? SCN_KERNEL_CONV_ROWS : rows_out <= 148 * 256 ? SCN_KERNEL_CONV_TC : SCN_KERNEL_CONV_WIDE;
     return SCN_OK;

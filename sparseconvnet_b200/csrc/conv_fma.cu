@@ -44,7 +44,7 @@ struct FmaParams {
   const float *bias, *bn_scale, *bn_shift;
   float leak;
   const int *nbr;
-  const int *order;  // null: rows in their own order
+  const int *order, *packed;  // null: rows in their own order
   const unsigned *tile_bits;
   int words, K, cin, cout, n_split;
   long long n_pos;
@@ -62,7 +62,7 @@ struct FmaShape {
 };
 
 template <int ROWS, int BN>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, ROWS == 128 && BN == 64 ? 3 : 4)
 k_conv_fma(FmaParams P) {
   using S = FmaShape<ROWS, BN>;
   constexpr int TM = S::TM, TN = S::TN;
@@ -70,18 +70,14 @@ k_conv_fma(FmaParams P) {
   __shared__ unsigned mask[4];
   const int tid = threadIdx.x, lane = tid & 31;
   const int tx = tid % S::TX, ty = tid / S::TX;
-  const long long pos0 = (long long)blockIdx.x * ROWS;
+  // from the back: packed tiles come in ascending order of their masks, and the ones with the most offsets are best started
+  // first
+  const long long pos0 = (long long)(gridDim.x - 1 - blockIdx.x) * ROWS;
   const int n0 = blockIdx.y * BN;
 
   // ---- copying role: eight threads per row, 16 rows (of ROWS) at a time ----------------------------------------------
   const int cj = (tid & 7) * 4, cr = tid >> 3;
   constexpr int CI = ROWS / 16;
-  int orow[CI];
-#pragma unroll
-  for (int i = 0; i < CI; ++i) {
-    const long long p = pos0 + cr + 16 * i;
-    orow[i] = P.order ? __ldg(P.order + p) : p < P.n_out ? (int)p : -1;
-  }
 
   // ---- offsets with a rule for any of the rows ------------------------------------------------------------------------
   unsigned m[4];
@@ -118,30 +114,28 @@ k_conv_fma(FmaParams P) {
     return 0;
   };
   for (int i = 0; i < skip; ++i) next_offset();
+  // packed: the entries of the tile's next offset, then those of the one after, ...
+  const int *packed = P.order ? P.packed + (pos0 / kOrderTile * P.K + skip) * kOrderTile + pos0 % kOrderTile + cr : nullptr;
 
   const int nch = (P.cin + kChunk - 1) / kChunk;
   const int steps = n_offsets * nch;
   int k_issue = 0, c_issue = 0, left = n_offsets;  // of the step to be issued next
-  int v[CI], v_next[CI];                           // its rows' rulebook entries, and those of the offset after it
-  auto entries = [&](int k, int(&e)[CI]) {
+  int v[CI];                                       // its rows' rulebook entries
+  auto take_offset = [&] {
+    if (left-- <= 0) return;
+    k_issue = next_offset();
 #pragma unroll
     for (int i = 0; i < CI; ++i) {
-      e[i] = orow[i] >= 0 ? __ldg(P.nbr + (long long)k * P.n_out + orow[i]) : -1;
-      if (e[i] >= P.n_in) {
-        atomicOr(P.flags, FLAG_BAD_ROW);
-        e[i] = -1;
+      if (P.order) {
+        v[i] = __ldg(packed + 16 * i);
+      } else {
+        const long long p = pos0 + cr + 16 * i;
+        v[i] = p < P.n_out ? __ldg(P.nbr + (long long)k_issue * P.n_out + p) : -1;
       }
     }
+    if (P.order) packed += kOrderTile;
   };
-  int k_next = 0;
-  if (left > 0) {
-    k_issue = next_offset();
-    entries(k_issue, v);
-    if (--left > 0) {
-      k_next = next_offset();
-      entries(k_next, v_next);
-    }
-  }
+  take_offset();
   constexpr int WP = BN / 4, WR = kThreads / WP;  // 16-byte pieces of a weight row; rows per pass
   const int wc = (tid % WP) * 4, wr = tid / WP;
   auto issue = [&](int s) {  // one cp.async group per call, empty past the end
@@ -151,8 +145,11 @@ k_conv_fma(FmaParams P) {
       if (c0 + cj < P.cin) {
         const float *src = P.in + c0 + cj;
 #pragma unroll
-        for (int i = 0; i < CI; ++i)
-          cp_async16(smem_u32(a + (cr + 16 * i) * kAStride + cj), v[i] >= 0 ? src + (long long)v[i] * P.cin : P.in, v[i] >= 0 ? 16u : 0u);
+        for (int i = 0; i < CI; ++i) {
+          const bool hit = (unsigned)v[i] < (unsigned)P.n_in;
+          if (v[i] >= 0 && !hit) atomicOr(P.flags, FLAG_BAD_ROW);
+          cp_async16(smem_u32(a + (cr + 16 * i) * kAStride + cj), hit ? src + (long long)v[i] * P.cin : P.in, hit ? 16u : 0u);
+        }
       }
       const float *wk = P.weight + ((long long)k_issue * P.cin + c0) * P.cout + n0 + wc;
       const int rows = min(kChunk, P.cin - c0);
@@ -164,13 +161,7 @@ k_conv_fma(FmaParams P) {
       }
       if (++c_issue == nch) {
         c_issue = 0;
-        k_issue = k_next;
-#pragma unroll
-        for (int i = 0; i < CI; ++i) v[i] = v_next[i];
-        if (--left > 0) {
-          k_next = next_offset();
-          entries(k_next, v_next);
-        }
+        take_offset();
       }
     }
     cp_async_commit();
@@ -299,6 +290,7 @@ int conv_forward_fma(const float *in, long long n_in, float *out, long long n_ou
   P.leak = leak;
   P.nbr = table;
   P.order = ord ? ord->order : nullptr;
+  P.packed = ord ? ord->packed : nullptr;
   P.tile_bits = ord ? ord->tile_bits : nullptr;
   P.words = ord ? ord->words : 0;
   P.K = K;

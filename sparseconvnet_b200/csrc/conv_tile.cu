@@ -20,8 +20,8 @@
 //
 // Roles (15 warps, one CTA per SM, persistent).  A step is one filter offset of one tile and SP input planes; the
 // steps of a CTA are numbered through all its tiles and step n uses stage n % n_stages of one ring.
-//   scheduler   publishes a slot per (tile, filter offset with a rule): the input row of every tile row, brought in by
-//               4-byte cp.async so that it never waits for them; up to kSlots offsets ahead
+//   entries     one thread: a slot per (tile, filter offset with a rule), the input row of every tile row, one 512-byte
+//               bulk copy from the packed table; up to kSlots offsets ahead
 //   producers   8 warps, warp w takes steps w, w + 8, ...: all 128 rows of the step by 16-byte cp.async pieces
 //               straight into the swizzled operand layout, zero fill where a row has no rule; the barrier arrival
 //               happens when a lane's copies have landed.  (One warp per step: with a step spread over all warps its
@@ -51,7 +51,7 @@ namespace {
 
 constexpr int kRows = kOrderTile;  // rows of a tile = MMA M
 constexpr int kProdWarps = 8;
-constexpr int kEpi0 = kProdWarps, kMma = kProdWarps + 4, kWgt = kMma + 1, kSched = kMma + 2;
+constexpr int kEpi0 = kProdWarps, kMma = kProdWarps + 4, kWgt = kMma + 1, kEntries = kMma + 2;
 constexpr int kThreads = (kProdWarps + 7) * 32;
 constexpr int kSlots = 16;      // offsets the scheduler runs ahead
 constexpr int kMaxStages = 12;
@@ -66,8 +66,7 @@ struct TileParams {
   const unsigned char *wprep;
   const float *bias, *bn_scale, *bn_shift;
   float leak;
-  const int *nbr;
-  const int *order;
+  const int *order, *packed;
   const unsigned *tile_bits;
   int words;
   int K, n_slices;
@@ -82,13 +81,10 @@ template <int TERMS, int SP>
 struct TileShape {
   static constexpr int PARTS = TERMS == 3 ? 2 : 1;
   static constexpr int PP = SP * 2 * PARTS / 16;      // 16-byte pieces per row and step
-  static constexpr int RPI = 32 / PP;                 // rows per copy instruction of a warp
-  static constexpr int NI = kRows / RPI;              // copy instructions per step
+  static constexpr int NI = kRows / (32 / PP);        // copy instructions per step and lane
   static constexpr unsigned ROW = PP * 16;            // bytes of a row in a stage: 128 or 64
   static constexpr unsigned A_BYTES = kRows * ROW;
   static_assert(PP == 8 || PP == 4, "a row of a step is 128 or 64 bytes");
-  // where the entry of tile row r is kept in a slot: the NI rows of a lane follow one another
-  __device__ static constexpr int entry(int r) { return (r % RPI) * NI + r / RPI; }
 };
 
 // Operand descriptor of a stage of gathered rows: K-major, 128- or 64-byte swizzle (a row's 16-byte chunk c is stored
@@ -106,25 +102,21 @@ __device__ __forceinline__ unsigned long long rows_desc(unsigned addr, unsigned 
   return d;
 }
 
+constexpr int kNoRules = 1 << 20;
+
 // control block behind the ring
 struct Ctl {
   unsigned long long full[kMaxStages], empty[kMaxStages];  // rows and weights landed; MMAs done
   unsigned long long s_full[kSlots], s_empty[kSlots], acc_full[4], acc_empty[4];
-  int slot_k[kSlots];  // filter offset of the slot; -1: no more work
+  int slot_k[kSlots];  // filter offset of the slot; -1: no more work; kNoRules: offset 0 with rows of zeros
   unsigned tmem;
   int abort;
 };
-
-// what a tile row past the end of the matrix reads as its rulebook entry
-__device__ const int d_no_rule = -1;
 
 __host__ __device__ inline unsigned tile_idesc(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(kRows >> 4) << 24);
 }
 
-__device__ __forceinline__ void cp_async4(unsigned dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_arrive(unsigned long long *bar) {  // when this thread's copies have landed
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -187,21 +179,27 @@ __device__ __forceinline__ void keep_range(unsigned (&m)[4], int lo, int hi) {
   }
 }
 
+// The tile of an item, from the back: packed tiles come in ascending order of their masks, and the ones with the most
+// offsets are best started first.
+__device__ __forceinline__ long long item_tile(const TileParams &P, long long item) {
+  return P.n_tiles - 1 - item / P.n_split;
+}
+
 // filter offsets of an item: those of its tile, or its share of them when the offsets are divided
 __device__ __forceinline__ int item_offsets(const TileParams &P, long long item) {
   if (item >= P.n_items) return 0;
-  const long long t = item / P.n_split;
+  const long long t = item_tile(P, item);
   int total = 0;
   for (int w = 0; w < P.words; ++w) total += __popc(__ldg(P.tile_bits + t * P.words + w));
   if (P.n_split == 1) return total;
-  const int part = (int)(item - t * P.n_split);
+  const int part = (int)(item % P.n_split);
   return total * (part + 1) / P.n_split - total * part / P.n_split;
 }
 
 template <int TERMS, int SP>
 __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
   using Shape = TileShape<TERMS, SP>;
-  constexpr int PP = Shape::PP, RPI = Shape::RPI, NI = Shape::NI, PARTS = Shape::PARTS;
+  constexpr int PP = Shape::PP, NI = Shape::NI, PARTS = Shape::PARTS;
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const unsigned w_part = (unsigned)P.coutp * SP * 2;  // one bf16 weight slab
@@ -221,7 +219,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
       mbar_init(&C.empty[i], 1);
     }
     for (int i = 0; i < kSlots; ++i) {
-      mbar_init(&C.s_full[i], 32 + 1);             // the scheduler's copies, and its lane 0 for the words beside them
+      mbar_init(&C.s_full[i], 1);
       mbar_init(&C.s_empty[i], P.n_slices + 1);    // a producer warp per slice, and the weights
     }
     for (int i = 0; i < 4; ++i) {
@@ -241,8 +239,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
 
   if (warp < kProdWarps) {
     // ==================================== producers =============================================
-    const int j = lane % PP, q = lane / PP;  // this lane's piece, and the first of its rows q, q + RPI, ...
-    const unsigned chunk = (unsigned)(PP == 8 ? j ^ q : j ^ ((q >> 1) & 3)) * 16 + (unsigned)q * Shape::ROW;
+    // this lane's 16-byte piece of the rows q NI .. q NI + NI - 1 (the entries of a lane follow one another)
+    const int j = lane % PP, q = lane / PP;
+    const unsigned lane_dst = (unsigned)(q * NI) * Shape::ROW + (unsigned)j * 16;
     // No more warps than stages: a warp at step n has seen the consumption of step n - active - n_stages, and its wait
     // below can tell step n - n_stages from the one a round earlier only if that one is not later than this.
     const int active = min(kProdWarps, P.n_stages);
@@ -257,13 +256,15 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
         ok = false;
         break;
       }
-      if (C.slot_k[si] < 0 || *abort) break;
+      const int slot_k = C.slot_k[si];
+      if (slot_k < 0 || *abort) break;
+      const int rows_in = slot_k == kNoRules ? 0 : (int)P.n_in;  // entries below it are rows
       const int4 *ent = reinterpret_cast<const int4 *>(entries + si * kRows + q * NI);
       if (!mbar_wait(&C.empty[st], (round + 1) & 1)) {  // (the first round passes)
         ok = false;
         break;
       }
-      const unsigned dst = smem0 + (unsigned)st * stage_bytes + chunk;
+      const unsigned dst = smem0 + (unsigned)st * stage_bytes + lane_dst;
       const unsigned char *col = P.in_split + slice * (SP * 2 * PARTS) + j * 16;
 #pragma unroll
       for (int i = 0; i < NI; i += 4) {
@@ -271,11 +272,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
         const int v[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const bool hit = (unsigned)v[e] < (unsigned)P.n_in;
-          bad |= v[e] >= (int)P.n_in;
-          // (eight pieces: rows four apart alternate between the two halves of the swizzle pattern)
-          cp_async16((PP == 8 && (e & 1) ? dst ^ 64u : dst) + (i + e) * RPI * Shape::ROW,
-                     col + (size_t)(unsigned)(hit ? v[e] : 0) * P.row_bytes, hit ? 16u : 0u);
+          const bool hit = (unsigned)v[e] < (unsigned)rows_in;
+          bad |= v[e] >= (int)P.n_in && slot_k != kNoRules;
+          const unsigned swizzle = (PP == 8 ? (i + e) & 7 : ((i + e) >> 1) & 3) * 16;  // (q NI is a multiple of eight)
+          cp_async16((dst ^ swizzle) + (i + e) * Shape::ROW, col + (size_t)(unsigned)(hit ? v[e] : 0) * P.row_bytes, hit ? 16u : 0u);
         }
       }
       cp_async_arrive(&C.full[st]);
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
         const int k = C.slot_k[si];
         mbar_arrive(&C.s_empty[si]);
         if (k < 0) break;
-        const unsigned char *src = P.wprep + (size_t)k * P.n_slices * w_bytes;
+        const unsigned char *src = P.wprep + (size_t)(k == kNoRules ? 0 : k) * P.n_slices * w_bytes;
         for (int s = 0; s < P.n_slices; ++s) {
           if (!mbar_wait(&C.empty[st], par) || *abort) {
             ok = false;
@@ -386,98 +386,80 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
       if (++buf == n_acc) buf = 0, buf_par ^= 1, d = tmem;
     }
     if (!ok) *abort = 1;
-  } else if (warp == kSched) {
-    // ==================================== scheduler =============================================
-    int slot = 0;
-    bool ok = true;
-    const int words = P.words;
-    const unsigned entries0 = smem_u32(entries) + 4 * Shape::entry(4 * lane);
-    // lane holds rows 4 lane .. 4 lane + 3 of a tile; the next item's are fetched one item ahead
-    int4 o_next;
-    unsigned b_next[4];
-    auto fetch = [&](long long item) {
-      const long long t = item / P.n_split;
-      const bool in = item < P.n_items;
-      o_next = in ? __ldg(reinterpret_cast<const int4 *>(P.order + t * kRows) + lane) : make_int4(-1, -1, -1, -1);
+  } else if (warp == kEntries) {
+    // ==================================== entries ===============================================
+    if (lane == 0) {
+      int slot = 0;
+      bool ok = true;
+      unsigned b_next[4];
+      auto fetch = [&](long long item) {
 #pragma unroll
-      for (int w = 0; w < 4; ++w) b_next[w] = in && w < words ? __ldg(P.tile_bits + t * words + w) : 0u;
-    };
-    fetch(blockIdx.x);
-    for (long long it = 0; it < my_items && ok; ++it) {
-      const long long item = blockIdx.x + it * gridDim.x;
-      const int o[4] = {o_next.x, o_next.y, o_next.z, o_next.w};
-      unsigned u[4];
+        for (int w = 0; w < 4; ++w)
+          b_next[w] = item < P.n_items && w < P.words ? __ldg(P.tile_bits + item_tile(P, item) * P.words + w) : 0u;
+      };
+      fetch(blockIdx.x);
+      for (long long it = 0; it < my_items && ok; ++it) {
+        const long long item = blockIdx.x + it * gridDim.x;
+        unsigned u[4];
 #pragma unroll
-      for (int w = 0; w < 4; ++w) u[w] = b_next[w];
-      fetch(item + gridDim.x);
-      if (P.n_split > 1) {
-        const int total = __popc(u[0]) + __popc(u[1]) + __popc(u[2]) + __popc(u[3]), part = (int)(item % P.n_split);
-        keep_range(u, total * part / P.n_split, total * (part + 1) / P.n_split);
-      }
-      // a tile (or part) without any rule still gets one step: its rows are all zero fill and so is its sum
-      const bool none = (u[0] | u[1] | u[2] | u[3]) == 0;
-      if (none) u[0] = 1u;
-      const int *p[4];
-      bool row[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        row[e] = o[e] >= 0 && !none;
-        p[e] = row[e] ? P.nbr + o[e] : &d_no_rule;
-      }
-      const bool whole = __all_sync(0xffffffffu, row[0] && row[1] && row[2] && row[3]);
+        for (int w = 0; w < 4; ++w) u[w] = b_next[w];
+        fetch(item + gridDim.x);
+        const int *src = P.packed + item_tile(P, item) * P.K * kRows;
+        if (P.n_split > 1) {
+          const int total = __popc(u[0]) + __popc(u[1]) + __popc(u[2]) + __popc(u[3]), part = (int)(item % P.n_split);
+          const int first = total * part / P.n_split;
+          keep_range(u, first, total * (part + 1) / P.n_split);
+          src += first * kRows;
+        }
+        // a tile (or part) without any rule still gets one step, of weights and rows of zeros
+        bool none = (u[0] | u[1] | u[2] | u[3]) == 0;
+        if (none) u[0] = 1u;
 #pragma unroll 1
-      for (int w = 0; w < words && ok; ++w) {
-        unsigned m = u[0];
-        u[0] = u[1], u[1] = u[2], u[2] = u[3], u[3] = 0;
-        while (m) {
-          const int k = w * 32 + __ffs(m) - 1;
-          m &= m - 1;
-          const int si = slot % kSlots;
-          if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1) || *abort) {
-            ok = false;
-            break;
+        for (int w = 0; w < 4 && ok; ++w) {
+          unsigned m = u[0];
+          u[0] = u[1], u[1] = u[2], u[2] = u[3], u[3] = 0;
+          for (; m; m &= m - 1, ++slot, src += kRows) {
+            const int si = slot % kSlots;
+            if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1) || *abort) {
+              ok = false;
+              break;
+            }
+            C.slot_k[si] = none ? kNoRules : w * 32 + __ffs(m) - 1;
+            if (none) {
+              mbar_arrive(&C.s_full[si]);
+            } else {
+              mbar_expect_tx(&C.s_full[si], kRows * 4);
+              bulk_copy_g2s(smem_u32(entries + si * kRows), src, kRows * 4, &C.s_full[si]);
+            }
           }
-          const unsigned dst = entries0 + si * (kRows * 4);
-          const long long col = (long long)k * P.n_out;
-          if (whole) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) cp_async4(dst + 4 * (Shape::entry(4 * lane + e) - Shape::entry(4 * lane)), p[e] + col);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              cp_async4(dst + 4 * (Shape::entry(4 * lane + e) - Shape::entry(4 * lane)), p[e] + (row[e] ? col : 0));
-          }
-          cp_async_arrive(&C.s_full[si]);
-          if (lane == 0) {
-            C.slot_k[si] = k;
-            mbar_arrive(&C.s_full[si]);
-          }
-          ++slot;
         }
       }
-    }
-    // every producer warp finds its next step in a slot that ends it
-    for (int i = 0; i <= (kProdWarps + P.n_slices - 1) / P.n_slices && ok; ++i, ++slot) {
-      const int si = slot % kSlots;
-      if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1)) {
-        ok = false;
-        break;
-      }
-      cp_async_arrive(&C.s_full[si]);
-      if (lane == 0) {
+      const int filled = slot;
+      // every producer warp finds its next step in a slot that ends it
+      for (int i = 0; i <= (kProdWarps + P.n_slices - 1) / P.n_slices && ok; ++i, ++slot) {
+        const int si = slot % kSlots;
+        if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1)) {
+          ok = false;
+          break;
+        }
         C.slot_k[si] = -1;
         mbar_arrive(&C.s_full[si]);
       }
+      if (!ok) {  // copies in flight must land before the CTA's shared memory goes away
+        *abort = 1;
+        for (int i = 0; i < kSlots; ++i) {
+          const int uses = (filled + kSlots - 1 - i) / kSlots;
+          if (uses > 0) mbar_wait(&C.s_full[i], (unsigned)((uses - 1) & 1));
+        }
+      }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    if (!ok) *abort = 1;
   } else {
     // ==================================== epilogue ==============================================
     const int quad = warp & 3;
     const int nc = P.cout;
     int buf = 0, buf_par = 0;
     for (long long it = 0; it < my_items; ++it) {
-      const long long item = blockIdx.x + it * gridDim.x, t = item / P.n_split;
+      const long long item = blockIdx.x + it * gridDim.x, t = item_tile(P, item);
       const int part = (int)(item % P.n_split);
       const int orow = __ldg(P.order + t * kRows + quad * 32 + lane);
       int got = 1;
@@ -694,10 +676,10 @@ static int split_parts(long long n_tiles, int K, int n_slices, double step_cycle
   return best_s;
 }
 
-// out [n_out, cout] = act((bias + sum_k in[table[k][.]] @ W[k]) * bn_scale + bn_shift), the input optionally a join and
-// behind a BatchNorm of its own (see k_tile_split).  `ord`: the packing of the table's rows.
+// out [n_out, cout] = act((bias + sum_k in[table[k][.]] @ W[k]) * bn_scale + bn_shift) for the table that `ord` packs, the
+// input optionally a join and behind a BatchNorm of its own (see k_tile_split)
 int conv_forward_tile(const float *in, long long n_in, float *out, long long n_out, const float *weight,
-                      const float *bias, const float *bn_scale, const float *bn_shift, float leak, const int *table,
+                      const float *bias, const float *bn_scale, const float *bn_shift, float leak,
                       const RowOrder &ord, int K, int cin, int cout, int precision, int *flags, cudaStream_t stream,
                       const float *pre_scale, const float *pre_shift, float pre_leak, const float *in_b, int planes_a) {
   if (n_out == 0) return SCN_OK;
@@ -748,8 +730,8 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
   P.bn_scale = bn_scale;
   P.bn_shift = bn_shift;
   P.leak = bn_scale ? leak : 1.f;
-  P.nbr = table;
   P.order = ord.order;
+  P.packed = ord.packed;
   P.tile_bits = ord.tile_bits;
   P.words = ord.words;
   P.K = K;

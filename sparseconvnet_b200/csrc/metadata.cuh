@@ -46,13 +46,15 @@ int count_ticket_total(CountTicket *t, long long *total);  // waits for the valu
 
 // The packing of a table's output rows into tensor-core tiles (row_order.cu): order[p] = output row at position
 // p, -1 past the end (padded to whole tiles); tile_bits[t][words] = filter offsets for which any of the 128 rows
-// of tile t has a rule.
+// of tile t has a rule; packed[t][j][128] = the table's entries of the tile's rows for the j-th of those offsets,
+// -1 where a row has no rule (room for all K offsets per tile, only the tile's own are written).
 constexpr int kOrderTile = 128;
 constexpr int kOrderMaxOffsets = 128;
 inline int mask_words(int K) { return K <= 32 ? 1 : 4; }
 struct RowOrder {
   int *order = nullptr;
   unsigned *tile_bits = nullptr;
+  int *packed = nullptr;
   int words = 1;  // 32-bit words per tile: 1 up to 32 offsets, else 4
   long long n_tiles = 0;
 };

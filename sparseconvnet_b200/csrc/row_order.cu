@@ -13,8 +13,10 @@
 //   stride-2 transposed layers (8 offsets, one rule per row): -> 1
 //
 // Steps: k_order_keys (mask -> sort key, and the digit counts of the first pass), then one stable counting pass per
-// digit of at most nine bits (k_order_scatter, with k_order_count between two passes), then k_order_tiles (the union
-// of the masks of every 128 rows).
+// digit of at most nine bits (k_order_scatter, with k_order_count between two passes), then k_order_tiles: the union
+// of the masks of every 128 rows, and the table's entries of those rows laid out one after the other.  Rows of one tile
+// lie far apart in the table (52 to 99 sectors per 128 entries): looked up by the convolutions themselves, that was as
+// much traffic as a quarter to a half of the rows they gather, once per layer.
 #include <stdlib.h>
 
 #include <algorithm>
@@ -168,112 +170,122 @@ k_order_scatter(const KEY *__restrict__ keys, const int *__restrict__ rows_in, l
   }
 }
 
-// Levels too small to sort: the identity order and its tiles in one launch, one warp per tile.
-template <int WORDS>
-__global__ void __launch_bounds__(256)
-k_order_plain(const int *__restrict__ nbr, long long n, int K, int *__restrict__ order, unsigned *__restrict__ tile_bits,
-              long long n_tiles) {
-  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (t >= n_tiles) return;
-#pragma unroll
-  for (int i = 0; i < kTile / 32; ++i) {
-    const long long p = t * kTile + i * 32 + lane;
-    order[p] = p < n ? (int)p : -1;
+// Levels too small to sort: the identity order, its tiles and their entries in one launch, one block per tile.
+__global__ void __launch_bounds__(kTile)
+k_order_plain(const int *__restrict__ nbr, long long n, int K, int words, int *__restrict__ order,
+              unsigned *__restrict__ tile_bits, int *__restrict__ packed) {
+  __shared__ unsigned bits[4];
+  const long long t = blockIdx.x, p = t * kTile + threadIdx.x;
+  if (threadIdx.x < 4) bits[threadIdx.x] = 0;
+  order[p] = p < n ? (int)p : -1;
+  __syncthreads();
+  unsigned seen = 0;  // of the current word, by this warp
+#pragma unroll 9
+  for (int k = 0; k < K; ++k) {
+    const int v = p < n ? __ldg(nbr + (long long)k * n + p) : -1;
+    if (__any_sync(0xffffffffu, v >= 0)) seen |= 1u << (k & 31);
+    if ((k & 31) == 31 || k == K - 1) {
+      if ((threadIdx.x & 31) == 0 && seen) atomicOr(&bits[k >> 5], seen);
+      seen = 0;
+    }
   }
-#pragma unroll
-  for (int w = 0; w < WORDS; ++w) {
-    unsigned bits = 0;
+  __syncthreads();
+  int *dst = packed + t * K * kTile + threadIdx.x;
+  for (int w = 0; w < words; ++w) {
+    const unsigned all = bits[w];
+    if (threadIdx.x == 0) tile_bits[t * words + w] = all;
 #pragma unroll 4
-    for (int b = 0; b < 32 && w * 32 + b < K; ++b) {
-      bool any = false;
-#pragma unroll
-      for (int i = 0; i < kTile / 32; ++i) {
-        const long long p = t * kTile + i * 32 + lane;
-        any |= p < n && __ldg(nbr + (long long)(w * 32 + b) * n + p) >= 0;
-      }
-      if (__any_sync(0xffffffffu, any)) bits |= 1u << b;
+    for (unsigned u = all; u; u &= u - 1) {
+      const int k = w * 32 + __ffs(u) - 1;
+      *dst = p < n ? __ldg(nbr + (long long)k * n + p) : -1;
+      dst += kTile;
     }
-    if (lane == 0) tile_bits[t * WORDS + w] = bits;
   }
 }
 
-// tile_bits[t][WORDS]: offsets for which any of the tile's rows has a rule; one warp per tile.  The order array
-// is filled with -1 up to its padded length.
+// One warp per tile, four rows per lane: tile_bits, packed, and -1 in the order array past the last row.
 template <int WORDS>
 __global__ void __launch_bounds__(256)
-k_order_tiles(int *__restrict__ order, long long n, long long n_padded, const unsigned *__restrict__ masks,
-              unsigned *__restrict__ tile_bits, long long n_tiles) {
+k_order_tiles(int *__restrict__ order, long long n, int K, const int *__restrict__ nbr, const unsigned *__restrict__ masks,
+              unsigned *__restrict__ tile_bits, int *__restrict__ packed, long long n_tiles) {
   const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= n_tiles) return;
-  unsigned m[WORDS];
-#pragma unroll
-  for (int w = 0; w < WORDS; ++w) m[w] = 0;
-#pragma unroll
-  for (int i = 0; i < kTile / 32; ++i) {
-    const long long p = t * kTile + i * 32 + lane;
-    if (p < n) {
-      const long long r = order[p];
-#pragma unroll
-      for (int w = 0; w < WORDS; ++w) m[w] |= __ldg(masks + r * WORDS + w);
-    } else if (p < n_padded) {
-      order[p] = -1;
-    }
+  const long long p = t * kTile + lane * 4;
+  int4 o = *reinterpret_cast<const int4 *>(order + p);
+  if (p + 3 >= n) {
+    o.x = p < n ? o.x : -1, o.y = p + 1 < n ? o.y : -1, o.z = p + 2 < n ? o.z : -1, o.w = -1;
+    *reinterpret_cast<int4 *>(order + p) = o;
   }
+  const int row[4] = {o.x, o.y, o.z, o.w};
+  unsigned m[4][WORDS];
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) m[e][w] = row[e] >= 0 ? __ldg(masks + (long long)row[e] * WORDS + w) : 0u;
+  int *dst = packed + t * K * kTile + lane * 4;
 #pragma unroll
   for (int w = 0; w < WORDS; ++w) {
-    const unsigned u = __reduce_or_sync(0xffffffffu, m[w]);
-    if (lane == 0) tile_bits[t * WORDS + w] = u;
+    const unsigned all = __reduce_or_sync(0xffffffffu, m[0][w] | m[1][w] | m[2][w] | m[3][w]);
+    if (lane == 0) tile_bits[t * WORDS + w] = all;
+#pragma unroll 4
+    for (unsigned u = all; u; u &= u - 1) {
+      const int b = __ffs(u) - 1;
+      const int *col = nbr + (long long)(w * 32 + b) * n;
+      int v[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = m[e][w] >> b & 1u ? __ldg(col + row[e]) : -1;
+      *reinterpret_cast<int4 *>(dst) = make_int4(v[0], v[1], v[2], v[3]);
+      dst += kTile;
+    }
   }
 }
 
-// Which key bits the offsets set (pos[k], 255 for none), and how many bits there are.  Fewer bits cost fewer passes,
+// Which key bits the offsets set, and how many bits there are.  Fewer bits cost fewer passes,
 // and below about 65 000 rows a coarser key also packs better, because full masks are hardly ever repeated.  Offsets
 // per tile of 128 rows on rooms of 405 k / 119 k / 37 k / 15 k rows, 27 offsets (in coordinate order 22.4 / 23.9 /
 // 23.8 / 25.6):
 //   27 bits, the first offset highest               9.48   9.88  10.3  17.3   three passes
 //   the 12 edges, then the 6 faces                   9.70  10.2   11.4  18.1   two
 //   OR-ed over the middle dimension (9 bits)        13.0   12.8   11.3  14.4   one
-// A 4-D filter of size 3 puts the offsets of the earlier and later time slice first, OR-ed over one spatial dimension,
-// then the slice of the site itself in full (45 bits: 35.2 offsets per tile of moving shells; all 81 bits in filter
-// order: 40.8), or OR-ed as well (27 bits: 38.2).  Other large filters: groups of consecutive offsets.
-int key_bits(const Rulebook &rb, int K, long long n, unsigned char *pos) {
-  for (int k = 0; k < kOrderMaxOffsets; ++k) pos[k] = 255;
+// A 4-D filter of size 3 (81 offsets, nearly every site of moving shells has a mask of its own): for the earlier and the
+// later time slice whether any offset with x (y, z) = -1, 0, 1 has a rule, then the slice of the site itself OR-ed over
+// y: 27 bits, 36.7 offsets per tile; all 81 bits in filter order 40.8; the time slices OR-ed over y and the middle one in
+// full 35.2, but the rows of a tile lie a third farther apart.  Other large filters: groups of consecutive offsets.
+// An offset may set several bits: bit[k] is their union.
+int key_bits(const Rulebook &rb, int K, long long n, unsigned long long *bit) {
+  for (int k = 0; k < K; ++k) bit[k] = 0;
   bool three = rb.dim >= 3;
   for (int d = 0; d < rb.dim; ++d) three &= rb.filter[d] == 3;
   if (rb.dim == 3 && three && n < 65536) {
-    for (int k = 0; k < 27; ++k) pos[k] = (unsigned char)(8 - ((k / 9) * 3 + k % 3));
+    for (int k = 0; k < 27; ++k) bit[k] = 1ull << (8 - ((k / 9) * 3 + k % 3));
     return 9;
   }
   if (rb.dim == 3 && three && n < 524288) {
     int edges = 0, faces = 0;
     for (int k = 0; k < 27; ++k) {
       const int far = (k % 3 != 1) + (k / 3 % 3 != 1) + (k / 9 != 1);
-      if (far == 2) pos[k] = (unsigned char)(17 - edges++);
-      if (far == 1) pos[k] = (unsigned char)(5 - faces++);
+      if (far == 2) bit[k] = 1ull << (17 - edges++);
+      if (far == 1) bit[k] = 1ull << (5 - faces++);
     }
     return 18;
   }
   if (K <= 32) {
-    for (int k = 0; k < K; ++k) pos[k] = (unsigned char)(K - 1 - k);
+    for (int k = 0; k < K; ++k) bit[k] = 1ull << (K - 1 - k);
     return K;
   }
   if (rb.dim == 4 && three) {
-    const bool full = n >= 262144;
     for (int k = 0; k < 81; ++k) {
       const int t = k % 3, z = (k / 3) % 3, y = (k / 9) % 3, x = k / 27;
-      int rank;  // 0 = highest bit
       if (t == 1)
-        rank = 18 + (full ? (x * 3 + y) * 3 + z : x * 3 + z);
+        bit[k] = 1ull << (8 - (x * 3 + z));
       else
-        rank = (t == 0 ? 0 : 9) + x * 3 + z;
-      pos[k] = (unsigned char)((full ? 44 : 26) - rank);
+        bit[k] = ((1ull << (8 - x)) | (1ull << (5 - y)) | (1ull << (2 - z))) << (t == 0 ? 18 : 9);
     }
-    return full ? 45 : 27;
+    return 27;
   }
   const int most = n >= 262144 ? 45 : 27, group = (K + most - 1) / most, bits = (K + group - 1) / group;
-  for (int k = 0; k < K; ++k) pos[k] = (unsigned char)(bits - 1 - k / group);
+  for (int k = 0; k < K; ++k) bit[k] = 1ull << (bits - 1 - k / group);
   return bits;
 }
 
@@ -293,7 +305,7 @@ struct Scratch {  // freed on every way out
 };
 
 template <typename KEY, int WORDS>
-int build(const int *table, const unsigned *known, long long n, int K, const unsigned char *pos, int bits, RowOrder &ord, cudaStream_t stream) {
+int build(const int *table, const unsigned *known, long long n, int K, const unsigned long long *bit, int bits, RowOrder &ord, cudaStream_t stream) {
   Scratch tmp(stream);
   unsigned *masks = nullptr;
   KEY *keys[2] = {nullptr, nullptr};
@@ -304,7 +316,7 @@ int build(const int *table, const unsigned *known, long long n, int K, const uns
   const long long rpb = std::min<long long>(ceil_div(ceil_div(n, 148), kThreads), 63) * kThreads;
   const int blocks = (int)ceil_div(n, rpb);
   KeyBits<KEY> B{};
-  for (int k = 0; k < K; ++k) B.bit[k] = pos[k] == 255 ? (KEY)0 : (KEY)1 << pos[k];
+  for (int k = 0; k < K; ++k) B.bit[k] = (KEY)bit[k];
   if (!known) SCN_TRY(tmp.get((void **)&masks, sizeof(unsigned) * WORDS * (size_t)n));
   SCN_TRY(tmp.get((void **)&keys[0], sizeof(KEY) * (size_t)n));
   SCN_TRY(tmp.get((void **)&counts, sizeof(int) * (size_t)blocks * R));
@@ -324,7 +336,7 @@ int build(const int *table, const unsigned *known, long long n, int K, const uns
     SCN_LAUNCH((k_order_scatter<KEY>), blocks, kThreads, 0, stream, kin, src, n, (int)rpb, p * digit, R, counts, totals + (size_t)p * R, kout, dst);
     src = dst;
   }
-  SCN_LAUNCH((k_order_tiles<WORDS>), (unsigned)ceil_div(ord.n_tiles * 32, 256), 256, 0, stream, ord.order, n, ord.n_tiles * kTile, known ? known : masks, ord.tile_bits, ord.n_tiles);
+  SCN_LAUNCH((k_order_tiles<WORDS>), (unsigned)ceil_div(ord.n_tiles * 32, 256), 256, 0, stream, ord.order, n, K, table, known ? known : masks, ord.tile_bits, ord.packed, ord.n_tiles);
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }
@@ -334,6 +346,7 @@ int build(const int *table, const unsigned *known, long long n, int K, const uns
 void free_row_order(RowOrder &o, cudaStream_t stream) {
   device_free(o.order, stream);
   device_free(o.tile_bits, stream);
+  device_free(o.packed, stream);
   o = RowOrder{};
 }
 
@@ -347,25 +360,22 @@ int rulebook_row_order(const Rulebook &rb, const int *table, long long n, RowOrd
   o.n_tiles = ceil_div(n, kTile);
   int st = device_alloc((void **)&o.order, sizeof(int) * (size_t)o.n_tiles * kTile, stream);
   if (st == SCN_OK) st = device_alloc((void **)&o.tile_bits, sizeof(unsigned) * (size_t)o.words * o.n_tiles, stream);
+  if (st == SCN_OK) st = device_alloc((void **)&o.packed, sizeof(int) * (size_t)o.n_tiles * K * kTile, stream);
   // Small levels are bound by latency whatever the order, and the sort takes as long as one of their layers.
   long long least = 8192;
   if (const char *e = getenv("SCN_ORDER_MIN_ROWS")) least = atoll(e);
   if (st == SCN_OK && n < least) {
-    const unsigned grid = (unsigned)ceil_div(o.n_tiles * 32, 256);
-    if (K <= 32)
-      SCN_LAUNCH(k_order_plain<1>, grid, 256, 0, stream, table, n, K, o.order, o.tile_bits, o.n_tiles);
-    else
-      SCN_LAUNCH(k_order_plain<4>, grid, 256, 0, stream, table, n, K, o.order, o.tile_bits, o.n_tiles);
+    SCN_LAUNCH(k_order_plain, (unsigned)o.n_tiles, kTile, 0, stream, table, n, K, o.words, o.order, o.tile_bits, o.packed);
     if (cudaGetLastError() != cudaSuccess) {
       set_error("row order: launch failed");
       st = SCN_ERR_CUDA;
     }
   } else if (st == SCN_OK) {
-    unsigned char pos[kOrderMaxOffsets];
-    const int bits = key_bits(rb, K, n, pos);
+    unsigned long long bit[kOrderMaxOffsets];
+    const int bits = key_bits(rb, K, n, bit);
     const unsigned *known = table == rb.nbr ? rb.masks : nullptr;
-    st = K <= 32 ? build<unsigned, 1>(table, known, n, K, pos, bits, o, stream)
-                 : build<unsigned long long, 4>(table, known, n, K, pos, bits, o, stream);
+    st = K <= 32 ? build<unsigned, 1>(table, known, n, K, bit, bits, o, stream)
+                 : build<unsigned long long, 4>(table, known, n, K, bit, bits, o, stream);
   }
   if (st != SCN_OK) {
     free_row_order(o, stream);
