@@ -12,9 +12,9 @@
 //            while the other is multiplied
 //   compute  per four planes TM + TN 128-bit loads for 4 TM TN multiply-adds (16 for 256 at 128 x 64)
 //
-// Bound by the FMA pipe on large levels.  ROWS = 32 on levels with few tiles, so that there are four times as many CTAs,
-// and with still fewer the offsets are divided over CTAs whose partial sums are added in a fixed order.  Small levels are
-// not packed at all (order null): the CTA finds its offsets by reading its rows' column of the table.
+// Bound by the FMA pipe on large levels.  On levels with few tiles the offsets are divided over CTAs whose partial
+// sums are added in a fixed order.  Small levels are not packed (order null, ROWS = 32): the CTA finds its offsets by
+// reading its rows' column of the table.
 #include <stdlib.h>
 
 #include <algorithm>
@@ -270,8 +270,8 @@ bool conv_fma_supported(const float *in, const float *out, const float *weight, 
          ((uintptr_t)in | (uintptr_t)out | (uintptr_t)weight | (uintptr_t)bias) % 16 == 0;
 }
 
-// Below this many rows the rows are not packed: the levels are bound by latency, and the packing is launches of its own.
-bool conv_fma_wants_order(long long n_out) { return n_out >= 8192; }
+// Below this many rows the rows are not packed: a layer takes about as long as the packing's launch.
+bool conv_fma_wants_order(long long n_out) { return n_out >= 2048; }
 
 // out [n_out, cout] = act((bias + sum_k in[table[k][.]] @ W[k]) * bn_scale + bn_shift); `ord` null: unpacked rows
 int conv_forward_fma(const float *in, long long n_in, float *out, long long n_out, const float *weight, const float *bias,
@@ -297,11 +297,12 @@ int conv_forward_fma(const float *in, long long n_in, float *out, long long n_ou
   P.cin = cin;
   P.cout = cout;
   P.flags = flags;
-  // 64 planes per CTA unless that leaves half of them unused; 128 rows once they fill the SMs twice over, 32 below; then
-  // the offsets over as many CTAs as still leave each about four steps
+  // 64 planes per CTA unless that leaves half of them unused; 128 rows where they are packed (16 shared-memory loads for
+  // 256 multiply-adds instead of 8 for 64), 32 otherwise; then the offsets over as many CTAs as still leave each about
+  // four steps
   const int bn = cout <= 16 ? 16 : cout <= 32 || (cout % 64 != 0 && cout % 64 <= 32 && cout < 128) ? 32 : 64;
   const long long cols = ceil_div(cout, bn);
-  const int rows = ord && ceil_div(n_out, 128) * cols >= 2 * 148 ? 128 : 32;
+  const int rows = ord ? 128 : 32;
   P.n_pos = ord ? ord->n_tiles * kOrderTile : ceil_div(n_out, 32) * 32;
   const long long ctas = P.n_pos / rows * cols;
   const int steps = (int)(K * ceil_div(cin, kChunk));
