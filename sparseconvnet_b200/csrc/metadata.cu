@@ -650,7 +650,9 @@ k_submanifold_rules(KeyLayout L, HashTable T, const unsigned long long *__restri
     sh_count[kk - k0] = 0;
   }
   __syncthreads();
-  long long site = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  // at most a few blocks per SM, each over several runs of sites: the counts below are atomics on K addresses per block
+  for (long long site0 = (long long)blockIdx.x * blockDim.x; site0 < n; site0 += (long long)gridDim.x * blockDim.x) {
+  const long long site = site0 + threadIdx.x;
   bool active = site < n;
   unsigned long long key = active ? row_keys[site] : kEmptyKey;
   active = active && (key != kEmptyKey);  // blank key: overwritten duplicate, in no map
@@ -690,6 +692,7 @@ k_submanifold_rules(KeyLayout L, HashTable T, const unsigned long long *__restri
     if ((threadIdx.x & 31) == 0 && hits) atomicAdd(&sh_count[kk - k0], __popc(hits));
   }
   if (masks && bits) atomicOr(&masks[site * mask_words + word], bits);
+  }
   __syncthreads();
   for (int kk = k0 + threadIdx.x; kk < k1; kk += blockDim.x)
     if (sh_count[kk - k0]) {
@@ -766,7 +769,7 @@ int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
     int k_chunk = (int)ceil_div(k_end, want_y);
     int gy = (int)ceil_div(k_end, k_chunk);
     size_t smem = (size_t)k_chunk * (sizeof(long long) + sizeof(int) + md->dim);
-    SCN_LAUNCH(k_submanifold_rules, dim3((unsigned)bx, (unsigned)gy), threads, smem, stream, g->layout, g->table, g->row_keys, n, (int)K, F, k_chunk, rb.nbr, rb.counts_dev, mirrored ? 1 : 0, rb.masks, words, ticket_dev(rb));
+    SCN_LAUNCH(k_submanifold_rules, dim3((unsigned)std::min<long long>(bx, 148 * 16), (unsigned)gy), threads, smem, stream, g->layout, g->table, g->row_keys, n, (int)K, F, k_chunk, rb.nbr, rb.counts_dev, mirrored ? 1 : 0, rb.masks, words, ticket_dev(rb));
     SCN_CUDA_CHECK(cudaGetLastError());
   }
   rb.built = true;
@@ -849,42 +852,49 @@ __global__ void k_strided_insert(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Ha
   slot_of[id] = __shfl_sync(peers, s_out, leader);
 }
 
-__device__ __forceinline__ void strided_fill_one(const KeyLayout &Lin, const FilterDesc &F, const Slot *__restrict__ slots,
-                                                 const unsigned long long *__restrict__ in_keys,
-                                                 const int *__restrict__ slot_of, long long n_in, long long n_out,
-                                                 const int *__restrict__ n_out_dev, long long capacity,
-                                                 int *__restrict__ nbr, unsigned long long *counts) {
-  long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= n_in * F.tmax) return;
-  int s = slot_of[id];
-  if (s < 0) return;
-  if (n_out_dev) {  // inside a chain: the level's row count is on the device only
-    n_out = *n_out_dev;
-    if (n_out > capacity) return;  // the level overflowed its arrays and will be rebuilt
-  }
-  long long i = id / F.tmax;
-  int t = (int)(id % F.tmax);
-  int x[kMaxDim], o[kMaxDim], b, k;
-  unpack_key(Lin, in_keys[i], x, b);
-  strided_target(Lin, F, x, t, o, k);
-  // one read of the slot per group of lanes that share it
-  const unsigned same = __match_any_sync(__activemask(), s);
-  const int first = __ffs(same) - 1;
-  int orow = ((int)(threadIdx.x & 31) == first) ? slots[s].row : 0;
-  orow = __shfl_sync(same, orow, first);
-  nbr[(long long)k * n_out + orow] = (int)i;
-  // one counter update per distinct offset in the warp
-  unsigned peers = __match_any_sync(__activemask(), k);
-  if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&counts[k], (unsigned long long)__popc(peers));
-}
-
-__global__ void k_strided_fill(KeyLayout Lin, FilterDesc F, const Slot *__restrict__ slots,
-                               const unsigned long long *__restrict__ in_keys,
-                               const int *__restrict__ slot_of, long long n_in, long long n_out,
-                               const int *__restrict__ n_out_dev, long long capacity,
-                               int *__restrict__ nbr, unsigned long long *counts, int K,
-                               volatile unsigned long long *counts_host) {
-  strided_fill_one(Lin, F, slots, in_keys, slot_of, n_in, n_out, n_out_dev, capacity, nbr, counts);
+// A few blocks per SM, each over several runs of candidates, with the rule counts of up to kFillCounts offsets summed in
+// shared memory first: counted in global memory per warp, a 3 / 2 layer's eight rules per candidate were 370 us of
+// atomics on 27 addresses for 184 k sites.
+constexpr int kFillCounts = 1024;
+__global__ void __launch_bounds__(256)
+k_strided_fill(KeyLayout Lin, FilterDesc F, const Slot *__restrict__ slots, const unsigned long long *__restrict__ in_keys,
+               const int *__restrict__ slot_of, long long n_in, long long n_out, const int *__restrict__ n_out_dev,
+               long long capacity, int *__restrict__ nbr, unsigned long long *counts, int K,
+               volatile unsigned long long *counts_host) {
+  __shared__ int sh_count[kFillCounts];
+  const bool shared = K <= kFillCounts;
+  if (shared)
+    for (int k = threadIdx.x; k < K; k += blockDim.x) sh_count[k] = 0;
+  __syncthreads();
+  if (n_out_dev) n_out = *n_out_dev;  // inside a chain: the level's row count is on the device only
+  const long long n_ids = n_in * F.tmax;
+  if (n_out <= capacity)  // otherwise the level overflowed its arrays and will be rebuilt
+    for (long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < n_ids; id += (long long)gridDim.x * blockDim.x) {
+      const int s = slot_of[id];
+      if (s < 0) continue;
+      const long long i = id / F.tmax;
+      const int t = (int)(id % F.tmax);
+      int x[kMaxDim], o[kMaxDim], b, k;
+      unpack_key(Lin, in_keys[i], x, b);
+      strided_target(Lin, F, x, t, o, k);
+      // one read of the slot per group of lanes that share it
+      const unsigned act = __activemask();
+      const unsigned same = __match_any_sync(act, s);
+      const int first = __ffs(same) - 1;
+      int orow = ((int)(threadIdx.x & 31) == first) ? slots[s].row : 0;
+      orow = __shfl_sync(same, orow, first);
+      nbr[(long long)k * n_out + orow] = (int)i;
+      // one counter update per distinct offset in the warp
+      const unsigned peers = __match_any_sync(act, k);
+      if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) {
+        if (shared) atomicAdd(&sh_count[k], __popc(peers));
+        else atomicAdd(&counts[k], (unsigned long long)__popc(peers));
+      }
+    }
+  __syncthreads();
+  if (shared)
+    for (int k = threadIdx.x; k < K; k += blockDim.x)
+      if (sh_count[k]) atomicAdd(&counts[k], (unsigned long long)sh_count[k]);
   post_counts(counts, K, counts_host);
 }
 
@@ -995,7 +1005,7 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
     unsigned blocks = (unsigned)ceil_div(n_ids, threads);
     const long long n_slots = 2 * (long long)gout.table.n_buckets;
     SCN_LAUNCH(k_number_slots, (unsigned)ceil_div(n_slots, threads), threads, 0, stream, gout.table.slots, n_slots, rank, n_out, md->flags_dev, gout.row_keys);
-    SCN_LAUNCH(k_strided_fill, blocks, threads, 0, stream, gin->layout, F, gout.table.slots, gin->row_keys, slot_of, n_in, n_out, nullptr, n_out, rb.nbr, rb.counts_dev, (int)K, ticket_dev(rb));
+    SCN_LAUNCH(k_strided_fill, std::min(blocks, 148u * 8u), threads, 0, stream, gin->layout, F, gout.table.slots, gin->row_keys, slot_of, n_in, n_out, nullptr, n_out, rb.nbr, rb.counts_dev, (int)K, ticket_dev(rb));
     SCN_CUDA_CHECK(cudaGetLastError());
   }
   device_free(slot_of, stream);
@@ -1099,7 +1109,7 @@ static int chain_enqueue(scn_metadata *md, const Grid *gin, std::vector<ChainLev
       SCN_TRY(exclusive_scan_i32(lv.flag, lv.rank, n_ids, n_out_dev, stream, lv.scan));
       const long long n_slots = 2 * (long long)lv.gout.table.n_buckets;
       SCN_LAUNCH(k_number_slots, (unsigned)ceil_div(n_slots, threads), threads, 0, stream, lv.gout.table.slots, n_slots, lv.rank, lv.cap_out, level_flags, lv.gout.row_keys);
-      SCN_LAUNCH(k_strided_fill, blocks, threads, 0, stream, Lin, lv.F, lv.gout.table.slots, in_keys, lv.slot_of, lv.bound_in, 0ll, n_out_dev, lv.cap_out, lv.rb.nbr, lv.rb.counts_dev, (int)lv.K, ticket_dev(lv.rb));
+      SCN_LAUNCH(k_strided_fill, std::min(blocks, 148u * 8u), threads, 0, stream, Lin, lv.F, lv.gout.table.slots, in_keys, lv.slot_of, lv.bound_in, 0ll, n_out_dev, lv.cap_out, lv.rb.nbr, lv.rb.counts_dev, (int)lv.K, ticket_dev(lv.rb));
       SCN_CUDA_CHECK(cudaGetLastError());
     }
     in_keys = lv.gout.row_keys;
