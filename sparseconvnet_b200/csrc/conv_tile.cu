@@ -29,8 +29,9 @@
 //               cycles against the 512 the copies need.)
 //   weights     one thread: one bulk copy per step
 //   MMA         one thread
-//   epilogue    4 warps: tcgen05.ld -> bias -> optional BatchNorm scale / shift / leaky ReLU -> 16-byte stores,
-//               one thread per row (a row's columns are contiguous)
+//   epilogue    4 warps: tcgen05.ld (a lane holds a row) -> shared memory, 16 planes at a time -> bias -> optional
+//               BatchNorm scale / shift / leaky ReLU -> 16-byte stores, four lanes per row.  (Stored straight from the TMEM
+//               lanes every instruction touched 32 lines: a fifth of the cycles in which the gather could have issued.)
 //
 // With fewer tiles than SMs the offsets of a tile are divided over n_split items whose partial sums are added in a
 // fixed order (k_tile_sum).
@@ -53,8 +54,9 @@ constexpr int kRows = kOrderTile;  // rows of a tile = MMA M
 constexpr int kProdWarps = 8;
 constexpr int kEpi0 = kProdWarps, kMma = kProdWarps + 4, kWgt = kMma + 1, kEntries = kMma + 2;
 constexpr int kThreads = (kProdWarps + 7) * 32;
-constexpr int kSlots = 16;      // offsets the scheduler runs ahead
+constexpr int kSlots = 8;       // offsets the entries run ahead; at least kProdWarps (the slots that end the work)
 constexpr int kMaxStages = 12;
+constexpr int kEpiBytes = 32 * 64;  // per epilogue warp: 32 rows x 16 planes on their way from TMEM lanes to whole lines
 
 struct TileParams {
   const unsigned char *in_split;  // split rows: per slice [SP h | SP m] (three-term) or [SP h]
@@ -208,7 +210,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
   const unsigned smem0 = smem_u32(smem);
   unsigned char *tail = smem + (size_t)P.n_stages * stage_bytes;
   int *entries = reinterpret_cast<int *>(tail);  // [kSlots][128] input row of every tile row, or -1
-  Ctl &C = *reinterpret_cast<Ctl *>(tail + sizeof(int) * kSlots * kRows);
+  unsigned char *epi = tail + sizeof(int) * kSlots * kRows;
+  Ctl &C = *reinterpret_cast<Ctl *>(epi + 4 * kEpiBytes);
   const bool joint = TERMS == 3 && P.coutp <= 64;  // [W_h | W_m] as one operand
   const int dcols = ((joint ? 2 : 1) * P.coutp + 31) & ~31;
   const int n_acc = min(4, P.tmem_cols / dcols);
@@ -436,7 +439,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
       }
       const int filled = slot;
       // every producer warp finds its next step in a slot that ends it
-      for (int i = 0; i <= (kProdWarps + P.n_slices - 1) / P.n_slices && ok; ++i, ++slot) {
+      const int ends = (min(kProdWarps, P.n_stages) - 1) / P.n_slices + 1;
+      for (int i = 0; i < ends && ok; ++i, ++slot) {
         const int si = slot % kSlots;
         if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1)) {
           ok = false;
@@ -457,6 +461,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     // ==================================== epilogue ==============================================
     const int quad = warp & 3;
     const int nc = P.cout;
+    float4 *my_epi = reinterpret_cast<float4 *>(epi + quad * kEpiBytes);
     int buf = 0, buf_par = 0;
     for (long long it = 0; it < my_items; ++it) {
       const long long item = blockIdx.x + it * gridDim.x, t = item_tile(P, item);
@@ -470,39 +475,52 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
         break;
       }
       tc_fence_after();
-      float *dst = P.n_split > 1 ? P.out + ((long long)part * P.n_tiles * kRows + t * kRows + quad * 32 + lane) * nc
-                                 : P.out + (long long)orow * nc;
       const unsigned base = tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(buf * dcols);
+      // where rows lane / 4, + 8, + 16, + 24 of the warp go, and this lane's four planes of them
+      long long at[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = __shfl_sync(0xffffffffu, orow, i * 8 + (lane >> 2));
+        at[i] = r < 0 ? -1 : (P.n_split > 1 ? ((long long)part * P.n_tiles + t) * kRows + quad * 32 + i * 8 + (lane >> 2) : r) * nc + (lane & 3) * 4;
+      }
       for (int c0 = 0; c0 < nc; c0 += 16) {
         unsigned a[16], b[16];
         tmem_ld16_nowait(base + c0, a);
         if (joint) tmem_ld16_nowait(base + P.coutp + c0, b);
         tmem_wait_ld();
-        if (orow >= 0) {  // (no early way out of this iteration: the loads above need the whole warp)
 #pragma unroll
-          for (int e = 0; e < 16; e += 4) {
-            if (c0 + e >= nc) break;
-            float4 v;
-            v.x = __uint_as_float(a[e]), v.y = __uint_as_float(a[e + 1]), v.z = __uint_as_float(a[e + 2]), v.w = __uint_as_float(a[e + 3]);
-            if (joint) {
-              v.x += __uint_as_float(b[e]), v.y += __uint_as_float(b[e + 1]);
-              v.z += __uint_as_float(b[e + 2]), v.w += __uint_as_float(b[e + 3]);
+        for (int e = 0; e < 16; e += 4) {
+          float4 v;
+          v.x = __uint_as_float(a[e]), v.y = __uint_as_float(a[e + 1]), v.z = __uint_as_float(a[e + 2]), v.w = __uint_as_float(a[e + 3]);
+          if (joint) {
+            v.x += __uint_as_float(b[e]), v.y += __uint_as_float(b[e + 1]);
+            v.z += __uint_as_float(b[e + 2]), v.w += __uint_as_float(b[e + 3]);
+          }
+          my_epi[lane * 4 + ((e >> 2) ^ ((lane >> 1) & 3))] = v;
+        }
+        __syncwarp();
+        const int c = c0 + (lane & 3) * 4;
+        if (c < nc) {
+          float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), sc = bias, sh = bias;
+          const bool finish = P.n_split == 1;
+          if (finish && P.bias) bias = __ldg(reinterpret_cast<const float4 *>(P.bias + c));
+          if (finish && P.bn_scale) {
+            sc = __ldg(reinterpret_cast<const float4 *>(P.bn_scale + c));
+            sh = __ldg(reinterpret_cast<const float4 *>(P.bn_shift + c));
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int row = i * 8 + (lane >> 2);
+            float4 v = my_epi[row * 4 + ((lane & 3) ^ ((row >> 1) & 3))];
+            if (at[i] < 0) continue;
+            if (finish && P.bias) v.x += bias.x, v.y += bias.y, v.z += bias.z, v.w += bias.w;
+            if (finish && P.bn_scale) {  // separate multiply and add, as the stand-alone BatchNorm kernel rounds them
+              v.x = __fadd_rn(__fmul_rn(v.x, sc.x), sh.x), v.y = __fadd_rn(__fmul_rn(v.y, sc.y), sh.y);
+              v.z = __fadd_rn(__fmul_rn(v.z, sc.z), sh.z), v.w = __fadd_rn(__fmul_rn(v.w, sc.w), sh.w);
+              v.x *= v.x > 0.f ? 1.f : P.leak, v.y *= v.y > 0.f ? 1.f : P.leak;
+              v.z *= v.z > 0.f ? 1.f : P.leak, v.w *= v.w > 0.f ? 1.f : P.leak;
             }
-            if (P.n_split == 1) {
-              if (P.bias) {
-                const float4 b4 = __ldg(reinterpret_cast<const float4 *>(P.bias + c0 + e));
-                v.x += b4.x, v.y += b4.y, v.z += b4.z, v.w += b4.w;
-              }
-              if (P.bn_scale) {  // separate multiply and add, as the stand-alone BatchNorm kernel rounds them
-                const float4 sc = __ldg(reinterpret_cast<const float4 *>(P.bn_scale + c0 + e));
-                const float4 sh = __ldg(reinterpret_cast<const float4 *>(P.bn_shift + c0 + e));
-                v.x = __fadd_rn(__fmul_rn(v.x, sc.x), sh.x), v.y = __fadd_rn(__fmul_rn(v.y, sc.y), sh.y);
-                v.z = __fadd_rn(__fmul_rn(v.z, sc.z), sh.z), v.w = __fadd_rn(__fmul_rn(v.w, sc.w), sh.w);
-                v.x *= v.x > 0.f ? 1.f : P.leak, v.y *= v.y > 0.f ? 1.f : P.leak;
-                v.z *= v.z > 0.f ? 1.f : P.leak, v.w *= v.w > 0.f ? 1.f : P.leak;
-              }
-            }
-            *reinterpret_cast<float4 *>(dst + c0 + e) = v;
+            *reinterpret_cast<float4 *>(P.out + at[i] + c0) = v;
           }
         }
         __syncwarp();
@@ -624,7 +642,7 @@ int launch_tile(TileParams &P, int n_sm, int dev, cudaStream_t stream) {
     configured[dev].store(true);
   }
   const size_t stage = Shape::A_BYTES + ((size_t)P.coutp * SP * 2 * Shape::PARTS + 1023) / 1024 * 1024;
-  const size_t fixed = sizeof(int) * kSlots * kRows + sizeof(Ctl);
+  const size_t fixed = sizeof(int) * kSlots * kRows + 4 * kEpiBytes + sizeof(Ctl);
   const int dcols = ((TERMS == 3 && P.coutp <= 64 ? 2 : 1) * P.coutp + 31) & ~31;
   // Two CTAs per SM, each with half of the shared memory and of the TMEM columns, where that leaves four stages and two
   // accumulators: one CTA's issue overhead and epilogue run beside the other's tensor instructions.
