@@ -27,23 +27,44 @@ def _keeps_sites(m):
     return False
 
 
-def _chain_ahead(steps):
-    """The first downsampling Convolution that announces further levels (``levels_below > 1``) and is reached
-    from the start of `steps` through modules that keep the sites and the spatial size -- so that its input grid
-    is the grid of the tensor that enters `steps` -- looking into the branches of a ConcatTable.  None if there
-    is none."""
+def _window(m):
+    """(size, stride) of a module that goes one level down, None for any other."""
     from . import layers
-    for m in steps:
-        if isinstance(m, layers.Convolution):
-            return m if m.levels_below > 1 else None
-        if type(m) is ConcatTable:
-            for branch in m._modules.values():
-                found = _chain_ahead(_flatten(branch, []) if type(branch) is Sequential else [branch])
-                if found is not None:
-                    return found
-        if not _keeps_sites(m):
-            return None
+    if isinstance(m, layers.Convolution):
+        return m.filter_size, m.filter_stride
+    if isinstance(m, (layers.MaxPooling, layers.AveragePooling)):
+        return m.pool_size, m.pool_stride
     return None
+
+
+def _chain_ahead(steps):
+    """(size, stride, levels) of the first run of levels below `steps` that can be built together: the first module
+    that goes down, reached from the start of `steps` through modules that keep the sites and the spatial size -- so
+    that its input grid is the grid of the tensor that enters `steps` -- looking into the branches of a ConcatTable,
+    and the modules behind it that go down by the same window, up to the first that does something else.  A Convolution
+    that knows how far the network goes down (``levels_below``) ends the count.  None if there are not two levels."""
+    found, levels = None, 0
+    for m in steps:
+        window = _window(m)
+        if window is not None:
+            if found is None:
+                found = window
+            elif not (torch.equal(found[0], window[0]) and torch.equal(found[1], window[1])):
+                break
+            below = getattr(m, "levels_below", 1)
+            levels += below
+            if below > 1:
+                break
+        elif type(m) is ConcatTable and not _keeps_sites(m):
+            for branch in m._modules.values():
+                ahead = _chain_ahead(_flatten(branch, []) if type(branch) is Sequential else [branch])
+                if ahead is not None and (found is None or (torch.equal(found[0], ahead[0]) and torch.equal(found[1], ahead[1]))):
+                    found, levels = ahead[:2], levels + ahead[2]
+                    break
+            break
+        elif not _keeps_sites(m):
+            break
+    return None if levels < 2 else (found[0], found[1], levels)
 
 
 class Sequential(torch.nn.Sequential):
@@ -57,26 +78,25 @@ class Sequential(torch.nn.Sequential):
     followed by a BatchNormalization alone is one pass without the concatenation.
 
     And one look ahead (`Sequential.prefetch_rulebooks = False` turns it off): the first Sequential that sees a
-    tensor of a new Metadata looks for the encoder's first downsampling Convolution behind the layers that keep
-    the sites (the builders mark it with the number of levels below it) and has the grids and rulebooks of all
-    those levels started on the library's side stream (SCN.strided_chain_start).  They are built while the
-    layers of the finest level run, and the Convolution, when its turn comes, finds them finished instead of
-    building them and waiting with an empty stream."""
+    tensor of a new Metadata looks for the first layer that goes down -- a Convolution, which the builders mark with
+    the number of levels below it, or a pooling -- behind the layers that keep the sites, counts the levels that go
+    down by the same window, and has the grids and rulebooks of all of them started on the library's side stream
+    (SCN.strided_chain_start).  They are built while the layers of the finest level run, and the layer, when its turn
+    comes, finds them finished instead of building its own and waiting with an empty stream."""
     fuse = True
     prefetch_rulebooks = True
 
     def forward(self, input):
         from . import layers
         steps = _flatten(self, [])
-        if (Sequential.prefetch_rulebooks and isinstance(input, SparseConvNetTensor) and input.features.is_cuda
-                and not getattr(input.metadata, "chain_looked_for", True)):
-            input.metadata.chain_looked_for = True  # one look per Metadata, by the outermost container
-            conv = _chain_ahead(steps)
-            if conv is not None:
-                layers.SCN.strided_chain_start(input.metadata, input.spatial_size, conv.filter_size, conv.filter_stride,
-                                               conv.levels_below, input.features.device)
         i, n = 0, len(steps)
         while i < n:
+            if (Sequential.prefetch_rulebooks and isinstance(input, SparseConvNetTensor)
+                    and not getattr(input.metadata, "chain_looked_for", True) and input.features.is_cuda):
+                input.metadata.chain_looked_for = True  # one look per Metadata, by the outermost container
+                ahead = _chain_ahead(steps[i:])
+                if ahead is not None:
+                    layers.SCN.strided_chain_start(input.metadata, input.spatial_size, *ahead, input.features.device)
             m = steps[i]
             nxt = steps[i + 1] if i + 1 < n else None
             if (Sequential.fuse and isinstance(m, layers._ConvBase) and isinstance(nxt, layers.BatchNormalization)

@@ -119,18 +119,37 @@ __host__ __device__ inline unsigned long long mix64(unsigned long long k) {
 }
 
 #ifdef __CUDACC__
-// Returns the slot index holding `key` (inserting it if absent) or -1 if the bounded walk
-// gave up.
-__device__ inline long long hash_insert(const HashTable &T, unsigned long long key) {
-  unsigned long long mask = T.n_buckets - 1;
+// The slot of `key`, claimed if it is not there yet, or -1 if the bounded walk gave up.  LAST: the slot's row becomes the
+// largest id that named the key; otherwise its aux becomes the smallest.  A free slot is claimed and its id written by one
+// 16-byte compare-and-swap (a compare-and-swap on the key and an atomic on the id were two trips to L2).  LOOK: read the
+// slot first, where most calls find their key there, named by a smaller id, and need no atomic at all.
+template <bool LAST, bool LOOK>
+__device__ inline long long hash_claim(const HashTable &T, unsigned long long key, unsigned id) {
+  const unsigned long long mask = T.n_buckets - 1;
   unsigned long long b = mix64(key) & mask;
-  unsigned long long limit = T.n_buckets < 4096 ? T.n_buckets : 4096;
+  const unsigned long long limit = T.n_buckets < 4096 ? T.n_buckets : 4096;
+  const Slot vacant{kEmptyKey, -1, 0xFFFFFFFFu}, mine{key, LAST ? (int)id : -1, LAST ? 0xFFFFFFFFu : id};
   for (unsigned long long p = 0; p < limit; ++p) {
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      unsigned long long idx = 2 * b + s;
-      unsigned long long prev = atomicCAS(&T.slots[idx].key, kEmptyKey, key);
-      if (prev == kEmptyKey || prev == key) return (long long)idx;
+      Slot *at = T.slots + 2 * b + s;
+      Slot was = vacant;
+      if (LOOK) {
+        const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(at));
+        was.key = ((unsigned long long)v.y << 32) | v.x;
+        was.row = (int)v.z;
+        was.aux = v.w;
+      }
+      if (was.key == kEmptyKey) was = atomicCAS(at, vacant, mine);
+      if (was.key == kEmptyKey) return (long long)(at - T.slots);
+      if (was.key == key) {
+        if (LAST) {
+          if (was.row < (int)id) atomicMax(&at->row, (int)id);
+        } else if (was.aux > id) {
+          atomicMin(&at->aux, id);
+        }
+        return (long long)(at - T.slots);
+      }
     }
     b = (b + 1) & mask;
   }
@@ -200,8 +219,6 @@ int device_free(void *p, cudaStream_t stream);
 
 // Exclusive prefix sum of n int32 values (out may alias in).  total_dev (may be null)
 // receives the sum of all inputs as int32.
-int exclusive_scan_i32(const int *in, int *out, long long n, int *total_dev, cudaStream_t stream,
-                       int *scratch = nullptr);
-size_t exclusive_scan_scratch_ints(long long n);  // ints of caller-owned scratch that make the scan allocation-free
+int exclusive_scan_i32(const int *in, int *out, long long n, int *total_dev, cudaStream_t stream);
 
 }  // namespace scn

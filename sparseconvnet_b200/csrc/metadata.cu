@@ -79,9 +79,47 @@ static int alloc_table(HashTable &T, long long expected_sites, cudaStream_t stre
   unsigned long long slots = next_pow2((unsigned long long)std::max<long long>(64, 2 * expected_sites));
   SCN_REQUIRE(slots < (1ull << 31), SCN_ERR_UNSUPPORTED, "site table too large (%llu slots)", slots);
   T.n_buckets = slots / 2;
-  SCN_TRY(device_alloc((void **)&T.slots, slots * sizeof(Slot), stream));
-  // key = all ones (free), row = -1, aux = 0xFFFFFFFF
-  SCN_CUDA_CHECK(cudaMemsetAsync(T.slots, 0xFF, slots * sizeof(Slot), stream));
+  return device_alloc((void **)&T.slots, slots * sizeof(Slot), stream);
+}
+
+// ---- what the builders start from ------------------------------------------------------------------
+// Site tables and rule tables all ones (a free key, no row), counters zero: up to kMaxFills arrays in ONE launch, for a
+// whole chain of levels at once.  (One memset each was three calls of 3 to 10 us on the host per level.)
+constexpr int kMaxFills = 48;
+struct Fills {
+  int *p[kMaxFills];
+  long long n[kMaxFills];  // 4-byte words
+  unsigned ones;           // no: zeros
+  unsigned ones_hi;
+  int count;
+};
+static void fill_add(Fills &f, void *p, size_t bytes, bool ones) {
+  if (!bytes) return;
+  f.p[f.count] = (int *)p;
+  f.n[f.count] = (long long)(bytes / 4);
+  if (ones) (f.count < 32 ? f.ones : f.ones_hi) |= 1u << (f.count & 31);
+  ++f.count;
+}
+
+__global__ void __launch_bounds__(256) k_fill(const __grid_constant__ Fills f) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  for (int a = 0; a < f.count; ++a) {
+    const int v = (((a < 32 ? f.ones : f.ones_hi) >> (a & 31)) & 1u) ? -1 : 0;
+    int *p = f.p[a];
+    const long long n = f.n[a];
+    const bool wide = (uintptr_t)p % 16 == 0;
+    const long long n4 = wide ? n / 4 : 0;
+    for (long long j = i; j < n4; j += step) reinterpret_cast<int4 *>(p)[j] = make_int4(v, v, v, v);
+    for (long long j = n4 * 4 + i; j < n; j += step) p[j] = v;
+  }
+}
+
+static int fill_launch(const Fills &f, cudaStream_t stream) {
+  long long most = 0;
+  for (int a = 0; a < f.count; ++a) most = std::max(most, f.n[a]);
+  if (!most) return SCN_OK;
+  SCN_LAUNCH(k_fill, (unsigned)std::min<long long>(148 * 8, ceil_div(most, 4 * 256)), 256, 0, stream, f);
+  SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }
 
@@ -224,27 +262,74 @@ static void count_ticket_zero(Rulebook &rb) {  // nothing will be launched: no r
     for (int k = 0; k < rb.ticket->n; ++k) rb.ticket->host[k] = 0;
 }
 
-__global__ void k_post_scalars(int *flags_dev, const int *scalars_dev, volatile int *mailbox) {
+__global__ void k_post_flags(int *flags_dev, volatile int *mailbox) {
   mailbox[0] = *flags_dev;
   *flags_dev = 0;
-  if (scalars_dev)
-    for (int i = 0; i < 4; ++i) mailbox[1 + i] = scalars_dev[i];
   __threadfence_system();
 }
 
+// Where the last block of a pass leaves what the host waits for: pinned, device-mapped words.  `ready` is written last.
+constexpr int kNotPosted = INT_MIN;
+struct HostPost {
+  volatile int *ready, *flags, *total, *extra;  // each may be null
+};
+__device__ __forceinline__ void post_to_host(const HostPost &h, int *flags_dev, bool clear_flags, int total, const int *extra) {
+  if (h.flags) *h.flags = clear_flags ? atomicExch(flags_dev, 0) : *(volatile int *)flags_dev;
+  if (h.total) *h.total = total;
+  if (h.extra) *h.extra = *(const volatile int *)extra;
+  if (h.ready) {
+    __threadfence_system();
+    *h.ready = 0;
+  }
+  __threadfence_system();
+}
+
+// Waits for a post.  The word itself is looked at for a while (it arrives a few us before cudaStreamSynchronize would
+// return, and the stream may still be working on what follows); then the host sleeps on the stream.
+static inline void cpu_relax() {
+#if defined(__x86_64__)
+  asm volatile("pause");
+#elif defined(__aarch64__)
+  asm volatile("yield");
+#endif
+}
+static int wait_posted(const volatile int *ready, cudaStream_t stream) {
+  note_host_wait();
+  for (int i = 0; i < 20000; ++i) {
+    if (*ready != kNotPosted) {
+      std::atomic_thread_fence(std::memory_order_acquire);
+      return SCN_OK;
+    }
+    cpu_relax();
+  }
+  SCN_CUDA_CHECK(cudaStreamSynchronize(stream));
+  SCN_REQUIRE(*ready != kNotPosted, SCN_ERR_CUDA, "a site count did not arrive");
+  return SCN_OK;
+}
+
 // Reads (and clears) the device flag word; waits for the stream.
-static int fetch_flags(scn_metadata *md, cudaStream_t stream, int *flags, int *scalars4) {
+static int fetch_flags(scn_metadata *md, cudaStream_t stream, int *flags) {
   if (!md->mailbox) SCN_TRY(mailbox_acquire(&md->mailbox));
   int *mailbox_dev = nullptr;
   SCN_CUDA_CHECK(cudaHostGetDevicePointer((void **)&mailbox_dev, md->mailbox, 0));
-  SCN_LAUNCH(k_post_scalars, 1, 1, 0, stream, md->flags_dev, scalars4 ? md->scalars_dev : nullptr, mailbox_dev);
+  SCN_LAUNCH(k_post_flags, 1, 1, 0, stream, md->flags_dev, mailbox_dev);
   SCN_CUDA_CHECK(cudaGetLastError());
   note_host_wait();
   SCN_CUDA_CHECK(cudaStreamSynchronize(stream));
-  const volatile int *host = md->mailbox;
-  *flags = host[0];
-  if (scalars4)
-    for (int i = 0; i < 4; ++i) scalars4[i] = host[1 + i];
+  *flags = *(const volatile int *)md->mailbox;
+  return SCN_OK;
+}
+
+// A mailbox whose first word is "not posted", and the device's view of it: [0] ready, [1] flags, [2] total, [3] extra.
+static int post_begin(scn_metadata *md, HostPost &h) {
+  if (!md->mailbox) SCN_TRY(mailbox_acquire(&md->mailbox));
+  int *dev = nullptr;
+  SCN_CUDA_CHECK(cudaHostGetDevicePointer((void **)&dev, md->mailbox, 0));
+  *(volatile int *)md->mailbox = kNotPosted;
+  h.ready = dev;
+  h.flags = dev + 1;
+  h.total = dev + 2;
+  h.extra = dev + 3;
   return SCN_OK;
 }
 
@@ -280,7 +365,7 @@ static int flags_to_status(int flags) {
 __global__ void k_insert_input(KeyLayout L, HashTable T, const long long *__restrict__ coords,
                                long long n, int ncols, int mode, long long bl_length,
                                unsigned long long *__restrict__ row_keys, int *__restrict__ slot_of,
-                               int *flags, int *scalars) {
+                               int *flags, int *n_samples) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const long long *c = coords + i * ncols;
@@ -305,46 +390,140 @@ __global__ void k_insert_input(KeyLayout L, HashTable T, const long long *__rest
     return;
   }
   unsigned long long key = pack_key(L, x, (int)bl);
-  long long s = hash_insert(T, key);
+  const long long s = mode == 0 ? hash_claim<true, false>(T, key, (unsigned)i) : hash_claim<false, false>(T, key, (unsigned)i);
   if (s < 0) {
     atomicOr(flags, FLAG_TABLE_FULL);
     if (mode == 0) row_keys[i] = kEmptyKey;
     slot_of[i] = -1;
     return;
   }
-  // largest batch index: one atomic per warp, and none once the word already holds the value
+  // batch indices in use: one atomic per warp, and none once the word already holds the value
   {
     const unsigned peers = __activemask();
-    const int warp_max = __reduce_max_sync(peers, (int)bl);
-    if ((threadIdx.x & 31) == __ffs(peers) - 1 && warp_max > *(volatile int *)&scalars[1])
-      atomicMax(&scalars[1], warp_max);
+    const int warp_max = __reduce_max_sync(peers, (int)bl + 1);
+    if ((threadIdx.x & 31) == __ffs(peers) - 1 && warp_max > *(volatile int *)n_samples) atomicMax(n_samples, warp_max);
   }
   slot_of[i] = (int)s;
-  if (mode == 0) {
-    row_keys[i] = key;
-    atomicMax(&T.slots[s].row, (int)i);
-  } else {
-    atomicMin(&T.slots[s].aux, (unsigned)i);
-  }
+  if (mode == 0) row_keys[i] = key;
 }
 
 // Input mode 0 with repeated coordinates: the site belongs to the last row that named it.
 // Earlier rows keep their feature row but are in no map of the reference, so no rule ever
 // touches them and getSpatialLocations leaves them zero; here their key is blanked.
-__global__ void k_blank_overwritten(const Slot *__restrict__ slots, const int *__restrict__ slot_of,
-                                    long long n, unsigned long long *__restrict__ row_keys) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// Block 0 tells the host what the inserts found.
+__global__ void __launch_bounds__(256)
+k_blank_overwritten(const Slot *__restrict__ slots, const int *__restrict__ slot_of, long long n,
+                    unsigned long long *__restrict__ row_keys, int *flags, const int *n_samples, HostPost post) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) post_to_host(post, flags, true, 0, n_samples);
   if (i >= n) return;
-  int s = slot_of[i];
+  const int s = slot_of[i];
   if (s >= 0 && slots[s].row != (int)i) row_keys[i] = kEmptyKey;
 }
 
-__global__ void k_flag_first(const Slot *__restrict__ slots, const int *__restrict__ slot_of,
-                             long long n, int *__restrict__ flag) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int s = slot_of[i];
-  flag[i] = (s >= 0 && slots[s].aux == (unsigned)i) ? 1 : 0;
+// ---- row numbers in the order of first touch --------------------------------------------------------
+// A candidate (input row; pair of a site and an output it feeds) is the first of its site if the site's slot holds its
+// id.  The site's row is the number of such candidates before it: a bit per candidate, 32 of them with the count before
+// them in their run of kRankTile candidates (`words`), and the count before the run (`base`), which the block that
+// finishes last sums up.  Whoever needs a row reads the 8-byte word and the base, both in L2: no array of ranks, no flags,
+// and one pass where there were a flag pass, a scan of two or three kernels and a pass over all slots of the table.
+constexpr int kRankTile = 1024;
+
+__device__ __forceinline__ int row_of_first(const uint2 *__restrict__ words, const int *__restrict__ base, unsigned id) {
+  const uint2 w = words[id >> 5];
+  return base[id / kRankTile] + (int)w.y + __popc(w.x & ((1u << (id & 31)) - 1u));
+}
+
+// The number of input sites comes from the host (`n_in`, n_in_dev null) or, inside a chain of levels whose counts the host
+// has not seen yet, from the device, with `n_in` the bound that sized the launch and the arrays.  A level that did not
+// fit its arrays hands nothing on: it will be built again, and so will what is below it.
+__device__ __forceinline__ long long sites_here(const int *n_dev, long long bound) {
+  if (!n_dev) return bound;
+  const long long n = *n_dev;
+  return n <= bound ? n : 0;
+}
+
+__global__ void __launch_bounds__(256)
+k_first_ranks(const Slot *__restrict__ slots, const int *__restrict__ slot_of, long long n_in, const int *__restrict__ n_in_dev,
+              int per_site, uint2 *__restrict__ words, int *base, int *done, int *total_dev, int *flags, bool clear_flags,
+              const int *extra, HostPost post) {
+  __shared__ unsigned sh_bits[32];
+  __shared__ int sh_sum[8];
+  __shared__ bool last;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const long long n = sites_here(n_in_dev, n_in) * per_site, at = (long long)blockIdx.x * kRankTile;
+  if (at < n) {
+    int s[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const long long id = at + j * 256 + t;
+      s[j] = id < n ? slot_of[id] : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const unsigned id = (unsigned)(at + j * 256 + t);
+      const unsigned bits = __ballot_sync(0xffffffffu, s[j] >= 0 && slots[s[j] < 0 ? 0 : s[j]].aux == id);
+      if (lane == 0) sh_bits[j * 8 + warp] = bits;
+    }
+  } else if (t < 32) {
+    sh_bits[t] = 0;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const unsigned bits = sh_bits[lane];
+    int incl = __popc(bits);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += v;
+    }
+    if (at < n) words[(at >> 5) + lane] = make_uint2(bits, (unsigned)(incl - __popc(bits)));
+    if (lane == 31) {
+      base[blockIdx.x] = incl;
+      __threadfence();
+      last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    }
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  int run = 0;
+  for (long long b0 = 0; b0 < gridDim.x; b0 += 1024) {  // four per thread and round
+    int v[4], sum = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const long long b = b0 + t * 4 + j;
+      v[j] = b < gridDim.x ? __ldcg(base + b) : 0;
+      sum += v[j];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += u;
+    }
+    if (lane == 31) sh_sum[warp] = incl;
+    __syncthreads();
+    int before = run, all = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      if (w < warp) before += sh_sum[w];
+      all += sh_sum[w];
+    }
+    int excl = before + incl - sum;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const long long b = b0 + t * 4 + j;
+      if (b < gridDim.x) base[b] = excl;
+      excl += v[j];
+    }
+    run += all;
+    __syncthreads();
+  }
+  if (t == 0) {
+    if (total_dev) *total_dev = run;
+    post_to_host(post, flags, clear_flags, run, extra);
+  }
 }
 
 // The row that touched a site first gives the site its row number: its rank among such rows in input
@@ -354,21 +533,14 @@ __global__ void k_flag_first(const Slot *__restrict__ slots, const int *__restri
 // (the rank of the slot's first toucher, the row -> key array) is a few MB that stay in L2.  The
 // candidate-order form of this pass (a random read-modify-write of a slot per numbered site) was bound by
 // the DRAM's random-access rate: 198 us against 142 us for the inserts themselves at 1.6 M sites.
-// `capacity`: rows the output arrays were sized for; a site numbered beyond it (a chain level that
-// shrank less than guessed) is not written and raises FLAG_TABLE_FULL in `level_flags`.
-__global__ void k_number_slots(Slot *slots, long long n_slots, const int *__restrict__ rank,
-                               long long capacity, int *level_flags,
-                               unsigned long long *__restrict__ row_keys) {
+__global__ void k_number_slots(Slot *slots, long long n_slots, const uint2 *__restrict__ words,
+                               const int *__restrict__ base, unsigned long long *__restrict__ row_keys) {
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_slots) return;
   const uint4 v = *reinterpret_cast<const uint4 *>(slots + idx);
   const unsigned long long key = ((unsigned long long)v.y << 32) | v.x;
   if (key == kEmptyKey || v.w == 0xFFFFFFFFu) return;
-  const int r = rank[v.w];
-  if (r >= capacity) {
-    atomicOr(level_flags, FLAG_TABLE_FULL);
-    return;
-  }
+  const int r = row_of_first(words, base, v.w);
   slots[idx].row = r;
   row_keys[r] = key;
 }
@@ -437,13 +609,6 @@ __global__ void k_sort_segments(const int *__restrict__ start, long long n_sites
   }
 }
 
-__global__ void k_init_scalars(int *scalars) {
-  scalars[0] = 0;
-  scalars[1] = -1;
-  scalars[2] = 0;
-  scalars[3] = 0;
-}
-
 static void clear_input_rules(scn_metadata *md, cudaStream_t stream) {
   device_free(md->input_csr_start, stream);
   device_free(md->input_csr_rows, stream);
@@ -498,34 +663,46 @@ static int md_input_layer(scn_metadata *md, const int64_t *spatial_size, const i
 
   const int threads = 256;
   unsigned blocks = (unsigned)ceil_div(std::max<int64_t>(n, 1), threads);
-  SCN_LAUNCH(k_init_scalars, 1, 1, 0, stream, md->scalars_dev);
-  int *slot_of = nullptr, *flag = nullptr, *rank = nullptr, *cursor = nullptr;
+  int *n_samples = md->scalars_dev, *done = md->scalars_dev + 1;  // batch indices in use; finished blocks
+  Fills fills{};
+  fill_add(fills, g.table.slots, 2 * g.table.n_buckets * sizeof(Slot), true);
+  fill_add(fills, n_samples, 2 * sizeof(int), false);
+  SCN_TRY(fill_launch(fills, stream));
+  HostPost post{};
+  SCN_TRY(post_begin(md, post));
+  int *slot_of = nullptr, *base = nullptr, *cursor = nullptr;
+  uint2 *words = nullptr;
   SCN_TRY(device_alloc((void **)&slot_of, sizeof(int) * (size_t)std::max<int64_t>(n, 1), stream));
   if (n > 0) {
-    SCN_LAUNCH(k_insert_input, blocks, threads, 0, stream, g.layout, g.table, coords_dev, n, ncols, mode, (long long)bl_length, g.row_keys, slot_of, md->flags_dev, md->scalars_dev);
+    SCN_LAUNCH(k_insert_input, blocks, threads, 0, stream, g.layout, g.table, coords_dev, n, ncols, mode, (long long)bl_length, g.row_keys, slot_of, md->flags_dev, n_samples);
     if (mode == 0)
-      SCN_LAUNCH(k_blank_overwritten, blocks, threads, 0, stream, g.table.slots, slot_of, n, g.row_keys);
+      SCN_LAUNCH(k_blank_overwritten, blocks, threads, 0, stream, g.table.slots, slot_of, n, g.row_keys, md->flags_dev, n_samples, post);
     SCN_CUDA_CHECK(cudaGetLastError());
   }
   if (mode != 0 && n > 0) {
-    SCN_TRY(device_alloc((void **)&flag, sizeof(int) * (size_t)n, stream));
-    SCN_TRY(device_alloc((void **)&rank, sizeof(int) * (size_t)n, stream));
-    SCN_LAUNCH(k_flag_first, blocks, threads, 0, stream, g.table.slots, slot_of, n, flag);
-    SCN_TRY(exclusive_scan_i32(flag, rank, n, &md->scalars_dev[0], stream));
+    const unsigned tiles = (unsigned)ceil_div(n, kRankTile);
+    SCN_TRY(device_alloc((void **)&words, sizeof(uint2) * (kRankTile / 32) * (size_t)tiles, stream));
+    SCN_TRY(device_alloc((void **)&base, sizeof(int) * (size_t)tiles, stream));
+    SCN_LAUNCH(k_first_ranks, tiles, 256, 0, stream, g.table.slots, slot_of, (long long)n, nullptr, 1, words, base, done, nullptr, md->flags_dev, true, n_samples, post);
     const long long n_slots = 2 * (long long)g.table.n_buckets;
-    SCN_LAUNCH(k_number_slots, (unsigned)ceil_div(n_slots, threads), threads, 0, stream, g.table.slots, n_slots, rank, (long long)n, md->flags_dev, g.row_keys);
+    SCN_LAUNCH(k_number_slots, (unsigned)ceil_div(n_slots, threads), threads, 0, stream, g.table.slots, n_slots, words, base, g.row_keys);
     SCN_CUDA_CHECK(cudaGetLastError());
   }
 
   // stream-ordered: what only the kernels above read goes back before the host waits
   device_free(staged, stream);
-  device_free(flag, stream);
-  device_free(rank, stream);
+  device_free(words, stream);
+  device_free(base, stream);
   staged = nullptr;
-  flag = rank = nullptr;
-  int flags = 0, sc[4];
-  SCN_TRY(fetch_flags(md, stream, &flags, sc));
-  long long active = (mode == 0) ? n : (n > 0 ? sc[0] : 0);
+  int flags = 0, total = 0, samples = 0;
+  if (n > 0) {
+    SCN_TRY(wait_posted(md->mailbox, stream));
+    const volatile int *host = md->mailbox;
+    flags = host[1];
+    total = host[2];
+    samples = host[3];
+  }
+  long long active = (mode == 0) ? n : total;
   // Every point has a site of its own (no repeated coordinates, no empty slots): rows are numbered in
   // order of first occurrence, so row i is point i and the rule table is the identity -- the feature
   // pass is then the plain copy of mode 0 and no table is built.  Otherwise: CSR of the input rows of
@@ -561,7 +738,7 @@ static int md_input_layer(scn_metadata *md, const int64_t *spatial_size, const i
   else if (ncols == md->dim)
     g.batch_size = 1;
   else
-    g.batch_size = std::max<long long>(batch_size, (long long)sc[1] + 1);
+    g.batch_size = std::max<long long>(batch_size, samples);
   md->input_mode = identity ? 0 : mode;  // what the feature passes do (a copy when the table is the identity)
   md->input_n_rows = n;
   md->input_n_active = active;
@@ -805,26 +982,11 @@ __device__ inline bool strided_target(const KeyLayout &L, const FilterDesc &F, c
   return true;
 }
 
-// The builders of a strided rulebook take the number of input sites either from the host (`n_in`,
-// n_in_dev null) or, inside a chain of levels whose counts the host has not seen yet, from the device
-// (*n_in_dev, with `n_in` the host's upper bound that sized the launch and the arrays): candidates
-// between the real count and the bound are marked "no site" so that the scan over the bound counts
-// only real ones.
-__device__ __forceinline__ long long sites_here(const int *n_dev, long long bound) {
-  if (!n_dev) return bound;
-  long long n = *n_dev;
-  return n < bound ? n : bound;
-}
-
 __global__ void k_strided_insert(KeyLayout Lin, KeyLayout Lout, FilterDesc F, HashTable Tout,
                                  const unsigned long long *__restrict__ in_keys, long long n_in,
                                  const int *__restrict__ n_in_dev, int *__restrict__ slot_of, int *flags) {
   long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= n_in * F.tmax) return;
-  if (id >= sites_here(n_in_dev, n_in) * F.tmax) {
-    slot_of[id] = -1;
-    return;
-  }
+  if (id >= sites_here(n_in_dev, n_in) * F.tmax) return;
   long long i = id / F.tmax;
   int t = (int)(id % F.tmax);
   unsigned long long key = in_keys[i];
@@ -841,13 +1003,11 @@ __global__ void k_strided_insert(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Ha
   const int leader = __ffs(peers) - 1;
   int s_out = -1;
   if (okey != kEmptyKey && (int)(threadIdx.x & 31) == leader) {
-    long long s = hash_insert(Tout, okey);
+    const long long s = hash_claim<false, true>(Tout, okey, (unsigned)id);
     if (s < 0)
       atomicOr(flags, FLAG_TABLE_FULL);
-    else {
+    else
       s_out = (int)s;
-      atomicMin(&Tout.slots[s].aux, (unsigned)id);
-    }
   }
   slot_of[id] = __shfl_sync(peers, s_out, leader);
 }
@@ -857,17 +1017,18 @@ __global__ void k_strided_insert(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Ha
 // atomics on 27 addresses for 184 k sites.
 constexpr int kFillCounts = 1024;
 __global__ void __launch_bounds__(256)
-k_strided_fill(KeyLayout Lin, FilterDesc F, const Slot *__restrict__ slots, const unsigned long long *__restrict__ in_keys,
-               const int *__restrict__ slot_of, long long n_in, long long n_out, const int *__restrict__ n_out_dev,
-               long long capacity, int *__restrict__ nbr, unsigned long long *counts, int K,
-               volatile unsigned long long *counts_host) {
+k_strided_fill(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Slot *slots, const unsigned long long *__restrict__ in_keys,
+               const int *__restrict__ slot_of, long long n_in, const int *__restrict__ n_in_dev, long long n_out,
+               const int *__restrict__ n_out_dev, long long capacity, const uint2 *__restrict__ words,
+               const int *__restrict__ base, unsigned long long *__restrict__ row_keys, int *__restrict__ nbr,
+               unsigned long long *counts, int K, volatile unsigned long long *counts_host) {
   __shared__ int sh_count[kFillCounts];
   const bool shared = K <= kFillCounts;
   if (shared)
     for (int k = threadIdx.x; k < K; k += blockDim.x) sh_count[k] = 0;
   __syncthreads();
   if (n_out_dev) n_out = *n_out_dev;  // inside a chain: the level's row count is on the device only
-  const long long n_ids = n_in * F.tmax;
+  const long long n_ids = sites_here(n_in_dev, n_in) * F.tmax;
   if (n_out <= capacity)  // otherwise the level overflowed its arrays and will be rebuilt
     for (long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < n_ids; id += (long long)gridDim.x * blockDim.x) {
       const int s = slot_of[id];
@@ -877,11 +1038,20 @@ k_strided_fill(KeyLayout Lin, FilterDesc F, const Slot *__restrict__ slots, cons
       int x[kMaxDim], o[kMaxDim], b, k;
       unpack_key(Lin, in_keys[i], x, b);
       strided_target(Lin, F, x, t, o, k);
-      // one read of the slot per group of lanes that share it
+      // one look at the slot per group of lanes that share it; the site's first candidate, always the lowest lane of its
+      // group, leaves the row in the slot and the site's key in its row
       const unsigned act = __activemask();
       const unsigned same = __match_any_sync(act, s);
       const int first = __ffs(same) - 1;
-      int orow = ((int)(threadIdx.x & 31) == first) ? slots[s].row : 0;
+      int orow = 0;
+      if ((int)(threadIdx.x & 31) == first) {
+        const unsigned toucher = slots[s].aux;
+        orow = row_of_first(words, base, toucher);
+        if (toucher == (unsigned)id) {
+          slots[s].row = orow;
+          row_keys[orow] = pack_key(Lout, o, b);
+        }
+      }
       orow = __shfl_sync(same, orow, first);
       nbr[(long long)k * n_out + orow] = (int)i;
       // one counter update per distinct offset in the warp
@@ -950,22 +1120,31 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
   gout.batch_size = gin->batch_size;
 
   const int threads = 256;
-  int *slot_of = nullptr, *flag = nullptr, *rank = nullptr;
+  int *slot_of = nullptr, *base = nullptr;
+  uint2 *words = nullptr;
   long long n_out = 0;
   if (n_ids > 0) {
     SCN_TRY(device_alloc((void **)&slot_of, sizeof(int) * (size_t)n_ids, stream));
-    SCN_TRY(device_alloc((void **)&flag, sizeof(int) * (size_t)n_ids, stream));
-    SCN_TRY(device_alloc((void **)&rank, sizeof(int) * (size_t)n_ids, stream));
+    const unsigned tiles = (unsigned)ceil_div(n_ids, kRankTile);
+    SCN_TRY(device_alloc((void **)&words, sizeof(uint2) * (kRankTile / 32) * (size_t)tiles, stream));
+    SCN_TRY(device_alloc((void **)&base, sizeof(int) * (size_t)tiles, stream));
     unsigned blocks = (unsigned)ceil_div(n_ids, threads);
     long long expect = n_in;
     for (int attempt = 0;; ++attempt) {
       SCN_TRY(alloc_table(gout.table, expect, stream));
+      int *done = md->scalars_dev;
+      Fills fills{};
+      fill_add(fills, gout.table.slots, 2 * gout.table.n_buckets * sizeof(Slot), true);
+      fill_add(fills, done, sizeof(int), false);
+      SCN_TRY(fill_launch(fills, stream));
+      HostPost post{};
+      SCN_TRY(post_begin(md, post));
+      post.extra = nullptr;
       SCN_LAUNCH(k_strided_insert, blocks, threads, 0, stream, gin->layout, gout.layout, F, gout.table, gin->row_keys, n_in, nullptr, slot_of, md->flags_dev);
-      SCN_LAUNCH(k_flag_first, blocks, threads, 0, stream, gout.table.slots, slot_of, n_ids, flag);
-      SCN_TRY(exclusive_scan_i32(flag, rank, n_ids, &md->scalars_dev[0], stream));
+      SCN_LAUNCH(k_first_ranks, tiles, 256, 0, stream, gout.table.slots, slot_of, n_in, nullptr, F.tmax, words, base, done, nullptr, md->flags_dev, true, nullptr, post);
       SCN_CUDA_CHECK(cudaGetLastError());
-      int flags = 0, sc[4];
-      SCN_TRY(fetch_flags(md, stream, &flags, sc));
+      SCN_TRY(wait_posted(md->mailbox, stream));
+      const int flags = ((const volatile int *)md->mailbox)[1];
       if ((flags & FLAG_TABLE_FULL) && attempt < 3) {  // more coarse sites than guessed: grow
         device_free(gout.table.slots, stream);
         gout.table = HashTable{};
@@ -975,13 +1154,13 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
       int st = flags_to_status(flags);
       if (st != SCN_OK) {
         device_free(slot_of, stream);
-        device_free(flag, stream);
-        device_free(rank, stream);
+        device_free(words, stream);
+        device_free(base, stream);
         free_grid(gout, stream);
         md->strided_rules.erase(key);
         return st;
       }
-      n_out = sc[0];
+      n_out = ((const volatile int *)md->mailbox)[2];
       break;
     }
   } else {
@@ -996,21 +1175,24 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
   rb.n_out = n_out;
   size_t nbr_bytes = sizeof(int) * (size_t)(K * std::max<long long>(n_out, 1));
   SCN_TRY(device_alloc((void **)&rb.nbr, nbr_bytes, stream));
-  SCN_CUDA_CHECK(cudaMemsetAsync(rb.nbr, 0xFF, nbr_bytes, stream));
   SCN_TRY(device_alloc((void **)&rb.counts_dev, sizeof(unsigned long long) * (size_t)(K + 1), stream));
-  SCN_CUDA_CHECK(cudaMemsetAsync(rb.counts_dev, 0, sizeof(unsigned long long) * (size_t)(K + 1), stream));
   SCN_TRY(count_ticket_new(rb));
-  if (n_ids == 0) count_ticket_zero(rb);
+  Fills fills{};
+  fill_add(fills, rb.nbr, nbr_bytes, true);
+  fill_add(fills, rb.counts_dev, sizeof(unsigned long long) * (size_t)(K + 1), false);
+  if (n_ids == 0) {
+    fill_add(fills, gout.table.slots, 2 * gout.table.n_buckets * sizeof(Slot), true);
+    count_ticket_zero(rb);
+  }
+  SCN_TRY(fill_launch(fills, stream));
   if (n_ids > 0) {
     unsigned blocks = (unsigned)ceil_div(n_ids, threads);
-    const long long n_slots = 2 * (long long)gout.table.n_buckets;
-    SCN_LAUNCH(k_number_slots, (unsigned)ceil_div(n_slots, threads), threads, 0, stream, gout.table.slots, n_slots, rank, n_out, md->flags_dev, gout.row_keys);
-    SCN_LAUNCH(k_strided_fill, std::min(blocks, 148u * 8u), threads, 0, stream, gin->layout, F, gout.table.slots, gin->row_keys, slot_of, n_in, n_out, nullptr, n_out, rb.nbr, rb.counts_dev, (int)K, ticket_dev(rb));
+    SCN_LAUNCH(k_strided_fill, std::min(blocks, 148u * 8u), threads, 0, stream, gin->layout, gout.layout, F, gout.table.slots, gin->row_keys, slot_of, n_in, nullptr, n_out, nullptr, n_out, words, base, gout.row_keys, rb.nbr, rb.counts_dev, (int)K, ticket_dev(rb));
     SCN_CUDA_CHECK(cudaGetLastError());
   }
   device_free(slot_of, stream);
-  device_free(flag, stream);
-  device_free(rank, stream);
+  device_free(words, stream);
+  device_free(base, stream);
   md->grids[okey] = gout;
   rb.built = true;
   g_rulebook_builds.fetch_add(1);
@@ -1038,24 +1220,16 @@ struct ChainLevel {
   Grid gout;
   Rulebook rb;
   long long bound_in = 0, cap_out = 0;
-  int *slot_of = nullptr, *flag = nullptr, *rank = nullptr, *scan = nullptr;  // scratch of the level's build
+  int *slot_of = nullptr, *base = nullptr;  // scratch of the level's build
+  uint2 *words = nullptr;
 };
-
-__global__ void k_chain_init(int *lev, int n_ints, int n0) {
-  for (int i = threadIdx.x; i < n_ints; i += blockDim.x) lev[i] = i == 0 ? n0 : 0;
-}
-
-__global__ void k_chain_post(const int *lev, int n_ints, volatile int *mailbox) {
-  for (int i = threadIdx.x; i < n_ints; i += blockDim.x) mailbox[i] = lev[i];
-  __threadfence_system();
-}
 
 static void chain_free_level(ChainLevel &lv, bool keep_result, cudaStream_t stream) {
   device_free(lv.slot_of, stream);
-  device_free(lv.flag, stream);
-  device_free(lv.rank, stream);
-  device_free(lv.scan, stream);
-  lv.slot_of = lv.flag = lv.rank = lv.scan = nullptr;
+  device_free(lv.words, stream);
+  device_free(lv.base, stream);
+  lv.slot_of = lv.base = nullptr;
+  lv.words = nullptr;
   if (!keep_result) {
     free_grid(lv.gout, stream);
     free_rulebook(lv.rb, stream);
@@ -1070,9 +1244,9 @@ static int chain_allocate(std::vector<ChainLevel> &plan, cudaStream_t alloc_stre
   for (auto &lv : plan) {
     const size_t n_ids = (size_t)std::max<long long>(lv.bound_in * lv.F.tmax, 1), cap = (size_t)std::max<long long>(lv.cap_out, 1);
     SCN_TRY(device_alloc((void **)&lv.slot_of, sizeof(int) * n_ids, alloc_stream));
-    SCN_TRY(device_alloc((void **)&lv.flag, sizeof(int) * n_ids, alloc_stream));
-    SCN_TRY(device_alloc((void **)&lv.rank, sizeof(int) * n_ids, alloc_stream));
-    SCN_TRY(device_alloc((void **)&lv.scan, sizeof(int) * exclusive_scan_scratch_ints((long long)n_ids), alloc_stream));
+    const size_t tiles = (size_t)ceil_div((long long)n_ids, kRankTile);
+    SCN_TRY(device_alloc((void **)&lv.words, sizeof(uint2) * (kRankTile / 32) * tiles, alloc_stream));
+    SCN_TRY(device_alloc((void **)&lv.base, sizeof(int) * tiles, alloc_stream));
     const unsigned long long slots = next_pow2((unsigned long long)std::max<long long>(64, 2 * lv.cap_out));
     SCN_REQUIRE(slots < (1ull << 31), SCN_ERR_UNSUPPORTED, "site table too large (%llu slots)", slots);
     lv.gout.table.n_buckets = slots / 2;
@@ -1087,29 +1261,45 @@ static int chain_allocate(std::vector<ChainLevel> &plan, cudaStream_t alloc_stre
   return SCN_OK;
 }
 
-static int chain_enqueue(scn_metadata *md, const Grid *gin, std::vector<ChainLevel> &plan, int *lev,
+// lev: [0, L) row counts of the levels, [L, 2 L) their flags, [2 L, 3 L) finished blocks of their numbering.
+// mailbox: [0] ready, [1, L] the counts, [L + 1, 2 L] the flags -- each level's numbering posts its own, the last one
+// the ready word (the rule tables are finished a little later: the reader is ordered behind the chain's stream).
+static int chain_enqueue(scn_metadata *md, const Grid *gin, std::vector<ChainLevel> &plan, int *lev, int *mailbox,
                          cudaStream_t stream) {
   const int L = (int)plan.size(), threads = 256;
-  SCN_LAUNCH(k_chain_init, 1, 64, 0, stream, lev, 2 * L + 1, (int)gin->n_active);
+  int *mailbox_dev = nullptr;
+  SCN_CUDA_CHECK(cudaHostGetDevicePointer((void **)&mailbox_dev, mailbox, 0));
+  for (int i = 1; i <= 2 * L; ++i) ((volatile int *)mailbox)[i] = 0;
+  *(volatile int *)mailbox = plan[L - 1].bound_in > 0 ? kNotPosted : 0;
+  Fills fills{};
+  fill_add(fills, lev, sizeof(int) * 3 * L, false);
+  for (auto &lv : plan) {
+    if (fills.count + 3 > kMaxFills) {
+      SCN_TRY(fill_launch(fills, stream));
+      fills = Fills{};
+    }
+    const size_t cap = (size_t)std::max<long long>(lv.cap_out, 1);
+    fill_add(fills, lv.gout.table.slots, 2 * lv.gout.table.n_buckets * sizeof(Slot), true);
+    fill_add(fills, lv.rb.nbr, sizeof(int) * (size_t)lv.K * cap, true);
+    fill_add(fills, lv.rb.counts_dev, sizeof(unsigned long long) * (size_t)(lv.K + 1), false);
+  }
+  SCN_TRY(fill_launch(fills, stream));
   const unsigned long long *in_keys = gin->row_keys;
   KeyLayout Lin = gin->layout;
   for (int l = 0; l < L; ++l) {
     ChainLevel &lv = plan[l];
-    const size_t cap = (size_t)std::max<long long>(lv.cap_out, 1);
-    // key = all ones (free), row = -1, aux = 0xFFFFFFFF
-    SCN_CUDA_CHECK(cudaMemsetAsync(lv.gout.table.slots, 0xFF, 2 * lv.gout.table.n_buckets * sizeof(Slot), stream));
-    SCN_CUDA_CHECK(cudaMemsetAsync(lv.rb.nbr, 0xFF, sizeof(int) * (size_t)lv.K * cap, stream));
-    SCN_CUDA_CHECK(cudaMemsetAsync(lv.rb.counts_dev, 0, sizeof(unsigned long long) * (size_t)(lv.K + 1), stream));
     if (lv.bound_in > 0) {
       const long long n_ids = lv.bound_in * lv.F.tmax;  // (site, output it may feed) candidates
       const unsigned blocks = (unsigned)ceil_div(n_ids, threads);
-      int *n_in_dev = lev + l, *n_out_dev = lev + l + 1, *level_flags = lev + L + 1 + l;
+      const int *n_in_dev = l ? lev + l - 1 : nullptr;
+      int *level_flags = lev + L + l;
+      HostPost post{};
+      post.total = mailbox_dev + 1 + l;
+      post.flags = mailbox_dev + 1 + L + l;
+      post.ready = l == L - 1 ? mailbox_dev : nullptr;
       SCN_LAUNCH(k_strided_insert, blocks, threads, 0, stream, Lin, lv.gout.layout, lv.F, lv.gout.table, in_keys, lv.bound_in, n_in_dev, lv.slot_of, level_flags);
-      SCN_LAUNCH(k_flag_first, blocks, threads, 0, stream, lv.gout.table.slots, lv.slot_of, n_ids, lv.flag);
-      SCN_TRY(exclusive_scan_i32(lv.flag, lv.rank, n_ids, n_out_dev, stream, lv.scan));
-      const long long n_slots = 2 * (long long)lv.gout.table.n_buckets;
-      SCN_LAUNCH(k_number_slots, (unsigned)ceil_div(n_slots, threads), threads, 0, stream, lv.gout.table.slots, n_slots, lv.rank, lv.cap_out, level_flags, lv.gout.row_keys);
-      SCN_LAUNCH(k_strided_fill, std::min(blocks, 148u * 8u), threads, 0, stream, Lin, lv.F, lv.gout.table.slots, in_keys, lv.slot_of, lv.bound_in, 0ll, n_out_dev, lv.cap_out, lv.rb.nbr, lv.rb.counts_dev, (int)lv.K, ticket_dev(lv.rb));
+      SCN_LAUNCH(k_first_ranks, (unsigned)ceil_div(n_ids, kRankTile), 256, 0, stream, lv.gout.table.slots, lv.slot_of, lv.bound_in, n_in_dev, lv.F.tmax, lv.words, lv.base, lev + 2 * L + l, lev + l, level_flags, false, nullptr, post);
+      SCN_LAUNCH(k_strided_fill, std::min(blocks, 148u * 8u), threads, 0, stream, Lin, lv.gout.layout, lv.F, lv.gout.table.slots, in_keys, lv.slot_of, lv.bound_in, n_in_dev, 0ll, lev + l, lv.cap_out, lv.words, lv.base, lv.gout.row_keys, lv.rb.nbr, lv.rb.counts_dev, (int)lv.K, ticket_dev(lv.rb));
       SCN_CUDA_CHECK(cudaGetLastError());
     }
     in_keys = lv.gout.row_keys;
@@ -1118,7 +1308,7 @@ static int chain_enqueue(scn_metadata *md, const Grid *gin, std::vector<ChainLev
   return SCN_OK;
 }
 
-// ---- plan / launch / collect: the three parts of a chain ------------------------------------------------------
+// ---- plan / enqueue / collect: the three parts of a chain -----------------------------------------------------
 // plan: sizes, layouts and bounds of the levels below `start` that can be chained (stops at the first level that
 // is already there, does not divide, or does not fit the key)
 static void chain_plan(scn_metadata *md, const Grid *gin, const std::vector<int64_t> &start, const int64_t *filter,
@@ -1170,19 +1360,6 @@ static void chain_plan(scn_metadata *md, const Grid *gin, const std::vector<int6
     cur = lv.out_size;
     plan.push_back(std::move(lv));
   }
-}
-
-// launch: every level's kernels and the post of all counts and flags into `mailbox` (pinned, mapped), on `stream`;
-// the plan's arrays and `lev` (2 L + 1 ints) were allocated before
-static int chain_launch(scn_metadata *md, const Grid *gin, std::vector<ChainLevel> &plan, int *lev, int *mailbox,
-                        cudaStream_t stream) {
-  const int L = (int)plan.size();
-  int *mailbox_dev = nullptr;
-  SCN_CUDA_CHECK(cudaHostGetDevicePointer((void **)&mailbox_dev, mailbox, 0));
-  SCN_TRY(chain_enqueue(md, gin, plan, lev, stream));
-  SCN_LAUNCH(k_chain_post, 1, 64, 0, stream, lev, 2 * L + 1, mailbox_dev);
-  SCN_CUDA_CHECK(cudaGetLastError());
-  return SCN_OK;
 }
 
 // collect (after the host has seen the mailbox): the levels up to the first that overflowed its arrays become
@@ -1261,10 +1438,18 @@ static int chain_finalize(scn_metadata *md, cudaStream_t stream, int *n_built) {
   PendingChain *p = md->pending;
   if (!p) return SCN_OK;
   md->pending = nullptr;
-  if (cudaEventQuery(p->done) != cudaSuccess) note_host_wait();
   int st = SCN_OK;
-  if (cudaEventSynchronize(p->done) != cudaSuccess) {
-    set_error("strided chain: CUDA error while waiting for the level counts");
+  if (*(const volatile int *)p->mailbox == kNotPosted) {
+    note_host_wait();
+    if (cudaEventSynchronize(p->done) != cudaSuccess || *(const volatile int *)p->mailbox == kNotPosted) {
+      set_error("strided chain: CUDA error while waiting for the level counts");
+      st = SCN_ERR_CUDA;
+    }
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  // the counts are here, the last level's tables perhaps not yet: what follows on `stream` comes behind them
+  if (st == SCN_OK && cudaStreamWaitEvent(stream, p->done, 0) != cudaSuccess) {
+    set_error("strided chain: could not order the caller's stream behind the side stream");
     st = SCN_ERR_CUDA;
   }
   cudaEventDestroy(p->done);
@@ -1311,16 +1496,12 @@ static int build_strided_chain_from(scn_metadata *md, std::vector<int64_t> start
     if (L < 2) return SCN_OK;
     if (!md->mailbox) SCN_TRY(mailbox_acquire(&md->mailbox));
     int *lev = nullptr;
-    int st = device_alloc((void **)&lev, sizeof(int) * (2 * L + 1), stream);
+    int st = device_alloc((void **)&lev, sizeof(int) * 3 * L, stream);
     if (st == SCN_OK) st = chain_allocate(plan, stream);
-    if (st == SCN_OK) st = chain_launch(md, gin, plan, lev, md->mailbox, stream);
+    if (st == SCN_OK) st = chain_enqueue(md, gin, plan, lev, md->mailbox, stream);
     device_free(lev, stream);
     if (st == SCN_OK) {
-      note_host_wait();
-      if (cudaStreamSynchronize(stream) != cudaSuccess) {
-        set_error("strided chain: CUDA error while waiting for the level counts");
-        st = SCN_ERR_CUDA;
-      }
+      st = wait_posted(md->mailbox, stream);
     }
     if (st != SCN_OK) {
       for (auto &lv : plan) chain_free_level(lv, false, stream);
@@ -1377,7 +1558,7 @@ int start_strided_chain(scn_metadata *md, const int64_t *input_size, const int64
   cudaEvent_t ready = nullptr;
   int st = side_stream(&side);
   if (st == SCN_OK) st = mailbox_acquire(&p->mailbox);
-  if (st == SCN_OK) st = device_alloc((void **)&p->lev, sizeof(int) * (2 * p->plan.size() + 1), stream);
+  if (st == SCN_OK) st = device_alloc((void **)&p->lev, sizeof(int) * 3 * p->plan.size(), stream);
   if (st == SCN_OK) st = chain_allocate(p->plan, stream);
   if (st == SCN_OK && (cudaEventCreateWithFlags(&ready, cudaEventDisableTiming) != cudaSuccess ||
                        cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming) != cudaSuccess ||
@@ -1387,7 +1568,7 @@ int start_strided_chain(scn_metadata *md, const int64_t *input_size, const int64
   }
   bool launched = false;
   if (st == SCN_OK) {
-    st = chain_launch(md, gin, p->plan, p->lev, p->mailbox, side);
+    st = chain_enqueue(md, gin, p->plan, p->lev, p->mailbox, side);
     launched = true;  // (possibly in part)
   }
   if (st == SCN_OK && cudaEventRecord(p->done, side) != cudaSuccess) {
@@ -1627,7 +1808,7 @@ int scn_md_poll_errors(scn_metadata *md, void *stream) {
   if (!md->flags_dev) return SCN_OK;
   SCN_TRY(md_touch(md, (cudaStream_t)stream));
   int flags = 0;
-  SCN_TRY(fetch_flags(md, (cudaStream_t)stream, &flags, nullptr));
+  SCN_TRY(fetch_flags(md, (cudaStream_t)stream, &flags));
   return flags_to_status(flags);
 }
 

@@ -113,7 +113,7 @@ struct scn_metadata {
 
   int *flags_dev = nullptr;   // device word the kernels OR DeviceFlag bits into
   int *mailbox = nullptr;     // pinned, device-mapped host slot (8 ints) the waited-for integers are posted to
-  int *scalars_dev = nullptr; // small device scratch: [0] count, [1] max batch index
+  int *scalars_dev = nullptr; // small device scratch: [0] batch indices in use, [1] finished blocks
 };
 
 namespace scn {
