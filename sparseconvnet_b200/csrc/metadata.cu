@@ -362,34 +362,41 @@ static int flags_to_status(int flags) {
 // the other modes record the first row that touched the site.
 // bl_length > 0: coords are [batch, bl_length, dim] (BLInputLayer, IOLayersRules.h:134-288):
 // the sample index is i / bl_length and a point whose first coordinate is negative is empty.
+// packed (coordinates that came from the host): the checked keys, the empty key for an empty slot.
 __global__ void k_insert_input(KeyLayout L, HashTable T, const long long *__restrict__ coords,
+                               const unsigned long long *__restrict__ packed,
                                long long n, int ncols, int mode, long long bl_length,
                                unsigned long long *__restrict__ row_keys, int *__restrict__ slot_of,
                                int *flags, int *n_samples) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const long long *c = coords + i * ncols;
-  if (bl_length > 0 && c[0] < 0) {  // empty slot of the batch x length array: in no map, in no rule
+  unsigned long long key = kEmptyKey;
+  long long bl = -1;
+  if (packed) {
+    key = packed[i];
+  } else {
+    const long long *c = coords + i * ncols;
+    if (!(bl_length > 0 && c[0] < 0)) {  // otherwise an empty slot of the batch x length array: in no map, in no rule
+      int x[kMaxDim];
+      bool ok = true;
+      for (int d = 0; d < L.dim; ++d) {
+        long long v = c[d];
+        ok &= (v >= 0 && v < L.size[d]);
+        x[d] = (int)v;
+      }
+      bl = bl_length > 0 ? i / bl_length : ((ncols > L.dim) ? c[L.dim] : 0);
+      ok &= (bl >= 0 && bl < (1ll << L.batch_bits));
+      if (ok)
+        key = pack_key(L, x, (int)bl);
+      else
+        atomicOr(flags, FLAG_COORD_RANGE);
+    }
+  }
+  if (key == kEmptyKey) {
     if (mode == 0) row_keys[i] = kEmptyKey;
     slot_of[i] = -1;
     return;
   }
-  int x[kMaxDim];
-  bool ok = true;
-  for (int d = 0; d < L.dim; ++d) {
-    long long v = c[d];
-    ok &= (v >= 0 && v < L.size[d]);
-    x[d] = (int)v;
-  }
-  long long bl = bl_length > 0 ? i / bl_length : ((ncols > L.dim) ? c[L.dim] : 0);
-  ok &= (bl >= 0 && bl < (1ll << L.batch_bits));
-  if (!ok) {
-    atomicOr(flags, FLAG_COORD_RANGE);
-    if (mode == 0) row_keys[i] = kEmptyKey;
-    slot_of[i] = -1;
-    return;
-  }
-  unsigned long long key = pack_key(L, x, (int)bl);
   const long long s = mode == 0 ? hash_claim<true, false>(T, key, (unsigned)i) : hash_claim<false, false>(T, key, (unsigned)i);
   if (s < 0) {
     atomicOr(flags, FLAG_TABLE_FULL);
@@ -398,7 +405,7 @@ __global__ void k_insert_input(KeyLayout L, HashTable T, const long long *__rest
     return;
   }
   // batch indices in use: one atomic per warp, and none once the word already holds the value
-  {
+  if (!packed) {
     const unsigned peers = __activemask();
     const int warp_max = __reduce_max_sync(peers, (int)bl + 1);
     if ((threadIdx.x & 31) == __ffs(peers) - 1 && warp_max > *(volatile int *)n_samples) atomicMax(n_samples, warp_max);
@@ -629,6 +636,8 @@ static int md_clear(scn_metadata *md, cudaStream_t stream) {
   return SCN_OK;
 }
 
+constexpr int64_t kPackRows = 4 << 20;  // host coordinates: packed by the host up to here (32 MB of pinned memory)
+
 static int md_input_layer(scn_metadata *md, const int64_t *spatial_size, const int64_t *coords,
                           int coords_on_device, int64_t n, int ncols, int64_t batch_size, int mode,
                           int64_t bl_length, cudaStream_t stream, int64_t *n_active) {
@@ -654,7 +663,20 @@ static int md_input_layer(scn_metadata *md, const int64_t *spatial_size, const i
 
   const long long *coords_dev = (const long long *)coords;
   long long *staged = nullptr;
-  if (!coords_on_device && n > 0) {
+  unsigned long long *packed = nullptr, *packed_dev = nullptr;
+  size_t packed_bytes = 0;
+  int packed_samples = 0;
+  if (!coords_on_device && n > 0 && n <= kPackRows) {
+    SCN_TRY(pinned_acquire(sizeof(unsigned long long) * (size_t)n, (void **)&packed, &packed_bytes));
+    bool bad = false;
+    pack_keys(g.layout, coords_dev, n, ncols, bl_length, packed, &packed_samples, &bad);
+    if (bad) {
+      pinned_release(packed, packed_bytes);
+      free_grid(g, stream);
+      return flags_to_status(FLAG_COORD_RANGE);
+    }
+    SCN_CUDA_CHECK(cudaHostGetDevicePointer((void **)&packed_dev, packed, 0));
+  } else if (!coords_on_device && n > 0) {
     size_t bytes = sizeof(long long) * (size_t)n * ncols;
     SCN_TRY(device_alloc((void **)&staged, bytes, stream));
     SCN_CUDA_CHECK(cudaMemcpyAsync(staged, coords, bytes, cudaMemcpyHostToDevice, stream));
@@ -674,7 +696,7 @@ static int md_input_layer(scn_metadata *md, const int64_t *spatial_size, const i
   uint2 *words = nullptr;
   SCN_TRY(device_alloc((void **)&slot_of, sizeof(int) * (size_t)std::max<int64_t>(n, 1), stream));
   if (n > 0) {
-    SCN_LAUNCH(k_insert_input, blocks, threads, 0, stream, g.layout, g.table, coords_dev, n, ncols, mode, (long long)bl_length, g.row_keys, slot_of, md->flags_dev, n_samples);
+    SCN_LAUNCH(k_insert_input, blocks, threads, 0, stream, g.layout, g.table, coords_dev, packed_dev, n, ncols, mode, (long long)bl_length, g.row_keys, slot_of, md->flags_dev, n_samples);
     if (mode == 0)
       SCN_LAUNCH(k_blank_overwritten, blocks, threads, 0, stream, g.table.slots, slot_of, n, g.row_keys, md->flags_dev, n_samples, post);
     SCN_CUDA_CHECK(cudaGetLastError());
@@ -696,11 +718,13 @@ static int md_input_layer(scn_metadata *md, const int64_t *spatial_size, const i
   staged = nullptr;
   int flags = 0, total = 0, samples = 0;
   if (n > 0) {
-    SCN_TRY(wait_posted(md->mailbox, stream));
+    const int waited = wait_posted(md->mailbox, stream);
+    if (waited == SCN_OK) pinned_release(packed, packed_bytes);  // (after an error nobody knows who still reads it)
+    SCN_TRY(waited);
     const volatile int *host = md->mailbox;
     flags = host[1];
     total = host[2];
-    samples = host[3];
+    samples = packed ? packed_samples : host[3];
   }
   long long active = (mode == 0) ? n : total;
   // Every point has a site of its own (no repeated coordinates, no empty slots): rows are numbered in

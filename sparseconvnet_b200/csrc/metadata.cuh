@@ -129,4 +129,11 @@ int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
 int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int64_t *output_size,
                          const int64_t *filter_size, const int64_t *filter_stride,
                          cudaStream_t stream, Rulebook **out);
+// host_keys.cu: host coordinates as packed keys in pinned, device-mapped memory
+int pinned_acquire(size_t bytes, void **p, size_t *got);
+void pinned_release(void *p, size_t bytes);
+void pinned_trim();
+void pack_keys(const KeyLayout &L, const long long *coords, long long n, int ncols, long long bl_length,
+               unsigned long long *keys, int *samples, bool *bad);
+
 }  // namespace scn

@@ -11,6 +11,7 @@
 #include "common.cuh"
 
 namespace scn {
+void pinned_trim();  // host_keys.cu
 
 static thread_local char g_last_error[512] = "";
 static std::atomic<long long> g_launches{0};
@@ -283,6 +284,7 @@ int scn_memory_usage(uint64_t *reserved_bytes, uint64_t *used_bytes) {
 
 int scn_trim_memory(uint64_t keep_bytes) {
   using namespace scn;
+  pinned_trim();
   DeviceCache *c = nullptr;
   SCN_TRY(device_cache(&c));
   std::lock_guard<std::mutex> lock(c->mu);

@@ -1,0 +1,32 @@
+"""Coordinates on the host are checked and packed there: the same sites, rows and errors as for coordinates on the GPU."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _locations(scn, dim, coords, size, mode):
+    feats = torch.arange(coords.size(0), dtype=torch.float32, device="cuda")[:, None].contiguous()
+    out = scn.InputLayer(dim, torch.LongTensor([size] * dim), mode=mode)([coords, feats])
+    return out.get_spatial_locations().cpu(), out.features.cpu()
+
+
+# pieces of 16384 points are shared out to helper threads
+@pytest.mark.parametrize("n", [1, 16383, 16384, 16385, 100003])
+@pytest.mark.parametrize("dim,mode", [(2, 0), (3, 3), (4, 4), (1, 2)])
+def test_host_and_device_coordinates(n, dim, mode):
+    import sparseconvnet_b200 as scn
+    g = torch.Generator().manual_seed(n + dim)
+    coords = torch.randint(0, 40, (n, dim + 1), generator=g)
+    for a, b in zip(_locations(scn, dim, coords, 40, mode), _locations(scn, dim, coords.cuda(), 40, mode)):
+        assert torch.equal(a, b)  # whole numbers, and sums of whole numbers below 2^24 or means of the same rows
+
+
+@pytest.mark.parametrize("row", [0, 16384, 40000])
+@pytest.mark.parametrize("value", [-1, 40, 1 << 40])
+def test_host_coordinate_out_of_range(row, value):
+    import sparseconvnet_b200 as scn
+    coords = torch.zeros(40001, 4, dtype=torch.int64)
+    coords[row, 1] = value
+    with pytest.raises(RuntimeError, match="outside the spatial size"):
+        _locations(scn, 3, coords, 40, 3)
