@@ -32,6 +32,10 @@ int conv_forward_simt(const float *in, long long n_in, float *out, long long n_o
                       const float *bias, const int *table, int K, int cin, int cout, int groups, int *flags,
                       cudaStream_t stream);
 
+bool dweight_tile_supported(const float *in, const float *d_out, const Rulebook &rb, int cin, int cout);
+int dweight_tile(const float *in, long long rows_in, const float *d_out, long long rows_out, const Rulebook &rb,
+                 bool swap, int cin, int cout, float *d_weight, int *flags, cudaStream_t stream);
+
 // W [K][groups][cin][cout] -> [K][groups][cout][cin]; mirror_groups > 0 (the number of groups): offset k goes to K - 1 - k
 __global__ void k_transpose_weight(const float *__restrict__ w, float *__restrict__ wt, long long n_mats, int cin,
                                    int cout, int mirror_groups) {
@@ -429,7 +433,11 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
   {
     const long long n_entries = rb.n_out;  // nbr is [K][rb.n_out]
     const bool fma_only = getenv("SCN_DWEIGHT_FMA") && atoi(getenv("SCN_DWEIGHT_FMA")) != 0;
-    if (groups == 1 && !fma_only) {
+    const char *tile = getenv("SCN_DWEIGHT_TILE");
+    if (groups == 1 && !fma_only && !(tile && atoi(tile) == 0) && dweight_tile_supported(in, d_out, rb, cin, cout)) {
+      SCN_TRY(rulebook_row_order(rb, rb.nbr, rb.n_out, rb.order, stream));
+      SCN_TRY(dweight_tile(in, rows_in, d_out, rows_out, rb, transposed, cin, cout, d_weight, md->flags_dev, stream));
+    } else if (groups == 1 && !fma_only) {
       decltype(&launch_dweight<1, 1>) const by_side[3][3] = {{launch_dweight<1, 1>, launch_dweight<1, 2>, launch_dweight<1, 3>},
                                                              {launch_dweight<2, 1>, launch_dweight<2, 2>, launch_dweight<2, 3>},
                                                              {launch_dweight<3, 1>, launch_dweight<3, 2>, launch_dweight<3, 3>}};
