@@ -423,6 +423,11 @@ def InputLayer_updateOutput(m, spatial_size, input_coords, input_features, outpu
                             batch_size, mode):
     """sparseconvnet.h:163-167.  ``input_coords`` may be a CPU or CUDA LongTensor."""
     f = _features(input_features, "input_features")
+    if output_features is None:  # the result is returned
+        out = _binding.input_layer(m.handle, spatial_size, input_coords, f, int(batch_size), int(mode))
+        m.device, m.n_input_rows, m.bl_shape = f.device, f.size(0), None
+        m.chain_looked_for = m.chain_started = False
+        return out
     if input_coords.dtype != torch.int64 or input_coords.dim() != 2:
         raise RuntimeError("input_coords must be a 2-d LongTensor")
     if input_coords.size(0) != f.size(0):

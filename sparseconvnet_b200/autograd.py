@@ -2,7 +2,8 @@
 
 The modules in ``layers.py`` call the C ABI directly when no gradient is wanted (inference, the
 measured path); when gradients are enabled and an input or a parameter requires them, they go
-through the Functions here, which save what the backward entry points need.  The reference does the
+through here.  Convolutions, BatchNorm and pooling become native graph nodes (binding.cpp); the Functions below
+are their Python form, for profiled passes, and the only form of the other operators.  The reference does the
 same with one Function per operator (e.g. submanifoldConvolution.py:62-113)."""
 import torch
 
@@ -58,6 +59,10 @@ class _Convolution(torch.autograd.Function):
 
 def convolution(kind, features, weight, bias, metadata, in_size, out_size, filter_size, filter_stride):
     """Returns (output features, multiply-add count)."""
+    if SCN.Profile.active is None:
+        out, macs = SCN._binding.convolution_train(kind, metadata, metadata.handle, in_size, out_size, filter_size,
+                                                   filter_stride, features, weight, bias, SCN._precision)
+        return out, SCN._macs(macs)
     info = {}
     out = _Convolution.apply(features, weight, bias, kind, metadata, in_size, out_size, filter_size, filter_stride,
                              info)
@@ -91,6 +96,9 @@ class _BatchNorm(torch.autograd.Function):
 
 
 def batchnorm(features, weight, bias, running_mean, running_var, eps, momentum, train, leakiness):
+    if SCN.Profile.active is None:
+        return SCN._binding.batchnorm_train(features, weight, bias, running_mean, running_var, eps, momentum, train,
+                                            leakiness)
     return _BatchNorm.apply(features, weight, bias, running_mean, running_var, eps, momentum, train, leakiness)
 
 
@@ -129,6 +137,9 @@ def batchnorm_across_ranks(features, weight, bias, running_mean, running_var, ep
                                        group)
 
 
+_POOLINGS = ("max", "avg", "unpool")  # numbered as in the binding
+
+
 class _Pooling(torch.autograd.Function):
     """kind: 'max' | 'avg' | 'unpool'."""
 
@@ -161,6 +172,9 @@ class _Pooling(torch.autograd.Function):
 
 
 def pooling(kind, features, metadata, in_size, out_size, pool_size, pool_stride, drop):
+    if SCN.Profile.active is None:
+        return SCN._binding.pooling_train(_POOLINGS.index(kind), metadata, metadata.handle, in_size, out_size, pool_size,
+                                          pool_stride, features, drop)
     return _Pooling.apply(features, kind, metadata, in_size, out_size, pool_size, pool_stride, drop)
 
 

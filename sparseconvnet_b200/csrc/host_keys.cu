@@ -1,10 +1,9 @@
-// Host coordinates -> packed site keys, in pinned memory the input layer's insert kernel reads.
+// Host coordinates -> packed site keys in pinned memory.
 //
 // A point arrives as dim + 1 64-bit integers in pageable memory.  Copied as they are (32 bytes a point in 3-D, through the
 // driver's staging buffers at 12.5 GB/s, with the host held until the stream reaches the copy) 400 k points were 1.0 ms of
 // a training step's 9.5.  Here a few host threads check and pack each point into the 8 bytes the site table stores anyway
-// (bound by reading the coordinates once), and the kernel fetches those over the bus itself: a quarter of the bytes, no
-// staging, no copy call.
+// (bound by reading the coordinates once), and the insert kernel reads those across the bus: a quarter of the bytes, no staging.
 #include <stdlib.h>
 
 #include <algorithm>

@@ -55,10 +55,10 @@ class InputLayer(Module):
         batch_size = 0 if len(input) == 2 else input[2]
 
         def run(f):
-            out = f.new_empty(0)
-            SCN.InputLayer_updateOutput(output.metadata, self.spatial_size, coords.long(),
-                                        f.detach().float().contiguous(), out, batch_size, self.mode)
-            return out
+            out = None if SCN.Profile.active is None else f.new_empty(0)
+            made = SCN.InputLayer_updateOutput(output.metadata, self.spatial_size, coords.long(),
+                                               f.detach().float().contiguous(), out, batch_size, self.mode)
+            return out if out is not None else made
 
         if autograd.needs_grad(features):
             output.features = autograd.input_features(features, output.metadata, run)
