@@ -353,6 +353,34 @@ static int flags_to_status(int flags) {
   return SCN_OK;
 }
 
+// The site kernels are compiled for 1 to 4 dimensions (and once for any number): with the number of dimensions known only
+// at run time a site's coordinates lived in local memory, 5 M sectors each way beside the 6 M of the table for 400 k sites.
+template <int DIM>
+__device__ __forceinline__ void unpack_site(const KeyLayout &L, unsigned long long k, int (&x)[DIM ? DIM : kMaxDim], int &b) {
+  const int dim = DIM ? DIM : L.dim;
+#pragma unroll
+  for (int d = 0; d < dim; ++d) x[d] = (int)(k >> L.shift[d]) & (int)((1u << L.bits[d]) - 1u);
+  b = (int)(k >> L.batch_shift);
+}
+template <int DIM>
+__device__ __forceinline__ unsigned long long pack_site(const KeyLayout &L, const int (&x)[DIM ? DIM : kMaxDim], int b) {
+  const int dim = DIM ? DIM : L.dim;
+  unsigned long long k = (unsigned long long)(unsigned)b << L.batch_shift;
+#pragma unroll
+  for (int d = 0; d < dim; ++d) k |= (unsigned long long)(unsigned)x[d] << L.shift[d];
+  return k;
+}
+#define SCN_LAUNCH_DIM(dim, kernel, ...)                                     \
+  do {                                                                       \
+    switch (dim) {                                                           \
+      case 1: SCN_LAUNCH(kernel<1>, __VA_ARGS__); break;                     \
+      case 2: SCN_LAUNCH(kernel<2>, __VA_ARGS__); break;                     \
+      case 3: SCN_LAUNCH(kernel<3>, __VA_ARGS__); break;                     \
+      case 4: SCN_LAUNCH(kernel<4>, __VA_ARGS__); break;                     \
+      default: SCN_LAUNCH(kernel<0>, __VA_ARGS__);                           \
+    }                                                                        \
+  } while (0)
+
 // ------------------------------------------------------------------------------------------
 // input layer
 // ------------------------------------------------------------------------------------------
@@ -363,6 +391,7 @@ static int flags_to_status(int flags) {
 // bl_length > 0: coords are [batch, bl_length, dim] (BLInputLayer, IOLayersRules.h:134-288):
 // the sample index is i / bl_length and a point whose first coordinate is negative is empty.
 // packed (coordinates that came from the host): the checked keys, the empty key for an empty slot.
+template <int DIM>
 __global__ void k_insert_input(KeyLayout L, HashTable T, const long long *__restrict__ coords,
                                const unsigned long long *__restrict__ packed,
                                long long n, int ncols, int mode, long long bl_length,
@@ -377,9 +406,12 @@ __global__ void k_insert_input(KeyLayout L, HashTable T, const long long *__rest
   } else {
     const long long *c = coords + i * ncols;
     if (!(bl_length > 0 && c[0] < 0)) {  // otherwise an empty slot of the batch x length array: in no map, in no rule
-      int x[kMaxDim];
+      constexpr int kDim = DIM ? DIM : kMaxDim;
+      const int dim = DIM ? DIM : L.dim;
+      int x[kDim];
       bool ok = true;
-      for (int d = 0; d < L.dim; ++d) {
+#pragma unroll
+      for (int d = 0; d < dim; ++d) {
         long long v = c[d];
         ok &= (v >= 0 && v < L.size[d]);
         x[d] = (int)v;
@@ -387,7 +419,7 @@ __global__ void k_insert_input(KeyLayout L, HashTable T, const long long *__rest
       bl = bl_length > 0 ? i / bl_length : ((ncols > L.dim) ? c[L.dim] : 0);
       ok &= (bl >= 0 && bl < (1ll << L.batch_bits));
       if (ok)
-        key = pack_key(L, x, (int)bl);
+        key = pack_site<DIM>(L, x, (int)bl);
       else
         atomicOr(flags, FLAG_COORD_RANGE);
     }
@@ -697,7 +729,7 @@ static int md_input_layer(scn_metadata *md, const int64_t *spatial_size, const i
   uint2 *words = nullptr;
   SCN_TRY(device_alloc((void **)&slot_of, sizeof(int) * (size_t)std::max<int64_t>(n, 1), stream));
   if (n > 0) {
-    SCN_LAUNCH(k_insert_input, blocks, threads, 0, stream, g.layout, g.table, coords_dev, packed_dev, n, ncols, mode, (long long)bl_length, g.row_keys, slot_of, md->flags_dev, n_samples);
+    SCN_LAUNCH_DIM(md->dim, k_insert_input, blocks, threads, 0, stream, g.layout, g.table, coords_dev, packed_dev, n, ncols, mode, (long long)bl_length, g.row_keys, slot_of, md->flags_dev, n_samples);
     if (mode == 0)
       SCN_LAUNCH(k_blank_overwritten, blocks, threads, 0, stream, g.table.slots, slot_of, n, g.row_keys, md->flags_dev, n_samples, post);
     SCN_CUDA_CHECK(cudaGetLastError());
@@ -819,88 +851,115 @@ __device__ __forceinline__ void post_counts(unsigned long long *counts, int K, v
   __threadfence_system();
 }
 
-// One thread per output site, looping over this block's range of filter offsets.  Offset k
+// One thread per output site, looping over this block's range of at most 32 filter offsets.  Offset k
 // (row-major over the filter, last dimension fastest, RectangularRegions.h:30-38) looks at
 // input = output + delta_k with delta = k_d - f_d / 2 (SubmanifoldConvolutionRules.h:15-19).
 // The neighbour's key is the site's key plus a per-offset constant, so a probe is a bounds
-// check, one 64-bit add and one 32-byte bucket read.
+// check, one 64-bit add and one 32-byte bucket read; the buckets of kAhead offsets are read before the first is looked at.
+// Bound by instruction issue and the latency of the bucket reads: 400 k sites, 27 offsets: 85 us (101 with coordinates
+// in local memory and one bucket at a time).
+template <int DIM>
 __global__ void __launch_bounds__(256)
 k_submanifold_rules(KeyLayout L, HashTable T, const unsigned long long *__restrict__ row_keys,
                     long long n, int K, FilterDesc F, int k_chunk, int *__restrict__ nbr,
                     unsigned long long *counts, int mirrored, unsigned *__restrict__ masks, int mask_words,
                     volatile unsigned long long *counts_host) {
-  extern __shared__ long long sh_raw[];
-  long long *sh_keydelta = sh_raw;                         // [k_chunk]
-  int *sh_count = (int *)(sh_keydelta + k_chunk);          // [k_chunk]
-  signed char *sh_delta = (signed char *)(sh_count + k_chunk);  // [k_chunk][dim]
+  constexpr int kDim = DIM ? DIM : kMaxDim, kAhead = 3;
+  __shared__ long long sh_keydelta[32];
+  __shared__ int sh_count[32];
+  __shared__ signed char sh_delta[32][kDim];
+  const int dim = DIM ? DIM : L.dim, lane = threadIdx.x & 31;
   // mirrored (all filter sizes odd): offset K-1-k is offset k seen from the neighbour, so only the
   // offsets up to the centre are looked up; a hit also fills the neighbour's entry at the mirrored
   // offset (pre-set to -1 by the caller), and the centre is the site itself.
   const int k_end = mirrored ? K / 2 + 1 : K;
-  int k0 = blockIdx.y * k_chunk;
-  int k1 = min(k_end, k0 + k_chunk);
-  for (int kk = k0 + threadIdx.x; kk < k1; kk += blockDim.x) {
-    int rem = kk;
+  const int k0 = blockIdx.y * k_chunk, k1 = min(k_end, k0 + k_chunk);
+  if (k0 + (int)threadIdx.x < k1) {
+    int rem = k0 + threadIdx.x;
     long long kd = 0;
-    for (int d = L.dim - 1; d >= 0; --d) {
-      int delta = rem % F.f[d] - F.f[d] / 2;
+    for (int d = dim - 1; d >= 0; --d) {
+      const int delta = rem % F.f[d] - F.f[d] / 2;
       rem /= F.f[d];
-      sh_delta[(kk - k0) * L.dim + d] = (signed char)delta;
+      sh_delta[threadIdx.x][d] = (signed char)delta;
       kd += (long long)delta * (1ll << L.shift[d]);
     }
-    sh_keydelta[kk - k0] = kd;
-    sh_count[kk - k0] = 0;
+    sh_keydelta[threadIdx.x] = kd;
+    sh_count[threadIdx.x] = 0;
   }
   __syncthreads();
+  const unsigned long long bucket_mask = T.n_buckets - 1;
+  int my_count = 0;  // of offset k0 + lane, by this warp
   // at most a few blocks per SM, each over several runs of sites: the counts below are atomics on K addresses per block
   for (long long site0 = (long long)blockIdx.x * blockDim.x; site0 < n; site0 += (long long)gridDim.x * blockDim.x) {
-  const long long site = site0 + threadIdx.x;
-  bool active = site < n;
-  unsigned long long key = active ? row_keys[site] : kEmptyKey;
-  active = active && (key != kEmptyKey);  // blank key: overwritten duplicate, in no map
-  int x[kMaxDim], b = 0;
-  if (active) unpack_key(L, key, x, b);
-  // masks (optional, zeroed by the caller): the offsets of every site as bits, both ends of a hit OR theirs in.  Six
-  // million of these at 1.6 M sites disappear beside the lookups; reading the finished table back took 109 us.
-  unsigned bits = 0;
-  int word = k0 >> 5;
-  for (int kk = k0; kk < k1; ++kk) {
-    if (masks && (kk >> 5) != word) {
-      if (bits) atomicOr(&masks[site * mask_words + word], bits);
-      bits = 0;
-      word = kk >> 5;
-    }
-    int row = -1;
-    if (active) {
-      bool ok = true;
-      const signed char *dl = sh_delta + (kk - k0) * L.dim;
-      for (int d = 0; d < L.dim; ++d) {
-        int y = x[d] + dl[d];
-        ok &= ((unsigned)y < (unsigned)L.size[d]);
+    const long long site = site0 + threadIdx.x;
+    unsigned long long key = site < n ? row_keys[site] : kEmptyKey;
+    const bool active = key != kEmptyKey;  // blank key: overwritten duplicate, in no map
+    int x[kDim], b = 0;
+    unpack_site<DIM>(L, key, x, b);
+    // masks (optional, zeroed by the caller): the offsets of every site as bits, both ends of a hit OR theirs in.  Six
+    // million of these at 1.6 M sites disappear beside the lookups; reading the finished table back took 109 us.
+    unsigned bits = 0;
+    int word = k0 >> 5;
+    int *out = nbr + (long long)k0 * n + site, *back = nbr + (long long)(K - 1 - k0) * n;  // offset kk, and its mirror
+    for (int kb = k0; kb < k1; kb += kAhead) {
+      unsigned long long want[kAhead];
+      uint4 s0[kAhead], s1[kAhead];
+      bool look[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int i = kb + u - k0;
+        look[u] = active && kb + u < k1 && !(mirrored && kb + u == K / 2);
+        if (kb + u < k1) {
+#pragma unroll
+          for (int d = 0; d < dim; ++d) look[u] &= (unsigned)(x[d] + sh_delta[i][d]) < (unsigned)L.size[d];
+          want[u] = key + (unsigned long long)sh_keydelta[i];
+        }
+        if (look[u]) {
+          const uint4 *q = reinterpret_cast<const uint4 *>(T.slots + 2 * (mix64(want[u]) & bucket_mask));
+          s0[u] = __ldg(q);
+          s1[u] = __ldg(q + 1);
+        }
       }
-      if (mirrored && kk == K / 2)
-        row = (int)site;
-      else if (ok)
-        row = hash_find_row(T, key + (unsigned long long)sh_keydelta[kk - k0]);
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int kk = kb + u;
+        if (kk >= k1) break;
+        int row = -1;
+        if (look[u]) {
+          const unsigned long long e0 = ((unsigned long long)s0[u].y << 32) | s0[u].x;
+          const unsigned long long e1 = ((unsigned long long)s1[u].y << 32) | s1[u].x;
+          if (e0 == want[u]) row = (int)s0[u].z;
+          else if (e1 == want[u]) row = (int)s1[u].z;
+          else if (e0 != kEmptyKey && e1 != kEmptyKey) row = hash_find_row(T, want[u]);  // a full bucket: walk on
+        }
+        if (mirrored && kk == K / 2 && active) row = (int)site;
+        if (masks && (kk >> 5) != word) {
+          if (bits) atomicOr(&masks[site * mask_words + word], bits);
+          bits = 0;
+          word = kk >> 5;
+        }
+        if (site < n) *out = row;
+        if (masks && row >= 0) bits |= 1u << (kk & 31);
+        if (mirrored && kk < K / 2 && row >= 0) {
+          back[row] = (int)site;
+          const int kr = K - 1 - kk;
+          if (masks) atomicOr(&masks[(long long)row * mask_words + (kr >> 5)], 1u << (kr & 31));
+        }
+        out += n;
+        back -= n;
+        const unsigned hits = __ballot_sync(0xffffffffu, row >= 0);
+        if (lane == kk - k0) my_count += __popc(hits);
+      }
     }
-    if (site < n) nbr[(long long)kk * n + site] = row;
-    if (masks && row >= 0) bits |= 1u << (kk & 31);
-    if (mirrored && kk < K / 2 && row >= 0) {
-      const int back = K - 1 - kk;
-      nbr[(long long)back * n + row] = (int)site;
-      if (masks) atomicOr(&masks[(long long)row * mask_words + (back >> 5)], 1u << (back & 31));
-    }
-    unsigned hits = __ballot_sync(0xffffffffu, row >= 0);
-    if ((threadIdx.x & 31) == 0 && hits) atomicAdd(&sh_count[kk - k0], __popc(hits));
+    if (masks && bits) atomicOr(&masks[site * mask_words + word], bits);
   }
-  if (masks && bits) atomicOr(&masks[site * mask_words + word], bits);
-  }
+  if (my_count) atomicAdd(&sh_count[lane], my_count);
   __syncthreads();
-  for (int kk = k0 + threadIdx.x; kk < k1; kk += blockDim.x)
-    if (sh_count[kk - k0]) {
-      atomicAdd(&counts[kk], (unsigned long long)sh_count[kk - k0]);
-      if (mirrored && kk < K / 2) atomicAdd(&counts[K - 1 - kk], (unsigned long long)sh_count[kk - k0]);
-    }
+  if (k0 + (int)threadIdx.x < k1 && sh_count[threadIdx.x]) {
+    const int kk = k0 + threadIdx.x;
+    atomicAdd(&counts[kk], (unsigned long long)sh_count[threadIdx.x]);
+    if (mirrored && kk < K / 2) atomicAdd(&counts[K - 1 - kk], (unsigned long long)sh_count[threadIdx.x]);
+  }
   post_counts(counts, K, counts_host);
 }
 
@@ -968,10 +1027,9 @@ int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
     SCN_LAUNCH(k_rules_init, (unsigned)std::min<long long>(148 * 8, ceil_div(std::max(n_back / 4, n * words), 256)), 256, 0, stream, rb.counts_dev, (int)K + 1, rb.masks, rb.masks ? n * words : 0, rb.nbr + k_end * n, n_back);
     // enough blocks to fill the machine even for few sites: split the offsets over grid.y
     long long want_y = std::max<long long>(1, std::min<long long>(k_end, ceil_div(148 * 16, bx)));
-    int k_chunk = (int)ceil_div(k_end, want_y);
+    const int k_chunk = (int)ceil_div(k_end, std::max(want_y, ceil_div(k_end, 32)));  // at most 32: a lane counts an offset
     int gy = (int)ceil_div(k_end, k_chunk);
-    size_t smem = (size_t)k_chunk * (sizeof(long long) + sizeof(int) + md->dim);
-    SCN_LAUNCH(k_submanifold_rules, dim3((unsigned)std::min<long long>(bx, 148 * 16), (unsigned)gy), threads, smem, stream, g->layout, g->table, g->row_keys, n, (int)K, F, k_chunk, rb.nbr, rb.counts_dev, mirrored ? 1 : 0, rb.masks, words, ticket_dev(rb));
+    SCN_LAUNCH_DIM(md->dim, k_submanifold_rules, dim3((unsigned)std::min<long long>(bx, 148 * 16), (unsigned)gy), threads, 0, stream, g->layout, g->table, g->row_keys, n, (int)K, F, k_chunk, rb.nbr, rb.counts_dev, mirrored ? 1 : 0, rb.masks, words, ticket_dev(rb));
     SCN_CUDA_CHECK(cudaGetLastError());
   }
   rb.built = true;
@@ -988,38 +1046,49 @@ int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
 // Output region per dimension: lb = max(0, (x - f + s) / s), ub = min(out - 1, x / s)
 // (RectangularRegions.h:108-119); offset = sum (x_d - o_d * s_d) * prod_{j>d} f_j
 // (RectangularRegions.h:30-38,94-105).
-__device__ inline bool strided_target(const KeyLayout &L, const FilterDesc &F, const int *x, int t,
-                                      int *o, int &k) {
+template <int DIM>
+__device__ __forceinline__ bool strided_target(const KeyLayout &L, const FilterDesc &F, const int (&x)[DIM ? DIM : kMaxDim],
+                                               int t, int (&o)[DIM ? DIM : kMaxDim], int &k) {
+  const int dim = DIM ? DIM : L.dim;
   k = 0;
   int mult = 1;
-  for (int d = L.dim - 1; d >= 0; --d) {
-    int num = x[d] - F.f[d] + F.s[d];
-    int lb = num > 0 ? num / F.s[d] : 0;
-    int ub = min(F.out_size[d] - 1, x[d] / F.s[d]);
-    int j = t % F.tdim[d];
-    t /= F.tdim[d];
-    int od = lb + j;
-    if (od > ub) return false;
+#pragma unroll
+  for (int d = dim - 1; d >= 0; --d) {
+    int lb, ub, j = 0;
+    if (F.tmax == 1) {  // windows side by side
+      lb = ub = (int)((unsigned)x[d] / (unsigned)F.s[d]);
+    } else {
+      const int num = x[d] - F.f[d] + F.s[d];
+      lb = num > 0 ? (int)((unsigned)num / (unsigned)F.s[d]) : 0;
+      ub = (int)((unsigned)x[d] / (unsigned)F.s[d]);
+      j = (int)((unsigned)t % (unsigned)F.tdim[d]);
+      t = (int)((unsigned)t / (unsigned)F.tdim[d]);
+    }
+    const int od = lb + j;
+    if (od > min(F.out_size[d] - 1, ub)) return false;
     o[d] = od;
-    k += (x[d] - od * F.s[d]) * mult;
+    const int kd = x[d] - od * F.s[d];
+    if (kd >= F.f[d]) return false;  // (a window narrower than the stride)
+    k += kd * mult;
     mult *= F.f[d];
   }
   return true;
 }
 
-__global__ void k_strided_insert(KeyLayout Lin, KeyLayout Lout, FilterDesc F, HashTable Tout,
-                                 const unsigned long long *__restrict__ in_keys, long long n_in,
-                                 const int *__restrict__ n_in_dev, int *__restrict__ slot_of, int *flags) {
-  long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+template <int DIM>
+__global__ void __launch_bounds__(256)
+k_strided_insert(KeyLayout Lin, KeyLayout Lout, FilterDesc F, HashTable Tout, const unsigned long long *__restrict__ in_keys,
+                 long long n_in, const int *__restrict__ n_in_dev, int *__restrict__ slot_of, int *flags) {
+  const unsigned id = blockIdx.x * blockDim.x + threadIdx.x;  // (fewer than 2^31 candidates)
   if (id >= sites_here(n_in_dev, n_in) * F.tmax) return;
-  long long i = id / F.tmax;
-  int t = (int)(id % F.tmax);
-  unsigned long long key = in_keys[i];
+  const unsigned i = F.tmax == 1 ? id : id / (unsigned)F.tmax;
+  const int t = (int)(id - i * (unsigned)F.tmax);
+  const unsigned long long key = in_keys[i];
   unsigned long long okey = kEmptyKey;
   if (key != kEmptyKey) {
-    int x[kMaxDim], o[kMaxDim], b, k;
-    unpack_key(Lin, key, x, b);
-    if (strided_target(Lin, F, x, t, o, k)) okey = pack_key(Lout, o, b);
+    int x[DIM ? DIM : kMaxDim], o[DIM ? DIM : kMaxDim], b, k;
+    unpack_site<DIM>(Lin, key, x, b);
+    if (strided_target<DIM>(Lin, F, x, t, o, k)) okey = pack_site<DIM>(Lout, o, b);
   }
   // Candidates of one warp that name the same output site (neighbouring input rows usually do) insert
   // it once: the lowest lane of the group, which also holds the group's smallest id, does the insert
@@ -1028,7 +1097,7 @@ __global__ void k_strided_insert(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Ha
   const int leader = __ffs(peers) - 1;
   int s_out = -1;
   if (okey != kEmptyKey && (int)(threadIdx.x & 31) == leader) {
-    const long long s = hash_claim<false, true>(Tout, okey, (unsigned)id);
+    const long long s = hash_claim<false, true>(Tout, okey, id);
     if (s < 0)
       atomicOr(flags, FLAG_TABLE_FULL);
     else
@@ -1041,6 +1110,7 @@ __global__ void k_strided_insert(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Ha
 // shared memory first: counted in global memory per warp, a 3 / 2 layer's eight rules per candidate were 370 us of
 // atomics on 27 addresses for 184 k sites.
 constexpr int kFillCounts = 1024;
+template <int DIM>
 __global__ void __launch_bounds__(256)
 k_strided_fill(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Slot *slots, const unsigned long long *__restrict__ in_keys,
                const int *__restrict__ slot_of, long long n_in, const int *__restrict__ n_in_dev, long long n_out,
@@ -1058,11 +1128,11 @@ k_strided_fill(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Slot *slots, const u
     for (long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < n_ids; id += (long long)gridDim.x * blockDim.x) {
       const int s = slot_of[id];
       if (s < 0) continue;
-      const long long i = id / F.tmax;
-      const int t = (int)(id % F.tmax);
-      int x[kMaxDim], o[kMaxDim], b, k;
-      unpack_key(Lin, in_keys[i], x, b);
-      strided_target(Lin, F, x, t, o, k);
+      const unsigned i = F.tmax == 1 ? (unsigned)id : (unsigned)id / (unsigned)F.tmax;
+      const int t = (int)((unsigned)id - i * (unsigned)F.tmax);
+      int x[DIM ? DIM : kMaxDim], o[DIM ? DIM : kMaxDim], b, k;
+      unpack_site<DIM>(Lin, in_keys[i], x, b);
+      strided_target<DIM>(Lin, F, x, t, o, k);
       // one look at the slot per group of lanes that share it; the site's first candidate, always the lowest lane of its
       // group, leaves the row in the slot and the site's key in its row
       const unsigned act = __activemask();
@@ -1074,7 +1144,7 @@ k_strided_fill(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Slot *slots, const u
         orow = row_of_first(words, base, toucher);
         if (toucher == (unsigned)id) {
           slots[s].row = orow;
-          row_keys[orow] = pack_key(Lout, o, b);
+          row_keys[orow] = pack_site<DIM>(Lout, o, b);
         }
       }
       orow = __shfl_sync(same, orow, first);
@@ -1165,7 +1235,7 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
       HostPost post{};
       SCN_TRY(post_begin(md, post));
       post.extra = nullptr;
-      SCN_LAUNCH(k_strided_insert, blocks, threads, 0, stream, gin->layout, gout.layout, F, gout.table, gin->row_keys, n_in, nullptr, slot_of, md->flags_dev);
+      SCN_LAUNCH_DIM(md->dim, k_strided_insert, blocks, threads, 0, stream, gin->layout, gout.layout, F, gout.table, gin->row_keys, n_in, nullptr, slot_of, md->flags_dev);
       SCN_LAUNCH(k_first_ranks, tiles, 256, 0, stream, gout.table.slots, slot_of, n_in, nullptr, F.tmax, words, base, done, nullptr, md->flags_dev, true, nullptr, post);
       SCN_CUDA_CHECK(cudaGetLastError());
       SCN_TRY(wait_posted(md->mailbox, stream));
@@ -1212,7 +1282,7 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
   SCN_TRY(fill_launch(fills, stream));
   if (n_ids > 0) {
     unsigned blocks = (unsigned)ceil_div(n_ids, threads);
-    SCN_LAUNCH(k_strided_fill, std::min(blocks, 148u * 8u), threads, 0, stream, gin->layout, gout.layout, F, gout.table.slots, gin->row_keys, slot_of, n_in, nullptr, n_out, nullptr, n_out, words, base, gout.row_keys, rb.nbr, rb.counts_dev, (int)K, ticket_dev(rb));
+    SCN_LAUNCH_DIM(md->dim, k_strided_fill, std::min(blocks, 148u * 8u), threads, 0, stream, gin->layout, gout.layout, F, gout.table.slots, gin->row_keys, slot_of, n_in, nullptr, n_out, nullptr, n_out, words, base, gout.row_keys, rb.nbr, rb.counts_dev, (int)K, ticket_dev(rb));
     SCN_CUDA_CHECK(cudaGetLastError());
   }
   device_free(slot_of, stream);
@@ -1322,9 +1392,9 @@ static int chain_enqueue(scn_metadata *md, const Grid *gin, std::vector<ChainLev
       post.total = mailbox_dev + 1 + l;
       post.flags = mailbox_dev + 1 + L + l;
       post.ready = l == L - 1 ? mailbox_dev : nullptr;
-      SCN_LAUNCH(k_strided_insert, blocks, threads, 0, stream, Lin, lv.gout.layout, lv.F, lv.gout.table, in_keys, lv.bound_in, n_in_dev, lv.slot_of, level_flags);
+      SCN_LAUNCH_DIM(md->dim, k_strided_insert, blocks, threads, 0, stream, Lin, lv.gout.layout, lv.F, lv.gout.table, in_keys, lv.bound_in, n_in_dev, lv.slot_of, level_flags);
       SCN_LAUNCH(k_first_ranks, (unsigned)ceil_div(n_ids, kRankTile), 256, 0, stream, lv.gout.table.slots, lv.slot_of, lv.bound_in, n_in_dev, lv.F.tmax, lv.words, lv.base, lev + 2 * L + l, lev + l, level_flags, false, nullptr, post);
-      SCN_LAUNCH(k_strided_fill, std::min(blocks, 148u * 8u), threads, 0, stream, Lin, lv.gout.layout, lv.F, lv.gout.table.slots, in_keys, lv.slot_of, lv.bound_in, n_in_dev, 0ll, lev + l, lv.cap_out, lv.words, lv.base, lv.gout.row_keys, lv.rb.nbr, lv.rb.counts_dev, (int)lv.K, ticket_dev(lv.rb));
+      SCN_LAUNCH_DIM(md->dim, k_strided_fill, std::min(blocks, 148u * 8u), threads, 0, stream, Lin, lv.gout.layout, lv.F, lv.gout.table.slots, in_keys, lv.slot_of, lv.bound_in, n_in_dev, 0ll, lev + l, lv.cap_out, lv.words, lv.base, lv.gout.row_keys, lv.rb.nbr, lv.rb.counts_dev, (int)lv.K, ticket_dev(lv.rb));
       SCN_CUDA_CHECK(cudaGetLastError());
     }
     in_keys = lv.gout.row_keys;
