@@ -372,6 +372,10 @@ SCN_API int scn_batchnorm_join_forward(const float *in_a, int planes_a, const fl
 SCN_API int scn_rows_affine_forward(const float *in_features, float *out_features, int64_t n_rows,
                                     int n_in_planes, int n_out_planes, const float *weight, const float *bias,
                                     void *stream);
+/* Its weight gradients: d_weight [n_in_planes][n_out_planes] = in_features^T * d_out_features and, unless null, d_bias =
+ * the column sums of d_out_features, in fp32 and in a fixed order, for any plane counts. */
+SCN_API int scn_rows_affine_backward(const float *in_features, const float *d_out_features, int64_t n_rows,
+                                     int n_in_planes, int n_out_planes, float *d_weight, float *d_bias, void *stream);
 SCN_API int scn_submanifold_convolution_bn_forward(scn_metadata *md, const int64_t *spatial_size,
                                                    const int64_t *filter_size, const float *in_features,
                                                    float *out_features, const float *weight, const float *bias,

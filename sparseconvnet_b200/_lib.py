@@ -65,6 +65,7 @@ SIGNATURES = {
     "scn_batchnorm_join_forward": (C.c_int, [_vp, C.c_int, _vp, C.c_int, _vp, C.c_int64, _vp, _vp, _vp, _vp, C.c_double,
                                              C.c_double, _vp]),
     "scn_rows_affine_forward": (C.c_int, [_vp, _vp, C.c_int64, C.c_int, C.c_int, _vp, _vp, _vp]),
+    "scn_rows_affine_backward": (C.c_int, [_vp, _vp, C.c_int64, C.c_int, C.c_int, _vp, _vp, _vp]),
     "scn_batchnorm_fold": (C.c_int, [_vp, _vp, _vp, _vp, C.c_double, C.c_int, _vp, _vp, _vp]),
     "scn_submanifold_convolution_bn_forward": (C.c_int, [_vp, _i64p, _i64p, _vp, _vp, _vp, _vp, _vp, _vp, C.c_double,
                                                          C.c_int, C.c_int, C.c_int, C.c_int, _vp,

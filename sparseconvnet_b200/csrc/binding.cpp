@@ -751,6 +751,86 @@ SCN_FN(batchnorm_train) {
   SCN_END
 }
 
+// rows @ weight (+ bias) on the library's kernel for narrow results, on torch's matrix product otherwise
+bool rows_affine_takes(int64_t nin, int64_t nout) { return nout <= 32 && nin % 4 == 0 && nin >= 4 && nin <= 256; }
+
+struct RowsAffineNode : ag::Node {
+  ag::SavedVariable features_, weight_;
+  bool with_bias = false;
+  std::string name() const override { return "NetworkInNetworkBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    features_.reset_data();
+    weight_.reset_data();
+  }
+  ag::variable_list apply(ag::variable_list &&grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    ag::variable_list result(3);
+    if (!grads[0].defined()) return result;
+    if (at::GradMode::is_enabled()) {  // the gradient is to be differentiated itself
+      const at::Tensor f = features_.unpack(), w = weight_.unpack();
+      if (task_should_compute_output(0)) result[0] = grads[0].mm(w.t());
+      if (task_should_compute_output(1)) result[1] = f.t().mm(grads[0]);
+      if (with_bias && task_should_compute_output(2)) result[2] = grads[0].sum(0);
+      return result;
+    }
+    const at::Tensor f = features_.unpack(), w = weight_.unpack(), go = grads[0].contiguous();
+    TORCH_CHECK(go.is_cuda() && go.scalar_type() == at::kFloat, "the gradient must be CUDA float32");
+    const OnDevice on(f);
+    const int64_t n = f.size(0), nin = w.size(0), nout = w.size(1);
+    if (task_should_compute_output(0)) {
+      if (rows_affine_takes(nout, nin)) {
+        const at::Tensor wt = w.t().contiguous();
+        result[0] = at::empty({n, nin}, go.options());
+        check_free(scn_rows_affine_forward(ptr(go), ptr(result[0]), n, (int)nout, (int)nin, ptr(wt), nullptr, on.stream));
+      } else {
+        result[0] = at::mm(go, w.t());
+      }
+    }
+    if (task_should_compute_output(1) || task_should_compute_output(2)) {
+      at::Tensor dw = at::empty_like(w), db;
+      if (with_bias) db = at::empty({nout}, go.options());
+      check_free(scn_rows_affine_backward(ptr(f), ptr(go), n, (int)nin, (int)nout, ptr(dw), with_bias ? ptr(db) : nullptr,
+                                          on.stream));
+      result[1] = dw;
+      result[2] = db;
+    }
+    return result;
+  }
+};
+
+// (features, weight [nIn, nOut], bias or None) -> output
+SCN_FN(rows_affine_train) {
+  SCN_BEGIN(3)
+  const at::Tensor &given = tensor(a[0], "input_features"), &w = features(a[1], "weight");
+  const at::Tensor bias = a[2] == Py_None ? at::Tensor() : features(a[2], "bias");
+  at::Tensor f, out;
+  {
+    const at::NoGradGuard no_grad;
+    f = contiguous_features(a[0]);
+    if (f.dim() != 2 || w.dim() != 2 || f.size(1) != w.size(0)) fail("features and weight do not match");
+    const OnDevice on(f);
+    const int64_t n = f.size(0), nin = w.size(0), nout = w.size(1);
+    if (rows_affine_takes(nin, nout)) {
+      out = at::empty({n, nout}, f.options());
+      SCN_CALL(scn_rows_affine_forward(ptr(f), ptr(out), n, (int)nin, (int)nout, ptr(w), bias.defined() ? ptr(bias) : nullptr,
+                                       on.stream));
+    } else {
+      out = bias.defined() ? at::addmm(bias, f, w) : at::mm(f, w);
+    }
+  }
+  if (ag::compute_requires_grad(given, w, bias)) {
+    std::shared_ptr<RowsAffineNode> node(new RowsAffineNode(), ag::deleteNode);
+    node->set_next_edges(ag::collect_next_edges(given, w, bias));
+    node->features_ = ag::SavedVariable(f, false);
+    node->weight_ = ag::SavedVariable(w, false);
+    node->with_bias = bias.defined();
+    ag::set_history(out, node);
+  }
+  return THPVariable_Wrap(std::move(out));
+  SCN_END
+}
+
 // (kind, metadata, md, in_size, out_size, pool, stride, features, drop) -> output
 SCN_FN(pooling_train) {
   SCN_BEGIN(9)
@@ -878,7 +958,7 @@ PyMethodDef methods[] = {
     SCN_METHOD(pooling_forward),         SCN_METHOD(pooling_backward),   SCN_METHOD(sparse_to_dense),
     SCN_METHOD(active_sites),            SCN_METHOD(strided_size),       SCN_METHOD(transposed_size),
     SCN_METHOD(convolution_train),       SCN_METHOD(batchnorm_train),    SCN_METHOD(pooling_train),
-    SCN_METHOD(input_layer),             SCN_METHOD(versions),           SCN_METHOD(set_check),                    {nullptr, nullptr, 0, nullptr}};
+    SCN_METHOD(rows_affine_train),       SCN_METHOD(input_layer),             SCN_METHOD(versions),           SCN_METHOD(set_check),                    {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_binding", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

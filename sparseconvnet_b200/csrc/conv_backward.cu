@@ -51,7 +51,7 @@ __global__ void k_transpose_weight(const float *__restrict__ w, float *__restric
 // partial[chunk][k][g][c][n] = sum over the chunk's rulebook entries j of offset k of
 //   in[in_row(j)][g*cin + c] * d_out[out_row(j)][g*cout + n]
 // where (in_row, out_row) = (nbr[k][j], j), or (j, nbr[k][j]) when the operator runs the rulebook
-// backwards (Deconvolution).  grid = (chunks, K, groups * c-tiles * n-tiles), 256 threads,
+// backwards (Deconvolution); nbr null: (j, j), a dense product.  grid = (chunks, K, groups * c-tiles * n-tiles), 256 threads,
 // 32 x 32 tile, 2 x 2 outputs per thread.
 __global__ void __launch_bounds__(256)
 k_conv_dweight(const float *__restrict__ in, int ld_in, long long n_in_rows, const float *__restrict__ dout,
@@ -76,7 +76,7 @@ k_conv_dweight(const float *__restrict__ in, int ld_in, long long n_in_rows, con
     const long long j = jb + lr;
     long long ri = -1, ro = -1;
     if (j < j1) {
-      const int a = nbr[(long long)k * n_entries + j];
+      const int a = nbr ? nbr[(long long)k * n_entries + j] : (int)j;
       if (a >= 0) {
         ri = swap ? j : a;
         ro = swap ? a : j;
@@ -118,7 +118,15 @@ __global__ void k_sum_chunks(const float *__restrict__ partial, int chunks, long
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float acc = 0.f;
-  for (int c = 0; c < chunks; ++c) acc += partial[(long long)c * n + i];
+  int c = 0;
+  for (; c + 8 <= chunks; c += 8) {  // eight loads on their way
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = partial[(long long)(c + u) * n + i];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc += v[u];
+  }
+  for (; c < chunks; ++c) acc += partial[(long long)c * n + i];
   out[i] = acc;
 }
 
@@ -505,6 +513,36 @@ int scn_convolution_backward(scn_metadata *md, const int64_t *input_size, const 
   SCN_TRY(get_strided_rulebook(md, input_size, output_size, filter_size, filter_stride, stream, &rb));
   return run_conv_backward(md, *rb, false, in_features, d_in_features, d_out_features, weight, d_weight, d_bias,
                            n_in_planes, n_out_planes, groups, stream);
+}
+
+int scn_rows_affine_backward(const float *in_features, const float *d_out_features, int64_t n_rows, int n_in_planes,
+                             int n_out_planes, float *d_weight, float *d_bias, void *stream_) {
+  cudaStream_t stream = (cudaStream_t)stream_;
+  SCN_REQUIRE(n_in_planes >= 1 && n_out_planes >= 1 && d_weight, SCN_ERR_BAD_ARG, "rows_affine_backward: bad arguments");
+  SCN_REQUIRE(n_rows >= 0 && n_rows < (1ll << 31), SCN_ERR_UNSUPPORTED, "row count %lld unsupported", (long long)n_rows);
+  const long long w_elems = (long long)n_in_planes * n_out_planes;
+  if (n_rows == 0) {
+    SCN_CUDA_CHECK(cudaMemsetAsync(d_weight, 0, sizeof(float) * (size_t)w_elems, stream));
+    if (d_bias) SCN_CUDA_CHECK(cudaMemsetAsync(d_bias, 0, sizeof(float) * (size_t)n_out_planes, stream));
+    return SCN_OK;
+  }
+  SCN_REQUIRE(in_features && d_out_features, SCN_ERR_BAD_ARG, "null features");
+  // four waves of CTAs, each at least 16 slabs of 32 rows
+  const int tiles = (int)(ceil_div(n_in_planes, 32) * ceil_div(n_out_planes, 32));
+  const long long chunks = std::max<long long>(1, std::min<long long>(148 * 32 / tiles, n_rows / 512));
+  const long long chunk_rows = ceil_div(ceil_div(n_rows, chunks), 32) * 32;
+  const int grid_x = (int)ceil_div(n_rows, chunk_rows);
+  float *partial = nullptr;
+  SCN_TRY(device_alloc((void **)&partial, sizeof(float) * (size_t)grid_x * (size_t)(w_elems + n_out_planes), stream));
+  float *bias_partial = partial + (size_t)grid_x * w_elems;
+  SCN_LAUNCH(k_conv_dweight, dim3((unsigned)grid_x, 1, (unsigned)tiles), 256, 0, stream, in_features, n_in_planes, (long long)n_rows, d_out_features, n_out_planes, (long long)n_rows, nullptr, (long long)n_rows, 0, n_in_planes, n_out_planes, 1, chunk_rows, partial, nullptr);
+  SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 32), 32, 0, stream, partial, grid_x, w_elems, d_weight);
+  if (d_bias) {
+    SCN_LAUNCH(k_column_sums, dim3((unsigned)ceil_div(n_out_planes, 32), (unsigned)grid_x), 256, 0, stream, d_out_features, (long long)n_rows, n_out_planes, chunk_rows, bias_partial);
+    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(n_out_planes, 32), 32, 0, stream, bias_partial, grid_x, (long long)n_out_planes, d_bias);
+  }
+  SCN_CUDA_CHECK(cudaGetLastError());
+  return device_free(partial, stream);
 }
 
 int scn_deconvolution_backward(scn_metadata *md, const int64_t *input_size, const int64_t *output_size,

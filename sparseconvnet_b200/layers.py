@@ -605,10 +605,7 @@ class NetworkInNetwork(Module):
         assert input.features.nelement() == 0 or input.features.size(1) == self.nIn
         output = SparseConvNetTensor(metadata=input.metadata, spatial_size=input.spatial_size)
         if autograd.needs_grad(input.features, self.weight):
-            # a dense matrix product: torch's own autograd covers it (the reference calls addmm as well)
-            output.features = input.features @ self.weight
-            if hasattr(self, "bias"):
-                output.features = output.features + self.bias
+            output.features = autograd.rows_affine(input.features, self.weight, getattr(self, "bias", None))
             macs = float(input.features.size(0) * self.nIn * self.nOut)
             SCN.flop_counter.add(macs)
             _pkg.forward_pass_hidden_states += output.features.nelement()

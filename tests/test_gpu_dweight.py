@@ -53,3 +53,48 @@ def test_weight_gradient(n, size, cin, cout, cuda):
             want.index_add_(0, r[:, 0].long(), gd[r[:, 1].long()] @ w.t())
         e = helpers.rel_err(f.grad.double().cpu().numpy(), want.cpu().numpy())
         assert e <= helpers.FP32_TOL, (layer, "input gradient", e)
+
+
+@pytest.mark.parametrize("cin,cout", [(1, 1), (4, 32), (32, 20), (33, 40), (48, 20), (100, 7)])
+@pytest.mark.parametrize("n", [1, 31, 512, 513, 70001])
+def test_network_in_network_gradients(n, cin, cout, cuda):
+    """One fp32 sum of n products per weight, in chunks of at least 512 rows: 2^-24 sqrt(n) of the largest, far below the
+    package's fp32 bar."""
+    import sparseconvnet_b200 as scn
+    torch.manual_seed(n + cin)
+    layer = scn.NetworkInNetwork(cin, cout, True).to(cuda)
+    f = torch.randn(n, cin, device=cuda, requires_grad=True)
+    y = layer(scn.SparseConvNetTensor(f, None, None)).features
+    g = torch.randn_like(y)
+    y.backward(g)
+    fd, gd, wd = f.detach().double(), g.double(), layer.weight.detach().double()
+    for got, want in ((y, fd @ wd + layer.bias.detach().double()), (f.grad, gd @ wd.t()), (layer.weight.grad, fd.t() @ gd),
+                      (layer.bias.grad, gd.sum(0))):
+        assert helpers.rel_err(got.detach().double().cpu().numpy(), want.cpu().numpy()) <= helpers.FP32_TOL
+
+
+@pytest.mark.parametrize("planes", [4, 20, 32, 36, 100])
+@pytest.mark.parametrize("n", [5, 33, 64, 257, 40001])
+def test_batchnorm_training_sums(n, planes, cuda):
+    """k_bn_stats4 and k_bn_back_sums4 against torch in float64; fp32 sums of a few hundred values each, added in double.
+    At least five rows: the gradient is g minus its projections on 1 and on the normalised row, and with two rows nothing
+    but eps / var of it is left, rounding errors of 2^-23 g times up to var / eps = 1e4."""
+    import sparseconvnet_b200 as scn
+    torch.manual_seed(n + planes)
+    layer = scn.BatchNormLeakyReLU(planes, leakiness=0.25).to(cuda)
+    torch.nn.init.uniform_(layer.weight, 0.5, 1.5)
+    torch.nn.init.uniform_(layer.bias, -1, 1)
+    x = torch.randn(n, planes, device=cuda, requires_grad=True)
+    y = layer(scn.SparseConvNetTensor(x, None, None)).features
+    g = torch.randn_like(y)
+    y.backward(g)
+    xd, w, b = (t.detach().double().requires_grad_() for t in (x, layer.weight, layer.bias))
+    mean, var = xd.mean(0), xd.var(0, unbiased=False)
+    z = (xd - mean) / torch.sqrt(var + layer.eps) * w + b
+    yd = torch.where(z > 0, z, 0.25 * z)
+    yd.backward(torch.where((y.detach() > 0) == (z.detach() > 0), g, torch.zeros_like(g)).double())
+    assert helpers.rel_err(y.detach().double().cpu().numpy(), yd.detach().cpu().numpy()) <= helpers.FP32_TOL
+    same = ((y.detach() > 0) == (z.detach() > 0)).all()
+    if same:  # (a value within rounding of zero may take the other slope)
+        for got, want in ((x.grad, xd.grad), (layer.weight.grad, w.grad), (layer.bias.grad, b.grad)):
+            assert helpers.rel_err(got.double().cpu().numpy(), want.cpu().numpy()) <= helpers.FP32_TOL
