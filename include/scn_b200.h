@@ -395,7 +395,8 @@ SCN_API int scn_convolution_bn_forward(scn_metadata *md, const int64_t *input_si
  * store (bn_scale / bn_shift, may be NULL).  groups = 1; planes_a a multiple of eight, planes_b of four.  The
  * tcgen05 kernels read the two matrices where they lie, in the pass that splits their input rows; for the other
  * kernels the library writes the (normalised) concatenation to a scratch matrix first.  Same bits as JoinTable,
- * BatchNormalization, SubmanifoldConvolution, BatchNormalization one after the other.  Not in the reference. */
+ * BatchNormalization, SubmanifoldConvolution, BatchNormalization one after the other.  in_b NULL with planes_b 0: a
+ * single matrix behind a BatchNormalization.  Not in the reference. */
 SCN_API int scn_submanifold_convolution_joined_forward(scn_metadata *md, const int64_t *spatial_size,
                                                        const int64_t *filter_size, const float *in_a, int planes_a,
                                                        const float *in_b, int planes_b, float *out_features,

@@ -548,7 +548,7 @@ def SubmanifoldConvolution_updateOutput(inputSize, filterSize, m, input_features
     """sparseconvnet.h:101-104.  `epilogue` (not in the reference): see batchnorm_fold.  `token`: see weight_token."""
     if Profile.active is None:  # the convolution entry finds or builds the rulebook itself
         return _macs(_binding.submanifold_convolution(m.handle, inputSize, filterSize, input_features, output_features,
-                                                      weight, bias, epilogue, _precision, token))
+                                                      weight, bias, epilogue, _precision, token, None))
     f, w, b, groups, cin, cout = _conv_args(input_features, weight, bias)
     macs = C.c_double()
     with _on_device(f.device), weight_token(token):

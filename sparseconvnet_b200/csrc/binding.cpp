@@ -240,9 +240,9 @@ struct Output {
 // ---- convolutions -------------------------------------------------------------------------------------------------
 // Every forward call takes the output tensor it is to size and fill, or None: then it makes one and returns (output,
 // count) instead of the count alone.
-// (md, size, filter, features, out, weight, bias, epilogue, precision, token)
+// (md, size, filter, features, out, weight, bias, epilogue, precision, token, prologue)
 SCN_FN(submanifold_convolution) {
-  SCN_BEGIN(10)
+  SCN_BEGIN(11)
   scn_metadata *md = md_of(a[0]);
   const Sizes size(a[1]), filter(a[2]);
   const at::Tensor &f = features(a[3], "input_features");
@@ -251,7 +251,7 @@ SCN_FN(submanifold_convolution) {
   const int nin = w.groups * w.cin, nout = w.groups * w.cout;
   if (f.numel() && f.size(1) != nin) fail("features have %d planes, weight expects %d", (int)f.size(1), nin);
   const float *bias = optional(a[6], f, "bias");
-  const Affine bn(a[7], f, nout);
+  const Affine bn(a[7], f, nout), pre(a[10], f, nin);
   const int precision = (int)PyLong_AsLong(a[8]);
   const OnDevice on(f);
   const Token token(a[9]);
@@ -259,7 +259,11 @@ SCN_FN(submanifold_convolution) {
   same_rows(f, n);
   out.size({n, nout});
   double macs = 0;
-  if (bn.scale)
+  if (pre.scale)
+    SCN_CALL(scn_submanifold_convolution_joined_forward(md, size.p, filter.p, ptr(f), nin, nullptr, 0, out.ptr(), ptr(w.w), bias,
+                                                        pre.scale, pre.shift, pre.leak, bn.scale, bn.shift, bn.leak, nout,
+                                                        precision, on.stream, &macs));
+  else if (bn.scale)
     SCN_CALL(scn_submanifold_convolution_bn_forward(md, size.p, filter.p, ptr(f), out.ptr(), ptr(w.w), bias, bn.scale,
                                                  bn.shift, bn.leak, nin, nout, w.groups, precision, on.stream, &macs));
   else

@@ -597,14 +597,16 @@ int scn_submanifold_convolution_joined_forward(scn_metadata *md, const int64_t *
                                                int n_out_planes, int precision, void *stream_, double *macs) {
   cudaStream_t stream = (cudaStream_t)stream_;
   SCN_REQUIRE(md && spatial_size && filter_size, SCN_ERR_BAD_ARG, "null argument");
-  SCN_REQUIRE(planes_a >= 8 && planes_b >= 4 && planes_a % 8 == 0 && planes_b % 4 == 0, SCN_ERR_UNSUPPORTED,
-              "joined input: %d + %d planes unsupported (a multiple of eight, then a multiple of four)", planes_a, planes_b);
+  const bool single = planes_b == 0 && !in_b;  // no join, only the BatchNorm in front
+  SCN_REQUIRE(single ? planes_a >= 1 : planes_a >= 8 && planes_b >= 4 && planes_a % 8 == 0 && planes_b % 4 == 0,
+              SCN_ERR_UNSUPPORTED, "joined input: %d + %d planes unsupported (a multiple of eight, then a multiple of four)",
+              planes_a, planes_b);
   Rulebook *rb = nullptr;
   SCN_TRY(get_submanifold_rulebook(md, spatial_size, filter_size, stream, &rb));
-  SCN_REQUIRE(rb->n_in == 0 || (in_a && in_b), SCN_ERR_BAD_ARG, "null features");
+  SCN_REQUIRE(rb->n_in == 0 || (in_a && (in_b || single)), SCN_ERR_BAD_ARG, "null features");
   return run_conv(md, *rb, false, in_a, out_features, weight, bias, planes_a + planes_b, n_out_planes, 1, precision,
                   stream, macs, false, bn_scale, bn_shift, (float)leakiness, pre_scale, pre_shift, (float)pre_leakiness,
-                  in_b, planes_a);
+                  in_b, single ? 0 : planes_a);
 }
 
 int scn_convolution_bn_bn_forward(scn_metadata *md, const int64_t *input_size, const int64_t *output_size,

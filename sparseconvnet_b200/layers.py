@@ -211,15 +211,15 @@ class SubmanifoldConvolution(_ConvBase):
         Module.__init__(self)
         self._init_weight(dimension, nIn, nOut, filter_size, bias, groups)
 
-    def forward(self, input, bn=None):
-        """`bn` (used by Sequential): an eval-mode BatchNormalization that follows this layer and is
-        applied in the convolution's store instead of as a pass of its own."""
+    def forward(self, input, bn=None, pre_bn=None):
+        """`bn` / `pre_bn` (used by Sequential): eval-mode BatchNormalizations behind / in front of this layer that are
+        applied in the convolution's store / in the pass that splits its rows, instead of as passes of their own."""
         features, params = input.features, self._parameters
         weight, bias = params["weight"], params.get("bias")
         assert features.nelement() == 0 or features.size(1) == self.nIn, (self.nIn, self.nOut, input)
         output = SparseConvNetTensor(metadata=input.metadata, spatial_size=input.spatial_size)
         if autograd.needs_grad(features, weight, bias):
-            assert bn is None
+            assert bn is None and pre_bn is None
             bias = optional_tensor(self, "bias")
             output.features, macs = autograd.convolution(
                 autograd.SUBMANIFOLD, features, weight, bias.to(weight.device), input.metadata,
@@ -227,8 +227,10 @@ class SubmanifoldConvolution(_ConvBase):
         elif SCN.Profile.active is None:
             return self._run(SCN._binding.submanifold_convolution, output, input.metadata.handle, input.spatial_size,
                              self.filter_size, features.contiguous(), None, weight, bias,
-                             bn.folded() if bn is not None else None, SCN._precision, self._weight_token())
+                             bn.folded() if bn is not None else None, SCN._precision, self._weight_token(),
+                             pre_bn.folded() if pre_bn is not None else None)
         else:
+            assert pre_bn is None  # (Sequential asks for it in unprofiled passes only)
             output.features = features.new_empty(0)
             macs = SCN.SubmanifoldConvolution_updateOutput(
                 input.spatial_size, self.filter_size, input.metadata, features.detach().contiguous(),

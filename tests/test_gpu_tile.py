@@ -126,3 +126,34 @@ def test_fp32_tiles(n, split, cin, cout, cuda, monkeypatch):
             e = helpers.rel_err(y.double().cpu().numpy(), want.cpu().numpy())
             assert e <= 1e-5, (layer, e)
             x.metadata.poll_errors()
+
+
+@pytest.mark.parametrize("precision", ["tf32x3", "bf16"])
+@pytest.mark.parametrize("n,planes", [(1, 8), (700, 24), (9000, 32), (9000, 64)])
+def test_batchnorm_in_front(n, planes, precision, cuda):
+    """A residual block's BatchNorm in front of its convolution rides in the pass that splits the rows: the same bits."""
+    import sparseconvnet_b200 as scn
+    torch.manual_seed(planes)
+    net = scn.Sequential()
+    for _ in range(2):
+        net.add(scn.ConcatTable().add(scn.Identity()).add(
+            scn.Sequential().add(scn.BatchNormLeakyReLU(planes, leakiness=0.2)).add(scn.SubmanifoldConvolution(3, planes, planes, 3, True))
+            .add(scn.BatchNormReLU(planes)).add(scn.SubmanifoldConvolution(3, planes, planes, 3, False)))).add(scn.AddTable())
+    for m in net.modules():
+        if isinstance(m, scn.BatchNormalization):
+            for t in (m.running_mean, m.running_var, m.weight, m.bias):
+                torch.nn.init.uniform_(t, 0.3, 1.0)
+    net.to(cuda).eval()
+    coords = _points(n, 3, 120, n)
+    feats = torch.randn(len(coords), planes, device=cuda)
+    outs = []
+    try:
+        scn.set_precision(precision)
+        for fuse in (False, True):
+            scn.Sequential.fuse = fuse
+            with torch.no_grad():
+                outs.append(net(scn.InputLayer(3, 120, mode=0)([torch.from_numpy(coords), feats])).features)
+    finally:
+        scn.set_precision("fp32")
+        scn.Sequential.fuse = True
+    assert torch.equal(*outs)
