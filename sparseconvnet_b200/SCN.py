@@ -648,12 +648,15 @@ def SubmanifoldConvolution_joined(inputSize, filterSize, m, inputs, output_featu
 def strided_chain_start(m, inputSize, filterSize, filterStride, levels, device):
     """strided_chain without the wait (scn_md_strided_chain_start): the chain's kernels go to the library's side
     stream behind what the current stream holds now and run beside what is enqueued next; the call that first
-    needs one of the levels takes them over.  Not in the reference."""
+    needs one of the levels takes them over.  Not in the reference.  `device`: that of the features, or a tensor on it."""
     if levels < 2:
         return
-    with _on_device(device):
-        check(lib.scn_md_strided_chain_start(m._h, sizes(inputSize), sizes(filterSize), sizes(filterStride),
-                                             int(levels), _stream()))
+    if torch.is_tensor(device):
+        _binding.strided_chain_start(m.handle, inputSize, filterSize, filterStride, int(levels), device)
+    else:
+        with _on_device(device):
+            check(lib.scn_md_strided_chain_start(m._h, sizes(inputSize), sizes(filterSize), sizes(filterStride),
+                                                 int(levels), _stream()))
     m.chain_started = True
 
 

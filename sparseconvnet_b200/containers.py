@@ -1,6 +1,7 @@
 """Containers (reference: sparseconvnet/sequential.py:10-33, sparseconvnet/tables.py:13-55)."""
 import torch
 
+from . import layers
 from .sparse_tensor import SparseConvNetTensor
 
 
@@ -16,7 +17,6 @@ def _flatten(seq, out):
 
 def _keeps_sites(m):
     """True for a module whose output has the sites and the spatial size of its input."""
-    from . import layers
     if isinstance(m, (layers.SubmanifoldConvolution, layers.BatchNormalization, layers.Identity, layers.NetworkInNetwork,
                       AddTable, JoinTable)):
         return True
@@ -29,7 +29,6 @@ def _keeps_sites(m):
 
 def _window(m):
     """(size, stride) of a module that goes one level down, None for any other."""
-    from . import layers
     if isinstance(m, layers.Convolution):
         return m.filter_size, m.filter_stride
     if isinstance(m, (layers.MaxPooling, layers.AveragePooling)):
@@ -87,7 +86,6 @@ class Sequential(torch.nn.Sequential):
     prefetch_rulebooks = True
 
     def forward(self, input):
-        from . import layers
         steps = _flatten(self, [])
         i, n = 0, len(steps)
         while i < n:
@@ -96,13 +94,13 @@ class Sequential(torch.nn.Sequential):
                 input.metadata.chain_looked_for = True  # one look per Metadata, by the outermost container
                 ahead = _chain_ahead(steps[i:])
                 if ahead is not None:
-                    layers.SCN.strided_chain_start(input.metadata, input.spatial_size, *ahead, input.features.device)
+                    layers.SCN.strided_chain_start(input.metadata, input.spatial_size, *ahead, input.features)
             m = steps[i]
             nxt = steps[i + 1] if i + 1 < n else None
             if (Sequential.fuse and isinstance(m, layers._ConvBase) and isinstance(nxt, layers.BatchNormalization)
                     and not m._forward_hooks and not m._forward_pre_hooks
                     and input.features.nelement() > 0 and nxt.fusable(input.features)
-                    and not layers.autograd.needs_grad(input.features, m.weight)):
+                    and not layers.autograd.needs_grad(input.features, m._parameters["weight"])):
                 input = m.forward(input, bn=nxt)  # (no output rows: nothing to apply, as the BatchNorm itself)
                 i += 2
                 continue
@@ -114,7 +112,7 @@ class Sequential(torch.nn.Sequential):
                     and not m._forward_hooks and not m._forward_pre_hooks and not nxt._forward_hooks
                     and not nxt._forward_pre_hooks and isinstance(input, SparseConvNetTensor)
                     and input.features.nelement() > 0 and m.fusable(input.features)
-                    and not layers.autograd.needs_grad(input.features, nxt.weight, getattr(nxt, "bias", None))):
+                    and not layers.autograd.needs_grad(input.features, nxt._parameters["weight"], nxt._parameters.get("bias"))):
                 post = nxt2 if (isinstance(nxt2, layers.BatchNormalization) and nxt2.fusable(input.features)) else None
                 input = nxt.forward(input, bn=post, pre_bn=m)
                 i += 3 if post is not None else 2
@@ -127,7 +125,7 @@ class Sequential(torch.nn.Sequential):
                     and not m._forward_hooks and not m._forward_pre_hooks and not nxt._forward_hooks
                     and not nxt._forward_pre_hooks and isinstance(input, SparseConvNetTensor)
                     and input.features.nelement() > 0 and input.features.size(1) == nxt.nIn and m.fusable(input.features)
-                    and not layers.autograd.needs_grad(input.features, nxt.weight, getattr(nxt, "bias", None))):
+                    and not layers.autograd.needs_grad(input.features, nxt._parameters["weight"], nxt._parameters.get("bias"))):
                 post = nxt2 if (isinstance(nxt2, layers.BatchNormalization) and nxt2.fusable(input.features)) else None
                 input = nxt.forward(input, bn=post, pre_bn=m)
                 i += 3 if post is not None else 2
@@ -141,7 +139,7 @@ class Sequential(torch.nn.Sequential):
                     and len(input) == 2 and all(t.features.nelement() > 0 and t.features.dim() == 2 for t in input)
                     and nxt.fusable(input[0].features) and nxt2.groups == 1
                     and not any(layers.autograd.needs_grad(t.features) for t in input)
-                    and not layers.autograd.needs_grad(input[0].features, nxt2.weight, getattr(nxt2, "bias", None))):
+                    and not layers.autograd.needs_grad(input[0].features, nxt2._parameters["weight"], nxt2._parameters.get("bias"))):
                 nxt3 = steps[i + 3] if i + 3 < n else None
                 post = nxt3 if (isinstance(nxt3, layers.BatchNormalization) and nxt3.fusable(input[0].features)) else None
                 joined = nxt2.forward_joined(input, pre_bn=nxt, bn=post)

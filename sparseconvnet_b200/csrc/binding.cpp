@@ -894,6 +894,18 @@ SCN_FN(input_layer) {
   SCN_END
 }
 
+// (md, size, filter, stride, levels, features): the levels below `size` started on the side stream
+SCN_FN(strided_chain_start) {
+  SCN_BEGIN(6)
+  scn_metadata *md = md_of(a[0]);
+  const Sizes size(a[1]), filter(a[2]), stride(a[3]);
+  const int levels = (int)PyLong_AsLong(a[4]);
+  const OnDevice on(tensor(a[5], "features"));
+  SCN_CALL(scn_md_strided_chain_start(md, size.p, filter.p, stride.p, levels, on.stream));
+  Py_RETURN_NONE;
+  SCN_END
+}
+
 // ---- small things the layers ask for on every call ----------------------------------------------------------------
 // (md, size) -> active sites
 SCN_FN(active_sites) {
@@ -962,7 +974,7 @@ PyMethodDef methods[] = {
     SCN_METHOD(pooling_forward),         SCN_METHOD(pooling_backward),   SCN_METHOD(sparse_to_dense),
     SCN_METHOD(active_sites),            SCN_METHOD(strided_size),       SCN_METHOD(transposed_size),
     SCN_METHOD(convolution_train),       SCN_METHOD(batchnorm_train),    SCN_METHOD(pooling_train),
-    SCN_METHOD(rows_affine_train),       SCN_METHOD(input_layer),             SCN_METHOD(versions),           SCN_METHOD(set_check),                    {nullptr, nullptr, 0, nullptr}};
+    SCN_METHOD(strided_chain_start),     SCN_METHOD(rows_affine_train),       SCN_METHOD(input_layer),             SCN_METHOD(versions),           SCN_METHOD(set_check),                    {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_binding", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -856,15 +856,16 @@ __device__ __forceinline__ void post_counts(unsigned long long *counts, int K, v
 // input = output + delta_k with delta = k_d - f_d / 2 (SubmanifoldConvolutionRules.h:15-19).
 // The neighbour's key is the site's key plus a per-offset constant, so a probe is a bounds
 // check, one 64-bit add and one 32-byte bucket read; the buckets of kAhead offsets are read before the first is looked at.
-// Bound by instruction issue and the latency of the bucket reads: 400 k sites, 27 offsets: 85 us (101 with coordinates
-// in local memory and one bucket at a time).
+// Bound by instruction issue and the latency of the bucket reads, which threads hide better than reads ahead do, whose
+// registers cost threads (400 k sites, 27 offsets: 76, 81, 91, 104 us with 1, 2, 3, 5 ahead, 101 with coordinates in local
+// memory; 1.5 M sites, 81 offsets: 758, 714, 796 us with 1, 2, 3).
 template <int DIM>
 __global__ void __launch_bounds__(256)
 k_submanifold_rules(KeyLayout L, HashTable T, const unsigned long long *__restrict__ row_keys,
                     long long n, int K, FilterDesc F, int k_chunk, int *__restrict__ nbr,
                     unsigned long long *counts, int mirrored, unsigned *__restrict__ masks, int mask_words,
                     volatile unsigned long long *counts_host) {
-  constexpr int kDim = DIM ? DIM : kMaxDim, kAhead = 3;
+  constexpr int kDim = DIM ? DIM : kMaxDim, kAhead = DIM == 4 ? 2 : 1;
   __shared__ long long sh_keydelta[32];
   __shared__ int sh_count[32];
   __shared__ signed char sh_delta[32][kDim];
