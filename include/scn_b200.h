@@ -261,6 +261,13 @@ SCN_API int scn_tc_probe_mma(int m, int n, int kind_bf16, int a_in_tmem, int n_m
  * of the call that first needed it; calls on other streams must be ordered after that one.
  * No counterpart in the reference. */
 SCN_API int scn_set_weight_token(uint64_t token);
+/* Feature rows in the form the tensor-core convolutions read: per row and slice of planes the bf16 parts h = bf16(x) and,
+ * except for SCN_PRECISION_BF16, m = bf16(x - h); 2 or 4 bytes per plane, opaque to the caller.  The calling thread's next
+ * forward convolution on those kernels reads in_split (may be NULL) instead of splitting its input -- rows that an earlier
+ * convolution of the same precision left there -- and leaves its result at out_split (may be NULL; n_out * n_out_planes * 4
+ * or 2 bytes) as well.  scn_split_rows_written: whether it did; forgets both.  No counterpart in the reference. */
+SCN_API int scn_set_split_rows(const void *in_split, void *out_split);
+SCN_API int scn_split_rows_written(void);
 SCN_API int scn_release_weight_token(uint64_t token, void *stream);
 
 /* The convolution operators return the reference's multiply-add count (rules x planes in x planes

@@ -548,7 +548,7 @@ def SubmanifoldConvolution_updateOutput(inputSize, filterSize, m, input_features
     """sparseconvnet.h:101-104.  `epilogue` (not in the reference): see batchnorm_fold.  `token`: see weight_token."""
     if Profile.active is None:  # the convolution entry finds or builds the rulebook itself
         return _macs(_binding.submanifold_convolution(m.handle, inputSize, filterSize, input_features, output_features,
-                                                      weight, bias, epilogue, _precision, token, None))
+                                                      weight, bias, epilogue, _precision, token, None, None, False))
     f, w, b, groups, cin, cout = _conv_args(input_features, weight, bias)
     macs = C.c_double()
     with _on_device(f.device), weight_token(token):
@@ -617,7 +617,7 @@ def SubmanifoldConvolution_joined(inputSize, filterSize, m, inputs, output_featu
         return None
     if Profile.active is None:
         return _macs(_binding.submanifold_joined(m.handle, inputSize, filterSize, inputs[0], inputs[1], output_features,
-                                                 weight, bias, prologue, epilogue, _precision, token))
+                                                 weight, bias, prologue, epilogue, _precision, token, False))
     fa, fb = (_features(f, "input_features") for f in inputs)
     ca, cb = fa.size(1), fb.size(1)
     if fa.size(0) != fb.size(0) or ca % 8 or cb % 4 or fa.device != fb.device or weight.size(2) != ca + cb:
@@ -666,7 +666,8 @@ def Convolution_updateOutput(inputSize, outputSize, filterSize, filterStride, m,
     reference): the same triple for an eval-mode BatchNorm in FRONT of the layer (scn_convolution_bn_bn_forward)."""
     if Profile.active is None:
         return _macs(_binding.convolution(m.handle, inputSize, outputSize, filterSize, filterStride, input_features,
-                                          output_features, weight, bias, epilogue, prologue, _precision, token))
+                                          output_features, weight, bias, epilogue, prologue, _precision, token, None,
+                                          False))
     f, w, b, groups, cin, cout = _conv_args(input_features, weight, bias)
     macs = C.c_double()
     n_out = C.c_int64()
@@ -716,7 +717,7 @@ def Deconvolution_updateOutput(inputSize, outputSize, filterSize, filterStride, 
     """sparseconvnet.h:149-154.  `epilogue` (not in the reference): see batchnorm_fold."""
     if Profile.active is None:
         return _macs(_binding.deconvolution(m.handle, inputSize, outputSize, filterSize, filterStride, input_features,
-                                            output_features, weight, bias, epilogue, _precision, token))
+                                            output_features, weight, bias, epilogue, _precision, token, None, False))
     f, w, b, groups, cin, cout = _conv_args(input_features, weight, bias)
     macs = C.c_double()
     with _on_device(f.device), weight_token(token):

@@ -24,6 +24,8 @@ SIGNATURES = {
     "scn_tc_probe_mma": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _vp,
                                    C.POINTER(C.c_double), C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "scn_test_drop_barrier_arrival": (C.c_int, []),
+    "scn_set_split_rows": (C.c_int, [_vp, _vp]),
+    "scn_split_rows_written": (C.c_int, []),
     "scn_set_weight_token": (C.c_int, [C.c_uint64]),
     "scn_release_weight_token": (C.c_int, [C.c_uint64, _vp]),
     "scn_set_deferred_counts": (C.c_int, [C.c_int]),

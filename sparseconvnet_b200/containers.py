@@ -66,6 +66,15 @@ def _chain_ahead(steps):
     return None if levels < 2 else (found[0], found[1], levels)
 
 
+def _wants_split(conv, follower):
+    """True if the convolution behind `conv` reads what `conv` makes, and in the split form of the tensor-core kernels."""
+    return (follower is not None and type(follower) in (layers.SubmanifoldConvolution, layers.Convolution, layers.Deconvolution)
+            and layers.SCN._precision != layers.SCN.PRECISION_FP32 and conv.groups == 1 and follower.groups == 1
+            and conv.nOut == follower.nIn and conv.nOut % 16 == 0 and layers.SCN.Profile.active is None
+            and type(conv) in (layers.SubmanifoldConvolution, layers.Convolution, layers.Deconvolution)
+            and not torch.is_inference_mode_enabled())  # (inference tensors have no version to check)
+
+
 class Sequential(torch.nn.Sequential):
     """Runs its children in order, like the reference's container.  Peepholes (inference only, same
     arithmetic and the same bits as the separate layers; `Sequential.fuse = False` turns them off):
@@ -75,6 +84,9 @@ class Sequential(torch.nn.Sequential):
     (or of a SubmanifoldConvolution on the tensor cores) is applied by that convolution to its input; JoinTable -> BatchNormalization ->
     SubmanifoldConvolution is one call on the tensors that would have been joined; a JoinTable
     followed by a BatchNormalization alone is one pass without the concatenation.
+
+    A convolution whose result the next step's convolution reads leaves it in that one's split form as well, in its
+    own store, which saves the pass that would make it.
 
     And one look ahead (`Sequential.prefetch_rulebooks = False` turns it off): the first Sequential that sees a
     tensor of a new Metadata looks for the first layer that goes down -- a Convolution, which the builders mark with
@@ -101,7 +113,10 @@ class Sequential(torch.nn.Sequential):
                     and not m._forward_hooks and not m._forward_pre_hooks
                     and input.features.nelement() > 0 and nxt.fusable(input.features)
                     and not layers.autograd.needs_grad(input.features, m._parameters["weight"])):
-                input = m.forward(input, bn=nxt)  # (no output rows: nothing to apply, as the BatchNorm itself)
+                if _wants_split(m, steps[i + 2] if i + 2 < n else None):
+                    input = m.forward(input, bn=nxt, want_split=True)
+                else:
+                    input = m.forward(input, bn=nxt)  # (no output rows: nothing to apply, as the BatchNorm itself)
                 i += 2
                 continue
             # an eval-mode BatchNormalization whose result goes straight into a strided Convolution (the way down of a
@@ -114,8 +129,10 @@ class Sequential(torch.nn.Sequential):
                     and input.features.nelement() > 0 and m.fusable(input.features)
                     and not layers.autograd.needs_grad(input.features, nxt._parameters["weight"], nxt._parameters.get("bias"))):
                 post = nxt2 if (isinstance(nxt2, layers.BatchNormalization) and nxt2.fusable(input.features)) else None
-                input = nxt.forward(input, bn=post, pre_bn=m)
-                i += 3 if post is not None else 2
+                after = i + (3 if post is not None else 2)
+                input = nxt.forward(input, bn=post, pre_bn=m,
+                                    want_split=_wants_split(nxt, steps[after] if after < n else None))
+                i = after
                 continue
             # the same in front of a SubmanifoldConvolution on the tensor cores, which has that pass (a residual block: the
             # sum in front of the BatchNormalization is needed as it is as well)
@@ -127,8 +144,10 @@ class Sequential(torch.nn.Sequential):
                     and input.features.nelement() > 0 and input.features.size(1) == nxt.nIn and m.fusable(input.features)
                     and not layers.autograd.needs_grad(input.features, nxt._parameters["weight"], nxt._parameters.get("bias"))):
                 post = nxt2 if (isinstance(nxt2, layers.BatchNormalization) and nxt2.fusable(input.features)) else None
-                input = nxt.forward(input, bn=post, pre_bn=m)
-                i += 3 if post is not None else 2
+                after = i + (3 if post is not None else 2)
+                input = nxt.forward(input, bn=post, pre_bn=m,
+                                    want_split=_wants_split(nxt, steps[after] if after < n else None))
+                i = after
                 continue
             # JoinTable -> eval-mode BatchNormalization -> SubmanifoldConvolution (-> BatchNormalization): the layers
             # behind the skip connection of a U-Net as one call; the convolution reads the joined tensors where they
@@ -142,10 +161,12 @@ class Sequential(torch.nn.Sequential):
                     and not layers.autograd.needs_grad(input[0].features, nxt2._parameters["weight"], nxt2._parameters.get("bias"))):
                 nxt3 = steps[i + 3] if i + 3 < n else None
                 post = nxt3 if (isinstance(nxt3, layers.BatchNormalization) and nxt3.fusable(input[0].features)) else None
-                joined = nxt2.forward_joined(input, pre_bn=nxt, bn=post)
+                after = i + (4 if post is not None else 3)
+                joined = nxt2.forward_joined(input, pre_bn=nxt, bn=post,
+                                             want_split=_wants_split(nxt2, steps[after] if after < n else None))
                 if joined is not None:
                     input = joined
-                    i += 4 if post is not None else 3
+                    i = after
                     continue
             # a JoinTable whose result goes straight into an eval-mode BatchNormalization: every joined tensor is
             # normalised into its columns of the result, the concatenation itself is never written

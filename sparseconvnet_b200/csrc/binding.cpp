@@ -190,6 +190,48 @@ struct Token {  // prepared weight images are kept under it while the call runs
   }
 };
 
+// Rows in the tensor cores' split form that travel with a tensor from the convolution that makes them to the one that reads
+// them: the input's (or None), and whether the result is wanted in that form too.
+struct Split {
+  at::Tensor made;
+  bool want;
+  Split(PyObject *in, PyObject *wanted) : want(PyObject_IsTrue(wanted) == 1) {
+    in_ = in == Py_None ? nullptr : tensor(in, "split rows").data_ptr();
+  }
+  void begin(const at::Tensor &out, int precision) {
+    if (!want && !in_) return;
+    if (want) {
+      const int64_t parts = precision == SCN_PRECISION_BF16 ? 1 : 2;
+      made = at::empty({out.size(0), out.size(1) * 2 * parts}, out.options().dtype(at::kByte));
+    }
+    scn_set_split_rows(in_, want && made.numel() ? made.data_ptr() : nullptr);
+    set_ = true;
+  }
+  // (output, count), or (output, count, split rows or None)
+  PyObject *finish(PyObject *pair) {
+    const bool written = set_ && scn_split_rows_written();
+    set_ = false;
+    if (!want || !pair || !PyTuple_Check(pair)) return pair;
+    PyObject *three = PyTuple_New(3);
+    for (int i = 0; i < 2; ++i) {
+      PyObject *o = PyTuple_GET_ITEM(pair, i);
+      Py_INCREF(o);
+      PyTuple_SET_ITEM(three, i, o);
+    }
+    Py_DECREF(pair);
+    if (!written) Py_INCREF(Py_None);
+    PyTuple_SET_ITEM(three, 2, written ? THPVariable_Wrap(std::move(made)) : Py_None);
+    return three;
+  }
+  ~Split() {
+    if (set_) scn_split_rows_written();  // (an error on the way)
+  }
+
+ private:
+  const void *in_ = nullptr;
+  bool set_ = false;
+};
+
 void size_to(const at::Tensor &t, at::IntArrayRef shape) { const_cast<at::Tensor &>(t).resize_(shape); }
 
 // The output of an operator: the caller's tensor, sized here, or (None) a new one that the call returns.
@@ -240,9 +282,10 @@ struct Output {
 // ---- convolutions -------------------------------------------------------------------------------------------------
 // Every forward call takes the output tensor it is to size and fill, or None: then it makes one and returns (output,
 // count) instead of the count alone.
-// (md, size, filter, features, out, weight, bias, epilogue, precision, token, prologue)
+// (md, size, filter, features, out, weight, bias, epilogue, precision, token, prologue, split rows, want split rows)
 SCN_FN(submanifold_convolution) {
-  SCN_BEGIN(11)
+  SCN_BEGIN(13)
+  Split split(a[11], a[12]);
   scn_metadata *md = md_of(a[0]);
   const Sizes size(a[1]), filter(a[2]);
   const at::Tensor &f = features(a[3], "input_features");
@@ -258,6 +301,7 @@ SCN_FN(submanifold_convolution) {
   const int64_t n = n_active(md, size);
   same_rows(f, n);
   out.size({n, nout});
+  split.begin(out.t, precision);
   double macs = 0;
   if (pre.scale)
     SCN_CALL(scn_submanifold_convolution_joined_forward(md, size.p, filter.p, ptr(f), nin, nullptr, 0, out.ptr(), ptr(w.w), bias,
@@ -269,14 +313,15 @@ SCN_FN(submanifold_convolution) {
   else
     SCN_CALL(scn_submanifold_convolution_forward(md, size.p, filter.p, ptr(f), out.ptr(), ptr(w.w), bias, nin, nout, w.groups,
                                               precision, on.stream, &macs));
-  return out.result(macs_result(md, macs));
+  return split.finish(out.result(macs_result(md, macs)));
   SCN_END
 }
 
-// (md, size, filter, features_a, features_b, out, weight, bias, prologue, epilogue, precision, token) -> None when the
+// (md, size, filter, features_a, features_b, out, weight, bias, prologue, epilogue, precision, token, want split rows) -> None when the
 // shapes are not ones the call takes
 SCN_FN(submanifold_joined) {
-  SCN_BEGIN(12)
+  SCN_BEGIN(13)
+  Split split(Py_None, a[12]);
   scn_metadata *md = md_of(a[0]);
   const Sizes size(a[1]), filter(a[2]);
   const at::Tensor &fa = features(a[3], "input_features"), &fb = features(a[4], "input_features");
@@ -293,17 +338,20 @@ SCN_FN(submanifold_joined) {
   const int64_t n = n_active(md, size);
   same_rows(fa, n);
   out.size({n, w.cout});
+  split.begin(out.t, precision);
   double macs = 0;
   SCN_CALL(scn_submanifold_convolution_joined_forward(md, size.p, filter.p, ptr(fa), ca, ptr(fb), cb, out.ptr(), ptr(w.w), bias,
                                                    pre.scale, pre.shift, pre.leak, bn.scale, bn.shift, bn.leak, w.cout,
                                                    precision, on.stream, &macs));
-  return out.result(macs_result(md, macs));
+  return split.finish(out.result(macs_result(md, macs)));
   SCN_END
 }
 
-// (md, in_size, out_size, filter, stride, features, out, weight, bias, epilogue, prologue, precision, token)
+// (md, in_size, out_size, filter, stride, features, out, weight, bias, epilogue, prologue, precision, token, split rows, want
+// split rows)
 SCN_FN(convolution) {
-  SCN_BEGIN(13)
+  SCN_BEGIN(15)
+  Split split(a[13], a[14]);
   scn_metadata *md = md_of(a[0]);
   const Sizes in_size(a[1]), out_size(a[2]), filter(a[3]), stride(a[4]);
   const at::Tensor &f = features(a[5], "input_features");
@@ -320,6 +368,7 @@ SCN_FN(convolution) {
   int64_t n_out = 0;
   SCN_CALL(scn_md_strided_rulebook(md, in_size.p, out_size.p, filter.p, stride.p, on.stream, &n_out, nullptr));
   out.size({n_out, nout});
+  split.begin(out.t, precision);
   double macs = 0;
   if (pre.scale)
     SCN_CALL(scn_convolution_bn_bn_forward(md, in_size.p, out_size.p, filter.p, stride.p, ptr(f), out.ptr(), ptr(w.w), bias,
@@ -331,13 +380,14 @@ SCN_FN(convolution) {
   else
     SCN_CALL(scn_convolution_forward(md, in_size.p, out_size.p, filter.p, stride.p, ptr(f), out.ptr(), ptr(w.w), bias, nin,
                                   nout, w.groups, precision, on.stream, &macs));
-  return out.result(macs_result(md, macs));
+  return split.finish(out.result(macs_result(md, macs)));
   SCN_END
 }
 
-// (md, in_size, out_size, filter, stride, features, out, weight, bias, epilogue, precision, token)
+// (md, in_size, out_size, filter, stride, features, out, weight, bias, epilogue, precision, token, split rows, want split rows)
 SCN_FN(deconvolution) {
-  SCN_BEGIN(12)
+  SCN_BEGIN(14)
+  Split split(a[12], a[13]);
   scn_metadata *md = md_of(a[0]);
   const Sizes in_size(a[1]), out_size(a[2]), filter(a[3]), stride(a[4]);
   const at::Tensor &f = features(a[5], "input_features");
@@ -354,6 +404,7 @@ SCN_FN(deconvolution) {
   SCN_CALL(scn_md_strided_rulebook(md, out_size.p, in_size.p, filter.p, stride.p, on.stream, nullptr, nullptr));
   same_rows(f, n_active(md, in_size));
   out.size({n_active(md, out_size), nout});
+  split.begin(out.t, precision);
   double macs = 0;
   if (bn.scale)
     SCN_CALL(scn_deconvolution_bn_forward(md, in_size.p, out_size.p, filter.p, stride.p, ptr(f), out.ptr(), ptr(w.w), bias,
@@ -361,7 +412,7 @@ SCN_FN(deconvolution) {
   else
     SCN_CALL(scn_deconvolution_forward(md, in_size.p, out_size.p, filter.p, stride.p, ptr(f), out.ptr(), ptr(w.w), bias, nin,
                                     nout, w.groups, precision, on.stream, &macs));
-  return out.result(macs_result(md, macs));
+  return split.finish(out.result(macs_result(md, macs)));
   SCN_END
 }
 

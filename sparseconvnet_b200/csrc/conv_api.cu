@@ -92,6 +92,16 @@ int split_mode_of_env(int dflt) {
   return dflt;
 }
 
+// ---- rows in split form from one layer to the next ------------------------------------------------------
+static thread_local SplitRows g_split_rows;
+static thread_local bool g_split_written = false;
+SplitRows take_split_rows() {
+  const SplitRows r = g_split_rows;
+  g_split_rows = SplitRows{};
+  return r;
+}
+void split_rows_written() { g_split_written = true; }
+
 // ---- prepared weight images kept under a caller-chosen token ------------------------------------------
 namespace {
 struct WeightKey {
@@ -450,6 +460,20 @@ using namespace scn;
 extern "C" {
 
 int scn_last_conv_kernel(void) { return g_last_kernel; }
+
+int scn_set_split_rows(const void *in_split, void *out_split) {
+  g_split_rows.in = in_split;
+  g_split_rows.out = out_split;
+  g_split_written = false;
+  return SCN_OK;
+}
+
+int scn_split_rows_written(void) {
+  const bool w = g_split_written;
+  g_split_written = false;
+  g_split_rows = SplitRows{};
+  return w;
+}
 
 int scn_set_weight_token(uint64_t token) {
   g_weight_token = token;

@@ -27,7 +27,7 @@ namespace scn {
 
 int sum_partial_tiles(const float *partial, int n_split, long long n_pos, int cout, const int *order, long long n_out,
                       const float *bias, const float *bn_scale, const float *bn_shift, float leak, float *out,
-                      cudaStream_t stream);
+                      cudaStream_t stream, unsigned char *out_split = nullptr, int out_sp = 1, int parts = 1);
 
 namespace {
 

@@ -75,6 +75,8 @@ struct TileParams {
   int n_stages, tmem_cols;
   long long n_tiles, n_items;
   int n_split;
+  unsigned char *out_split;  // (optional, n_split 1) the result once more as split rows, slices of out_sp planes
+  int out_sp;
   int drop;         // test hook: leave out one barrier arrival of the first CTA
   int *flags;
 };
@@ -148,7 +150,7 @@ __device__ __forceinline__ int item_offsets(const TileParams &P, long long item)
   return total * (part + 1) / P.n_split - total * part / P.n_split;
 }
 
-template <int TERMS, int SP>
+template <int TERMS, int SP, bool OUT_SPLIT>
 __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
   using Shape = TileShape<TERMS, SP>;
   constexpr int PP = Shape::PP, NI = Shape::NI, PARTS = Shape::PARTS;
@@ -426,33 +428,47 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
       }
       tc_fence_after();
       const unsigned base = tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(buf * dcols);
-      // where rows lane / 4, + 8, + 16, + 24 of the warp go, and this lane's four planes of them
+      // where rows lane / 4, + 8, + 16, + 24 of the warp go: this lane's four planes of them, or (OUT_SPLIT, which is short of
+      // registers) the row.  Two CTAs of 15 warps have 64 registers a thread, and which form fits them was measured: 32 planes
+      // on 200 k rows 51 us in both kernels, 56 with rows and eight columns at a time where nothing is split; 160 planes on
+      // 3 k rows 24 us, 26 with rows and sixteen columns.
       long long at[4];
+      int to[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = __shfl_sync(0xffffffffu, orow, i * 8 + (lane >> 2));
-        at[i] = r < 0 ? -1 : (P.n_split > 1 ? ((long long)part * P.n_tiles + t) * kRows + quad * 32 + i * 8 + (lane >> 2) : r) * nc + (lane & 3) * 4;
+        if (OUT_SPLIT) to[i] = r;
+        else at[i] = r < 0 ? -1 : (P.n_split > 1 ? ((long long)part * P.n_tiles + t) * kRows + quad * 32 + i * 8 + (lane >> 2) : r) * nc + (lane & 3) * 4;
       }
       for (int c0 = 0; c0 < nc; c0 += 16) {
-        unsigned a[16], b[16];
-        tmem_ld16_nowait(base + c0, a);
-        if (joint) tmem_ld16_nowait(base + P.coutp + c0, b);
-        tmem_wait_ld();
+        constexpr int kCols = OUT_SPLIT ? 8 : 16;
 #pragma unroll
-        for (int e = 0; e < 16; e += 4) {
-          float4 v;
-          v.x = __uint_as_float(a[e]), v.y = __uint_as_float(a[e + 1]), v.z = __uint_as_float(a[e + 2]), v.w = __uint_as_float(a[e + 3]);
-          if (joint) {
-            v.x += __uint_as_float(b[e]), v.y += __uint_as_float(b[e + 1]);
-            v.z += __uint_as_float(b[e + 2]), v.w += __uint_as_float(b[e + 3]);
+        for (int half = 0; half < 16; half += kCols) {
+          unsigned a[kCols], b[kCols];
+          if constexpr (OUT_SPLIT) {
+            tmem_ld8_nowait(base + c0 + half, a);
+            if (joint) tmem_ld8_nowait(base + P.coutp + c0 + half, b);
+          } else {
+            tmem_ld16_nowait(base + c0, a);
+            if (joint) tmem_ld16_nowait(base + P.coutp + c0, b);
           }
-          my_epi[lane * 4 + ((e >> 2) ^ ((lane >> 1) & 3))] = v;
+          tmem_wait_ld();
+#pragma unroll
+          for (int e = 0; e < kCols; e += 4) {
+            float4 v;
+            v.x = __uint_as_float(a[e]), v.y = __uint_as_float(a[e + 1]), v.z = __uint_as_float(a[e + 2]), v.w = __uint_as_float(a[e + 3]);
+            if (joint) {
+              v.x += __uint_as_float(b[e]), v.y += __uint_as_float(b[e + 1]);
+              v.z += __uint_as_float(b[e + 2]), v.w += __uint_as_float(b[e + 3]);
+            }
+            my_epi[lane * 4 + (((half + e) >> 2) ^ ((lane >> 1) & 3))] = v;
+          }
         }
         __syncwarp();
         const int c = c0 + (lane & 3) * 4;
         if (c < nc) {
           float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), sc = bias, sh = bias;
-          const bool finish = P.n_split == 1;
+          const bool finish = OUT_SPLIT || P.n_split == 1;
           if (finish && P.bias) bias = __ldg(reinterpret_cast<const float4 *>(P.bias + c));
           if (finish && P.bn_scale) {
             sc = __ldg(reinterpret_cast<const float4 *>(P.bn_scale + c));
@@ -462,7 +478,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
           for (int i = 0; i < 4; ++i) {
             const int row = i * 8 + (lane >> 2);
             float4 v = my_epi[row * 4 + ((lane & 3) ^ ((row >> 1) & 3))];
-            if (at[i] < 0) continue;
+            if (OUT_SPLIT ? to[i] < 0 : at[i] < 0) continue;
             if (finish && P.bias) v.x += bias.x, v.y += bias.y, v.z += bias.z, v.w += bias.w;
             if (finish && P.bn_scale) {  // separate multiply and add, as the stand-alone BatchNorm kernel rounds them
               v.x = __fadd_rn(__fmul_rn(v.x, sc.x), sh.x), v.y = __fadd_rn(__fmul_rn(v.y, sc.y), sh.y);
@@ -470,7 +486,16 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
               v.x *= v.x > 0.f ? 1.f : P.leak, v.y *= v.y > 0.f ? 1.f : P.leak;
               v.z *= v.z > 0.f ? 1.f : P.leak, v.w *= v.w > 0.f ? 1.f : P.leak;
             }
-            *reinterpret_cast<float4 *>(P.out + at[i] + c0) = v;
+            *reinterpret_cast<float4 *>(P.out + (OUT_SPLIT ? (long long)to[i] * nc + c : at[i] + c0)) = v;
+            if (OUT_SPLIT) {
+              uint2 h, m;
+              split_bf16_pair(v.x, v.y, h.x, m.x);
+              split_bf16_pair(v.z, v.w, h.y, m.y);
+              const int slice = c0 & -P.out_sp;  // (16, 32 or 64 planes)
+              unsigned char *q = P.out_split + ((long long)to[i] * nc + slice) * (2 * PARTS) + (c - slice) * 2;
+              *reinterpret_cast<uint2 *>(q) = h;
+              if (PARTS == 2) *reinterpret_cast<uint2 *>(q + P.out_sp * 2) = m;
+            }
           }
         }
         __syncwarp();
@@ -491,7 +516,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
 __global__ void __launch_bounds__(256)
 k_tile_sum(const float4 *__restrict__ partial, int n_split, long long n_pos, int cout4, const int *__restrict__ order,
            long long n_out, const float *__restrict__ bias, const float *__restrict__ bn_scale, const float *__restrict__ bn_shift,
-           float leak, float4 *__restrict__ out) {
+           float leak, float4 *__restrict__ out, unsigned char *__restrict__ out_split, int out_sp, int parts) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_pos * cout4) return;
   const int c = (int)(i % cout4);
@@ -514,6 +539,14 @@ k_tile_sum(const float4 *__restrict__ partial, int n_split, long long n_pos, int
     q.z *= q.z > 0.f ? 1.f : leak, q.w *= q.w > 0.f ? 1.f : leak;
   }
   out[r * cout4 + c] = q;
+  if (out_split) {
+    uint2 h, m;
+    split_bf16_pair(q.x, q.y, h.x, m.x);
+    split_bf16_pair(q.z, q.w, h.y, m.y);
+    unsigned char *s = out_split + (r * cout4 * 4 + c * 4 / out_sp * out_sp) * (2 * parts) + c * 4 % out_sp * 2;
+    *reinterpret_cast<uint2 *>(s) = h;
+    if (parts == 2) *reinterpret_cast<uint2 *>(s + out_sp * 2) = m;
+  }
 }
 
 // in [n][cin] fp32 (or the column-wise concatenation [in (planes_a) | in_b], read where the two lie) -> per row and
@@ -582,11 +615,11 @@ int slice_planes(int terms, int cin) {
   return c % 32 == 0 ? 32 : 16;
 }
 
-template <int TERMS, int SP>
-int launch_tile(TileParams &P, int n_sm, int dev, cudaStream_t stream) {
+template <int TERMS, int SP, bool OUT_SPLIT>
+int launch_tile_as(TileParams &P, int n_sm, int dev, cudaStream_t stream) {
   using Shape = TileShape<TERMS, SP>;
   static std::atomic<bool> configured[64];
-  auto kernel = k_conv_tile<TERMS, SP>;
+  auto kernel = k_conv_tile<TERMS, SP, OUT_SPLIT>;
   if (!configured[dev].load()) {
     SCN_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
     configured[dev].store(true);
@@ -608,14 +641,19 @@ int launch_tile(TileParams &P, int n_sm, int dev, cudaStream_t stream) {
   return SCN_OK;
 }
 
+template <int TERMS, int SP>
+int launch_tile(TileParams &P, int n_sm, int dev, cudaStream_t stream) {
+  return P.out_split ? launch_tile_as<TERMS, SP, true>(P, n_sm, dev, stream) : launch_tile_as<TERMS, SP, false>(P, n_sm, dev, stream);
+}
+
 }  // namespace
 
 // out = act((bias + the parts of partial [n_split][n_pos][cout], in order) * bn_scale + bn_shift); position p is row
-// order[p] (order null: row p)
+// order[p] (order null: row p).  out_split (optional): the result as split rows as well, see k_tile_split
 int sum_partial_tiles(const float *partial, int n_split, long long n_pos, int cout, const int *order, long long n_out,
                       const float *bias, const float *bn_scale, const float *bn_shift, float leak, float *out,
-                      cudaStream_t stream) {
-  SCN_LAUNCH(k_tile_sum, (unsigned)ceil_div(n_pos * (cout / 4), 256), 256, 0, stream, (const float4 *)partial, n_split, n_pos, cout / 4, order, n_out, bias, bn_scale, bn_shift, leak, (float4 *)out);
+                      cudaStream_t stream, unsigned char *out_split, int out_sp, int parts) {
+  SCN_LAUNCH(k_tile_sum, (unsigned)ceil_div(n_pos * (cout / 4), 256), 256, 0, stream, (const float4 *)partial, n_split, n_pos, cout / 4, order, n_out, bias, bn_scale, bn_shift, leak, (float4 *)out, out_split, out_sp, parts);
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }
@@ -672,11 +710,13 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
     SCN_LAUNCH(k_tile_weights, (unsigned)ceil_div((long long)K * cinp * coutp, 256), 256, 0, stream, weight,
                (unsigned char *)wi.ptr, K, cin, cout, coutp, n_slices, SP, parts);
 
-  // the input rows as bf16 parts, made once per call: a row is gathered by up to K output rows
+  // the input rows as bf16 parts, made once per call: a row is gathered by up to K output rows.  The layer that made the
+  // rows may have left them in this form already, and the next one may want them so.
+  const SplitRows rows = take_split_rows();
   unsigned char *split = nullptr;
-  const long long rows_in = std::max<long long>(n_in, 1);
-  SCN_TRY(device_alloc((void **)&split, (size_t)rows_in * cinp * 2 * parts, stream));
-  if (n_in > 0) {
+  const bool given = rows.in && !pre_scale && !in_b && cinp == cin;
+  if (!given) SCN_TRY(device_alloc((void **)&split, (size_t)std::max<long long>(n_in, 1) * cinp * 2 * parts, stream));
+  if (n_in > 0 && !given) {
     const int ppr = cinp / 8;
     const long long n_pieces = n_in * ppr;
     if (parts == 2)
@@ -686,7 +726,9 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
   }
 
   TileParams P{};
-  P.in_split = split;
+  P.in_split = given ? (const unsigned char *)rows.in : split;
+  P.out_sp = slice_planes(terms, cout);
+  unsigned char *out_split = rows.out && cout % P.out_sp == 0 ? (unsigned char *)rows.out : nullptr;
   P.row_bytes = (long long)cinp * 2 * parts;
   P.n_in = n_in;
   P.out = out;
@@ -713,6 +755,7 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
   P.n_split = e ? std::max(1, atoi(e)) : split_parts(P.n_tiles, K, n_slices, (a_bytes + w_bytes) / 32.0, cout, n_sm);
   float *partial = nullptr;
   int rc = SCN_OK;
+  P.out_split = P.n_split > 1 ? nullptr : out_split;
   if (P.n_split > 1) {
     rc = device_alloc((void **)&partial, (size_t)P.n_split * P.n_tiles * kRows * cout * sizeof(float), stream);
     P.out = partial;
@@ -724,7 +767,9 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
       rc = SP == 64 ? launch_tile<1, 64>(P, n_sm, dev, stream) : launch_tile<1, 32>(P, n_sm, dev, stream);
   }
   if (rc == SCN_OK && P.n_split > 1)
-    rc = sum_partial_tiles(partial, P.n_split, P.n_tiles * kRows, cout, ord.order, n_out, bias, bn_scale, bn_shift, leak, out, stream);
+    rc = sum_partial_tiles(partial, P.n_split, P.n_tiles * kRows, cout, ord.order, n_out, bias, bn_scale, bn_shift, leak, out, stream,
+                           out_split, P.out_sp, parts);
+  if (rc == SCN_OK && out_split) split_rows_written();
   device_free(partial, stream);
   device_free(split, stream);
   const int rf = weight_image_put(wi, stream);

@@ -129,6 +129,16 @@ int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
 int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int64_t *output_size,
                          const int64_t *filter_size, const int64_t *filter_stride,
                          cudaStream_t stream, Rulebook **out);
+// Feature rows in the split form of the tensor-core kernels (k_tile_split), handed from the layer that makes them to the
+// one that reads them: what the calling thread's next convolution may read instead of splitting its input, and where it may
+// leave its result in that form (scn_set_split_rows).
+struct SplitRows {
+  const void *in = nullptr;
+  void *out = nullptr;
+};
+SplitRows take_split_rows();  // (once)
+void split_rows_written();
+
 // host_keys.cu: host coordinates as packed keys in pinned, device-mapped memory
 int pinned_acquire(size_t bytes, void **p, size_t *got);
 void pinned_release(void *p, size_t bytes);

@@ -197,8 +197,11 @@ class _ConvBase(Module):
     def _run(self, call, output, *args):
         """A native convolution call that makes its own output tensor (inference; profiled passes and gradients take the
         functions of SCN.py)."""
-        output.features, macs = call(*args)
-        self._count(SCN._macs(macs), output.features)
+        made = call(*args)
+        output.features = features = made[0]
+        if len(made) == 3 and made[2] is not None:
+            output.split = (made[2], features, features._version, SCN._precision)
+        self._count(SCN._macs(made[1]), features)
         return output
 
     def _count(self, macs, output_features):
@@ -206,14 +209,21 @@ class _ConvBase(Module):
         _pkg.forward_pass_hidden_states += output_features.nelement()
 
 
+def _split_rows(input):
+    """The split form of a tensor's features, if it travels with them and still is theirs."""
+    s = input.split
+    return s[0] if s is not None and s[1] is input.features and s[2] == s[1]._version and s[3] == SCN._precision else None
+
+
 class SubmanifoldConvolution(_ConvBase):
     def __init__(self, dimension, nIn, nOut, filter_size, bias, groups=1):
         Module.__init__(self)
         self._init_weight(dimension, nIn, nOut, filter_size, bias, groups)
 
-    def forward(self, input, bn=None, pre_bn=None):
+    def forward(self, input, bn=None, pre_bn=None, want_split=False):
         """`bn` / `pre_bn` (used by Sequential): eval-mode BatchNormalizations behind / in front of this layer that are
-        applied in the convolution's store / in the pass that splits its rows, instead of as passes of their own."""
+        applied in the convolution's store / in the pass that splits its rows, instead of as passes of their own.
+        `want_split`: a convolution follows, which reads the result in split form."""
         features, params = input.features, self._parameters
         weight, bias = params["weight"], params.get("bias")
         assert features.nelement() == 0 or features.size(1) == self.nIn, (self.nIn, self.nOut, input)
@@ -228,7 +238,7 @@ class SubmanifoldConvolution(_ConvBase):
             return self._run(SCN._binding.submanifold_convolution, output, input.metadata.handle, input.spatial_size,
                              self.filter_size, features.contiguous(), None, weight, bias,
                              bn.folded() if bn is not None else None, SCN._precision, self._weight_token(),
-                             pre_bn.folded() if pre_bn is not None else None)
+                             pre_bn.folded() if pre_bn is not None else None, _split_rows(input), want_split)
         else:
             assert pre_bn is None  # (Sequential asks for it in unprofiled passes only)
             output.features = features.new_empty(0)
@@ -239,11 +249,18 @@ class SubmanifoldConvolution(_ConvBase):
         self._count(macs, output.features)
         return output
 
-    def forward_joined(self, inputs, pre_bn=None, bn=None):
+    def forward_joined(self, inputs, pre_bn=None, bn=None, want_split=False):
         """This layer applied to the concatenation of `inputs` (what a JoinTable in front of it would produce),
         through the eval-mode BatchNormalization `pre_bn` between the two if given, without the concatenation and
         the normalised copy being built as tensors of their own.  None when the shapes do not allow it."""
         output = SparseConvNetTensor(metadata=inputs[0].metadata, spatial_size=inputs[0].spatial_size)
+        if SCN.Profile.active is None and len(inputs) == 2:
+            a, b = (i.features.detach().contiguous() for i in inputs)
+            made = SCN._binding.submanifold_joined(
+                output.metadata.handle, output.spatial_size, self.filter_size, a, b, None, self._parameters["weight"],
+                self._parameters.get("bias"), pre_bn.folded() if pre_bn is not None else None,
+                bn.folded() if bn is not None else None, SCN._precision, self._weight_token(), want_split)
+            return None if made is None else self._run(lambda: made, output)
         output.features = inputs[0].features.new_empty(0)
         macs = SCN.SubmanifoldConvolution_joined(
             inputs[0].spatial_size, self.filter_size, inputs[0].metadata,
@@ -278,9 +295,10 @@ class Convolution(_ConvBase):
         self._init_weight(dimension, nIn, nOut, filter_size, bias, groups)
         self.filter_stride = to_long_tensor(dimension, filter_stride)
 
-    def forward(self, input, bn=None, pre_bn=None):
+    def forward(self, input, bn=None, pre_bn=None, want_split=False):
         """`bn` / `pre_bn` (used by Sequential): eval-mode BatchNormalizations behind / in front of this layer that
-        are applied inside the convolution call instead of as passes of their own."""
+        are applied inside the convolution call instead of as passes of their own.  `want_split` as in
+        SubmanifoldConvolution."""
         features, params = input.features, self._parameters
         weight, bias = params["weight"], params.get("bias")
         assert features.nelement() == 0 or features.size(1) == self.nIn
@@ -300,7 +318,7 @@ class Convolution(_ConvBase):
             return self._run(SCN._binding.convolution, output, input.metadata.handle, input.spatial_size, out_size,
                              self.filter_size, self.filter_stride, features.contiguous(), None, weight, bias,
                              bn.folded() if bn is not None else None, pre_bn.folded() if pre_bn is not None else None,
-                             SCN._precision, self._weight_token())
+                             SCN._precision, self._weight_token(), _split_rows(input), want_split)
         else:
             output.features = features.new_empty(0)
             macs = SCN.Convolution_updateOutput(
@@ -325,7 +343,7 @@ class Deconvolution(_ConvBase):
         self._init_weight(dimension, nIn, nOut, filter_size, bias, groups)
         self.filter_stride = to_long_tensor(dimension, filter_stride)
 
-    def forward(self, input, bn=None):
+    def forward(self, input, bn=None, want_split=False):
         features, params = input.features, self._parameters
         weight, bias = params["weight"], params.get("bias")
         assert features.nelement() == 0 or features.size(1) == self.nIn
@@ -339,7 +357,7 @@ class Deconvolution(_ConvBase):
         elif SCN.Profile.active is None:
             return self._run(SCN._binding.deconvolution, output, input.metadata.handle, input.spatial_size, out_size,
                              self.filter_size, self.filter_stride, features.contiguous(), None, weight, bias,
-                             bn.folded() if bn is not None else None, SCN._precision, self._weight_token())
+                             bn.folded() if bn is not None else None, SCN._precision, self._weight_token(), _split_rows(input), want_split)
         else:
             output.features = features.new_empty(0)
             macs = SCN.Deconvolution_updateOutput(

@@ -23,6 +23,10 @@ def optional_tensor(module, name):
 
 
 class SparseConvNetTensor(object):
+    # The features once more in the split form the tensor-core convolutions read, left by the convolution that made them
+    # for the one that follows: (rows, the features they belong to, their version, precision).  Not in the reference.
+    split = None
+
     def __init__(self, features=None, metadata=None, spatial_size=None):
         self.features = features
         self.metadata = metadata

@@ -157,3 +157,30 @@ def test_batchnorm_in_front(n, planes, precision, cuda):
         scn.set_precision("fp32")
         scn.Sequential.fuse = True
     assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("precision,planes", [("tf32x3", 16), ("tf32x3", 48), ("tf32x3", 64), ("bf16", 32), ("bf16", 64)])
+@pytest.mark.parametrize("n,split", [(1, "1"), (700, "1"), (700, "3"), (20000, None)])
+def test_split_rows_left_for_the_next_layer(n, split, planes, precision, cuda, monkeypatch):
+    """A convolution's result in split form, from its own store or from the sum of its parts: the next layer gives the same
+    bits with it as without, and does not use it once the features have changed."""
+    import sparseconvnet_b200 as scn
+    if split:
+        monkeypatch.setenv("SCN_TILE_SPLIT", split)
+    torch.manual_seed(planes)
+    a, b = (scn.SubmanifoldConvolution(3, planes, planes, 3, True).to(cuda) for _ in range(2))
+    coords = _points(n, 3, 120, n)
+    try:
+        scn.set_precision(precision)
+        with torch.no_grad():
+            x = scn.InputLayer(3, 120, mode=0)([torch.from_numpy(coords), torch.randn(len(coords), planes, device=cuda)])
+            y, z = a.forward(x, want_split=True), a(x)
+            assert y.split is not None and z.split is None
+            assert torch.equal(y.features, z.features)
+            assert torch.equal(b(y).features, b(z).features)
+            y.features.mul_(2)
+            z.features.mul_(2)
+            assert torch.equal(b(y).features, b(z).features)
+            x.metadata.poll_errors()
+    finally:
+        scn.set_precision("fp32")
