@@ -59,8 +59,7 @@ LIMITS = {
 DTYPE_LABEL = {
     "fp32": "f32 (fp32 FMA in every convolution)",
     "tf32x3": "f32-class split arithmetic, fp32 accumulate: every operand as two bf16 parts, three bf16 products "
-              "per term -- warp-level mma.sync.m16n8k16 for 32/64 output planes, tcgen05 kind::f16 with TMEM "
-              "accumulators for wider layers",
+              "per term on tcgen05 kind::f16 with TMEM accumulators",
     "tf32": "tf32 (single pass, fp32 accumulate)",
     "bf16": "bf16 (single pass, fp32 accumulate)",
 }

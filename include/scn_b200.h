@@ -22,8 +22,9 @@
  *    (sparseconvnet/SCN/Metadata/Metadata.h:44-167).  It is not thread safe, like the
  *    reference object.
  *  - device memory for tables, rulebooks and per-call scratch comes from a stream-ordered memory
- *    pool that the library creates per device (not the device's default pool); freed blocks stay
- *    in that pool for reuse until scn_trim_memory gives them back to the driver.
+ *    pool that the library creates per device (not the device's default pool), through a cache of
+ *    freed blocks per stream (at most an eighth of the device's memory idle); scn_trim_memory gives
+ *    idle blocks, and idle pinned staging memory of host coordinates, back to the driver.
  *  - a scn_metadata belongs to the device that was current at its first use; using it with
  *    another device current is SCN_ERR_BAD_ARG.  It may be used on one stream at a time.
  */
@@ -75,15 +76,17 @@ enum scn_precision {
 };
 /* which convolution kernel the last convolution call of this thread ran (for profiling) */
 enum scn_conv_kernel {
-  SCN_KERNEL_CONV_SIMT = 0,          /* k_conv_pipe / k_conv_simt / k_conv_thin: fp32 FMA     */
-  SCN_KERNEL_CONV_TC = 1,            /* k_conv_tc: tcgen05, one tile per CTA                  */
+  SCN_KERNEL_CONV_SIMT = 0,          /* fp32 FMA: k_conv_fma (mask-sorted tiles), k_conv_pipe, k_conv_simt, k_conv_thin */
+  SCN_KERNEL_CONV_TC = 1,            /* tcgen05, more than 64 output planes, small levels: k_conv_tile, k_conv_tc */
   SCN_KERNEL_CONV_TC_PERSISTENT = 2, /* k_conv_tma: tcgen05, persistent, double-buffered TMEM */
   SCN_KERNEL_CONV_PIPE_MMA = 3,      /* k_conv_pipe with three tf32 mma.sync passes           */
-  SCN_KERNEL_CONV_ROWS = 4,          /* k_conv_rows: row-stationary, warp-level mma.sync      */
-  SCN_KERNEL_CONV_WIDE = 5           /* k_conv_wide: tcgen05, persistent, rows split to bf16 parts once per call and copied in by cp.async */
+  SCN_KERNEL_CONV_ROWS = 4,          /* up to 64 output planes: k_conv_tile (tcgen05); k_conv_rows (warp-level mma.sync) */
+  SCN_KERNEL_CONV_WIDE = 5           /* tcgen05, more than 64 output planes, large levels: k_conv_tile, k_conv_wide */
 };
-/* The tensor-core modes need groups == 1, n_in_planes % 32 == 0, n_out_planes % 16 == 0 and
- * n_out_planes <= 256; other shapes run the fp32 kernel whatever the precision says. */
+/* The tensor-core modes run on tcgen05 (k_conv_tile) for groups == 1, filters of at most 128 offsets, n_in_planes and
+ * n_out_planes multiples of eight, n_out_planes <= 256 and 16-byte aligned rows; other shapes run on the older tensor
+ * kernels where those take them (n_in_planes % 32 == 0, n_out_planes % 16 == 0, n_out_planes <= 256) or on the fp32
+ * kernels, whatever the precision says. */
 
 /* which rulebook of a metadata object an export call refers to */
 enum scn_rulebook_kind {
@@ -310,8 +313,8 @@ SCN_API int scn_submanifold_convolution_forward(scn_metadata *md, const int64_t 
  * mbarrier another role arrives on) is bounded: when it runs out the kernel raises a status bit,
  * all its roles leave their loops, tensor memory is freed and the kernel returns; the host reads the
  * status through scn_md_poll_errors as SCN_ERR_CUDA with a message naming the wait.  After this call
- * the NEXT per-tile tensor-core convolution of the calling thread (k_conv_tc: a level with at most
- * 148 tiles of 256 rows, precision tf32 / bf16 / tf32x3) leaves out one barrier arrival in one of
+ * the NEXT tensor-core convolution of the calling thread on k_conv_tile or k_conv_tc (precision
+ * tf32 / bf16 / tf32x3) leaves out one barrier arrival in one of
  * its CTAs -- a flag that nothing sets -- so that exactly this path runs: the call itself returns
  * SCN_OK (the kernel is asynchronous), its output is incomplete, scn_md_poll_errors reports the
  * expired wait, and the next convolution works again.  Nothing traps, faults or waits without a
