@@ -70,7 +70,7 @@ struct DwParams {
   const unsigned char *t_rows, *g_rows;  // split: the table's side (rows order[.]) and the gathered side (rows packed[.])
   int t_planes, g_planes;
   long long n_t, n_g;
-  const int *order, *packed;
+  const int *order, *packed, *by_work;
   const unsigned *tile_bits;
   int words, K, n_groups, n_chunks, blocks_g;
   unsigned group_bits[32][4];  // the offsets of a group, ascending, are the bits of its mask
@@ -260,12 +260,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
       for (int w = 0; w < 4; ++w) mine[w] = P.group_bits[group][w];
       constexpr int kFetch = 4;  // tiles whose masks are on their way
       unsigned u[kFetch][4];
-      auto fetch = [&](int i, long long t) {
+      long long tile[kFetch];
+      // the tiles with the most offsets first, back and forth over the chunks
+      auto place = [&](long long it) { return it & 1 ? (it + 1) * P.n_chunks - 1 - chunk : it * P.n_chunks + chunk; };
+      auto fetch = [&](int i, long long it) {
+        const long long at = place(it);
+        tile[i] = at < P.n_tiles ? (P.by_work ? (long long)__ldg(P.by_work + at) : at) : -1;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) u[i][w] = t < P.n_tiles && w < P.words ? __ldg(P.tile_bits + t * P.words + w) : 0u;
+        for (int w = 0; w < 4; ++w) u[i][w] = tile[i] >= 0 && w < P.words ? __ldg(P.tile_bits + tile[i] * P.words + w) : 0u;
       };
+      const long long full = P.n_tiles / P.n_chunks, rounds = full + (place(full) < P.n_tiles ? 1 : 0);
 #pragma unroll
-      for (int i = 0; i < kFetch; ++i) fetch(i, chunk + (long long)i * P.n_chunks);
+      for (int i = 0; i < kFetch; ++i) fetch(i, i);
       int n = 0;
       bool ok = true;
       auto put = [&](int job, const int *src) {
@@ -283,10 +289,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
         }
         ++n;
       };
-      for (long long t = chunk; t < P.n_tiles && ok;) {
+      for (long long it = 0; it < rounds && ok;) {
 #pragma unroll
         for (int i = 0; i < kFetch; ++i) {
-          if (t >= P.n_tiles || !ok) break;
+          if (it >= rounds || !ok) break;
+          const long long t = tile[i];
           if ((u[i][0] & mine[0]) | (u[i][1] & mine[1]) | (u[i][2] & mine[2]) | (u[i][3] & mine[3])) {
             put(kTRows, P.order + t * kRows);
             const int *src = P.packed + t * P.K * kRows;
@@ -301,8 +308,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
               j += __popc(mine[w]);
             }
           }
-          fetch(i, t + (long long)kFetch * P.n_chunks);
-          t += P.n_chunks;
+          fetch(i, it + kFetch);
+          ++it;
         }
       }
       const int filled = n;
@@ -530,6 +537,7 @@ int dweight_tile(const float *in, long long rows_in, const float *d_out, long lo
   P.n_g = swap ? rows_out : rows_in;
   P.order = ord.order;
   P.packed = ord.packed;
+  P.by_work = ord.by_work;
   P.tile_bits = ord.tile_bits;
   P.words = ord.words;
   P.n_tiles = ord.n_tiles;

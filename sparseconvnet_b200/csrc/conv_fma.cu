@@ -44,7 +44,7 @@ struct FmaParams {
   const float *bias, *bn_scale, *bn_shift;
   float leak;
   const int *nbr;
-  const int *order, *packed;  // null: rows in their own order
+  const int *order, *packed, *by_work;  // null: rows in their own order
   const unsigned *tile_bits;
   int words, K, cin, cout, n_split;
   long long n_pos;
@@ -70,9 +70,8 @@ k_conv_fma(FmaParams P) {
   __shared__ unsigned mask[4];
   const int tid = threadIdx.x, lane = tid & 31;
   const int tx = tid % S::TX, ty = tid / S::TX;
-  // from the back: packed tiles come in ascending order of their masks, and the ones with the most offsets are best started
-  // first
-  const long long pos0 = (long long)(gridDim.x - 1 - blockIdx.x) * ROWS;
+  // the tiles with the most offsets first (packed tiles come in ascending order of their masks)
+  const long long pos0 = (P.by_work ? (long long)__ldg(P.by_work + blockIdx.x) : (long long)(gridDim.x - 1 - blockIdx.x)) * ROWS;
   const int n0 = blockIdx.y * BN;
 
   // ---- copying role: eight threads per row, 16 rows (of ROWS) at a time ----------------------------------------------
@@ -291,6 +290,7 @@ int conv_forward_fma(const float *in, long long n_in, float *out, long long n_ou
   P.nbr = table;
   P.order = ord ? ord->order : nullptr;
   P.packed = ord ? ord->packed : nullptr;
+  P.by_work = ord ? ord->by_work : nullptr;  // (tiles are ROWS = 128 rows then)
   P.tile_bits = ord ? ord->tile_bits : nullptr;
   P.words = ord ? ord->words : 0;
   P.K = K;

@@ -68,7 +68,7 @@ struct TileParams {
   const unsigned char *wprep;
   const float *bias, *bn_scale, *bn_shift;
   float leak;
-  const int *order, *packed;
+  const int *order, *packed, *by_work;
   const unsigned *tile_bits;
   int words;
   int K, n_slices;
@@ -133,10 +133,19 @@ __device__ __forceinline__ void keep_range(unsigned (&m)[4], int lo, int hi) {
   }
 }
 
-// The tile of an item, from the back: packed tiles come in ascending order of their masks, and the ones with the most
-// offsets are best started first.
+// The items of a CTA: back and forth over the CTAs, so that of items in descending order of work each gets about the same.
+__device__ __forceinline__ long long item_of(long long it) {
+  return it & 1 ? (it + 1) * gridDim.x - 1 - blockIdx.x : it * gridDim.x + blockIdx.x;
+}
+__device__ __forceinline__ long long items_here(const TileParams &P) {
+  const long long full = P.n_items / gridDim.x;
+  return full + (item_of(full) < P.n_items ? 1 : 0);
+}
+// The tile of an item: the tiles with the most offsets first (packed tiles come in ascending order of their masks, so from
+// the back where they have not been sorted by work).
 __device__ __forceinline__ long long item_tile(const TileParams &P, long long item) {
-  return P.n_tiles - 1 - item / P.n_split;
+  const long long i = P.n_split == 1 ? item : item / P.n_split;
+  return P.by_work ? __ldg(P.by_work + i) : P.n_tiles - 1 - i;
 }
 
 // filter offsets of an item: those of its tile, or its share of them when the offsets are divided
@@ -190,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
   tc_fence_after();
   const unsigned tmem = C.tmem;
   volatile int *abort = &C.abort;
-  const long long my_items = (P.n_items - blockIdx.x + gridDim.x - 1) / gridDim.x;  // (the grid has at most n_items CTAs)
+  const long long my_items = items_here(P);  // (the grid has at most n_items CTAs)
 
   if (warp < kProdWarps) {
     // ==================================== producers =============================================
@@ -297,10 +306,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     unsigned at = 0, d = tmem;
     bool ok = true;
     const bool leader = elect_one();
-    int offsets_next = item_offsets(P, blockIdx.x);
+    int offsets_next = item_offsets(P, item_of(0));
     for (int i = 0; i < items && ok; ++i) {
       const int steps = __reduce_max_sync(0xffffffffu, max(1, offsets_next)) * P.n_slices;
-      offsets_next = item_offsets(P, blockIdx.x + (long long)(i + 1) * gridDim.x);
+      offsets_next = item_offsets(P, item_of(i + 1));
       // the item's accumulator must have been drained
       if (!mbar_wait_warp(&C.acc_empty[buf], buf_par) || __any_sync(0xffffffffu, *abort != 0)) {
         ok = false;
@@ -352,13 +361,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
         for (int w = 0; w < 4; ++w)
           b_next[w] = item < P.n_items && w < P.words ? __ldg(P.tile_bits + item_tile(P, item) * P.words + w) : 0u;
       };
-      fetch(blockIdx.x);
+      fetch(item_of(0));
       for (long long it = 0; it < my_items && ok; ++it) {
-        const long long item = blockIdx.x + it * gridDim.x;
+        const long long item = item_of(it);
         unsigned u[4];
 #pragma unroll
         for (int w = 0; w < 4; ++w) u[w] = b_next[w];
-        fetch(item + gridDim.x);
+        fetch(item_of(it + 1));
         const int *src = P.packed + item_tile(P, item) * P.K * kRows;
         if (P.n_split > 1) {
           const int total = __popc(u[0]) + __popc(u[1]) + __popc(u[2]) + __popc(u[3]), part = (int)(item % P.n_split);
@@ -416,7 +425,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     float4 *my_epi = reinterpret_cast<float4 *>(epi + quad * kEpiBytes);
     int buf = 0, buf_par = 0;
     for (long long it = 0; it < my_items; ++it) {
-      const long long item = blockIdx.x + it * gridDim.x, t = item_tile(P, item);
+      const long long item = item_of(it), t = item_tile(P, item);
       const int part = (int)(item % P.n_split);
       const int orow = __ldg(P.order + t * kRows + quad * 32 + lane);
       int got = 1;
@@ -742,6 +751,7 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
   P.leak = bn_scale ? leak : 1.f;
   P.order = ord.order;
   P.packed = ord.packed;
+  P.by_work = ord.by_work;
   P.tile_bits = ord.tile_bits;
   P.words = ord.words;
   P.K = K;

@@ -55,6 +55,7 @@ struct RowOrder {
   int *order = nullptr;
   unsigned *tile_bits = nullptr;
   int *packed = nullptr;
+  int *by_work = nullptr;  // the tiles, those with the most offsets first (null: small levels, tiles in their order)
   int words = 1;  // 32-bit words per tile: 1 up to 32 offsets, else 4
   long long n_tiles = 0;
 };

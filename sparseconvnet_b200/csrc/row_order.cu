@@ -203,14 +203,95 @@ k_order_plain(const int *__restrict__ nbr, long long n, int K, int words, int *_
   }
 }
 
+// The tiles by how many offsets they have, most first, stable (run by one block of 256 threads, the last of k_order_tiles to
+// pack its own: it adds 4 us to 21 us at 300 k rows).  Handed out in ascending order of their masks the tiles left the
+// busiest SM 1.1 to 1.7 times the average; most offsets first, back and forth over the CTAs, 1.02 to 1.2: 32 -> 32 planes
+// on 1.6 M rows 335 -> 317 us, 96 -> 96 on 155 k rows 169 -> 133 us.  Below 149 tiles no CTA has two; from 65536 on the
+// counts would not fit their 16 bits and each CTA has hundreds of tiles, which is balance enough.
+constexpr int kWorkBins = 32;
+template <int WORDS>
+__device__ void tiles_by_work(const unsigned *tile_bits, int n_tiles, int K, int *by_work) {
+  __shared__ __align__(16) unsigned short hist[kWorkBins][256];
+  __shared__ int bin_sum[kWorkBins];
+  static_assert(kWorkBins == 32, "a lane per bin");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int per = (n_tiles + 255) / 256, t0 = min(n_tiles, tid * per), t1 = min(n_tiles, t0 + per);
+  const unsigned scale = ((unsigned)kWorkBins << 16) / (unsigned)(K + 1);
+  // each tile of the thread's run in order, sixteen masks on their way (the block works alone: every trip to L2 shows);
+  // the bins of a run of up to sixteen stay in registers for the second walk
+  int b[16];
+  auto load = [&](int t) {
+    unsigned bits[16][WORDS];
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+#pragma unroll
+      for (int w = 0; w < WORDS; ++w) bits[i][w] = t + i < t1 ? __ldcg(tile_bits + (long long)(t + i) * WORDS + w) : 0u;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      unsigned c = 0;
+#pragma unroll
+      for (int w = 0; w < WORDS; ++w) c += __popc(bits[i][w]);
+      b[i] = (kWorkBins - 1) - (int)(c * scale >> 16);
+    }
+  };
+  auto each = [&](bool again, auto use) {
+    for (int t = t0; t < t1; t += 16) {
+      if (!again || per > 16) load(t);
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (t + i < t1) use(t + i, b[i]);
+    }
+  };
+#pragma unroll
+  for (int b = 0; b < kWorkBins; ++b) hist[b][tid] = 0;
+  each(false, [&](int, int b) { ++hist[b][tid]; });
+  __syncthreads();
+  // exclusive sums over (bin, thread): a warp has four bins, a lane eight neighbouring threads' counts of each
+  int before[4];
+  uint4 v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[i] = *reinterpret_cast<const uint4 *>(&hist[warp * 4 + i][lane * 8]);
+    const unsigned pairs = v[i].x + v[i].y + v[i].z + v[i].w;  // (no half overflows: fewer than 65536 tiles)
+    const int sum = (int)(pairs & 0xFFFFu) + (int)(pairs >> 16);
+    int incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += u;
+    }
+    before[i] = incl - sum;
+    if (lane == 31) bin_sum[warp * 4 + i] = incl;
+  }
+  __syncthreads();
+  int base = bin_sum[lane], own = base;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, base, d);
+    if (lane >= d) base += u;
+  }
+  base -= own;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    unsigned at = (unsigned)(before[i] + __shfl_sync(0xffffffffu, base, warp * 4 + i));
+    unsigned *w = reinterpret_cast<unsigned *>(&v[i]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const unsigned lo = w[e] & 0xFFFFu, hi = w[e] >> 16;
+      w[e] = (at & 0xFFFFu) | ((at + lo) << 16);
+      at += lo + hi;
+    }
+    *reinterpret_cast<uint4 *>(&hist[warp * 4 + i][lane * 8]) = v[i];
+  }
+  __syncthreads();
+  each(true, [&](int t, int b) { by_work[hist[b][tid]++] = t; });
+}
+
 // One warp per tile, four rows per lane: tile_bits, packed, and -1 in the order array past the last row.
 template <int WORDS>
-__global__ void __launch_bounds__(256)
-k_order_tiles(int *__restrict__ order, long long n, int K, const int *__restrict__ nbr, const unsigned *__restrict__ masks,
-              unsigned *__restrict__ tile_bits, int *__restrict__ packed, long long n_tiles) {
-  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (t >= n_tiles) return;
+__device__ __forceinline__ void pack_tile(int *__restrict__ order, long long n, int K, const int *__restrict__ nbr,
+                                          const unsigned *__restrict__ masks, unsigned *tile_bits, int *__restrict__ packed,
+                                          long long t, int lane) {
   const long long p = t * kTile + lane * 4;
   int4 o = *reinterpret_cast<const int4 *>(order + p);
   if (p + 3 >= n) {
@@ -239,6 +320,22 @@ k_order_tiles(int *__restrict__ order, long long n, int K, const int *__restrict
       dst += kTile;
     }
   }
+}
+
+template <int WORDS>
+__global__ void __launch_bounds__(256)
+k_order_tiles(int *__restrict__ order, long long n, int K, const int *__restrict__ nbr, const unsigned *__restrict__ masks,
+              unsigned *tile_bits, int *__restrict__ packed, long long n_tiles, int *by_work, int *done) {
+  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (t < n_tiles) pack_tile<WORDS>(order, n, K, nbr, masks, tile_bits, packed, t, lane);
+  if (!by_work) return;
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (last) tiles_by_work<WORDS>(tile_bits, (int)n_tiles, K, by_work);
 }
 
 // Which key bits the offsets set, and how many bits there are.  Fewer bits cost fewer passes,
@@ -320,12 +417,13 @@ int build(const int *table, const unsigned *known, long long n, int K, const uns
   if (!known) SCN_TRY(tmp.get((void **)&masks, sizeof(unsigned) * WORDS * (size_t)n));
   SCN_TRY(tmp.get((void **)&keys[0], sizeof(KEY) * (size_t)n));
   SCN_TRY(tmp.get((void **)&counts, sizeof(int) * (size_t)blocks * R));
-  SCN_TRY(tmp.get((void **)&totals, sizeof(int) * (size_t)passes * R));
+  SCN_TRY(tmp.get((void **)&totals, sizeof(int) * ((size_t)passes * R + 1)));  // and the blocks that have packed their tiles
   if (passes > 1) {
     SCN_TRY(tmp.get((void **)&keys[1], sizeof(KEY) * (size_t)n));
     SCN_TRY(tmp.get((void **)&rows, sizeof(int) * (size_t)n));
   }
-  SCN_CUDA_CHECK(cudaMemsetAsync(totals, 0, sizeof(int) * (size_t)passes * R, stream));
+  SCN_CUDA_CHECK(cudaMemsetAsync(totals, 0, sizeof(int) * ((size_t)passes * R + 1), stream));
+  if (ord.n_tiles > 148 && ord.n_tiles < 65536) SCN_TRY(device_alloc((void **)&ord.by_work, sizeof(int) * (size_t)ord.n_tiles, stream));
   SCN_LAUNCH((k_order_keys<KEY, WORDS>), blocks, kThreads, 0, stream, table, known, n, K, B, (int)rpb, R, keys[0], masks, counts, totals);
   const int *src = nullptr;
   for (int p = 0; p < passes; ++p) {
@@ -336,7 +434,7 @@ int build(const int *table, const unsigned *known, long long n, int K, const uns
     SCN_LAUNCH((k_order_scatter<KEY>), blocks, kThreads, 0, stream, kin, src, n, (int)rpb, p * digit, R, counts, totals + (size_t)p * R, kout, dst);
     src = dst;
   }
-  SCN_LAUNCH((k_order_tiles<WORDS>), (unsigned)ceil_div(ord.n_tiles * 32, 256), 256, 0, stream, ord.order, n, K, table, known ? known : masks, ord.tile_bits, ord.packed, ord.n_tiles);
+  SCN_LAUNCH((k_order_tiles<WORDS>), (unsigned)ceil_div(ord.n_tiles * 32, 256), 256, 0, stream, ord.order, n, K, table, known ? known : masks, ord.tile_bits, ord.packed, ord.n_tiles, ord.by_work, totals + (size_t)passes * R);
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }
@@ -347,6 +445,7 @@ void free_row_order(RowOrder &o, cudaStream_t stream) {
   device_free(o.order, stream);
   device_free(o.tile_bits, stream);
   device_free(o.packed, stream);
+  device_free(o.by_work, stream);
   o = RowOrder{};
 }
 

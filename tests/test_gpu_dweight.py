@@ -98,3 +98,39 @@ def test_batchnorm_training_sums(n, planes, cuda):
     if same:  # (a value within rounding of zero may take the other slope)
         for got, want in ((x.grad, xd.grad), (layer.weight.grad, w.grad), (layer.bias.grad, b.grad)):
             assert helpers.rel_err(got.double().cpu().numpy(), want.cpu().numpy()) <= helpers.FP32_TOL
+
+
+@pytest.mark.parametrize("tiles,extra", [(148, 0), (148, 1), (149, 0), (4096, 0), (4096, 1), (65535, 0), (65535, 1)])
+def test_tiles_by_work(tiles, extra, cuda):
+    """Row counts around the levels whose tiles are sorted by their offsets (149 to 65535 tiles of 128 rows; up to 4096 of
+    them the sort keeps its bins in registers), masks of every fill: outputs and weight gradient, each tile once."""
+    import sparseconvnet_b200 as scn
+    n = tiles * 128 + extra
+    size = int(np.ceil((2.3 * n) ** (1 / 3)))
+    torch.manual_seed(tiles + extra)
+    cell = (torch.rand(size ** 3, device=cuda) < torch.arange(size ** 3, device=cuda) / size ** 3).nonzero()[:, 0]
+    cell = cell[torch.randperm(len(cell), device=cuda)[:n]]
+    pts = torch.stack([cell // size ** 2, cell // size % size, cell % size], 1)
+    assert len(pts) == n
+    x = scn.InputLayer(3, size, mode=0)([pts.cpu(), torch.randn(n, 16, device=cuda)])
+    layer = scn.SubmanifoldConvolution(3, 16, 40, 3, False).to(cuda)
+    f = x.features
+    g = torch.randn_like(layer(x).features)
+    rules = [r.long() for r in x.metadata.rulebook(0, x.spatial_size, [3, 3, 3])]
+    w = layer.weight.detach()[:, 0]
+    want = torch.zeros(n, 40, dtype=torch.float64, device=cuda)
+    for r, wk in zip(rules, w.double()):
+        want.index_add_(0, r[:, 1], f.double()[r[:, 0]] @ wk)
+    want_w = torch.stack([f[r[:, 0]].double().t() @ g[r[:, 1]].double() for r in rules])
+    try:
+        for precision in ("fp32", "tf32x3"):
+            scn.set_precision(precision)
+            layer.weight.grad = None
+            y = layer(x).features
+            y.backward(g)
+            assert float((y.detach() - want).abs().max() / want.abs().max()) <= helpers.FP32_TOL, precision
+            e = float((layer.weight.grad[:, 0] - want_w).abs().max() / want_w.abs().max())
+            assert e <= helpers.FP32_TOL, (precision, e)
+        x.metadata.poll_errors()
+    finally:
+        scn.set_precision("fp32")
