@@ -371,6 +371,102 @@ static int launch_dweight(const float *in, int ld_in, long long n_in_rows, const
   return SCN_OK;
 }
 
+// Up to three input planes (the first layer of a network) and 32 output planes: no matrix to speak of.  A lane owns an
+// output plane and keeps the sums of nine offsets x CIN planes in registers, in full fp32; d_out rows are read as they lie.
+// Per batch of 32 rows a warp fetches the nine table entries of a row and the inputs they name with one lane per row, leaves
+// them in shared memory (zeros where there is no rule) and reads them back row by row, the same for all lanes.  Most
+// multiply-adds of surface data are with such zeros, which is cheaper than finding the others; bound by the L1 pipe (the
+// scattered 4-byte loads, and the shared memory both ways).  k_conv_dweight_mma, whose steps are padded to 16 planes, took
+// 218 us for 3 -> 32 planes of two rooms (120 now), 28 for 3 k rows (8), 41 for 1 -> 16 planes on 100 k pixels (15); with four
+// input planes (97 against 120 us at 400 k scattered rows) and with two blocks of output planes (141, 184) it stays ahead.
+constexpr int kThinOffsets = 9;
+
+template <int CIN>
+__global__ void __launch_bounds__(256, 2)
+k_conv_dweight_thin(const float *__restrict__ in, long long n_in, const float *__restrict__ dout, long long n_out,
+                    const int *__restrict__ nbr, int K, int cout, long long chunk_rows, float *__restrict__ partial, int *flags) {
+  constexpr int N = kThinOffsets * CIN, W = (N + 3) / 4 * 4;  // values of a row
+  __shared__ __align__(16) float values[8][32][W];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int blocks_p = (cout + 31) / 32, k0 = (int)blockIdx.y / blocks_p * kThinOffsets, p = (int)blockIdx.y % blocks_p * 32 + lane;
+  const int n_off = min(kThinOffsets, K - k0);
+  const long long begin = blockIdx.x * chunk_rows, end = min(n_out, begin + chunk_rows);
+  float acc[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) acc[i] = 0.f;
+  bool bad = false;
+  int e[kThinOffsets];
+  auto fetch = [&](long long row) {
+#pragma unroll
+    for (int k = 0; k < kThinOffsets; ++k) e[k] = k < n_off && row < end ? __ldg(nbr + (long long)(k0 + k) * n_out + row) : -1;
+  };
+  fetch(begin + warp * 32 + lane);
+  for (long long r0 = begin + warp * 32; r0 < end; r0 += 256) {
+#pragma unroll
+    for (int k = 0; k < kThinOffsets; ++k) {
+      const bool hit = (unsigned)e[k] < (unsigned long long)n_in;
+      bad |= e[k] >= n_in;
+#pragma unroll
+      for (int c = 0; c < CIN; ++c) values[warp][lane][k * CIN + c] = hit ? __ldg(in + (long long)e[k] * CIN + c) : 0.f;
+    }
+    fetch(r0 + 256 + lane);  // the next batch's, on their way while this one is summed
+    __syncwarp();
+    const int rows = (int)min(32ll, end - r0);
+    for (int r = 0; r < rows; r += 8) {
+      float d[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) d[u] = r + u < rows && p < cout ? __ldg(dout + (r0 + r + u) * cout + p) : 0.f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float4 *v = reinterpret_cast<const float4 *>(values[warp][r + u]);
+#pragma unroll
+        for (int i = 0; i < W / 4; ++i) {
+          const float4 x = v[i];
+          acc[i * 4] = fmaf(x.x, d[u], acc[i * 4]);
+          if (i * 4 + 1 < N) acc[i * 4 + 1] = fmaf(x.y, d[u], acc[i * 4 + 1]);
+          if (i * 4 + 2 < N) acc[i * 4 + 2] = fmaf(x.z, d[u], acc[i * 4 + 2]);
+          if (i * 4 + 3 < N) acc[i * 4 + 3] = fmaf(x.w, d[u], acc[i * 4 + 3]);
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (bad) atomicOr(flags, FLAG_BAD_ROW);
+  // the warps' sums in order
+  __syncthreads();
+  float(*sums)[N][32] = reinterpret_cast<float(*)[N][32]>(&values[0][0][0]);
+#pragma unroll
+  for (int i = 0; i < N; ++i) sums[warp][i][lane] = acc[i];
+  __syncthreads();
+  if (p >= cout) return;
+  for (int i = warp; i < n_off * CIN; i += 8) {
+    float x = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) x += sums[w][i][lane];
+    partial[(((long long)blockIdx.x * K + k0) * CIN + i) * cout + p] = x;  // [chunk][offset][input plane][output plane]
+  }
+}
+
+static int dweight_thin(const float *in, long long rows_in, const float *d_out, long long rows_out, const int *nbr, int K, int cin,
+                        int cout, float *d_weight, int *flags, cudaStream_t stream) {
+  // one wave of two CTAs per SM, in whole batches
+  const int columns = (int)(ceil_div(K, kThinOffsets) * ceil_div(cout, 32));
+  const long long wanted = std::max<long long>(1, std::min<long long>(148 * 2 / columns, ceil_div(rows_out, 256)));
+  const long long chunk_rows = ceil_div(ceil_div(rows_out, wanted), 256) * 256;
+  const int chunks = (int)ceil_div(rows_out, chunk_rows);
+  const long long w_elems = (long long)K * cin * cout;
+  float *partial = d_weight;
+  if (chunks > 1) SCN_TRY(device_alloc((void **)&partial, sizeof(float) * (size_t)chunks * w_elems, stream));
+  const auto kernel = cin == 1 ? k_conv_dweight_thin<1> : cin == 2 ? k_conv_dweight_thin<2> : k_conv_dweight_thin<3>;
+  SCN_LAUNCH(kernel, dim3((unsigned)chunks, (unsigned)columns), 256, 0, stream, in, rows_in, d_out, rows_out, nbr, K, cout, chunk_rows, partial, flags);
+  if (chunks > 1) {
+    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, chunks, w_elems, d_weight);
+    SCN_TRY(device_free(partial, stream));
+  }
+  SCN_CUDA_CHECK(cudaGetLastError());
+  return SCN_OK;
+}
+
 // 32-plane tiles per side: one CTA tile up to 96 planes, beyond that whichever of 64 and 96 pads less
 static int dweight_side(int planes) {
   if (planes <= 96) return (planes + 31) / 32;
@@ -445,6 +541,8 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
     if (groups == 1 && !fma_only && !(tile && atoi(tile) == 0) && dweight_tile_supported(in, d_out, rb, cin, cout)) {
       SCN_TRY(rulebook_row_order(rb, rb.nbr, rb.n_out, rb.order, stream));
       SCN_TRY(dweight_tile(in, rows_in, d_out, rows_out, rb, transposed, cin, cout, d_weight, md->flags_dev, stream));
+    } else if (groups == 1 && !fma_only && cin <= 3 && cout <= 32 && !transposed && rows_out > 0) {
+      SCN_TRY(dweight_thin(in, rows_in, d_out, rows_out, rb.nbr, K, cin, cout, d_weight, md->flags_dev, stream));
     } else if (groups == 1 && !fma_only) {
       decltype(&launch_dweight<1, 1>) const by_side[3][3] = {{launch_dweight<1, 1>, launch_dweight<1, 2>, launch_dweight<1, 3>},
                                                              {launch_dweight<2, 1>, launch_dweight<2, 2>, launch_dweight<2, 3>},

@@ -134,3 +134,11 @@ def test_tiles_by_work(tiles, extra, cuda):
         x.metadata.poll_errors()
     finally:
         scn.set_precision("fp32")
+
+
+@pytest.mark.parametrize("cin", [1, 2, 3])
+@pytest.mark.parametrize("cout", [1, 20, 32])
+@pytest.mark.parametrize("n,size", [(1, 8), (300, 16), (6000, 40), (120001, 160)])
+def test_thin_weight_gradient(n, size, cin, cout, cuda):
+    """k_conv_dweight_thin: batches of 32 rows, nine offsets and the planes with and without remainders."""
+    test_weight_gradient(n, size, cin, cout, cuda)
