@@ -135,7 +135,7 @@ __global__ void k_sum_chunks(const float *__restrict__ partial, int chunks, long
 // them on surface data), in a list in shared memory, and walks the list in steps of 32 or 64 rules: the rules' input and
 // output rows travel with cp.async through a ring of stages, then each warp multiplies
 // in^T [32 x 8 rules] x d_out [8 rules x 32] per block of eight rules with mma.sync.m16n8k8 on the hi/lo split of both
-// operands (hi x hi + hi x lo + lo x hi, fp32 accumulate: fp32-class accuracy).  With few 32 x 32 tiles several warps
+// operands (hi x hi + hi x lo + lo x hi; as accurate as fp32 multiply-adds, see dw_split and the sums).  With few 32 x 32 tiles several warps
 // share the blocks of a step and their sums are added in warp order, so the result does not depend on timing.  Plane
 // counts that are no multiple of the tile are padded with zeros in the stage only.
 //
@@ -147,9 +147,12 @@ __device__ __forceinline__ void dw_mma(float (&d)[4], const unsigned (&a)[4], co
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
+// x = hi + lo, both rounded to the nearest tf32: what is left out (lo x lo and a bit of lo, 2^-23 of x) has either sign as
+// often as the other.  Cut off instead of rounded it all had the sign of x: 8e-6 of a sum of 100 k products of one sign, 1e-7
+// now, and 4e-6 against 2e-7 with signs mixed.
 __device__ __forceinline__ void dw_split(float x, unsigned &hi, unsigned &lo) {
-  hi = __float_as_uint(x) & 0xFFFFE000u;
-  lo = __float_as_uint(x - __uint_as_float(hi));
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(x - __uint_as_float(hi)));
 }
 __device__ __forceinline__ void dw_copy4(unsigned dst, const float *src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4u : 0u) : "memory");
@@ -196,6 +199,8 @@ k_conv_dweight_mma(const float *__restrict__ in, int ld_in, long long n_in_rows,
     __syncthreads();
   }
 
+  // The tensor core cuts off what does not fit its running sum, always towards zero: it adds up eight rules at a time
+  // (from zero), and fp32 additions add those.
   float d[MT][4][4];
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
@@ -294,18 +299,25 @@ k_conv_dweight_mma(const float *__restrict__ in, int ld_in, long long n_in_rows,
           dw_split(b0[nt * 8], bh[nt][0], bl[nt][0]);
           dw_split(b1[nt * 8], bh[nt][1], bl[nt][1]);
         }
+        float p[MT][4][4] = {};
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-          for (int nt = 0; nt < 4; ++nt) dw_mma(d[mt][nt], al[mt], bh[nt]);
+          for (int nt = 0; nt < 4; ++nt) dw_mma(p[mt][nt], al[mt], bh[nt]);
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-          for (int nt = 0; nt < 4; ++nt) dw_mma(d[mt][nt], ah[mt], bl[nt]);
+          for (int nt = 0; nt < 4; ++nt) dw_mma(p[mt][nt], ah[mt], bl[nt]);
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-          for (int nt = 0; nt < 4; ++nt) dw_mma(d[mt][nt], ah[mt], bh[nt]);
+          for (int nt = 0; nt < 4; ++nt) dw_mma(p[mt][nt], ah[mt], bh[nt]);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) d[mt][nt][e] += p[mt][nt][e];
       }
     }
     cp_async_wait<0>();
@@ -337,6 +349,8 @@ k_conv_dweight_mma(const float *__restrict__ in, int ld_in, long long n_in_rows,
   }
 }
 
+static int n_chunks(long long rows) { return (int)std::max<long long>(1, std::min<long long>(64, rows / 4096)); }
+
 template <int WM, int WN, int MT = 2>
 static int launch_dweight(const float *in, int ld_in, long long n_in_rows, const float *dout, int ld_out,
                           long long n_out_rows, const int *nbr, long long n_entries, int swap, int K, int cin, int cout,
@@ -351,10 +365,12 @@ static int launch_dweight(const float *in, int ld_in, long long n_in_rows, const
     SCN_CUDA_CHECK(cudaFuncSetAttribute(k_conv_dweight_mma<WM, WN, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
     configured[dev].store(true);
   }
-  // about four waves of the CTAs the SMs hold, in chunks of whole lists
+  // about four waves of the CTAs the SMs hold, in chunks of whole lists; no fewer than one per 4096 entries (up to 64), which
+  // bounds how many additions a sum goes through before the chunks' sums are added
   const int tiles = (int)(ceil_div(cin, S::M) * ceil_div(cout, S::N));
   const int per_sm = std::max(1, (int)(220 * 1024 / S::SMEM));
-  const int chunks = (int)std::max<long long>(1, std::min<long long>(ceil_div(148 * 4 * per_sm, (long long)K * tiles), n_entries / S::LIST));
+  const long long wanted = std::max<long long>(ceil_div(148 * 4 * per_sm, (long long)K * tiles), n_chunks(n_entries));
+  const int chunks = (int)std::max<long long>(1, std::min<long long>(wanted, n_entries / S::LIST));
   const long long chunk_rows = ceil_div(ceil_div(n_entries, chunks), S::LIST) * S::LIST;
   const int grid_x = (int)ceil_div(n_entries, chunk_rows);
   const long long w_elems = (long long)K * cin * cout;
@@ -467,8 +483,12 @@ static int dweight_thin(const float *in, long long rows_in, const float *d_out, 
   return SCN_OK;
 }
 
-// 32-plane tiles per side: one CTA tile up to 96 planes, beyond that whichever of 64 and 96 pads less
-static int dweight_side(int planes) {
+// 32-plane tiles per side: one CTA tile up to 96 planes, beyond that whichever of 64 and 96 pads less.  Few entries
+// make few chunks, and tiles of 32 x 32 fill the SMs instead: 80 x 80 weights on 7 k rows 84 against 381 us, 25 k rows 191
+// against 382, 96 x 48 on 25 k rows 134 against 213; from about 50 k rows on the second fetch of the rows costs as much
+// (48 x 48 on 56 k rows 169 against 160 us, on 160 k rows 375 against 291).
+static int dweight_side(int planes, long long n_entries) {
+  if (n_entries < 32768) return 1;
   if (planes <= 96) return (planes + 31) / 32;
   return ceil_div(planes, 96) * 96 < ceil_div(planes, 64) * 64 ? 3 : 2;
 }
@@ -493,8 +513,6 @@ k_column_sums(const float *__restrict__ x, long long n_rows, int planes, long lo
     partial[(long long)blockIdx.y * planes + p] = t;
   }
 }
-
-static int n_chunks(long long rows) { return (int)std::max<long long>(1, std::min<long long>(64, rows / 4096)); }
 
 // Runs the backward pass for one operator call.  `transposed` as in the forward pass (Deconvolution).
 static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, const float *in, float *d_in,
@@ -547,7 +565,7 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
       decltype(&launch_dweight<1, 1>) const by_side[3][3] = {{launch_dweight<1, 1>, launch_dweight<1, 2>, launch_dweight<1, 3>},
                                                              {launch_dweight<2, 1>, launch_dweight<2, 2>, launch_dweight<2, 3>},
                                                              {launch_dweight<3, 1>, launch_dweight<3, 2>, launch_dweight<3, 3>}};
-      auto launch = by_side[dweight_side(cin) - 1][dweight_side(cout) - 1];
+      auto launch = by_side[dweight_side(cin, n_entries) - 1][dweight_side(cout, n_entries) - 1];
       if (cin <= 16) launch = cout <= 32 ? launch_dweight<1, 1, 1> : cout <= 64 ? launch_dweight<1, 2, 1> : launch_dweight<1, 3, 1>;
       SCN_TRY(launch(in, n_in_planes, rows_in, d_out, n_out_planes, rows_out, rb.nbr, n_entries, transposed ? 1 : 0, K, cin,
                      cout, d_weight, md->flags_dev, stream));

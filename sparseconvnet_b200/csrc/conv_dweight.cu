@@ -8,8 +8,7 @@
 // planes contiguous, and read M- / N-major by the MMA -- no transposition anywhere.
 //
 //   arithmetic  x = h + m + l, three bf16 parts that hold all 24 bits of x; every product of the parts but m l, l m and
-//               l l (2^-24 of a product) is summed in fp32: no less than the tf32 hi / lo form of k_conv_dweight_mma
-//               (2^-20).  The parts of T are lanes of one accumulator (M = 128: h and m of 64 planes, or h, m and l of 32),
+//               l l (2^-24 of a product) is summed in fp32.  The parts of T are lanes of one accumulator (M = 128: h and m of 64 planes, or h, m and l of 32),
 //               those of G its columns, and the blocks are added when the sums are done; the products with an l go where
 //               those with an m go.  The tensor core truncates its running sum at every instruction, half a unit of 2^-24 on
 //               average: a CTA takes at most kMaxTiles tiles, 8 instructions each, before its sums are added in fp32.
@@ -518,9 +517,12 @@ int launch(DwParams &P, const Rulebook &rb, const float *t_rows, const float *g_
 // Rows of whole 16-byte pieces and more than 32 planes on one side: 32 x 32 weights are half as much work per gathered
 // byte, and k_conv_dweight_mma takes as long (400 k rows: 255 against 275 us; 64 x 64 at 124 k: 211 against 143, 96 x 96 at
 // 45 k: 339 against 225, 128 x 128 at 6 k: 114 against 67).  Below 2048 rows an order has to be there already.
+// Multiples of 32 planes only: the running sums in TMEM cut off where fp32 additions round, 4e-6 of a sum of 100 k products
+// of mixed signs and 8e-6 with one sign.  That is no more than these shapes ever had (5e-6 and 1e-5 with truncated tf32 parts);
+// the others had plain fp32 sums (9e-7, 1.4e-7), which k_conv_dweight_mma matches.
 bool dweight_tile_supported(const float *in, const float *d_out, const Rulebook &rb, int cin, int cout) {
-  return (rb.n_out >= 2048 || (rb.n_out > 0 && rb.order.order)) && std::max(cin, cout) > 32 && rb.n_offsets <= kOrderMaxOffsets && cin % 4 == 0 &&
-         cout % 4 == 0 && ((uintptr_t)in | (uintptr_t)d_out) % 16 == 0;
+  return cin % 32 == 0 && cout % 32 == 0 && (rb.n_out >= 2048 || (rb.n_out > 0 && rb.order.order)) && std::max(cin, cout) > 32 && rb.n_offsets <= kOrderMaxOffsets &&
+         ((uintptr_t)in | (uintptr_t)d_out) % 16 == 0;
 }
 
 // rb.order packs the rulebook's own table; swap: the operator ran it backwards (d_out is the gathered side)

@@ -142,3 +142,25 @@ def test_tiles_by_work(tiles, extra, cuda):
 def test_thin_weight_gradient(n, size, cin, cout, cuda):
     """k_conv_dweight_thin: batches of 32 rows, nine offsets and the planes with and without remainders."""
     test_weight_gradient(n, size, cin, cout, cuda)
+
+
+@pytest.mark.parametrize("cin,cout", [(8, 16), (24, 24), (32, 32), (48, 48), (80, 36), (100, 160)])
+@pytest.mark.parametrize("n,size", [(6000, 40), (60000, 120)])
+def test_weight_gradient_is_as_accurate_as_fp32_sums(n, size, cin, cout, cuda):
+    """Products of one sign, where everything that is cut off instead of rounded adds up.  Rounded to nearest, the two tf32
+    parts of an operand leave out at most 2^-23 of it and lo x lo 2^-22 of a product, of either sign, and n fp32 additions
+    2^-24 sqrt(n) / 2 of the sum: below 5e-7 for the 3 k rules of an entry and chunk here.  (Parts cut off: 4e-6 to 8e-6.)"""
+    import sparseconvnet_b200 as scn
+    torch.manual_seed(cin)
+    pts = torch.randint(0, size, (n, 3))
+    pts[:, 2] = size // 2 + (size // 5 * torch.sin(pts[:, 0] / 6.0)).long() + torch.randint(0, 2, (n,))
+    x = scn.InputLayer(3, size, mode=4)([pts, torch.zeros(n, 1, device=cuda)])
+    layer = scn.SubmanifoldConvolution(3, cin, cout, 3, False).to(cuda)
+    f = torch.rand(x.features.size(0), cin, device=cuda)
+    y = layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features
+    g = torch.rand_like(y)
+    y.backward(g)
+    want = torch.stack([f[r[:, 0].long()].double().t() @ g[r[:, 1].long()].double()
+                        for r in x.metadata.rulebook(0, x.spatial_size, [3, 3, 3])])
+    e = float((layer.weight.grad[:, 0] - want).norm() / want.norm())
+    assert e <= 5e-7, e
