@@ -62,17 +62,24 @@ int md_touch(scn_metadata *md, cudaStream_t stream) {
   return SCN_OK;
 }
 
-static int chain_finalize(scn_metadata *md, cudaStream_t stream, int *n_built);
+static int chain_finalize(scn_metadata *md, cudaStream_t stream, int *n_built, bool on_host = false);
 static void chain_abandon(scn_metadata *md, cudaStream_t stream);
 
-Grid *find_grid(scn_metadata *md, const int64_t *spatial_size) {
+static Grid *find_grid_now(scn_metadata *md, const int64_t *spatial_size) {  // no pending chain is waited for
   auto it = md->grids.find(make_key(md->dim, spatial_size));
-  if (it == md->grids.end() && md->pending) {
-    // the grid may be one of a chain that was started on the side stream: take the chain over, then look again
-    if (chain_finalize(md, md->last_stream, nullptr) != SCN_OK) return nullptr;
-    it = md->grids.find(make_key(md->dim, spatial_size));
-  }
   return it == md->grids.end() ? nullptr : &it->second;
+}
+
+Grid *find_grid(scn_metadata *md, const int64_t *spatial_size) {
+  Grid *g = find_grid_now(md, spatial_size);
+  if (!g && md->pending) {
+    // the grid may be one of a chain that was started on the side stream: take the chain over, then look again.  Nobody
+    // says which stream will read the grid (a caller that can takes the chain over itself, before), so the host waits
+    // until the tables are finished.
+    if (chain_finalize(md, md->last_stream, nullptr, true) != SCN_OK) return nullptr;
+    g = find_grid_now(md, spatial_size);
+  }
+  return g;
 }
 
 static int alloc_table(HashTable &T, long long expected_sites, cudaStream_t stream) {
@@ -985,7 +992,8 @@ int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
   Rulebook &rb = md->sub_rules[key];
   *out = &rb;
   if (rb.built) return SCN_OK;
-  Grid *g = find_grid(md, spatial_size);
+  if (md->pending && !find_grid_now(md, spatial_size)) SCN_TRY(chain_finalize(md, stream, nullptr));
+  Grid *g = find_grid_now(md, spatial_size);
   if (!g) {
     md->sub_rules.erase(key);
     set_error("submanifold rulebook: no grid for that spatial size");
@@ -1497,11 +1505,6 @@ static bool chain_applies(int dim, const int64_t *filter_size, const int64_t *fi
   return true;
 }
 
-static Grid *find_grid_now(scn_metadata *md, const int64_t *spatial_size) {  // no pending chain is waited for
-  auto it = md->grids.find(make_key(md->dim, spatial_size));
-  return it == md->grids.end() ? nullptr : &it->second;
-}
-
 // A chain that was started on the side stream and whose counts the host has not looked at yet.
 struct PendingChain {
   std::vector<ChainLevel> plan;
@@ -1529,14 +1532,15 @@ static int build_strided_chain_from(scn_metadata *md, std::vector<int64_t> start
                                     const int64_t *stride, int levels, bool safe, cudaStream_t stream, int *n_built);
 
 // The host looks at a started chain: waits for its event (usually long past), makes its levels the object's, and
-// builds again, on `stream` and with the safe bounds, whatever overflowed.
-static int chain_finalize(scn_metadata *md, cudaStream_t stream, int *n_built) {
+// builds again, on `stream` and with the safe bounds, whatever overflowed.  The tables are finished for what follows on
+// `stream`, and with `on_host` for whatever is enqueued anywhere after this call.
+static int chain_finalize(scn_metadata *md, cudaStream_t stream, int *n_built, bool on_host) {
   PendingChain *p = md->pending;
   if (!p) return SCN_OK;
   md->pending = nullptr;
   int st = SCN_OK;
-  if (*(const volatile int *)p->mailbox == kNotPosted) {
-    note_host_wait();
+  if (*(const volatile int *)p->mailbox == kNotPosted || on_host) {
+    if (cudaEventQuery(p->done) == cudaErrorNotReady) note_host_wait();
     if (cudaEventSynchronize(p->done) != cudaSuccess || *(const volatile int *)p->mailbox == kNotPosted) {
       set_error("strided chain: CUDA error while waiting for the level counts");
       st = SCN_ERR_CUDA;
@@ -1565,6 +1569,7 @@ static int chain_finalize(scn_metadata *md, cudaStream_t stream, int *n_built) {
   delete p;
   if (st == SCN_OK && good < L)
     st = build_strided_chain_from(md, rest, filter.data(), stride.data(), L - good, true, stream, n_built);
+  if (st == SCN_OK && good < L && on_host) SCN_CUDA_CHECK(cudaStreamSynchronize(stream));
   return st;
 }
 

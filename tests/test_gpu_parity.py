@@ -524,6 +524,44 @@ def test_chained_strided_levels_equal_level_by_level(kind, fsize, size, cuda):
         assert b[2] == 1                               # one wait for the whole chain
 
 
+@pytest.mark.parametrize("dense", [False, True])
+def test_started_chain_taken_over_by_a_query_from_another_stream(dense, cuda):
+    """The chain is started with stream A, stream B waits for A, and the first question for a deep grid (a call that takes no
+    stream) comes under B: the tables that B reads from then on must be finished, not only ordered before A's next work.
+    `dense`: the levels shrink less than the chain's first guess, so that the query builds them once more."""
+    import sparseconvnet_b200 as scn
+    from sparseconvnet_b200 import SCN
+    rng = np.random.default_rng(5)
+    size, levels = 128, 4
+    pts = rng.integers(0, size, (400000, 3)) * (1 if not dense else 2) % size
+    coords, feats = torch.from_numpy(pts), torch.zeros(len(pts), 1, device=cuda)
+    f = torch.LongTensor([2, 2, 2])
+    want = None
+    for started in (False, True):
+        a, b = torch.cuda.Stream(), torch.cuda.Stream()
+        with torch.cuda.stream(a):
+            x = scn.InputLayer(3, size, mode=3)([coords, feats])
+            if started:
+                SCN.strided_chain_start(x.metadata, x.spatial_size, f, f, levels, cuda)
+        b.wait_stream(a)
+        got = []
+        with torch.cuda.stream(b):
+            sizes = [torch.LongTensor([size >> l] * 3) for l in range(levels + 1)]
+            for l in range(levels, 0, -1) if started else ():
+                assert x.metadata.getNActive(sizes[l]) > 0
+            with torch.no_grad():
+                y = scn.SparseConvNetTensor(x.features, x.metadata, x.spatial_size)
+                for l in range(levels):
+                    y = scn.MaxPooling(3, 2, 2)(y)
+            for l in range(1, levels + 1):
+                got.append(x.metadata.getSpatialLocations(sizes[l]))
+                got += [r.cpu() for r in x.metadata.rulebook(1, sizes[l - 1], f, f)]
+        b.synchronize()
+        if want is None:
+            want = got
+        assert len(got) == len(want) and all(torch.equal(p, q) for p, q in zip(got, want))
+
+
 def test_started_chain_is_dropped_with_its_metadata(cuda):
     """A chain started on the side stream and never asked for: clearing the Metadata, giving it a new input and
     destroying it all release it, and the library's pool holds no more than before."""
