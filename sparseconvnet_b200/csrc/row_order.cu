@@ -119,12 +119,13 @@ k_order_scatter(const KEY *__restrict__ keys, const int *__restrict__ rows_in, l
   const int seg = rows_per_block / kWarps;  // a multiple of 32
   const long long s0 = (long long)blockIdx.x * rows_per_block + (long long)warp * seg;
   const long long s1 = min(n, s0 + seg);
-  for (long long r = s0 + lane; r < s1; r += 32) {
-    const unsigned act = __activemask();
-    const int d = (int)(keys[r] >> shift) & (R - 1);
-    const unsigned peers = __match_any_sync(act, d);
-    if (lane == __ffs(peers) - 1) cnt[warp][d] += (unsigned short)__popc(peers);
-    __syncwarp(act);
+  // all 32 lanes together to the end (digit -1 past it): the counts are plain additions by one lane per digit, and the
+  // places handed out below are in lane order
+  for (long long c0 = s0; c0 < s1; c0 += 32) {
+    const int d = c0 + lane < s1 ? (int)(keys[c0 + lane] >> shift) & (R - 1) : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    if (d >= 0 && lane == __ffs(peers) - 1) cnt[warp][d] += (unsigned short)__popc(peers);
+    __syncwarp();
   }
   // rows of digit d in the blocks before this one: two threads per digit, every other block each
   const int d = tid & (kMaxDigit - 1), half = tid / kMaxDigit;
@@ -156,15 +157,17 @@ k_order_scatter(const KEY *__restrict__ keys, const int *__restrict__ rows_in, l
     }
   }
   __syncthreads();
-  for (long long r = s0 + lane; r < s1; r += 32) {
-    const unsigned act = __activemask();
-    const KEY key = keys[r];
-    const int dg = (int)(key >> shift) & (R - 1);
-    const unsigned peers = __match_any_sync(act, dg);
-    const int pos = base[dg] + cnt[warp][dg] + __popc(peers & ((1u << lane) - 1u));
-    __syncwarp(act);
-    if (lane == __ffs(peers) - 1) cnt[warp][dg] += (unsigned short)__popc(peers);
-    __syncwarp(act);
+  for (long long c0 = s0; c0 < s1; c0 += 32) {
+    const long long r = c0 + lane;
+    const bool here = r < s1;
+    const KEY key = here ? keys[r] : 0;
+    const int dg = here ? (int)(key >> shift) & (R - 1) : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, dg);
+    const int pos = here ? base[dg] + cnt[warp][dg] + __popc(peers & ((1u << lane) - 1u)) : 0;
+    __syncwarp();
+    if (here && lane == __ffs(peers) - 1) cnt[warp][dg] += (unsigned short)__popc(peers);
+    __syncwarp();
+    if (!here) continue;
     if (keys_out) keys_out[pos] = key;
     rows_out[pos] = rows_in ? rows_in[r] : (int)r;
   }
