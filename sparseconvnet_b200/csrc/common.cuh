@@ -123,6 +123,11 @@ __host__ __device__ inline unsigned long long mix64(unsigned long long k) {
 // largest id that named the key; otherwise its aux becomes the smallest.  A free slot is claimed and its id written by one
 // 16-byte compare-and-swap (a compare-and-swap on the key and an atomic on the id were two trips to L2).  LOOK: read the
 // slot first, where most calls find their key there, named by a smaller id, and need no atomic at all.
+// The look is two relaxed 64-bit loads, the key one of them: a key changes once, from free to its value, and is seen as one
+// or the other, never half of each (four 32-bit accesses could show half, and the walk would claim the key a second time).
+// The id beside it may be older than the key; an old one is larger (LAST: smaller) than the present one and costs an atomic
+// that changes nothing.  The 32-bit atomics on row and aux only ever touch slots that are claimed, where the 16-byte
+// compare-and-swap fails on the key whatever half it sees of them.
 template <bool LAST, bool LOOK>
 __device__ inline long long hash_claim(const HashTable &T, unsigned long long key, unsigned id) {
   const unsigned long long mask = T.n_buckets - 1;
@@ -135,10 +140,10 @@ __device__ inline long long hash_claim(const HashTable &T, unsigned long long ke
       Slot *at = T.slots + 2 * b + s;
       Slot was = vacant;
       if (LOOK) {
-        const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(at));
-        was.key = ((unsigned long long)v.y << 32) | v.x;
-        was.row = (int)v.z;
-        was.aux = v.w;
+        unsigned long long ids;
+        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(was.key), "=l"(ids) : "l"(at) : "memory");
+        was.row = (int)(unsigned)ids;
+        was.aux = (unsigned)(ids >> 32);
       }
       if (was.key == kEmptyKey) was = atomicCAS(at, vacant, mine);
       if (was.key == kEmptyKey) return (long long)(at - T.slots);
