@@ -23,7 +23,8 @@
  *    reference object.
  *  - device memory for tables, rulebooks and per-call scratch comes from a stream-ordered memory
  *    pool that the library creates per device (not the device's default pool), through a cache of
- *    freed blocks per stream (at most an eighth of the device's memory idle); scn_trim_memory gives
+ *    freed blocks per stream (at most an eighth of the device's memory idle; calls on a stream that is
+ *    being captured bypass it, their scratch becomes memory nodes of the graph); scn_trim_memory gives
  *    idle blocks, and idle pinned staging memory of host coordinates, back to the driver.
  *  - a scn_metadata belongs to the device that was current at its first use; using it with
  *    another device current is SCN_ERR_BAD_ARG.  It may be used on one stream at a time.

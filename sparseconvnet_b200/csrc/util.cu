@@ -35,6 +35,8 @@ void set_error(const char *fmt, ...) {
 //   * A block freed on a stream is only handed out again to allocations on the same stream (by cudaStreamGetId, which
 //     is not reused as handles are), so stream order alone makes the reuse safe, as for cudaFreeAsync.
 //   * Sizes are rounded up to four steps per power of two, and a request takes a block up to two steps larger.
+//   * While a stream is being captured its blocks come from the pool itself and go back to it, as memory nodes of the graph:
+//     an idle block that a graph has been recorded with would be handed out again and written by every replay.
 //   * Idle blocks are bounded by an eighth of the device's memory; what comes back beyond that goes to the pool, and
 //     the pool returns it to the driver (release threshold 64 MB).  A failing allocation first gives back every idle
 //     block, and so does scn_trim_memory.
@@ -52,7 +54,11 @@ struct DeviceCache {
   std::mutex mu;
   cudaMemPool_t pool = nullptr;
   size_t idle = 0, used = 0, idle_limit = 0;
-  std::unordered_map<void *, int> live;                                                        // block -> step
+  struct Block {
+    int step;
+    bool cached;  // goes to the idle list (no: to the pool)
+  };
+  std::unordered_map<void *, Block> live;
   std::unordered_map<unsigned long long, std::array<std::vector<void *>, kSteps>> idle_blocks;  // per stream id
 };
 DeviceCache *const g_cache = new DeviceCache[64];  // never destroyed: objects may be released while the process ends
@@ -82,6 +88,19 @@ int make_pool(DeviceCache &c) {  // c.mu held
   SCN_CUDA_CHECK(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
   c.idle_limit = total / 8;
   c.pool = p;
+  return SCN_OK;
+}
+
+// Is `stream` being captured?  Otherwise its id, which a stream under capture must not be asked for (the question ends the
+// capture).  The legacy stream is never captured, and must not be asked either while a stream it waits for is.
+int stream_state(cudaStream_t stream, bool *capture, unsigned long long *id) {
+  *capture = false;
+  *id = ~0ull;
+  if (stream == nullptr || stream == cudaStreamLegacy) return SCN_OK;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  SCN_CUDA_CHECK(cudaStreamIsCapturing(stream, &status));
+  *capture = status != cudaStreamCaptureStatusNone;
+  if (!*capture) SCN_CUDA_CHECK(cudaStreamGetId(stream, id));
   return SCN_OK;
 }
 
@@ -115,11 +134,12 @@ int device_alloc(void **p, size_t bytes, cudaStream_t stream) {
   DeviceCache *c = nullptr;
   SCN_TRY(device_cache(&c));
   unsigned long long id = 0;
-  SCN_CUDA_CHECK(cudaStreamGetId(stream, &id));
+  bool capture = false;
+  SCN_TRY(stream_state(stream, &capture, &id));
   const int step = size_step(bytes);
   SCN_REQUIRE(step < kSteps, SCN_ERR_UNSUPPORTED, "allocation of %zu bytes", bytes);
   std::lock_guard<std::mutex> lock(c->mu);
-  auto mine = c->idle_blocks.find(id);
+  auto mine = capture ? c->idle_blocks.end() : c->idle_blocks.find(id);
   if (mine != c->idle_blocks.end())
     for (int s = step; s <= step + 2 && s < kSteps; ++s) {
       auto &list = mine->second[s];
@@ -132,14 +152,14 @@ int device_alloc(void **p, size_t bytes, cudaStream_t stream) {
     }
   SCN_TRY(make_pool(*c));
   cudaError_t e = cudaMallocFromPoolAsync(p, step_bytes(step), c->pool, stream);
-  if (e == cudaErrorMemoryAllocation) {
+  if (e == cudaErrorMemoryAllocation && !capture) {
     cudaGetLastError();
     SCN_TRY(release_idle(*c, 0));
     SCN_CUDA_CHECK(cudaMemPoolTrimTo(c->pool, 0));
     e = cudaMallocFromPoolAsync(p, step_bytes(step), c->pool, stream);
   }
   SCN_CUDA_CHECK(e);
-  c->live[*p] = step;
+  c->live[*p] = {step, !capture};
   c->used += step_bytes(step);
   return SCN_OK;
 }
@@ -149,19 +169,22 @@ int device_free(void *p, cudaStream_t stream) {
   DeviceCache *c = nullptr;
   SCN_TRY(device_cache(&c));
   unsigned long long id = 0;
-  SCN_CUDA_CHECK(cudaStreamGetId(stream, &id));
+  bool capture = false;
+  SCN_TRY(stream_state(stream, &capture, &id));
   std::lock_guard<std::mutex> lock(c->mu);
   auto it = c->live.find(p);
   SCN_REQUIRE(it != c->live.end(), SCN_ERR_BAD_ARG, "freed memory is not a block of the current device");
-  const size_t bytes = step_bytes(it->second);
+  const size_t bytes = step_bytes(it->second.step);
+  // (nobody may write it any more, the graph reads it at every replay: it stays taken)
+  SCN_REQUIRE(!it->second.cached || !capture, SCN_ERR_UNSUPPORTED, "memory taken before a stream capture cannot be given back inside it");
   c->used -= bytes;
-  if (c->idle + bytes > c->idle_limit) {
+  if (!it->second.cached || c->idle + bytes > c->idle_limit) {
     c->live.erase(it);
     SCN_CUDA_CHECK(cudaFreeAsync(p, stream));
     return SCN_OK;
   }
   c->idle += bytes;
-  c->idle_blocks[id][it->second].push_back(p);
+  c->idle_blocks[id][it->second.step].push_back(p);
   return SCN_OK;
 }
 
