@@ -321,6 +321,9 @@ SCN_API int scn_submanifold_convolution_forward(scn_metadata *md, const int64_t 
  * expired wait, and the next convolution works again.  Nothing traps, faults or waits without a
  * bound.  No counterpart in the reference. */
 SCN_API int scn_test_drop_barrier_arrival(void);
+/* Test hook: the `which`-th allocation (device memory or pinned staging) of the calling thread from now on fails with
+ * SCN_ERR_CUDA as if memory had run out; 0: none does. */
+SCN_API int scn_test_fail_allocation(int which);
 
 /* Allocation-free SubmanifoldConvolution.  No counterpart in the reference.
  *

@@ -24,6 +24,7 @@ SIGNATURES = {
     "scn_tc_probe_mma": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _vp,
                                    C.POINTER(C.c_double), C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "scn_test_drop_barrier_arrival": (C.c_int, []),
+    "scn_test_fail_allocation": (C.c_int, [C.c_int]),
     "scn_set_split_rows": (C.c_int, [_vp, _vp]),
     "scn_split_rows_written": (C.c_int, []),
     "scn_set_weight_token": (C.c_int, [C.c_uint64]),

@@ -221,6 +221,31 @@ inline long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
 // whose release threshold is raised once so freed blocks are reused instead of returned).
 int device_alloc(void **p, size_t bytes, cudaStream_t stream);
 int device_free(void *p, cudaStream_t stream);
+int test_allocation();  // the test hook of device_alloc, for the pinned buffers too
+
+// Blocks that go back, stream-ordered, on every way out of a function.
+class Scratch {
+ public:
+  explicit Scratch(cudaStream_t stream) : stream_(stream) {}
+  Scratch(const Scratch &) = delete;
+  ~Scratch() {
+    for (int i = 0; i < n_; ++i) device_free(p_[i], stream_);
+  }
+  template <typename T>
+  int get(T **p, size_t bytes) {
+    SCN_REQUIRE(n_ < kMost, SCN_ERR_UNSUPPORTED, "more than %d scratch blocks", kMost);
+    void *q = nullptr;
+    SCN_TRY(device_alloc(&q, bytes, stream_));
+    *p = (T *)(p_[n_++] = q);
+    return SCN_OK;
+  }
+
+ private:
+  static constexpr int kMost = 8;
+  void *p_[kMost];
+  int n_ = 0;
+  cudaStream_t stream_;
+};
 
 // Exclusive prefix sum of n int32 values (out may alias in).  total_dev (may be null)
 // receives the sum of all inputs as int32.

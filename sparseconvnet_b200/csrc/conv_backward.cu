@@ -374,15 +374,14 @@ static int launch_dweight(const float *in, int ld_in, long long n_in_rows, const
   const long long chunk_rows = ceil_div(ceil_div(n_entries, chunks), S::LIST) * S::LIST;
   const int grid_x = (int)ceil_div(n_entries, chunk_rows);
   const long long w_elems = (long long)K * cin * cout;
+  Scratch tmp(stream);
   float *partial = d_weight;
-  if (grid_x > 1) SCN_TRY(device_alloc((void **)&partial, sizeof(float) * (size_t)grid_x * w_elems, stream));
+  if (grid_x > 1) SCN_TRY(tmp.get(&partial, sizeof(float) * (size_t)grid_x * w_elems));
   const int vec_in = cin % 4 == 0 && ld_in % 4 == 0 && (uintptr_t)in % 16 == 0;
   const int vec_out = cout % 4 == 0 && ld_out % 4 == 0 && (uintptr_t)dout % 16 == 0;
   SCN_LAUNCH((k_conv_dweight_mma<WM, WN, MT>), dim3((unsigned)grid_x, (unsigned)K, (unsigned)tiles), S::THREADS, S::SMEM, stream, in, ld_in, n_in_rows, dout, ld_out, n_out_rows, nbr, n_entries, swap, cin, cout, vec_in, vec_out, chunk_rows, partial, flags);
-  if (grid_x > 1) {
+  if (grid_x > 1)
     SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, grid_x, w_elems, d_weight);
-    SCN_TRY(device_free(partial, stream));
-  }
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }
@@ -471,14 +470,13 @@ static int dweight_thin(const float *in, long long rows_in, const float *d_out, 
   const long long chunk_rows = ceil_div(ceil_div(rows_out, wanted), 256) * 256;
   const int chunks = (int)ceil_div(rows_out, chunk_rows);
   const long long w_elems = (long long)K * cin * cout;
+  Scratch tmp(stream);
   float *partial = d_weight;
-  if (chunks > 1) SCN_TRY(device_alloc((void **)&partial, sizeof(float) * (size_t)chunks * w_elems, stream));
+  if (chunks > 1) SCN_TRY(tmp.get(&partial, sizeof(float) * (size_t)chunks * w_elems));
   const auto kernel = cin == 1 ? k_conv_dweight_thin<1> : cin == 2 ? k_conv_dweight_thin<2> : k_conv_dweight_thin<3>;
   SCN_LAUNCH(kernel, dim3((unsigned)chunks, (unsigned)columns), 256, 0, stream, in, rows_in, d_out, rows_out, nbr, K, cout, chunk_rows, partial, flags);
-  if (chunks > 1) {
+  if (chunks > 1)
     SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, chunks, w_elems, d_weight);
-    SCN_TRY(device_free(partial, stream));
-  }
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }
@@ -543,12 +541,12 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
   if (d_bias) {
     const int chunks = n_chunks(rows_out);
     const long long chunk_rows = ceil_div(rows_out, chunks);
+    Scratch tmp(stream);
     float *partial = nullptr;
-    SCN_TRY(device_alloc((void **)&partial, sizeof(float) * (size_t)chunks * n_out_planes, stream));
+    SCN_TRY(tmp.get(&partial, sizeof(float) * (size_t)chunks * n_out_planes));
     SCN_LAUNCH(k_column_sums, dim3((unsigned)ceil_div(n_out_planes, 32), (unsigned)chunks), 256, 0, stream, d_out, rows_out, n_out_planes, chunk_rows, partial);
     SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(n_out_planes, 256), 256, 0, stream, partial, chunks, (long long)n_out_planes, d_bias);
     SCN_CUDA_CHECK(cudaGetLastError());
-    SCN_TRY(device_free(partial, stream));
   }
 
   // ---- d_weight -----------------------------------------------------------------------------------
@@ -572,20 +570,21 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
     } else {
       const int chunks = n_chunks(n_entries);
       const long long chunk_rows = ceil_div(ceil_div(n_entries, chunks), 32) * 32;
+      Scratch tmp(stream);
       float *partial = nullptr;
-      SCN_TRY(device_alloc((void **)&partial, sizeof(float) * (size_t)chunks * w_elems, stream));
+      SCN_TRY(tmp.get(&partial, sizeof(float) * (size_t)chunks * w_elems));
       const int tiles = groups * (int)ceil_div(cin, 32) * (int)ceil_div(cout, 32);
       SCN_LAUNCH(k_conv_dweight, dim3((unsigned)chunks, (unsigned)K, (unsigned)tiles), 256, 0, stream, in, n_in_planes, rows_in, d_out, n_out_planes, rows_out, rb.nbr, n_entries, transposed ? 1 : 0, cin, cout, groups, chunk_rows, partial, md->flags_dev);
       SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, chunks, w_elems, d_weight);
       SCN_CUDA_CHECK(cudaGetLastError());
-      SCN_TRY(device_free(partial, stream));
     }
   }
 
   // ---- d_input ------------------------------------------------------------------------------------
   if (d_in) {
+    Scratch tmp(stream);
     float *wt = nullptr;
-    SCN_TRY(device_alloc((void **)&wt, sizeof(float) * (size_t)w_elems, stream));
+    SCN_TRY(tmp.get(&wt, sizeof(float) * (size_t)w_elems));
     // Deconvolution: coarse row <- fine rows, the table as built.  A submanifold rulebook of odd filter sizes is its own
     // transposed one with the offsets in reverse, so that its table and row order serve the backward pass as well.
     const bool mirrored = !transposed && rb.symmetric;
@@ -594,7 +593,6 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
     if (use_tnbr) SCN_TRY(rulebook_transposed(rb, stream));
     SCN_TRY(conv_forward_table(rb, use_tnbr, d_out, rows_out, d_in, rows_in, wt, nullptr, cout, cin, groups,
                                g_backward_precision.load(), md->flags_dev, stream));
-    SCN_TRY(device_free(wt, stream));
   }
   return SCN_OK;
 }
@@ -648,8 +646,9 @@ int scn_rows_affine_backward(const float *in_features, const float *d_out_featur
   const long long chunks = std::max<long long>(1, std::min<long long>(148 * 32 / tiles, n_rows / 512));
   const long long chunk_rows = ceil_div(ceil_div(n_rows, chunks), 32) * 32;
   const int grid_x = (int)ceil_div(n_rows, chunk_rows);
+  Scratch tmp(stream);
   float *partial = nullptr;
-  SCN_TRY(device_alloc((void **)&partial, sizeof(float) * (size_t)grid_x * (size_t)(w_elems + n_out_planes), stream));
+  SCN_TRY(tmp.get(&partial, sizeof(float) * (size_t)grid_x * (size_t)(w_elems + n_out_planes)));
   float *bias_partial = partial + (size_t)grid_x * w_elems;
   SCN_LAUNCH(k_conv_dweight, dim3((unsigned)grid_x, 1, (unsigned)tiles), 256, 0, stream, in_features, n_in_planes, (long long)n_rows, d_out_features, n_out_planes, (long long)n_rows, nullptr, (long long)n_rows, 0, n_in_planes, n_out_planes, 1, chunk_rows, partial, nullptr);
   SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 32), 32, 0, stream, partial, grid_x, w_elems, d_weight);
@@ -658,7 +657,7 @@ int scn_rows_affine_backward(const float *in_features, const float *d_out_featur
     SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(n_out_planes, 32), 32, 0, stream, bias_partial, grid_x, (long long)n_out_planes, d_bias);
   }
   SCN_CUDA_CHECK(cudaGetLastError());
-  return device_free(partial, stream);
+  return SCN_OK;
 }
 
 int scn_deconvolution_backward(scn_metadata *md, const int64_t *input_size, const int64_t *output_size,

@@ -493,23 +493,22 @@ int launch(DwParams &P, const Rulebook &rb, const float *t_rows, const float *g_
   const long long per_wave = std::max(1, 148 / (P.n_groups * pairs));
   P.n_chunks = (int)std::min<long long>(P.n_tiles, per_wave * ceil_div(P.n_tiles, per_wave * kMaxTiles));
   const long long w_elems = (long long)P.K * P.cin * P.cout;
+  Scratch tmp(stream);
   P.partial = d_weight;
-  if (P.n_chunks > 1) SCN_TRY(device_alloc((void **)&P.partial, sizeof(float) * (size_t)P.n_chunks * w_elems, stream));
+  if (P.n_chunks > 1) SCN_TRY(tmp.get(&P.partial, sizeof(float) * (size_t)P.n_chunks * w_elems));
   unsigned char *split = nullptr;
   const int t_per = (int)ceil_div(P.t_planes, PT) * PT / 8, g_per = (int)ceil_div(P.g_planes, PG) * PG / 8;
   const size_t t_size = (size_t)(P.n_t * split_row_bytes(t_per, PT)), g_size = (size_t)(P.n_g * split_row_bytes(g_per, PG));
-  SCN_TRY(device_alloc((void **)&split, t_size + g_size, stream));
+  SCN_TRY(tmp.get(&split, t_size + g_size));
   P.t_rows = split;
   P.g_rows = split + t_size;
   SCN_LAUNCH(k_dweight_split, (unsigned)ceil_div(P.n_t * t_per, 256), 256, 0, stream, t_rows, split, P.n_t * t_per, P.t_planes, t_per, PT);
   SCN_LAUNCH(k_dweight_split, (unsigned)ceil_div(P.n_g * g_per, 256), 256, 0, stream, g_rows, split + t_size, P.n_g * g_per, P.g_planes, g_per, PG);
   SCN_LAUNCH((k_dweight_tile<PT, PG>), dim3((unsigned)P.n_groups, (unsigned)P.n_chunks, (unsigned)pairs), kThreads, S::SMEM, stream, P);
-  if (P.n_chunks > 1) {
+  if (P.n_chunks > 1)
     SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, P.partial, P.n_chunks, w_elems, d_weight);
-    SCN_TRY(device_free(P.partial, stream));
-  }
   SCN_CUDA_CHECK(cudaGetLastError());
-  return device_free(split, stream);
+  return SCN_OK;
 }
 
 }  // namespace

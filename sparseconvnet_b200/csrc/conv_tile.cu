@@ -712,7 +712,11 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
     sm_count[dev].store(n_sm);
   }
 
-  WeightImage wi;
+  struct Image : WeightImage {
+    cudaStream_t stream;
+    ~Image() { weight_image_put(*this, stream); }
+  } wi;
+  wi.stream = stream;
   bool build = true;
   SCN_TRY(weight_image_get(WIMG_TILE, K, cin, cout, SP * 4 + parts, (size_t)K * cinp * coutp * 2 * parts, stream, &wi, &build));
   if (build)
@@ -722,9 +726,10 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
   // the input rows as bf16 parts, made once per call: a row is gathered by up to K output rows.  The layer that made the
   // rows may have left them in this form already, and the next one may want them so.
   const SplitRows rows = take_split_rows();
+  Scratch tmp(stream);
   unsigned char *split = nullptr;
   const bool given = rows.in && !pre_scale && !in_b && cinp == cin;
-  if (!given) SCN_TRY(device_alloc((void **)&split, (size_t)std::max<long long>(n_in, 1) * cinp * 2 * parts, stream));
+  if (!given) SCN_TRY(tmp.get(&split, (size_t)std::max<long long>(n_in, 1) * cinp * 2 * parts));
   if (n_in > 0 && !given) {
     const int ppr = cinp / 8;
     const long long n_pieces = n_in * ppr;
@@ -763,27 +768,15 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
   const double w_bytes = (double)coutp * SP * 2 * parts, a_bytes = kRows * SP * 2.0 * parts;
   const char *e = getenv("SCN_TILE_SPLIT");
   P.n_split = e ? std::max(1, atoi(e)) : split_parts(P.n_tiles, K, n_slices, (a_bytes + w_bytes) / 32.0, cout, n_sm);
-  float *partial = nullptr;
-  int rc = SCN_OK;
   P.out_split = P.n_split > 1 ? nullptr : out_split;
-  if (P.n_split > 1) {
-    rc = device_alloc((void **)&partial, (size_t)P.n_split * P.n_tiles * kRows * cout * sizeof(float), stream);
-    P.out = partial;
-  }
-  if (rc == SCN_OK) {
-    if (terms == 3)
-      rc = SP == 32 ? launch_tile<3, 32>(P, n_sm, dev, stream) : launch_tile<3, 16>(P, n_sm, dev, stream);
-    else
-      rc = SP == 64 ? launch_tile<1, 64>(P, n_sm, dev, stream) : launch_tile<1, 32>(P, n_sm, dev, stream);
-  }
-  if (rc == SCN_OK && P.n_split > 1)
-    rc = sum_partial_tiles(partial, P.n_split, P.n_tiles * kRows, cout, ord.order, n_out, bias, bn_scale, bn_shift, leak, out, stream,
-                           out_split, P.out_sp, parts);
-  if (rc == SCN_OK && out_split) split_rows_written();
-  device_free(partial, stream);
-  device_free(split, stream);
-  const int rf = weight_image_put(wi, stream);
-  return rc != SCN_OK ? rc : rf;
+  if (P.n_split > 1) SCN_TRY(tmp.get(&P.out, (size_t)P.n_split * P.n_tiles * kRows * cout * sizeof(float)));
+  const auto launch = terms == 3 ? (SP == 32 ? launch_tile<3, 32> : launch_tile<3, 16>) : (SP == 64 ? launch_tile<1, 64> : launch_tile<1, 32>);
+  SCN_TRY(launch(P, n_sm, dev, stream));
+  if (P.n_split > 1)
+    SCN_TRY(sum_partial_tiles(P.out, P.n_split, P.n_tiles * kRows, cout, ord.order, n_out, bias, bn_scale, bn_shift, leak, out,
+                              stream, out_split, P.out_sp, parts));
+  if (out_split) split_rows_written();
+  return SCN_OK;
 }
 
 }  // namespace scn

@@ -142,6 +142,7 @@ void pack_rows(const KeyLayout &L, const long long *coords, long long first, lon
 }  // namespace
 
 int pinned_acquire(size_t bytes, void **p, size_t *got) {
+  SCN_TRY(test_allocation());
   size_t want = 4096;
   while (want < bytes) want <<= 1;
   *got = want;

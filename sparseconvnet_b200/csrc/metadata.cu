@@ -677,6 +677,116 @@ static int md_clear(scn_metadata *md, cudaStream_t stream) {
 
 constexpr int64_t kPackRows = 4 << 20;  // host coordinates: packed by the host up to here (32 MB of pinned memory)
 
+// Packed keys of host coordinates; given back unless a kernel may still be reading them (after an error nobody knows).
+struct PinnedKeys {
+  unsigned long long *p = nullptr;
+  size_t bytes = 0;
+  bool in_use = false;
+  ~PinnedKeys() {
+    if (p && !in_use) pinned_release(p, bytes);
+  }
+};
+
+// The site table `g` and the input rules of `coords`; what it leaves behind when it fails is the caller's to free.
+static int build_input(scn_metadata *md, const int64_t *coords, int coords_on_device, int64_t n, int ncols,
+                       int64_t batch_size, int mode, int64_t bl_length, cudaStream_t stream, Grid &g) {
+  SCN_TRY(alloc_table(g.table, n, stream));
+  SCN_TRY(device_alloc((void **)&g.row_keys, sizeof(unsigned long long) * (size_t)std::max<int64_t>(n, 1), stream));
+  const unsigned tiles = (unsigned)ceil_div(std::max<int64_t>(n, 1), kRankTile);
+  Scratch tmp(stream);
+  int *slot_of = nullptr, *base = nullptr, *cursor = nullptr;
+  uint2 *words = nullptr;
+  SCN_TRY(tmp.get(&slot_of, sizeof(int) * (size_t)std::max<int64_t>(n, 1)));
+  if (mode != 0) {
+    SCN_TRY(tmp.get(&words, sizeof(uint2) * (kRankTile / 32) * (size_t)tiles));
+    SCN_TRY(tmp.get(&base, sizeof(int) * (size_t)tiles));
+  }
+
+  const long long *coords_dev = (const long long *)coords;
+  PinnedKeys packed;
+  unsigned long long *packed_dev = nullptr;
+  int packed_samples = 0;
+  if (!coords_on_device && n > 0 && n <= kPackRows) {
+    SCN_TRY(pinned_acquire(sizeof(unsigned long long) * (size_t)n, (void **)&packed.p, &packed.bytes));
+    bool bad = false;
+    pack_keys(g.layout, coords_dev, n, ncols, bl_length, packed.p, &packed_samples, &bad);
+    if (bad) return flags_to_status(FLAG_COORD_RANGE);
+    // (copied to the device first, 400 k keys took 240 us longer: the bus is what the insert kernel waits for either way)
+    SCN_CUDA_CHECK(cudaHostGetDevicePointer((void **)&packed_dev, packed.p, 0));
+  } else if (!coords_on_device && n > 0) {
+    const size_t bytes = sizeof(long long) * (size_t)n * ncols;
+    long long *staged = nullptr;
+    SCN_TRY(tmp.get(&staged, bytes));
+    SCN_CUDA_CHECK(cudaMemcpyAsync(staged, coords, bytes, cudaMemcpyHostToDevice, stream));
+    coords_dev = staged;
+  }
+
+  const int threads = 256;
+  unsigned blocks = (unsigned)ceil_div(std::max<int64_t>(n, 1), threads);
+  int *n_samples = md->scalars_dev, *done = md->scalars_dev + 1;  // batch indices in use; finished blocks
+  Fills fills{};
+  fill_add(fills, g.table.slots, 2 * g.table.n_buckets * sizeof(Slot), true);
+  fill_add(fills, n_samples, 2 * sizeof(int), false);
+  SCN_TRY(fill_launch(fills, stream));
+  HostPost post{};
+  SCN_TRY(post_begin(md, post));
+  if (n > 0) {
+    packed.in_use = true;
+    SCN_LAUNCH_DIM(md->dim, k_insert_input, blocks, threads, 0, stream, g.layout, g.table, coords_dev, packed_dev, n, ncols, mode, (long long)bl_length, g.row_keys, slot_of, md->flags_dev, n_samples);
+    if (mode == 0)
+      SCN_LAUNCH(k_blank_overwritten, blocks, threads, 0, stream, g.table.slots, slot_of, n, g.row_keys, md->flags_dev, n_samples, post);
+    SCN_CUDA_CHECK(cudaGetLastError());
+  }
+  if (mode != 0 && n > 0) {
+    SCN_LAUNCH(k_first_ranks, tiles, 256, 0, stream, g.table.slots, slot_of, (long long)n, nullptr, 1, words, base, done, nullptr, md->flags_dev, true, n_samples, post);
+    const long long n_slots = 2 * (long long)g.table.n_buckets;
+    SCN_LAUNCH(k_number_slots, (unsigned)ceil_div(n_slots, threads), threads, 0, stream, g.table.slots, n_slots, words, base, g.row_keys);
+    SCN_CUDA_CHECK(cudaGetLastError());
+  }
+
+  int flags = 0, total = 0, samples = 0;
+  if (n > 0) {
+    SCN_TRY(wait_posted(md->mailbox, stream));
+    packed.in_use = false;
+    const volatile int *host = md->mailbox;
+    flags = host[1];
+    total = host[2];
+    samples = packed.p ? packed_samples : host[3];
+  }
+  SCN_TRY(flags_to_status(flags));
+  long long active = (mode == 0) ? n : total;
+  // Every point has a site of its own (no repeated coordinates, no empty slots): rows are numbered in
+  // order of first occurrence, so row i is point i and the rule table is the identity -- the feature
+  // pass is then the plain copy of mode 0 and no table is built.  Otherwise: CSR of the input rows of
+  // every site, each site's rows ascending (the order the reference sums them in).
+  const bool identity = mode != 0 && active == n;
+  if (mode != 0 && n > 0 && active > 0 && !identity) {
+    SCN_TRY(device_alloc((void **)&md->input_csr_start, sizeof(int) * (size_t)(n + 1), stream));
+    SCN_TRY(device_alloc((void **)&md->input_csr_rows, sizeof(int) * (size_t)n, stream));
+    SCN_TRY(tmp.get(&cursor, sizeof(int) * (size_t)(n + 1)));
+    SCN_CUDA_CHECK(cudaMemsetAsync(cursor, 0, sizeof(int) * (size_t)(n + 1), stream));
+    SCN_LAUNCH(k_count_per_site, blocks, threads, 0, stream, g.table.slots, slot_of, n, cursor);
+    SCN_TRY(exclusive_scan_i32(cursor, md->input_csr_start, n + 1, nullptr, stream));
+    SCN_CUDA_CHECK(cudaMemsetAsync(cursor, 0, sizeof(int) * (size_t)(n + 1), stream));
+    SCN_LAUNCH(k_fill_per_site, blocks, threads, 0, stream, g.table.slots, slot_of, n, md->input_csr_start, cursor, md->input_csr_rows);
+    unsigned sblocks = (unsigned)ceil_div(active, threads);
+    SCN_LAUNCH(k_sort_segments, sblocks, threads, 0, stream, md->input_csr_start, active, md->input_csr_rows);
+    SCN_CUDA_CHECK(cudaGetLastError());
+  }
+  g.n_active = active;
+  g.may_have_blank_rows = (mode == 0);
+  // batch size: IOLayersRules.h:25,35,52-53 -- one sample when there is no batch column,
+  // otherwise max(requested, largest index + 1)
+  if (bl_length > 0)
+    g.batch_size = batch_size;
+  else if (ncols == md->dim)
+    g.batch_size = 1;
+  else
+    g.batch_size = std::max<long long>(batch_size, samples);
+  md->input_mode = identity ? 0 : mode;  // what the feature passes do (a copy when the table is the identity)
+  return SCN_OK;
+}
+
 static int md_input_layer(scn_metadata *md, const int64_t *spatial_size, const int64_t *coords,
                           int coords_on_device, int64_t n, int ncols, int64_t batch_size, int mode,
                           int64_t bl_length, cudaStream_t stream, int64_t *n_active) {
@@ -693,121 +803,19 @@ static int md_input_layer(scn_metadata *md, const int64_t *spatial_size, const i
   // the old input would otherwise stay cached with the old row counts.  (The reference asserts that
   // the object is empty, IOLayersRules.h:22-24.)
   SCN_TRY(md_clear(md, stream));
-  auto key = make_key(md->dim, spatial_size);
 
   Grid g;
   SCN_TRY(make_layout(md->dim, spatial_size, g.layout));
-  SCN_TRY(alloc_table(g.table, n, stream));
-  SCN_TRY(device_alloc((void **)&g.row_keys, sizeof(unsigned long long) * (size_t)std::max<int64_t>(n, 1), stream));
-
-  const long long *coords_dev = (const long long *)coords;
-  long long *staged = nullptr;
-  unsigned long long *packed = nullptr, *packed_dev = nullptr;
-  size_t packed_bytes = 0;
-  int packed_samples = 0;
-  if (!coords_on_device && n > 0 && n <= kPackRows) {
-    SCN_TRY(pinned_acquire(sizeof(unsigned long long) * (size_t)n, (void **)&packed, &packed_bytes));
-    bool bad = false;
-    pack_keys(g.layout, coords_dev, n, ncols, bl_length, packed, &packed_samples, &bad);
-    if (bad) {
-      pinned_release(packed, packed_bytes);
-      free_grid(g, stream);
-      return flags_to_status(FLAG_COORD_RANGE);
-    }
-    // (copied to the device first, 400 k keys took 240 us longer: the bus is what the insert kernel waits for either way)
-    SCN_CUDA_CHECK(cudaHostGetDevicePointer((void **)&packed_dev, packed, 0));
-  } else if (!coords_on_device && n > 0) {
-    size_t bytes = sizeof(long long) * (size_t)n * ncols;
-    SCN_TRY(device_alloc((void **)&staged, bytes, stream));
-    SCN_CUDA_CHECK(cudaMemcpyAsync(staged, coords, bytes, cudaMemcpyHostToDevice, stream));
-    coords_dev = staged;
-  }
-
-  const int threads = 256;
-  unsigned blocks = (unsigned)ceil_div(std::max<int64_t>(n, 1), threads);
-  int *n_samples = md->scalars_dev, *done = md->scalars_dev + 1;  // batch indices in use; finished blocks
-  Fills fills{};
-  fill_add(fills, g.table.slots, 2 * g.table.n_buckets * sizeof(Slot), true);
-  fill_add(fills, n_samples, 2 * sizeof(int), false);
-  SCN_TRY(fill_launch(fills, stream));
-  HostPost post{};
-  SCN_TRY(post_begin(md, post));
-  int *slot_of = nullptr, *base = nullptr, *cursor = nullptr;
-  uint2 *words = nullptr;
-  SCN_TRY(device_alloc((void **)&slot_of, sizeof(int) * (size_t)std::max<int64_t>(n, 1), stream));
-  if (n > 0) {
-    SCN_LAUNCH_DIM(md->dim, k_insert_input, blocks, threads, 0, stream, g.layout, g.table, coords_dev, packed_dev, n, ncols, mode, (long long)bl_length, g.row_keys, slot_of, md->flags_dev, n_samples);
-    if (mode == 0)
-      SCN_LAUNCH(k_blank_overwritten, blocks, threads, 0, stream, g.table.slots, slot_of, n, g.row_keys, md->flags_dev, n_samples, post);
-    SCN_CUDA_CHECK(cudaGetLastError());
-  }
-  if (mode != 0 && n > 0) {
-    const unsigned tiles = (unsigned)ceil_div(n, kRankTile);
-    SCN_TRY(device_alloc((void **)&words, sizeof(uint2) * (kRankTile / 32) * (size_t)tiles, stream));
-    SCN_TRY(device_alloc((void **)&base, sizeof(int) * (size_t)tiles, stream));
-    SCN_LAUNCH(k_first_ranks, tiles, 256, 0, stream, g.table.slots, slot_of, (long long)n, nullptr, 1, words, base, done, nullptr, md->flags_dev, true, n_samples, post);
-    const long long n_slots = 2 * (long long)g.table.n_buckets;
-    SCN_LAUNCH(k_number_slots, (unsigned)ceil_div(n_slots, threads), threads, 0, stream, g.table.slots, n_slots, words, base, g.row_keys);
-    SCN_CUDA_CHECK(cudaGetLastError());
-  }
-
-  // stream-ordered: what only the kernels above read goes back before the host waits
-  device_free(staged, stream);
-  device_free(words, stream);
-  device_free(base, stream);
-  staged = nullptr;
-  int flags = 0, total = 0, samples = 0;
-  if (n > 0) {
-    const int waited = wait_posted(md->mailbox, stream);
-    if (waited == SCN_OK) pinned_release(packed, packed_bytes);  // (after an error nobody knows who still reads it)
-    SCN_TRY(waited);
-    const volatile int *host = md->mailbox;
-    flags = host[1];
-    total = host[2];
-    samples = packed ? packed_samples : host[3];
-  }
-  long long active = (mode == 0) ? n : total;
-  // Every point has a site of its own (no repeated coordinates, no empty slots): rows are numbered in
-  // order of first occurrence, so row i is point i and the rule table is the identity -- the feature
-  // pass is then the plain copy of mode 0 and no table is built.  Otherwise: CSR of the input rows of
-  // every site, each site's rows ascending (the order the reference sums them in).
-  const bool identity = mode != 0 && flags == 0 && active == n;
-  if (mode != 0 && n > 0 && flags == 0 && active > 0 && !identity) {
-    SCN_TRY(device_alloc((void **)&md->input_csr_start, sizeof(int) * (size_t)(n + 1), stream));
-    SCN_TRY(device_alloc((void **)&md->input_csr_rows, sizeof(int) * (size_t)n, stream));
-    SCN_TRY(device_alloc((void **)&cursor, sizeof(int) * (size_t)(n + 1), stream));
-    SCN_CUDA_CHECK(cudaMemsetAsync(cursor, 0, sizeof(int) * (size_t)(n + 1), stream));
-    SCN_LAUNCH(k_count_per_site, blocks, threads, 0, stream, g.table.slots, slot_of, n, cursor);
-    SCN_TRY(exclusive_scan_i32(cursor, md->input_csr_start, n + 1, nullptr, stream));
-    SCN_CUDA_CHECK(cudaMemsetAsync(cursor, 0, sizeof(int) * (size_t)(n + 1), stream));
-    SCN_LAUNCH(k_fill_per_site, blocks, threads, 0, stream, g.table.slots, slot_of, n, md->input_csr_start, cursor, md->input_csr_rows);
-    unsigned sblocks = (unsigned)ceil_div(active, threads);
-    SCN_LAUNCH(k_sort_segments, sblocks, threads, 0, stream, md->input_csr_start, active, md->input_csr_rows);
-    SCN_CUDA_CHECK(cudaGetLastError());
-  }
-  device_free(slot_of, stream);
-  device_free(cursor, stream);
-  int st = flags_to_status(flags);
+  const int st = build_input(md, coords, coords_on_device, n, ncols, batch_size, mode, bl_length, stream, g);
   if (st != SCN_OK) {
     free_grid(g, stream);
     clear_input_rules(md, stream);
     return st;
   }
-  g.n_active = active;
-  g.may_have_blank_rows = (mode == 0);
-  // batch size: IOLayersRules.h:25,35,52-53 -- one sample when there is no batch column,
-  // otherwise max(requested, largest index + 1)
-  if (bl_length > 0)
-    g.batch_size = batch_size;
-  else if (ncols == md->dim)
-    g.batch_size = 1;
-  else
-    g.batch_size = std::max<long long>(batch_size, samples);
-  md->input_mode = identity ? 0 : mode;  // what the feature passes do (a copy when the table is the identity)
   md->input_n_rows = n;
-  md->input_n_active = active;
-  md->grids[key] = g;
-  *n_active = active;
+  md->input_n_active = g.n_active;
+  md->grids[make_key(md->dim, spatial_size)] = g;
+  *n_active = g.n_active;
   return SCN_OK;
 }
 
@@ -985,20 +993,8 @@ k_rules_init(unsigned long long *counts, int n_counts, unsigned *masks, long lon
   }
 }
 
-int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
-                             const int64_t *filter_size, cudaStream_t stream, Rulebook **out) {
-  SCN_TRY(md_touch(md, stream));
-  auto key = make_key(md->dim, spatial_size, filter_size);
-  Rulebook &rb = md->sub_rules[key];
-  *out = &rb;
-  if (rb.built) return SCN_OK;
-  if (md->pending && !find_grid_now(md, spatial_size)) SCN_TRY(chain_finalize(md, stream, nullptr));
-  Grid *g = find_grid_now(md, spatial_size);
-  if (!g) {
-    md->sub_rules.erase(key);
-    set_error("submanifold rulebook: no grid for that spatial size");
-    return SCN_ERR_NO_GRID;
-  }
+// (what it leaves in `rb` when it fails is the caller's to free)
+static int build_submanifold(scn_metadata *md, Grid *g, const int64_t *filter_size, cudaStream_t stream, Rulebook &rb) {
   long long K = 1;
   FilterDesc F{};
   for (int d = 0; d < md->dim; ++d) {
@@ -1043,6 +1039,28 @@ int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
   }
   rb.built = true;
   g_rulebook_builds.fetch_add(1);
+  return SCN_OK;
+}
+
+int get_submanifold_rulebook(scn_metadata *md, const int64_t *spatial_size,
+                             const int64_t *filter_size, cudaStream_t stream, Rulebook **out) {
+  SCN_TRY(md_touch(md, stream));
+  auto key = make_key(md->dim, spatial_size, filter_size);
+  auto have = md->sub_rules.find(key);
+  if (have != md->sub_rules.end()) {
+    *out = &have->second;
+    return SCN_OK;
+  }
+  if (md->pending && !find_grid_now(md, spatial_size)) SCN_TRY(chain_finalize(md, stream, nullptr));
+  Grid *g = find_grid_now(md, spatial_size);
+  SCN_REQUIRE(g, SCN_ERR_NO_GRID, "submanifold rulebook: no grid for that spatial size");
+  Rulebook rb;
+  const int st = build_submanifold(md, g, filter_size, stream, rb);
+  if (st != SCN_OK) {
+    free_rulebook(rb, stream);
+    return st;
+  }
+  *out = &(md->sub_rules[key] = rb);
   return SCN_OK;
 }
 
@@ -1172,24 +1190,9 @@ k_strided_fill(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Slot *slots, const u
   post_counts(counts, K, counts_host);
 }
 
-int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int64_t *output_size,
-                         const int64_t *filter_size, const int64_t *filter_stride,
-                         cudaStream_t stream, Rulebook **out) {
-  SCN_TRY(md_touch(md, stream));
-  auto key = make_key(md->dim, input_size, filter_size, filter_stride);
-  Rulebook &rb = md->strided_rules[key];
-  *out = &rb;
-  if (rb.built) return SCN_OK;
-  if (md->pending) {  // it may be one of a chain that was started on the side stream
-    SCN_TRY(chain_finalize(md, stream, nullptr));
-    if (rb.built) return SCN_OK;
-  }
-  Grid *gin = find_grid(md, input_size);
-  if (!gin) {
-    md->strided_rules.erase(key);
-    set_error("strided rulebook: no grid for the input spatial size");
-    return SCN_ERR_NO_GRID;
-  }
+// (what it leaves in `gout` and `rb` when it fails is the caller's to free)
+static int build_strided(scn_metadata *md, Grid *gin, const int64_t *output_size, const int64_t *filter_size,
+                         const int64_t *filter_stride, cudaStream_t stream, Grid &gout, Rulebook &rb) {
   SCN_TRY(ensure_scratch(md, stream));
   FilterDesc F{};
   long long K = 1;
@@ -1210,13 +1213,11 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
   long long n_ids = n_in * F.tmax;
   SCN_REQUIRE(n_ids < (1ll << 31), SCN_ERR_UNSUPPORTED, "too many (site, output) candidates");
 
-  auto okey = make_key(md->dim, output_size);
-  auto old = md->grids.find(okey);
+  auto old = md->grids.find(make_key(md->dim, output_size));
   if (old != md->grids.end()) {
     free_grid(old->second, stream);
     md->grids.erase(old);
   }
-  Grid gout;
   SCN_TRY(make_layout(md->dim, output_size, gout.layout));
   SCN_REQUIRE(gout.layout.batch_bits >= gin->layout.batch_bits ||
                   gin->batch_size <= (1ll << gout.layout.batch_bits),
@@ -1224,14 +1225,15 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
   gout.batch_size = gin->batch_size;
 
   const int threads = 256;
+  Scratch tmp(stream);
   int *slot_of = nullptr, *base = nullptr;
   uint2 *words = nullptr;
   long long n_out = 0;
   if (n_ids > 0) {
-    SCN_TRY(device_alloc((void **)&slot_of, sizeof(int) * (size_t)n_ids, stream));
+    SCN_TRY(tmp.get(&slot_of, sizeof(int) * (size_t)n_ids));
     const unsigned tiles = (unsigned)ceil_div(n_ids, kRankTile);
-    SCN_TRY(device_alloc((void **)&words, sizeof(uint2) * (kRankTile / 32) * (size_t)tiles, stream));
-    SCN_TRY(device_alloc((void **)&base, sizeof(int) * (size_t)tiles, stream));
+    SCN_TRY(tmp.get(&words, sizeof(uint2) * (kRankTile / 32) * (size_t)tiles));
+    SCN_TRY(tmp.get(&base, sizeof(int) * (size_t)tiles));
     unsigned blocks = (unsigned)ceil_div(n_ids, threads);
     long long expect = n_in;
     for (int attempt = 0;; ++attempt) {
@@ -1255,15 +1257,7 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
         expect *= 4;
         continue;
       }
-      int st = flags_to_status(flags);
-      if (st != SCN_OK) {
-        device_free(slot_of, stream);
-        device_free(words, stream);
-        device_free(base, stream);
-        free_grid(gout, stream);
-        md->strided_rules.erase(key);
-        return st;
-      }
+      SCN_TRY(flags_to_status(flags));
       n_out = ((const volatile int *)md->mailbox)[2];
       break;
     }
@@ -1294,12 +1288,37 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
     SCN_LAUNCH_DIM(md->dim, k_strided_fill, std::min(blocks, 148u * 8u), threads, 0, stream, gin->layout, gout.layout, F, gout.table.slots, gin->row_keys, slot_of, n_in, nullptr, n_out, nullptr, n_out, words, base, gout.row_keys, rb.nbr, rb.counts_dev, (int)K, ticket_dev(rb));
     SCN_CUDA_CHECK(cudaGetLastError());
   }
-  device_free(slot_of, stream);
-  device_free(words, stream);
-  device_free(base, stream);
-  md->grids[okey] = gout;
   rb.built = true;
   g_rulebook_builds.fetch_add(1);
+  return SCN_OK;
+}
+
+int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int64_t *output_size,
+                         const int64_t *filter_size, const int64_t *filter_stride,
+                         cudaStream_t stream, Rulebook **out) {
+  SCN_TRY(md_touch(md, stream));
+  auto key = make_key(md->dim, input_size, filter_size, filter_stride);
+  auto have = md->strided_rules.find(key);
+  if (have == md->strided_rules.end() && md->pending) {  // it may be one of a chain that was started on the side stream
+    SCN_TRY(chain_finalize(md, stream, nullptr));
+    have = md->strided_rules.find(key);
+  }
+  if (have != md->strided_rules.end()) {
+    *out = &have->second;
+    return SCN_OK;
+  }
+  Grid *gin = find_grid_now(md, input_size);
+  SCN_REQUIRE(gin, SCN_ERR_NO_GRID, "strided rulebook: no grid for the input spatial size");
+  Grid gout;
+  Rulebook rb;
+  const int st = build_strided(md, gin, output_size, filter_size, filter_stride, stream, gout, rb);
+  if (st != SCN_OK) {
+    free_grid(gout, stream);
+    free_rulebook(rb, stream);
+    return st;
+  }
+  md->grids[make_key(md->dim, output_size)] = gout;
+  *out = &(md->strided_rules[key] = rb);
   return SCN_OK;
 }
 

@@ -883,14 +883,13 @@ int scn_batchnorm_backward(const float *in_features, float *d_in_features, const
   const long long chunk_rows = ceil_div(n_rows, chunks);
   double *partial = nullptr;
   float *coef = nullptr;
-  SCN_TRY(device_alloc((void **)&partial, sizeof(double) * 2 * (size_t)chunks * n_planes, stream));
-  SCN_TRY(device_alloc((void **)&coef, sizeof(float) * 2 * (size_t)n_planes, stream));
+  Scratch tmp(stream);
+  SCN_TRY(tmp.get(&partial, sizeof(double) * 2 * (size_t)chunks * n_planes));
+  SCN_TRY(tmp.get(&coef, sizeof(float) * 2 * (size_t)n_planes));
   launch_bn_back_sums(in_features, out_features, d_out_features, n_rows, n_planes, in_stride, out_stride, save_mean, (float)leakiness, chunks, chunk_rows, partial, stream);
   SCN_LAUNCH(k_bn_back_finalize, (unsigned)ceil_div(n_planes, 8), 256, 0, stream, partial, chunks, n_planes, n_rows, save_invstd, d_weight, d_bias, coef);
   launch_bn_back_apply(in_features, d_in_features, out_features, d_out_features, n_rows, n_planes, in_stride, out_stride, save_mean, save_invstd, weight, coef, (float)leakiness, stream);
   SCN_CUDA_CHECK(cudaGetLastError());
-  SCN_TRY(device_free(partial, stream));
-  SCN_TRY(device_free(coef, stream));
   return SCN_OK;
 }
 

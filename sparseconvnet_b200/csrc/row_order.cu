@@ -389,21 +389,6 @@ int key_bits(const Rulebook &rb, int K, long long n, unsigned long long *bit) {
   return bits;
 }
 
-struct Scratch {  // freed on every way out
-  void *p[8] = {nullptr};
-  int n = 0;
-  cudaStream_t stream;
-  explicit Scratch(cudaStream_t s) : stream(s) {}
-  ~Scratch() {
-    for (int i = 0; i < n; ++i) device_free(p[i], stream);
-  }
-  int get(void **q, size_t bytes) {
-    SCN_TRY(device_alloc(q, bytes, stream));
-    p[n++] = *q;
-    return SCN_OK;
-  }
-};
-
 template <typename KEY, int WORDS>
 int build(const int *table, const unsigned *known, long long n, int K, const unsigned long long *bit, int bits, RowOrder &ord, cudaStream_t stream) {
   Scratch tmp(stream);
@@ -417,13 +402,13 @@ int build(const int *table, const unsigned *known, long long n, int K, const uns
   const int blocks = (int)ceil_div(n, rpb);
   KeyBits<KEY> B{};
   for (int k = 0; k < K; ++k) B.bit[k] = (KEY)bit[k];
-  if (!known) SCN_TRY(tmp.get((void **)&masks, sizeof(unsigned) * WORDS * (size_t)n));
-  SCN_TRY(tmp.get((void **)&keys[0], sizeof(KEY) * (size_t)n));
-  SCN_TRY(tmp.get((void **)&counts, sizeof(int) * (size_t)blocks * R));
-  SCN_TRY(tmp.get((void **)&totals, sizeof(int) * ((size_t)passes * R + 1)));  // and the blocks that have packed their tiles
+  if (!known) SCN_TRY(tmp.get(&masks, sizeof(unsigned) * WORDS * (size_t)n));
+  SCN_TRY(tmp.get(&keys[0], sizeof(KEY) * (size_t)n));
+  SCN_TRY(tmp.get(&counts, sizeof(int) * (size_t)blocks * R));
+  SCN_TRY(tmp.get(&totals, sizeof(int) * ((size_t)passes * R + 1)));  // and the blocks that have packed their tiles
   if (passes > 1) {
-    SCN_TRY(tmp.get((void **)&keys[1], sizeof(KEY) * (size_t)n));
-    SCN_TRY(tmp.get((void **)&rows, sizeof(int) * (size_t)n));
+    SCN_TRY(tmp.get(&keys[1], sizeof(KEY) * (size_t)n));
+    SCN_TRY(tmp.get(&rows, sizeof(int) * (size_t)n));
   }
   SCN_CUDA_CHECK(cudaMemsetAsync(totals, 0, sizeof(int) * ((size_t)passes * R + 1), stream));
   if (ord.n_tiles > 148 && ord.n_tiles < 65536) SCN_TRY(device_alloc((void **)&ord.by_work, sizeof(int) * (size_t)ord.n_tiles, stream));

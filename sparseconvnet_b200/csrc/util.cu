@@ -129,8 +129,16 @@ int release_idle(DeviceCache &c, size_t keep) {
 }
 }  // namespace
 
+// scn_test_fail_allocation: does the allocation that is being asked for fail?
+static thread_local int g_fail_in = 0;
+int test_allocation() {
+  SCN_REQUIRE(!g_fail_in || --g_fail_in, SCN_ERR_CUDA, "out of memory (asked for by scn_test_fail_allocation)");
+  return SCN_OK;
+}
+
 int device_alloc(void **p, size_t bytes, cudaStream_t stream) {
   *p = nullptr;
+  SCN_TRY(test_allocation());
   DeviceCache *c = nullptr;
   SCN_TRY(device_cache(&c));
   unsigned long long id = 0;
@@ -302,6 +310,11 @@ int scn_memory_usage(uint64_t *reserved_bytes, uint64_t *used_bytes) {
     *reserved_bytes = r;
     *used_bytes = c->used;
   }
+  return SCN_OK;
+}
+
+int scn_test_fail_allocation(int which) {
+  scn::g_fail_in = which > 0 ? which : 0;
   return SCN_OK;
 }
 

@@ -53,3 +53,70 @@ def test_captured_convolution(n, precision, cuda):
             del graph
     finally:
         scn.set_precision("fp32")
+
+
+def _used():
+    import ctypes as C
+    from sparseconvnet_b200._lib import check, lib
+    reserved, used = C.c_uint64(), C.c_uint64()
+    check(lib.scn_memory_usage(C.byref(reserved), C.byref(used)))
+    return reserved.value, used.value
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32x3"])
+@pytest.mark.parametrize("n,coords", [(3000, "cpu"), (3000, "cuda"), (300, "cpu")])
+def test_nothing_is_lost_when_memory_runs_out(n, coords, precision, cuda):
+    """Input layer, rulebooks, row order, forward and backward pass with the first, second, ... allocation failing: an error
+    each time, every block given back with the object, and the next pass gives what an undisturbed one does."""
+    import sparseconvnet_b200 as scn
+    from sparseconvnet_b200 import SCN
+    from sparseconvnet_b200._lib import ScnError, lib
+    torch.manual_seed(n)
+    pts = _surface(n, 48).to(coords)
+    feats = torch.randn(n, 32, device=cuda)
+    size, half, three, two = torch.LongTensor([48] * 3), torch.LongTensor([24] * 3), torch.LongTensor([3] * 3), torch.LongTensor([2] * 3)
+    w = [torch.randn(27, 1, 32, 64, device=cuda), torch.randn(8, 1, 64, 40, device=cuda)]
+    none = torch.empty(0)
+
+    def run():
+        m = SCN.Metadata_3()
+        try:
+            x = SCN.InputLayer_updateOutput(m, size, pts, feats, None, 0, 3)
+            y, z = (feats.new_empty(0) for _ in range(2))
+            SCN.SubmanifoldConvolution_updateOutput(size, three, m, x, y, w[0], none)
+            SCN.Convolution_updateOutput(size, half, two, two, m, y, z, w[1], none)
+            g = [torch.empty_like(t) for t in (w[0], w[1], x, y)]
+            SCN.Convolution_backward(size, half, two, two, m, y, g[3], torch.ones_like(z), w[1], g[1], None)
+            SCN.SubmanifoldConvolution_backward(size, three, m, x, g[2], g[3], w[0], g[0], None)
+            mean, var, d_b = (torch.empty(64, device=cuda) for _ in range(3))
+            out, d_in = torch.empty_like(y), torch.empty_like(y)
+            SCN.BatchNormalization_updateOutput(y, out, mean, var, torch.zeros(64, device=cuda), torch.ones(64, device=cuda),
+                                                none, none, 1e-4, 0.9, True, 0.0)
+            SCN.BatchNormalization_backward(y, d_in, out, g[3], mean, var, None, None, none, none, None, d_b, 0.0)
+            return [x, y, z] + g
+        finally:
+            lib.scn_test_fail_allocation(0)
+            del m
+
+    try:
+        scn.set_precision(precision)
+        scn.set_backward_precision(precision)
+        want = run()
+        torch.cuda.synchronize()
+        before = _used()[1]
+        failed = 0
+        for which in range(1, 200):
+            lib.scn_test_fail_allocation(which)
+            try:
+                run()
+                break
+            except ScnError as e:
+                assert "out of memory" in str(e), e
+                failed += 1
+            assert _used()[1] == before, (which, _used()[1] - before)
+        assert failed > 15 and which > failed
+        assert all(torch.equal(a, b) for a, b in zip(run(), want))
+        assert _used()[1] == before
+    finally:
+        scn.set_precision("fp32")
+        scn.set_backward_precision("fp32")
