@@ -39,7 +39,7 @@ void set_error(const char *fmt, ...) {
 //     an idle block that a graph has been recorded with would be handed out again and written by every replay.
 //   * Idle blocks are bounded by an eighth of the device's memory; what comes back beyond that goes to the pool, and
 //     the pool returns it to the driver (release threshold 64 MB).  A failing allocation first gives back every idle
-//     block, and so does scn_trim_memory.
+//     block, and so does scn_trim_memory; if the rounded size still does not fit, the size itself is tried.
 namespace {
 constexpr int kSteps = 4 * 40;
 int size_step(size_t bytes) {  // the smallest step that holds `bytes`
@@ -55,8 +55,8 @@ struct DeviceCache {
   cudaMemPool_t pool = nullptr;
   size_t idle = 0, used = 0, idle_limit = 0;
   struct Block {
-    int step;
-    bool cached;  // goes to the idle list (no: to the pool)
+    size_t bytes;
+    int step;  // -1: goes back to the pool, not to the idle lists
   };
   std::unordered_map<void *, Block> live;
   std::unordered_map<unsigned long long, std::array<std::vector<void *>, kSteps>> idle_blocks;  // per stream id
@@ -159,16 +159,22 @@ int device_alloc(void **p, size_t bytes, cudaStream_t stream) {
       return SCN_OK;
     }
   SCN_TRY(make_pool(*c));
-  cudaError_t e = cudaMallocFromPoolAsync(p, step_bytes(step), c->pool, stream);
+  DeviceCache::Block block{step_bytes(step), capture ? -1 : step};
+  cudaError_t e = cudaMallocFromPoolAsync(p, block.bytes, c->pool, stream);
   if (e == cudaErrorMemoryAllocation && !capture) {
     cudaGetLastError();
     SCN_TRY(release_idle(*c, 0));
     SCN_CUDA_CHECK(cudaMemPoolTrimTo(c->pool, 0));
-    e = cudaMallocFromPoolAsync(p, step_bytes(step), c->pool, stream);
+    e = cudaMallocFromPoolAsync(p, block.bytes, c->pool, stream);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      block = {bytes ? bytes : 1, -1};
+      e = cudaMallocFromPoolAsync(p, block.bytes, c->pool, stream);
+    }
   }
   SCN_CUDA_CHECK(e);
-  c->live[*p] = {step, !capture};
-  c->used += step_bytes(step);
+  c->live[*p] = block;
+  c->used += block.bytes;
   return SCN_OK;
 }
 
@@ -182,11 +188,11 @@ int device_free(void *p, cudaStream_t stream) {
   std::lock_guard<std::mutex> lock(c->mu);
   auto it = c->live.find(p);
   SCN_REQUIRE(it != c->live.end(), SCN_ERR_BAD_ARG, "freed memory is not a block of the current device");
-  const size_t bytes = step_bytes(it->second.step);
+  const size_t bytes = it->second.bytes;
   // (nobody may write it any more, the graph reads it at every replay: it stays taken)
-  SCN_REQUIRE(!it->second.cached || !capture, SCN_ERR_UNSUPPORTED, "memory taken before a stream capture cannot be given back inside it");
+  SCN_REQUIRE(it->second.step < 0 || !capture, SCN_ERR_UNSUPPORTED, "memory taken before a stream capture cannot be given back inside it");
   c->used -= bytes;
-  if (!it->second.cached || c->idle + bytes > c->idle_limit) {
+  if (it->second.step < 0 || c->idle + bytes > c->idle_limit) {
     c->live.erase(it);
     SCN_CUDA_CHECK(cudaFreeAsync(p, stream));
     return SCN_OK;
