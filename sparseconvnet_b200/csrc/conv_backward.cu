@@ -113,11 +113,11 @@ k_conv_dweight(const float *__restrict__ in, int ld_in, long long n_in_rows, con
     }
 }
 
-// out[i] = sum over chunks, in order, of partial[chunk][i]
-__global__ void k_sum_chunks(const float *__restrict__ partial, int chunks, long long n, float *__restrict__ out) {
+// out[i] = sum over chunks, in order, of partial[chunk][i]; `add`: behind what is there already
+__global__ void k_sum_chunks(const float *__restrict__ partial, int chunks, long long n, float *__restrict__ out, bool add) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float acc = 0.f;
+  float acc = add ? out[i] : 0.f;
   int c = 0;
   for (; c + 8 <= chunks; c += 8) {  // eight loads on their way
     float v[8];
@@ -381,7 +381,7 @@ static int launch_dweight(const float *in, int ld_in, long long n_in_rows, const
   const int vec_out = cout % 4 == 0 && ld_out % 4 == 0 && (uintptr_t)dout % 16 == 0;
   SCN_LAUNCH((k_conv_dweight_mma<WM, WN, MT>), dim3((unsigned)grid_x, (unsigned)K, (unsigned)tiles), S::THREADS, S::SMEM, stream, in, ld_in, n_in_rows, dout, ld_out, n_out_rows, nbr, n_entries, swap, cin, cout, vec_in, vec_out, chunk_rows, partial, flags);
   if (grid_x > 1)
-    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, grid_x, w_elems, d_weight);
+    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, grid_x, w_elems, d_weight, false);
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }
@@ -476,7 +476,7 @@ static int dweight_thin(const float *in, long long rows_in, const float *d_out, 
   const auto kernel = cin == 1 ? k_conv_dweight_thin<1> : cin == 2 ? k_conv_dweight_thin<2> : k_conv_dweight_thin<3>;
   SCN_LAUNCH(kernel, dim3((unsigned)chunks, (unsigned)columns), 256, 0, stream, in, rows_in, d_out, rows_out, nbr, K, cout, chunk_rows, partial, flags);
   if (chunks > 1)
-    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, chunks, w_elems, d_weight);
+    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, chunks, w_elems, d_weight, false);
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }
@@ -545,7 +545,7 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
     float *partial = nullptr;
     SCN_TRY(tmp.get(&partial, sizeof(float) * (size_t)chunks * n_out_planes));
     SCN_LAUNCH(k_column_sums, dim3((unsigned)ceil_div(n_out_planes, 32), (unsigned)chunks), 256, 0, stream, d_out, rows_out, n_out_planes, chunk_rows, partial);
-    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(n_out_planes, 256), 256, 0, stream, partial, chunks, (long long)n_out_planes, d_bias);
+    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(n_out_planes, 256), 256, 0, stream, partial, chunks, (long long)n_out_planes, d_bias, false);
     SCN_CUDA_CHECK(cudaGetLastError());
   }
 
@@ -575,7 +575,7 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
       SCN_TRY(tmp.get(&partial, sizeof(float) * (size_t)chunks * w_elems));
       const int tiles = groups * (int)ceil_div(cin, 32) * (int)ceil_div(cout, 32);
       SCN_LAUNCH(k_conv_dweight, dim3((unsigned)chunks, (unsigned)K, (unsigned)tiles), 256, 0, stream, in, n_in_planes, rows_in, d_out, n_out_planes, rows_out, rb.nbr, n_entries, transposed ? 1 : 0, cin, cout, groups, chunk_rows, partial, md->flags_dev);
-      SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, chunks, w_elems, d_weight);
+      SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, partial, chunks, w_elems, d_weight, false);
       SCN_CUDA_CHECK(cudaGetLastError());
     }
   }
@@ -651,10 +651,10 @@ int scn_rows_affine_backward(const float *in_features, const float *d_out_featur
   SCN_TRY(tmp.get(&partial, sizeof(float) * (size_t)grid_x * (size_t)(w_elems + n_out_planes)));
   float *bias_partial = partial + (size_t)grid_x * w_elems;
   SCN_LAUNCH(k_conv_dweight, dim3((unsigned)grid_x, 1, (unsigned)tiles), 256, 0, stream, in_features, n_in_planes, (long long)n_rows, d_out_features, n_out_planes, (long long)n_rows, nullptr, (long long)n_rows, 0, n_in_planes, n_out_planes, 1, chunk_rows, partial, nullptr);
-  SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 32), 32, 0, stream, partial, grid_x, w_elems, d_weight);
+  SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 32), 32, 0, stream, partial, grid_x, w_elems, d_weight, false);
   if (d_bias) {
     SCN_LAUNCH(k_column_sums, dim3((unsigned)ceil_div(n_out_planes, 32), (unsigned)grid_x), 256, 0, stream, d_out_features, (long long)n_rows, n_out_planes, chunk_rows, bias_partial);
-    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(n_out_planes, 32), 32, 0, stream, bias_partial, grid_x, (long long)n_out_planes, d_bias);
+    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(n_out_planes, 32), 32, 0, stream, bias_partial, grid_x, (long long)n_out_planes, d_bias, false);
   }
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;

@@ -11,11 +11,13 @@
 //               l l (2^-24 of a product) is summed in fp32.  The parts of T are lanes of one accumulator (M = 128: h and m of 64 planes, or h, m and l of 32),
 //               those of G its columns, and the blocks are added when the sums are done; the products with an l go where
 //               those with an m go.  The tensor core truncates its running sum at every instruction, half a unit of 2^-24 on
-//               average: a CTA takes at most kMaxTiles tiles, 8 instructions each, before its sums are added in fp32.
+//               average: a CTA takes at most kMaxTiles tiles, 8 instructions each for the sums of h h (up to 24 for the
+//               others, which are 2^-8 as large), before its sums are added in fp32.
 //   split       The accumulators of a CTA stay in TMEM from its first rule to its last: 5 filter offsets x 96 columns (32
 //               gathered planes) or 4 x 128 (64).  A CTA is one such group of offsets, one pair of plane blocks and every
 //               n_chunks-th tile; the chunks' sums are added in order (k_sum_chunks), so the result does not depend on
-//               timing.
+//               timing.  The partial sums of a launch take at most kMostPartial bytes; a layer with more chunks than fit
+//               is done in several launches, each adding to the sum of those before.
 //   jobs        One thread walks the tiles: a job is the T rows of a tile or the G rows of one of its offsets, a slot of a
 //               ring with the 128 row numbers (a 512-byte bulk copy) and what they are for.
 //   staging     8 warps copy rows of the split matrices (k_dweight_split, once per call) with 16-byte cp.async straight into
@@ -37,7 +39,7 @@
 
 namespace scn {
 
-__global__ void k_sum_chunks(const float *__restrict__ partial, int chunks, long long n, float *__restrict__ out);
+__global__ void k_sum_chunks(const float *__restrict__ partial, int chunks, long long n, float *__restrict__ out, bool add);
 
 namespace {
 
@@ -47,6 +49,7 @@ constexpr int kMma = kLoadWarps, kJobs = kLoadWarps + 1;
 constexpr int kThreads = (kLoadWarps + 2) * 32;
 constexpr int kSlots = 8;           // jobs ahead
 constexpr int kMaxTiles = 48;       // tiles of a CTA
+constexpr long long kMostPartial = 256ll << 20;
 constexpr int kAtom = kRows * 128;  // 128 rules x 64 elements
 
 template <int PT, int PG>
@@ -71,12 +74,12 @@ struct DwParams {
   long long n_t, n_g;
   const int *order, *packed, *by_work;
   const unsigned *tile_bits;
-  int words, K, n_groups, n_chunks, blocks_g;
+  int words, K, n_groups, n_chunks, first_chunk, blocks_g;  // (first_chunk: of the launch)
   unsigned group_bits[32][4];  // the offsets of a group, ascending, are the bits of its mask
   long long n_tiles;
   int t_is_out;    // T is d_out (else `in`, the operator ran the table backwards)
   int cin, cout;
-  float *partial;  // [n_chunks][K][cin][cout]
+  float *partial;  // [chunks of the launch][K][cin][cout]
   int *flags;
 };
 
@@ -172,7 +175,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ Ctl C;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int group = blockIdx.x, chunk = blockIdx.y, pair = blockIdx.z;
+  const int group = blockIdx.x, chunk = P.first_chunk + blockIdx.y, pair = blockIdx.z;
   const int t0 = pair / P.blocks_g * PT, g0 = pair % P.blocks_g * PG;  // first planes of the pair
   const int n_off = __popc(P.group_bits[group][0]) + __popc(P.group_bits[group][1]) + __popc(P.group_bits[group][2]) +
                     __popc(P.group_bits[group][3]);
@@ -431,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
         tc_fence_before();
       }
       __syncthreads();
-      float *out = P.partial + ((long long)chunk * P.K + k) * P.cin * P.cout;
+      float *out = P.partial + ((long long)blockIdx.y * P.K + k) * P.cin * P.cout;
       for (int i = tid; i < PT * PG; i += kThreads) {
         const int tp = P.t_is_out ? i % PT : i / PG, gp = P.t_is_out ? i / PT : i % PG;
         if (t0 + tp >= P.t_planes || g0 + gp >= P.g_planes) continue;
@@ -495,7 +498,8 @@ int launch(DwParams &P, const Rulebook &rb, const float *t_rows, const float *g_
   const long long w_elems = (long long)P.K * P.cin * P.cout;
   Scratch tmp(stream);
   P.partial = d_weight;
-  if (P.n_chunks > 1) SCN_TRY(tmp.get(&P.partial, sizeof(float) * (size_t)P.n_chunks * w_elems));
+  const int at_once = (int)std::min<long long>(P.n_chunks, std::max<long long>(per_wave, kMostPartial / ((long long)sizeof(float) * w_elems)));
+  if (P.n_chunks > 1) SCN_TRY(tmp.get(&P.partial, sizeof(float) * (size_t)at_once * w_elems));
   unsigned char *split = nullptr;
   const int t_per = (int)ceil_div(P.t_planes, PT) * PT / 8, g_per = (int)ceil_div(P.g_planes, PG) * PG / 8;
   const size_t t_size = (size_t)(P.n_t * split_row_bytes(t_per, PT)), g_size = (size_t)(P.n_g * split_row_bytes(g_per, PG));
@@ -504,9 +508,12 @@ int launch(DwParams &P, const Rulebook &rb, const float *t_rows, const float *g_
   P.g_rows = split + t_size;
   SCN_LAUNCH(k_dweight_split, (unsigned)ceil_div(P.n_t * t_per, 256), 256, 0, stream, t_rows, split, P.n_t * t_per, P.t_planes, t_per, PT);
   SCN_LAUNCH(k_dweight_split, (unsigned)ceil_div(P.n_g * g_per, 256), 256, 0, stream, g_rows, split + t_size, P.n_g * g_per, P.g_planes, g_per, PG);
-  SCN_LAUNCH((k_dweight_tile<PT, PG>), dim3((unsigned)P.n_groups, (unsigned)P.n_chunks, (unsigned)pairs), kThreads, S::SMEM, stream, P);
-  if (P.n_chunks > 1)
-    SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, P.partial, P.n_chunks, w_elems, d_weight);
+  for (; P.first_chunk < P.n_chunks; P.first_chunk += at_once) {
+    const int here = std::min(at_once, P.n_chunks - P.first_chunk);
+    SCN_LAUNCH((k_dweight_tile<PT, PG>), dim3((unsigned)P.n_groups, (unsigned)here, (unsigned)pairs), kThreads, S::SMEM, stream, P);
+    if (P.n_chunks > 1)
+      SCN_LAUNCH(k_sum_chunks, (unsigned)ceil_div(w_elems, 256), 256, 0, stream, P.partial, here, w_elems, d_weight, P.first_chunk > 0);
+  }
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }

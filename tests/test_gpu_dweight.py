@@ -1,7 +1,8 @@
 """Weight gradients of the convolutions (k_conv_dweight_mma, k_dweight_tile) against a float64 product over the exported rulebook.
 
 Shapes of more than 32 planes on one side run on k_dweight_tile from 2048 rows, with blocks of 32 or 64 planes per side;
-its six bf16 products drop 2^-24 of a product and its running sums lose at most 2^-24 per instruction, 1 152 of them.
+its six bf16 products drop 2^-24 of a product and its running sums lose at most 2^-24 per instruction: 384 of them in the sums
+of the large parts, 1 152 in those of the others, which are 2^-8 as large.
 
 Tolerance: three tf32 products of the hi / lo split drop lo x lo and the low bits of lo, 2^-21 of a product, and n fp32
 additions of random sign add 2^-24 sqrt(n) of the running sum: below 1e-5 of the largest entry for the row counts here;
@@ -144,12 +145,14 @@ def test_thin_weight_gradient(n, size, cin, cout, cuda):
     test_weight_gradient(n, size, cin, cout, cuda)
 
 
-@pytest.mark.parametrize("cin,cout", [(8, 16), (24, 24), (32, 32), (48, 48), (80, 36), (100, 160)])
+@pytest.mark.parametrize("cin,cout", [(8, 16), (24, 24), (32, 32), (48, 48), (80, 36), (100, 160), (64, 64), (64, 96)])
 @pytest.mark.parametrize("n,size", [(6000, 40), (60000, 120)])
 def test_weight_gradient_is_as_accurate_as_fp32_sums(n, size, cin, cout, cuda):
     """Products of one sign, where everything that is cut off instead of rounded adds up.  Rounded to nearest, the two tf32
     parts of an operand leave out at most 2^-23 of it and lo x lo 2^-22 of a product, of either sign, and n fp32 additions
-    2^-24 sqrt(n) / 2 of the sum: below 5e-7 for the 3 k rules of an entry and chunk here.  (Parts cut off: 4e-6 to 8e-6.)"""
+    2^-24 sqrt(n) / 2 of the sum: below 5e-7 for the 3 k rules of an entry and chunk here.  (Parts cut off: 4e-6 to 8e-6.)
+    On k_dweight_tile (multiples of 32 planes, more than 32 on a side) up to 384 instructions each cut 2^-24 of a running sum
+    that is half of the last one on average: 1.2e-5."""
     import sparseconvnet_b200 as scn
     torch.manual_seed(cin)
     pts = torch.randint(0, size, (n, 3))
@@ -163,4 +166,4 @@ def test_weight_gradient_is_as_accurate_as_fp32_sums(n, size, cin, cout, cuda):
     want = torch.stack([f[r[:, 0].long()].double().t() @ g[r[:, 1].long()].double()
                         for r in x.metadata.rulebook(0, x.spatial_size, [3, 3, 3])])
     e = float((layer.weight.grad[:, 0] - want).norm() / want.norm())
-    assert e <= 5e-7, e
+    assert e <= (1.2e-5 if cin % 32 == 0 and cout > 32 and cout % 32 == 0 else 5e-7), e

@@ -120,3 +120,37 @@ def test_nothing_is_lost_when_memory_runs_out(n, coords, precision, cuda):
     finally:
         scn.set_precision("fp32")
         scn.set_backward_precision("fp32")
+
+
+def test_weight_gradient_scratch_is_bounded(cuda):
+    """125 offsets of 256 x 256 weights are 33 MB per chunk of tiles: 25 chunks of 48 tiles, of which at most 256 MB at a
+    time; the gradient is the sum of all of them."""
+    import sparseconvnet_b200 as scn
+    from sparseconvnet_b200 import SCN
+    from sparseconvnet_b200._lib import check, lib
+    torch.manual_seed(3)
+    n, planes = 150000, 256
+    cell = torch.randperm(96 ** 3, device=cuda)[:n]
+    pts = torch.stack([cell // 96 ** 2, cell // 96 % 96, cell % 96], 1)
+    x = scn.InputLayer(3, 96, mode=0)([pts, torch.zeros(n, 1, device=cuda)])
+    w, dw = torch.randn(125, 1, planes, planes, device=cuda), torch.empty(125, 1, planes, planes, device=cuda)
+    f, g = torch.randn(n, planes, device=cuda), torch.randn(n, planes, device=cuda)
+    five = torch.LongTensor([5] * 3)
+
+    def backward(f, g, w, dw):
+        SCN.SubmanifoldConvolution_backward(x.spatial_size, five, x.metadata, f, None, g, w, dw, None)
+    backward(f[:, :64].contiguous(), g[:, :64].contiguous(), w[:, :, :64, :64].contiguous(),
+             torch.empty(125, 1, 64, 64, device=cuda))  # the rulebook and its row order
+    torch.cuda.synchronize()
+    check(lib.scn_trim_memory(0))
+    before = _used()[0]
+    backward(f, g, w, dw)
+    torch.cuda.synchronize()
+    rows = 2 * n * planes * 6      # both sides as three bf16 parts
+    assert _used()[0] - before <= 1.25 * (rows + (256 << 20)) + (64 << 20)
+    rules = x.metadata.rulebook(0, x.spatial_size, five)
+    for k in (0, 31, 62, 124):
+        r = rules[k].long()
+        want = f[r[:, 0]].double().t() @ g[r[:, 1]].double()
+        assert float((dw[k, 0] - want).norm() / want.norm()) <= 1e-5
+    x.metadata.poll_errors()
