@@ -180,11 +180,14 @@ def pooling(kind, features, metadata, in_size, out_size, pool_size, pool_stride,
 
 def rows_affine(features, weight, bias):
     """features @ weight (+ bias) of a NetworkInNetwork.  Its weight gradient is a tall and thin product (400 k rows,
-    32 x 20 weights) that torch's matrix product spends 405 us on; the library's takes 30."""
-    if features.nelement() == 0 or features.dim() != 2 or not features.is_cuda or features.dtype != torch.float32:
+    32 x 20 weights) that torch's matrix product spends 405 us on; the library's takes 30.  Wide layers and everything
+    but plain tensors are torch's own operators."""
+    out = SCN._binding.rows_affine_train(features, weight, bias)
+    if out is None:
         out = features @ weight
-        return out if bias is None else out + bias
-    return SCN._binding.rows_affine_train(features, weight, bias)
+        if bias is not None:
+            out = out + bias
+    return out
 
 
 class _SparseToDense(torch.autograd.Function):

@@ -167,3 +167,68 @@ def test_weight_gradient_is_as_accurate_as_fp32_sums(n, size, cin, cout, cuda):
                         for r in x.metadata.rulebook(0, x.spatial_size, [3, 3, 3])])
     e = float((layer.weight.grad[:, 0] - want).norm() / want.norm())
     assert e <= (1.2e-5 if cin % 32 == 0 and cout > 32 and cout % 32 == 0 else 5e-7), e
+
+
+def _affine(features, weight, bias):
+    """NetworkInNetwork's training path on these operands."""
+    from sparseconvnet_b200 import autograd
+    return autograd.rows_affine(features, weight, bias)
+
+
+def test_network_in_network_takes_what_a_matrix_product_takes(cuda):
+    """Operands that torch's product accepts or refuses, on the training path: a transposed weight, offset, strided and
+    double-precision features, a bias of one value, one of a wrong length, operands on the host."""
+    torch.manual_seed(0)
+    flat = torch.randn(1 + 600 * 32, device=cuda)
+    base = torch.randn(20, 32, device=cuda).t()
+    for f in (flat[1:].view(600, 32), flat[:600 * 32].view(32, 600).t(), flat[:600 * 32].view(600, 32).double()):
+        for bias in (None, torch.randn(1, device=cuda, dtype=f.dtype), torch.randn(20, device=cuda, dtype=f.dtype)):
+            w = base.to(f.dtype).detach().requires_grad_()
+            got = _affine(f, w, bias)
+            want = f.double() @ w.detach().double() + (bias.double() if bias is not None else 0)
+            assert got.dtype == f.dtype and float((got - want).abs().max()) < 1e-4
+            got.sum().backward()
+            assert float((w.grad - f.double().sum(0)[:, None]).abs().max()) < 1e-2
+    f, w = flat[:-1].view(600, 32), torch.randn(32, 20, device=cuda, requires_grad=True)
+    g = torch.randn(1 + 600 * 20, device=cuda)[1:].view(600, 20)   # an offset gradient
+    fr = f.clone().requires_grad_()
+    _affine(fr, w, None).backward(g)
+    assert float((fr.grad.double() - g.double() @ w.detach().double().t()).abs().max()) < 1e-4
+    for bad in ((f, w, torch.zeros(19, device=cuda)), (f, w, torch.zeros(20)), (f, w.detach().cpu().requires_grad_(), None),
+                (f, torch.randn(31, 20, device=cuda, requires_grad=True), None)):
+        with pytest.raises(RuntimeError):
+            _affine(*bad)
+
+
+def test_network_in_network_under_torchs_transforms(cuda):
+    """Second derivatives, forward mode, vmap, torch.func.grad, autocast and saved-tensor hooks see a matrix product."""
+    import torch.autograd.forward_ad as fwd
+    torch.manual_seed(1)
+    f = torch.randn(50, 12, device=cuda)
+    w, b = torch.randn(12, 8, device=cuda, requires_grad=True), torch.randn(8, device=cuda, requires_grad=True)
+
+    def plain(f, w, b):
+        return f @ w + b
+
+    for view in (lambda t: t, lambda t: t.t().contiguous().t()):   # contiguous and strided rows
+        second = []
+        for op in (_affine, plain):
+            x = f.clone().requires_grad_()
+            y = op(view(x * x), w, b)
+            (gx,) = torch.autograd.grad((y ** 3).sum(), x, create_graph=True)
+            second.append(torch.autograd.grad((gx ** 2).sum(), (x, w)))
+        assert all(torch.allclose(p, q, rtol=1e-3, atol=1e-2 * float(q.abs().max())) for p, q in zip(*second))
+    with fwd.dual_level():
+        t = torch.randn_like(f)
+        out = fwd.unpack_dual(_affine(fwd.make_dual(f, t), w, b))
+        assert out.tangent is not None and torch.allclose(out.tangent, t @ w, atol=1e-4)
+    grad = torch.func.grad(lambda f: _affine(f, w, b).pow(2).sum())(f)
+    assert torch.allclose(grad, 2 * plain(f, w, b) @ w.t(), atol=1e-3)
+    batched = torch.func.vmap(lambda f: _affine(f, w, b))(torch.stack([f, 2 * f]))
+    assert torch.allclose(batched[1], plain(2 * f, w, b), atol=1e-4)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert _affine(f, w, None).dtype == (f @ w).dtype
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append(t) or t, lambda t: t):
+        _affine(f.clone().requires_grad_(), w, b)
+    assert len(seen) == 2
