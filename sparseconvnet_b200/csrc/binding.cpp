@@ -707,6 +707,17 @@ struct PoolingNode : ag::Node {
   }
 };
 
+bool has_tangent(const at::Tensor &t) { return t.defined() && t._fw_grad(0).defined(); }
+
+// Forward-mode differentiation has no rule here, as a Python Function without jvp has none; a tangent must not get lost.
+template <typename... T>
+void no_tangents(const T &...t) {
+  if ((has_tangent(t) || ...)) {
+    PyErr_SetString(PyExc_NotImplementedError, "this operator has no forward-mode derivative");
+    throw Fail{};
+  }
+}
+
 at::Tensor contiguous_features(PyObject *o) {
   const at::Tensor &t = tensor(o, "input_features");
   if (!t.is_cuda()) fail("input_features must be a CUDA tensor: sparseconvnet_b200 has no CPU path");
@@ -724,6 +735,7 @@ SCN_FN(convolution_train) {
   at::Tensor f, out;
   double macs = 0;
   const Weight w(a[8], given);
+  no_tangents(given, w.w, bias_t);
   {
     const at::NoGradGuard no_grad;
     f = contiguous_features(a[7]);
@@ -779,6 +791,7 @@ SCN_FN(batchnorm_train) {
   const double eps = PyFloat_AsDouble(a[5]), momentum = PyFloat_AsDouble(a[6]), leak = PyFloat_AsDouble(a[8]);
   const int train = PyObject_IsTrue(a[7]);
   if (PyErr_Occurred()) throw Fail{};
+  no_tangents(given, weight_t, bias_t);
   at::Tensor f, out, mean, invstd;
   {
     const at::NoGradGuard no_grad;
@@ -807,8 +820,6 @@ SCN_FN(batchnorm_train) {
   return THPVariable_Wrap(std::move(out));
   SCN_END
 }
-
-bool has_tangent(const at::Tensor &t) { return t.defined() && t._fw_grad(0).defined(); }
 
 // rows @ weight (+ bias): the product on the library's kernel for narrow results, on torch's matrix product otherwise
 bool rows_affine_takes(const at::Tensor &rows, int64_t nin, int64_t nout) {
@@ -918,6 +929,7 @@ SCN_FN(pooling_train) {
   scn_metadata *md = md_of(a[2]);
   const Sizes in_size(a[3]), out_size(a[4]), pool(a[5]), stride(a[6]);
   const at::Tensor &given = tensor(a[7], "input_features");
+  no_tangents(given);
   at::Tensor f, out;
   {
     const at::NoGradGuard no_grad;

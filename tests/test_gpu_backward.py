@@ -342,3 +342,20 @@ def test_unet_training_step_reduces_the_loss(cuda):
         losses.append(loss.item())
         opt.step()
     assert losses[-1] < losses[0], losses
+
+
+def test_forward_mode_is_refused(cuda):
+    """No operator of the training path has a forward-mode derivative: a tangent raises, as it did with Python Functions
+    without jvp, and is not dropped."""
+    import torch.autograd.forward_ad as fwd
+
+    import sparseconvnet_b200 as scn
+    x = scn.InputLayer(3, 16, mode=3)([torch.randint(0, 16, (200, 3)), torch.ones(200, 8, device=cuda)])
+    layers = [scn.SubmanifoldConvolution(3, 8, 8, 3, True), scn.Convolution(3, 8, 8, 2, 2, False), scn.BatchNormReLU(8),
+              scn.MaxPooling(3, 2, 2), scn.AveragePooling(3, 2, 2)]
+    for layer in layers:
+        layer.to(cuda)(x)
+        with fwd.dual_level():
+            f = fwd.make_dual(x.features.clone().requires_grad_(), torch.ones_like(x.features))
+            with pytest.raises(NotImplementedError):
+                layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size))
