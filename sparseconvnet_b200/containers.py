@@ -112,7 +112,7 @@ class Sequential(torch.nn.Sequential):
             if (Sequential.fuse and isinstance(m, layers._ConvBase) and isinstance(nxt, layers.BatchNormalization)
                     and not m._forward_hooks and not m._forward_pre_hooks
                     and input.features.nelement() > 0 and nxt.fusable(input.features)
-                    and not layers.autograd.needs_grad(input.features, m._parameters["weight"])):
+                    and not layers.autograd.needs_grad(input.features, layers.parameter(m, "weight"))):
                 if _wants_split(m, steps[i + 2] if i + 2 < n else None):
                     input = m.forward(input, bn=nxt, want_split=True)
                 else:
@@ -127,7 +127,7 @@ class Sequential(torch.nn.Sequential):
                     and not m._forward_hooks and not m._forward_pre_hooks and not nxt._forward_hooks
                     and not nxt._forward_pre_hooks and isinstance(input, SparseConvNetTensor)
                     and input.features.nelement() > 0 and m.fusable(input.features)
-                    and not layers.autograd.needs_grad(input.features, nxt._parameters["weight"], nxt._parameters.get("bias"))):
+                    and not layers.autograd.needs_grad(input.features, layers.parameter(nxt, "weight"), layers.parameter(nxt, "bias"))):
                 post = nxt2 if (isinstance(nxt2, layers.BatchNormalization) and nxt2.fusable(input.features)) else None
                 after = i + (3 if post is not None else 2)
                 input = nxt.forward(input, bn=post, pre_bn=m,
@@ -142,7 +142,7 @@ class Sequential(torch.nn.Sequential):
                     and not m._forward_hooks and not m._forward_pre_hooks and not nxt._forward_hooks
                     and not nxt._forward_pre_hooks and isinstance(input, SparseConvNetTensor)
                     and input.features.nelement() > 0 and input.features.size(1) == nxt.nIn and m.fusable(input.features)
-                    and not layers.autograd.needs_grad(input.features, nxt._parameters["weight"], nxt._parameters.get("bias"))):
+                    and not layers.autograd.needs_grad(input.features, layers.parameter(nxt, "weight"), layers.parameter(nxt, "bias"))):
                 post = nxt2 if (isinstance(nxt2, layers.BatchNormalization) and nxt2.fusable(input.features)) else None
                 after = i + (3 if post is not None else 2)
                 input = nxt.forward(input, bn=post, pre_bn=m,
@@ -158,7 +158,7 @@ class Sequential(torch.nn.Sequential):
                     and len(input) == 2 and all(t.features.nelement() > 0 and t.features.dim() == 2 for t in input)
                     and nxt.fusable(input[0].features) and nxt2.groups == 1
                     and not any(layers.autograd.needs_grad(t.features) for t in input)
-                    and not layers.autograd.needs_grad(input[0].features, nxt2._parameters["weight"], nxt2._parameters.get("bias"))):
+                    and not layers.autograd.needs_grad(input[0].features, layers.parameter(nxt2, "weight"), layers.parameter(nxt2, "bias"))):
                 nxt3 = steps[i + 3] if i + 3 < n else None
                 post = nxt3 if (isinstance(nxt3, layers.BatchNormalization) and nxt3.fusable(input[0].features)) else None
                 after = i + (4 if post is not None else 3)

@@ -161,6 +161,15 @@ class BLOutputLayer(Module):
         return "BLOutputLayer()"
 
 
+def parameter(module, name):
+    """A module's weight or bias, None if it has none: as registered (the quick way), or what a wrapper has put in the
+    parameter's place -- weight_norm, pruning and data-parallel replicas an attribute, a parametrization a property."""
+    t = module._parameters.get(name)
+    if t is None and (name in module.__dict__ or hasattr(type(module), name)):
+        t = getattr(module, name)
+    return t
+
+
 class _ConvBase(Module):
     def _init_weight(self, dimension, nIn, nOut, filter_size, bias, groups):
         self.dimension = dimension
@@ -180,9 +189,9 @@ class _ConvBase(Module):
     def _weight_token(self):
         """Token under which this layer's prepared weight images are kept by the library: renewed
         whenever the weight tensor is written (version counter) or moved (data pointer)."""
-        if not _ConvBase.cache_weight_images:
+        w = self._parameters.get("weight")
+        if w is None or not _ConvBase.cache_weight_images:  # (what a wrapper computes anew has no version to go by)
             return 0
-        w = self._parameters["weight"]
         key = (w.data_ptr(), w._version)
         if getattr(self, "_wkey", None) != key:
             old = getattr(self, "_wtoken", 0)
@@ -224,8 +233,8 @@ class SubmanifoldConvolution(_ConvBase):
         """`bn` / `pre_bn` (used by Sequential): eval-mode BatchNormalizations behind / in front of this layer that are
         applied in the convolution's store / in the pass that splits its rows, instead of as passes of their own.
         `want_split`: a convolution follows, which reads the result in split form."""
-        features, params = input.features, self._parameters
-        weight, bias = params["weight"], params.get("bias")
+        features = input.features
+        weight, bias = parameter(self, "weight"), parameter(self, "bias")
         assert features.nelement() == 0 or features.size(1) == self.nIn, (self.nIn, self.nOut, input)
         output = SparseConvNetTensor(metadata=input.metadata, spatial_size=input.spatial_size)
         if autograd.needs_grad(features, weight, bias):
@@ -257,15 +266,15 @@ class SubmanifoldConvolution(_ConvBase):
         if SCN.Profile.active is None and len(inputs) == 2:
             a, b = (i.features.detach().contiguous() for i in inputs)
             made = SCN._binding.submanifold_joined(
-                output.metadata.handle, output.spatial_size, self.filter_size, a, b, None, self._parameters["weight"],
-                self._parameters.get("bias"), pre_bn.folded() if pre_bn is not None else None,
+                output.metadata.handle, output.spatial_size, self.filter_size, a, b, None, parameter(self, "weight"),
+                parameter(self, "bias"), pre_bn.folded() if pre_bn is not None else None,
                 bn.folded() if bn is not None else None, SCN._precision, self._weight_token(), want_split)
             return None if made is None else self._run(lambda: made, output)
         output.features = inputs[0].features.new_empty(0)
         macs = SCN.SubmanifoldConvolution_joined(
             inputs[0].spatial_size, self.filter_size, inputs[0].metadata,
-            [i.features.detach().contiguous() for i in inputs], output.features, self._parameters["weight"],
-            self._parameters.get("bias"), prologue=pre_bn.folded() if pre_bn is not None else None,
+            [i.features.detach().contiguous() for i in inputs], output.features, parameter(self, "weight"),
+            parameter(self, "bias"), prologue=pre_bn.folded() if pre_bn is not None else None,
             epilogue=bn.folded() if bn is not None else None, token=self._weight_token())
         if macs is None:
             return None
@@ -299,8 +308,8 @@ class Convolution(_ConvBase):
         """`bn` / `pre_bn` (used by Sequential): eval-mode BatchNormalizations behind / in front of this layer that
         are applied inside the convolution call instead of as passes of their own.  `want_split` as in
         SubmanifoldConvolution."""
-        features, params = input.features, self._parameters
-        weight, bias = params["weight"], params.get("bias")
+        features = input.features
+        weight, bias = parameter(self, "weight"), parameter(self, "bias")
         assert features.nelement() == 0 or features.size(1) == self.nIn
         out_size = SCN._binding.strided_size(input.spatial_size, self.filter_size, self.filter_stride)
         assert out_size is not None, (input.spatial_size, self.filter_size, self.filter_stride)
@@ -344,8 +353,8 @@ class Deconvolution(_ConvBase):
         self.filter_stride = to_long_tensor(dimension, filter_stride)
 
     def forward(self, input, bn=None, want_split=False):
-        features, params = input.features, self._parameters
-        weight, bias = params["weight"], params.get("bias")
+        features = input.features
+        weight, bias = parameter(self, "weight"), parameter(self, "bias")
         assert features.nelement() == 0 or features.size(1) == self.nIn
         out_size = SCN._binding.transposed_size(input.spatial_size, self.filter_size, self.filter_stride)
         output = SparseConvNetTensor(metadata=input.metadata, spatial_size=out_size)
@@ -397,12 +406,13 @@ class BatchNormalization(Module):
         """(scale, shift, leakiness) of this layer in eval mode, for a convolution that applies it in its
         store.  Kept until a parameter or running statistic changes (tensor version counters)."""
         buffers, params = self._buffers, self._parameters
-        key = SCN._binding.versions(buffers["running_mean"], buffers["running_var"], params.get("weight"),
-                                    params.get("bias"))
+        weight, bias = parameter(self, "weight"), parameter(self, "bias")
+        if weight is not params.get("weight") or bias is not params.get("bias"):  # computed anew by a wrapper: nothing to go by
+            return SCN.batchnorm_fold(self.running_mean, self.running_var, weight, bias, self.eps) + (self.leakiness,)
+        key = SCN._binding.versions(buffers["running_mean"], buffers["running_var"], weight, bias)
         cached = self.__dict__.get("_folded")
         if cached is None or cached[0] != key or cached[1] != self.eps:
-            scale, shift = SCN.batchnorm_fold(self.running_mean, self.running_var, optional_tensor(self, "weight"),
-                                              optional_tensor(self, "bias"), self.eps)
+            scale, shift = SCN.batchnorm_fold(self.running_mean, self.running_var, weight, bias, self.eps)
             cached = self._folded = (key, self.eps, scale, shift)
         return cached[2], cached[3], self.leakiness
 
@@ -411,9 +421,9 @@ class BatchNormalization(Module):
         wanted, statistics on the features' device."""
         if self.training or self._forward_hooks or self._forward_pre_hooks:
             return False
-        mean, params = self._buffers["running_mean"], self._parameters
+        mean = self._buffers["running_mean"]
         return (mean.is_cuda and mean.device == features.device
-                and not autograd.needs_grad(features, params.get("weight"), params.get("bias")))
+                and not autograd.needs_grad(features, parameter(self, "weight"), parameter(self, "bias")))
 
     def forward_joined(self, inputs):
         """This layer (eval mode) applied to the concatenation of `inputs` (what a JoinTable in front of

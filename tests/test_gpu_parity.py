@@ -628,3 +628,72 @@ def test_unet_prefetches_its_encoder_rulebooks(cuda):
         scn.Sequential.prefetch_rulebooks = True
         scn.set_precision("fp32")
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32x3"])
+@pytest.mark.parametrize("how", ["weight_norm", "prune", "parametrize", "replicate"])
+def test_wrapped_parameters(how, precision, cuda):
+    """Layers whose weight (and a BatchNorm's scale) something else has put in place of the registered parameter, in eval and
+    in training, give what plain layers with those values do, also after the values have changed."""
+    import sparseconvnet_b200 as scn
+    torch.manual_seed(2)
+
+    def build():
+        net = scn.Sequential().add(scn.SubmanifoldConvolution(3, 16, 32, 3, True)).add(scn.BatchNormReLU(32)).add(
+            scn.Convolution(3, 32, 16, 2, 2, True)).add(scn.BatchNormReLU(16)).add(scn.Deconvolution(3, 16, 8, 2, 2, True))
+        return net.to(cuda)
+    net, plain = build(), build()
+    for m in net:
+        for t in list(m.parameters()) + list(m.buffers()):
+            torch.nn.init.uniform_(t, 0.2, 1.0)
+    coords = torch.randint(0, 32, (4000, 3))
+    feats = torch.randn(len(coords), 16, device=cuda)
+    run = lambda m: m(scn.InputLayer(3, 32, mode=3)([coords, feats])).features
+    convs, norms = [net[0], net[2], net[4]], [net[1], net[3]]
+    wrapped = net
+    if how == "weight_norm":
+        with pytest.warns(FutureWarning):
+            for m in convs:
+                torch.nn.utils.weight_norm(m)
+        value = lambda m: m.weight_v * (m.weight_g / m.weight_v.flatten(1).norm(dim=1).view_as(m.weight_g))
+    elif how == "prune":
+        import torch.nn.utils.prune as prune
+        for m in convs + norms:
+            prune.random_unstructured(m, "weight", 0.3)
+        value = lambda m: m.weight_orig * m.weight_mask
+    elif how == "parametrize":
+        class Twice(torch.nn.Module):
+            def forward(self, w):
+                return 2 * w
+        for m in convs + norms:
+            torch.nn.utils.parametrize.register_parametrization(m, "weight", Twice())
+        value = lambda m: 2 * m.parametrizations.weight.original
+    else:
+        wrapped = torch.nn.parallel.replicate(net, [cuda])[0]
+        value = lambda m: m.weight
+    try:
+        scn.set_precision(precision)
+        for change in range(2):
+            with torch.no_grad():
+                if change:
+                    for m in net:
+                        for _, t in m.named_parameters():
+                            t.mul_(0.7)
+                    if how == "replicate":
+                        wrapped = torch.nn.parallel.replicate(net, [cuda])[0]
+                for a, b in zip(net, plain):
+                    b.weight.copy_(value(a) if a in convs or how in ("prune", "parametrize") else a.weight)
+                    b.bias.copy_(a.bias)
+                    if a in norms:
+                        b.running_mean.copy_(a.running_mean)
+                        b.running_var.copy_(a.running_var)
+                for m in (wrapped, plain):
+                    m.eval()
+                want = run(plain)
+                for again in range(2):
+                    assert helpers.rel_err(run(wrapped).cpu().numpy(), want.cpu().numpy()) <= 1e-5
+        for m in (wrapped, plain):
+            m.train()
+        assert helpers.rel_err(run(wrapped).detach().cpu().numpy(), run(plain).detach().cpu().numpy()) <= 1e-4
+    finally:
+        scn.set_precision("fp32")
