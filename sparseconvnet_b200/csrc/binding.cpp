@@ -18,6 +18,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -103,8 +104,12 @@ struct Sizes {
     }
     PyObject *seq = PySequence_Fast(o, "a size must be a tensor or a sequence");
     if (!seq) throw Fail{};
-    n = (int)PySequence_Fast_GET_SIZE(seq);
-    for (int i = 0; i < n && i < 16; ++i) {
+    n = (int)std::min<Py_ssize_t>(PySequence_Fast_GET_SIZE(seq), 17);
+    if (n > 16) {
+      Py_DECREF(seq);
+      fail("a size of more than 16 dimensions");
+    }
+    for (int i = 0; i < n; ++i) {
       PyObject *v = PyNumber_Long(PySequence_Fast_GET_ITEM(seq, i));
       own[i] = v ? PyLong_AsLongLong(v) : 0;
       Py_XDECREF(v);
@@ -1003,10 +1008,19 @@ SCN_FN(active_sites) {
   SCN_END
 }
 
+// filter and stride of as many dimensions as the size (the C entries read that many values)
+void same_dimensions(const Sizes &size, const Sizes &filter, const Sizes &stride) {
+  if (filter.n != size.n || stride.n != size.n)
+    fail("spatial size, filter size and stride have %d, %d and %d dimensions", size.n, filter.n, stride.n);
+}
+
 // (size, filter, stride) -> LongTensor (size - filter) / stride + 1; None when the filter does not tile the size
 SCN_FN(strided_size) {
   SCN_BEGIN(3)
   const Sizes size(a[0]), filter(a[1]), stride(a[2]);
+  same_dimensions(size, filter, stride);
+  for (int d = 0; d < size.n; ++d)
+    if (stride.p[d] < 1) fail("stride %lld", (long long)stride.p[d]);  // (0 would end the process)
   at::Tensor out = at::empty({size.n}, at::kLong);
   int64_t *o = (int64_t *)out.data_ptr();
   for (int d = 0; d < size.n; ++d) {
@@ -1021,6 +1035,7 @@ SCN_FN(strided_size) {
 SCN_FN(transposed_size) {
   SCN_BEGIN(3)
   const Sizes size(a[0]), filter(a[1]), stride(a[2]);
+  same_dimensions(size, filter, stride);
   at::Tensor out = at::empty({size.n}, at::kLong);
   int64_t *o = (int64_t *)out.data_ptr();
   for (int d = 0; d < size.n; ++d) o[d] = (size.p[d] - 1) * stride.p[d] + filter.p[d];

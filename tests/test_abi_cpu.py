@@ -119,3 +119,19 @@ def test_batchnorm_layers_are_switched_to_shared_statistics():
     assert shard.sum_gradients(p) == 0 and all(float(t.grad[0]) == 2.0 for t in p)
     shard.sum_gradients(p, scale=0.5)
     assert all(float(t.grad[0]) == 1.0 for t in p)
+
+
+def test_output_sizes_of_strided_layers():
+    """The host arithmetic in front of a strided layer: a stride of zero and sizes of different lengths are errors, in this
+    process, as torch's own division was."""
+    from sparseconvnet_b200 import _binding
+    lt = torch.LongTensor
+    assert _binding.strided_size(lt([9, 7, 4]), lt([3, 3, 2]), lt([2, 2, 2])).tolist() == [4, 3, 2]
+    assert _binding.strided_size([8, 7], [2, 2], [2, 2]) is None
+    assert _binding.transposed_size(lt([4, 3]), lt([3, 2]), lt([2, 2])).tolist() == [9, 6]
+    for call, args in ((_binding.strided_size, (lt([8, 8]), lt([2, 2]), lt([2, 0]))),
+                       (_binding.strided_size, (lt([8, 8, 8]), lt([2, 2]), lt([2, 2, 2]))),
+                       (_binding.transposed_size, (lt([8, 8, 8]), lt([2, 2, 2]), lt([2]))),
+                       (_binding.transposed_size, ([8] * 20, [2] * 20, [2] * 20))):
+        with pytest.raises(RuntimeError):
+            call(*args)
