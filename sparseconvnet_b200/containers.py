@@ -247,7 +247,8 @@ class AddTable(torch.nn.Sequential):
         features = input[0].features
         for i in input[1:]:
             features = features + i.features
-        output.features = features
+        # (the sum of one is a tensor of its own too: what changes it in place must not change the branch)
+        output.features = features if len(input) > 1 else features.clone()
         return output
 
     def input_spatial_size(self, out_size):

@@ -135,3 +135,11 @@ def test_output_sizes_of_strided_layers():
                        (_binding.transposed_size, ([8] * 20, [2] * 20, [2] * 20))):
         with pytest.raises(RuntimeError):
             call(*args)
+
+
+def test_add_table_of_one_branch_is_a_tensor_of_its_own():
+    import sparseconvnet_b200 as scn
+    a = scn.SparseConvNetTensor(torch.ones(3, 2), None, None)
+    y = scn.AddTable()([a])
+    y.features.mul_(5)
+    assert torch.equal(a.features, torch.ones(3, 2)) and torch.equal(y.features, 5 * torch.ones(3, 2))
