@@ -72,6 +72,7 @@ def _wants_split(conv, follower):
             and layers.SCN._precision != layers.SCN.PRECISION_FP32 and conv.groups == 1 and follower.groups == 1
             and conv.nOut == follower.nIn and conv.nOut % 16 == 0 and layers.SCN.Profile.active is None
             and type(conv) in (layers.SubmanifoldConvolution, layers.Convolution, layers.Deconvolution)
+            and not follower._forward_pre_hooks  # (which may change the features in ways that leave no trace, as .data does)
             and not torch.is_inference_mode_enabled())  # (inference tensors have no version to check)
 
 

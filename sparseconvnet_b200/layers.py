@@ -220,7 +220,7 @@ class _ConvBase(Module):
 
 def _split_rows(input):
     """The split form of a tensor's features, if it travels with them and still is theirs."""
-    s = input.split
+    s = getattr(input, "split", None)
     return s[0] if s is not None and s[1] is input.features and s[2] == s[1]._version and s[3] == SCN._precision else None
 
 

@@ -184,3 +184,37 @@ def test_split_rows_left_for_the_next_layer(n, split, planes, precision, cuda, m
             x.metadata.poll_errors()
     finally:
         scn.set_precision("fp32")
+
+
+@pytest.mark.parametrize("precision", ["tf32x3", "bf16"])
+def test_split_rows_and_a_hook_on_the_next_layer(precision, cuda):
+    """A forward pre-hook that changes the features through .data, which leaves their version as it is, and an input that
+    only looks like a SparseConvNetTensor: the next layer computes with the features as they are."""
+    import sparseconvnet_b200 as scn
+    torch.manual_seed(0)
+    net = scn.Sequential().add(scn.SubmanifoldConvolution(3, 32, 32, 3, True)).add(scn.BatchNormReLU(32)).add(
+        scn.SubmanifoldConvolution(3, 32, 48, 3, True)).to(cuda).eval()
+
+    class Looks:
+        def __init__(self, x):
+            self.features, self.metadata, self.spatial_size = x.features, x.metadata, x.spatial_size
+    try:
+        scn.set_precision(precision)
+        with torch.no_grad():
+            coords = _points(5000, 3, 60, 0)
+            x = scn.InputLayer(3, 60, mode=0)([torch.from_numpy(coords), torch.randn(len(coords), 32, device=cuda)])
+            plain = net(x).features.clone()
+            mid = net[1](net[0](x))
+            mid.features.mul_(3)
+            want = net[2](mid).features
+            assert torch.equal(net[2](Looks(mid)).features, want)
+
+            def triple(module, args):
+                args[0].features.data.mul_(3)
+            handle = net[2].register_forward_pre_hook(triple)
+            got = net(x).features
+            handle.remove()
+            assert torch.equal(got, want) and not torch.equal(got, plain)
+            assert torch.equal(net(x).features, plain)
+    finally:
+        scn.set_precision("fp32")
