@@ -409,6 +409,16 @@ static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float
   SCN_REQUIRE(precision >= SCN_PRECISION_FP32 && precision <= SCN_PRECISION_TF32X3, SCN_ERR_BAD_ARG,
               "unknown precision %d", precision);
   SCN_REQUIRE(weight, SCN_ERR_BAD_ARG, "null weight");
+  // The kernels read a BatchNorm's scale and shift in 16-byte pieces; a slice of a larger array goes through a copy.
+  Scratch tmp(stream);
+  for (const float **v : {&bn_scale, &bn_shift, &pre_scale, &pre_shift}) {
+    if ((uintptr_t)*v % 16 == 0) continue;
+    const size_t bytes = sizeof(float) * (size_t)(v == &bn_scale || v == &bn_shift ? n_out_planes : n_in_planes);
+    float *copy = nullptr;
+    SCN_TRY(tmp.get(&copy, bytes));
+    SCN_CUDA_CHECK(cudaMemcpyAsync(copy, *v, bytes, cudaMemcpyDeviceToDevice, stream));
+    *v = copy;
+  }
   int cin = n_in_planes / groups, cout = n_out_planes / groups;
   long long rows_in = transposed ? rb.n_out : rb.n_in;
   long long rows_out = transposed ? rb.n_in : rb.n_out;

@@ -218,3 +218,37 @@ def test_split_rows_and_a_hook_on_the_next_layer(precision, cuda):
             assert torch.equal(net(x).features, plain)
     finally:
         scn.set_precision("fp32")
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32x3", "bf16"])
+@pytest.mark.parametrize("n", [300, 30000])
+@pytest.mark.parametrize("cin,cout", [(16, 16), (32, 96)])
+def test_scale_and_shift_anywhere(n, cin, cout, precision, cuda):
+    """Scale and shift of a BatchNorm in front of and behind a convolution as slices that start at any multiple of four
+    bytes: the same bits as from arrays of their own."""
+    import sparseconvnet_b200 as scn
+    from sparseconvnet_b200 import SCN
+    torch.manual_seed(n)
+    coords = _points(n, 3, 120, n)
+    x = scn.InputLayer(3, 120, mode=0)([torch.from_numpy(coords), torch.randn(len(coords), cin, device=cuda)])
+    w, three = torch.randn(27, 1, cin, cout, device=cuda), torch.LongTensor([3] * 3)
+    post, pre = torch.rand(2, cout, device=cuda) + 0.5, torch.rand(2, cin, device=cuda) + 0.5
+    try:
+        scn.set_precision(precision)
+        results = []
+        for offset in (0, 1, 2, 3):
+            def place(v):
+                return torch.empty(offset + v.numel(), device=cuda)[offset:].copy_(v)
+            out, both = (x.features.new_empty(0) for _ in range(2))
+            epilogue = (place(post[0]), place(post[1]), 0.25)
+            SCN.SubmanifoldConvolution_updateOutput(x.spatial_size, three, x.metadata, x.features, out, w, None, epilogue=epilogue)
+            half = cin // 2
+            assert SCN.SubmanifoldConvolution_joined(
+                x.spatial_size, three, x.metadata, [x.features[:, :half].contiguous(), x.features[:, half:].contiguous()], both, w,
+                None, prologue=(place(pre[0]), place(pre[1]), 0.5), epilogue=epilogue) is not None
+            results.append((out, both))
+        x.metadata.poll_errors()
+        for out, both in results[1:]:
+            assert torch.equal(out, results[0][0]) and torch.equal(both, results[0][1])
+    finally:
+        scn.set_precision("fp32")
