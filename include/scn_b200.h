@@ -77,12 +77,21 @@ enum scn_precision {
 };
 /* which convolution kernel the last convolution call of this thread ran (for profiling) */
 enum scn_conv_kernel {
-  SCN_KERNEL_CONV_SIMT = 0,          /* fp32 FMA: k_conv_fma (mask-sorted tiles), k_conv_pipe, k_conv_simt, k_conv_thin */
-  SCN_KERNEL_CONV_TC = 1,            /* tcgen05, more than 64 output planes, small levels: k_conv_tile, k_conv_tc */
+  SCN_KERNEL_CONV_SIMT = 0,          /* k_conv_pipe / k_conv_simt / k_conv_thin: fp32 FMA     */
+  SCN_KERNEL_CONV_TC = 1,            /* k_conv_tc: tcgen05, one tile per CTA                  */
   SCN_KERNEL_CONV_TC_PERSISTENT = 2, /* k_conv_tma: tcgen05, persistent, double-buffered TMEM */
   SCN_KERNEL_CONV_PIPE_MMA = 3,      /* k_conv_pipe with three tf32 mma.sync passes           */
-  SCN_KERNEL_CONV_ROWS = 4,          /* up to 64 output planes: k_conv_tile (tcgen05); k_conv_rows (warp-level mma.sync) */
-  SCN_KERNEL_CONV_WIDE = 5           /* tcgen05, more than 64 output planes, large levels: k_conv_tile, k_conv_wide */
+  SCN_KERNEL_CONV_ROWS = 4,          /* k_conv_rows and its first-layer forms: row-stationary, warp-level mma.sync */
+  SCN_KERNEL_CONV_WIDE = 5,          /* k_conv_wide: tcgen05, persistent, rows split to bf16 parts once per call and copied in by cp.async */
+  SCN_KERNEL_CONV_TILE = 6,          /* k_conv_tile: tcgen05, persistent, mask-sorted row tiles */
+  SCN_KERNEL_CONV_FMA = 7            /* k_conv_fma: fp32 FMA, mask-sorted row tiles           */
+};
+/* which kernel the last weight gradient of a convolution ran, whatever thread asked for it (autograd has its own) */
+enum scn_dweight_kernel {
+  SCN_KERNEL_DWEIGHT_FMA = 0,        /* k_conv_dweight: fp32 FMA (several groups)             */
+  SCN_KERNEL_DWEIGHT_MMA = 1,        /* k_conv_dweight_mma: warp-level mma.sync               */
+  SCN_KERNEL_DWEIGHT_TILE = 2,       /* k_dweight_tile: tcgen05, mask-sorted row tiles        */
+  SCN_KERNEL_DWEIGHT_THIN = 3        /* k_conv_dweight_thin: fp32 FMA in registers, first layers */
 };
 /* The tensor-core modes run on tcgen05 (k_conv_tile) for groups == 1, filters of at most 128 offsets, n_in_planes and
  * n_out_planes multiples of eight, n_out_planes <= 256 and 16-byte aligned rows; other shapes run on the older tensor
@@ -242,6 +251,7 @@ SCN_API int scn_md_rulebook_export(scn_metadata *md, int kind, const int64_t *si
 /* -1 before the first convolution, else an scn_conv_kernel value.  No counterpart in the
  * reference; lets a profiler attribute a call's time to the kernel that ran it. */
 SCN_API int scn_last_conv_kernel(void);
+SCN_API int scn_last_dweight_kernel(void);
 
 /* Self-calibration of the tensor path.  No counterpart in the reference.  Issues `n_mma`
  * tcgen05.mma instructions of shape M x N (x 8 tf32 / 16 bf16 along K) back to back from one

@@ -368,7 +368,7 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
     SCN_TRY(rulebook_row_order(rb, table, rows_out, ord, stream));
     SCN_TRY(conv_forward_tile(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, ord, rb.n_offsets,
                               cin, cout, precision, flags, stream, pre_scale, pre_shift, pre_leak, in_b, planes_a));
-    g_last_kernel = cout <= 64 ? SCN_KERNEL_CONV_ROWS : rows_out <= 148 * 256 ? SCN_KERNEL_CONV_TC : SCN_KERNEL_CONV_WIDE;
+    g_last_kernel = SCN_KERNEL_CONV_TILE;
     return SCN_OK;
   }
   // fp32: the same tiles on the FMA pipe (first layers of at most four input planes keep their own kernel), unless a
@@ -391,7 +391,7 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
     rc = conv_forward_fma(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, table, ord, rb.n_offsets, cin,
                           cout, flags, stream);
   device_free(pre_copy, stream);
-  g_last_kernel = SCN_KERNEL_CONV_SIMT;
+  g_last_kernel = SCN_KERNEL_CONV_FMA;
   return rc;
 }
 

@@ -512,6 +512,8 @@ k_column_sums(const float *__restrict__ x, long long n_rows, int planes, long lo
   }
 }
 
+static std::atomic<int> g_last_dweight_kernel{-1};
+
 // Runs the backward pass for one operator call.  `transposed` as in the forward pass (Deconvolution).
 static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, const float *in, float *d_in,
                              const float *d_out, const float *weight, float *d_weight, float *d_bias,
@@ -556,8 +558,10 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
     const char *tile = getenv("SCN_DWEIGHT_TILE");
     if (groups == 1 && !fma_only && !(tile && atoi(tile) == 0) && dweight_tile_supported(in, d_out, rb, cin, cout)) {
       SCN_TRY(rulebook_row_order(rb, rb.nbr, rb.n_out, rb.order, stream));
+      g_last_dweight_kernel = SCN_KERNEL_DWEIGHT_TILE;
       SCN_TRY(dweight_tile(in, rows_in, d_out, rows_out, rb, transposed, cin, cout, d_weight, md->flags_dev, stream));
     } else if (groups == 1 && !fma_only && cin <= 3 && cout <= 32 && !transposed && rows_out > 0) {
+      g_last_dweight_kernel = SCN_KERNEL_DWEIGHT_THIN;
       SCN_TRY(dweight_thin(in, rows_in, d_out, rows_out, rb.nbr, K, cin, cout, d_weight, md->flags_dev, stream));
     } else if (groups == 1 && !fma_only) {
       decltype(&launch_dweight<1, 1>) const by_side[3][3] = {{launch_dweight<1, 1>, launch_dweight<1, 2>, launch_dweight<1, 3>},
@@ -565,9 +569,11 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
                                                              {launch_dweight<3, 1>, launch_dweight<3, 2>, launch_dweight<3, 3>}};
       auto launch = by_side[dweight_side(cin, n_entries) - 1][dweight_side(cout, n_entries) - 1];
       if (cin <= 16) launch = cout <= 32 ? launch_dweight<1, 1, 1> : cout <= 64 ? launch_dweight<1, 2, 1> : launch_dweight<1, 3, 1>;
+      g_last_dweight_kernel = SCN_KERNEL_DWEIGHT_MMA;
       SCN_TRY(launch(in, n_in_planes, rows_in, d_out, n_out_planes, rows_out, rb.nbr, n_entries, transposed ? 1 : 0, K, cin,
                      cout, d_weight, md->flags_dev, stream));
     } else {
+      g_last_dweight_kernel = SCN_KERNEL_DWEIGHT_FMA;
       const int chunks = n_chunks(n_entries);
       const long long chunk_rows = ceil_div(ceil_div(n_entries, chunks), 32) * 32;
       Scratch tmp(stream);
@@ -602,6 +608,8 @@ static int run_conv_backward(scn_metadata *md, Rulebook &rb, bool transposed, co
 using namespace scn;
 
 extern "C" {
+
+int scn_last_dweight_kernel(void) { return g_last_dweight_kernel; }
 
 int scn_submanifold_convolution_backward(scn_metadata *md, const int64_t *spatial_size, const int64_t *filter_size,
                                          const float *in_features, float *d_in_features,

@@ -3,9 +3,10 @@ unmodified Python package (its scn.UNet / SparseResNet / SparseVggNet builders, 
 on its own CPU extension, both staged under oracle/_ref by oracle/build_ref.py.
 
 Every convolution kernel of the library is also compared here, one layer at a time, with the
-reference's CPU operator directly (not with another CUDA kernel): the row-stationary
-warp-level kernel, the persistent tcgen05 kernel in every arithmetic mode, and the per-tile
-tcgen05 kernel with and without the split of the filter offsets.
+reference's CPU operator directly (not with another CUDA kernel): the tcgen05 kernel on mask-sorted
+tiles that runs by default, and the kernels behind it, each forced: the row-stationary warp-level kernel,
+the persistent tcgen05 kernel in every arithmetic mode, and the per-tile tcgen05 kernel with and without
+the split of the filter offsets.
 
 Tolerances relative to the tensor's largest magnitude: 1e-4 for fp32 and the fp32-class split
 mode, 1e-2 for single-pass tf32 / bf16."""
@@ -72,19 +73,18 @@ def _gpu_forward(config, samples, precision, profile=False):
 
 @pytest.mark.parametrize("precision,tol", [("tf32x3", helpers.FP32_TOL), ("fp32", helpers.FP32_TOL)])
 def test_config3_full_batch_vs_reference(precision, tol, cuda):
-    """The benchmark's own shape: the U-Net on all 8 rooms (~1.6 M voxels).  In the fp32-class mode
-    every convolution kernel class of the step must have run: warp-level rows kernel (32 / 64
-    output planes), persistent tcgen05 (96 / 128 planes on the large levels), per-tile tcgen05
-    (the small deep levels)."""
+    """The benchmark's own shape: the U-Net on all 8 rooms (~1.6 M voxels).  Every layer but
+    the first must have run on mask-sorted tiles, tcgen05 ones in the fp32-class mode and fp32 ones in
+    fp32; the first, of three input planes, on its own kernel of each mode."""
     loc_r, feat_r, _ = _reference_forward(3, list(range(8)), "c3x8")
     loc_g, feat_g, _, kernels = _gpu_forward(3, list(range(8)), precision, profile=True)
     e = helpers.assert_features_match(loc_g, feat_g, loc_r, feat_r, tol, what="config 3 x 8 rooms " + precision)
     print("config3 x8 %s rel err %.3g kernels %s" % (precision, e, sorted(set(kernels))))
     assert len(kernels) == 39
     if precision == "tf32x3":
-        assert {"k_conv_rows", "k_conv_wide", "k_conv_tc"} <= set(kernels), sorted(set(kernels))
+        assert kernels == ["k_conv_rows"] + ["k_conv_tile"] * 38, kernels
     else:
-        assert set(kernels) == {"k_conv_simt"}, sorted(set(kernels))
+        assert kernels == ["k_conv_simt"] + ["k_conv_fma"] * 38, kernels
 
 
 @pytest.mark.parametrize("precision,tol", [("fp32", helpers.FP32_TOL), ("tf32x3", helpers.FP32_TOL)])
@@ -206,5 +206,13 @@ def test_per_tile_tcgen05_vs_reference(cin, cout, precision, form, tol, split, c
 def test_rows_kernel_vs_reference(cin, cout, precision, form, tol, cuda, monkeypatch):
     """k_conv_rows (32 / 64 output planes) in its arithmetic modes, both forms of the fp32-class one."""
     e, rows = _layer_vs_reference(cin, cout, precision, tol, 4, monkeypatch=monkeypatch, bias=(cin == 64),
-                                  env={"SCN_X3_FORM": form})
+                                  env={"SCN_X3_FORM": form, "SCN_CONV_TILE": "0"})
     print("k_conv_rows %d->%d %s/%s: %d rows, rel err %.3g" % (cin, cout, precision, form, rows, e))
+
+
+@pytest.mark.parametrize("precision,tol,kernel", [("tf32x3", helpers.FP32_TOL, 6), ("tf32", helpers.FP32_TOL, 6),
+                                                  ("bf16", helpers.TC_TOL, 6), ("fp32", helpers.FP32_TOL, 7)])
+@pytest.mark.parametrize("cin,cout", [(32, 32), (48, 64), (96, 96), (160, 224)])
+def test_mask_sorted_tiles_vs_reference(cin, cout, precision, tol, kernel, cuda, monkeypatch):
+    """k_conv_tile and k_conv_fma, the default kernels; tf32 runs the three-term form as well."""
+    _layer_vs_reference(cin, cout, precision, tol, kernel, monkeypatch=monkeypatch, bias=(cin == 48))

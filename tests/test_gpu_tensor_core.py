@@ -203,7 +203,7 @@ def test_bounded_wait_runs_out_and_the_library_recovers(cuda, restore_precision)
         want = sc(x).features
         scn.set_precision("bf16")
         good = sc(x).features.clone()
-        assert lib.scn_last_conv_kernel() == 1      # the per-tile kernel: the one the hook reaches
+        assert lib.scn_last_conv_kernel() == 6      # k_conv_tile: the next kernel the hook reaches
         x.metadata.poll_errors()
         assert lib.scn_test_drop_barrier_arrival() == 0
         sc(x)                                        # returns: the launch is asynchronous

@@ -36,6 +36,7 @@ def _compare(layers, coords, dim, size, cin, precision, cuda, mode=3):
                 want = layer.to(cuda)(x)
                 scn.set_precision(precision)
                 got = layer(x)
+                assert scn.SCN.lib.scn_last_conv_kernel() == 6, "not on k_conv_tile"
                 again = layer(x)
                 x.metadata.poll_errors()
                 assert got.features.shape == want.features.shape
@@ -117,6 +118,7 @@ def test_fp32_tiles(n, split, cin, cout, cuda, monkeypatch):
                 layer.bias.normal_()
             f = torch.randn(x.metadata.getNActive(spatial), cin, device=cuda)
             y = layer(scn.SparseConvNetTensor(f, x.metadata, spatial)).features
+            assert scn.SCN.lib.scn_last_conv_kernel() == 7 or y.size(0) == 0, "not on k_conv_fma"
             want = torch.zeros(y.shape, dtype=torch.float64, device=cuda)
             if hasattr(layer, "bias"):
                 want += layer.bias.double()
