@@ -41,27 +41,22 @@ UNIT = "voxels/s"
 # launches against their algorithmic bytes).  The traffic grows with the rows, like the
 # algorithmic bytes: DRAM sees input, rulebook and output about once, the gather's re-reads
 # (which the algorithmic figure counts per rule) hit L2.
-TRAFFIC_RATIO = {"k_conv_tma": 0.22, "k_conv_pipe_mma": 0.22, "k_conv_rows": 0.24, "k_conv_simt": 0.25,
-                 "k_conv_wide": 0.17}
+TRAFFIC_RATIO = {"k_conv_tile": 0.27, "k_conv_fma": 0.25}
 # (bound reported for the kernel, what the ncu captures show as its limiter)
 LIMITS = {
-    "k_conv_tma": ("hbm", "shared-memory data pipe 77 % busy, tensor pipe 40-46 % (ncu, 4-room case)"),
-    "k_conv_pipe_mma": ("hbm", "instruction issue and the shared-memory data pipe of small (offset, 128-row) steps"),
-    "k_conv_rows": ("hbm", "no saturated pipe (ncu, 4-room case): warp-level tensor pipe 41-53 % active, LSU wavefronts "
-                           "39-47 % of peak, issue slots 42-57 %; the warp's dependent chain rulebook entry -> gather -> "
-                           "fragment loads -> bf16 split -> tensor instruction with 13-19 warps per SM; DRAM sees 0.19-0.24 "
-                           "of the algorithmic bytes, the gather's re-reads hit L2"),
-    "k_conv_wide": ("hbm", "shared-memory bandwidth: a 32-plane step writes 45 KB of tiles and slabs and the tensor core reads "
-                           "72 KB of operands, against 128 B per cycle; tensor pipe 47.5 % active (ncu, 4-room case)"),
-    "k_conv_tc": ("hbm", "latency: few 256-row tiles per level (tensor pipe 13-16 %)"),
+    "k_conv_tile": ("hbm", "the gather of whole rows from L2 into shared memory by 16-byte cp.async (ncu, 4-room case): LSU "
+                           "wavefronts 39 % of peak on average and up to 53 %, tensor pipe 25 % (43 % on the widest levels), "
+                           "issue slots 28 %; DRAM sees 0.27 of the algorithmic bytes"),
+    "k_conv_fma": ("hbm", "the FMA pipe behind two block barriers per step (ncu, 4-room case, the four finest levels): FMA pipe "
+                          "51 % (60 % at 64 planes), issue slots 64 %, LSU wavefronts 48 %, a fifth of the warp slots filled"),
 }
 # what `dtype` says for each arithmetic mode: the type the path computes in, kernel by kernel
 DTYPE_LABEL = {
     "fp32": "f32 (fp32 FMA in every convolution)",
     "tf32x3": "f32-class split arithmetic, fp32 accumulate: every operand as two bf16 parts, three bf16 products "
               "per term on tcgen05 kind::f16 with TMEM accumulators",
-    "tf32": "tf32 (single pass, fp32 accumulate)",
-    "bf16": "bf16 (single pass, fp32 accumulate)",
+    "tf32": "f32-class split arithmetic as tf32x3 (the mode asks for no less than one tf32 product); the first layer fp32",
+    "bf16": "bf16 (single pass, fp32 accumulate); the first layer fp32",
 }
 CONFIG_NAMES = {
     1: "config1: SubmanifoldConvolution 3D f3 32->32, 256^3 shells and planes, batch 1, fresh Metadata per step",
@@ -269,11 +264,15 @@ class ReferenceCpu(object):
 
 def run_reference(args, rank):
     """The reference's CPU implementation on the host cores, on the same batch as rank 0 of the GPU
-    arm: K steps of all 8 rooms each."""
+    arm: K steps of all 8 rooms each.  Nothing of this package's models or kernels takes part."""
     if rank != 0:
         return
+    from oracle import refpkg
+    if not refpkg.available("cpu"):
+        print(json.dumps({"impl": "reference", "unavailable": "the compiled reference (oracle/_ref) is not present"}))
+        return
     cpu = ReferenceCpu(load_workloads())
-    samples = list(range(args.rooms)) if cpu.kind == "reference" else [0]
+    samples = list(range(args.rooms))
     v, sec, n = cpu.time(CONFIG, samples, args.warmup, args.steps)
     sample = "the whole batch of rank 0 (%d rooms, %d voxels) per step, %d steps" % (len(samples), n, args.steps)
     print(json.dumps({
@@ -281,8 +280,7 @@ def run_reference(args, rank):
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * sec,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": {"workload": workload_name(len(samples)), "voxels_per_step": n, "sample": sample,
-                   "path": "the reference's own Python package and CPU extension" if cpu.kind == "reference"
-                   else "numpy restatement (the compiled reference is absent)"},
+                   "path": "the reference's own Python package and CPU extension"},
         "cpu_baseline": {"value": v, "unit": UNIT, "cores": cpu.cores, "kind": cpu.kind, "sample": sample},
         "e2e": {"value": v, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
         "gpu_launches": 0,
@@ -623,7 +621,8 @@ def main():
     # An operator's pair of events also sees the GPU idle when the host is late with the launch in between (seen:
     # one call of 4 ms among its 0.6 ms peers).  So the step is profiled four times with the cyclic GC held off as
     # in the timed regions; the first pass, which creates the events' pool, is dropped and every call is given
-    # the median of its three times.
+    # the median of its three times.  Two forms of the timed step do not run here: a convolution does not leave its result
+    # in split form for the next, and a BatchNorm in front of a SubmanifoldConvolution runs by itself.
     import gc
     gc.collect()
     gc.disable()

@@ -64,16 +64,15 @@ enum scn_status {
 /* arithmetic used inside the convolution kernels */
 enum scn_precision {
   SCN_PRECISION_FP32 = 0, /* fp32 FMA, fp32 accumulate (matches the reference's float path)  */
-  SCN_PRECISION_TF32 = 1, /* one tf32 product, fp32 accumulate: warp-level mma.sync for 32 / 64 output
-                             planes, tcgen05 kind::tf32 with the accumulator in TMEM above          */
-  SCN_PRECISION_BF16 = 2, /* one bf16 product, fp32 accumulate: mma.sync for 32 / 64 output planes,
-                             tcgen05 kind::f16 with the accumulator in TMEM above                   */
+  SCN_PRECISION_TF32 = 1, /* at least one tf32 product, fp32 accumulate.  k_conv_tile computes it as
+                             SCN_PRECISION_TF32X3, which is more accurate and takes it no longer; the
+                             older kernels behind it issue one tf32 product                         */
+  SCN_PRECISION_BF16 = 2, /* one bf16 product, fp32 accumulate                                      */
   SCN_PRECISION_TF32X3 = 3 /* fp32-class accuracy on the tensor paths (1e-4 of the reference's fp32
                              results): every operand is split in two bf16 parts, x = h + m, and the
-                             three products h h, m h, h m are accumulated in fp32 -- warp-level
-                             mma.sync.m16n8k16 for 32 / 64 output planes, tcgen05 kind::f16 in TMEM
-                             for wider layers.  (The name is kept from the first form, three tf32
-                             products of a tf32 hi / lo split, which SCN_X3_FORM=tf32 still selects.) */
+                             three products h h, m h, h m are accumulated in fp32.  An infinity becomes
+                             NaN (its low part is inf - inf).  (The name is kept from the first form, three
+                             tf32 products of a tf32 hi / lo split, which SCN_X3_FORM=tf32 still selects.) */
 };
 /* which convolution kernel the last convolution call of this thread ran (for profiling) */
 enum scn_conv_kernel {

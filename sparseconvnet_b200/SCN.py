@@ -147,8 +147,9 @@ _precision = PRECISION_FP32
 
 def set_precision(p):
     """Arithmetic of the convolution kernels: 'fp32' (default; fp32 FMA), 'tf32x3' (tensor-core
-    tiles over the hi/lo split of both operands: fp32-class accuracy), 'tf32' or 'bf16'
-    (single-pass tensor-core tiles, fp32 accumulation)."""
+    tiles over the hi/lo split of both operands: fp32-class accuracy), 'tf32' (no less than one tf32
+    product; the layers that run on k_conv_tile get the three products of 'tf32x3') or 'bf16' (one
+    bf16 product), all with fp32 accumulation."""
     global _precision
     table = {"fp32": 0, "tf32": 1, "bf16": 2, "tf32x3": 3, 0: 0, 1: 1, 2: 2, 3: 3}
     if p not in table:
@@ -166,7 +167,7 @@ _backward_precision = PRECISION_FP32
 def set_backward_precision(p):
     """Arithmetic of the input-gradient pass of the convolutions' backward (the forward kernels on
     the opposite rulebook table): 'fp32' (default) or 'tf32x3' keep fp32-class gradients, 'tf32' /
-    'bf16' are single-pass.  Weight and bias gradients are always reduced in fp32."""
+    'bf16' as in set_precision.  Weight and bias gradients are always reduced in fp32."""
     global _backward_precision
     table = {"fp32": 0, "tf32": 1, "bf16": 2, "tf32x3": 3, 0: 0, 1: 1, 2: 2, 3: 3}
     if p not in table:
