@@ -521,8 +521,8 @@ int launch(DwParams &P, const Rulebook &rb, const float *t_rows, const float *g_
 }  // namespace
 
 // Rows of whole 16-byte pieces and more than 32 planes on one side: 32 x 32 weights are half as much work per gathered
-// byte, and k_conv_dweight_mma takes as long (400 k rows: 255 against 275 us; 64 x 64 at 124 k: 211 against 143, 96 x 96 at
-// 45 k: 339 against 225, 128 x 128 at 6 k: 114 against 67).  Below 2048 rows an order has to be there already.
+// byte, and k_conv_dweight_mma takes as long (278 us on 434 k rows).  Both kernels on the others: 64 x 64 on 119 k rows 230
+// and, here, 160 us, 96 x 96 on 49 k 412 and 229, 128 x 128 on 6 k 110 and 79.  Below 2048 rows an order has to be there already.
 // Multiples of 32 planes only: the running sums in TMEM cut off where fp32 additions round, 4e-6 of a sum of 100 k products
 // of mixed signs and 8e-6 with one sign.  That is no more than these shapes ever had (5e-6 and 1e-5 with truncated tf32 parts);
 // the others had plain fp32 sums (9e-7, 1.4e-7), which k_conv_dweight_mma matches.

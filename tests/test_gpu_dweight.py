@@ -198,7 +198,7 @@ def test_network_in_network_takes_what_a_matrix_product_takes(cuda):
             w = base.to(f.dtype).detach().requires_grad_()
             got = _affine(f, w, bias)
             want = f.double() @ w.detach().double() + (bias.double() if bias is not None else 0)
-            assert got.dtype == f.dtype and float((got - want).abs().max()) < 1e-4
+            assert got.dtype == f.dtype and float((got.detach() - want).abs().max()) < 1e-4
             got.sum().backward()
             assert float((w.grad - f.double().sum(0)[:, None]).abs().max()) < 1e-2
     f, w = flat[:-1].view(600, 32), torch.randn(32, 20, device=cuda, requires_grad=True)
