@@ -158,6 +158,7 @@ std::atomic<int> g_backward_precision{SCN_PRECISION_FP32};  // arithmetic of the
 // convolution whose kernel has no fused epilogue
 __global__ void k_scale_shift_act(float *__restrict__ y, long long n_rows, int planes, const float *__restrict__ scale,
                                   const float *__restrict__ shift, float leak) {
+  SCN_GRID_WAIT();
   const long long total = n_rows * planes;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int c = (int)(i % planes);
@@ -171,6 +172,7 @@ __global__ void k_scale_shift_act(float *__restrict__ y, long long n_rows, int p
 // (planes a multiple of four and 16-byte aligned matrices: four planes per thread; otherwise one)
 __global__ void k_scale_shift_act_to(const float *__restrict__ x, float *__restrict__ y, long long n_rows, int planes,
                                      const float *__restrict__ scale, const float *__restrict__ shift, float leak, int vec) {
+  SCN_GRID_WAIT();
   if (vec) {
     const long long total = n_rows * planes / 4;
     const int pv = planes / 4;
@@ -201,6 +203,7 @@ __global__ void k_scale_shift_act_to(const float *__restrict__ x, float *__restr
 __global__ void k_scale_shift_act_join_to(const float *__restrict__ a, int ca, const float *__restrict__ b, int cb,
                                           float *__restrict__ y, long long n_rows, const float *__restrict__ scale,
                                           const float *__restrict__ shift, float leak) {
+  SCN_GRID_WAIT();
   const int pv = (ca + cb) / 4, av = ca / 4;
   const long long total = n_rows * pv;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -224,6 +227,7 @@ __global__ void k_scale_shift_act_join_to(const float *__restrict__ a, int ca, c
 __global__ void k_bn_fold(const float *__restrict__ mean, const float *__restrict__ var, const float *__restrict__ gamma,
                           const float *__restrict__ beta, float eps, int planes, float *__restrict__ scale,
                           float *__restrict__ shift) {
+  SCN_GRID_WAIT();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= planes) return;
   const float w = powf(var[c] + eps, -0.5f) * (gamma ? gamma[c] : 1.f);

@@ -39,6 +39,7 @@ int dweight_tile(const float *in, long long rows_in, const float *d_out, long lo
 // W [K][groups][cin][cout] -> [K][groups][cout][cin]; mirror_groups > 0 (the number of groups): offset k goes to K - 1 - k
 __global__ void k_transpose_weight(const float *__restrict__ w, float *__restrict__ wt, long long n_mats, int cin,
                                    int cout, int mirror_groups) {
+  SCN_GRID_WAIT();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long per = (long long)cin * cout;
   if (idx >= n_mats * per) return;
@@ -57,6 +58,7 @@ __global__ void __launch_bounds__(256)
 k_conv_dweight(const float *__restrict__ in, int ld_in, long long n_in_rows, const float *__restrict__ dout,
                int ld_out, long long n_out_rows, const int *__restrict__ nbr, long long n_entries, int swap,
                int cin, int cout, int groups, long long chunk_rows, float *__restrict__ partial, int *flags) {
+  SCN_GRID_WAIT();
   __shared__ float A[32][33], B[32][33];
   const int tid = threadIdx.x;
   const int k = blockIdx.y;
@@ -115,6 +117,7 @@ k_conv_dweight(const float *__restrict__ in, int ld_in, long long n_in_rows, con
 
 // out[i] = sum over chunks, in order, of partial[chunk][i]; `add`: behind what is there already
 __global__ void k_sum_chunks(const float *__restrict__ partial, int chunks, long long n, float *__restrict__ out, bool add) {
+  SCN_GRID_WAIT();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float acc = add ? out[i] : 0.f;
@@ -178,6 +181,7 @@ __global__ void __launch_bounds__(DwShape<WM, WN, MT>::THREADS)
 k_conv_dweight_mma(const float *__restrict__ in, int ld_in, long long n_in_rows, const float *__restrict__ dout,
                    int ld_out, long long n_out_rows, const int *__restrict__ nbr, long long n_entries, int swap,
                    int cin, int cout, int vec_in, int vec_out, long long chunk_rows, float *__restrict__ partial, int *flags) {
+  SCN_GRID_WAIT();
   using S = DwShape<WM, WN, MT>;
   constexpr unsigned kFull = 0xffffffffu;
   constexpr int kWarps = S::THREADS / 32;
@@ -400,6 +404,7 @@ template <int CIN>
 __global__ void __launch_bounds__(256, 2)
 k_conv_dweight_thin(const float *__restrict__ in, long long n_in, const float *__restrict__ dout, long long n_out,
                     const int *__restrict__ nbr, int K, int cout, long long chunk_rows, float *__restrict__ partial, int *flags) {
+  SCN_GRID_WAIT();
   constexpr int N = kThinOffsets * CIN, W = (N + 3) / 4 * 4;  // values of a row
   __shared__ __align__(16) float values[8][32][W];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -495,6 +500,7 @@ static int dweight_side(int planes, long long n_entries) {
 __global__ void __launch_bounds__(256)
 k_column_sums(const float *__restrict__ x, long long n_rows, int planes, long long chunk_rows,
               float *__restrict__ partial) {
+  SCN_GRID_WAIT();
   __shared__ float sh[8][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int p = blockIdx.x * 32 + lane;

@@ -112,6 +112,7 @@ __host__ __device__ inline long long split_row_bytes(int pieces, int B) { return
 // per 8 planes.  Bound by HBM: 32 bytes in, 48 out.
 __global__ void __launch_bounds__(256)
 k_dweight_split(const float *__restrict__ x, unsigned char *__restrict__ out, long long n_pieces, int planes, int per_row, int B) {
+  SCN_GRID_WAIT();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_pieces) return;
   const long long row = i / per_row;
@@ -171,6 +172,7 @@ struct Ctl {
 
 template <int PT, int PG>
 __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_constant__ DwParams P) {
+  SCN_GRID_WAIT();
   using S = DwTile<PT, PG>;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ Ctl C;

@@ -64,6 +64,7 @@ struct FmaShape {
 template <int ROWS, int BN>
 __global__ void __launch_bounds__(kThreads, ROWS == 128 && BN == 64 ? 3 : 4)
 k_conv_fma(FmaParams P) {
+  SCN_GRID_WAIT();
   using S = FmaShape<ROWS, BN>;
   constexpr int TM = S::TM, TN = S::TN;
   extern __shared__ __align__(16) float fma_smem[];

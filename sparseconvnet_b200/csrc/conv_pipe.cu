@@ -160,6 +160,7 @@ k_conv_pipe(const float *__restrict__ in, int ld_in, long long n_in, float *__re
             long long n_out, const float *__restrict__ weight, long long w_offset_stride,
             long long w_group_stride, const float *__restrict__ bias, const int *__restrict__ nbr, int K,
             int cin, int cout, int *flags) {
+  SCN_GRID_WAIT();
   constexpr int BN = NPL * 8;
   constexpr unsigned kFull = 0xffffffffu;
   extern __shared__ __align__(16) unsigned char smem_raw[];

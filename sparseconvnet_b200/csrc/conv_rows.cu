@@ -88,6 +88,7 @@ __device__ __forceinline__ unsigned rows_pack_bf16(float first, float second) {
 //   [0] = tf32 hi of W[P+t][n], W[P+t+4][n], W[P+8+t][n], W[P+12+t][n]       (n = 8 nt + g)
 //   [1] = bf16 pairs (W[P+t], W[P+t+4]), (W[P+8+t], W[P+12+t]), then the same of W - hi
 __global__ void k_rows_prepare(const float *__restrict__ w, uint4 *__restrict__ img, int K, int cin, int cout) {
+  SCN_GRID_WAIT();
   const int nt_n = cout / 8, nch = cin / kRChunk;
   const long long total = (long long)K * nch * 2 * nt_n * 32;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -121,6 +122,7 @@ __global__ void k_rows_prepare(const float *__restrict__ w, uint4 *__restrict__ 
 // The image of the bf16 three-term form: [K][cin / 32][2][cout / 8][32] of uint4 =
 //   bf16 pairs (h(W[P+t]), h(W[P+t+4])), (h(W[P+8+t]), h(W[P+12+t])), then the same of m = bf16(W - h)
 __global__ void k_rows_prepare_b3(const float *__restrict__ w, uint4 *__restrict__ img, int K, int cin, int cout) {
+  SCN_GRID_WAIT();
   const int nt_n = cout / 8, nch = cin / kRChunk;
   const long long total = (long long)K * nch * 2 * nt_n * 32;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -345,6 +347,7 @@ k_conv_rows(const float *__restrict__ in, int ld_in, long long n_in, float *__re
             long long n_out, const uint4 *__restrict__ img, const float *__restrict__ bias,
             const float *__restrict__ bn_scale, const float *__restrict__ bn_shift, float leak,
             const int *__restrict__ nbr, int K, int nch_arg, int *flags) {
+  SCN_GRID_WAIT();
   const int nch = NCH ? NCH : nch_arg;
   // the specialised kernels are launched on dense matrices only: the row strides are constants as well
   if (NCH) {
@@ -509,6 +512,7 @@ __device__ __forceinline__ void rows_mma_k4(float (&d)[4], const unsigned (&a)[2
 
 // W [K][cin][cout] -> image [K][cout / 8][32] of (hi, lo) of W[k][t][8 nt + g], zero for t >= cin
 __global__ void k_rows_thin_prepare(const float *__restrict__ w, uint2 *__restrict__ img, int K, int cin, int cout) {
+  SCN_GRID_WAIT();
   const int nt_n = cout / 8;
   const long long total = (long long)K * nt_n * 32;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -526,6 +530,7 @@ k_conv_rows_thin(const float *__restrict__ in, long long n_in, float *__restrict
                  const uint2 *__restrict__ img, const float *__restrict__ bias, const float *__restrict__ bn_scale,
                  const float *__restrict__ bn_shift, float leak, const int *__restrict__ nbr, int K, int cin,
                  int *flags) {
+  SCN_GRID_WAIT();
   constexpr unsigned kFull = 0xffffffffu;
   constexpr int kGroup = 4;  // offsets in flight
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -623,6 +628,7 @@ k_conv_rows_thin(const float *__restrict__ in, long long n_in, float *__restrict
 // (which is bound by the issue rate of those: 0.27 ms for 1.59 M rows, 27 offsets, 3 -> 32 planes; this form
 // 0.21 ms, bound by its scalar loads of the input values).
 __global__ void k_rows_thin_prepare_b3(const float *__restrict__ w, uint4 *__restrict__ img, int K, int cin, int cout) {
+  SCN_GRID_WAIT();
   const int nt_n = cout / 8, n_groups = (K + 3) / 4;
   const long long total = (long long)n_groups * nt_n * 32;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -649,6 +655,7 @@ k_conv_rows_thin_b3(const float *__restrict__ in, long long n_in, float *__restr
                     const uint4 *__restrict__ img, const float *__restrict__ bias, const float *__restrict__ bn_scale,
                     const float *__restrict__ bn_shift, float leak, const int *__restrict__ nbr, int K, int cin,
                     int *flags) {
+  SCN_GRID_WAIT();
   constexpr unsigned kFull = 0xffffffffu;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const long long row0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
@@ -814,6 +821,7 @@ k_conv_rows_scatter(const float *__restrict__ in, int ld_in, long long n_in, flo
                     long long n_out, const uint4 *__restrict__ img, const float *__restrict__ bias,
                     const float *__restrict__ bn_scale, const float *__restrict__ bn_shift, float leak,
                     const int *__restrict__ child_of /* [K][n_in] -> output row */, int K, int nch_arg, int *flags) {
+  SCN_GRID_WAIT();
   const int nch = NCH ? NCH : nch_arg;
   if (NCH) {  // dense matrices: constant row strides
     ld_in = NCH * kRChunk;

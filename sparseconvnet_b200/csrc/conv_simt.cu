@@ -49,6 +49,7 @@ k_conv_simt(const float *__restrict__ in, int ld_in, long long n_in, float *__re
             int ld_out, long long n_out, const float *__restrict__ weight, long long w_offset_stride,
             long long w_group_stride, const float *__restrict__ bias, const int *__restrict__ nbr,
             int K, int cin, int cout, int vec_in, int vec_w, int *flags) {
+  SCN_GRID_WAIT();
   constexpr int PM = BN / 8;                // pairs per thread
   constexpr int TXN = BN / 4;               // threads across the output planes
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(128)
 k_conv_thin(const float *__restrict__ in, int ld_in, long long n_in, float *__restrict__ out, int ld_out,
             long long n_out, const float *__restrict__ weight, const float *__restrict__ bias,
             const int *__restrict__ nbr, int K, int cin, int cout, int *flags) {
+  SCN_GRID_WAIT();
   extern __shared__ __align__(16) float w_s[];  // [K][cin][32]: planes n0 .. n0+31 of this CTA, zero padded
   const int n0 = blockIdx.y * kThinPlanes;
   for (int i = threadIdx.x; i < K * cin * kThinPlanes; i += blockDim.x) {

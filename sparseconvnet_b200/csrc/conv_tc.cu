@@ -72,6 +72,7 @@ __host__ __device__ inline unsigned instr_desc(bool bf16) {
 // ---------------------------------------------------------------------------------------------
 __global__ void k_prepare_weights(const float *__restrict__ w, unsigned char *__restrict__ out, int K, int cin,
                                   int cout, int kc, int mode) {
+  SCN_GRID_WAIT();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long total = (long long)K * cin * cout;
   if (idx >= total) return;
@@ -157,6 +158,7 @@ __device__ __forceinline__ void cp_async_wait_dyn(int n) {
 //   acc_full   tcgen05.commit after the last MMA of the tile
 template <int MODE>
 __global__ void __launch_bounds__(kTcThreads) k_conv_tc(TcParams P) {
+  SCN_GRID_WAIT();
   constexpr bool kBf16 = (MODE == TC_BF16 || MODE == TC_BF16X3);     // operands are bf16, converted while staging
   constexpr bool kSplit = (MODE == TC_TF32X3 || MODE == TC_BF16X3);  // two parts per operand, three products
   constexpr int kEsize = kBf16 ? 2 : 4;
@@ -571,6 +573,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(TcParams P) {
 __global__ void k_sum_partials(const float4 *__restrict__ partial, int n_split, long long n4, const float *__restrict__ bias,
                                const float *__restrict__ bn_scale, const float *__restrict__ bn_shift, float leak,
                                int cout, float4 *__restrict__ out) {
+  SCN_GRID_WAIT();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n4) return;
   const int plane = (int)((i * 4) % cout);

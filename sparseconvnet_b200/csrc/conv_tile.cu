@@ -161,6 +161,7 @@ __device__ __forceinline__ int item_offsets(const TileParams &P, long long item)
 
 template <int TERMS, int SP, bool OUT_SPLIT>
 __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
+  SCN_GRID_WAIT();
   using Shape = TileShape<TERMS, SP>;
   constexpr int PP = Shape::PP, NI = Shape::NI, PARTS = Shape::PARTS;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -526,6 +527,7 @@ __global__ void __launch_bounds__(256)
 k_tile_sum(const float4 *__restrict__ partial, int n_split, long long n_pos, int cout4, const int *__restrict__ order,
            long long n_out, const float *__restrict__ bias, const float *__restrict__ bn_scale, const float *__restrict__ bn_shift,
            float leak, float4 *__restrict__ out, unsigned char *__restrict__ out_split, int out_sp, int parts) {
+  SCN_GRID_WAIT();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_pos * cout4) return;
   const int c = (int)(i % cout4);
@@ -567,6 +569,7 @@ __global__ void __launch_bounds__(256)
 k_tile_split(const float *__restrict__ in, unsigned char *__restrict__ out, long long n_pieces, int cin, int ppr, int SP,
              const float *__restrict__ pre_scale, const float *__restrict__ pre_shift, float pre_leak,
              const float *__restrict__ in_b, int planes_a) {
+  SCN_GRID_WAIT();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_pieces) return;
   const long long row = idx / ppr;
@@ -600,6 +603,7 @@ k_tile_split(const float *__restrict__ in, unsigned char *__restrict__ out, long
 // W [K][cin][cout] -> [K][slice][part][coutp x SP] bf16 in the K-major core-matrix layout of the MMA's B operand
 __global__ void k_tile_weights(const float *__restrict__ w, unsigned char *__restrict__ out, int K, int cin, int cout,
                                int coutp, int n_slices, int SP, int parts) {
+  SCN_GRID_WAIT();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int cp = n_slices * SP;
   if (idx >= (long long)K * cp * coutp) return;

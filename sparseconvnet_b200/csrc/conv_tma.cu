@@ -88,6 +88,7 @@ __host__ __device__ inline unsigned instr_desc_tma(bool bf16) {
 template <int MODE, bool TMA_GATHER>
 __global__ void __launch_bounds__(N_WARPS * 32, 1)
 k_conv_tma(const __grid_constant__ CUtensorMap in_map, TmaParams P) {
+  SCN_GRID_WAIT();
   constexpr bool kBf16 = (MODE == TC_BF16 || MODE == TC_BF16X3);     // bf16 operands, made by the transform warps
   constexpr bool kSplit = (MODE == TC_TF32X3 || MODE == TC_BF16X3);  // two parts per operand, three products
   constexpr bool kB3 = (MODE == TC_BF16X3);

@@ -91,6 +91,7 @@ __host__ __device__ inline unsigned wide_idesc(int rows) {
 // 1.5 M rows).
 template <int TERMS, int ROWS, int PW, int TRC>
 __global__ void __launch_bounds__((PW + 5) * 32, 1) k_conv_wide(WideParams P) {
+  SCN_GRID_WAIT();
   constexpr int kWProducerWarps = PW, kWProducers = PW * 32;
   constexpr int kWEpilogue0 = PW, kWMmaWarp = PW + 4;
   constexpr unsigned kTmemCols = 512u;
@@ -430,6 +431,7 @@ __global__ void __launch_bounds__(256)
 k_wide_split_rows(const float *__restrict__ in, unsigned char *__restrict__ out, long long n_pieces, int cin,
                   const float *__restrict__ pre_scale, const float *__restrict__ pre_shift, float pre_leak,
                   const float *__restrict__ in_b, int planes_a) {
+  SCN_GRID_WAIT();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_pieces) return;
   const int ppr = cin / 8;  // pieces per row

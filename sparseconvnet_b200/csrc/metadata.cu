@@ -109,6 +109,7 @@ static void fill_add(Fills &f, void *p, size_t bytes, bool ones) {
 }
 
 __global__ void __launch_bounds__(256) k_fill(const __grid_constant__ Fills f) {
+  SCN_GRID_WAIT();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
   for (int a = 0; a < f.count; ++a) {
     const int v = (((a < 32 ? f.ones : f.ones_hi) >> (a & 31)) & 1u) ? -1 : 0;
@@ -270,6 +271,7 @@ static void count_ticket_zero(Rulebook &rb) {  // nothing will be launched: no r
 }
 
 __global__ void k_post_flags(int *flags_dev, volatile int *mailbox) {
+  SCN_GRID_WAIT();
   mailbox[0] = *flags_dev;
   *flags_dev = 0;
   __threadfence_system();
@@ -404,6 +406,7 @@ __global__ void k_insert_input(KeyLayout L, HashTable T, const long long *__rest
                                long long n, int ncols, int mode, long long bl_length,
                                unsigned long long *__restrict__ row_keys, int *__restrict__ slot_of,
                                int *flags, int *n_samples) {
+  SCN_GRID_WAIT();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   unsigned long long key = kEmptyKey;
@@ -460,6 +463,7 @@ __global__ void k_insert_input(KeyLayout L, HashTable T, const long long *__rest
 __global__ void __launch_bounds__(256)
 k_blank_overwritten(const Slot *__restrict__ slots, const int *__restrict__ slot_of, long long n,
                     unsigned long long *__restrict__ row_keys, int *flags, const int *n_samples, HostPost post) {
+  SCN_GRID_WAIT();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) post_to_host(post, flags, true, 0, n_samples);
   if (i >= n) return;
@@ -493,6 +497,7 @@ __global__ void __launch_bounds__(256)
 k_first_ranks(const Slot *__restrict__ slots, const int *__restrict__ slot_of, long long n_in, const int *__restrict__ n_in_dev,
               int per_site, uint2 *__restrict__ words, int *base, int *done, int *total_dev, int *flags, bool clear_flags,
               const int *extra, HostPost post) {
+  SCN_GRID_WAIT();
   __shared__ unsigned sh_bits[32];
   __shared__ int sh_sum[8];
   __shared__ bool last;
@@ -581,6 +586,7 @@ k_first_ranks(const Slot *__restrict__ slots, const int *__restrict__ slot_of, l
 // the DRAM's random-access rate: 198 us against 142 us for the inserts themselves at 1.6 M sites.
 __global__ void k_number_slots(Slot *slots, long long n_slots, const uint2 *__restrict__ words,
                                const int *__restrict__ base, unsigned long long *__restrict__ row_keys) {
+  SCN_GRID_WAIT();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_slots) return;
   const uint4 v = *reinterpret_cast<const uint4 *>(slots + idx);
@@ -593,6 +599,7 @@ __global__ void k_number_slots(Slot *slots, long long n_slots, const uint2 *__re
 
 __global__ void k_count_per_site(const Slot *__restrict__ slots, const int *__restrict__ slot_of,
                                  long long n, int *cnt) {
+  SCN_GRID_WAIT();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int s = slot_of[i];
@@ -602,6 +609,7 @@ __global__ void k_count_per_site(const Slot *__restrict__ slots, const int *__re
 __global__ void k_fill_per_site(const Slot *__restrict__ slots, const int *__restrict__ slot_of,
                                 long long n, const int *__restrict__ start, int *cursor,
                                 int *__restrict__ csr_rows) {
+  SCN_GRID_WAIT();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int s = slot_of[i];
@@ -614,6 +622,7 @@ __global__ void k_fill_per_site(const Slot *__restrict__ slots, const int *__res
 // Puts the input rows of every site in ascending order (heap sort, in place, one thread per
 // site; sites with duplicates hold a handful of rows).
 __global__ void k_sort_segments(const int *__restrict__ start, long long n_sites, int *csr_rows) {
+  SCN_GRID_WAIT();
   long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n_sites) return;
   int *a = csr_rows + start[r];
@@ -828,6 +837,7 @@ static int md_input_layer(scn_metadata *md, const int64_t *spatial_size, const i
 // rows reachable from the maps).
 __global__ void k_spatial_locations(KeyLayout L, const unsigned long long *__restrict__ row_keys,
                                     long long n, long long *__restrict__ out) {
+  SCN_GRID_WAIT();
   long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   unsigned long long key = row_keys[r];
@@ -880,6 +890,7 @@ k_submanifold_rules(KeyLayout L, HashTable T, const unsigned long long *__restri
                     long long n, int K, FilterDesc F, int k_chunk, int *__restrict__ nbr,
                     unsigned long long *counts, int mirrored, unsigned *__restrict__ masks, int mask_words,
                     volatile unsigned long long *counts_host) {
+  SCN_GRID_WAIT();
   constexpr int kDim = DIM ? DIM : kMaxDim, kAhead = DIM == 4 ? 2 : 1;
   __shared__ long long sh_keydelta[32];
   __shared__ int sh_count[32];
@@ -982,6 +993,7 @@ k_submanifold_rules(KeyLayout L, HashTable T, const unsigned long long *__restri
 // What a submanifold rulebook starts from, in one launch: counts and masks zero, the mirrored half of the table empty.
 __global__ void __launch_bounds__(256)
 k_rules_init(unsigned long long *counts, int n_counts, unsigned *masks, long long n_masks, int *nbr, long long n_nbr) {
+  SCN_GRID_WAIT();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
   for (long long j = i; j < n_counts; j += step) counts[j] = 0;
   for (long long j = i; j < n_masks; j += step) masks[j] = 0;
@@ -1106,6 +1118,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256)
 k_strided_insert(KeyLayout Lin, KeyLayout Lout, FilterDesc F, HashTable Tout, const unsigned long long *__restrict__ in_keys,
                  long long n_in, const int *__restrict__ n_in_dev, int *__restrict__ slot_of, int *flags) {
+  SCN_GRID_WAIT();
   const unsigned id = blockIdx.x * blockDim.x + threadIdx.x;  // (fewer than 2^31 candidates)
   if (id >= sites_here(n_in_dev, n_in) * F.tmax) return;
   const unsigned i = F.tmax == 1 ? id : id / (unsigned)F.tmax;
@@ -1144,6 +1157,7 @@ k_strided_fill(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Slot *slots, const u
                const int *__restrict__ n_out_dev, long long capacity, const uint2 *__restrict__ words,
                const int *__restrict__ base, unsigned long long *__restrict__ row_keys, int *__restrict__ nbr,
                unsigned long long *counts, int K, volatile unsigned long long *counts_host) {
+  SCN_GRID_WAIT();
   __shared__ int sh_count[kFillCounts];
   const bool shared = K <= kFillCounts;
   if (shared)
@@ -1792,6 +1806,7 @@ int rulebook_counts(Rulebook &rb, cudaStream_t stream) {
 
 __global__ void k_transpose_rules(const int *__restrict__ nbr, long long n_out, long long n_in, int K,
                                   int *__restrict__ tnbr) {
+  SCN_GRID_WAIT();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)K * n_out) return;
   int i = nbr[idx];
@@ -1814,11 +1829,13 @@ int rulebook_transposed(Rulebook &rb, cudaStream_t stream) {
 }
 
 __global__ void k_rule_flags(const int *__restrict__ nbr, long long total, int *__restrict__ flag) {
+  SCN_GRID_WAIT();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < total) flag[idx] = nbr[idx] >= 0;
 }
 __global__ void k_rule_compact(const int *__restrict__ nbr, const int *__restrict__ pos, long long total,
                                long long n_out, int *__restrict__ pairs) {
+  SCN_GRID_WAIT();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   int i = nbr[idx];

@@ -14,6 +14,7 @@ namespace scn {
 __global__ void k_input_features(const float *__restrict__ in, float *__restrict__ out,
                                  const int *__restrict__ start, const int *__restrict__ rows,
                                  long long n_out, int C, int mode) {
+  SCN_GRID_WAIT();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_out * C) return;
   long long r = idx / C;
@@ -38,6 +39,7 @@ __global__ void k_input_features(const float *__restrict__ in, float *__restrict
 __global__ void k_output_features(const float *__restrict__ in, float *__restrict__ out,
                                   const int *__restrict__ start, const int *__restrict__ rows,
                                   long long n_sites, int C, int mode, int scale_mean) {
+  SCN_GRID_WAIT();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_sites * C) return;
   long long r = idx / C;
@@ -63,6 +65,7 @@ __global__ void k_output_features(const float *__restrict__ in, float *__restric
 __global__ void __launch_bounds__(256)
 k_bn_stats(const float *__restrict__ in, long long n_rows, int C, long long in_stride,
            double *__restrict__ sums /* [2][C] */) {
+  SCN_GRID_WAIT();
   __shared__ float sh_s[8][33], sh_q[8][33];
   int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
   int c = blockIdx.x * 32 + lane;
@@ -91,6 +94,7 @@ k_bn_stats(const float *__restrict__ in, long long n_rows, int C, long long in_s
 // in flight.  Bound by HBM: the 14 layers of a U-Net training step on 400 k points 165 us (198 with one value per load).
 __global__ void __launch_bounds__(256)
 k_bn_stats4(const float *__restrict__ in, int n_rows, int C, int in_stride, double *__restrict__ sums /* [2][C] */) {
+  SCN_GRID_WAIT();
   __shared__ float sh[2][8][33];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
   const int q = lane & 7, c = blockIdx.x * 32 + q * 4;
@@ -150,7 +154,8 @@ static void launch_bn_stats(const float *in, long long n_rows, int C, long long 
 __global__ void k_bn_finalize(int C, long long n_rows, const double *__restrict__ sums,
                               float *save_mean, float *save_invstd, float *running_mean,
                               float *running_var, float eps, float momentum, int train,
-                              int count_follows_sums = 0) {
+                              int count_follows_sums) {
+  SCN_GRID_WAIT();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   if (count_follows_sums) {  // the row count of all devices, summed along with the array
@@ -180,6 +185,7 @@ k_bn_apply(const float *__restrict__ in, float *__restrict__ out, long long n_ro
            long long in_stride, long long out_stride, float *save_mean, float *save_invstd,
            const float *__restrict__ running_mean, const float *__restrict__ running_var, float eps,
            const float *__restrict__ weight, const float *__restrict__ bias, float leak) {
+  SCN_GRID_WAIT();
   extern __shared__ float sh_wb[];  // [2][C]
   for (int c = threadIdx.x; c < C; c += blockDim.x) {
     float mean, invstd;
@@ -237,6 +243,7 @@ k_bn_back_sums(const float *__restrict__ in, const float *__restrict__ out, cons
                long long n_rows, int C, long long in_stride, long long out_stride,
                const float *__restrict__ mean, float leak, long long chunk_rows,
                double *__restrict__ partial /* [chunks][2][C] */) {
+  SCN_GRID_WAIT();
   __shared__ double sh_s[8][33], sh_q[8][33];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -288,6 +295,7 @@ __global__ void __launch_bounds__(256)
 k_bn_back_sums4(const float *__restrict__ in, const float *__restrict__ out, const float *__restrict__ d_out, int n_rows, int C,
                 int in_stride, int out_stride, const float *__restrict__ mean, float leak, int chunk_rows,
                 double *__restrict__ partial /* [chunks][2][C] */) {
+  SCN_GRID_WAIT();
   __shared__ double sh[2][8][33];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
   const int lq = lane & 7, c = blockIdx.x * 32 + lq * 4;
@@ -372,6 +380,7 @@ __global__ void __launch_bounds__(256)
 k_bn_back_finalize(const double *__restrict__ partial, int chunks, int C, long long n_rows,
                    const float *__restrict__ invstd, float *__restrict__ d_weight, float *__restrict__ d_bias,
                    float *__restrict__ coef /* [2][C] */) {
+  SCN_GRID_WAIT();
   const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (c >= C) return;
   double s, q;
@@ -388,6 +397,7 @@ k_bn_back_finalize(const double *__restrict__ partial, int chunks, int C, long l
 // added in their fixed order ...
 __global__ void __launch_bounds__(256)
 k_bn_back_reduce(const double *__restrict__ partial, int chunks, int C, double *__restrict__ sums) {
+  SCN_GRID_WAIT();
   const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (c >= C) return;
   double s, q;
@@ -403,6 +413,7 @@ __global__ void k_bn_back_coef(const double *__restrict__ local, const double *_
                                long long n_rows_total, const float *__restrict__ invstd,
                                float *__restrict__ d_weight, float *__restrict__ d_bias,
                                float *__restrict__ coef /* [2][C] */) {
+  SCN_GRID_WAIT();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   if (n_rows_total < 0) n_rows_total = (long long)total[2 * C];  // summed along with the array
@@ -419,6 +430,7 @@ k_bn_back_apply(const float *__restrict__ in, float *__restrict__ d_in, const fl
                 const float *__restrict__ d_out, long long n_rows, int C, long long in_stride,
                 long long out_stride, const float *__restrict__ mean, const float *__restrict__ invstd,
                 const float *__restrict__ weight, const float *__restrict__ coef, float leak) {
+  SCN_GRID_WAIT();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_rows * C) return;
   const long long r = idx / C;
@@ -434,6 +446,7 @@ __global__ void __launch_bounds__(256)
 k_bn_back_apply4(const float4 *__restrict__ in, float4 *__restrict__ d_in, const float4 *__restrict__ out,
                  const float4 *__restrict__ d_out, unsigned n4, unsigned C4, const float *__restrict__ mean,
                  const float *__restrict__ invstd, const float *__restrict__ weight, const float *__restrict__ coef, float leak) {
+  SCN_GRID_WAIT();
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n4) return;
   const int c = (int)(i % C4) * 4, C = (int)C4 * 4;
@@ -469,6 +482,7 @@ static void launch_bn_back_apply(const float *in, float *d_in, const float *out,
 __global__ void __launch_bounds__(256)
 k_max_pool(const float *__restrict__ in, float *__restrict__ out, const int *__restrict__ nbr,
            long long n_out, long long n_in, int K, int C_out, int in_stride, int drop, int *flags) {
+  SCN_GRID_WAIT();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_out * C_out) return;
   long long o = idx / C_out;
@@ -498,6 +512,7 @@ template <bool AVERAGE>
 __global__ void __launch_bounds__(256)
 k_sum_pool(const float *__restrict__ in, float *__restrict__ out, const int *__restrict__ nbr,
            long long n_out, long long n_in, int K, int C_out, int in_stride, int drop, int *flags) {
+  SCN_GRID_WAIT();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_out * C_out) return;
   long long o = idx / C_out;
@@ -524,6 +539,7 @@ __global__ void __launch_bounds__(256)
 k_sparse_to_dense(KeyLayout L, const unsigned long long *__restrict__ row_keys,
                   const float *__restrict__ in, float *__restrict__ out, long long n_rows, int C,
                   long long volume) {
+  SCN_GRID_WAIT();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_rows * C) return;
   long long r = idx / C;
@@ -551,6 +567,7 @@ __global__ void __launch_bounds__(256)
 k_pool_backward(const float *__restrict__ in, float *__restrict__ d_in, const float *__restrict__ out,
                 const float *__restrict__ d_out, const int *__restrict__ table, long long n_rows,
                 long long n_other, int K, int C_in, int drop, int *flags) {
+  SCN_GRID_WAIT();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_rows * C_in) return;
   const long long i = idx / C_in;
@@ -587,6 +604,7 @@ __global__ void __launch_bounds__(256)
 k_dense_to_sparse_grad(KeyLayout L, const unsigned long long *__restrict__ row_keys,
                        const float *__restrict__ d_dense, float *__restrict__ d_in, long long n_rows, int C,
                        long long volume) {
+  SCN_GRID_WAIT();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_rows * C) return;
   long long r = idx / C;
@@ -620,6 +638,7 @@ template <int COUT4>
 __global__ void __launch_bounds__(256)
 k_rows_affine(const float *__restrict__ in, float *__restrict__ out, long long n_rows, int cin, int cout,
               const float *__restrict__ weight, const float *__restrict__ bias) {
+  SCN_GRID_WAIT();
   extern __shared__ float4 sh_w4[];  // [cin][COUT4], then one [32][kAffineStride] tile per warp
   float *sh_w = reinterpret_cast<float *>(sh_w4);
   constexpr int CP = COUT4 * 4;
@@ -756,7 +775,7 @@ int scn_batchnorm_forward(const float *in_features, float *out_features, int64_t
     launch_bn_stats(in_features, n_rows, n_planes, in_stride, sums, stream);
   }
   if (train)
-    SCN_LAUNCH(k_bn_finalize, (unsigned)ceil_div(n_planes, 128), 128, 0, stream, n_planes, n_rows, sums, save_mean, save_invstd, running_mean, running_var, (float)eps, (float)momentum, train);
+    SCN_LAUNCH(k_bn_finalize, (unsigned)ceil_div(n_planes, 128), 128, 0, stream, n_planes, n_rows, sums, save_mean, save_invstd, running_mean, running_var, (float)eps, (float)momentum, train, 0);
   const float *rm = train ? nullptr : running_mean, *rv = train ? nullptr : running_var;
   bool vec4 = (n_planes % 4 == 0) && (in_stride % 4 == 0) && (out_stride % 4 == 0) &&
               ((uintptr_t)in_features % 16 == 0) && ((uintptr_t)out_features % 16 == 0);
@@ -779,6 +798,7 @@ __global__ void __launch_bounds__(256)
 k_bn_apply_join(const float *__restrict__ a, int ca, const float *__restrict__ b, int cb, float *__restrict__ out,
                 long long n_rows, const float *__restrict__ running_mean, const float *__restrict__ running_var,
                 float eps, const float *__restrict__ weight, const float *__restrict__ bias, float leak) {
+  SCN_GRID_WAIT();
   extern __shared__ float sh_wb[];  // [2][ca + cb]
   const int C = ca + cb;
   for (int c = threadIdx.x; c < C; c += blockDim.x) {

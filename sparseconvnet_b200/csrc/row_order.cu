@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(kThreads)
 k_order_keys(const int *__restrict__ nbr, const unsigned *__restrict__ known, long long n, int K, KeyBits<KEY> B,
              int rows_per_block, int R, KEY *__restrict__ keys, unsigned *__restrict__ masks,
              int *__restrict__ block_count, int *__restrict__ total) {
+  SCN_GRID_WAIT();
   __shared__ int h[kMaxDigit];
   for (int i = threadIdx.x; i < R; i += kThreads) h[i] = 0;
   __syncthreads();
@@ -93,6 +94,7 @@ template <typename KEY>
 __global__ void __launch_bounds__(kThreads)
 k_order_count(const KEY *__restrict__ keys, long long n, int rows_per_block, int shift, int R,
               int *__restrict__ block_count, int *__restrict__ total) {
+  SCN_GRID_WAIT();
   __shared__ int h[kMaxDigit];
   for (int i = threadIdx.x; i < R; i += kThreads) h[i] = 0;
   __syncthreads();
@@ -110,6 +112,7 @@ __global__ void __launch_bounds__(kThreads)
 k_order_scatter(const KEY *__restrict__ keys, const int *__restrict__ rows_in, long long n, int rows_per_block,
                 int shift, int R, const int *__restrict__ block_count, const int *__restrict__ total,
                 KEY *__restrict__ keys_out, int *__restrict__ rows_out) {
+  SCN_GRID_WAIT();
   __shared__ unsigned short cnt[kWarps][kMaxDigit];  // rows of digit d in warp w's segment, then in the warps before it
   __shared__ int base[kMaxDigit], part[kMaxDigit];   // (a block has fewer than 65536 rows)
   __shared__ int warp_sum[kWarps];
@@ -177,6 +180,7 @@ k_order_scatter(const KEY *__restrict__ keys, const int *__restrict__ rows_in, l
 __global__ void __launch_bounds__(kTile)
 k_order_plain(const int *__restrict__ nbr, long long n, int K, int words, int *__restrict__ order,
               unsigned *__restrict__ tile_bits, int *__restrict__ packed) {
+  SCN_GRID_WAIT();
   __shared__ unsigned bits[4];
   const long long t = blockIdx.x, p = t * kTile + threadIdx.x;
   if (threadIdx.x < 4) bits[threadIdx.x] = 0;
@@ -329,6 +333,7 @@ template <int WORDS>
 __global__ void __launch_bounds__(256)
 k_order_tiles(int *__restrict__ order, long long n, int K, const int *__restrict__ nbr, const unsigned *__restrict__ masks,
               unsigned *tile_bits, int *__restrict__ packed, long long n_tiles, int *by_work, int *done) {
+  SCN_GRID_WAIT();
   const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t < n_tiles) pack_tile<WORDS>(order, n, K, nbr, masks, tile_bits, packed, t, lane);

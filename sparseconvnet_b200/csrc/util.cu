@@ -239,6 +239,7 @@ __device__ inline int block_exclusive_scan(int v, int &block_total) {
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_tile_sums(const int *in, int *tile_sums,
                                                                  long long n) {
+  SCN_GRID_WAIT();
   __shared__ int total;
   long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
   int s = 0;
@@ -252,6 +253,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tile_sums(const int *in, 
 __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int *in, int *out,
                                                              const int *tile_base, long long n,
                                                              int *total_dev) {
+  SCN_GRID_WAIT();
   __shared__ int total;
   long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
   int v[kScanItems];
@@ -271,7 +273,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int *in, int 
     *total_dev = total + (tile_base ? tile_base[blockIdx.x] : 0);
 }
 
-__global__ void k_set_zero(int *p) { *p = 0; }
+__global__ void k_set_zero(int *p) {
+  SCN_GRID_WAIT(); *p = 0; }
 
 int exclusive_scan_i32(const int *in, int *out, long long n, int *total_dev, cudaStream_t stream) {
   if (n <= 0) {
