@@ -63,7 +63,10 @@ enum scn_status {
 
 /* arithmetic used inside the convolution kernels */
 enum scn_precision {
-  SCN_PRECISION_FP32 = 0, /* fp32 FMA, fp32 accumulate (matches the reference's float path)  */
+  SCN_PRECISION_FP32 = 0, /* fp32 operands and sums (matches the reference's float path): fp32 FMA, or on the tensor
+                             cores with every operand as three bf16 parts, which hold it exactly, the six largest products
+                             of the parts and fp32 sums -- a smaller error than the FMA chain's.  Non-finite and extreme
+                             values are multiplied as plain fp32 */
   SCN_PRECISION_TF32 = 1, /* at least one tf32 product, fp32 accumulate.  k_conv_tile computes it as
                              SCN_PRECISION_TF32X3, which is more accurate and takes it no longer; the
                              older kernels behind it issue one tf32 product                         */
@@ -83,7 +86,7 @@ enum scn_conv_kernel {
   SCN_KERNEL_CONV_ROWS = 4,          /* k_conv_rows and its first-layer forms: row-stationary, warp-level mma.sync */
   SCN_KERNEL_CONV_WIDE = 5,          /* k_conv_wide: tcgen05, persistent, rows split to bf16 parts once per call and copied in by cp.async */
   SCN_KERNEL_CONV_TILE = 6,          /* k_conv_tile: tcgen05, persistent, mask-sorted row tiles */
-  SCN_KERNEL_CONV_FMA = 7            /* k_conv_fma: fp32 FMA, mask-sorted row tiles           */
+  SCN_KERNEL_CONV_FMA = 7            /* fp32 on mask-sorted row tiles: k_conv_fma, or k_conv_six (scn_last_conv_six) */
 };
 /* which kernel the last weight gradient of a convolution ran, whatever thread asked for it (autograd has its own) */
 enum scn_dweight_kernel {
@@ -250,6 +253,8 @@ SCN_API int scn_md_rulebook_export(scn_metadata *md, int kind, const int64_t *si
 /* -1 before the first convolution, else an scn_conv_kernel value.  No counterpart in the
  * reference; lets a profiler attribute a call's time to the kernel that ran it. */
 SCN_API int scn_last_conv_kernel(void);
+/* 1 if the last convolution call of this thread ran on k_conv_six (fp32 by six bf16 products on tcgen05) */
+SCN_API int scn_last_conv_six(void);
 SCN_API int scn_last_dweight_kernel(void);
 
 /* Self-calibration of the tensor path.  No counterpart in the reference.  Issues `n_mma`

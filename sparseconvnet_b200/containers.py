@@ -82,7 +82,7 @@ class Sequential(torch.nn.Sequential):
     a convolution whose output goes straight into an eval-mode BatchNormalization (possibly across
     the boundary of a nested Sequential, as in the U-Net's blocks) applies that layer's scale, shift
     and leaky ReLU in its own store; an eval-mode BatchNormalization in front of a strided Convolution
-    (or of a SubmanifoldConvolution on the tensor cores) is applied by that convolution to its input; JoinTable -> BatchNormalization ->
+    (or of a SubmanifoldConvolution) is applied by that convolution to its input; JoinTable -> BatchNormalization ->
     SubmanifoldConvolution is one call on the tensors that would have been joined; a JoinTable
     followed by a BatchNormalization alone is one pass without the concatenation.
 
@@ -135,11 +135,10 @@ class Sequential(torch.nn.Sequential):
                                     want_split=_wants_split(nxt, steps[after] if after < n else None))
                 i = after
                 continue
-            # the same in front of a SubmanifoldConvolution on the tensor cores, which has that pass (a residual block: the
-            # sum in front of the BatchNormalization is needed as it is as well)
+            # the same in front of a SubmanifoldConvolution (a residual block: the sum in front of the BatchNormalization is
+            # needed as it is as well)
             if (Sequential.fuse and isinstance(m, layers.BatchNormalization) and type(nxt) is layers.SubmanifoldConvolution
-                    and nxt.groups == 1 and layers.SCN._precision != layers.SCN.PRECISION_FP32 and nxt.nIn % 8 == 0
-                    and nxt.nOut % 8 == 0 and layers.SCN.Profile.active is None
+                    and nxt.groups == 1 and nxt.nIn % 8 == 0 and nxt.nOut % 8 == 0 and layers.SCN.Profile.active is None
                     and not m._forward_hooks and not m._forward_pre_hooks and not nxt._forward_hooks
                     and not nxt._forward_pre_hooks and isinstance(input, SparseConvNetTensor)
                     and input.features.nelement() > 0 and input.features.size(1) == nxt.nIn and m.fusable(input.features)

@@ -64,6 +64,12 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
 bool conv_fma_supported(const float *in, const float *out, const float *weight, const float *bias, int K, int cin, int cout,
                         int groups);
 bool conv_fma_wants_order(long long n_out);
+bool conv_six_takes(const float *in, const float *in_b, int planes_a, const float *out, const float *bias, int K, int cin,
+                    int cout, int groups, long long rows_in, long long rows_out);
+int conv_forward_six(const float *in, long long n_in, float *out, long long n_out, const float *weight, const float *bias,
+                     const float *bn_scale, const float *bn_shift, float leak, const RowOrder &ord, int K, int cin, int cout,
+                     int *flags, cudaStream_t stream, const float *pre_scale, const float *pre_shift, float pre_leak,
+                     const float *in_b, int planes_a);
 int conv_forward_fma(const float *in, long long n_in, float *out, long long n_out, const float *weight, const float *bias,
                      const float *bn_scale, const float *bn_shift, float leak, const int *table, const RowOrder *ord, int K,
                      int cin, int cout, int *flags, cudaStream_t stream);
@@ -83,6 +89,13 @@ static bool tile_enabled(bool narrow) {
     if (getenv(k)) return false;
   if (getenv("SCN_X3_FORM") && getenv("SCN_X3_FORM")[0] == 't') return false;
   return !(narrow && getenv("SCN_X3_ROWS"));
+}
+
+// SCN_CONV_SIX=0 turns the fp32 kernel on tensor cores off, and so does the knob that tunes the one on the FMA pipe.
+static bool six_enabled() {
+  if (!any_knob()) return true;
+  if (getenv("SCN_CONV_SIX")) return atoi(getenv("SCN_CONV_SIX")) != 0;
+  return !getenv("SCN_FMA_SPLIT");
 }
 
 int split_mode_of_env(int dflt) {
@@ -149,6 +162,7 @@ int weight_image_put(WeightImage &img, cudaStream_t stream) {
 }
 
 static thread_local int g_last_kernel = -1;
+static thread_local bool g_last_six = false;  // k_conv_six, which reports as SCN_KERNEL_CONV_FMA
 static std::atomic<int> g_deferred_counts{0};
 std::atomic<int> g_backward_precision{SCN_PRECISION_FP32};  // arithmetic of the input-gradient pass
 
@@ -367,22 +381,35 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
                        float leak, const float *pre_scale, const float *pre_shift, float pre_leak, const float *in_b,
                        int planes_a) {
   const int *table = transposed_table ? rb.tnbr : rb.nbr;
+  g_last_six = false;
   if (tile_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, precision, rows_out)) {
     RowOrder &ord = transposed_table ? rb.torder : rb.order;
     SCN_TRY(rulebook_row_order(rb, table, rows_out, ord, stream));
+    ord.fp32_only = false;
     SCN_TRY(conv_forward_tile(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, ord, rb.n_offsets,
                               cin, cout, precision, flags, stream, pre_scale, pre_shift, pre_leak, in_b, planes_a));
     g_last_kernel = SCN_KERNEL_CONV_TILE;
     return SCN_OK;
   }
-  // fp32: the same tiles on the FMA pipe (first layers of at most four input planes keep their own kernel), unless a
-  // BatchNorm or a join in front has to be applied to a copy of the input first
+  // fp32: the same tiles, on the tensor cores with operands in three parts, or on the FMA pipe (first layers of at most four
+  // input planes keep their own kernel), where a BatchNorm or a join in front is applied to a copy of the input first
   const bool fma = precision == SCN_PRECISION_FP32 && rows_out > 0 && cin > 4 &&
                    conv_fma_supported(in, out, weight, bias, rb.n_offsets, cin, cout, groups) &&
                    !(any_knob() && getenv("SCN_SIMT_BLOCK") && atoi(getenv("SCN_SIMT_BLOCK")) != 0);
   if (!fma)
     return conv_forward_dispatch(in, rows_in, out, rows_out, weight, bias, table, rb.n_offsets, cin, cout, groups, precision,
                                  flags, stream, bn_scale, bn_shift, leak, pre_scale, pre_shift, pre_leak, in_b, planes_a);
+  if (six_enabled() && conv_six_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, rows_in, rows_out)) {
+    RowOrder &ord = transposed_table ? rb.torder : rb.order;
+    const bool there = ord.order != nullptr;
+    SCN_TRY(rulebook_row_order(rb, table, rows_out, ord, stream));
+    if (!there) ord.fp32_only = true;
+    SCN_TRY(conv_forward_six(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, ord, rb.n_offsets, cin, cout,
+                             flags, stream, pre_scale, pre_shift, pre_leak, in_b, planes_a));
+    g_last_kernel = SCN_KERNEL_CONV_FMA;
+    g_last_six = true;
+    return SCN_OK;
+  }
   float *pre_copy = nullptr;
   SCN_TRY(prepared_input(&in, rows_in, cin, groups, pre_scale, pre_shift, pre_leak, in_b, planes_a, &pre_copy, stream));
   RowOrder *ord = nullptr;
@@ -474,6 +501,7 @@ using namespace scn;
 extern "C" {
 
 int scn_last_conv_kernel(void) { return g_last_kernel; }
+int scn_last_conv_six(void) { return g_last_kernel == SCN_KERNEL_CONV_FMA && g_last_six; }
 
 int scn_set_split_rows(const void *in_split, void *out_split) {
   g_split_rows.in = in_split;

@@ -524,12 +524,13 @@ int launch(DwParams &P, const Rulebook &rb, const float *t_rows, const float *g_
 
 // Rows of whole 16-byte pieces and more than 32 planes on one side: 32 x 32 weights are half as much work per gathered
 // byte, and k_conv_dweight_mma takes as long (278 us on 434 k rows).  Both kernels on the others: 64 x 64 on 119 k rows 230
-// and, here, 160 us, 96 x 96 on 49 k 412 and 229, 128 x 128 on 6 k 110 and 79.  Below 2048 rows an order has to be there already.
+// and, here, 160 us, 96 x 96 on 49 k 412 and 229, 128 x 128 on 6 k 110 and 79.  Below 2048 rows an order has to be there
+// already, and not only because an fp32 convolution has made it.
 // Multiples of 32 planes only: the running sums in TMEM cut off where fp32 additions round, 4e-6 of a sum of 100 k products
 // of mixed signs and 8e-6 with one sign.  That is no more than these shapes ever had (5e-6 and 1e-5 with truncated tf32 parts);
 // the others had plain fp32 sums (9e-7, 1.4e-7), which k_conv_dweight_mma matches.
 bool dweight_tile_supported(const float *in, const float *d_out, const Rulebook &rb, int cin, int cout) {
-  return cin % 32 == 0 && cout % 32 == 0 && (rb.n_out >= 2048 || (rb.n_out > 0 && rb.order.order)) && std::max(cin, cout) > 32 && rb.n_offsets <= kOrderMaxOffsets &&
+  return cin % 32 == 0 && cout % 32 == 0 && (rb.n_out >= 2048 || (rb.n_out > 0 && rb.order.order && !rb.order.fp32_only)) && std::max(cin, cout) > 32 && rb.n_offsets <= kOrderMaxOffsets &&
          ((uintptr_t)in | (uintptr_t)d_out) % 16 == 0;
 }
 

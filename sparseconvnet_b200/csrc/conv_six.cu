@@ -1,0 +1,810 @@
+// fp32 sparse convolution on tcgen05 tensor cores over mask-sorted row tiles: results as accurate as fp32 multiply-adds.
+//
+// Same mathematics as the other convolution kernels (the reference's per-offset gather / GEMM / scatter-add is
+// CPU/Convolution.cpp:137-148, CUDA/Convolution.cu:57-233), in the precision of k_conv_fma (conv_fma.cu):
+//   * Every operand is written as the sum of three bf16 values, x = h + m + l: h = bf16(x), m = bf16(x - h), l = bf16(x - h - m).
+//     The three hold the 24 bits of x exactly.  A product is the six terms h h', h m', m h', h l', m m', l h'; what is left
+//     out is below 2^-26 of it, less than an fp32 product is rounded by.
+//   * The tensor core truncates its running sum, so it never runs far: one step of 32 planes of one filter offset is
+//     summed there, the large terms and the small ones in accumulators of their own, and every step's sums are added to
+//     fp32 registers, rounded to nearest (the "drain" warps).
+// Time and error against float64 beside k_conv_fma's: the table at conv_six_takes.
+//
+// The range of bf16 is that of fp32 except at its ends: the low parts of a tiny value would be lost, and an infinity has no
+// low part.  The pass that splits rows and weights leaves the largest magnitude of either; where a product could overflow, or
+// fall to where its parts do not reach, the kernel multiplies plain fp32 values instead (slow_item).
+//
+// Roles (19 or 16 warps, one CTA per SM, persistent), as in k_conv_tile but for the drain:
+//   entries     one thread: a slot per (tile, filter offset with a rule), 512 bytes of input rows from the packed table
+//   producers   8 (5) warps, a step each: 128 rows of 192 bytes ([32 h | 32 m] and [32 l]) by 16-byte cp.async
+//   weights     one thread: one bulk copy of [W_h | W_m | W_l] per step
+//   MMA         up to 80 output planes three instructions per 16 input planes, h (W_h | W_m | W_l), m (W_h | W_m), l W_h, into
+//               three column ranges; above that six, into two ranges (the large terms, the small ones)
+//   drain       8 warps, a row and half of the planes per lane: TMEM -> registers after every step, and after the tile's
+//               last one through shared memory -> bias -> optional BatchNorm -> 16-byte stores, four lanes per row
+// Bound by the copies into shared memory, 24 KB of rows and 6 (32 output planes) to 24 KB (128) of weights per step at about
+// 32 bytes per cycle and SM, against 336 to 768 cycles of tensor work; as multiply-adds the same step is 1 024 to 4 096 cycles
+// of the whole FMA pipe.  Rows split once per call, not once per gather: with fp32 rows (16 KB per step) split by the
+// producers on their way through registers a step took twice as long (32 -> 32 planes on 200 k rows 157 us, 88 with the split
+// pass; 96 -> 96 682 and 309).
+//
+// Every wait is bounded; on expiry the role raises the abort flag, everybody leaves, tensor memory is freed and
+// the host sees FLAG_TC_TIMEOUT through scn_md_poll_errors.
+#include <stdlib.h>
+
+#include <algorithm>
+#include <atomic>
+
+#include "conv_tile.cuh"
+
+namespace scn {
+
+namespace {
+
+constexpr int kRows = kOrderTile;
+constexpr int kDrainWarps = 8;
+constexpr int kSlots = 8;  // offsets the entries run ahead; at least the producing warps (the slots that end the work)
+constexpr int kMaxStages = 12;
+constexpr int kEpiBytes = 32 * 64;   // per drain warp: 32 rows x 16 planes on their way from lanes to whole lines
+constexpr int kRangeWords = 512;     // behind split rows and weight image: largest magnitude (float bits), one per block
+constexpr int kPrepareThreads = 512, kPrepareBlocks = 296;
+
+struct SixParams {
+  const unsigned char *in_split;  // per row and slice of SP planes [SP h | SP m | SP l]
+  const unsigned *in_range;
+  long long row_bytes;
+  long long n_in;
+  float *out;  // n_split == 1: [n_out][cout]; else partial sums [n_split][n_tiles * 128][cout]
+  int cout, cb, n_cb;  // output planes; planes of a column block (a multiple of 16, at most 128); column blocks
+  const unsigned char *wprep;  // [K][column block][slice][h, m, l]
+  const unsigned *w_range;
+  const float *bias, *bn_scale, *bn_shift;
+  float leak;
+  const int *order, *packed, *by_work;
+  const unsigned *tile_bits;
+  int words;
+  int K, n_slices, log2_terms;  // log2_terms: of the products of a sum, rounded up
+  int n_stages;
+  long long n_tiles, n_items;
+  int n_split;
+  // for slow_item: the operands as they are
+  const float *in, *in_b, *weight, *pre_scale, *pre_shift;
+  float pre_leak;
+  int cin, planes_a;
+  int drop;  // test hook: leave out one barrier arrival of the first CTA
+  int *flags;
+};
+
+// Warps by role.  With 64 planes per drain lane (and weights that leave room for four or five stages) fewer producers, for
+// 128 registers a thread.
+template <int NA>
+struct SixWarps {
+  static constexpr int PROD = NA == 64 ? 5 : 8;
+  static constexpr int DRAIN0 = PROD, MMA = DRAIN0 + kDrainWarps, WGT = MMA + 1, ENTRIES = MMA + 2, THREADS = (ENTRIES + 1) * 32;
+};
+
+template <int SP>
+struct SixShape {
+  static constexpr unsigned HM = SP * 4, L = SP * 2;  // bytes of a row of a stage: [h | m], and [l]
+  static constexpr unsigned A_BYTES = kRows * (HM + L);
+  static constexpr int PIECES = HM / 16, NI = kRows / (32 / PIECES);     // 16-byte pieces per row, rows per lane
+  static constexpr int L_PIECES = L / 16, L_NI = kRows / (32 / L_PIECES);
+  static_assert(HM == 128 || HM == 64, "swizzled rows");
+};
+
+struct Ctl {
+  unsigned long long full[kMaxStages], empty[kMaxStages];  // rows and weights landed; MMAs done
+  unsigned long long s_full[kSlots], s_empty[kSlots], acc_full[4], acc_empty[4];
+  int slot_k[kSlots];  // filter offset + (column block << 10); -1: no more work; + kNoRules: offset 0 with rows of zeros
+  unsigned tmem, range[2];
+  int abort;
+};
+
+struct Item {
+  long long tile;
+  int part, block;
+};
+__device__ __forceinline__ Item item_at(const SixParams &P, long long item) {
+  const int per = P.n_split * P.n_cb, rest = (int)(item % per);
+  const long long i = item / per;
+  return Item{P.by_work ? (long long)__ldg(P.by_work + i) : P.n_tiles - 1 - i, rest / P.n_cb, rest % P.n_cb};
+}
+
+// filter offsets of an item: those of its tile, or its share of them when the offsets are divided
+__device__ __forceinline__ int item_offsets(const SixParams &P, long long item) {
+  if (item >= P.n_items) return 0;
+  const Item I = item_at(P, item);
+  int total = 0;
+  for (int w = 0; w < P.words; ++w) total += __popc(__ldg(P.tile_bits + I.tile * P.words + w));
+  return total * (I.part + 1) / P.n_split - total * I.part / P.n_split;
+}
+
+// Where a row of an item's result goes.
+__device__ __forceinline__ float *result_row(const SixParams &P, const Item &I, int position, int row) {
+  return P.out + (P.n_split > 1 ? ((long long)I.part * P.n_tiles + I.tile) * kRows + position : (long long)row) * P.cout;
+}
+
+__device__ __forceinline__ float finished(const SixParams &P, float v, int c) {
+  if (P.n_split > 1) return v;
+  if (P.bias) v += __ldg(P.bias + c);
+  if (P.bn_scale) {  // separate multiply and add, as the stand-alone BatchNorm kernel rounds them
+    v = __fadd_rn(__fmul_rn(v, __ldg(P.bn_scale + c)), __ldg(P.bn_shift + c));
+    v *= v > 0.f ? 1.f : P.leak;
+  }
+  return v;
+}
+
+// Operands whose parts bf16 cannot hold: infinities, NaN, the last powers of two at either end.  Plain fp32 multiply-adds in
+// the order of k_conv_fma, a warp per row, a lane per plane.
+__device__ __forceinline__ void slow_item(const SixParams &P, long long item, int warp, int warps, int lane) {
+  const Item I = item_at(P, item);
+  unsigned m[4];
+#pragma unroll
+  for (int w = 0; w < 4; ++w) m[w] = w < P.words ? __ldg(P.tile_bits + I.tile * P.words + w) : 0u;
+  const int total = __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]), first = total * I.part / P.n_split;
+  if (P.n_split > 1) keep_range(m, first, total * (I.part + 1) / P.n_split);
+  for (int p = warp; p < kRows; p += warps) {
+    const int row = __ldg(P.order + I.tile * kRows + p);
+    if (row < 0) continue;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};  // planes lane, + 32, + 64, + 96 of the block
+    const int *entry = P.packed + (I.tile * P.K + first) * kRows + p;
+#pragma unroll
+    for (int w = 0; w < 4; ++w)
+      for (unsigned u = m[w]; u; u &= u - 1, entry += kRows) {
+        const int v = __ldg(entry);
+        if (v < 0 || v >= P.n_in) {
+          if (v >= 0 && lane == 0) atomicOr(P.flags, FLAG_BAD_ROW);
+          continue;
+        }
+        const float *wk = P.weight + (long long)(w * 32 + __ffs(u) - 1) * P.cin * P.cout;
+        for (int c = 0; c < P.cin; ++c) {
+          float x = !P.in_b || c < P.planes_a ? __ldg(P.in + (long long)v * (P.in_b ? P.planes_a : P.cin) + c)
+                                              : __ldg(P.in_b + (long long)v * (P.cin - P.planes_a) + (c - P.planes_a));
+          if (P.pre_scale) {
+            x = __fadd_rn(__fmul_rn(x, __ldg(P.pre_scale + c)), __ldg(P.pre_shift + c));
+            x *= x > 0.f ? 1.f : P.pre_leak;
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int n = I.block * P.cb + i * 32 + lane;
+            if (i * 32 + lane < P.cb && n < P.cout) acc[i] = fmaf(x, __ldg(wk + (long long)c * P.cout + n), acc[i]);
+          }
+        }
+      }
+    float *to = result_row(P, I, p, row);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int n = I.block * P.cb + i * 32 + lane;
+      if (i * 32 + lane < P.cb && n < P.cout) to[n] = finished(P, acc[i], n);
+    }
+  }
+}
+
+// Can sums of 2^log2_terms products of values up to x and w in magnitude (float bits) be made of bf16 parts?  Nothing may
+// reach infinity on the way, and the last part of the largest values has to stay a normal number.
+__device__ __forceinline__ bool parts_reach(unsigned x, unsigned w, int log2_terms) {
+  const int ex = (int)(x >> 23) - 127, ew = (int)(w >> 23) - 127;  // (128: infinity or NaN)
+  if (ex >= 126 || ew >= 126) return false;
+  if (x == 0 || w == 0) return true;
+  return ex >= -60 && ew >= -60 && ex + ew >= -90 && ex + ew + 2 + log2_terms < 126;
+}
+
+// x = h + m + l, two values at a time (the first in the low half)
+__device__ __forceinline__ void split3_pair(float a, float b, unsigned &h, unsigned &m, unsigned &l) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  h = *reinterpret_cast<unsigned *>(&v);
+  const float a1 = a - __uint_as_float(h << 16), b1 = b - __uint_as_float(h & 0xFFFF0000u);
+  v = __floats2bfloat162_rn(a1, b1);
+  m = *reinterpret_cast<unsigned *>(&v);
+  v = __floats2bfloat162_rn(a1 - __uint_as_float(m << 16), b1 - __uint_as_float(m & 0xFFFF0000u));
+  l = *reinterpret_cast<unsigned *>(&v);
+}
+
+// SP: input planes of a step; NA: planes of a drain warp, a multiple of 16
+template <int SP, int NA>
+__global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams P) {
+  SCN_GRID_WAIT();
+  using Shape = SixShape<SP>;
+  using Warps = SixWarps<NA>;
+  constexpr int kProdWarps = Warps::PROD, kDrain0 = Warps::DRAIN0, kMma = Warps::MMA, kWgt = Warps::WGT, kEntries = Warps::ENTRIES;
+  constexpr int GROUP = 32 / SP;  // steps summed in tensor memory before they are drained
+  extern __shared__ __align__(1024) unsigned char smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const unsigned w_part = (unsigned)P.cb * SP * 2, w_bytes = w_part * 3;
+  const unsigned stage_bytes = Shape::A_BYTES + ((w_bytes + 1023u) & ~1023u);  // the swizzle pattern repeats every 1 KB
+  const unsigned smem0 = smem_u32(smem);
+  unsigned char *tail = smem + (size_t)P.n_stages * stage_bytes;
+  int *entries = reinterpret_cast<int *>(tail);  // [kSlots][128] input row of every tile row, or -1
+  unsigned char *epi = tail + sizeof(int) * kSlots * kRows;
+  Ctl &C = *reinterpret_cast<Ctl *>(epi + kDrainWarps * kEpiBytes);
+  const bool joint = 3 * P.cb <= 256;  // [W_h | W_m | W_l] as one operand
+  const int dcols = ((joint ? 3 : 2) * P.cb + 31) & ~31;
+  const int n_acc = min(4, 512 / dcols);
+  const long long my_items = items_here(P.n_items);  // (the grid has at most n_items CTAs)
+
+  if (tid < 2) C.range[tid] = 0;
+  if (tid == 0) {
+    for (int i = 0; i < P.n_stages; ++i) {
+      mbar_init(&C.full[i], 32 + 1);  // the producing warp's lanes and the weights
+      mbar_init(&C.empty[i], 1);
+    }
+    for (int i = 0; i < kSlots; ++i) {
+      mbar_init(&C.s_full[i], 1);
+      mbar_init(&C.s_empty[i], P.n_slices + 1);    // a producer warp per slice, and the weights
+    }
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(&C.acc_full[i], 1);
+      mbar_init(&C.acc_empty[i], kDrainWarps);
+    }
+    C.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  static_assert(Warps::THREADS >= kRangeWords, "a thread per range word");
+  if (tid < kRangeWords) {
+    const unsigned x = __reduce_max_sync(0xffffffffu, __ldg(P.in_range + tid)), w = __reduce_max_sync(0xffffffffu, __ldg(P.w_range + tid));
+    if (lane == 0) atomicMax(&C.range[0], x), atomicMax(&C.range[1], w);
+  }
+  if (warp == kMma) tmem_alloc(&C.tmem, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const unsigned tmem = C.tmem;
+  volatile int *abort = &C.abort;
+
+  if (!parts_reach(C.range[0], C.range[1], P.log2_terms)) {
+    for (long long it = 0; it < my_items; ++it) slow_item(P, item_of(it), warp, Warps::THREADS / 32, lane);
+  } else if (warp < kProdWarps) {
+    // ==================================== producers =============================================
+    // this lane's 16-byte piece of the rows q NI .. q NI + NI - 1, for [h | m] and again for [l]
+    const int j = lane % Shape::PIECES, q = lane / Shape::PIECES, lj = lane % Shape::L_PIECES, lq = lane / Shape::L_PIECES;
+    const unsigned hm_dst = (unsigned)(q * Shape::NI) * Shape::HM + (unsigned)j * 16;
+    const unsigned l_dst = kRows * Shape::HM + (unsigned)(lq * Shape::L_NI) * Shape::L + (unsigned)lj * 16;
+    // No more warps than stages: a warp at step n has seen the consumption of step n - active - n_stages, and its wait
+    // below can tell step n - n_stages from the one a round earlier only if that one is not later than this.
+    const int active = min(kProdWarps, P.n_stages);
+    const int d_slot = active / P.n_slices, d_slice = active % P.n_slices;
+    const int d_round = active / P.n_stages, d_st = active % P.n_stages;
+    int slot = warp / P.n_slices, slice = warp % P.n_slices;
+    int round = warp / P.n_stages, st = warp % P.n_stages;
+    bool ok = true, bad = false;
+    while (warp < active) {
+      const int si = slot % kSlots;
+      if (!mbar_wait(&C.s_full[si], (slot / kSlots) & 1)) {
+        ok = false;
+        break;
+      }
+      const int slot_k = C.slot_k[si];
+      if (slot_k < 0 || *abort) break;
+      const int rows_in = slot_k >= kNoRules ? 0 : (int)P.n_in;  // entries below it are rows
+      const int4 *ent = reinterpret_cast<const int4 *>(entries + si * kRows + q * Shape::NI);
+      const int4 *l_ent = reinterpret_cast<const int4 *>(entries + si * kRows + lq * Shape::L_NI);
+      if (!mbar_wait(&C.empty[st], (round + 1) & 1)) {  // (the first round passes)
+        ok = false;
+        break;
+      }
+      const unsigned stage = smem0 + (unsigned)st * stage_bytes;
+      const unsigned char *col = P.in_split + slice * (SP * 6);
+#pragma unroll
+      for (int i = 0; i < Shape::NI; i += 4) {
+        const int4 e4 = ent[i / 4];
+        const int v[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool hit = (unsigned)v[e] < (unsigned)rows_in;
+          bad |= v[e] >= (int)P.n_in && slot_k < kNoRules;
+          const unsigned swizzle = (Shape::HM == 128 ? (i + e) & 7 : ((i + e) >> 1) & 3) * 16;  // (q NI is a multiple of eight)
+          cp_async16(((stage + hm_dst) ^ swizzle) + (i + e) * Shape::HM, col + j * 16 + (size_t)(unsigned)(hit ? v[e] : 0) * P.row_bytes, hit ? 16u : 0u);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < Shape::L_NI; i += 4) {
+        const int4 e4 = l_ent[i / 4];
+        const int v[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool hit = (unsigned)v[e] < (unsigned)rows_in;
+          const unsigned swizzle = (Shape::L == 64 ? ((i + e) >> 1) & 3 : ((i + e) >> 2) & 1) * 16;
+          cp_async16(((stage + l_dst) ^ swizzle) + (i + e) * Shape::L, col + SP * 4 + lj * 16 + (size_t)(unsigned)(hit ? v[e] : 0) * P.row_bytes, hit ? 16u : 0u);
+        }
+      }
+      cp_async_arrive(&C.full[st]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&C.s_empty[si]);
+      slot += d_slot, slice += d_slice;
+      if (slice >= P.n_slices) slice -= P.n_slices, ++slot;
+      round += d_round, st += d_st;
+      if (st >= P.n_stages) st -= P.n_stages, ++round;
+    }
+    if (bad) atomicOr(P.flags, FLAG_BAD_ROW);
+    asm volatile("cp.async.wait_all;" ::: "memory");  // they must land before the CTA's shared memory goes away
+    if (!ok) *abort = 1;
+  } else if (warp == kWgt) {
+    // ==================================== weights ===============================================
+    if (lane == 0) {
+      int st = 0, par = 1;
+      long long filled = 0;
+      bool ok = true;
+      for (int slot = 0; ok; ++slot) {
+        const int si = slot % kSlots;
+        if (!mbar_wait(&C.s_full[si], (slot / kSlots) & 1)) {
+          ok = false;
+          break;
+        }
+        const int slot_k = C.slot_k[si];
+        mbar_arrive(&C.s_empty[si]);
+        if (slot_k < 0) break;
+        const int k = slot_k & 1023, block = slot_k >> 10 & 1;
+        const unsigned char *src = P.wprep + (size_t)(k * P.n_cb + block) * P.n_slices * w_bytes;
+        for (int s = 0; s < P.n_slices; ++s) {
+          if (!mbar_wait(&C.empty[st], par) || *abort) {
+            ok = false;
+            break;
+          }
+          if (!(P.drop && blockIdx.x == 0 && filled == 0)) {
+            mbar_expect_tx(&C.full[st], w_bytes);
+            bulk_copy_g2s(smem0 + (unsigned)st * stage_bytes + Shape::A_BYTES, src + (size_t)s * w_bytes, w_bytes, &C.full[st]);
+          }
+          ++filled;
+          if (++st == P.n_stages) st = 0, par ^= 1;
+        }
+      }
+      if (!ok) {  // slabs in flight must land before the CTA's shared memory goes away
+        *abort = 1;
+        for (int i = 0; i < P.n_stages; ++i) {
+          const long long uses = (filled + P.n_stages - 1 - i) / P.n_stages;
+          if (uses > 0) mbar_wait(&C.full[i], (unsigned)((uses - 1) & 1));
+        }
+      }
+    }
+  } else if (warp == kMma) {
+    // ==================================== MMA issue =============================================
+    // The whole warp runs the loop and one elected lane issues: with warp-uniform control flow and operands the
+    // descriptors stay in uniform registers.
+    const unsigned id1 = tile_idesc(P.cb), id2 = tile_idesc(2 * P.cb), id3 = tile_idesc(joint ? 3 * P.cb : 16);
+    const unsigned long long a_desc = rows_desc<Shape::HM>(smem0, 0), l_desc = rows_desc<Shape::L>(smem0, kRows * Shape::HM);
+    const unsigned long long w_desc = smem_desc(smem0 + Shape::A_BYTES, 128, SP / 8 * 128);
+    const unsigned a_hi = (unsigned)(a_desc >> 32), l_hi = (unsigned)(l_desc >> 32), w_hi = (unsigned)(w_desc >> 32);
+    const unsigned a0 = (unsigned)a_desc, l0 = (unsigned)l_desc, w0 = (unsigned)w_desc;
+    const unsigned stage_step = stage_bytes >> 4, wm_step = w_part >> 4;
+    const int items = (int)my_items, n_stages = P.n_stages, cb = P.cb;
+    int st = 0, par = 0, buf = 0, buf_par = 1;
+    unsigned at = 0, d = tmem;
+    bool ok = true;
+    const bool leader = elect_one();
+    int offsets_next = item_offsets(P, item_of(0));
+    for (int i = 0; i < items && ok; ++i) {
+      const int steps = __reduce_max_sync(0xffffffffu, max(1, offsets_next)) * P.n_slices;
+      offsets_next = item_offsets(P, item_of(i + 1));
+      for (int s = 0; s < steps; ++s) {
+        const bool opens = GROUP == 1 || s % GROUP == 0, closes = GROUP == 1 || s % GROUP == GROUP - 1 || s == steps - 1;
+        // the accumulators must have been drained
+        if (opens && (!mbar_wait_warp(&C.acc_empty[buf], buf_par) || __any_sync(0xffffffffu, *abort != 0))) {
+          ok = false;
+          break;
+        }
+        if (!mbar_wait_warp(&C.full[st], par)) {
+          ok = false;
+          break;
+        }
+        if (leader) {
+          // order the copied rows (acquired through the barrier) before the tensor core's async-proxy reads
+          fence_proxy_async_smem();
+          tc_fence_after();
+#pragma unroll
+          for (int jj = 0; jj < SP / 16; ++jj) {
+            const unsigned ah = a0 + at + jj * 2, am = ah + SP / 8, al = l0 + at + jj * 2, wh = w0 + at + jj * 16;
+            if (jj == 0) mma_bf16(d, ah, a_hi, wh, w_hi, joint ? id3 : id2, opens ? 0u : 1u);
+            else mma_bf16_acc(d, ah, a_hi, wh, w_hi, joint ? id3 : id2);
+            if (joint) {
+              mma_bf16_acc(d + cb, am, a_hi, wh, w_hi, id2);
+              mma_bf16_acc(d + 2 * cb, al, l_hi, wh, w_hi, id1);
+            } else {
+              mma_bf16_acc(d + cb, am, a_hi, wh, w_hi, id1);
+              mma_bf16_acc(d + cb, am, a_hi, wh + wm_step, w_hi, id1);
+              mma_bf16_acc(d + cb, ah, a_hi, wh + 2 * wm_step, w_hi, id1);
+              mma_bf16_acc(d + cb, al, l_hi, wh, w_hi, id1);
+            }
+          }
+          tc_commit(&C.empty[st]);
+          if (closes) tc_commit(&C.acc_full[buf]);
+        }
+        __syncwarp();
+        at += stage_step;
+        if (++st == n_stages) st = 0, par ^= 1, at = 0;
+        if (closes) {
+          d += dcols;
+          if (++buf == n_acc) buf = 0, buf_par ^= 1, d = tmem;
+        }
+      }
+    }
+    if (!ok) *abort = 1;
+  } else if (warp == kEntries) {
+    // ==================================== entries ===============================================
+    if (lane == 0) {
+      int slot = 0;
+      bool ok = true;
+      for (long long it = 0; it < my_items && ok; ++it) {
+        const Item I = item_at(P, item_of(it));
+        unsigned u[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) u[w] = w < P.words ? __ldg(P.tile_bits + I.tile * P.words + w) : 0u;
+        const int *src = P.packed + I.tile * P.K * kRows;
+        if (P.n_split > 1) {
+          const int total = __popc(u[0]) + __popc(u[1]) + __popc(u[2]) + __popc(u[3]);
+          const int first = total * I.part / P.n_split;
+          keep_range(u, first, total * (I.part + 1) / P.n_split);
+          src += first * kRows;
+        }
+        // a tile (or part) without any rule still gets one step, of weights and rows of zeros
+        const bool none = (u[0] | u[1] | u[2] | u[3]) == 0;
+        if (none) u[0] = 1u;
+#pragma unroll 1
+        for (int w = 0; w < 4 && ok; ++w) {
+          unsigned m = u[0];
+          u[0] = u[1], u[1] = u[2], u[2] = u[3], u[3] = 0;
+          for (; m; m &= m - 1, ++slot, src += kRows) {
+            const int si = slot % kSlots;
+            if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1) || *abort) {
+              ok = false;
+              break;
+            }
+            C.slot_k[si] = (none ? kNoRules : w * 32 + __ffs(m) - 1) + (I.block << 10);
+            if (none) {
+              mbar_arrive(&C.s_full[si]);
+            } else {
+              mbar_expect_tx(&C.s_full[si], kRows * 4);
+              bulk_copy_g2s(smem_u32(entries + si * kRows), src, kRows * 4, &C.s_full[si]);
+            }
+          }
+        }
+      }
+      const int filled = slot;
+      // every producer warp finds its next step in a slot that ends it
+      const int ends = (min(kProdWarps, P.n_stages) - 1) / P.n_slices + 1;
+      for (int i = 0; i < ends && ok; ++i, ++slot) {
+        const int si = slot % kSlots;
+        if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1)) {
+          ok = false;
+          break;
+        }
+        C.slot_k[si] = -1;
+        mbar_arrive(&C.s_full[si]);
+      }
+      if (!ok) {  // copies in flight must land before the CTA's shared memory goes away
+        *abort = 1;
+        for (int i = 0; i < kSlots; ++i) {
+          const int uses = (filled + kSlots - 1 - i) / kSlots;
+          if (uses > 0) mbar_wait(&C.s_full[i], (unsigned)((uses - 1) & 1));
+        }
+      }
+    }
+  } else {
+    // ==================================== drain =================================================
+    const int quad = warp & 3, half = (warp - kDrain0) >> 2;
+    const int units = P.cb / 16, first_unit = half ? (units + 1) / 2 : 0, my_units = half ? units / 2 : (units + 1) / 2;
+    float4 *my_epi = reinterpret_cast<float4 *>(epi + (warp - kDrain0) * kEpiBytes);
+    const unsigned base0 = tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(first_unit * 16);
+    const int nc = P.cout, cb = P.cb;
+    int buf = 0, buf_par = 0;
+    bool ok = true;
+    int offsets_next = item_offsets(P, item_of(0));
+    for (long long it = 0; it < my_items && ok; ++it) {
+      const long long item = item_of(it);
+      const Item I = item_at(P, item);
+      const int orow = __ldg(P.order + I.tile * kRows + quad * 32 + lane);
+      const int groups = (__reduce_max_sync(0xffffffffu, max(1, offsets_next)) * P.n_slices + GROUP - 1) / GROUP;
+      offsets_next = item_offsets(P, item_of(it + 1));
+      float acc[NA];
+#pragma unroll
+      for (int e = 0; e < NA; ++e) acc[e] = 0.f;
+      for (int g = 0; g < groups; ++g) {
+        if (!mbar_wait_warp(&C.acc_full[buf], buf_par) || __any_sync(0xffffffffu, *abort != 0)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const unsigned base = base0 + (unsigned)(buf * dcols);
+#pragma unroll
+        for (int u = 0; u < NA / 16; ++u)
+          if (u < my_units) {
+#pragma unroll
+            for (int e0 = 0; e0 < 16; e0 += 8) {
+              unsigned a[8], b[8], c[8];
+              tmem_ld8_nowait(base + u * 16 + e0, a);
+              tmem_ld8_nowait(base + cb + u * 16 + e0, b);
+              if (joint) tmem_ld8_nowait(base + 2 * cb + u * 16 + e0, c);
+              tmem_wait_ld();
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                float small = __uint_as_float(b[e]);
+                if (joint) small += __uint_as_float(c[e]);
+                acc[u * 16 + e0 + e] += __uint_as_float(a[e]) + small;
+              }
+            }
+          }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&C.acc_empty[buf]);
+        if (++buf == n_acc) buf = 0, buf_par ^= 1;
+      }
+      if (!ok) break;
+      // where rows lane / 4, + 8, + 16, + 24 of the warp go
+      int to[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) to[i] = __shfl_sync(0xffffffffu, orow, i * 8 + (lane >> 2));
+#pragma unroll
+      for (int u = 0; u < NA / 16; ++u)
+        if (u < my_units) {
+#pragma unroll
+          for (int e = 0; e < 16; e += 4)
+            my_epi[lane * 4 + ((e >> 2) ^ ((lane >> 1) & 3))] = make_float4(acc[u * 16 + e], acc[u * 16 + e + 1], acc[u * 16 + e + 2], acc[u * 16 + e + 3]);
+          __syncwarp();
+          const int c = I.block * cb + (first_unit + u) * 16 + (lane & 3) * 4;
+          if (c < nc) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int row = i * 8 + (lane >> 2);
+              float4 v = my_epi[row * 4 + ((lane & 3) ^ ((row >> 1) & 3))];
+              if (to[i] < 0) continue;
+              v.x = finished(P, v.x, c), v.y = finished(P, v.y, c + 1), v.z = finished(P, v.z, c + 2), v.w = finished(P, v.w, c + 3);
+              *reinterpret_cast<float4 *>(result_row(P, I, quad * 32 + row, to[i]) + c) = v;
+            }
+          }
+          __syncwarp();
+        }
+    }
+    if (!ok) *abort = 1;
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (*abort && tid == 0) atomicOr(P.flags, FLAG_TC_TIMEOUT);
+  if (warp == kMma) tmem_dealloc(tmem, 512);
+}
+
+struct PrepareParams {
+  const float *in, *in_b;  // [n][cin], or the column-wise concatenation [in (planes_a) | in_b]
+  unsigned char *rows;
+  unsigned *in_range;
+  long long n_pieces;      // of eight planes
+  int cin, ppr, planes_a;
+  const float *pre_scale, *pre_shift;
+  float pre_leak;
+  const float *weight;
+  unsigned char *image;
+  unsigned *w_range;
+  long long w_pieces;
+  int cout, cb, n_cb, n_slices;
+  int row_blocks;          // the first blocks split rows, the others weights
+};
+
+__device__ __forceinline__ void split3_eight(const float (&x)[8], unsigned char *to, size_t part) {
+  uint4 h, m, l;
+  split3_pair(x[0], x[1], h.x, m.x, l.x);
+  split3_pair(x[2], x[3], h.y, m.y, l.y);
+  split3_pair(x[4], x[5], h.z, m.z, l.z);
+  split3_pair(x[6], x[7], h.w, m.w, l.w);
+  *reinterpret_cast<uint4 *>(to) = h;
+  *reinterpret_cast<uint4 *>(to + part) = m;
+  *reinterpret_cast<uint4 *>(to + 2 * part) = l;
+}
+
+// The operands of a layer as three bf16 parts, in one launch, and the largest magnitude of each (range words):
+// rows     [n][cin] (or a join), optionally behind an eval-mode BatchNorm -> per row and slice of SP planes [SP h | SP m | SP l],
+//          planes past cin zero; eight planes per thread and turn.  Bound by HBM: 32 bytes in, 48 out.
+// weights  [K][cin][cout] -> [K][column block][slice][h, m, l][cb x SP] in the K-major core-matrix layout of the MMA's B operand,
+//          eight input planes of an output plane per thread and turn.  Made anew in every call: nothing in this mode is computed
+//          with weights of an earlier one.
+template <int SP>
+__global__ void __launch_bounds__(kPrepareThreads) k_six_prepare(PrepareParams P) {
+  SCN_GRID_WAIT();
+  const bool rows = (int)blockIdx.x < P.row_blocks;
+  const int block = rows ? blockIdx.x : blockIdx.x - P.row_blocks, blocks = rows ? P.row_blocks : gridDim.x - P.row_blocks;
+  const long long total = rows ? P.n_pieces : P.w_pieces;
+  unsigned most = 0;
+  for (long long idx = (long long)block * kPrepareThreads + threadIdx.x; idx < total; idx += (long long)blocks * kPrepareThreads) {
+    float x[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = 0.f;
+    if (rows) {
+      const long long row = idx / P.ppr;
+      const int c = (int)(idx - row * P.ppr) * 8;
+#pragma unroll
+      for (int half = 0; half < 8; half += 4)
+        if (c + half < P.cin) {
+          const int at = c + half;
+          const float *src = !P.in_b ? P.in + row * P.cin + at
+                                     : (at < P.planes_a ? P.in + row * P.planes_a + at : P.in_b + row * (P.cin - P.planes_a) + (at - P.planes_a));
+          const float4 v = __ldg(reinterpret_cast<const float4 *>(src));
+          x[half] = v.x, x[half + 1] = v.y, x[half + 2] = v.z, x[half + 3] = v.w;
+          if (P.pre_scale) {
+#pragma unroll
+            for (int e = half; e < half + 4; ++e) {  // separate multiply and add, as the stand-alone BatchNorm kernel rounds them
+              const float y = __fadd_rn(__fmul_rn(x[e], __ldg(P.pre_scale + c + e)), __ldg(P.pre_shift + c + e));
+              x[e] = y * (y > 0.f ? 1.f : P.pre_leak);
+            }
+          }
+        }
+      split3_eight(x, P.rows + (row * (P.ppr * 8 / SP) + c / SP) * (size_t)(SP * 6) + c % SP * 2, SP * 2);
+    } else {
+      const int columns = P.cb * P.n_cb, n = (int)(idx % columns);
+      const int c = (int)((idx / columns) % P.ppr) * 8, k = (int)(idx / ((long long)columns * P.ppr));
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (c + e < P.cin && n < P.cout) x[e] = __ldg(P.weight + ((long long)k * P.cin + c + e) * P.cout + n);
+      const int nn = n % P.cb;
+      const size_t part = (size_t)P.cb * SP * 2;
+      split3_eight(x, P.image + (((size_t)k * P.n_cb + n / P.cb) * P.n_slices + c / SP) * 3 * part +
+                          ((size_t)(nn / 8) * (SP / 8) + (c % SP) / 8) * 128 + (nn % 8) * 16, part);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) most = max(most, __float_as_uint(x[e]) & 0x7FFFFFFFu);
+  }
+  __shared__ unsigned all;
+  if (threadIdx.x == 0) all = 0;
+  __syncthreads();
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((threadIdx.x & 31) == 0) atomicMax(&all, most);
+  __syncthreads();
+  unsigned *range = rows ? P.in_range : P.w_range;
+  for (int i = block + threadIdx.x * blocks; i < kRangeWords; i += kPrepareThreads * blocks) range[i] = all;
+}
+
+constexpr size_t kSmemBudget = 226 * 1024;
+
+template <int SP, int NA>
+int launch_six(SixParams &P, int n_sm, int dev, cudaStream_t stream) {
+  static std::atomic<bool> configured[64];
+  auto kernel = k_conv_six<SP, NA>;
+  if (!configured[dev].load()) {
+    SCN_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    configured[dev].store(true);
+  }
+  const size_t stage = SixShape<SP>::A_BYTES + ((size_t)P.cb * SP * 6 + 1023) / 1024 * 1024;
+  const size_t fixed = sizeof(int) * kSlots * kRows + kDrainWarps * kEpiBytes + sizeof(Ctl);
+  P.n_stages = (int)std::min<size_t>(kMaxStages, (kSmemBudget - fixed) / stage);
+  P.n_items = P.n_tiles * P.n_split * P.n_cb;
+  SCN_LAUNCH(kernel, (unsigned)std::min<long long>(P.n_items, (long long)n_sm), SixWarps<NA>::THREADS, kSmemBudget, stream, P);
+  SCN_CUDA_CHECK(cudaGetLastError());
+  return SCN_OK;
+}
+
+// Into how many parts a tile's offsets are divided: as in conv_tile.cu, the smallest estimate of (waves of items) x (steps of
+// an item) in SM cycles, plus, with more than one part, the partial sums' traffic and the second launch.
+int split_parts(long long n_tiles, int n_cb, int K, int n_slices, double step_cycles, int cout, int n_sm) {
+  const double offsets = n_tiles >= 2 * n_sm ? 0.5 * K : 0.75 * K;
+  double best = 0;
+  int best_s = 1;
+  for (int s = 1; s <= 16 && s <= K; ++s) {
+    const double waves = (double)ceil_div(n_tiles * n_cb * s, n_sm);
+    double t = waves * (offsets / s * n_slices * step_cycles + 2500.0);
+    if (s > 1) t += 6000.0 + (s + 1.0) * n_tiles * kRows * cout * 4.0 / 3400.0;
+    if (s == 1 || t < 0.95 * best) best = t, best_s = s;
+  }
+  return best_s;
+}
+
+}  // namespace
+
+extern thread_local int g_drop_arrival;  // test hook (conv_tc.cu)
+
+// Which fp32 convolutions run here instead of on k_conv_fma (which is left for few output planes on many rows, whose
+// multiply-adds cost less than six bytes per input value and rule, and for little work, where its one launch is the shorter
+// chain).  One layer,
+// 27 offsets, us on this kernel / on k_conv_fma, and the error of each against float64 (2-norm, products of mixed sign):
+//                 16->16      16->32      32->16      32->32      64->64       96->96       160->160      error (96->96)
+//   300 rows     14.4/12.1   15.3/11.8   14.7/11.3   13.7/12.0   16.0/11.3    19.7/11.9    22.1/17.1     0.8e-7 / 1.9e-7
+//   1 000        14.6/11.2   14.1/11.6   15.6/11.9   14.3/13.1   17.5/17.8    21.4/33.7    28.8/66.0     0.9e-7 / 2.8e-7
+//   2 000        14.6/11.7   15.3/12.4   14.4/13.2   14.6/14.4   18.8/26.3    24.3/51.2    39.9/104.8    0.8e-7 / 3.4e-7
+//   100 000      40/49                               51/84      109/224      179/561       483/1467
+//   200 000      63/57       65/77       84/77       86/114      185/354      302/895      813/2406      1.1e-7 / 5.3e-7
+//   1 600 000    446/403     441/601     617/544     615/872
+//   99 000, 3-D shapes, 27 offsets: 8->16 45/42, 16->16 45/51, 32->16 57/67, 16->32 45/63
+//   91 000, 2-D strokes, 9 offsets: 16->16 28/21, 32->16 33/27, 16->32 28/26, 24->32 34/31, 32->32 34/37
+// Its error was the smaller one for every plane count from 8 to 224, 60 to 200 000 rows, products of mixed and of one sign.
+bool conv_six_takes(const float *in, const float *in_b, int planes_a, const float *out, const float *bias, int K, int cin,
+                    int cout, int groups, long long rows_in, long long rows_out) {
+  return groups == 1 && K <= kOrderMaxOffsets && cin % 4 == 0 && cout % 4 == 0 && cout <= 256 && (cout > 16 || rows_out <= 131072) &&
+         (!in_b || planes_a % 4 == 0) && ((uintptr_t)in | (uintptr_t)in_b | (uintptr_t)out | (uintptr_t)bias) % 16 == 0 &&
+         rows_in < (1ll << 31) && rows_out < (1ll << 31) && rows_out >= 512 &&
+         (double)K * cin * cout >= (K < 27 ? 9000 : 6900) && (double)K * rows_out * cin * cout >= 80e6;
+}
+
+// out [n_out, cout] = act((bias + sum_k in[table[k][.]] @ W[k]) * bn_scale + bn_shift) for the table that `ord` packs, the
+// input optionally a join and behind a BatchNorm of its own
+int conv_forward_six(const float *in, long long n_in, float *out, long long n_out, const float *weight, const float *bias,
+                     const float *bn_scale, const float *bn_shift, float leak, const RowOrder &ord, int K, int cin, int cout,
+                     int *flags, cudaStream_t stream, const float *pre_scale, const float *pre_shift, float pre_leak,
+                     const float *in_b, int planes_a) {
+  if (n_out == 0) return SCN_OK;
+  const int SP = (cin + 15) / 16 * 16 % 32 == 0 ? 32 : 16, n_slices = (cin + SP - 1) / SP, cinp = n_slices * SP;
+  const int coutp = (cout + 15) / 16 * 16, n_cb = coutp > 128 ? 2 : 1, cb = n_cb == 1 ? coutp : (coutp / 2 + 15) / 16 * 16;
+  int dev = 0;
+  SCN_CUDA_CHECK(cudaGetDevice(&dev));
+  SCN_REQUIRE(dev >= 0 && dev < 64, SCN_ERR_UNSUPPORTED, "device index %d unsupported", dev);
+  static std::atomic<int> sm_count[64];
+  int n_sm = sm_count[dev].load();
+  if (!n_sm) {
+    SCN_CUDA_CHECK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+    sm_count[dev].store(n_sm);
+  }
+
+  Scratch tmp(stream);
+  unsigned char *image = nullptr, *rows = nullptr;
+  const size_t image_bytes = (size_t)K * cinp * cb * n_cb * 6, rows_bytes = (size_t)std::max<long long>(n_in, 1) * cinp * 6;
+  SCN_TRY(tmp.get(&image, image_bytes + sizeof(unsigned) * kRangeWords));  // (multiples of 16)
+  SCN_TRY(tmp.get(&rows, rows_bytes + sizeof(unsigned) * kRangeWords));
+  PrepareParams Q{};
+  Q.in = in;
+  Q.in_b = in_b;
+  Q.rows = rows;
+  Q.in_range = (unsigned *)(rows + rows_bytes);
+  Q.ppr = cinp / 8;
+  Q.n_pieces = n_in * Q.ppr;
+  Q.cin = cin;
+  Q.planes_a = planes_a;
+  Q.pre_scale = pre_scale;
+  Q.pre_shift = pre_shift;
+  Q.pre_leak = pre_leak;
+  Q.weight = weight;
+  Q.image = image;
+  Q.w_range = (unsigned *)(image + image_bytes);
+  Q.w_pieces = (long long)K * Q.ppr * cb * n_cb;
+  Q.cout = cout;
+  Q.cb = cb;
+  Q.n_cb = n_cb;
+  Q.n_slices = n_slices;
+  Q.row_blocks = (int)std::max<long long>(1, std::min<long long>(ceil_div(Q.n_pieces, kPrepareThreads), kPrepareBlocks));
+  const unsigned blocks = Q.row_blocks + (unsigned)std::min<long long>(ceil_div(Q.w_pieces, kPrepareThreads), kPrepareBlocks);
+  const auto prepare = SP == 32 ? k_six_prepare<32> : k_six_prepare<16>;
+  SCN_LAUNCH(prepare, blocks, kPrepareThreads, 0, stream, Q);
+
+  SixParams P{};
+  P.in_split = rows;
+  P.in_range = Q.in_range;
+  P.row_bytes = (long long)cinp * 6;
+  P.n_in = n_in;
+  P.out = out;
+  P.cout = cout;
+  P.cb = cb;
+  P.n_cb = n_cb;
+  P.wprep = image;
+  P.w_range = Q.w_range;
+  P.bias = bias;
+  P.bn_scale = bn_scale;
+  P.bn_shift = bn_shift;
+  P.leak = bn_scale ? leak : 1.f;
+  P.order = ord.order;
+  P.packed = ord.packed;
+  P.by_work = ord.by_work;
+  P.tile_bits = ord.tile_bits;
+  P.words = ord.words;
+  P.K = K;
+  P.n_slices = n_slices;
+  P.log2_terms = bit_length((unsigned long long)K * cin);
+  P.n_tiles = ord.n_tiles;
+  P.in = in;
+  P.in_b = in_b;
+  P.weight = weight;
+  P.pre_scale = pre_scale;
+  P.pre_shift = pre_shift;
+  P.pre_leak = pre_leak;
+  P.cin = cin;
+  P.planes_a = planes_a;
+  P.flags = flags;
+  P.drop = g_drop_arrival;
+  g_drop_arrival = 0;
+  const double chunk = cb <= 80 ? std::max(56.0, 1.5 * cb) + std::max(56.0, 1.0 * cb) + 56 : cb + 4 * std::max(56.0, 0.5 * cb);
+  const double step = std::max((kRows * SP * 6.0 + cb * SP * 6.0) / 32.0, chunk * SP / 16);
+  const char *e = getenv("SCN_SIX_SPLIT");
+  P.n_split = e ? std::max(1, std::min(atoi(e), 64)) : split_parts(P.n_tiles, n_cb, K, n_slices, step, cout, n_sm);
+  if (P.n_split > 1) SCN_TRY(tmp.get(&P.out, (size_t)P.n_split * P.n_tiles * kRows * cout * sizeof(float)));
+  const auto launch = SP == 32 ? (cb <= 32 ? launch_six<32, 16> : cb <= 64 ? launch_six<32, 32> : launch_six<32, 64>)
+                               : (cb <= 32 ? launch_six<16, 16> : cb <= 64 ? launch_six<16, 32> : launch_six<16, 64>);
+  SCN_TRY(launch(P, n_sm, dev, stream));
+  if (P.n_split > 1)
+    SCN_TRY(sum_partial_tiles(P.out, P.n_split, P.n_tiles * kRows, cout, ord.order, n_out, bias, bn_scale, bn_shift, leak, out, stream));
+  return SCN_OK;
+}
+
+}  // namespace scn

@@ -43,8 +43,7 @@
 #include <algorithm>
 #include <atomic>
 
-#include "metadata.cuh"
-#include "tc_ptx.cuh"
+#include "conv_tile.cuh"
 
 namespace scn {
 
@@ -91,23 +90,6 @@ struct TileShape {
   static_assert(PP == 8 || PP == 4, "a row of a step is 128 or 64 bytes");
 };
 
-// Operand descriptor of a stage of gathered rows: K-major, 128- or 64-byte swizzle (a row's 16-byte chunk c is stored
-// at chunk c ^ (r & 7), or c ^ ((r >> 1) & 3)), 8-row groups back to back.  `offset`: bytes along the row.
-// Whole rows being contiguous is what makes the gather fast: a row arrives as full 128-byte writes.  With the pieces
-// spread over core matrices 2 KB apart every 16 bytes were a write of their own: 1 700 cycles per 16 KB step.
-template <unsigned ROW>
-__device__ __forceinline__ unsigned long long rows_desc(unsigned addr, unsigned offset) {
-  unsigned long long d = 0;
-  d |= (unsigned long long)(((addr + offset) >> 4) & 0x3FFF);
-  d |= 1ull << 16;
-  d |= (unsigned long long)((ROW * 8) >> 4) << 32;
-  d |= 1ull << 46;
-  d |= (unsigned long long)(ROW == 128 ? 2 : 4) << 61;
-  return d;
-}
-
-constexpr int kNoRules = 1 << 20;
-
 // control block behind the ring
 struct Ctl {
   unsigned long long full[kMaxStages], empty[kMaxStages];  // rows and weights landed; MMAs done
@@ -117,30 +99,6 @@ struct Ctl {
   int abort;
 };
 
-__host__ __device__ inline unsigned tile_idesc(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(kRows >> 4) << 24);
-}
-
-// bits `lo` .. `hi` - 1 of the set bits of a 128-bit mask, counted from bit 0 (the offsets of one part of a split)
-__device__ __forceinline__ void keep_range(unsigned (&m)[4], int lo, int hi) {
-  int seen = 0;
-#pragma unroll
-  for (int w = 0; w < 4; ++w) {
-    unsigned keep = 0;
-    for (unsigned u = m[w]; u; u &= u - 1, ++seen)
-      if (seen >= lo && seen < hi) keep |= u & (0u - u);
-    m[w] = keep;
-  }
-}
-
-// The items of a CTA: back and forth over the CTAs, so that of items in descending order of work each gets about the same.
-__device__ __forceinline__ long long item_of(long long it) {
-  return it & 1 ? (it + 1) * gridDim.x - 1 - blockIdx.x : it * gridDim.x + blockIdx.x;
-}
-__device__ __forceinline__ long long items_here(const TileParams &P) {
-  const long long full = P.n_items / gridDim.x;
-  return full + (item_of(full) < P.n_items ? 1 : 0);
-}
 // The tile of an item: the tiles with the most offsets first (packed tiles come in ascending order of their masks, so from
 // the back where they have not been sorted by work).
 __device__ __forceinline__ long long item_tile(const TileParams &P, long long item) {
@@ -200,7 +158,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
   tc_fence_after();
   const unsigned tmem = C.tmem;
   volatile int *abort = &C.abort;
-  const long long my_items = items_here(P);  // (the grid has at most n_items CTAs)
+  const long long my_items = items_here(P.n_items);  // (the grid has at most n_items CTAs)
 
   if (warp < kProdWarps) {
     // ==================================== producers =============================================

@@ -57,6 +57,7 @@ struct RowOrder {
   int *packed = nullptr;
   int *by_work = nullptr;  // the tiles, those with the most offsets first (null: small levels, tiles in their order)
   int words = 1;  // 32-bit words per tile: 1 up to 32 offsets, else 4
+  bool fp32_only = false;  // made by an fp32 convolution of a small level: no reason for its weight gradient to use tiles
   long long n_tiles = 0;
 };
 

@@ -1,0 +1,155 @@
+"""k_conv_six: the fp32 mode on tensor cores, operands as three bf16 parts, six products.
+
+Per step of 32 planes the tensor core truncates two sums of 16 products each (2^-23 of them at most), everything else is
+rounded to nearest in fp32: the 2-norm of the error stays below 2^-22 of the result's, 2.4e-7, and below that of a chain of
+fp32 multiply-adds of a few hundred terms."""
+import pytest
+import torch
+
+from tests.test_gpu_tile import _points
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(x, layer, kind, filt, stride, f, shape):
+    want = torch.zeros(shape, dtype=torch.float64, device=f.device)
+    if hasattr(layer, "bias"):
+        want += layer.bias.double()
+    for r, w in zip(x.metadata.rulebook(kind, x.spatial_size, filt, stride), layer.weight.double()[:, 0]):
+        r = r.long()
+        want.index_add_(0, r[:, 1], f.double()[r[:, 0]] @ w)
+    return want
+
+
+@pytest.mark.parametrize("cin,cout", [(8, 24), (12, 20), (16, 32), (32, 32), (36, 64), (64, 80), (64, 84), (96, 96), (32, 128),
+                                      (100, 132), (64, 256)])
+@pytest.mark.parametrize("n,split", [(700, None), (8191, None), (20001, None), (8200, "3"), (150000, None)])
+def test_as_accurate_as_multiply_adds(n, split, cin, cout, cuda, monkeypatch):
+    """Every plane tile and both column layouts, packed and unpacked rows, divided offsets: submanifold and strided layers,
+    against float64 and against the error of k_conv_fma."""
+    import sparseconvnet_b200 as scn
+    lib = scn.SCN.lib
+    if split:
+        monkeypatch.setenv("SCN_SIX_SPLIT", split)
+    coords = _points(n, 3, 160 if n < 100000 else 512, n)
+    x = scn.InputLayer(3, 512, mode=0)([torch.from_numpy(coords), torch.zeros(len(coords), 1, device=cuda)])
+    torch.manual_seed(cin)
+    with torch.no_grad():
+        for layer, kind, filt, stride in [(scn.SubmanifoldConvolution(3, cin, cout, 3, True), 0, [3, 3, 3], None),
+                                          (scn.Convolution(3, cin, cout, 2, 2, False), 1, [2, 2, 2], [2, 2, 2])]:
+            layer.to(cuda)
+            if hasattr(layer, "bias"):
+                layer.bias.normal_()
+            f = torch.randn(len(coords), cin, device=cuda)
+            errors = []
+            for six in ("1", "0"):
+                monkeypatch.setenv("SCN_CONV_SIX", six)
+                y = layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features
+                if not errors and not lib.scn_last_conv_six():
+                    work = layer.weight.size(0) * cin * cout  # too little of it
+                    assert len(y) < 512 or work * len(y) < 80e6 or work < 9000
+                    break
+                want = _exact(x, layer, kind, filt, stride, f, y.shape)
+                errors.append(float((y.double() - want).norm() / want.norm()))
+            x.metadata.poll_errors()
+            if errors:
+                assert errors[0] <= 2.0 ** -22 and errors[0] <= 1.05 * errors[1], (layer, errors)
+
+
+@pytest.mark.parametrize("case", ["inf", "nan", "huge", "tiny", "tiny weights", "inf weight", "zeros"])
+@pytest.mark.parametrize("cin,cout,n", [(32, 32, 5000), (40, 136, 5000)])
+def test_values_the_parts_cannot_hold(case, cin, cout, n, cuda, monkeypatch):
+    """Infinities, NaN and the ends of the range: as fp32 multiply-adds in the order of k_conv_fma give them."""
+    import sparseconvnet_b200 as scn
+    coords = _points(n, 3, 60, 3)
+    x = scn.InputLayer(3, 60, mode=0)([torch.from_numpy(coords), torch.zeros(len(coords), 1, device=cuda)])
+    torch.manual_seed(1)
+    layer = scn.SubmanifoldConvolution(3, cin, cout, 3, True).to(cuda).requires_grad_(False)
+    f = torch.randn(len(coords), cin, device=cuda)
+    if case in ("inf", "nan"):
+        f[17, 3] = float(case)
+    elif case == "huge":
+        f[5] = 2.9e38
+    elif case == "tiny":
+        f *= 1e-38
+    elif case == "tiny weights":
+        f *= 1e-14
+        layer.weight *= 1e-14
+    elif case == "inf weight":
+        layer.weight[13, 0, 2, 1] = float("inf")
+    else:
+        f.zero_()
+    outs = []
+    for six, knob in (("1", "SCN_SIX_SPLIT"), ("0", "SCN_FMA_SPLIT")):
+        monkeypatch.setenv("SCN_CONV_SIX", six)
+        monkeypatch.setenv(knob, "1")
+        with torch.no_grad():
+            outs.append(layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features)
+        assert scn.SCN.lib.scn_last_conv_six() == int(six)
+    x.metadata.poll_errors()
+    got, want = outs
+    if case == "inf weight":  # k_conv_fma multiplies the rows without a rule by it as well
+        finite = torch.isfinite(want)
+        assert torch.equal(got[finite], want[finite]) and not torch.isfinite(got[:, 1]).all()
+    else:
+        assert torch.equal(torch.nan_to_num(got, nan=7.0), torch.nan_to_num(want, nan=7.0))
+
+
+@pytest.mark.parametrize("cin,cout", [(32, 48), (24, 160)])
+def test_weights_of_this_call(cin, cout, cuda):
+    """A weight written through .data, which leaves its version as it is, counts from the next call on."""
+    import sparseconvnet_b200 as scn
+    coords = _points(6000, 3, 60, 4)
+    x = scn.InputLayer(3, 60, mode=0)([torch.from_numpy(coords), torch.randn(len(coords), cin, device=cuda)])
+    layer = scn.SubmanifoldConvolution(3, cin, cout, 3, False).to(cuda)
+    with torch.no_grad():
+        one = layer(x).features
+        assert scn.SCN.lib.scn_last_conv_six()
+        layer.weight.data.mul_(2)
+        assert torch.equal(layer(x).features, 2 * one)
+
+
+@pytest.mark.parametrize("n", [700, 20000])
+def test_batchnorm_and_join_in_front(n, cuda):
+    """In the pass that splits the rows: the same bits as the layers one by one."""
+    import sparseconvnet_b200 as scn
+    torch.manual_seed(n)
+
+    def block(planes):
+        return scn.Sequential().add(scn.BatchNormLeakyReLU(planes, leakiness=0.2)).add(scn.SubmanifoldConvolution(3, planes, 32, 3, True))
+    net = scn.Sequential().add(scn.ConcatTable().add(scn.Identity()).add(block(32))).add(scn.JoinTable()).add(block(64)).to(cuda).eval()
+    for m in net.modules():
+        if isinstance(m, scn.BatchNormalization):
+            for t in (m.running_mean, m.running_var, m.weight, m.bias):
+                torch.nn.init.uniform_(t, 0.3, 1.0)
+    coords = _points(n, 3, 120, n)
+    feats = torch.randn(len(coords), 32, device=cuda)
+    outs = []
+    try:
+        for fuse in (False, True):
+            scn.Sequential.fuse = fuse
+            with torch.no_grad():
+                outs.append(net(scn.InputLayer(3, 120, mode=0)([torch.from_numpy(coords), feats])).features)
+    finally:
+        scn.Sequential.fuse = True
+    assert torch.equal(*outs)
+
+
+def test_bounded_wait_runs_out(cuda):
+    """One barrier arrival left out: the kernel returns by itself, the host learns of it, the next call is right."""
+    import sparseconvnet_b200 as scn
+    from sparseconvnet_b200._lib import ScnError, lib
+    coords = _points(20000, 3, 96, 5)
+    layer = scn.SubmanifoldConvolution(3, 96, 96, 3, False).to(cuda)
+    with torch.no_grad():
+        x = scn.InputLayer(3, 96, mode=0)([torch.from_numpy(coords), torch.randn(len(coords), 96, device=cuda)])
+        good = layer(x).features.clone()
+        assert lib.scn_last_conv_six()
+        x.metadata.poll_errors()
+        assert lib.scn_test_drop_barrier_arrival() == 0
+        layer(x)
+        torch.cuda.synchronize()
+        with pytest.raises(ScnError, match="bounded wait"):
+            x.metadata.poll_errors()
+        assert torch.equal(layer(x).features, good)
+        x.metadata.poll_errors()
