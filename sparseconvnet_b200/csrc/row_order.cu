@@ -41,11 +41,8 @@ __device__ __forceinline__ void count_digit(int *h, int d) {
   const unsigned peers = __match_any_sync(__activemask(), d);
   if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&h[d], __popc(peers));
 }
-__device__ __forceinline__ void store_counts(const int *h, int R, int *block_count, int *total) {
-  for (int i = threadIdx.x; i < R; i += kThreads) {
-    block_count[(long long)blockIdx.x * R + i] = h[i];
-    if (h[i]) atomicAdd(&total[i], h[i]);
-  }
+__device__ __forceinline__ void store_counts(const int *h, int R, int *block_count) {
+  for (int i = threadIdx.x; i < R; i += kThreads) block_count[(long long)blockIdx.x * R + i] = h[i];
 }
 
 // Which offsets of a row have a rule (read from the table unless the rulebook's builder has left them in `known`), and
@@ -54,9 +51,10 @@ template <typename KEY, int WORDS>
 __global__ void __launch_bounds__(kThreads)
 k_order_keys(const int *__restrict__ nbr, const unsigned *__restrict__ known, long long n, int K, KeyBits<KEY> B,
              int rows_per_block, int R, KEY *__restrict__ keys, unsigned *__restrict__ masks,
-             int *__restrict__ block_count, int *__restrict__ total) {
+             int *__restrict__ block_count, int *tiles_done) {
   SCN_GRID_WAIT();
   __shared__ int h[kMaxDigit];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *tiles_done = 0;  // (for k_order_tiles)
   for (int i = threadIdx.x; i < R; i += kThreads) h[i] = 0;
   __syncthreads();
   const long long r0 = (long long)blockIdx.x * rows_per_block, r1 = min(n, r0 + rows_per_block);
@@ -86,14 +84,14 @@ k_order_keys(const int *__restrict__ nbr, const unsigned *__restrict__ known, lo
     count_digit(h, (int)key & (R - 1));
   }
   __syncthreads();
-  store_counts(h, R, block_count, total);
+  store_counts(h, R, block_count);
 }
 
-// Digit counts of every block's rows (block_count [blocks][R]) and of all rows (total [R], zeroed before).
+// Digit counts of every block's rows (block_count [blocks][R]).
 template <typename KEY>
 __global__ void __launch_bounds__(kThreads)
 k_order_count(const KEY *__restrict__ keys, long long n, int rows_per_block, int shift, int R,
-              int *__restrict__ block_count, int *__restrict__ total) {
+              int *__restrict__ block_count) {
   SCN_GRID_WAIT();
   __shared__ int h[kMaxDigit];
   for (int i = threadIdx.x; i < R; i += kThreads) h[i] = 0;
@@ -101,20 +99,20 @@ k_order_count(const KEY *__restrict__ keys, long long n, int rows_per_block, int
   const long long r0 = (long long)blockIdx.x * rows_per_block, r1 = min(n, r0 + rows_per_block);
   for (long long r = r0 + threadIdx.x; r < r1; r += kThreads) count_digit(h, (int)(keys[r] >> shift) & (R - 1));
   __syncthreads();
-  store_counts(h, R, block_count, total);
+  store_counts(h, R, block_count);
 }
 
 // Stable scatter of a block's rows by one digit.  A block's first position of digit d is (rows of smaller
-// digits) + (rows of digit d in the blocks before it), both read from the counts; within the block the warps
-// own consecutive segments.  rows_in null: the row of position i is i.
+// digits) + (rows of digit d in the blocks before it), both added up from the blocks' counts (the last block reads as many
+// of them as all do: totals of their own, cleared by a launch and added to by atomics, saved nothing); within the block the
+// warps own consecutive segments.  rows_in null: the row of position i is i.
 template <typename KEY>
 __global__ void __launch_bounds__(kThreads)
 k_order_scatter(const KEY *__restrict__ keys, const int *__restrict__ rows_in, long long n, int rows_per_block,
-                int shift, int R, const int *__restrict__ block_count, const int *__restrict__ total,
-                KEY *__restrict__ keys_out, int *__restrict__ rows_out) {
+                int shift, int R, const int *__restrict__ block_count, KEY *__restrict__ keys_out, int *__restrict__ rows_out) {
   SCN_GRID_WAIT();
   __shared__ unsigned short cnt[kWarps][kMaxDigit];  // rows of digit d in warp w's segment, then in the warps before it
-  __shared__ int base[kMaxDigit], part[kMaxDigit];   // (a block has fewer than 65536 rows)
+  __shared__ int base[kMaxDigit], part[kMaxDigit], part_total[kMaxDigit];  // (a block has fewer than 65536 rows)
   __shared__ int warp_sum[kWarps];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int i = tid; i < kWarps * kMaxDigit / 2; i += kThreads) reinterpret_cast<unsigned *>(&cnt[0][0])[i] = 0;
@@ -130,15 +128,20 @@ k_order_scatter(const KEY *__restrict__ keys, const int *__restrict__ rows_in, l
     if (d >= 0 && lane == __ffs(peers) - 1) cnt[warp][d] += (unsigned short)__popc(peers);
     __syncwarp();
   }
-  // rows of digit d in the blocks before this one: two threads per digit, every other block each
+  // rows of digit d in the blocks before this one and in all: two threads per digit, every other block each
   const int d = tid & (kMaxDigit - 1), half = tid / kMaxDigit;
   int before = 0, tot = 0;
   if (d < R) {
 #pragma unroll 16
-    for (int b = half; b < (int)blockIdx.x; b += 2) before += __ldg(block_count + (long long)b * R + d);
-    if (half == 0) tot = total[d];
-    else part[d] = before;
+    for (int b = half; b < (int)gridDim.x; b += 2) {
+      const int c = __ldg(block_count + (long long)b * R + d);
+      tot += c;
+      before += b < (int)blockIdx.x ? c : 0;
+    }
+    if (half) part[d] = before, part_total[d] = tot;
   }
+  __syncthreads();
+  tot = half == 0 && d < R ? tot + part_total[d] : 0;
   int incl = tot;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -294,49 +297,61 @@ __device__ void tiles_by_work(const unsigned *tile_bits, int n_tiles, int K, int
   each(true, [&](int t, int b) { by_work[hist[b][tid]++] = t; });
 }
 
-// One warp per tile, four rows per lane: tile_bits, packed, and -1 in the order array past the last row.
-template <int WORDS>
-__device__ __forceinline__ void pack_tile(int *__restrict__ order, long long n, int K, const int *__restrict__ nbr,
-                                          const unsigned *__restrict__ masks, unsigned *tile_bits, int *__restrict__ packed,
-                                          long long t, int lane) {
-  const long long p = t * kTile + lane * 4;
-  int4 o = *reinterpret_cast<const int4 *>(order + p);
-  if (p + 3 >= n) {
-    o.x = p < n ? o.x : -1, o.y = p + 1 < n ? o.y : -1, o.z = p + 2 < n ? o.z : -1, o.w = -1;
-    *reinterpret_cast<int4 *>(order + p) = o;
-  }
-  const int row[4] = {o.x, o.y, o.z, o.w};
-  unsigned m[4][WORDS];
-#pragma unroll
-  for (int e = 0; e < 4; ++e)
-#pragma unroll
-    for (int w = 0; w < WORDS; ++w) m[e][w] = row[e] >= 0 ? __ldg(masks + (long long)row[e] * WORDS + w) : 0u;
-  int *dst = packed + t * K * kTile + lane * 4;
-#pragma unroll
-  for (int w = 0; w < WORDS; ++w) {
-    const unsigned all = __reduce_or_sync(0xffffffffu, m[0][w] | m[1][w] | m[2][w] | m[3][w]);
-    if (lane == 0) tile_bits[t * WORDS + w] = all;
-#pragma unroll 4
-    for (unsigned u = all; u; u &= u - 1) {
-      const int b = __ffs(u) - 1;
-      const int *col = nbr + (long long)(w * 32 + b) * n;
-      int v[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = m[e][w] >> b & 1u ? __ldg(col + row[e]) : -1;
-      *reinterpret_cast<int4 *>(dst) = make_int4(v[0], v[1], v[2], v[3]);
-      dst += kTile;
-    }
-  }
-}
-
+// Two tiles per block, a row per thread: tile_bits, packed, and -1 in the order array past the last row.  Bound by the trips to
+// L2 that the entries of rows far apart take, so many threads with eight of them on their way.  (A warp per tile, four rows
+// per lane: 104 us for the eleven sorted levels of one room where this takes 67, 25.7 and 22.3 on 267 k rows, 377 and 347 on
+// 1.5 M rows with 81 offsets.)
 template <int WORDS>
 __global__ void __launch_bounds__(256)
 k_order_tiles(int *__restrict__ order, long long n, int K, const int *__restrict__ nbr, const unsigned *__restrict__ masks,
               unsigned *tile_bits, int *__restrict__ packed, long long n_tiles, int *by_work, int *done) {
   SCN_GRID_WAIT();
-  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (t < n_tiles) pack_tile<WORDS>(order, n, K, nbr, masks, tile_bits, packed, t, lane);
+  __shared__ unsigned warp_bits[8][WORDS];
+  static_assert(kTile == 128, "a row per thread, four warps per tile");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, in_tile = threadIdx.x & (kTile - 1);
+  const long long t = (long long)blockIdx.x * 2 + threadIdx.x / kTile;
+  int row = -1;
+  unsigned m[WORDS];
+  if (t < n_tiles) {
+    const long long p = t * kTile + in_tile;
+    if (p < n) row = order[p];
+    else order[p] = -1;
+  }
+#pragma unroll
+  for (int w = 0; w < WORDS; ++w) m[w] = row >= 0 ? __ldg(masks + (long long)row * WORDS + w) : 0u;
+#pragma unroll
+  for (int w = 0; w < WORDS; ++w) {
+    const unsigned any = __reduce_or_sync(0xffffffffu, m[w]);
+    if (lane == 0) warp_bits[warp][w] = any;
+  }
+  __syncthreads();
+  if (t < n_tiles) {
+    int *dst = packed + t * K * kTile + in_tile;
+    const int w0 = warp & ~3;
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) {
+      const unsigned all = warp_bits[w0][w] | warp_bits[w0 + 1][w] | warp_bits[w0 + 2][w] | warp_bits[w0 + 3][w];
+      if (in_tile == 0) tile_bits[t * WORDS + w] = all;
+      unsigned u = all;
+      while (u) {  // eight offsets at a time
+        int v[8];
+        unsigned left = u;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int b = left ? __ffs(left) - 1 : 0;
+          v[e] = left && (m[w] >> b & 1u) ? __ldg(nbr + (long long)(w * 32 + b) * n + row) : -1;
+          left &= left - 1;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (u) {
+            *dst = v[e];
+            dst += kTile;
+            u &= u - 1;
+          }
+      }
+    }
+  }
   if (!by_work) return;
   __shared__ bool last;
   __threadfence();
@@ -399,7 +414,7 @@ int build(const int *table, const unsigned *known, long long n, int K, const uns
   Scratch tmp(stream);
   unsigned *masks = nullptr;
   KEY *keys[2] = {nullptr, nullptr};
-  int *rows = nullptr, *counts = nullptr, *totals = nullptr;
+  int *rows = nullptr, *counts = nullptr;
   const int passes = (bits + 8) / 9, digit = (bits + passes - 1) / passes, R = 1 << digit;
   // Rows per block: a multiple of the warps' 32-row chunks; one block per SM at most, because a block adds up the counts
   // of the blocks before it itself
@@ -409,25 +424,24 @@ int build(const int *table, const unsigned *known, long long n, int K, const uns
   for (int k = 0; k < K; ++k) B.bit[k] = (KEY)bit[k];
   if (!known) SCN_TRY(tmp.get(&masks, sizeof(unsigned) * WORDS * (size_t)n));
   SCN_TRY(tmp.get(&keys[0], sizeof(KEY) * (size_t)n));
-  SCN_TRY(tmp.get(&counts, sizeof(int) * (size_t)blocks * R));
-  SCN_TRY(tmp.get(&totals, sizeof(int) * ((size_t)passes * R + 1)));  // and the blocks that have packed their tiles
+  SCN_TRY(tmp.get(&counts, sizeof(int) * ((size_t)blocks * R + 1)));  // and the blocks that have packed their tiles
+  int *const done = counts + (size_t)blocks * R;
   if (passes > 1) {
     SCN_TRY(tmp.get(&keys[1], sizeof(KEY) * (size_t)n));
     SCN_TRY(tmp.get(&rows, sizeof(int) * (size_t)n));
   }
-  SCN_CUDA_CHECK(cudaMemsetAsync(totals, 0, sizeof(int) * ((size_t)passes * R + 1), stream));
   if (ord.n_tiles > 148 && ord.n_tiles < 65536) SCN_TRY(device_alloc((void **)&ord.by_work, sizeof(int) * (size_t)ord.n_tiles, stream));
-  SCN_LAUNCH((k_order_keys<KEY, WORDS>), blocks, kThreads, 0, stream, table, known, n, K, B, (int)rpb, R, keys[0], masks, counts, totals);
+  SCN_LAUNCH((k_order_keys<KEY, WORDS>), blocks, kThreads, 0, stream, table, known, n, K, B, (int)rpb, R, keys[0], masks, counts, done);
   const int *src = nullptr;
   for (int p = 0; p < passes; ++p) {
     int *dst = ((passes - 1 - p) & 1) ? rows : ord.order;  // alternating so that the last pass writes ord.order
     KEY *kin = keys[p & 1], *kout = p + 1 < passes ? keys[(p + 1) & 1] : nullptr;
     if (p > 0)
-      SCN_LAUNCH((k_order_count<KEY>), blocks, kThreads, 0, stream, kin, n, (int)rpb, p * digit, R, counts, totals + (size_t)p * R);
-    SCN_LAUNCH((k_order_scatter<KEY>), blocks, kThreads, 0, stream, kin, src, n, (int)rpb, p * digit, R, counts, totals + (size_t)p * R, kout, dst);
+      SCN_LAUNCH((k_order_count<KEY>), blocks, kThreads, 0, stream, kin, n, (int)rpb, p * digit, R, counts);
+    SCN_LAUNCH((k_order_scatter<KEY>), blocks, kThreads, 0, stream, kin, src, n, (int)rpb, p * digit, R, counts, kout, dst);
     src = dst;
   }
-  SCN_LAUNCH((k_order_tiles<WORDS>), (unsigned)ceil_div(ord.n_tiles * 32, 256), 256, 0, stream, ord.order, n, K, table, known ? known : masks, ord.tile_bits, ord.packed, ord.n_tiles, ord.by_work, totals + (size_t)passes * R);
+  SCN_LAUNCH((k_order_tiles<WORDS>), (unsigned)ceil_div(ord.n_tiles, 2), 256, 0, stream, ord.order, n, K, table, known ? known : masks, ord.tile_bits, ord.packed, ord.n_tiles, ord.by_work, done);
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }
