@@ -10,10 +10,11 @@
 // What this form is built on:
 //   * Tiles are packed from rows that have the same set of filter offsets (row_order.cu), so a tile of 128 rows
 //     runs 9 to 12 steps of 27 instead of 22 to 25 and nearly every row of a step holds a rule.
-//   * A tcgen05.mma takes max(56, N / 2) cycles for 128 rows (scn_tc_probe_mma).  With up to 64 output planes
-//     the slab [W_h | W_m] is one operand of 2 x planes columns: h (W_h | W_m) is ONE instruction whose two
-//     column ranges are the large and one small term, m W_h goes to the small range, the epilogue adds the two:
-//     2 instructions per 16 planes instead of 3.
+//   * A tcgen05.mma takes max(56, N / 2) cycles for 128 rows (scn_tc_probe_mma) and reads both operands from shared memory.
+//     With up to 128 output planes the slab [W_h | W_m] is one operand of 2 x planes columns: h (W_h | W_m) is ONE instruction
+//     whose two column ranges are the large and one small term, m W_h goes to the small range, the epilogue adds the two:
+//     2 instructions per 16 planes instead of 3, and the rows are read twice instead of three times.  (Above 64 planes too
+//     since the reads count: U-Net on eight rooms 6095 -> 6034 us, on one room 1912 -> 1884.)
 //   * What bounds it is the gather: 128 bytes per row and 32-plane step (16 + 16 bits per value) through 16-byte
 //     cp.async at about 32 bytes per cycle and SM, 512 cycles per step against 224 cycles of tensor work for 32
 //     output planes, 304 for 96.
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
   int *entries = reinterpret_cast<int *>(tail);  // [kSlots][128] input row of every tile row, or -1
   unsigned char *epi = tail + sizeof(int) * kSlots * kRows;
   Ctl &C = *reinterpret_cast<Ctl *>(epi + 4 * kEpiBytes);
-  const bool joint = TERMS == 3 && P.coutp <= 64;  // [W_h | W_m] as one operand
+  const bool joint = TERMS == 3 && P.coutp <= 128;  // [W_h | W_m] as one operand
   const int dcols = ((joint ? 2 : 1) * P.coutp + 31) & ~31;
   const int n_acc = min(4, P.tmem_cols / dcols);
 
@@ -597,7 +598,7 @@ int launch_tile_as(TileParams &P, int n_sm, int dev, cudaStream_t stream) {
   }
   const size_t stage = Shape::A_BYTES + ((size_t)P.coutp * SP * 2 * Shape::PARTS + 1023) / 1024 * 1024;
   const size_t fixed = sizeof(int) * kSlots * kRows + 4 * kEpiBytes + sizeof(Ctl);
-  const int dcols = ((TERMS == 3 && P.coutp <= 64 ? 2 : 1) * P.coutp + 31) & ~31;
+  const int dcols = ((TERMS == 3 && P.coutp <= 128 ? 2 : 1) * P.coutp + 31) & ~31;
   // Two CTAs per SM, each with half of the shared memory and of the TMEM columns, where that leaves four stages and two
   // accumulators: one CTA's issue overhead and epilogue run beside the other's tensor instructions.
   int ctas = dcols * 2 <= 256 && (kSmemBudget / 2 - fixed) / stage >= 4 ? 2 : 1;
