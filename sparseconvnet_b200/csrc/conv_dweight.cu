@@ -26,10 +26,12 @@
 //               per job); a tile's T rows are staged once for all the group's offsets, 16 rows by each warp.  (Splitting
 //               gathered fp32 rows on their way through the registers moves a third fewer bytes, but at 55 instructions per
 //               16 bytes the warps could not keep up: 5 600 cycles per piece.)
-//   MMA         one warp.
+//   MMA         two warps, a job's 128 rules at a time.  An instruction's issue takes as long as the tensor core does, and what
+//               a warp spends on barriers and its next job (some 800 cycles for 1 408 of instructions) came on top: 64 x 96
+//               weights on 131 k rows 346 us with one warp that waited for every 32 rules, 311 for 128, 302 with two warps.
 //
-// Bound by the gather (48 KB per 128 rules of 64 planes) and, close behind, the tensor instructions (176 cycles per 16
-// rules of 64 x 64).
+// Bound by the gather: 48 KB per 128 rules of 64 planes and a share of the tile's own rows, 72 KB in 2 100 cycles, beside
+// 1 408 cycles of tensor instructions.
 #include <algorithm>
 #include <atomic>
 #include <utility>
@@ -45,8 +47,8 @@ namespace {
 
 constexpr int kRows = kOrderTile;
 constexpr int kLoadWarps = 8;
-constexpr int kMma = kLoadWarps, kJobs = kLoadWarps + 1;
-constexpr int kThreads = (kLoadWarps + 2) * 32;
+constexpr int kMmaWarps = 2, kMma = kLoadWarps, kJobs = kMma + kMmaWarps;
+constexpr int kThreads = (kJobs + 1) * 32;
 constexpr int kSlots = 8;           // jobs ahead
 constexpr int kMaxTiles = 48;       // tiles of a CTA
 constexpr long long kMostPartial = 256ll << 20;
@@ -57,11 +59,12 @@ struct DwTile {
   static constexpr int T_ATOMS = PT == 64 ? 3 : 2;  // h, m, l, or (h m), (l 0)
   static constexpr int G_ATOMS = PG == 64 ? 3 : 2;
   static constexpr int T_PIECE = kRows / kLoadWarps;                             // rows of a warp
-  static constexpr int G_PIECE = 32;                                             // rows of a stage
+  static constexpr int G_PIECE = 32, PIECES = kRows / G_PIECE;                   // rows of a stage, stages of a job
   static constexpr int T_BYTES = T_ATOMS * kAtom, G_ATOM = G_PIECE * 128, G_BYTES = G_ATOMS * G_ATOM;
   // One stage per loading warp: a warp that comes back to its stage has seen the consumption of its last piece but one,
   // so that the parity it waits for cannot be one of an earlier round.
   static constexpr int STAGES = kLoadWarps;
+  static_assert(STAGES == 2 * PIECES, "two jobs' rows");
   static constexpr int COLS = PG == 64 ? 128 : 96;  // accumulator columns of an offset
   static constexpr int OFFSETS = 512 / COLS;
   static constexpr int ZERO = 2048;                 // 16 rules of zeros: what follows l in its operand
@@ -164,7 +167,7 @@ __device__ __forceinline__ bool copy_rows(unsigned dst, int atom, const int *row
 constexpr int kTRows = 100, kEnd = 101;
 
 struct Ctl {
-  unsigned long long full[8], empty[8], t_full[2], t_empty[2], s_full[kSlots], s_empty[kSlots], done;
+  unsigned long long full[2], empty[2], t_full[2], t_empty[2], s_full[kSlots], s_empty[kSlots], done;
   int job[kSlots];  // index of the offset in the group; kTRows; kEnd
   unsigned tmem, used;
   int abort;
@@ -192,19 +195,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
   for (int i = tid; i < S::ZERO / 16; i += kThreads) reinterpret_cast<uint4 *>(base + zero_at)[i] = make_uint4(0, 0, 0, 0);
   fence_proxy_async_smem();
   if (tid == 0) {
-    for (int i = 0; i < 8; ++i) {
-      mbar_init(&C.full[i], 32);  // the lanes of the copying warp
-      mbar_init(&C.empty[i], 1);
+    for (int i = 0; i < S::STAGES / S::PIECES; ++i) {
+      mbar_init(&C.full[i], 32 * S::PIECES);  // the lanes of the copying warps
+      mbar_init(&C.empty[i], kMmaWarps);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&C.t_full[i], kLoadWarps * 32);
-      mbar_init(&C.t_empty[i], 1);
+      mbar_init(&C.t_empty[i], kMmaWarps);
     }
     for (int i = 0; i < kSlots; ++i) {
       mbar_init(&C.s_full[i], 1);
-      mbar_init(&C.s_empty[i], kLoadWarps + 1);
+      mbar_init(&C.s_empty[i], kLoadWarps + kMmaWarps);
     }
-    mbar_init(&C.done, 1);
+    mbar_init(&C.done, kMmaWarps);
     C.abort = 0;
     C.used = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -218,7 +221,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
 
   if (warp < kLoadWarps) {
     // ==================================== rows ==================================================
-    constexpr int kPieces = kRows / S::G_PIECE;
     const long long t_bytes = split_row_bytes((P.t_planes + PT - 1) / PT * (PT / 8), PT), g_bytes = split_row_bytes((P.g_planes + PG - 1) / PG * (PG / 8), PG);
     const unsigned char *t_src = P.t_rows + t0 * 6, *g_src = P.g_rows + g0 * 6;
     const unsigned t_dst = smem0 + warp * (S::T_PIECE * 128), g_dst = smem0 + g_at + warp * S::G_BYTES;  // piece g: stage g % 8
@@ -241,13 +243,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
         ++n_t;
       } else {
         const int q = (warp - n_g) & (kLoadWarps - 1);  // the piece of the job that is this warp's
-        if (q < kPieces) {
-          ok = mbar_wait(&C.empty[warp], (unsigned)((n_g + q) / S::STAGES + 1) & 1);
+        if (q < S::PIECES) {
+          ok = mbar_wait(&C.empty[warp / S::PIECES], (unsigned)((n_g + q) / S::STAGES + 1) & 1);
           if (!ok) break;
           bad |= copy_rows<PG, S::G_PIECE>(g_dst, S::G_ATOM, row + q * S::G_PIECE, g_src, g_bytes, (int)P.n_g, lane);
-          cp_async_arrive(&C.full[warp]);
+          cp_async_arrive(&C.full[warp / S::PIECES]);
         }
-        n_g += kPieces;
+        n_g += S::PIECES;
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&C.s_empty[slot]);
@@ -329,8 +331,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
     __syncwarp();  // the other lanes must not go ahead: waiting for `done` they would hold up lane 0
   } else {
     // ==================================== MMA issue =============================================
-    // The whole warp runs the loop, one elected lane issues; the job is made warp-uniform by a reduction, so that the
-    // descriptors stay in uniform registers.
+    // Each warp issues the jobs of every second offset of the group: an accumulator belongs to one of them, and what one
+    // takes to learn of its next job and to wait for its rows passes while the other's instructions run.  The whole warp runs
+    // the loop, one elected lane issues; the job is made warp-uniform by a reduction, so that the descriptors stay in
+    // uniform registers.
+    const int parity = warp - kMma;
     int slot = 0, s_par = 0, st = 0, par = 0, tb = 1, t_par = 1;  // (the first tile's T rows are buffer 0, parity 0)
     unsigned used = 0;
     bool ok = true, first = true;
@@ -355,24 +360,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
         }
         continue;
       }
-      const unsigned a = smem0 + tb * S::T_BYTES, d = tmem + job * S::COLS;
-      const unsigned al = a + 2 * kAtom;
-      unsigned A = planes_desc_lo(a, kAtom), AL = planes_desc_lo(al, smem0 + zero_at - al);
-      unsigned acc = (used >> job) & 1u;
-      for (int q = 0; q < kRows / S::G_PIECE && ok; ++q) {
-        if (!mbar_wait_warp(&C.full[st], par)) {
-          ok = false;
-          break;
-        }
-        const unsigned B0 = planes_desc_lo(smem0 + g_at + st * S::G_BYTES, S::G_ATOM);
+      // (for the other warp's jobs too, and the rows go when both have been here: neither can fall a round behind, or run a
+      // round ahead, where a phase's parity is that of another)
+      if (!mbar_wait_warp(&C.full[st], par)) {
+        ok = false;
+        break;
+      }
+      if ((job & 1) != parity) {
+        if (lane == 0) mbar_arrive(&C.empty[st]);
+      } else {
+        const unsigned a = smem0 + tb * S::T_BYTES, d = tmem + job * S::COLS;
+        const unsigned al = a + 2 * kAtom;
+        const unsigned A = planes_desc_lo(a, kAtom), AL = planes_desc_lo(al, smem0 + zero_at - al);
+        const unsigned B0 = planes_desc_lo(smem0 + g_at + st * (S::PIECES * S::G_BYTES), S::G_ATOM);
+        const unsigned acc = (used >> job) & 1u;
         if (leader) {
           // order the stored rows (acquired through the barriers) before the tensor core's async-proxy reads; done here,
           // not by the warps that store: their fence would wait for the loads they have on their way
           fence_proxy_async_smem();
           tc_fence_after();
 #pragma unroll
-          for (int kk = 0; kk < S::G_PIECE / 16; ++kk) {
-            const unsigned B = B0 + kk * 128;  // 2 KB further
+          for (int kk = 0; kk < kRows / 16; ++kk) {
+            const unsigned B = B0 + kk / 2 * (S::G_BYTES >> 4) + kk % 2 * 128;  // a piece, and 2 KB further
             if (kk == 0) mma_bf16(d, A, kDescHi, B, kDescHi, idesc(PG == 64 ? 128 : 96), acc);
             else mma_bf16_acc(d, A + kk * 128, kDescHi, B, kDescHi, idesc(PG == 64 ? 128 : 96));
             if (PG == 64) mma_bf16_acc(d + 64, A + kk * 128, kDescHi, B + (2 * S::G_ATOM >> 4), kDescHi, idesc(64));
@@ -382,17 +391,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
           tc_commit(&C.empty[st]);
         }
         __syncwarp();
-        acc = 1;
-        A += S::G_PIECE * 8;
-        AL += S::G_PIECE * 8 - (unsigned)(S::G_PIECE * 8 << 16);
-        if (++st == S::STAGES) st = 0, par ^= 1;
+        used |= 1u << job;
       }
-      if (!ok) break;
-      used |= 1u << job;
+      if (++st == S::STAGES / S::PIECES) st = 0, par ^= 1;
     }
     if (!ok) *abort = 1;
     if (leader) {
-      C.used = used;
+      atomicOr(&C.used, used);
       tc_commit(&C.done);
     }
     __syncwarp();
