@@ -380,11 +380,16 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
                        int precision, int *flags, cudaStream_t stream, const float *bn_scale, const float *bn_shift,
                        float leak, const float *pre_scale, const float *pre_shift, float pre_leak, const float *in_b,
                        int planes_a) {
-  const int *table = transposed_table ? rb.tnbr : rb.nbr;
   g_last_six = false;
+  // the row order of the table: for a table of children (one rule per row) from the parents' side, without the table
+  const auto row_order = [&](RowOrder &ord) -> int {
+    if (transposed_table && rb.one_parent && rb.n_offsets <= kChildrenMaxOffsets) return rulebook_children_order(rb, ord, stream);
+    if (transposed_table) SCN_TRY(rulebook_transposed(rb, stream));
+    return rulebook_row_order(rb, transposed_table ? rb.tnbr : rb.nbr, rows_out, ord, stream);
+  };
   if (tile_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, precision, rows_out)) {
     RowOrder &ord = transposed_table ? rb.torder : rb.order;
-    SCN_TRY(rulebook_row_order(rb, table, rows_out, ord, stream));
+    SCN_TRY(row_order(ord));
     ord.fp32_only = false;
     SCN_TRY(conv_forward_tile(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, ord, rb.n_offsets,
                               cin, cout, precision, flags, stream, pre_scale, pre_shift, pre_leak, in_b, planes_a));
@@ -396,13 +401,17 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
   const bool fma = precision == SCN_PRECISION_FP32 && rows_out > 0 && cin > 4 &&
                    conv_fma_supported(in, out, weight, bias, rb.n_offsets, cin, cout, groups) &&
                    !(any_knob() && getenv("SCN_SIMT_BLOCK") && atoi(getenv("SCN_SIMT_BLOCK")) != 0);
+  const bool packed = fma && conv_fma_wants_order(rows_out);
+  if (transposed_table && !packed && !(fma && six_enabled() && conv_six_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, rows_in, rows_out)))
+    SCN_TRY(rulebook_transposed(rb, stream));
+  const int *table = transposed_table ? rb.tnbr : rb.nbr;
   if (!fma)
     return conv_forward_dispatch(in, rows_in, out, rows_out, weight, bias, table, rb.n_offsets, cin, cout, groups, precision,
                                  flags, stream, bn_scale, bn_shift, leak, pre_scale, pre_shift, pre_leak, in_b, planes_a);
   if (six_enabled() && conv_six_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, rows_in, rows_out)) {
     RowOrder &ord = transposed_table ? rb.torder : rb.order;
     const bool there = ord.order != nullptr;
-    SCN_TRY(rulebook_row_order(rb, table, rows_out, ord, stream));
+    SCN_TRY(row_order(ord));
     if (!there) ord.fp32_only = true;
     SCN_TRY(conv_forward_six(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, ord, rb.n_offsets, cin, cout,
                              flags, stream, pre_scale, pre_shift, pre_leak, in_b, planes_a));
@@ -414,9 +423,9 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
   SCN_TRY(prepared_input(&in, rows_in, cin, groups, pre_scale, pre_shift, pre_leak, in_b, planes_a, &pre_copy, stream));
   RowOrder *ord = nullptr;
   int rc = SCN_OK;
-  if (conv_fma_wants_order(rows_out)) {
+  if (packed) {
     ord = transposed_table ? &rb.torder : &rb.order;
-    rc = rulebook_row_order(rb, table, rows_out, *ord, stream);
+    rc = row_order(*ord);
   }
   if (rc == SCN_OK)
     rc = conv_forward_fma(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, table, ord, rb.n_offsets, cin,
@@ -424,6 +433,16 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
   device_free(pre_copy, stream);
   g_last_kernel = SCN_KERNEL_CONV_FMA;
   return rc;
+}
+
+// Has every fine row of a strided rulebook exactly one rule?  Filter = stride: the children of different coarse sites and
+// offsets never coincide.  (Rows in no map, earlier duplicates under input mode 0, have none.)
+bool one_rule_per_row(scn_metadata *md, const int64_t *fine_size, const int64_t *coarse_size, const int64_t *filter_size,
+                      const int64_t *filter_stride) {
+  for (int d = 0; d < md->dim; ++d)
+    if (filter_size[d] != filter_stride[d] || coarse_size[d] * filter_stride[d] < fine_size[d]) return false;
+  const Grid *fine = find_grid(md, fine_size);
+  return fine && !fine->may_have_blank_rows;
 }
 
 static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float *in, float *out,
@@ -466,7 +485,6 @@ static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float
                        !(getenv("SCN_X3_ROWS") && atoi(getenv("SCN_X3_ROWS")) == 0) &&
                        !(getenv("SCN_ROWS_SCATTER") && atoi(getenv("SCN_ROWS_SCATTER")) == 0) &&
                        conv_rows_supported(in, out, weight, bias, rb.n_offsets, cin, cout, groups);
-  if (transposed && !scatter) SCN_TRY(rulebook_transposed(rb, stream));
   if (rows_out > 0 && scatter) {
     SCN_TRY(conv_forward_rows_scatter(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, rb.nbr,
                                       rb.n_offsets, cin, cout, md->flags_dev, stream));
@@ -608,10 +626,7 @@ int scn_deconvolution_forward(scn_metadata *md, const int64_t *input_size, const
   Rulebook *rb = nullptr;
   // the rulebook of the matching Convolution: fine (this op's output) -> coarse (this op's input)
   SCN_TRY(get_strided_rulebook(md, output_size, input_size, filter_size, filter_stride, stream, &rb));
-  bool disjoint = true;  // filter = stride: the children of different coarse sites and offsets never coincide
-  for (int d = 0; d < md->dim; ++d) disjoint &= filter_size[d] == filter_stride[d];
-  const Grid *fine = find_grid(md, output_size);
-  disjoint &= fine && !fine->may_have_blank_rows;
+  const bool disjoint = rb->one_parent = one_rule_per_row(md, output_size, input_size, filter_size, filter_stride);
   return run_conv(md, *rb, true, in_features, out_features, weight, bias, n_in_planes, n_out_planes,
                   groups, precision, stream, macs, disjoint);
 }
@@ -701,10 +716,7 @@ int scn_deconvolution_bn_forward(scn_metadata *md, const int64_t *input_size, co
               "null argument");
   Rulebook *rb = nullptr;
   SCN_TRY(get_strided_rulebook(md, output_size, input_size, filter_size, filter_stride, stream, &rb));
-  bool disjoint = true;
-  for (int d = 0; d < md->dim; ++d) disjoint &= filter_size[d] == filter_stride[d];
-  const Grid *fine = find_grid(md, output_size);
-  disjoint &= fine && !fine->may_have_blank_rows;
+  const bool disjoint = rb->one_parent = one_rule_per_row(md, output_size, input_size, filter_size, filter_stride);
   return run_conv(md, *rb, true, in_features, out_features, weight, bias, n_in_planes, n_out_planes, groups,
                   precision, stream, macs, disjoint, bn_scale, bn_shift, (float)leakiness);
 }

@@ -306,8 +306,9 @@ int conv_forward_fma(const float *in, long long n_in, float *out, long long n_ou
   const int rows = ord ? 128 : 32;
   P.n_pos = ord ? ord->n_tiles * kOrderTile : ceil_div(n_out, 32) * 32;
   const long long ctas = P.n_pos / rows * cols;
-  const int steps = (int)(K * ceil_div(cin, kChunk));
-  P.n_split = (int)std::max<long long>(1, std::min<long long>({ceil_div(148 * 3, ctas), (long long)steps / 4, (long long)K, 16ll}));
+  const int offsets = ord && ord->one_offset ? 1 : K;  // of a tile
+  const int steps = (int)(offsets * ceil_div(cin, kChunk));
+  P.n_split = (int)std::max<long long>(1, std::min<long long>({ceil_div(148 * 3, ctas), (long long)steps / 4, (long long)offsets, 16ll}));
   if (const char *e = getenv("SCN_FMA_SPLIT")) P.n_split = std::max(1, std::min(atoi(e), 64));
   float *partial = nullptr;
   if (P.n_split > 1) {

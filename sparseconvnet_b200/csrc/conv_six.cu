@@ -797,7 +797,7 @@ int conv_forward_six(const float *in, long long n_in, float *out, long long n_ou
   const double chunk = cb <= 80 ? std::max(56.0, 1.5 * cb) + std::max(56.0, 1.0 * cb) + 56 : cb + 4 * std::max(56.0, 0.5 * cb);
   const double step = std::max((kRows * SP * 6.0 + cb * SP * 6.0) / 32.0, chunk * SP / 16);
   const char *e = getenv("SCN_SIX_SPLIT");
-  P.n_split = e ? std::max(1, std::min(atoi(e), 64)) : split_parts(P.n_tiles, n_cb, K, n_slices, step, cout, n_sm);
+  P.n_split = e ? std::max(1, std::min(atoi(e), 64)) : split_parts(P.n_tiles, n_cb, ord.one_offset ? 1 : K, n_slices, step, cout, n_sm);
   if (P.n_split > 1) SCN_TRY(tmp.get(&P.out, (size_t)P.n_split * P.n_tiles * kRows * cout * sizeof(float)));
   const auto launch = SP == 32 ? (cb <= 32 ? launch_six<32, 16> : cb <= 64 ? launch_six<32, 32> : launch_six<32, 64>)
                                : (cb <= 32 ? launch_six<16, 16> : cb <= 64 ? launch_six<16, 32> : launch_six<16, 64>);

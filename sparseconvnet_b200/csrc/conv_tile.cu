@@ -730,7 +730,7 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
   g_drop_arrival = 0;
   const double w_bytes = (double)coutp * SP * 2 * parts, a_bytes = kRows * SP * 2.0 * parts;
   const char *e = getenv("SCN_TILE_SPLIT");
-  P.n_split = e ? std::max(1, atoi(e)) : split_parts(P.n_tiles, K, n_slices, (a_bytes + w_bytes) / 32.0, cout, n_sm);
+  P.n_split = e ? std::max(1, atoi(e)) : split_parts(P.n_tiles, ord.one_offset ? 1 : K, n_slices, (a_bytes + w_bytes) / 32.0, cout, n_sm);
   P.out_split = P.n_split > 1 ? nullptr : out_split;
   if (P.n_split > 1) SCN_TRY(tmp.get(&P.out, (size_t)P.n_split * P.n_tiles * kRows * cout * sizeof(float)));
   const auto launch = terms == 3 ? (SP == 32 ? launch_tile<3, 32> : launch_tile<3, 16>) : (SP == 64 ? launch_tile<1, 64> : launch_tile<1, 32>);

@@ -57,6 +57,7 @@ struct RowOrder {
   int *packed = nullptr;
   int *by_work = nullptr;  // the tiles, those with the most offsets first (null: small levels, tiles in their order)
   int words = 1;  // 32-bit words per tile: 1 up to 32 offsets, else 4
+  bool one_offset = false; // every tile has at most one filter offset (rulebook_children_order)
   bool fp32_only = false;  // made by an fp32 convolution of a small level: no reason for its weight gradient to use tiles
   long long n_tiles = 0;
 };
@@ -72,11 +73,14 @@ struct Rulebook {
   // offsets with a rule of every output row of nbr, mask_words(K) words each (submanifold rulebooks up to
   // kOrderMaxOffsets offsets; null otherwise)
   unsigned *masks = nullptr;
-  unsigned long long *counts_dev = nullptr;  // [K] rules per offset, then the builder's count of finished blocks
+  // [K] rules per offset, then the builder's count of finished blocks; of a strided rulebook K more zeros behind them
+  // (rulebook_children_order)
+  unsigned long long *counts_dev = nullptr;
   std::vector<long long> counts_host;        // filled on first request (waits for the stream)
   long long total_rules = -1;
   CountTicket *ticket = nullptr;             // counts in flight (null above kTicketValues offsets)
   bool built = false;
+  bool one_parent = false; // strided: every input row has exactly one rule (set by the operators that ask for torder)
   bool symmetric = false;  // submanifold with odd filter sizes: tnbr[k] is nbr[K - 1 - k]
 };
 
@@ -86,6 +90,9 @@ int rulebook_counts_async(Rulebook &rb, cudaStream_t stream);
 int rulebook_transposed(Rulebook &rb, cudaStream_t stream);     // builds tnbr if missing
 // builds the packing order of the table [K][n] (nbr or tnbr of `rb`) if missing
 int rulebook_row_order(const Rulebook &rb, const int *table, long long n, RowOrder &ord, cudaStream_t stream);
+// the same for tnbr of a rulebook with `one_parent` and at most 32 offsets, from nbr in one launch
+int rulebook_children_order(const Rulebook &rb, RowOrder &ord, cudaStream_t stream);
+constexpr int kChildrenMaxOffsets = 32;
 void free_row_order(RowOrder &o, cudaStream_t stream);
 
 struct PendingChain;  // metadata.cu: levels of a strided chain whose kernels run on the side stream

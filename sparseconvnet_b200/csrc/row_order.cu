@@ -213,6 +213,78 @@ k_order_plain(const int *__restrict__ nbr, long long n, int K, int words, int *_
   }
 }
 
+// Fine rows with one rule each (a Deconvolution whose filter is its stride) by the offset of that rule, from the table as the
+// Convolution has it (nbr [K][n_out] = fine row or -1) and the rules per offset that its builder has counted: whole tiles
+// of one offset, -1 behind an offset's last row.  A block takes a run of the offset's places for its coarse rows, so the
+// blocks come in the order in which they get there; what a row's sum is does not depend on the tile it is in.  One launch
+// where the transposed table, its masks, a counting pass and the tiles were six: 17 us per level on small levels, 95 on
+// 1.6 M rows, now 5 and 14.
+__global__ void __launch_bounds__(256)
+k_order_children(const int *__restrict__ nbr, long long n_out, int K, const unsigned long long *__restrict__ counts,
+                 unsigned long long *cursors, long long n_tiles, int *__restrict__ order, unsigned *__restrict__ tile_bits,
+                 int *__restrict__ packed) {
+  SCN_GRID_WAIT();
+  __shared__ int start[kChildrenMaxOffsets + 1];  // first tile of an offset
+  __shared__ int before[8][kChildrenMaxOffsets];  // rules of an offset in this warp's coarse rows, then in the warps before
+  __shared__ long long base[kChildrenMaxOffsets];
+  static_assert(kChildrenMaxOffsets == 32, "a lane per offset");
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 0) {
+    const int tiles = lane < K ? (int)((counts[lane] + kTile - 1) / kTile) : 0;
+    int incl = tiles;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += u;
+    }
+    start[lane] = incl - tiles;
+    if (lane == 31) start[32] = incl;
+  }
+  const long long o = (long long)blockIdx.x * 256 + tid;
+#pragma unroll 8
+  for (int k = 0; k < K; ++k) {
+    const unsigned hits = __ballot_sync(0xffffffffu, o < n_out && __ldg(nbr + k * n_out + o) >= 0);
+    if (lane == 0) before[warp][k] = __popc(hits);
+  }
+  __syncthreads();
+  if (tid < K) {
+    int run = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const int c = before[w][tid];
+      before[w][tid] = run;
+      run += c;
+    }
+    base[tid] = run ? (long long)atomicAdd(&cursors[tid], (unsigned long long)run) : 0;
+  }
+  __syncthreads();
+#pragma unroll 8
+  for (int k = 0; k < K; ++k) {
+    const int v = o < n_out ? __ldg(nbr + k * n_out + o) : -1;
+    const unsigned hits = __ballot_sync(0xffffffffu, v >= 0);
+    if (v >= 0) {
+      const long long p = (long long)start[k] * kTile + base[k] + before[warp][k] + __popc(hits & ((1u << lane) - 1u));
+      order[p] = v;
+      packed[p / kTile * K * kTile + p % kTile] = (int)o;
+    }
+  }
+  for (long long t = o; t < n_tiles; t += (long long)gridDim.x * 256) {
+    unsigned bits = 0;
+    for (int k = 0; k < K; ++k)
+      if (t >= start[k] && t < start[k + 1]) bits = 1u << k;
+    tile_bits[t] = bits;
+  }
+  if (blockIdx.x == 0)
+    for (int k = warp; k <= K; k += 8) {  // behind the last row of an offset, and of all
+      const long long p0 = k < K ? (long long)start[k] * kTile + (long long)counts[k] : (long long)start[K] * kTile;
+      const long long p1 = k < K ? (long long)start[k + 1] * kTile : n_tiles * kTile;
+      for (long long p = p0 + lane; p < p1; p += 32) {
+        order[p] = -1;
+        packed[p / kTile * K * kTile + p % kTile] = -1;
+      }
+    }
+}
+
 // The tiles by how many offsets they have, most first, stable (run by one block of 256 threads, the last of k_order_tiles to
 // pack its own: it adds 4 us to 21 us at 300 k rows).  Handed out in ascending order of their masks the tiles left the
 // busiest SM 1.1 to 1.7 times the average; most offsets first, back and forth over the CTAs, 1.02 to 1.2: 32 -> 32 planes
@@ -454,6 +526,32 @@ void free_row_order(RowOrder &o, cudaStream_t stream) {
   device_free(o.packed, stream);
   device_free(o.by_work, stream);
   o = RowOrder{};
+}
+
+int rulebook_children_order(const Rulebook &rb, RowOrder &ord, cudaStream_t stream) {
+  if (ord.order || rb.n_in == 0) return SCN_OK;
+  const int K = rb.n_offsets;
+  SCN_REQUIRE(rb.one_parent && K <= kChildrenMaxOffsets && rb.n_in < (1ll << 31), SCN_ERR_UNSUPPORTED, "children order: %d offsets", K);
+  RowOrder o;
+  o.words = 1;
+  o.one_offset = true;
+  o.n_tiles = (rb.n_in + (long long)K * (kTile - 1)) / kTile;  // every offset's last tile may be nearly empty
+  int st = device_alloc((void **)&o.order, sizeof(int) * (size_t)o.n_tiles * kTile, stream);
+  if (st == SCN_OK) st = device_alloc((void **)&o.tile_bits, sizeof(unsigned) * (size_t)o.n_tiles, stream);
+  if (st == SCN_OK) st = device_alloc((void **)&o.packed, sizeof(int) * (size_t)o.n_tiles * K * kTile, stream);
+  if (st == SCN_OK) {
+    SCN_LAUNCH(k_order_children, (unsigned)std::max<long long>(1, ceil_div(rb.n_out, 256)), 256, 0, stream, rb.nbr, rb.n_out, K, rb.counts_dev, rb.counts_dev + K + 1, o.n_tiles, o.order, o.tile_bits, o.packed);
+    if (cudaGetLastError() != cudaSuccess) {
+      set_error("children order: launch failed");
+      st = SCN_ERR_CUDA;
+    }
+  }
+  if (st != SCN_OK) {
+    free_row_order(o, stream);
+    return st;
+  }
+  ord = o;
+  return SCN_OK;
 }
 
 // Builds the packing order of a rulebook table [K][n] if it is not there yet.

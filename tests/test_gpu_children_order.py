@@ -1,0 +1,65 @@
+"""Layers whose fine rows have one rule each (filter = stride), on tiles made from the parents' side in one launch: against
+float64 over the exported rulebook, at the edges of tiles and with offsets that few rows or none have."""
+import numpy as np
+import pytest
+import torch
+
+from tests import helpers
+
+pytestmark = pytest.mark.gpu
+
+
+def _points(n, dim, size, corner):
+    rng = np.random.default_rng(n + dim)
+    pts = rng.integers(0, size, (4 * n + 8, dim))
+    if corner:  # every site at the same place of its cell: one offset has all rules
+        pts = pts // 2 * 2 + 1
+    pts = np.unique(pts, axis=0)
+    pts = pts[rng.permutation(len(pts))][:n]
+    return np.concatenate([pts, rng.integers(0, 2, (len(pts), 1))], axis=1)
+
+
+# fp32: multiply-adds or three bf16 parts, sums of cin products; the others: what the split leaves out, one bf16 product
+@pytest.mark.parametrize("precision,tol", [("fp32", 1e-6), ("tf32x3", helpers.FP32_TOL), ("bf16", helpers.TC_TOL)])
+@pytest.mark.parametrize("n,dim,filt,corner", [(1, 3, 2, False), (127, 3, 2, False), (128, 3, 2, True), (129, 3, 2, True),
+                                               (5000, 3, 2, False), (40000, 3, 2, False), (3000, 2, 3, False), (9000, 3, 3, False),
+                                               (6000, 4, 2, False)])
+def test_children(n, dim, filt, corner, precision, tol, cuda):
+    import sparseconvnet_b200 as scn
+    size = {2: 96, 3: 48, 4: 24}[dim]
+    coords = _points(n, dim, size, corner)
+    cin, cout = 64, 48
+    torch.manual_seed(n)
+    up = scn.Deconvolution(dim, cin, cout, filt, filt, True).to(cuda)
+    down = scn.Convolution(dim, cout, cin, filt, filt, False).to(cuda)
+    up.bias.data.normal_()
+    coarse = torch.LongTensor([size // filt] * dim)
+    try:
+        scn.set_precision(precision)
+        scn.set_backward_precision(precision)
+        # mode 1: no rows that are in no map
+        x = scn.InputLayer(dim, size, mode=1)([torch.from_numpy(coords), torch.zeros(len(coords), 1, device=cuda)])
+        fine = torch.randn(x.features.size(0), cout, device=cuda, requires_grad=True)
+        y = down(scn.SparseConvNetTensor(fine, x.metadata, x.spatial_size)).features
+        g = torch.randn_like(y)
+        y.backward(g)
+        f = torch.randn(y.size(0), cin, device=cuda)
+        with torch.no_grad():
+            z = up(scn.SparseConvNetTensor(f, x.metadata, coarse)).features
+        x.metadata.poll_errors()
+    finally:
+        scn.set_precision("fp32")
+        scn.set_backward_precision("fp32")
+    want = up.bias.detach().double().expand(z.shape).clone()
+    grad = torch.zeros(fine.shape, dtype=torch.float64, device=cuda)
+    seen = 0
+    for r, w, v in zip(x.metadata.rulebook(1, x.spatial_size, [filt] * dim, [filt] * dim), up.weight.detach().double()[:, 0],
+                       down.weight.detach().double()[:, 0]):
+        r = r.long()
+        seen += len(r)
+        want.index_add_(0, r[:, 0], f.double()[r[:, 1]] @ w)
+        grad.index_add_(0, r[:, 0], g.double()[r[:, 1]] @ v.t())
+    assert seen == len(fine)
+    for got, exact in ((z, want), (fine.grad, grad)):
+        e = helpers.rel_err(got.double().cpu().numpy(), exact.cpu().numpy())
+        assert e <= tol, e
