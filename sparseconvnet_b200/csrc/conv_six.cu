@@ -6,8 +6,8 @@
 //     The three hold the 24 bits of x exactly.  A product is the six terms h h', h m', m h', h l', m m', l h'; what is left
 //     out is below 2^-26 of it, less than an fp32 product is rounded by.
 //   * The tensor core truncates its running sum, so it never runs far: one step of 32 planes of one filter offset is
-//     summed there, the large terms and the small ones in accumulators of their own, and every step's sums are added to
-//     fp32 registers, rounded to nearest (the "drain" warps).
+//     summed there, the large terms and the small ones apart or the small ones first, and every step's sums are added to fp32
+//     registers, rounded to nearest (the "drain" warps).
 // Time and error against float64 beside k_conv_fma's: the table at conv_six_takes.
 //
 // The range of bf16 is that of fp32 except at its ends: the low parts of a tiny value would be lost, and an infinity has no
@@ -18,8 +18,9 @@
 //   entries     one thread: a slot per (tile, filter offset with a rule), 512 bytes of input rows from the packed table
 //   producers   8 (5) warps, a step each: 128 rows of 192 bytes ([32 h | 32 m] and [32 l]) by 16-byte cp.async
 //   weights     one thread: one bulk copy of [W_h | W_m | W_l] per step
-//   MMA         up to 80 output planes three instructions per 16 input planes, h (W_h | W_m | W_l), m (W_h | W_m), l W_h, into
-//               three column ranges; above that six, into two ranges (the large terms, the small ones)
+//   MMA         up to 64 output planes three instructions per 16 input planes, h (W_h | W_m | W_l), m (W_h | W_m), l W_h, into
+//               three column ranges; above that six into one: the drain waits for what it reads beside the tensor core's own
+//               traffic, 1 100 cycles per step of 96 planes with two ranges, more than the step's 700 of instructions
 //   drain       8 warps, a row and half of the planes per lane: TMEM -> registers after every step, and after the tile's
 //               last one through shared memory -> bias -> optional BatchNorm -> 16-byte stores, four lanes per row
 // Bound by the copies into shared memory, 24 KB of rows and 6 (32 output planes) to 24 KB (128) of weights per step at about
@@ -76,7 +77,7 @@ struct SixParams {
 };
 
 // Warps by role.  With 64 planes per drain lane (and weights that leave room for four or five stages) fewer producers, for
-// 128 registers a thread.
+// 128 registers a thread.  (Two producing warps per step there: 96 -> 96 planes on 200 k rows 331 us, 288 with one.)
 template <int NA>
 struct SixWarps {
   static constexpr int PROD = NA == 64 ? 5 : 8;
@@ -87,7 +88,7 @@ template <int SP>
 struct SixShape {
   static constexpr unsigned HM = SP * 4, L = SP * 2;  // bytes of a row of a stage: [h | m], and [l]
   static constexpr unsigned A_BYTES = kRows * (HM + L);
-  static constexpr int PIECES = HM / 16, NI = kRows / (32 / PIECES);     // 16-byte pieces per row, rows per lane
+  static constexpr int PIECES = HM / 16, NI = kRows / (32 / PIECES);  // 16-byte pieces per row, rows per lane
   static constexpr int L_PIECES = L / 16, L_NI = kRows / (32 / L_PIECES);
   static_assert(HM == 128 || HM == 64, "swizzled rows");
 };
@@ -207,7 +208,6 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
   using Shape = SixShape<SP>;
   using Warps = SixWarps<NA>;
   constexpr int kProdWarps = Warps::PROD, kDrain0 = Warps::DRAIN0, kMma = Warps::MMA, kWgt = Warps::WGT, kEntries = Warps::ENTRIES;
-  constexpr int GROUP = 32 / SP;  // steps summed in tensor memory before they are drained
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const unsigned w_part = (unsigned)P.cb * SP * 2, w_bytes = w_part * 3;
@@ -217,8 +217,9 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
   int *entries = reinterpret_cast<int *>(tail);  // [kSlots][128] input row of every tile row, or -1
   unsigned char *epi = tail + sizeof(int) * kSlots * kRows;
   Ctl &C = *reinterpret_cast<Ctl *>(epi + kDrainWarps * kEpiBytes);
-  const bool joint = 3 * P.cb <= 256;  // [W_h | W_m | W_l] as one operand
-  const int dcols = ((joint ? 3 : 2) * P.cb + 31) & ~31;
+  constexpr bool kJoint = NA <= 32;             // (up to 64 planes) [W_h | W_m | W_l] as one operand, a range of columns for each
+  constexpr int kGroup = kJoint ? 32 / SP : 1;  // steps summed in tensor memory before they are drained
+  const int dcols = ((kJoint ? 3 : 1) * P.cb + 31) & ~31;
   const int n_acc = min(4, 512 / dcols);
   const long long my_items = items_here(P.n_items);  // (the grid has at most n_items CTAs)
 
@@ -258,8 +259,9 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
     // ==================================== producers =============================================
     // this lane's 16-byte piece of the rows q NI .. q NI + NI - 1, for [h | m] and again for [l]
     const int j = lane % Shape::PIECES, q = lane / Shape::PIECES, lj = lane % Shape::L_PIECES, lq = lane / Shape::L_PIECES;
-    const unsigned hm_dst = (unsigned)(q * Shape::NI) * Shape::HM + (unsigned)j * 16;
-    const unsigned l_dst = kRows * Shape::HM + (unsigned)(lq * Shape::L_NI) * Shape::L + (unsigned)lj * 16;
+    const int hm_row = q * Shape::NI, l_row = lq * Shape::L_NI;
+    const unsigned hm_dst = (unsigned)hm_row * Shape::HM + (unsigned)j * 16;
+    const unsigned l_dst = kRows * Shape::HM + (unsigned)l_row * Shape::L + (unsigned)lj * 16;
     // No more warps than stages: a warp at step n has seen the consumption of step n - active - n_stages, and its wait
     // below can tell step n - n_stages from the one a round earlier only if that one is not later than this.
     const int active = min(kProdWarps, P.n_stages);
@@ -277,8 +279,8 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
       const int slot_k = C.slot_k[si];
       if (slot_k < 0 || *abort) break;
       const int rows_in = slot_k >= kNoRules ? 0 : (int)P.n_in;  // entries below it are rows
-      const int4 *ent = reinterpret_cast<const int4 *>(entries + si * kRows + q * Shape::NI);
-      const int4 *l_ent = reinterpret_cast<const int4 *>(entries + si * kRows + lq * Shape::L_NI);
+      const int4 *ent = reinterpret_cast<const int4 *>(entries + si * kRows + hm_row);
+      const int4 *l_ent = reinterpret_cast<const int4 *>(entries + si * kRows + l_row);
       if (!mbar_wait(&C.empty[st], (round + 1) & 1)) {  // (the first round passes)
         ok = false;
         break;
@@ -293,7 +295,7 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
         for (int e = 0; e < 4; ++e) {
           const bool hit = (unsigned)v[e] < (unsigned)rows_in;
           bad |= v[e] >= (int)P.n_in && slot_k < kNoRules;
-          const unsigned swizzle = (Shape::HM == 128 ? (i + e) & 7 : ((i + e) >> 1) & 3) * 16;  // (q NI is a multiple of eight)
+          const unsigned swizzle = (Shape::HM == 128 ? (i + e) & 7 : ((i + e) >> 1) & 3) * 16;  // (hm_row is a multiple of eight)
           cp_async16(((stage + hm_dst) ^ swizzle) + (i + e) * Shape::HM, col + j * 16 + (size_t)(unsigned)(hit ? v[e] : 0) * P.row_bytes, hit ? 16u : 0u);
         }
       }
@@ -361,7 +363,7 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
     // ==================================== MMA issue =============================================
     // The whole warp runs the loop and one elected lane issues: with warp-uniform control flow and operands the
     // descriptors stay in uniform registers.
-    const unsigned id1 = tile_idesc(P.cb), id2 = tile_idesc(2 * P.cb), id3 = tile_idesc(joint ? 3 * P.cb : 16);
+    const unsigned id1 = tile_idesc(P.cb), id2 = tile_idesc(kJoint ? 2 * P.cb : 16), id3 = tile_idesc(kJoint ? 3 * P.cb : 16);
     const unsigned long long a_desc = rows_desc<Shape::HM>(smem0, 0), l_desc = rows_desc<Shape::L>(smem0, kRows * Shape::HM);
     const unsigned long long w_desc = smem_desc(smem0 + Shape::A_BYTES, 128, SP / 8 * 128);
     const unsigned a_hi = (unsigned)(a_desc >> 32), l_hi = (unsigned)(l_desc >> 32), w_hi = (unsigned)(w_desc >> 32);
@@ -377,8 +379,8 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
       const int steps = __reduce_max_sync(0xffffffffu, max(1, offsets_next)) * P.n_slices;
       offsets_next = item_offsets(P, item_of(i + 1));
       for (int s = 0; s < steps; ++s) {
-        const bool opens = GROUP == 1 || s % GROUP == 0, closes = GROUP == 1 || s % GROUP == GROUP - 1 || s == steps - 1;
-        // the accumulators must have been drained
+        const bool opens = s % kGroup == 0, closes = s % kGroup == kGroup - 1 || s == steps - 1;
+        // the accumulator must have been drained
         if (opens && (!mbar_wait_warp(&C.acc_empty[buf], buf_par) || __any_sync(0xffffffffu, *abort != 0))) {
           ok = false;
           break;
@@ -391,20 +393,33 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
           // order the copied rows (acquired through the barrier) before the tensor core's async-proxy reads
           fence_proxy_async_smem();
           tc_fence_after();
+          if (kJoint) {
 #pragma unroll
-          for (int jj = 0; jj < SP / 16; ++jj) {
-            const unsigned ah = a0 + at + jj * 2, am = ah + SP / 8, al = l0 + at + jj * 2, wh = w0 + at + jj * 16;
-            if (jj == 0) mma_bf16(d, ah, a_hi, wh, w_hi, joint ? id3 : id2, opens ? 0u : 1u);
-            else mma_bf16_acc(d, ah, a_hi, wh, w_hi, joint ? id3 : id2);
-            if (joint) {
+            for (int jj = 0; jj < SP / 16; ++jj) {
+              const unsigned ah = a0 + at + jj * 2, am = ah + SP / 8, al = l0 + at + jj * 2, wh = w0 + at + jj * 16;
+              if (jj == 0) mma_bf16(d, ah, a_hi, wh, w_hi, id3, opens ? 0u : 1u);
+              else mma_bf16_acc(d, ah, a_hi, wh, w_hi, id3);
               mma_bf16_acc(d + cb, am, a_hi, wh, w_hi, id2);
               mma_bf16_acc(d + 2 * cb, al, l_hi, wh, w_hi, id1);
-            } else {
-              mma_bf16_acc(d + cb, am, a_hi, wh, w_hi, id1);
-              mma_bf16_acc(d + cb, am, a_hi, wh + wm_step, w_hi, id1);
-              mma_bf16_acc(d + cb, ah, a_hi, wh + 2 * wm_step, w_hi, id1);
-              mma_bf16_acc(d + cb, al, l_hi, wh, w_hi, id1);
             }
+          } else {
+            const unsigned wm = wm_step, wl = 2 * wm_step;
+#pragma unroll
+            for (int jj = 0; jj < SP / 16; ++jj) {  // 2^-16 of a product, 2^-8, then the large ones
+              const unsigned ah = a0 + at + jj * 2, am = ah + SP / 8, al = l0 + at + jj * 2, wh = w0 + at + jj * 16;
+              if (jj == 0) mma_bf16(d, al, l_hi, wh, w_hi, id1, 0u);
+              else mma_bf16_acc(d, al, l_hi, wh, w_hi, id1);
+              mma_bf16_acc(d, ah, a_hi, wh + wl, w_hi, id1);
+              mma_bf16_acc(d, am, a_hi, wh + wm, w_hi, id1);
+            }
+#pragma unroll
+            for (int jj = 0; jj < SP / 16; ++jj) {
+              const unsigned ah = a0 + at + jj * 2, am = ah + SP / 8, wh = w0 + at + jj * 16;
+              mma_bf16_acc(d, am, a_hi, wh, w_hi, id1);
+              mma_bf16_acc(d, ah, a_hi, wh + wm, w_hi, id1);
+            }
+#pragma unroll
+            for (int jj = 0; jj < SP / 16; ++jj) mma_bf16_acc(d, a0 + at + jj * 2, a_hi, w0 + at + jj * 16, w_hi, id1);
           }
           tc_commit(&C.empty[st]);
           if (closes) tc_commit(&C.acc_full[buf]);
@@ -493,12 +508,12 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
       const long long item = item_of(it);
       const Item I = item_at(P, item);
       const int orow = __ldg(P.order + I.tile * kRows + quad * 32 + lane);
-      const int groups = (__reduce_max_sync(0xffffffffu, max(1, offsets_next)) * P.n_slices + GROUP - 1) / GROUP;
+      const int groups = (__reduce_max_sync(0xffffffffu, max(1, offsets_next)) * P.n_slices + kGroup - 1) / kGroup;
       offsets_next = item_offsets(P, item_of(it + 1));
       float acc[NA];
 #pragma unroll
       for (int e = 0; e < NA; ++e) acc[e] = 0.f;
-      for (int g = 0; g < groups; ++g) {
+      for (int s = 0; s < groups; ++s) {
         if (!mbar_wait_warp(&C.acc_full[buf], buf_par) || __any_sync(0xffffffffu, *abort != 0)) {
           ok = false;
           break;
@@ -508,18 +523,23 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
 #pragma unroll
         for (int u = 0; u < NA / 16; ++u)
           if (u < my_units) {
-#pragma unroll
-            for (int e0 = 0; e0 < 16; e0 += 8) {
-              unsigned a[8], b[8], c[8];
-              tmem_ld8_nowait(base + u * 16 + e0, a);
-              tmem_ld8_nowait(base + cb + u * 16 + e0, b);
-              if (joint) tmem_ld8_nowait(base + 2 * cb + u * 16 + e0, c);
+            if (!kJoint) {
+              unsigned a[16];
+              tmem_ld16_nowait(base + u * 16, a);
               tmem_wait_ld();
 #pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                float small = __uint_as_float(b[e]);
-                if (joint) small += __uint_as_float(c[e]);
-                acc[u * 16 + e0 + e] += __uint_as_float(a[e]) + small;
+              for (int e = 0; e < 16; ++e) acc[u * 16 + e] += __uint_as_float(a[e]);
+            } else {
+#pragma unroll
+              for (int e0 = 0; e0 < 16; e0 += 8) {
+                unsigned a[8], b[8], c[8];
+                tmem_ld8_nowait(base + u * 16 + e0, a);
+                tmem_ld8_nowait(base + cb + u * 16 + e0, b);
+                tmem_ld8_nowait(base + 2 * cb + u * 16 + e0, c);
+                tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                  acc[u * 16 + e0 + e] += __uint_as_float(a[e]) + (__uint_as_float(b[e]) + __uint_as_float(c[e]));
               }
             }
           }
@@ -692,22 +712,24 @@ extern thread_local int g_drop_arrival;  // test hook (conv_tc.cu)
 // multiply-adds cost less than six bytes per input value and rule, and for little work, where its one launch is the shorter
 // chain).  One layer,
 // 27 offsets, us on this kernel / on k_conv_fma, and the error of each against float64 (2-norm, products of mixed sign):
-//                 16->16      16->32      32->16      32->32      64->64       96->96       160->160      error (96->96)
-//   300 rows     14.4/12.1   15.3/11.8   14.7/11.3   13.7/12.0   16.0/11.3    19.7/11.9    22.1/17.1     0.8e-7 / 1.9e-7
-//   1 000        14.6/11.2   14.1/11.6   15.6/11.9   14.3/13.1   17.5/17.8    21.4/33.7    28.8/66.0     0.9e-7 / 2.8e-7
-//   2 000        14.6/11.7   15.3/12.4   14.4/13.2   14.6/14.4   18.8/26.3    24.3/51.2    39.9/104.8    0.8e-7 / 3.4e-7
-//   100 000      40/49                               51/84      109/224      179/561       483/1467
-//   200 000      63/57       65/77       84/77       86/114      185/354      302/895      813/2406      1.1e-7 / 5.3e-7
-//   1 600 000    446/403     441/601     617/544     615/872
+//                 16->16    16->32    24->32    32->32     64->64      96->96      160->160      error (96->96)
+//   600 rows      -         -         14.3/11.9 13.7/12.3  16.0/12.5   19.2/15.4   22.1/25.9     0.8e-7 / 2.0e-7
+//   1 000         14.6/11.2 14.1/11.6 14.1/12.1 14.3/13.1  16.6/14.3   20.0/24.3   24.1/47.2     0.9e-7 / 2.6e-7
+//   2 000         14.6/11.7 15.3/12.4 15.3/13.4 14.6/14.4  17.9/26.1   23.3/50.9   37.1/101.3    0.9e-7 / 3.4e-7
+//   9 000         -         21.2/19.8 19.2/22.3 19.2/25.3  28.8/59.5   42.7/123    92.9/329      1.0e-7 / 3.5e-7
+//   30 000        21/29     22/38     25/45     25/52      46/122      66/250      164/719       1.1e-7 / 5.3e-7
+//   200 000       63/57     66/80     83/100    85/118     180/370     281/932     709/2 622     1.2e-7 / 5.4e-7
+//   1 600 000     446/403   434/591   584/727   589/856
 //   99 000, 3-D shapes, 27 offsets: 8->16 45/42, 16->16 45/51, 32->16 57/67, 16->32 45/63
 //   91 000, 2-D strokes, 9 offsets: 16->16 28/21, 32->16 33/27, 16->32 28/26, 24->32 34/31, 32->32 34/37
-// Its error was the smaller one for every plane count from 8 to 224, 60 to 200 000 rows, products of mixed and of one sign.
+// Its error is the smaller one for every shape that comes here, 8 to 224 planes, 600 to 200 000 rows, products of mixed and
+// of one sign (16->32 on 9 000 rows of one sign, where k_conv_fma's sums are in parts: 6.5e-8 and 6.1e-8, so not here).
 bool conv_six_takes(const float *in, const float *in_b, int planes_a, const float *out, const float *bias, int K, int cin,
                     int cout, int groups, long long rows_in, long long rows_out) {
   return groups == 1 && K <= kOrderMaxOffsets && cin % 4 == 0 && cout % 4 == 0 && cout <= 256 && (cout > 16 || rows_out <= 131072) &&
          (!in_b || planes_a % 4 == 0) && ((uintptr_t)in | (uintptr_t)in_b | (uintptr_t)out | (uintptr_t)bias) % 16 == 0 &&
-         rows_in < (1ll << 31) && rows_out < (1ll << 31) && rows_out >= 512 &&
-         (double)K * cin * cout >= (K < 27 ? 9000 : 6900) && (double)K * rows_out * cin * cout >= 80e6;
+         rows_in < (1ll << 31) && rows_out < (1ll << 31) && rows_out >= 512 && (cin > 16 || rows_out >= 16384) &&
+         (double)K * cin * cout >= (K < 27 ? 9000 : 6900) && (double)K * rows_out * cin * cout >= (rows_out < 1500 ? 250e6 : 80e6);
 }
 
 // out [n_out, cout] = act((bias + sum_k in[table[k][.]] @ W[k]) * bn_scale + bn_shift) for the table that `ord` packs, the
@@ -794,7 +816,7 @@ int conv_forward_six(const float *in, long long n_in, float *out, long long n_ou
   P.flags = flags;
   P.drop = g_drop_arrival;
   g_drop_arrival = 0;
-  const double chunk = cb <= 80 ? std::max(56.0, 1.5 * cb) + std::max(56.0, 1.0 * cb) + 56 : cb + 4 * std::max(56.0, 0.5 * cb);
+  const double chunk = cb <= 64 ? std::max(56.0, 1.5 * cb) + std::max(56.0, 1.0 * cb) + 56 : 6 * std::max(56.0, 0.5 * cb);
   const double step = std::max((kRows * SP * 6.0 + cb * SP * 6.0) / 32.0, chunk * SP / 16);
   const char *e = getenv("SCN_SIX_SPLIT");
   P.n_split = e ? std::max(1, std::min(atoi(e), 64)) : split_parts(P.n_tiles, n_cb, ord.one_offset ? 1 : K, n_slices, step, cout, n_sm);
