@@ -1287,11 +1287,11 @@ static int build_strided(scn_metadata *md, Grid *gin, const int64_t *output_size
   rb.n_out = n_out;
   size_t nbr_bytes = sizeof(int) * (size_t)(K * std::max<long long>(n_out, 1));
   SCN_TRY(device_alloc((void **)&rb.nbr, nbr_bytes, stream));
-  SCN_TRY(device_alloc((void **)&rb.counts_dev, sizeof(unsigned long long) * (size_t)(2 * K + 1), stream));
+  SCN_TRY(device_alloc((void **)&rb.counts_dev, sizeof(unsigned long long) * (size_t)(2 * K + 2), stream));
   SCN_TRY(count_ticket_new(rb));
   Fills fills{};
   fill_add(fills, rb.nbr, nbr_bytes, true);
-  fill_add(fills, rb.counts_dev, sizeof(unsigned long long) * (size_t)(2 * K + 1), false);
+  fill_add(fills, rb.counts_dev, sizeof(unsigned long long) * (size_t)(2 * K + 2), false);
   if (n_ids == 0) {
     fill_add(fills, gout.table.slots, 2 * gout.table.n_buckets * sizeof(Slot), true);
     count_ticket_zero(rb);
@@ -1390,7 +1390,7 @@ static int chain_allocate(std::vector<ChainLevel> &plan, cudaStream_t alloc_stre
     SCN_TRY(device_alloc((void **)&lv.gout.table.slots, slots * sizeof(Slot), alloc_stream));
     SCN_TRY(device_alloc((void **)&lv.gout.row_keys, sizeof(unsigned long long) * cap, alloc_stream));
     SCN_TRY(device_alloc((void **)&lv.rb.nbr, sizeof(int) * (size_t)lv.K * cap, alloc_stream));
-    SCN_TRY(device_alloc((void **)&lv.rb.counts_dev, sizeof(unsigned long long) * (size_t)(2 * lv.K + 1), alloc_stream));
+    SCN_TRY(device_alloc((void **)&lv.rb.counts_dev, sizeof(unsigned long long) * (size_t)(2 * lv.K + 2), alloc_stream));
     lv.rb.n_offsets = (int)lv.K;
     SCN_TRY(count_ticket_new(lv.rb));
     if (lv.bound_in == 0) count_ticket_zero(lv.rb);
@@ -1418,7 +1418,7 @@ static int chain_enqueue(scn_metadata *md, const Grid *gin, std::vector<ChainLev
     const size_t cap = (size_t)std::max<long long>(lv.cap_out, 1);
     fill_add(fills, lv.gout.table.slots, 2 * lv.gout.table.n_buckets * sizeof(Slot), true);
     fill_add(fills, lv.rb.nbr, sizeof(int) * (size_t)lv.K * cap, true);
-    fill_add(fills, lv.rb.counts_dev, sizeof(unsigned long long) * (size_t)(2 * lv.K + 1), false);
+    fill_add(fills, lv.rb.counts_dev, sizeof(unsigned long long) * (size_t)(2 * lv.K + 2), false);
   }
   SCN_TRY(fill_launch(fills, stream));
   const unsigned long long *in_keys = gin->row_keys;

@@ -73,8 +73,8 @@ struct Rulebook {
   // offsets with a rule of every output row of nbr, mask_words(K) words each (submanifold rulebooks up to
   // kOrderMaxOffsets offsets; null otherwise)
   unsigned *masks = nullptr;
-  // [K] rules per offset, then the builder's count of finished blocks; of a strided rulebook K more zeros behind them
-  // (rulebook_children_order)
+  // [K] rules per offset, then the builder's count of finished blocks; of a strided rulebook K + 1 more zeros behind
+  // them (rulebook_children_order)
   unsigned long long *counts_dev = nullptr;
   std::vector<long long> counts_host;        // filled on first request (waits for the stream)
   long long total_rules = -1;

@@ -216,7 +216,8 @@ k_order_plain(const int *__restrict__ nbr, long long n, int K, int words, int *_
 // Fine rows with one rule each (a Deconvolution whose filter is its stride) by the offset of that rule, from the table as the
 // Convolution has it (nbr [K][n_out] = fine row or -1) and the rules per offset that its builder has counted: whole tiles
 // of one offset, -1 behind an offset's last row.  A block takes a run of the offset's places for its coarse rows, so the
-// blocks come in the order in which they get there; what a row's sum is does not depend on the tile it is in.  One launch
+// blocks come in the order in which they get there; what a row's sum is does not depend on the tile it is in.  The block
+// that finishes last clears the cursors, so that the launch can be repeated (a graph that has recorded it).  One launch
 // where the transposed table, its masks, a counting pass and the tiles were six: 17 us per level on small levels, 95 on
 // 1.6 M rows, now 5 and 14.
 __global__ void __launch_bounds__(256)
@@ -262,8 +263,9 @@ k_order_children(const int *__restrict__ nbr, long long n_out, int K, const unsi
   for (int k = 0; k < K; ++k) {
     const int v = o < n_out ? __ldg(nbr + k * n_out + o) : -1;
     const unsigned hits = __ballot_sync(0xffffffffu, v >= 0);
-    if (v >= 0) {
-      const long long p = (long long)start[k] * kTile + base[k] + before[warp][k] + __popc(hits & ((1u << lane) - 1u));
+    const long long at = base[k] + before[warp][k] + __popc(hits & ((1u << lane) - 1u));
+    if (v >= 0 && at < (long long)counts[k]) {
+      const long long p = (long long)start[k] * kTile + at;
       order[p] = v;
       packed[p / kTile * K * kTile + p % kTile] = (int)o;
     }
@@ -283,6 +285,9 @@ k_order_children(const int *__restrict__ nbr, long long n_out, int K, const unsi
         packed[p / kTile * K * kTile + p % kTile] = -1;
       }
     }
+  __syncthreads();
+  if (tid == 0 && atomicAdd(&cursors[K], 1ull) == (unsigned long long)gridDim.x - 1)
+    for (int k = 0; k <= K; ++k) cursors[k] = 0;
 }
 
 // The tiles by how many offsets they have, most first, stable (run by one block of 256 threads, the last of k_order_tiles to
