@@ -14,11 +14,11 @@
 // low part.  The pass that splits rows and weights leaves the largest magnitude of either; where a product could overflow, or
 // fall to where its parts do not reach, the kernel multiplies plain fp32 values instead (slow_item).
 //
-// Roles (19 or 16 warps, one CTA per SM, persistent), as in k_conv_tile but for the drain:
+// Roles (20 or 16 warps, one CTA per SM, persistent), as in k_conv_tile but for the drain:
 //   entries     one thread: a slot per (tile, filter offset with a rule), 512 bytes of input rows from the packed table
-//   producers   8 (5) warps, a step each: 128 rows of 192 bytes ([32 h | 32 m] and [32 l]) by 16-byte cp.async
+//   producers   8 (4) warps, a step each: 128 rows of 192 bytes ([32 h | 32 m] and [32 l]) by 16-byte cp.async
 //   weights     one thread: one bulk copy of [W_h | W_m | W_l] per step
-//   MMA         up to 64 output planes three instructions per 16 input planes, h (W_h | W_m | W_l), m (W_h | W_m), l W_h, into
+//   MMA         two warps; up to 64 output planes three instructions per 16 input planes, h (W_h | W_m | W_l), m (W_h | W_m), l W_h, into
 //               three column ranges; above that six into one: the drain waits for what it reads beside the tensor core's own
 //               traffic, 1 100 cycles per step of 96 planes with two ranges, more than the step's 700 of instructions
 //   drain       8 warps, a row and half of the planes per lane: TMEM -> registers after every step, and after the tile's
@@ -43,7 +43,7 @@ namespace scn {
 namespace {
 
 constexpr int kRows = kOrderTile;
-constexpr int kDrainWarps = 8;
+constexpr int kDrainWarps = 8, kMmaWarps = 2;
 constexpr int kSlots = 8;  // offsets the entries run ahead; at least the producing warps (the slots that end the work)
 constexpr int kMaxStages = 12;
 constexpr int kEpiBytes = 32 * 64;   // per drain warp: 32 rows x 16 planes on their way from lanes to whole lines
@@ -76,12 +76,12 @@ struct SixParams {
   int *flags;
 };
 
-// Warps by role.  With 64 planes per drain lane (and weights that leave room for four or five stages) fewer producers, for
+// Warps by role.  With 64 planes per drain lane (and weights that leave room for four stages) fewer producers, for
 // 128 registers a thread.  (Two producing warps per step there: 96 -> 96 planes on 200 k rows 331 us, 288 with one.)
 template <int NA>
 struct SixWarps {
-  static constexpr int PROD = NA == 64 ? 5 : 8;
-  static constexpr int DRAIN0 = PROD, MMA = DRAIN0 + kDrainWarps, WGT = MMA + 1, ENTRIES = MMA + 2, THREADS = (ENTRIES + 1) * 32;
+  static constexpr int PROD = NA == 64 ? 4 : 8;
+  static constexpr int DRAIN0 = PROD, MMA = DRAIN0 + kDrainWarps, WGT = MMA + kMmaWarps, ENTRIES = WGT + 1, THREADS = (ENTRIES + 1) * 32;
 };
 
 template <int SP>
@@ -220,14 +220,14 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
   constexpr bool kJoint = NA <= 32;             // (up to 64 planes) [W_h | W_m | W_l] as one operand, a range of columns for each
   constexpr int kGroup = kJoint ? 32 / SP : 1;  // steps summed in tensor memory before they are drained
   const int dcols = ((kJoint ? 3 : 1) * P.cb + 31) & ~31;
-  const int n_acc = min(4, 512 / dcols);
+  const int n_acc = min(4, 512 / dcols) & ~1;  // (an accumulator belongs to one of the issuing warps)
   const long long my_items = items_here(P.n_items);  // (the grid has at most n_items CTAs)
 
   if (tid < 2) C.range[tid] = 0;
   if (tid == 0) {
     for (int i = 0; i < P.n_stages; ++i) {
       mbar_init(&C.full[i], 32 + 1);  // the producing warp's lanes and the weights
-      mbar_init(&C.empty[i], 1);
+      mbar_init(&C.empty[i], kMmaWarps);
     }
     for (int i = 0; i < kSlots; ++i) {
       mbar_init(&C.s_full[i], 1);
@@ -359,10 +359,11 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
         }
       }
     }
-  } else if (warp == kMma) {
+  } else if (warp < kMma + kMmaWarps && warp >= kMma) {
     // ==================================== MMA issue =============================================
-    // The whole warp runs the loop and one elected lane issues: with warp-uniform control flow and operands the
-    // descriptors stay in uniform registers.
+    // Two warps take the accumulators in turn: what one spends on barriers passes while the other's instructions run (U-Net
+    // of two rooms 2 985 -> 2 950 us).  The whole warp runs the loop and one elected lane issues: with warp-uniform control
+    // flow and operands the descriptors stay in uniform registers.
     const unsigned id1 = tile_idesc(P.cb), id2 = tile_idesc(kJoint ? 2 * P.cb : 16), id3 = tile_idesc(kJoint ? 3 * P.cb : 16);
     const unsigned long long a_desc = rows_desc<Shape::HM>(smem0, 0), l_desc = rows_desc<Shape::L>(smem0, kRows * Shape::HM);
     const unsigned long long w_desc = smem_desc(smem0 + Shape::A_BYTES, 128, SP / 8 * 128);
@@ -374,6 +375,7 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
     unsigned at = 0, d = tmem;
     bool ok = true;
     const bool leader = elect_one();
+    bool mine = warp == kMma;  // the next accumulator is this warp's
     int offsets_next = item_offsets(P, item_of(0));
     for (int i = 0; i < items && ok; ++i) {
       const int steps = __reduce_max_sync(0xffffffffu, max(1, offsets_next)) * P.n_slices;
@@ -381,7 +383,7 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
       for (int s = 0; s < steps; ++s) {
         const bool opens = s % kGroup == 0, closes = s % kGroup == kGroup - 1 || s == steps - 1;
         // the accumulator must have been drained
-        if (opens && (!mbar_wait_warp(&C.acc_empty[buf], buf_par) || __any_sync(0xffffffffu, *abort != 0))) {
+        if (opens && mine && (!mbar_wait_warp(&C.acc_empty[buf], buf_par) || __any_sync(0xffffffffu, *abort != 0))) {
           ok = false;
           break;
         }
@@ -389,7 +391,11 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
           ok = false;
           break;
         }
-        if (leader) {
+        // (the other warp's steps too, and a stage goes when both have been here: neither can fall a round behind, or run a round
+        // ahead, where a phase's parity is that of another)
+        if (!mine) {
+          if (leader) mbar_arrive(&C.empty[st]);
+        } else if (leader) {
           // order the copied rows (acquired through the barrier) before the tensor core's async-proxy reads
           fence_proxy_async_smem();
           tc_fence_after();
@@ -428,6 +434,7 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
         at += stage_step;
         if (++st == n_stages) st = 0, par ^= 1, at = 0;
         if (closes) {
+          mine = !mine;
           d += dcols;
           if (++buf == n_acc) buf = 0, buf_par ^= 1, d = tmem;
         }
