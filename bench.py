@@ -41,18 +41,20 @@ UNIT = "voxels/s"
 # launches against their algorithmic bytes).  The traffic grows with the rows, like the
 # algorithmic bytes: DRAM sees input, rulebook and output about once, the gather's re-reads
 # (which the algorithmic figure counts per rule) hit L2.
-TRAFFIC_RATIO = {"k_conv_tile": 0.27, "k_conv_fma": 0.25}
+TRAFFIC_RATIO = {"k_conv_tile": 0.27}
 # (bound reported for the kernel, what the ncu captures show as its limiter)
 LIMITS = {
     "k_conv_tile": ("hbm", "the gather of whole rows from L2 into shared memory by 16-byte cp.async (ncu, 4-room case): LSU "
                            "wavefronts 39 % of peak on average and up to 53 %, tensor pipe 25 % (43 % on the widest levels), "
                            "issue slots 28 %; DRAM sees 0.27 of the algorithmic bytes"),
-    "k_conv_fma": ("hbm", "the FMA pipe behind two block barriers per step (ncu, 4-room case, the four finest levels): FMA pipe "
-                          "51 % (60 % at 64 planes), issue slots 64 %, LSU wavefronts 48 %, a fifth of the warp slots filled"),
+    "k_conv_fma": ("hbm", "fp32 on tiles, most of it k_conv_six: the copies of rows and weights into shared memory, 30 to 48 KB per "
+                          "step of 128 rows and 32 planes, and the drain of the step's sums beside the tensor core (timed inside "
+                          "the kernel: 1 050 to 1 700 cycles per step, 340 to 800 of them tensor instructions)"),
 }
 # what `dtype` says for each arithmetic mode: the type the path computes in, kernel by kernel
 DTYPE_LABEL = {
-    "fp32": "f32 (fp32 FMA in every convolution)",
+    "fp32": "f32 (fp32 FMA, or every operand as three bf16 parts that hold it exactly and six bf16 products per term on "
+            "tcgen05, added up in fp32 registers every 32 planes, with the smaller error of the two)",
     "tf32x3": "f32-class split arithmetic, fp32 accumulate: every operand as two bf16 parts, three bf16 products "
               "per term on tcgen05 kind::f16 with TMEM accumulators",
     "tf32": "f32-class split arithmetic as tf32x3 (the mode asks for no less than one tf32 product); the first layer fp32",

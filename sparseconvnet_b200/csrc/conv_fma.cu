@@ -1,4 +1,5 @@
-// fp32 sparse convolution (fused multiply-adds only) over mask-sorted row tiles.
+// fp32 sparse convolution (fused multiply-adds only) over mask-sorted row tiles: few output planes on many rows, small levels
+// and little work; the rest of the fp32 mode runs on tensor cores (conv_six.cu: conv_six_takes has the line and both sides).
 //
 // Same arithmetic class as k_conv_pipe (conv_pipe.cu) and k_conv_simt (conv_simt.cu; the reference's per-offset gather /
 // GEMM / scatter-add is CPU/Convolution.cpp:137-148, CUDA/Convolution.cu:57-233): fp32 products, fp32 sums.  A CTA of 128
