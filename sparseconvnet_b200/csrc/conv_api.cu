@@ -361,10 +361,6 @@ int conv_forward_dispatch(const float *in, long long rows_in, float *out, long l
   return SCN_OK;
 }
 
-// `disjoint` (only with `transposed`): every output row has exactly one rule (filter = stride).
-// `disjoint` additionally promises that every output row HAS a rule: the caller clears it when the
-// fine grid may hold rows that are in no map (earlier duplicates under input mode 0), whose output
-// the scatter form would leave unwritten while the gather form and the reference give them the bias.
 // Does the convolution of a rulebook table run on mask-sorted tensor-core tiles?  Every bf16-class shape the kernel takes.
 static bool tile_takes(const float *in, const float *in_b, int planes_a, const float *out, const float *bias, int K, int cin,
                        int cout, int groups, int precision, long long rows_out) {
@@ -435,19 +431,9 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
   return rc;
 }
 
-// Has every fine row of a strided rulebook exactly one rule?  Filter = stride: the children of different coarse sites and
-// offsets never coincide.  (Rows in no map, earlier duplicates under input mode 0, have none.)
-bool one_rule_per_row(scn_metadata *md, const int64_t *fine_size, const int64_t *coarse_size, const int64_t *filter_size,
-                      const int64_t *filter_stride) {
-  for (int d = 0; d < md->dim; ++d)
-    if (filter_size[d] != filter_stride[d] || coarse_size[d] * filter_stride[d] < fine_size[d]) return false;
-  const Grid *fine = find_grid(md, fine_size);
-  return fine && !fine->may_have_blank_rows;
-}
-
 static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float *in, float *out,
                     const float *weight, const float *bias, int n_in_planes, int n_out_planes, int groups,
-                    int precision, cudaStream_t stream, double *macs, bool disjoint = false,
+                    int precision, cudaStream_t stream, double *macs,
                     const float *bn_scale = nullptr, const float *bn_shift = nullptr, float leak = 1.f,
                     const float *pre_scale = nullptr, const float *pre_shift = nullptr, float pre_leak = 1.f,
                     const float *in_b = nullptr, int planes_a = 0) {
@@ -480,8 +466,9 @@ static int run_conv(scn_metadata *md, Rulebook &rb, bool transposed, const float
     }
   }
   const bool tile = tile_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, precision, rows_out);
-  // the transposed layer with one rule per output row runs from its input side, on the table as built
-  const bool scatter = !tile && transposed && disjoint && precision == SCN_PRECISION_TF32X3 && rows_in > 0 &&
+  // The transposed layer with one rule per output row runs from its input side, on the table as built.  (Rows without a rule,
+  // which get the bias, would be left unwritten: one_parent is false where there may be any.)
+  const bool scatter = !tile && transposed && rb.one_parent && precision == SCN_PRECISION_TF32X3 && rows_in > 0 &&
                        !(getenv("SCN_X3_ROWS") && atoi(getenv("SCN_X3_ROWS")) == 0) &&
                        !(getenv("SCN_ROWS_SCATTER") && atoi(getenv("SCN_ROWS_SCATTER")) == 0) &&
                        conv_rows_supported(in, out, weight, bias, rb.n_offsets, cin, cout, groups);
@@ -626,9 +613,8 @@ int scn_deconvolution_forward(scn_metadata *md, const int64_t *input_size, const
   Rulebook *rb = nullptr;
   // the rulebook of the matching Convolution: fine (this op's output) -> coarse (this op's input)
   SCN_TRY(get_strided_rulebook(md, output_size, input_size, filter_size, filter_stride, stream, &rb));
-  const bool disjoint = rb->one_parent = one_rule_per_row(md, output_size, input_size, filter_size, filter_stride);
   return run_conv(md, *rb, true, in_features, out_features, weight, bias, n_in_planes, n_out_planes,
-                  groups, precision, stream, macs, disjoint);
+                  groups, precision, stream, macs);
 }
 
 /* ---- convolutions with the eval-mode BatchNorm (+ leaky ReLU) that follows them applied in the store ---- */
@@ -653,7 +639,7 @@ int scn_submanifold_convolution_bn_forward(scn_metadata *md, const int64_t *spat
   Rulebook *rb = nullptr;
   SCN_TRY(get_submanifold_rulebook(md, spatial_size, filter_size, stream, &rb));
   return run_conv(md, *rb, false, in_features, out_features, weight, bias, n_in_planes, n_out_planes, groups,
-                  precision, stream, macs, false, bn_scale, bn_shift, (float)leakiness);
+                  precision, stream, macs, bn_scale, bn_shift, (float)leakiness);
 }
 
 int scn_convolution_bn_forward(scn_metadata *md, const int64_t *input_size, const int64_t *output_size,
@@ -667,7 +653,7 @@ int scn_convolution_bn_forward(scn_metadata *md, const int64_t *input_size, cons
   Rulebook *rb = nullptr;
   SCN_TRY(get_strided_rulebook(md, input_size, output_size, filter_size, filter_stride, stream, &rb));
   return run_conv(md, *rb, false, in_features, out_features, weight, bias, n_in_planes, n_out_planes, groups,
-                  precision, stream, macs, false, bn_scale, bn_shift, (float)leakiness);
+                  precision, stream, macs, bn_scale, bn_shift, (float)leakiness);
 }
 
 int scn_submanifold_convolution_joined_forward(scn_metadata *md, const int64_t *spatial_size, const int64_t *filter_size,
@@ -686,7 +672,7 @@ int scn_submanifold_convolution_joined_forward(scn_metadata *md, const int64_t *
   SCN_TRY(get_submanifold_rulebook(md, spatial_size, filter_size, stream, &rb));
   SCN_REQUIRE(rb->n_in == 0 || (in_a && (in_b || single)), SCN_ERR_BAD_ARG, "null features");
   return run_conv(md, *rb, false, in_a, out_features, weight, bias, planes_a + planes_b, n_out_planes, 1, precision,
-                  stream, macs, false, bn_scale, bn_shift, (float)leakiness, pre_scale, pre_shift, (float)pre_leakiness,
+                  stream, macs, bn_scale, bn_shift, (float)leakiness, pre_scale, pre_shift, (float)pre_leakiness,
                   in_b, single ? 0 : planes_a);
 }
 
@@ -702,7 +688,7 @@ int scn_convolution_bn_bn_forward(scn_metadata *md, const int64_t *input_size, c
   Rulebook *rb = nullptr;
   SCN_TRY(get_strided_rulebook(md, input_size, output_size, filter_size, filter_stride, stream, &rb));
   return run_conv(md, *rb, false, in_features, out_features, weight, bias, n_in_planes, n_out_planes, groups,
-                  precision, stream, macs, false, bn_scale, bn_shift, (float)leakiness, pre_scale, pre_shift,
+                  precision, stream, macs, bn_scale, bn_shift, (float)leakiness, pre_scale, pre_shift,
                   (float)pre_leakiness);
 }
 
@@ -716,8 +702,7 @@ int scn_deconvolution_bn_forward(scn_metadata *md, const int64_t *input_size, co
               "null argument");
   Rulebook *rb = nullptr;
   SCN_TRY(get_strided_rulebook(md, output_size, input_size, filter_size, filter_stride, stream, &rb));
-  const bool disjoint = rb->one_parent = one_rule_per_row(md, output_size, input_size, filter_size, filter_stride);
   return run_conv(md, *rb, true, in_features, out_features, weight, bias, n_in_planes, n_out_planes, groups,
-                  precision, stream, macs, disjoint, bn_scale, bn_shift, (float)leakiness);
+                  precision, stream, macs, bn_scale, bn_shift, (float)leakiness);
 }
 }

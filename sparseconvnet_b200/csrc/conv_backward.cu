@@ -22,8 +22,6 @@
 namespace scn {
 
 extern std::atomic<int> g_backward_precision;
-bool one_rule_per_row(scn_metadata *md, const int64_t *fine_size, const int64_t *coarse_size, const int64_t *filter_size,
-                      const int64_t *filter_stride);
 int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, long long rows_in, float *out,
                        long long rows_out, const float *weight, const float *bias, int cin, int cout, int groups,
                        int precision, int *flags, cudaStream_t stream, const float *bn_scale = nullptr,
@@ -640,7 +638,6 @@ int scn_convolution_backward(scn_metadata *md, const int64_t *input_size, const 
   SCN_REQUIRE(md && input_size && output_size && filter_size && filter_stride, SCN_ERR_BAD_ARG, "null argument");
   Rulebook *rb = nullptr;
   SCN_TRY(get_strided_rulebook(md, input_size, output_size, filter_size, filter_stride, stream, &rb));
-  rb->one_parent = one_rule_per_row(md, input_size, output_size, filter_size, filter_stride);
   return run_conv_backward(md, *rb, false, in_features, d_in_features, d_out_features, weight, d_weight, d_bias,
                            n_in_planes, n_out_planes, groups, stream);
 }

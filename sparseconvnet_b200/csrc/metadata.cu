@@ -1205,6 +1205,15 @@ k_strided_fill(KeyLayout Lin, KeyLayout Lout, FilterDesc F, Slot *slots, const u
 }
 
 // (what it leaves in `gout` and `rb` when it fails is the caller's to free)
+// Does every site of a fine grid have exactly one rule in the rulebook of F?  Filter = stride: the children of different
+// coarse sites and offsets never coincide, and none is left out where the coarse grid covers the fine one.  (Rows in no map,
+// earlier duplicates under input mode 0, have none.)
+static bool one_rule_per_row(const KeyLayout &fine, bool may_have_blank_rows, const FilterDesc &F) {
+  for (int d = 0; d < fine.dim; ++d)
+    if (F.f[d] != F.s[d] || (long long)F.out_size[d] * F.s[d] < fine.size[d]) return false;
+  return !may_have_blank_rows;
+}
+
 static int build_strided(scn_metadata *md, Grid *gin, const int64_t *output_size, const int64_t *filter_size,
                          const int64_t *filter_stride, cudaStream_t stream, Grid &gout, Rulebook &rb) {
   SCN_TRY(ensure_scratch(md, stream));
@@ -1285,6 +1294,7 @@ static int build_strided(scn_metadata *md, Grid *gin, const int64_t *output_size
   for (int d = 0; d < md->dim; ++d) rb.filter[d] = filter_size[d];
   rb.n_in = n_in;
   rb.n_out = n_out;
+  rb.one_parent = one_rule_per_row(gin->layout, gin->may_have_blank_rows, F);
   size_t nbr_bytes = sizeof(int) * (size_t)(K * std::max<long long>(n_out, 1));
   SCN_TRY(device_alloc((void **)&rb.nbr, nbr_bytes, stream));
   SCN_TRY(device_alloc((void **)&rb.counts_dev, sizeof(unsigned long long) * (size_t)(2 * K + 2), stream));
@@ -1480,6 +1490,8 @@ static void chain_plan(scn_metadata *md, const Grid *gin, const std::vector<int6
     if (make_layout(dim, lv.out_size.data(), lv.gout.layout) != SCN_OK) break;
     if (!(lv.gout.layout.batch_bits >= gin->layout.batch_bits || gin->batch_size <= (1ll << lv.gout.layout.batch_bits)))
       break;
+    lv.rb.one_parent = plan.empty() ? one_rule_per_row(gin->layout, gin->may_have_blank_rows, lv.F)
+                                    : one_rule_per_row(plan.back().gout.layout, false, lv.F);
     lv.bound_in = bound;
     // Sites of the level: at most one per candidate (and no more than the output volume).  Disjoint windows
     // (filter == stride) give at most one site per input site, and the arrays are first sized for half of that;

@@ -63,3 +63,52 @@ def test_children(n, dim, filt, corner, precision, tol, cuda):
     for got, exact in ((z, want), (fine.grad, grad)):
         e = helpers.rel_err(got.double().cpu().numpy(), exact.cpu().numpy())
         assert e <= tol, e
+
+
+@pytest.mark.parametrize("precision,tol", [("fp32", 1e-6), ("tf32x3", helpers.FP32_TOL)])
+def test_rows_without_a_rule(precision, tol, cuda):
+    """A rulebook built for a coarse grid that does not cover the fine one, found again by a call that names one that does
+    (rulebooks are found by fine size, filter and stride): the rows left out get the bias, and no gradient."""
+    import ctypes as C
+
+    import sparseconvnet_b200 as scn
+    from sparseconvnet_b200 import SCN
+    from sparseconvnet_b200._lib import check, lib, sizes
+    torch.manual_seed(5)
+    x = scn.InputLayer(3, 48, mode=1)([torch.from_numpy(_points(4000, 3, 48, False)), torch.zeros(4000, 1, device=cuda)])
+    md, n, two = x.metadata._h, x.features.size(0), sizes([2] * 3)
+    cin, cout = 64, 48
+    w, bias = torch.randn(8, 1, cin, cout, device=cuda), torch.randn(cout, device=cuda)
+    f = torch.randn(n, cout, device=cuda)
+    y = f.new_empty(0)
+    SCN.Convolution_updateOutput(x.spatial_size, torch.LongTensor([20] * 3), torch.LongTensor([2] * 3), torch.LongTensor([2] * 3),
+                                 x.metadata, f, y, torch.randn(8, 1, cout, cin, device=cuda), f.new_empty(0))
+    g = torch.randn(y.size(0), cin, device=cuda)
+    out, d_in = (torch.full((n, cout), float("nan"), device=cuda) for _ in range(2))
+    dw = torch.empty(8, 1, cout, cin, device=cuda)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def ptr(t):
+        return C.c_void_p(t.data_ptr())
+    wide = sizes([24] * 3), sizes([48] * 3)
+    w_back = w.transpose(2, 3).contiguous()
+    try:
+        scn.set_backward_precision(precision)
+        check(lib.scn_deconvolution_forward(md, wide[0], wide[1], two, two, ptr(g), ptr(out), ptr(w), ptr(bias), cin, cout, 1,
+                                            {"fp32": 0, "tf32x3": 3}[precision], stream, None))
+        check(lib.scn_convolution_backward(md, wide[1], wide[0], two, two, ptr(f), ptr(d_in), ptr(g), ptr(w_back), ptr(dw), None,
+                                           cout, cin, 1, stream))
+        x.metadata.poll_errors()
+    finally:
+        scn.set_backward_precision("fp32")
+    want, grad = bias.double().expand(n, cout).clone(), torch.zeros(n, cout, dtype=torch.float64, device=cuda)
+    seen = torch.zeros(n, dtype=torch.long, device=cuda)
+    for r, m in zip(x.metadata.rulebook(1, x.spatial_size, [2] * 3, [2] * 3), w.double()[:, 0]):
+        r = r.long()
+        seen[r[:, 0]] += 1
+        want.index_add_(0, r[:, 0], g.double()[r[:, 1]] @ m)
+        grad.index_add_(0, r[:, 0], g.double()[r[:, 1]] @ m)
+    assert 0 < int((seen == 0).sum()) < n and int(seen.max()) == 1
+    for got, exact in ((out, want), (d_in, grad)):
+        e = helpers.rel_err(got.double().cpu().numpy(), exact.cpu().numpy())
+        assert e <= tol, e
