@@ -10,9 +10,12 @@
 //     registers, rounded to nearest (the "drain" warps).
 // Time and error against float64 beside k_conv_fma's: the table at conv_six_takes.
 //
-// The range of bf16 is that of fp32 except at its ends: the low parts of a tiny value would be lost, and an infinity has no
-// low part.  The pass that splits rows and weights leaves the largest magnitude of either; where a product could overflow, or
-// fall to where its parts do not reach, the kernel multiplies plain fp32 values instead (slow_item).
+// The range of bf16 is that of fp32, so the low parts of a value near its lower end would be lost.  Rows and weights are split
+// 2^24 times as large as they are and sums made 2^48 times smaller: then the last bit of the smallest fp32 value is a normal
+// bf16 number, and the terms of a product are exact for every product that is a normal number, whatever stands beside it.
+// Upwards that leaves less room, and an infinity has no low part: the pass that splits leaves the largest magnitude of rows and
+// weights, and where a sum could overflow the kernel multiplies plain fp32 values instead (slow_item).  So it does where the
+// largest products are near the lower end, where k_conv_fma's own rounding of subnormal sums is kept.
 //
 // Roles (20 or 16 warps, one CTA per SM, persistent), as in k_conv_tile but for the drain:
 //   entries     one thread: a slot per (tile, filter offset with a rule), 512 bytes of input rows from the packed table
@@ -47,6 +50,8 @@ constexpr int kDrainWarps = 8, kMmaWarps = 2;
 constexpr int kSlots = 8;  // offsets the entries run ahead; at least the producing warps (the slots that end the work)
 constexpr int kMaxStages = 12;
 constexpr int kEpiBytes = 32 * 64;   // per drain warp: 32 rows x 16 planes on their way from lanes to whole lines
+constexpr int kScale = 24;           // of rows and of weights, as a power of two
+constexpr float kUp = 1 << kScale, kDown = 1.f / kUp / kUp;
 constexpr int kRangeWords = 512;     // behind split rows and weight image: largest magnitude (float bits), one per block
 constexpr int kPrepareThreads = 512, kPrepareBlocks = 296;
 
@@ -182,16 +187,17 @@ __device__ __forceinline__ void slow_item(const SixParams &P, long long item, in
 }
 
 // Can sums of 2^log2_terms products of values up to x and w in magnitude (float bits) be made of bf16 parts?  Nothing may
-// reach infinity on the way, and the last part of the largest values has to stay a normal number.
+// reach infinity on the way.
 __device__ __forceinline__ bool parts_reach(unsigned x, unsigned w, int log2_terms) {
   const int ex = (int)(x >> 23) - 127, ew = (int)(w >> 23) - 127;  // (128: infinity or NaN)
-  if (ex >= 126 || ew >= 126) return false;
+  if (ex + kScale >= 126 || ew + kScale >= 126) return false;
   if (x == 0 || w == 0) return true;
-  return ex >= -60 && ew >= -60 && ex + ew >= -90 && ex + ew + 2 + log2_terms < 126;
+  return ex >= -60 && ew >= -60 && ex + ew >= -90 && ex + ew + 2 * kScale + 2 + log2_terms < 126;
 }
 
-// x = h + m + l, two values at a time (the first in the low half)
+// 2^24 x = h + m + l, two values at a time (the first in the low half)
 __device__ __forceinline__ void split3_pair(float a, float b, unsigned &h, unsigned &m, unsigned &l) {
+  a *= kUp, b *= kUp;
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   h = *reinterpret_cast<unsigned *>(&v);
   const float a1 = a - __uint_as_float(h << 16), b1 = b - __uint_as_float(h & 0xFFFF0000u);
@@ -565,7 +571,7 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
         if (u < my_units) {
 #pragma unroll
           for (int e = 0; e < 16; e += 4)
-            my_epi[lane * 4 + ((e >> 2) ^ ((lane >> 1) & 3))] = make_float4(acc[u * 16 + e], acc[u * 16 + e + 1], acc[u * 16 + e + 2], acc[u * 16 + e + 3]);
+            my_epi[lane * 4 + ((e >> 2) ^ ((lane >> 1) & 3))] = make_float4(acc[u * 16 + e] * kDown, acc[u * 16 + e + 1] * kDown, acc[u * 16 + e + 2] * kDown, acc[u * 16 + e + 3] * kDown);
           __syncwarp();
           const int c = I.block * cb + (first_unit + u) * 16 + (lane & 3) * 4;
           if (c < nc) {

@@ -95,6 +95,35 @@ def test_values_the_parts_cannot_hold(case, cin, cout, n, cuda, monkeypatch):
         assert torch.equal(torch.nan_to_num(got, nan=7.0), torch.nan_to_num(want, nan=7.0))
 
 
+@pytest.mark.parametrize("small", [1e-30, 1e-35, 1e-37])
+@pytest.mark.parametrize("cin,cout", [(24, 32), (32, 32), (40, 136)])
+def test_small_values_beside_ordinary_ones(small, cin, cout, cuda):
+    """A sample of small values beside an ordinary one, output planes of small weights beside ordinary ones: each as accurate by
+    itself (results of 1e-36 and above, where fp32's own rounding of subnormal numbers is below 2^-22 of them)."""
+    import sparseconvnet_b200 as scn
+    coords = _points(20001, 3, 80, 9)
+    coords[:, 3] = coords[:, 0] >= 40  # (samples share no rule)
+    x = scn.InputLayer(3, 80, mode=0)([torch.from_numpy(coords), torch.zeros(len(coords), 1, device=cuda)])
+    torch.manual_seed(cin)
+    layer = scn.SubmanifoldConvolution(3, cin, cout, 3, False).to(cuda).requires_grad_(False)
+    layer.weight.normal_()
+    layer.weight[..., 8:12] *= small
+    f = torch.randn(len(coords), cin, device=cuda)
+    tiny = torch.from_numpy(coords[:, 3] == 1).to(cuda)
+    f[tiny] *= small
+    y = layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features
+    assert scn.SCN.lib.scn_last_conv_six()
+    x.metadata.poll_errors()
+    want = _exact(x, layer, 0, [3, 3, 3], None, f, y.shape)
+    plane = torch.zeros(cout, dtype=torch.bool, device=cuda)
+    plane[8:12] = True
+    for rows, planes in ((~tiny, ~plane), (tiny, ~plane), (~tiny, plane)):
+        got, exact = y.double()[rows][:, planes], want[rows][:, planes]
+        assert float(exact.norm()) > 0
+        e = (got - exact).norm(dim=1) / exact.norm(dim=1).clamp(min=1e-37)
+        assert float(e.max()) <= 2.0 ** -20 and float((got - exact).norm() / exact.norm()) <= 2.0 ** -22
+
+
 @pytest.mark.parametrize("cin,cout", [(32, 48), (24, 160)])
 def test_weights_of_this_call(cin, cout, cuda):
     """A weight written through .data, which leaves its version as it is, counts from the next call on."""
