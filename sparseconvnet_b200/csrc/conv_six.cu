@@ -14,7 +14,7 @@
 // 2^24 times as large as they are and sums made 2^48 times smaller: then the last bit of the smallest fp32 value is a normal
 // bf16 number, and the terms of a product are exact for every product that is a normal number, whatever stands beside it.
 // Upwards that leaves less room, and an infinity has no low part: the pass that splits leaves the largest magnitude of rows and
-// weights, and where a sum could overflow the kernel multiplies plain fp32 values instead (slow_item).  So it does where the
+// weights, and where a sum could overflow the kernel multiplies plain fp32 values instead (slow_items).  So it does where the
 // largest products are near the lower end, where k_conv_fma's own rounding of subnormal sums is kept.
 //
 // Roles (20 or 16 warps, one CTA per SM, persistent), as in k_conv_tile but for the drain:
@@ -38,6 +38,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "conv_tile.cuh"
 
@@ -73,7 +74,7 @@ struct SixParams {
   int n_stages;
   long long n_tiles, n_items;
   int n_split;
-  // for slow_item: the operands as they are
+  // for slow_items: the operands as they are
   const float *in, *in_b, *weight, *pre_scale, *pre_shift;
   float pre_leak;
   int cin, planes_a;
@@ -140,50 +141,167 @@ __device__ __forceinline__ float finished(const SixParams &P, float v, int c) {
   return v;
 }
 
-// Operands whose parts bf16 cannot hold: infinities, NaN, the last powers of two at either end.  Plain fp32 multiply-adds in
-// the order of k_conv_fma, a warp per row, a lane per plane.
-__device__ __forceinline__ void slow_item(const SixParams &P, long long item, int warp, int warps, int lane) {
+// Operands whose parts bf16 cannot hold: infinities, NaN, products near either end of the range.  Plain fp32 multiply-adds in
+// the order of k_conv_fma: the CTA's first 512 threads are four groups of 128, each with a tile and 32 of its planes, 8 x 4 results
+// in registers per thread, and rows and weights of 32 input planes in one of two stages while the other is multiplied.  Layers on
+// 200 k rows with one infinity, us here / on k_conv_fma: 32 -> 32 planes 297/190, 64 -> 64 977/574, 96 -> 96 1 818/1 478, 160 -> 160
+// 5 720/3 990; with a warp per row and a lane per plane, which reuses no weight, 5 580 to 62 600.  What it costs the layers
+// that do not come here decided its form: inlined, with 8 x 8 results, with eight rows per warp and no shared memory, or as a
+// kernel of its own behind every k_conv_six it took 1 to 3 % of their time; as a call across which nothing lives, none.
+constexpr int kFmaGroup = 128, kFmaGroups = 4, kFmaChunk = 32;  // threads of a group; input planes of a step
+constexpr int kFmaPlanes = 32, kFmaX = kFmaPlanes / 4, kFmaY = kFmaGroup / kFmaX, kFmaRows = kRows / kFmaY;
+constexpr int kFmaRing = 4;                                       // offsets whose entries are there
+constexpr int kFmaStride = kFmaChunk + 4;                         // floats of a row of a stage: broadcast loads on different banks
+constexpr int kFmaStage = kRows * kFmaStride + kFmaChunk * kFmaPlanes;  // floats: rows, weights
+constexpr int kFmaShare = 2 * kFmaStage + kFmaRing * kRows;
+// the threads of one group
+__device__ __forceinline__ void group_sync(int group) {
+  if (group == 0) asm volatile("bar.sync 1, %0;" ::"n"(kFmaGroup) : "memory");
+  else if (group == 1) asm volatile("bar.sync 2, %0;" ::"n"(kFmaGroup) : "memory");
+  else if (group == 2) asm volatile("bar.sync 3, %0;" ::"n"(kFmaGroup) : "memory");
+  else asm volatile("bar.sync 4, %0;" ::"n"(kFmaGroup) : "memory");
+}
+
+// one group's share (n0: its first plane in the column block) of an item
+__device__ __forceinline__ void slow_item(const SixParams &P, long long item, int n0, float *stages, bool finite_weights) {
+  constexpr int BN = kFmaPlanes, TM = kFmaRows;
+  const int tid = threadIdx.x % kFmaGroup, group = threadIdx.x / kFmaGroup;
   const Item I = item_at(P, item);
+  const int last_plane = min(P.cb, P.cout - I.block * P.cb) - n0;  // planes of the share, counted from n0
+  n0 += I.block * P.cb;
   unsigned m[4];
 #pragma unroll
   for (int w = 0; w < 4; ++w) m[w] = w < P.words ? __ldg(P.tile_bits + I.tile * P.words + w) : 0u;
   const int total = __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]), first = total * I.part / P.n_split;
-  if (P.n_split > 1) keep_range(m, first, total * (I.part + 1) / P.n_split);
-  for (int p = warp; p < kRows; p += warps) {
-    const int row = __ldg(P.order + I.tile * kRows + p);
-    if (row < 0) continue;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};  // planes lane, + 32, + 64, + 96 of the block
-    const int *entry = P.packed + (I.tile * P.K + first) * kRows + p;
+  const int last = total * (I.part + 1) / P.n_split;
+  if (P.n_split > 1) keep_range(m, first, last);
+  const int nch = (P.cin + kFmaChunk - 1) / kFmaChunk;
+  const int tx = tid % kFmaX, ty = tid / kFmaX;
+  static_assert(kRows == kFmaGroup, "a thread per entry");
+  int *ring = reinterpret_cast<int *>(stages + 2 * kFmaStage);
+  const int *packed = P.packed + (I.tile * P.K + first) * kRows + tid;
+  const int offsets = last - first;
+  for (int o = 0; o < min(2, offsets); ++o) ring[o * kRows + tid] = __ldg(packed + o * kRows);
+  group_sync(group);
+
+  // copying: eight threads per row, 16 rows at a time; a thread per 16 bytes of weights
+  constexpr int CR = kFmaGroup / 8, CI = kRows / CR, WP = BN / 4, WR = kFmaGroup / WP;
+  const int cj = (tid & 7) * 4, cr = tid >> 3, wc = tid % WP * 4, wr = tid / WP;
+  int k_issue = 0, c_issue = 0, o_issue = 0;  // filter offset, chunk and offset of the item of the step to be issued next
+  auto issue = [&](int s) {                   // one cp.async group per call, empty past the end
+    if (o_issue < offsets) {
+      if (c_issue == 0) {  // the lowest offset of those that are left
 #pragma unroll
-    for (int w = 0; w < 4; ++w)
-      for (unsigned u = m[w]; u; u &= u - 1, entry += kRows) {
-        const int v = __ldg(entry);
-        if (v < 0 || v >= P.n_in) {
-          if (v >= 0 && lane == 0) atomicOr(P.flags, FLAG_BAD_ROW);
-          continue;
+        for (int w = 3; w >= 0; --w)
+          if (m[w]) k_issue = w * 32 + __ffs(m[w]) - 1;
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+          if (w == k_issue >> 5) m[w] &= m[w] - 1;
+        if (o_issue + 2 < offsets)  // the entries of the offset after the next: here when they are asked for
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(ring + ((o_issue + 2) % kFmaRing) * kRows + tid)), "l"(packed + (o_issue + 2) * kRows) : "memory");
+      }
+      float *a = stages + (s & 1) * kFmaStage, *w = a + kRows * kFmaStride;
+      const int c = c_issue * kFmaChunk + cj;
+      if (c < P.cin) {
+        const float *src = !P.in_b ? P.in + c : c < P.planes_a ? P.in + c : P.in_b + (c - P.planes_a);
+        const int ld = !P.in_b ? P.cin : c < P.planes_a ? P.planes_a : P.cin - P.planes_a;
+        const int *entry = ring + o_issue % kFmaRing * kRows + cr;
+#pragma unroll
+        for (int i = 0; i < CI; ++i) {
+          const int v = entry[i * CR];
+          const bool hit = (unsigned)v < (unsigned)P.n_in;
+          if (v >= 0 && !hit) atomicOr(P.flags, FLAG_BAD_ROW);
+          cp_async16(smem_u32(a + (cr + i * CR) * kFmaStride + cj), hit ? src + (long long)v * ld : P.in, hit ? 16u : 0u);
         }
-        const float *wk = P.weight + (long long)(w * 32 + __ffs(u) - 1) * P.cin * P.cout;
-        for (int c = 0; c < P.cin; ++c) {
-          float x = !P.in_b || c < P.planes_a ? __ldg(P.in + (long long)v * (P.in_b ? P.planes_a : P.cin) + c)
-                                              : __ldg(P.in_b + (long long)v * (P.cin - P.planes_a) + (c - P.planes_a));
-          if (P.pre_scale) {
-            x = __fadd_rn(__fmul_rn(x, __ldg(P.pre_scale + c)), __ldg(P.pre_shift + c));
-            x *= x > 0.f ? 1.f : P.pre_leak;
-          }
+      }
+      const float *wk = P.weight + ((long long)k_issue * P.cin + c_issue * kFmaChunk) * P.cout + n0 + wc;
+      const int rows = min(kFmaChunk, P.cin - c_issue * kFmaChunk);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int n = I.block * P.cb + i * 32 + lane;
-            if (i * 32 + lane < P.cb && n < P.cout) acc[i] = fmaf(x, __ldg(wk + (long long)c * P.cout + n), acc[i]);
+      for (int i = 0; i < kFmaChunk / WR; ++i) {
+        const int r = wr + i * WR;
+        const bool ok = r < rows && wc < last_plane;
+        cp_async16(smem_u32(w + r * BN + wc), ok ? wk + (long long)r * P.cout : P.weight, ok ? 16u : 0u);
+      }
+      if (++c_issue == nch) c_issue = 0, ++o_issue;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  float acc[TM][4];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
+  issue(0);
+  issue(1);
+  int chunk = 0, o = 0;
+  const int steps = offsets * nch;
+  for (int s = 0; s < steps; ++s) {
+    float *a = stages + (s & 1) * kFmaStage;
+    const float *w = a + kRows * kFmaStride + tx * 4;
+    const int *entry = ring + o % kFmaRing * kRows;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    if (P.pre_scale && chunk * kFmaChunk + cj < P.cin) {  // the pieces that this thread has copied, rounded as in k_six_prepare
+      const int c = chunk * kFmaChunk + cj;
+#pragma unroll 1
+      for (int i = 0; i < CI; ++i)
+        if ((unsigned)entry[cr + i * CR] < (unsigned)P.n_in) {
+          float *x = a + (cr + i * CR) * kFmaStride + cj;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float y = __fadd_rn(__fmul_rn(x[e], __ldg(P.pre_scale + c + e)), __ldg(P.pre_shift + c + e));
+            x[e] = y * (y > 0.f ? 1.f : P.pre_leak);
+          }
+        }
+    }
+    group_sync(group);
+    const int kmax = min(kFmaChunk, P.cin - chunk * kFmaChunk);
+    a += ty * kFmaStride;
+    // A row without a rule counts as zeros, but is no business of an infinite weight.
+    auto multiply = [&](auto all) {
+#pragma unroll 1
+      for (int kk = 0; kk < kmax; kk += 4) {
+        float4 wv[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) wv[q] = *reinterpret_cast<const float4 *>(w + (kk + q) * BN);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+          if (!decltype(all)::value && (unsigned)entry[ty + i * kFmaY] >= (unsigned)P.n_in) continue;
+          const float4 av = *reinterpret_cast<const float4 *>(a + i * kFmaY * kFmaStride + kk);
+          const float x[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            acc[i][0] = fmaf(x[q], wv[q].x, acc[i][0]);
+            acc[i][1] = fmaf(x[q], wv[q].y, acc[i][1]);
+            acc[i][2] = fmaf(x[q], wv[q].z, acc[i][2]);
+            acc[i][3] = fmaf(x[q], wv[q].w, acc[i][3]);
           }
         }
       }
-    float *to = result_row(P, I, p, row);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int n = I.block * P.cb + i * 32 + lane;
-      if (i * 32 + lane < P.cb && n < P.cout) to[n] = finished(P, acc[i], n);
-    }
+    };
+    if (finite_weights) multiply(std::true_type());
+    else multiply(std::false_type());
+    if (++chunk == nch) chunk = 0, ++o;
+    group_sync(group);
+    issue(s + 2);
   }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int p = ty + i * kFmaY, row = __ldg(P.order + I.tile * kRows + p);
+    if (row < 0) continue;
+    float *to = result_row(P, I, p, row) + n0 + tx * 4;
+    if (tx * 4 < last_plane)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) to[e] = finished(P, acc[i][e], n0 + tx * 4 + e);
+  }
+}
+
+// all items of a CTA, by its first 512 threads
+__device__ __noinline__ void slow_items(const SixParams &P, float *smem, bool finite_weights) {
+  const int group = threadIdx.x / kFmaGroup, cols = (P.cb + kFmaPlanes - 1) / kFmaPlanes;
+  const long long n = items_here(P.n_items) * cols;
+  for (long long u = group; u < n; u += kFmaGroups)
+    slow_item(P, item_of(u / cols), (int)(u % cols) * kFmaPlanes, smem + group * kFmaShare, finite_weights);
 }
 
 // Can sums of 2^log2_terms products of values up to x and w in magnitude (float bits) be made of bf16 parts?  Nothing may
@@ -209,7 +327,7 @@ __device__ __forceinline__ void split3_pair(float a, float b, unsigned &h, unsig
 
 // SP: input planes of a step; NA: planes of a drain warp, a multiple of 16
 template <int SP, int NA>
-__global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams P) {
+__global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __grid_constant__ SixParams P) {
   SCN_GRID_WAIT();
   using Shape = SixShape<SP>;
   using Warps = SixWarps<NA>;
@@ -260,8 +378,12 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(SixParams
   volatile int *abort = &C.abort;
 
   if (!parts_reach(C.range[0], C.range[1], P.log2_terms)) {
-    for (long long it = 0; it < my_items; ++it) slow_item(P, item_of(it), warp, Warps::THREADS / 32, lane);
-  } else if (warp < kProdWarps) {
+    if (tid < kFmaGroups * kFmaGroup) slow_items(P, reinterpret_cast<float *>(smem), C.range[1] < 0x7F800000u);
+    __syncthreads();
+    if (threadIdx.x >> 5 == kMma) tmem_dealloc(C.tmem, 512);
+    return;
+  }
+  if (warp < kProdWarps) {
     // ==================================== producers =============================================
     // this lane's 16-byte piece of the rows q NI .. q NI + NI - 1, for [h | m] and again for [l]
     const int j = lane % Shape::PIECES, q = lane / Shape::PIECES, lj = lane % Shape::L_PIECES, lq = lane / Shape::L_PIECES;
@@ -696,6 +818,9 @@ int launch_six(SixParams &P, int n_sm, int dev, cudaStream_t stream) {
   const size_t stage = SixShape<SP>::A_BYTES + ((size_t)P.cb * SP * 6 + 1023) / 1024 * 1024;
   const size_t fixed = sizeof(int) * kSlots * kRows + kDrainWarps * kEpiBytes + sizeof(Ctl);
   P.n_stages = (int)std::min<size_t>(kMaxStages, (kSmemBudget - fixed) / stage);
+  static_assert(SixWarps<NA>::THREADS >= kFmaGroups * kFmaGroup, "slow_items");
+  SCN_REQUIRE((size_t)P.n_stages * stage + fixed - sizeof(Ctl) >= sizeof(float) * kFmaGroups * kFmaShare, SCN_ERR_UNSUPPORTED,
+              "k_conv_six: %d stages of %zu bytes", P.n_stages, stage);
   P.n_items = P.n_tiles * P.n_split * P.n_cb;
   SCN_LAUNCH(kernel, (unsigned)std::min<long long>(P.n_items, (long long)n_sm), SixWarps<NA>::THREADS, kSmemBudget, stream, P);
   SCN_CUDA_CHECK(cudaGetLastError());

@@ -95,6 +95,34 @@ def test_values_the_parts_cannot_hold(case, cin, cout, n, cuda, monkeypatch):
         assert torch.equal(torch.nan_to_num(got, nan=7.0), torch.nan_to_num(want, nan=7.0))
 
 
+@pytest.mark.parametrize("cin,cout,n,split", [(32, 32, 9000, "1"), (40, 48, 3000, "3"), (100, 136, 700, None), (64, 128, 9000, None)])
+def test_an_infinity_spoils_its_own_rows_only(cin, cout, n, split, cuda, monkeypatch):
+    """One infinite weight of an offset that some rows have: the others, and the planes beside it, as float64 gives them, with
+    the offsets whole and divided (sums of 27 x 100 fp32 products: 1e-5 as in the multiply-adds' own test)."""
+    import sparseconvnet_b200 as scn
+    if split:
+        monkeypatch.setenv("SCN_SIX_SPLIT", split)
+    coords = _points(n, 3, 160, n)
+    x = scn.InputLayer(3, 160, mode=0)([torch.from_numpy(coords), torch.zeros(len(coords), 1, device=cuda)])
+    torch.manual_seed(n)
+    layer = scn.SubmanifoldConvolution(3, cin, cout, 3, True).to(cuda).requires_grad_(False)
+    layer.bias.normal_()
+    f = torch.randn(len(coords), cin, device=cuda)
+    monkeypatch.setenv("SCN_CONV_SIX", "1")
+    layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size))
+    want = _exact(x, layer, 0, [3, 3, 3], None, f, (len(coords), cout))
+    book = x.metadata.rulebook(0, x.spatial_size, [3, 3, 3], None)
+    k = max((k for k in range(27) if k != 13), key=lambda k: len(book[k]))
+    layer.weight[k, 0, 2, 1] = float("inf")
+    y = layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features
+    assert scn.SCN.lib.scn_last_conv_six()
+    x.metadata.poll_errors()
+    hit = torch.zeros(len(coords), cout, dtype=torch.bool, device=cuda)
+    hit[book[k].long()[:, 1], 1] = True
+    assert 0 < int(hit.sum()) < len(coords) and torch.equal(hit, ~torch.isfinite(y))
+    assert float((y.double() - want)[~hit].abs().max() / want.abs().max()) <= 1e-5
+
+
 @pytest.mark.parametrize("small", [1e-30, 1e-35, 1e-37])
 @pytest.mark.parametrize("cin,cout", [(24, 32), (32, 32), (40, 136)])
 def test_small_values_beside_ordinary_ones(small, cin, cout, cuda):
@@ -138,9 +166,9 @@ def test_weights_of_this_call(cin, cout, cuda):
         assert torch.equal(layer(x).features, 2 * one)
 
 
-@pytest.mark.parametrize("n", [700, 20000])
-def test_batchnorm_and_join_in_front(n, cuda):
-    """In the pass that splits the rows: the same bits as the layers one by one."""
+@pytest.mark.parametrize("n,inf", [(700, False), (20000, False), (20000, True)])
+def test_batchnorm_and_join_in_front(n, inf, cuda):
+    """In the pass that splits the rows, and where they are multiplied unsplit: the same bits as the layers one by one."""
     import sparseconvnet_b200 as scn
     torch.manual_seed(n)
 
@@ -153,6 +181,8 @@ def test_batchnorm_and_join_in_front(n, cuda):
                 torch.nn.init.uniform_(t, 0.3, 1.0)
     coords = _points(n, 3, 120, n)
     feats = torch.randn(len(coords), 32, device=cuda)
+    if inf:
+        feats[7, 3] = float("inf")
     outs = []
     try:
         for fuse in (False, True):
@@ -161,7 +191,8 @@ def test_batchnorm_and_join_in_front(n, cuda):
                 outs.append(net(scn.InputLayer(3, 120, mode=0)([torch.from_numpy(coords), feats])).features)
     finally:
         scn.Sequential.fuse = True
-    assert torch.equal(*outs)
+    assert not inf or 0 < int((~torch.isfinite(outs[0])).sum()) < outs[0].numel() // 2
+    assert torch.equal(*(torch.nan_to_num(y, nan=7.0) for y in outs))
 
 
 def test_bounded_wait_runs_out(cuda):
