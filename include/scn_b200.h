@@ -337,7 +337,8 @@ SCN_API int scn_submanifold_convolution_forward(scn_metadata *md, const int64_t 
  * bound.  No counterpart in the reference. */
 SCN_API int scn_test_drop_barrier_arrival(void);
 /* Test hook: the `which`-th allocation (device memory or pinned staging) of the calling thread from now on fails with
- * SCN_ERR_CUDA as if memory had run out; 0: none does. */
+ * SCN_ERR_CUDA as if memory had run out; 0: none does.  Returns how many allocations an earlier request had still to go,
+ * 0 once it has come up. */
 SCN_API int scn_test_fail_allocation(int which);
 
 /* Allocation-free SubmanifoldConvolution.  No counterpart in the reference.

@@ -69,7 +69,7 @@ bool conv_six_takes(const float *in, const float *in_b, int planes_a, const floa
 int conv_forward_six(const float *in, long long n_in, float *out, long long n_out, const float *weight, const float *bias,
                      const float *bn_scale, const float *bn_shift, float leak, const RowOrder &ord, int K, int cin, int cout,
                      int *flags, cudaStream_t stream, const float *pre_scale, const float *pre_shift, float pre_leak,
-                     const float *in_b, int planes_a);
+                     const float *in_b, int planes_a, bool *no_memory);
 int conv_forward_fma(const float *in, long long n_in, float *out, long long n_out, const float *weight, const float *bias,
                      const float *bn_scale, const float *bn_shift, float leak, const int *table, const RowOrder *ord, int K,
                      int cin, int cout, int *flags, cudaStream_t stream);
@@ -398,23 +398,30 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
                    conv_fma_supported(in, out, weight, bias, rb.n_offsets, cin, cout, groups) &&
                    !(any_knob() && getenv("SCN_SIMT_BLOCK") && atoi(getenv("SCN_SIMT_BLOCK")) != 0);
   const bool packed = fma && conv_fma_wants_order(rows_out);
-  if (transposed_table && !packed && !(fma && six_enabled() && conv_six_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, rows_in, rows_out)))
-    SCN_TRY(rulebook_transposed(rb, stream));
+  if (fma && six_enabled() && conv_six_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, rows_in, rows_out)) {
+    RowOrder &ord = transposed_table ? rb.torder : rb.order;
+    const bool there = ord.order != nullptr;
+    bool no_memory = false;
+    const int rc = row_order(ord);
+    if (rc == SCN_OK) {
+      if (!there) ord.fp32_only = true;
+      SCN_TRY(conv_forward_six(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, ord, rb.n_offsets, cin, cout,
+                               flags, stream, pre_scale, pre_shift, pre_leak, in_b, planes_a, &no_memory));
+    } else if (packed) {
+      return rc;
+    }
+    if (rc == SCN_OK && !no_memory) {
+      g_last_kernel = SCN_KERNEL_CONV_FMA;
+      g_last_six = true;
+      return SCN_OK;
+    }
+    cudaGetLastError();  // (of the allocation) k_conv_fma does with less
+  }
+  if (transposed_table && !packed) SCN_TRY(rulebook_transposed(rb, stream));
   const int *table = transposed_table ? rb.tnbr : rb.nbr;
   if (!fma)
     return conv_forward_dispatch(in, rows_in, out, rows_out, weight, bias, table, rb.n_offsets, cin, cout, groups, precision,
                                  flags, stream, bn_scale, bn_shift, leak, pre_scale, pre_shift, pre_leak, in_b, planes_a);
-  if (six_enabled() && conv_six_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, rows_in, rows_out)) {
-    RowOrder &ord = transposed_table ? rb.torder : rb.order;
-    const bool there = ord.order != nullptr;
-    SCN_TRY(row_order(ord));
-    if (!there) ord.fp32_only = true;
-    SCN_TRY(conv_forward_six(in, rows_in, out, rows_out, weight, bias, bn_scale, bn_shift, leak, ord, rb.n_offsets, cin, cout,
-                             flags, stream, pre_scale, pre_shift, pre_leak, in_b, planes_a));
-    g_last_kernel = SCN_KERNEL_CONV_FMA;
-    g_last_six = true;
-    return SCN_OK;
-  }
   float *pre_copy = nullptr;
   SCN_TRY(prepared_input(&in, rows_in, cin, groups, pre_scale, pre_shift, pre_leak, in_b, planes_a, &pre_copy, stream));
   RowOrder *ord = nullptr;

@@ -871,11 +871,13 @@ bool conv_six_takes(const float *in, const float *in_b, int planes_a, const floa
 }
 
 // out [n_out, cout] = act((bias + sum_k in[table[k][.]] @ W[k]) * bn_scale + bn_shift) for the table that `ord` packs, the
-// input optionally a join and behind a BatchNorm of its own
+// input optionally a join and behind a BatchNorm of its own.  The operands in parts take 6 bytes per value of rows and
+// weights (0.6 GB for 64 planes on 1.6 M rows) that k_conv_fma does without: where they are not to be had, nothing has been
+// launched and *no_memory is set.
 int conv_forward_six(const float *in, long long n_in, float *out, long long n_out, const float *weight, const float *bias,
                      const float *bn_scale, const float *bn_shift, float leak, const RowOrder &ord, int K, int cin, int cout,
                      int *flags, cudaStream_t stream, const float *pre_scale, const float *pre_shift, float pre_leak,
-                     const float *in_b, int planes_a) {
+                     const float *in_b, int planes_a, bool *no_memory) {
   if (n_out == 0) return SCN_OK;
   const int SP = (cin + 15) / 16 * 16 % 32 == 0 ? 32 : 16, n_slices = (cin + SP - 1) / SP, cinp = n_slices * SP;
   const int coutp = (cout + 15) / 16 * 16, n_cb = coutp > 128 ? 2 : 1, cb = n_cb == 1 ? coutp : (coutp / 2 + 15) / 16 * 16;
@@ -892,8 +894,17 @@ int conv_forward_six(const float *in, long long n_in, float *out, long long n_ou
   Scratch tmp(stream);
   unsigned char *image = nullptr, *rows = nullptr;
   const size_t image_bytes = (size_t)K * cinp * cb * n_cb * 6, rows_bytes = (size_t)std::max<long long>(n_in, 1) * cinp * 6;
-  SCN_TRY(tmp.get(&image, image_bytes + sizeof(unsigned) * kRangeWords));  // (multiples of 16)
-  SCN_TRY(tmp.get(&rows, rows_bytes + sizeof(unsigned) * kRangeWords));
+  float *partial = nullptr;
+  const double chunk = cb <= 64 ? std::max(56.0, 1.5 * cb) + std::max(56.0, 1.0 * cb) + 56 : 6 * std::max(56.0, 0.5 * cb);
+  const double step = std::max((kRows * SP * 6.0 + cb * SP * 6.0) / 32.0, chunk * SP / 16);
+  const char *e = getenv("SCN_SIX_SPLIT");
+  const int n_split = e ? std::max(1, std::min(atoi(e), 64)) : split_parts(ord.n_tiles, n_cb, ord.one_offset ? 1 : K, n_slices, step, cout, n_sm);
+  if (tmp.get(&image, image_bytes + sizeof(unsigned) * kRangeWords) != SCN_OK ||  // (multiples of 16)
+      tmp.get(&rows, rows_bytes + sizeof(unsigned) * kRangeWords) != SCN_OK ||
+      (n_split > 1 && tmp.get(&partial, (size_t)n_split * ord.n_tiles * kRows * cout * sizeof(float)) != SCN_OK)) {
+    *no_memory = true;
+    return SCN_OK;
+  }
   PrepareParams Q{};
   Q.in = in;
   Q.in_b = in_b;
@@ -954,16 +965,13 @@ int conv_forward_six(const float *in, long long n_in, float *out, long long n_ou
   P.flags = flags;
   P.drop = g_drop_arrival;
   g_drop_arrival = 0;
-  const double chunk = cb <= 64 ? std::max(56.0, 1.5 * cb) + std::max(56.0, 1.0 * cb) + 56 : 6 * std::max(56.0, 0.5 * cb);
-  const double step = std::max((kRows * SP * 6.0 + cb * SP * 6.0) / 32.0, chunk * SP / 16);
-  const char *e = getenv("SCN_SIX_SPLIT");
-  P.n_split = e ? std::max(1, std::min(atoi(e), 64)) : split_parts(P.n_tiles, n_cb, ord.one_offset ? 1 : K, n_slices, step, cout, n_sm);
-  if (P.n_split > 1) SCN_TRY(tmp.get(&P.out, (size_t)P.n_split * P.n_tiles * kRows * cout * sizeof(float)));
+  P.n_split = n_split;
+  if (n_split > 1) P.out = partial;
   const auto launch = SP == 32 ? (cb <= 32 ? launch_six<32, 16> : cb <= 64 ? launch_six<32, 32> : launch_six<32, 64>)
                                : (cb <= 32 ? launch_six<16, 16> : cb <= 64 ? launch_six<16, 32> : launch_six<16, 64>);
   SCN_TRY(launch(P, n_sm, dev, stream));
-  if (P.n_split > 1)
-    SCN_TRY(sum_partial_tiles(P.out, P.n_split, P.n_tiles * kRows, cout, ord.order, n_out, bias, bn_scale, bn_shift, leak, out, stream));
+  if (n_split > 1)
+    SCN_TRY(sum_partial_tiles(partial, n_split, P.n_tiles * kRows, cout, ord.order, n_out, bias, bn_scale, bn_shift, leak, out, stream));
   return SCN_OK;
 }
 

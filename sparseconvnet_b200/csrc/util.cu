@@ -323,8 +323,9 @@ int scn_memory_usage(uint64_t *reserved_bytes, uint64_t *used_bytes) {
 }
 
 int scn_test_fail_allocation(int which) {
+  const int left = scn::g_fail_in;
   scn::g_fail_in = which > 0 ? which : 0;
-  return SCN_OK;
+  return left;
 }
 
 int scn_trim_memory(uint64_t keep_bytes) {

@@ -67,7 +67,8 @@ def _used():
 @pytest.mark.parametrize("n,coords", [(3000, "cpu"), (3000, "cuda"), (300, "cpu")])
 def test_nothing_is_lost_when_memory_runs_out(n, coords, precision, cuda):
     """Input layer, rulebooks, row order, forward and backward pass with the first, second, ... allocation failing: an error
-    each time, every block given back with the object, and the next pass gives what an undisturbed one does."""
+    each time -- or, where a layer does with less, the same results to rounding --, every block given back with the object, and the
+    next pass gives what an undisturbed one does."""
     import sparseconvnet_b200 as scn
     from sparseconvnet_b200 import SCN
     from sparseconvnet_b200._lib import ScnError, lib
@@ -77,6 +78,7 @@ def test_nothing_is_lost_when_memory_runs_out(n, coords, precision, cuda):
     size, half, three, two = torch.LongTensor([48] * 3), torch.LongTensor([24] * 3), torch.LongTensor([3] * 3), torch.LongTensor([2] * 3)
     w = [torch.randn(27, 1, 32, 64, device=cuda), torch.randn(8, 1, 64, 40, device=cuda)]
     none = torch.empty(0)
+    pending = [0]
 
     def run():
         m = SCN.Metadata_3()
@@ -95,7 +97,7 @@ def test_nothing_is_lost_when_memory_runs_out(n, coords, precision, cuda):
             SCN.BatchNormalization_backward(y, d_in, out, g[3], mean, var, None, None, none, none, None, d_b, 0.0)
             return [x, y, z] + g
         finally:
-            lib.scn_test_fail_allocation(0)
+            pending[0] = lib.scn_test_fail_allocation(0)
             del m
 
     try:
@@ -108,8 +110,11 @@ def test_nothing_is_lost_when_memory_runs_out(n, coords, precision, cuda):
         for which in range(1, 200):
             lib.scn_test_fail_allocation(which)
             try:
-                run()
-                break
+                got = run()
+                if pending[0]:  # there was no such allocation any more
+                    break
+                # (sums of at most 27 x 64 fp32 products, and of 3000 of them in the weights' gradients)
+                assert precision == "fp32" and all(float((a - b).norm()) <= 1e-5 * float(b.norm()) for a, b in zip(got, want)), which
             except ScnError as e:
                 assert "out of memory" in str(e), e
                 failed += 1

@@ -213,3 +213,50 @@ def test_bounded_wait_runs_out(cuda):
             x.metadata.poll_errors()
         assert torch.equal(layer(x).features, good)
         x.metadata.poll_errors()
+
+
+@pytest.mark.parametrize("kind,cin,cout,n", [("submanifold", 64, 96, 9000), ("submanifold", 64, 96, 1600), ("submanifold", 64, 64, 3000),
+                                             ("down", 96, 160, 9000), ("up", 160, 160, 30000)])
+def test_without_memory_for_the_parts(kind, cin, cout, n, cuda, monkeypatch):
+    """Every allocation of a layer whose rulebook is there fails in turn: where the operands' parts do not fit, or the row order of
+    a level that k_conv_fma takes as it is, that kernel's result; an error only for what it needs as well."""
+    import sparseconvnet_b200 as scn
+    from sparseconvnet_b200._lib import ScnError, lib
+    torch.manual_seed(n)
+    coords = torch.from_numpy(_points(n, 3, 160, n)).to(cuda)
+    make, small = ((lambda a, b: scn.SubmanifoldConvolution(3, a, b, 3, True),) * 2 if kind == "submanifold" else
+                   (lambda a, b: scn.Convolution(3, a, b, 2, 2, True),) * 2 if kind == "down" else
+                   (lambda a, b: scn.Deconvolution(3, a, b, 2, 2, True), lambda a, b: scn.Convolution(3, a, b, 2, 2, True)))
+    layer, first = make(cin, cout).to(cuda).requires_grad_(False), small(4, 4).to(cuda).requires_grad_(False)
+    feats = torch.randn(len(coords), cin, device=cuda)
+
+    def run(which, six):
+        monkeypatch.setenv("SCN_CONV_SIX", six)
+        x = scn.InputLayer(3, 160, mode=1)([coords, feats[:, :4].contiguous()])
+        y = first(x)  # the rulebook, on a kernel without tiles
+        rows = y.features.size(0) if kind == "up" else x.features.size(0)
+        z = scn.SparseConvNetTensor(feats[:rows], x.metadata, y.spatial_size if kind == "up" else x.spatial_size)
+        lib.scn_test_fail_allocation(which)
+        try:
+            out = layer(z).features
+        finally:
+            left = lib.scn_test_fail_allocation(0)
+        x.metadata.poll_errors()
+        return out, lib.scn_last_conv_six(), left
+    want, on_six, _ = run(0, "1")
+    plain, on_fma, _ = run(0, "0")
+    assert on_six and not on_fma
+    recovered, failed = 0, 0
+    for which in range(1, 40):
+        try:
+            out, six, left = run(which, "1")
+        except ScnError as e:
+            assert "out of memory" in str(e)
+            failed += 1
+            continue
+        assert torch.equal(out, want if six else plain), which
+        if left:
+            break
+        assert not six
+        recovered += 1
+    assert left and recovered >= 2 and (failed == 0) == (len(want) < 2048)
