@@ -65,7 +65,7 @@ bool conv_fma_supported(const float *in, const float *out, const float *weight, 
                         int groups);
 bool conv_fma_wants_order(long long n_out);
 bool conv_six_takes(const float *in, const float *in_b, int planes_a, const float *out, const float *bias, int K, int cin,
-                    int cout, int groups, long long rows_in, long long rows_out);
+                    int cout, int groups, long long rows_in, long long rows_out, bool disjoint, bool transposed);
 int conv_forward_six(const float *in, long long n_in, float *out, long long n_out, const float *weight, const float *bias,
                      const float *bn_scale, const float *bn_shift, float leak, const RowOrder &ord, int K, int cin, int cout,
                      int *flags, cudaStream_t stream, const float *pre_scale, const float *pre_shift, float pre_leak,
@@ -398,7 +398,7 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
                    conv_fma_supported(in, out, weight, bias, rb.n_offsets, cin, cout, groups) &&
                    !(any_knob() && getenv("SCN_SIMT_BLOCK") && atoi(getenv("SCN_SIMT_BLOCK")) != 0);
   const bool packed = fma && conv_fma_wants_order(rows_out);
-  if (fma && six_enabled() && conv_six_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, rows_in, rows_out)) {
+  if (fma && six_enabled() && conv_six_takes(in, in_b, planes_a, out, bias, rb.n_offsets, cin, cout, groups, rows_in, rows_out, rb.disjoint, transposed_table)) {
     RowOrder &ord = transposed_table ? rb.torder : rb.order;
     const bool there = ord.order != nullptr;
     bool no_memory = false;

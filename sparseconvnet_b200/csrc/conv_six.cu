@@ -848,8 +848,8 @@ extern thread_local int g_drop_arrival;  // test hook (conv_tc.cu)
 
 // Which fp32 convolutions run here instead of on k_conv_fma (which is left for few output planes on many rows, whose
 // multiply-adds cost less than six bytes per input value and rule, and for little work, where its one launch is the shorter
-// chain).  One layer,
-// 27 offsets, us on this kernel / on k_conv_fma, and the error of each against float64 (2-norm, products of mixed sign):
+// chain).  One layer, us on this kernel / on k_conv_fma.  27 offsets, submanifold, rows scattered over a surface; the error of
+// each against float64 (2-norm, products of mixed sign):
 //                 16->16    16->32    24->32    32->32     64->64      96->96      160->160      error (96->96)
 //   600 rows      -         -         14.3/11.9 13.7/12.3  16.0/12.5   19.2/15.4   22.1/25.9     0.8e-7 / 2.0e-7
 //   1 000         14.6/11.2 14.1/11.6 14.1/12.1 14.3/13.1  16.6/14.3   20.0/24.3   24.1/47.2     0.9e-7 / 2.6e-7
@@ -858,16 +858,38 @@ extern thread_local int g_drop_arrival;  // test hook (conv_tc.cu)
 //   30 000        21/29     22/38     25/45     25/52      46/122      66/250      164/719       1.1e-7 / 5.3e-7
 //   200 000       63/57     66/80     83/100    85/118     180/370     281/932     709/2 622     1.2e-7 / 5.4e-7
 //   1 600 000     446/403   434/591   584/727   589/856
-//   99 000, 3-D shapes, 27 offsets: 8->16 45/42, 16->16 45/51, 32->16 57/67, 16->32 45/63
-//   91 000, 2-D strokes, 9 offsets: 16->16 28/21, 32->16 33/27, 16->32 28/26, 24->32 34/31, 32->32 34/37
-// Its error is the smaller one for every shape that comes here, 8 to 224 planes, 600 to 200 000 rows, products of mixed and
-// of one sign (16->32 on 9 000 rows of one sign, where k_conv_fma's sums are in parts: 6.5e-8 and 6.1e-8, so not here).
+// The same on sphere shells, whose rows are closer together (k_conv_fma packs rows from 2 048 on):
+//                 32->32     64->64     64->96     96->96     128->128
+//   500 rows      13.5/11.0  16.2/13.3  17.8/15.6  18.8/19.2  21.0/22.5
+//   1 000         13.6/12.1  16.8/17.4  18.4/23.6  19.9/31.2  21.4/38.2
+//   2 000         13.7/9.3   16.2/14.6  18.5/17.3  19.0/22.1  22.5/31.9
+//   3 000         14.7/18.0  19.2/34.4  21.6/40.6  24.7/55.7  30.8/82.0
+// Other filters:
+//   3-D shapes, 99 000 rows, 27 offsets: 8->16 45/42, 16->16 45/51, 32->16 57/67, 16->32 45/63
+//   2-D strokes, 91 000 rows, 9 offsets: 16->16 28/21, 32->16 33/27, 16->32 28/26, 24->32 34/31, 32->32 34/37
+//   2-D, 25 offsets, 31 500 rows: 16->32 26/37, 32->32 29/51, 64->64 56/129; 4-D, 81 offsets, 60 000 rows: 32->32 76/221
+//   3 / 2, 27 offsets, 26 700 rows: 16->32 22/30, 32->32 27/40, 64->64 52/99, 128->128 115/361
+// Windows side by side (filter = stride), where a fine row has one rule and K * rows * planes says less about the work (2 / 2; 2^4 offsets alike):
+//   Convolution   32->48   64->64    96->64    64->96    96->96    128->128     Deconvolution  64->64    64->128  96->96   128->96  128->128  160->128
+//   1 800 rows    14/10    15/11     17/15     17/15     18/20     22/24        6 000 rows     12/11     15/11    14/12    15/15    17/16     17/18
+//   5 800         15/18    19/24     23/31     21/25     24/33     28/52        20 000         18/13     24/17    22/18    24/22    27/27     28/33
+//   60 000        35/38    57/67     76/97     65/97     83/138    112/182      60 000         29/29     41/40    39/42    41/51    48/67     50/79
+//   150 000       79/70    124/118   168/165   137/197   182/278   246/399      200 000        70/58     107/108  96/121   103/152  124/178   133/213
+// Its error is the smaller one, or the same, for every shape and table that comes here, 8 to 256 planes, products of mixed
+// and of one sign, rows behind a ReLU (16->32 on 9 000 rows of one sign, where k_conv_fma's sums are in parts: 6.5e-8 and
+// 6.1e-8, so not here).
 bool conv_six_takes(const float *in, const float *in_b, int planes_a, const float *out, const float *bias, int K, int cin,
-                    int cout, int groups, long long rows_in, long long rows_out) {
-  return groups == 1 && K <= kOrderMaxOffsets && cin % 4 == 0 && cout % 4 == 0 && cout <= 256 && (cout > 16 || rows_out <= 131072) &&
-         (!in_b || planes_a % 4 == 0) && ((uintptr_t)in | (uintptr_t)in_b | (uintptr_t)out | (uintptr_t)bias) % 16 == 0 &&
-         rows_in < (1ll << 31) && rows_out < (1ll << 31) && rows_out >= 512 && (cin > 16 || rows_out >= 16384) &&
-         (double)K * cin * cout >= (K < 27 ? 9000 : 6900) && (double)K * rows_out * cin * cout >= (rows_out < 1500 ? 250e6 : 80e6);
+                    int cout, int groups, long long rows_in, long long rows_out, bool disjoint, bool transposed) {
+  if (groups != 1 || K > kOrderMaxOffsets || cin % 4 != 0 || cout % 4 != 0 || cout > 256 || (in_b && planes_a % 4 != 0) ||
+      ((uintptr_t)in | (uintptr_t)in_b | (uintptr_t)out | (uintptr_t)bias) % 16 != 0 || rows_in >= (1ll << 31) || rows_out >= (1ll << 31))
+    return false;
+  const double weights = (double)K * cin * cout;
+  if (rows_out < 512 || (cin <= 16 && rows_out < 16384) || (cout <= 16 && rows_out > 131072) || weights < (K < 27 ? 9000 : 6900) ||
+      weights * rows_out < (rows_out >= 2048 ? 80e6 : disjoint ? 220e6 : 160e6))
+    return false;
+  if (!disjoint) return true;
+  if (!transposed) return cout > 64 || rows_out <= 90000;
+  return cin * cout >= 20000 || (cin >= 96 && cin * cout >= 8000 && rows_out >= 40000);
 }
 
 // out [n_out, cout] = act((bias + sum_k in[table[k][.]] @ W[k]) * bn_scale + bn_shift) for the table that `ord` packs, the

@@ -1294,6 +1294,7 @@ static int build_strided(scn_metadata *md, Grid *gin, const int64_t *output_size
   for (int d = 0; d < md->dim; ++d) rb.filter[d] = filter_size[d];
   rb.n_in = n_in;
   rb.n_out = n_out;
+  rb.disjoint = F.tmax == 1;
   rb.one_parent = one_rule_per_row(gin->layout, gin->may_have_blank_rows, F);
   size_t nbr_bytes = sizeof(int) * (size_t)(K * std::max<long long>(n_out, 1));
   SCN_TRY(device_alloc((void **)&rb.nbr, nbr_bytes, stream));
@@ -1490,6 +1491,7 @@ static void chain_plan(scn_metadata *md, const Grid *gin, const std::vector<int6
     if (make_layout(dim, lv.out_size.data(), lv.gout.layout) != SCN_OK) break;
     if (!(lv.gout.layout.batch_bits >= gin->layout.batch_bits || gin->batch_size <= (1ll << lv.gout.layout.batch_bits)))
       break;
+    lv.rb.disjoint = lv.F.tmax == 1;
     lv.rb.one_parent = plan.empty() ? one_rule_per_row(gin->layout, gin->may_have_blank_rows, lv.F)
                                     : one_rule_per_row(plan.back().gout.layout, false, lv.F);
     lv.bound_in = bound;

@@ -80,6 +80,7 @@ struct Rulebook {
   long long total_rules = -1;
   CountTicket *ticket = nullptr;             // counts in flight (null above kTicketValues offsets)
   bool built = false;
+  bool disjoint = false;   // strided: an input row has at most one rule (windows side by side)
   bool one_parent = false; // strided: every input row has exactly one rule (of the sizes it was built with)
   bool symmetric = false;  // submanifold with odd filter sizes: tnbr[k] is nbr[K - 1 - k]
 };

@@ -15,18 +15,33 @@ def _exact(x, layer, kind, filt, stride, f, shape):
     want = torch.zeros(shape, dtype=torch.float64, device=f.device)
     if hasattr(layer, "bias"):
         want += layer.bias.double()
+    up = type(layer).__name__ == "Deconvolution"
     for r, w in zip(x.metadata.rulebook(kind, x.spatial_size, filt, stride), layer.weight.double()[:, 0]):
-        r = r.long()
+        r = r.long().flip(1) if up else r.long()
         want.index_add_(0, r[:, 1], f.double()[r[:, 0]] @ w)
     return want
 
 
-@pytest.mark.parametrize("cin,cout", [(8, 24), (12, 20), (16, 32), (32, 32), (36, 64), (64, 80), (64, 84), (96, 96), (32, 128),
-                                      (100, 132), (64, 256)])
-@pytest.mark.parametrize("n,split", [(700, None), (8191, None), (20001, None), (8200, "3"), (150000, None)])
-def test_as_accurate_as_multiply_adds(n, split, cin, cout, cuda, monkeypatch):
-    """Every plane tile and both column layouts, packed and unpacked rows, divided offsets: submanifold and strided layers,
-    against float64 and against the error of k_conv_fma."""
+def _on_six(offsets, cin, cout, rows, side=None):
+    """Which layers run on k_conv_six; side: of windows side by side, "fine" rows or "coarse" ones."""
+    weights = offsets * cin * cout
+    if rows < 512 or (cin <= 16 and rows < 16384) or (cout <= 16 and rows > 131072) or weights < (9000 if offsets < 27 else 6900):
+        return False
+    if weights * rows < (80e6 if rows >= 2048 else 220e6 if side else 160e6):
+        return False
+    if side == "coarse":
+        return cout > 64 or rows <= 90000
+    return side is None or cin * cout >= 20000 or (cin >= 96 and cin * cout >= 8000 and rows >= 40000)
+
+
+@pytest.mark.parametrize("sign", ["mixed", "one"])
+@pytest.mark.parametrize("cin,cout", [(8, 32), (8, 64), (12, 48), (16, 32), (32, 32), (36, 64), (64, 80), (64, 84), (96, 96), (32, 128),
+                                      (100, 132), (160, 128), (64, 256)])
+@pytest.mark.parametrize("n,split", [(700, None), (1700, None), (8191, None), (20001, None), (8200, "3"), (150000, None)])
+def test_as_accurate_as_multiply_adds(n, split, cin, cout, sign, cuda, monkeypatch):
+    """Every plane tile and both column layouts, packed and unpacked rows, divided offsets, long and short sums, sums that
+    cancel and sums of one sign, where the tensor core's truncation is a bias: against float64 and against the error of
+    k_conv_fma (of sums of at most 27 x 160 fp32 products: 1e-5, as in its own test)."""
     import sparseconvnet_b200 as scn
     lib = scn.SCN.lib
     if split:
@@ -34,26 +49,53 @@ def test_as_accurate_as_multiply_adds(n, split, cin, cout, cuda, monkeypatch):
     coords = _points(n, 3, 160 if n < 100000 else 512, n)
     x = scn.InputLayer(3, 512, mode=0)([torch.from_numpy(coords), torch.zeros(len(coords), 1, device=cuda)])
     torch.manual_seed(cin)
+    ran = 0
     with torch.no_grad():
-        for layer, kind, filt, stride in [(scn.SubmanifoldConvolution(3, cin, cout, 3, True), 0, [3, 3, 3], None),
-                                          (scn.Convolution(3, cin, cout, 2, 2, False), 1, [2, 2, 2], [2, 2, 2])]:
+        for layer, kind, filt, stride, side in [(scn.SubmanifoldConvolution(3, cin, cout, 3, True), 0, 3, None, None),
+                                                (scn.Convolution(3, cin, cout, 2, 2, False), 1, 2, 2, "coarse"),
+                                                (scn.Deconvolution(3, cin, cout, 2, 2, False), 1, 2, 2, "fine")]:
             layer.to(cuda)
+            layer.weight.normal_()
             if hasattr(layer, "bias"):
                 layer.bias.normal_()
-            f = torch.randn(len(coords), cin, device=cuda)
+            spatial = x.spatial_size // 2 if side == "fine" else x.spatial_size
+            f = torch.randn(x.metadata.getNActive(spatial), cin, device=cuda)
+            if sign == "one":
+                for t in (f, layer.weight) + ((layer.bias,) if hasattr(layer, "bias") else ()):
+                    t.abs_()
             errors = []
             for six in ("1", "0"):
                 monkeypatch.setenv("SCN_CONV_SIX", six)
-                y = layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features
-                if not errors and not lib.scn_last_conv_six():
-                    work = layer.weight.size(0) * cin * cout  # too little of it
-                    assert len(y) < 1500 or work * len(y) < 80e6 or work < 9000 or (cin <= 16 and len(y) < 16384)
-                    break
-                want = _exact(x, layer, kind, filt, stride, f, y.shape)
+                y = layer(scn.SparseConvNetTensor(f, x.metadata, spatial)).features
+                if six == "1":
+                    expected = _on_six(filt ** 3, cin, cout, len(y), side)
+                    assert lib.scn_last_conv_six() == expected, (layer, len(y))
+                    if not expected:
+                        break
+                    want = _exact(x, layer, kind, [filt] * 3, stride and [stride] * 3, f, y.shape)
                 errors.append(float((y.double() - want).norm() / want.norm()))
             x.metadata.poll_errors()
             if errors:
-                assert errors[0] <= 2.0 ** -22 and errors[0] <= 1.05 * errors[1], (layer, errors)
+                ran += 1
+                assert errors[0] <= 2.0 ** -22 and errors[1] <= 1e-5 and errors[0] <= 1.05 * errors[1], (layer, errors)
+    assert ran or n < 10000
+
+
+@pytest.mark.parametrize("planes", [32, 96, 160])
+def test_largest_part_of_a_product_left_out(planes, cuda, monkeypatch):
+    """1.0038986 = h + m + l with m = 2^-8 and l = -2^-17: the terms m l' and l m' that are left out are 2^-24 of every product of
+    it with itself, the most there can be, all of one sign.  Beside them an fp32 rounding at the end of each step."""
+    import sparseconvnet_b200 as scn
+    coords = _points(20001, 3, 160, 1)
+    x = scn.InputLayer(3, 160, mode=0)([torch.from_numpy(coords), torch.zeros(len(coords), 1, device=cuda)])
+    layer = scn.SubmanifoldConvolution(3, planes, planes, 3, False).to(cuda).requires_grad_(False)
+    layer.weight.fill_(1.0038986)
+    f = torch.full((len(coords), planes), 1.0038986, device=cuda)
+    y = layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features
+    assert scn.SCN.lib.scn_last_conv_six()
+    want = _exact(x, layer, 0, [3, 3, 3], None, f, y.shape)
+    assert float((y.double() - want).norm() / want.norm()) <= 2.0 ** -22
+    assert float(((y.double() - want) / want).abs().max()) <= 2.0 ** -21
 
 
 @pytest.mark.parametrize("case", ["inf", "nan", "huge", "tiny", "tiny weights", "inf weight", "zeros"])
