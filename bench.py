@@ -47,9 +47,8 @@ LIMITS = {
     "k_conv_tile": ("hbm", "the gather of whole rows from L2 into shared memory by 16-byte cp.async (ncu, 4-room case): LSU "
                            "wavefronts 39 % of peak on average and up to 53 %, tensor pipe 25 % (43 % on the widest levels), "
                            "issue slots 28 %; DRAM sees 0.27 of the algorithmic bytes"),
-    "k_conv_fma": ("hbm", "fp32 on tiles, most of it k_conv_six: the copies of rows and weights into shared memory, 30 to 48 KB per "
-                          "step of 128 rows and 32 planes, and the drain of the step's sums beside the tensor core (timed inside "
-                          "the kernel: 1 050 to 1 700 cycles per step, 340 to 800 of them tensor instructions)"),
+    "k_conv_six": ("hbm", "the copies of rows and weights into shared memory, 30 to 48 KB per step of 128 rows and 32 planes, and "
+                          "the drain of the step's sums beside the tensor core"),
 }
 # what `dtype` says for each arithmetic mode: the type the path computes in, kernel by kernel
 DTYPE_LABEL = {

@@ -87,7 +87,8 @@ enum scn_conv_kernel {
   SCN_KERNEL_CONV_ROWS = 4,          /* k_conv_rows and its first-layer forms: row-stationary, warp-level mma.sync */
   SCN_KERNEL_CONV_WIDE = 5,          /* k_conv_wide: tcgen05, persistent, rows split to bf16 parts once per call and copied in by cp.async */
   SCN_KERNEL_CONV_TILE = 6,          /* k_conv_tile: tcgen05, persistent, mask-sorted row tiles */
-  SCN_KERNEL_CONV_FMA = 7            /* fp32 on mask-sorted row tiles: k_conv_fma, or k_conv_six (scn_last_conv_six) */
+  SCN_KERNEL_CONV_FMA = 7,           /* k_conv_fma: fp32 FMA, mask-sorted row tiles           */
+  SCN_KERNEL_CONV_SIX = 8            /* k_conv_six: fp32 by six bf16 products on tcgen05, mask-sorted row tiles */
 };
 /* which kernel the last weight gradient of a convolution ran, whatever thread asked for it (autograd has its own) */
 enum scn_dweight_kernel {
@@ -254,8 +255,6 @@ SCN_API int scn_md_rulebook_export(scn_metadata *md, int kind, const int64_t *si
 /* -1 before the first convolution, else an scn_conv_kernel value.  No counterpart in the
  * reference; lets a profiler attribute a call's time to the kernel that ran it. */
 SCN_API int scn_last_conv_kernel(void);
-/* 1 if the last convolution call of this thread ran on k_conv_six (fp32 by six bf16 products on tcgen05) */
-SCN_API int scn_last_conv_six(void);
 SCN_API int scn_last_dweight_kernel(void);
 
 /* Self-calibration of the tensor path.  No counterpart in the reference.  Issues `n_mma`

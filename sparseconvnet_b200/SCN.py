@@ -139,7 +139,7 @@ def _macs_result(m, macs):
 
 # scn_last_conv_kernel() -> name (enum scn_conv_kernel of include/scn_b200.h)
 _KERNEL_NAMES = ("k_conv_simt", "k_conv_tc", "k_conv_tma", "k_conv_pipe_mma", "k_conv_rows", "k_conv_wide", "k_conv_tile",
-                 "k_conv_fma")
+                 "k_conv_fma", "k_conv_six")
 
 PRECISION_FP32, PRECISION_TF32, PRECISION_BF16, PRECISION_TF32X3 = 0, 1, 2, 3
 _precision = PRECISION_FP32

@@ -21,7 +21,6 @@ SIGNATURES = {
     "scn_rulebook_build_count": (C.c_longlong, []),
     "scn_host_wait_count": (C.c_longlong, []),
     "scn_last_conv_kernel": (C.c_int, []),
-    "scn_last_conv_six": (C.c_int, []),
     "scn_last_dweight_kernel": (C.c_int, []),
     "scn_tc_probe_mma": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _vp,
                                    C.POINTER(C.c_double), C.POINTER(C.c_double), C.POINTER(C.c_double)]),

@@ -162,7 +162,6 @@ int weight_image_put(WeightImage &img, cudaStream_t stream) {
 }
 
 static thread_local int g_last_kernel = -1;
-static thread_local bool g_last_six = false;  // k_conv_six, which reports as SCN_KERNEL_CONV_FMA
 static std::atomic<int> g_deferred_counts{0};
 std::atomic<int> g_backward_precision{SCN_PRECISION_FP32};  // arithmetic of the input-gradient pass
 
@@ -376,7 +375,6 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
                        int precision, int *flags, cudaStream_t stream, const float *bn_scale, const float *bn_shift,
                        float leak, const float *pre_scale, const float *pre_shift, float pre_leak, const float *in_b,
                        int planes_a) {
-  g_last_six = false;
   // the row order of the table: for a table of children (one rule per row) from the parents' side, without the table
   const auto row_order = [&](RowOrder &ord) -> int {
     if (transposed_table && rb.one_parent && rb.n_offsets <= kChildrenMaxOffsets) return rulebook_children_order(rb, ord, stream);
@@ -411,8 +409,7 @@ int conv_forward_table(Rulebook &rb, bool transposed_table, const float *in, lon
       return rc;
     }
     if (rc == SCN_OK && !no_memory) {
-      g_last_kernel = SCN_KERNEL_CONV_FMA;
-      g_last_six = true;
+      g_last_kernel = SCN_KERNEL_CONV_SIX;
       return SCN_OK;
     }
     cudaGetLastError();  // (of the allocation) k_conv_fma does with less
@@ -513,7 +510,6 @@ using namespace scn;
 extern "C" {
 
 int scn_last_conv_kernel(void) { return g_last_kernel; }
-int scn_last_conv_six(void) { return g_last_kernel == SCN_KERNEL_CONV_FMA && g_last_six; }
 
 int scn_set_split_rows(const void *in_split, void *out_split) {
   g_split_rows.in = in_split;

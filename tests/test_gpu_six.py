@@ -9,6 +9,7 @@ import torch
 from tests.test_gpu_tile import _points
 
 pytestmark = pytest.mark.gpu
+FMA, SIX = 7, 8  # scn_last_conv_kernel
 
 
 def _exact(x, layer, kind, filt, stride, f, shape):
@@ -69,7 +70,7 @@ def test_as_accurate_as_multiply_adds(n, split, cin, cout, sign, cuda, monkeypat
                 y = layer(scn.SparseConvNetTensor(f, x.metadata, spatial)).features
                 if six == "1":
                     expected = _on_six(filt ** 3, cin, cout, len(y), side)
-                    assert lib.scn_last_conv_six() == expected, (layer, len(y))
+                    assert lib.scn_last_conv_kernel() == (SIX if expected else FMA), (layer, len(y))
                     if not expected:
                         break
                     want = _exact(x, layer, kind, [filt] * 3, stride and [stride] * 3, f, y.shape)
@@ -92,7 +93,7 @@ def test_largest_part_of_a_product_left_out(planes, cuda, monkeypatch):
     layer.weight.fill_(1.0038986)
     f = torch.full((len(coords), planes), 1.0038986, device=cuda)
     y = layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features
-    assert scn.SCN.lib.scn_last_conv_six()
+    assert scn.SCN.lib.scn_last_conv_kernel() == SIX
     want = _exact(x, layer, 0, [3, 3, 3], None, f, y.shape)
     assert float((y.double() - want).norm() / want.norm()) <= 2.0 ** -22
     assert float(((y.double() - want) / want).abs().max()) <= 2.0 ** -21
@@ -127,7 +128,7 @@ def test_values_the_parts_cannot_hold(case, cin, cout, n, cuda, monkeypatch):
         monkeypatch.setenv(knob, "1")
         with torch.no_grad():
             outs.append(layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features)
-        assert scn.SCN.lib.scn_last_conv_six() == int(six)
+        assert scn.SCN.lib.scn_last_conv_kernel() == (SIX if six == "1" else FMA)
     x.metadata.poll_errors()
     got, want = outs
     if case == "inf weight":  # k_conv_fma multiplies the rows without a rule by it as well
@@ -157,7 +158,7 @@ def test_an_infinity_spoils_its_own_rows_only(cin, cout, n, split, cuda, monkeyp
     k = max((k for k in range(27) if k != 13), key=lambda k: len(book[k]))
     layer.weight[k, 0, 2, 1] = float("inf")
     y = layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features
-    assert scn.SCN.lib.scn_last_conv_six()
+    assert scn.SCN.lib.scn_last_conv_kernel() == SIX
     x.metadata.poll_errors()
     hit = torch.zeros(len(coords), cout, dtype=torch.bool, device=cuda)
     hit[book[k].long()[:, 1], 1] = True
@@ -182,7 +183,7 @@ def test_small_values_beside_ordinary_ones(small, cin, cout, cuda):
     tiny = torch.from_numpy(coords[:, 3] == 1).to(cuda)
     f[tiny] *= small
     y = layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features
-    assert scn.SCN.lib.scn_last_conv_six()
+    assert scn.SCN.lib.scn_last_conv_kernel() == SIX
     x.metadata.poll_errors()
     want = _exact(x, layer, 0, [3, 3, 3], None, f, y.shape)
     plane = torch.zeros(cout, dtype=torch.bool, device=cuda)
@@ -203,7 +204,7 @@ def test_weights_of_this_call(cin, cout, cuda):
     layer = scn.SubmanifoldConvolution(3, cin, cout, 3, False).to(cuda)
     with torch.no_grad():
         one = layer(x).features
-        assert scn.SCN.lib.scn_last_conv_six()
+        assert scn.SCN.lib.scn_last_conv_kernel() == SIX
         layer.weight.data.mul_(2)
         assert torch.equal(layer(x).features, 2 * one)
 
@@ -246,7 +247,7 @@ def test_bounded_wait_runs_out(cuda):
     with torch.no_grad():
         x = scn.InputLayer(3, 96, mode=0)([torch.from_numpy(coords), torch.randn(len(coords), 96, device=cuda)])
         good = layer(x).features.clone()
-        assert lib.scn_last_conv_six()
+        assert lib.scn_last_conv_kernel() == SIX
         x.metadata.poll_errors()
         assert lib.scn_test_drop_barrier_arrival() == 0
         layer(x)
@@ -284,7 +285,7 @@ def test_without_memory_for_the_parts(kind, cin, cout, n, cuda, monkeypatch):
         finally:
             left = lib.scn_test_fail_allocation(0)
         x.metadata.poll_errors()
-        return out, lib.scn_last_conv_six(), left
+        return out, lib.scn_last_conv_kernel() == SIX, left
     want, on_six, _ = run(0, "1")
     plain, on_fma, _ = run(0, "0")
     assert on_six and not on_fma

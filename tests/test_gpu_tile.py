@@ -103,6 +103,7 @@ def test_fp32_tiles(n, split, cin, cout, cuda, monkeypatch):
     every plane tile, with and without divided offsets.  Sums of at most 27 x 100 fp32 products: 2700 x 2^-24 of the
     largest sum of magnitudes at the very worst, 2^-24 sqrt(2700) in practice; 1e-5."""
     import sparseconvnet_b200 as scn
+    monkeypatch.setenv("SCN_CONV_SIX", "0")
     if split:
         monkeypatch.setenv("SCN_FMA_SPLIT", split)
     coords = _points(n, 3, 160, n)
