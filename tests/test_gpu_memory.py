@@ -55,6 +55,59 @@ def test_captured_convolution(n, precision, cuda):
         scn.set_precision("fp32")
 
 
+@pytest.mark.parametrize("precision", ["fp32", "tf32x3"])
+@pytest.mark.parametrize("n", [700, 30000])
+def test_captured_row_orders(n, precision, cuda):
+    """A Deconvolution and the gradients of a Convolution whose row orders are made while they are recorded: every replay makes
+    them again, the children's tiles from cursors that the replay before has left as it found them."""
+    import sparseconvnet_b200 as scn
+    from sparseconvnet_b200 import SCN
+    torch.manual_seed(n)
+    planes, pts = 160, _surface(n, 96)
+    up = scn.Deconvolution(3, planes, planes, 2, 2, True).to(cuda).requires_grad_(False)
+    first = scn.Convolution(3, 4, 4, 2, 2, False).to(cuda).requires_grad_(False)
+    w = torch.randn(8, 1, planes, planes, device=cuda)
+    size, half, two = torch.LongTensor([96] * 3), torch.LongTensor([48] * 3), torch.LongTensor([2] * 3)
+
+    def start():
+        x = scn.InputLayer(3, 96, mode=4)([pts, torch.randn(n, 4, device=cuda)])
+        return x.metadata, first(x).features.size(0), x.features.size(0)
+
+    def run(m, coarse, fine, d_in, dw):
+        y = up(scn.SparseConvNetTensor(coarse, m, half)).features
+        SCN.Convolution_backward(size, half, two, two, m, fine, d_in, coarse, w, dw, None)
+        return y
+    try:
+        scn.set_precision(precision)
+        scn.set_backward_precision(precision)
+        m, n_coarse, n_fine = start()
+        coarse, fine = torch.randn(n_coarse, planes, device=cuda), torch.randn(n_fine, planes, device=cuda)
+        d_in, dw = torch.empty_like(fine), torch.empty_like(w)
+        run(start()[0], coarse, fine, d_in, dw)  # (what the process sets up once)
+        side = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            y = run(m, coarse, fine, d_in, dw)
+        for _ in range(3):
+            coarse.copy_(torch.randn_like(coarse))
+            fine.copy_(torch.randn_like(fine))
+            for t in (y, d_in, dw):
+                t.fill_(float("nan"))
+            graph.replay()
+            torch.cuda.synchronize()
+            other = torch.empty_like(d_in), torch.empty_like(dw)
+            want = run(start()[0], coarse, fine, *other)
+            for a, b in ((y, want), (d_in, other[0]), (dw, other[1])):
+                assert torch.equal(a, b)
+        m.poll_errors()
+        del m
+        del graph
+    finally:
+        scn.set_precision("fp32")
+        scn.set_backward_precision("fp32")
+
+
 def _used():
     import ctypes as C
     from sparseconvnet_b200._lib import check, lib
