@@ -53,7 +53,7 @@ LIMITS = {
 # what `dtype` says for each arithmetic mode: the type the path computes in, kernel by kernel
 DTYPE_LABEL = {
     "fp32": "f32 (fp32 FMA, or every operand as three bf16 parts that hold it exactly and six bf16 products per term on "
-            "tcgen05, added up in fp32 registers every 32 planes, with the smaller error of the two)",
+            "tcgen05, added up in fp32 registers every 32 planes, with an error no larger)",
     "tf32x3": "f32-class split arithmetic, fp32 accumulate: every operand as two bf16 parts, three bf16 products "
               "per term on tcgen05 kind::f16 with TMEM accumulators",
     "tf32": "f32-class split arithmetic as tf32x3 (the mode asks for no less than one tf32 product); the first layer fp32",

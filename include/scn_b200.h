@@ -65,7 +65,7 @@ enum scn_status {
 enum scn_precision {
   SCN_PRECISION_FP32 = 0, /* fp32 operands and sums (matches the reference's float path): fp32 FMA, or on the tensor
                              cores with every operand as three bf16 parts, which hold it exactly, the six largest products
-                             of the parts and fp32 sums -- a smaller error than the FMA chain's.  Layers with non-finite
+                             of the parts and fp32 sums -- an error no larger than the FMA chain's.  Layers with non-finite
                              values, or whose largest products are near the ends of the range, are multiplied as plain
                              fp32 */
   SCN_PRECISION_TF32 = 1, /* at least one tf32 product, fp32 accumulate.  k_conv_tile computes it as

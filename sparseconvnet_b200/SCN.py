@@ -147,7 +147,7 @@ _precision = PRECISION_FP32
 
 def set_precision(p):
     """Arithmetic of the convolution kernels: 'fp32' (default; fp32 FMA, or six bf16 products of operands
-    in three exact parts where that is faster, with a smaller error), 'tf32x3' (tensor-core
+    in three exact parts where that is faster, with an error no larger), 'tf32x3' (tensor-core
     tiles over the hi/lo split of both operands: fp32-class accuracy), 'tf32' (no less than one tf32
     product; the layers that run on k_conv_tile get the three products of 'tf32x3') or 'bf16' (one
     bf16 product), all with fp32 accumulation."""

@@ -48,10 +48,10 @@ void note_launch();
 void note_host_wait();
 // A pass is a chain of up to 250 short kernels on one stream, and each used to start 1 to 2 us after the one before it had
 // ended.  They are launched with programmatic stream serialisation: the next kernel's blocks are put in place as the last
-// blocks of the one before leave, and wait at their first instruction (SCN_GRID_WAIT).  U-Net on eight rooms (186 launches)
-// 6511 -> 6158 us, on one room (178) 2288 -> 1972, one layer on 267 k sites (15) 281 -> 255.  No kernel asks for its
-// successor any earlier (griddepcontrol.launch_dependents): blocks that wait in the last wave's free places are handed out
-// to whichever SM has room first instead of evenly, 6499, 2079 and 277 us.
+// blocks of the one before leave, and wait at their first instruction (SCN_GRID_WAIT).  U-Net on eight rooms (186 launches
+// then, 147 since) 6511 -> 6158 us, on one room (178, 139) 2288 -> 1972, one layer on 267 k sites (15, 12) 281 -> 255.  No
+// kernel asks for its successor any earlier (griddepcontrol.launch_dependents): blocks that wait in the last wave's free
+// places are handed out to whichever SM has room first instead of evenly, 6499, 2079 and 277 us.
 #define SCN_LAUNCH(kernel, grid, block, smem, stream, ...)                                      \
   do {                                                                                         \
     scn::note_launch();                                                                        \

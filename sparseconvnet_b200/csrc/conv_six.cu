@@ -3,8 +3,9 @@
 // Same mathematics as the other convolution kernels (the reference's per-offset gather / GEMM / scatter-add is
 // CPU/Convolution.cpp:137-148, CUDA/Convolution.cu:57-233), in the precision of k_conv_fma (conv_fma.cu):
 //   * Every operand is written as the sum of three bf16 values, x = h + m + l: h = bf16(x), m = bf16(x - h), l = bf16(x - h - m).
-//     The three hold the 24 bits of x exactly.  A product is the six terms h h', h m', m h', h l', m m', l h'; what is left
-//     out is below 2^-26 of it, less than an fp32 product is rounded by.
+//     The three hold the 24 bits of x exactly.  A product is the six terms h h', h m', m h', h l', m m', l h'.  With m up to
+//     2^-8 of the value's power of two and l up to 2^-17, the two terms left out, m l' and l m', reach 2^-24 of a product at the
+//     very worst, as much as rounding an fp32 product can take, and are some 2^-28 in the mean.
 //   * The tensor core truncates its running sum, so it never runs far: one step of 32 planes of one filter offset is
 //     summed there, the large terms and the small ones apart or the small ones first, and every step's sums are added to fp32
 //     registers, rounded to nearest (the "drain" warps).
@@ -29,8 +30,8 @@
 // Bound by the copies into shared memory, 24 KB of rows and 6 (32 output planes) to 24 KB (128) of weights per step at about
 // 32 bytes per cycle and SM, against 336 to 768 cycles of tensor work; as multiply-adds the same step is 1 024 to 4 096 cycles
 // of the whole FMA pipe.  Rows split once per call, not once per gather: with fp32 rows (16 KB per step) split by the
-// producers on their way through registers a step took twice as long (32 -> 32 planes on 200 k rows 157 us, 88 with the split
-// pass; 96 -> 96 682 and 309).
+// producers on their way through registers a step took twice as long (32 -> 32 planes on 200 k rows 157 us against 88 when both
+// forms were there, 96 -> 96 682 against 309; 85 and 281 since).
 //
 // Every wait is bounded; on expiry the role raises the abort flag, everybody leaves, tensor memory is freed and
 // the host sees FLAG_TC_TIMEOUT through scn_md_poll_errors.
