@@ -166,6 +166,31 @@ def test_an_infinity_spoils_its_own_rows_only(cin, cout, n, split, cuda, monkeyp
     assert float((y.double() - want)[~hit].abs().max() / want.abs().max()) <= 1e-5
 
 
+@pytest.mark.parametrize("case", ["4-D", "down", "up"])
+def test_an_infinity_on_other_tables(case, cuda, monkeypatch):
+    """81 offsets in four mask words, coarse rows, tiles of one offset with rows left over: the bits of k_conv_fma."""
+    import sparseconvnet_b200 as scn
+    dim, cin, cout = (4, 32, 48) if case == "4-D" else (3, 160, 132)
+    coords = _points(20000, dim, 24 if dim == 4 else 90, 2)
+    x = scn.InputLayer(dim, 24 if dim == 4 else 90, mode=0)([torch.from_numpy(coords), torch.zeros(len(coords), 4, device=cuda)])
+    torch.manual_seed(dim)
+    layer = {"4-D": lambda: scn.SubmanifoldConvolution(4, cin, cout, 3, True), "down": lambda: scn.Convolution(3, cin, cout, 2, 2, True),
+             "up": lambda: scn.Deconvolution(3, cin, cout, 2, 2, True)}[case]().to(cuda).requires_grad_(False)
+    if case == "up":
+        x = scn.Convolution(3, 4, 4, 2, 2, False).to(cuda).requires_grad_(False)(x)
+    f = torch.randn(x.features.size(0), cin, device=cuda)
+    f[5, 3] = float("inf")
+    outs = []
+    for six, knob in (("1", "SCN_SIX_SPLIT"), ("0", "SCN_FMA_SPLIT")):
+        monkeypatch.setenv("SCN_CONV_SIX", six)
+        monkeypatch.setenv(knob, "1")
+        outs.append(layer(scn.SparseConvNetTensor(f, x.metadata, x.spatial_size)).features)
+        assert scn.SCN.lib.scn_last_conv_kernel() == (SIX if six == "1" else FMA)
+    x.metadata.poll_errors()
+    assert 0 < int((~torch.isfinite(outs[1])).sum()) < outs[1].numel() // 2
+    assert torch.equal(*(torch.nan_to_num(y, nan=7.0) for y in outs))
+
+
 @pytest.mark.parametrize("small", [1e-30, 1e-35, 1e-37])
 @pytest.mark.parametrize("cin,cout", [(24, 32), (32, 32), (40, 136)])
 def test_small_values_beside_ordinary_ones(small, cin, cout, cuda):
