@@ -1236,11 +1236,6 @@ static int build_strided(scn_metadata *md, Grid *gin, const int64_t *output_size
   long long n_ids = n_in * F.tmax;
   SCN_REQUIRE(n_ids < (1ll << 31), SCN_ERR_UNSUPPORTED, "too many (site, output) candidates");
 
-  auto old = md->grids.find(make_key(md->dim, output_size));
-  if (old != md->grids.end()) {
-    free_grid(old->second, stream);
-    md->grids.erase(old);
-  }
   SCN_TRY(make_layout(md->dim, output_size, gout.layout));
   SCN_REQUIRE(gout.layout.batch_bits >= gin->layout.batch_bits ||
                   gin->batch_size <= (1ll << gout.layout.batch_bits),
@@ -1342,7 +1337,10 @@ int get_strided_rulebook(scn_metadata *md, const int64_t *input_size, const int6
     free_rulebook(rb, stream);
     return st;
   }
-  md->grids[make_key(md->dim, output_size)] = gout;
+  // (the grid of that size that was there goes only now: with filter and stride 1 it is the one that has been read)
+  Grid &place = md->grids[make_key(md->dim, output_size)];
+  free_grid(place, stream);
+  place = gout;
   *out = &(md->strided_rules[key] = rb);
   return SCN_OK;
 }

@@ -112,3 +112,27 @@ def test_rows_without_a_rule(precision, tol, cuda):
     for got, exact in ((out, want), (d_in, grad)):
         e = helpers.rel_err(got.double().cpu().numpy(), exact.cpu().numpy())
         assert e <= tol, e
+
+
+@pytest.mark.parametrize("precision,tol", [("fp32", 1e-6), ("tf32x3", helpers.FP32_TOL)])
+@pytest.mark.parametrize("n", [1, 5000])
+def test_windows_of_one_site(n, precision, tol, cuda):
+    """Filter and stride 1: the coarse grid has the fine one's size and takes its place while it is read.  Sums of cin products."""
+    import sparseconvnet_b200 as scn
+    torch.manual_seed(n)
+    x = scn.InputLayer(3, 48, mode=1)([torch.from_numpy(_points(n, 3, 48, False)), torch.randn(n, 64, device=cuda)])
+    where = x.get_spatial_locations()
+    a, b = scn.Convolution(3, 64, 96, 1, 1, False), scn.Deconvolution(3, 96, 32, 1, 1, False)
+    try:
+        scn.set_precision(precision)
+        with torch.no_grad():
+            y = a.to(cuda)(x)
+            z = b.to(cuda)(y)
+        y.metadata.poll_errors()
+    finally:
+        scn.set_precision("fp32")
+    assert torch.equal(y.get_spatial_locations(), where) and torch.equal(z.get_spatial_locations(), where)
+    want = x.features.double() @ a.weight.detach().double()[0, 0]
+    for got, exact in ((y.features, want), (z.features, y.features.double() @ b.weight.detach().double()[0, 0])):
+        e = helpers.rel_err(got.double().cpu().numpy(), exact.cpu().numpy())
+        assert e <= tol, e
