@@ -17,21 +17,27 @@
 //     since the reads count: U-Net on eight rooms 6095 -> 6034 us, on one room 1912 -> 1884.  The small terms are no longer cut
 //     off against the large ones, so the error against float64 fell: 128 -> 128 planes on 60 k rows 6.6e-6 -> 4.7e-6, of one
 //     sign 6.9e-6 -> 3.7e-6; smaller for every shape of 80 to 128 planes.)
-//   * What bounds it is the gather: 128 bytes per row and 32-plane step (16 + 16 bits per value) through 16-byte
-//     cp.async at about 32 bytes per cycle and SM, 512 cycles per step against 224 cycles of tensor work for 32
-//     output planes, 304 for 96.
+//   * What bounds it is shared memory, 128 bytes per cycle and SM: a step of 32 -> 32 planes writes 16 KB of rows and 4 KB of
+//     weights and its four instructions read 22 KB, 336 cycles (416 for 64 -> 64, 496 for 96 -> 96, 576 for 128 -> 128), against
+//     176, 224, 304 and 384 cycles of tensor work.  L2 is not the limit: 16-byte cp.async gathers of rows that lie in L2 reach
+//     75 bytes per cycle and SM, twice what a step needs.
+//   * So that shared memory is busy all the time no role may take longer per step than that, and every barrier, load and store
+//     of shared memory waits 100 to 200 cycles behind the copies.  With a thread of its own for the weights (two waits, a
+//     load, an arrival and the copy per step: 1 050 cycles) and instructions issued inside a branch of one lane (descriptors moved
+//     into uniform registers one by one: 135 cycles per four instructions, 38 with a predicate) the same tiles took, 8 rooms:
+//     32 -> 32 planes 253 us, now 202; 64 -> 64 145, 132; 96 -> 96 98, 88; 128 -> 128 83, 70; 224 -> 224 on 1.4 k rows 22.6, 19.6;
+//     4-D 64 -> 64 bf16 778, 671.
 //
-// Roles (15 warps, one CTA per SM, persistent).  A step is one filter offset of one tile and SP input planes; the
+// Roles (14 warps, one or two CTAs per SM, persistent).  A step is one filter offset of one tile and SP input planes; the
 // steps of a CTA are numbered through all its tiles and step n uses stage n % n_stages of one ring.
-//   entries     one thread: a slot per (tile, filter offset with a rule), the input row of every tile row, one 512-byte
-//               bulk copy from the packed table; up to kSlots offsets ahead
-//   producers   8 warps, warp w takes steps w, w + 8, ...: all 128 rows of the step by 16-byte cp.async pieces
-//               straight into the swizzled operand layout, zero fill where a row has no rule; the barrier arrival
-//               happens when a lane's copies have landed.  (One warp per step: with a step spread over all warps its
-//               chain of waits and address arithmetic, longer than its copies take, was the time of the step: 1 500
-//               cycles against the 512 the copies need.)
-//   weights     one thread: one bulk copy per step
-//   MMA         one thread
+//   entries     one thread: a record per tile (steps, where its rows go) for the roles below, then a slot per filter offset with
+//               a rule, the input row of every tile row, one 512-byte bulk copy from the packed table; up to kSlots offsets ahead
+//   producers   8 warps, four to a step: 32 rows each by 16-byte cp.async pieces straight into the swizzled operand layout,
+//               zero fill where a row has no rule; the barrier arrival happens when a lane's copies have landed.  A warp has
+//               the entries of its next step in registers before the stage is free, which also gives the slot back early.
+//               The first lane of a step's warps also orders its weights, one bulk copy.  (One warp per step: 2 000
+//               cycles from the first copy to the last, during which the stage waits.)
+//   MMA         one warp
 //   epilogue    4 warps: tcgen05.ld (a lane holds a row) -> shared memory, 16 planes at a time -> bias -> optional
 //               BatchNorm scale / shift / leaky ReLU -> 16-byte stores, four lanes per row.  (Stored straight from the TMEM
 //               lanes every instruction touched 32 lines: a fifth of the cycles in which the gather could have issued.)
@@ -53,11 +59,12 @@ namespace scn {
 namespace {
 
 constexpr int kRows = kOrderTile;  // rows of a tile = MMA M
-constexpr int kProdWarps = 8;
-constexpr int kEpi0 = kProdWarps, kMma = kProdWarps + 4, kWgt = kMma + 1, kEntries = kMma + 2;
-constexpr int kThreads = (kProdWarps + 7) * 32;
-constexpr int kSlots = 8;       // offsets the entries run ahead; at least kProdWarps (the slots that end the work)
+constexpr int kProdWarps = 8, kStepWarps = 4, kProdGroups = kProdWarps / kStepWarps;
+constexpr int kEpi0 = kProdWarps, kMma = kProdWarps + 4, kEntries = kMma + 1;
+constexpr int kThreads = (kProdWarps + 6) * 32;
+constexpr int kSlots = 8;       // offsets the entries run ahead; even, so that a producing warp comes by every slot or every second
 constexpr int kMaxStages = 12;
+constexpr int kRecords = 4;     // items the entries run ahead of the epilogue
 constexpr int kEpiBytes = 32 * 64;  // per epilogue warp: 32 rows x 16 planes on their way from TMEM lanes to whole lines
 
 struct TileParams {
@@ -87,7 +94,7 @@ template <int TERMS, int SP>
 struct TileShape {
   static constexpr int PARTS = TERMS == 3 ? 2 : 1;
   static constexpr int PP = SP * 2 * PARTS / 16;      // 16-byte pieces per row and step
-  static constexpr int NI = kRows / (32 / PP);        // copy instructions per step and lane
+  static constexpr int NI = 32 / (32 / PP);           // copy instructions per step and lane: a warp has 32 rows of a step
   static constexpr unsigned ROW = PP * 16;            // bytes of a row in a stage: 128 or 64
   static constexpr unsigned A_BYTES = kRows * ROW;
   static_assert(PP == 8 || PP == 4, "a row of a step is 128 or 64 bytes");
@@ -97,28 +104,45 @@ struct TileShape {
 struct Ctl {
   unsigned long long full[kMaxStages], empty[kMaxStages];  // rows and weights landed; MMAs done
   unsigned long long s_full[kSlots], s_empty[kSlots], acc_full[4], acc_empty[4];
+  unsigned long long r_full[kRecords], r_empty[kRecords];
+  struct Record {
+    int steps, tile, part, next_tile;  // of an item; the tile of the item behind it
+  } record[kRecords];
   int slot_k[kSlots];  // filter offset of the slot; -1: no more work; kNoRules: offset 0 with rows of zeros
   unsigned tmem;
   int abort;
 };
 
 // The tile of an item: the tiles with the most offsets first (packed tiles come in ascending order of their masks, so from
-// the back where they have not been sorted by work).
-__device__ __forceinline__ long long item_tile(const TileParams &P, long long item) {
-  const long long i = P.n_split == 1 ? item : item / P.n_split;
-  return P.by_work ? __ldg(P.by_work + i) : P.n_tiles - 1 - i;
+// the back where they have not been sorted by work).  Past the last item any tile.
+__device__ __forceinline__ int item_tile(const TileParams &P, long long item) {
+  if (item >= P.n_items) return 0;
+  const int i = P.n_split == 1 ? (int)item : (int)item / P.n_split;
+  return P.by_work ? __ldg(P.by_work + i) : (int)P.n_tiles - 1 - i;
 }
 
-// filter offsets of an item: those of its tile, or its share of them when the offsets are divided
-__device__ __forceinline__ int item_offsets(const TileParams &P, long long item) {
-  if (item >= P.n_items) return 0;
-  const long long t = item_tile(P, item);
-  int total = 0;
-  for (int w = 0; w < P.words; ++w) total += __popc(__ldg(P.tile_bits + t * P.words + w));
-  if (P.n_split == 1) return total;
-  const int part = (int)(item % P.n_split);
-  return total * (part + 1) / P.n_split - total * part / P.n_split;
-}
+// The tiles of a CTA's items in turn: the tile of an item is asked for three items ahead and its mask of offsets one ahead, so
+// that neither trip to memory is waited for between two tiles.
+struct Tiles {
+  int tile, next, next2;
+  unsigned mask[4], next_mask[4];
+  __device__ __forceinline__ void fetch(const TileParams &P, int t, unsigned (&m)[4]) {
+#pragma unroll
+    for (int w = 0; w < 4; ++w) m[w] = w < P.words ? __ldg(P.tile_bits + (long long)t * P.words + w) : 0u;
+  }
+  __device__ __forceinline__ explicit Tiles(const TileParams &P) {
+    tile = item_tile(P, item_of(0)), next = item_tile(P, item_of(1)), next2 = item_tile(P, item_of(2));
+    fetch(P, tile, mask);
+    fetch(P, next, next_mask);
+  }
+  // from item `it` to the one behind it
+  __device__ __forceinline__ void advance(const TileParams &P, long long it) {
+    tile = next, next = next2, next2 = item_tile(P, item_of(it + 3));
+#pragma unroll
+    for (int w = 0; w < 4; ++w) mask[w] = next_mask[w];
+    fetch(P, next, next_mask);
+  }
+};
 
 template <int TERMS, int SP, bool OUT_SPLIT>
 __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
@@ -141,12 +165,16 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
 
   if (tid == 0) {
     for (int i = 0; i < P.n_stages; ++i) {
-      mbar_init(&C.full[i], 32 + 1);  // the producing warp's lanes and the weights
+      mbar_init(&C.full[i], kStepWarps * 32 + 1);  // the lanes of the producing warps, and the weights
       mbar_init(&C.empty[i], 1);
     }
     for (int i = 0; i < kSlots; ++i) {
       mbar_init(&C.s_full[i], 1);
-      mbar_init(&C.s_empty[i], P.n_slices + 1);    // a producer warp per slice, and the weights
+      mbar_init(&C.s_empty[i], kStepWarps * min(P.n_slices, kProdGroups));  // the producing warps that come by
+    }
+    for (int i = 0; i < kRecords; ++i) {
+      mbar_init(&C.r_full[i], 1);
+      mbar_init(&C.r_empty[i], 4 + 1);  // the epilogue's warps and the issuing one
     }
     for (int i = 0; i < 4; ++i) {
       mbar_init(&C.acc_full[i], 1);
@@ -165,98 +193,81 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
 
   if (warp < kProdWarps) {
     // ==================================== producers =============================================
-    // this lane's 16-byte piece of the rows q NI .. q NI + NI - 1 (the entries of a lane follow one another)
-    const int j = lane % PP, q = lane / PP;
-    const unsigned lane_dst = (unsigned)(q * NI) * Shape::ROW + (unsigned)j * 16;
-    // No more warps than stages: a warp at step n has seen the consumption of step n - active - n_stages, and its wait
-    // below can tell step n - n_stages from the one a round earlier only if that one is not later than this.
-    const int active = min(kProdWarps, P.n_stages);
-    const int d_slot = active / P.n_slices, d_slice = active % P.n_slices;
-    const int d_round = active / P.n_stages, d_st = active % P.n_stages;
-    int slot = warp / P.n_slices, slice = warp % P.n_slices;
-    int round = warp / P.n_stages, st = warp % P.n_stages;
-    bool ok = true, bad = false;
-    while (warp < active) {
-      const int si = slot % kSlots;
-      if (!mbar_wait(&C.s_full[si], (slot / kSlots) & 1)) {
-        ok = false;
-        break;
-      }
-      const int slot_k = C.slot_k[si];
-      if (slot_k < 0 || *abort) break;
-      const int rows_in = slot_k == kNoRules ? 0 : (int)P.n_in;  // entries below it are rows
-      const int4 *ent = reinterpret_cast<const int4 *>(entries + si * kRows + q * NI);
-      if (!mbar_wait(&C.empty[st], (round + 1) & 1)) {  // (the first round passes)
-        ok = false;
-        break;
-      }
-      const unsigned dst = smem0 + (unsigned)st * stage_bytes + lane_dst;
-      const unsigned char *col = P.in_split + slice * (SP * 2 * PARTS) + j * 16;
-#pragma unroll
-      for (int i = 0; i < NI; i += 4) {
-        const int4 e4 = ent[i / 4];
-        const int v[4] = {e4.x, e4.y, e4.z, e4.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const bool hit = (unsigned)v[e] < (unsigned)rows_in;
-          bad |= v[e] >= (int)P.n_in && slot_k != kNoRules;
-          const unsigned swizzle = (PP == 8 ? (i + e) & 7 : ((i + e) >> 1) & 3) * 16;  // (q NI is a multiple of eight)
-          cp_async16((dst ^ swizzle) + (i + e) * Shape::ROW, col + (size_t)(unsigned)(hit ? v[e] : 0) * P.row_bytes, hit ? 16u : 0u);
-        }
-      }
-      cp_async_arrive(&C.full[st]);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&C.s_empty[si]);
-      slot += d_slot, slice += d_slice;
-      if (slice >= P.n_slices) slice -= P.n_slices, ++slot;
-      round += d_round, st += d_st;
-      if (st >= P.n_stages) st -= P.n_stages, ++round;
-    }
-    if (bad) atomicOr(P.flags, FLAG_BAD_ROW);
-    asm volatile("cp.async.wait_all;" ::: "memory");  // they must land before the CTA's shared memory goes away
-    if (!ok) *abort = 1;
-  } else if (warp == kWgt) {
-    // ==================================== weights ===============================================
-    if (lane == 0) {
-      int st = 0, par = 1;
-      long long filled = 0;
-      bool ok = true;
-      for (int slot = 0; ok; ++slot) {
+    // Group g of four warps takes the steps g, g + 2, ...; a warp copies 32 rows of a step, a lane one 16-byte piece of the
+    // rows q NI .. q NI + NI - 1 of them.  The input rows of the next step are in registers before its stage is free.
+    const int j = lane % PP, q = lane / PP, group = warp / kStepWarps, row0 = warp % kStepWarps * 32 + q * NI;
+    // (ROW 128: rows come in eights, chunk j of row r is stored at j ^ (r & 7); ROW 64: in fours, at j ^ ((r >> 1) & 3))
+    const unsigned lane_dst = smem0 + (unsigned)row0 * Shape::ROW + (unsigned)((PP == 8 ? j : j ^ (q & 1) * 2) * 16);
+    const int d_slot = kProdGroups / P.n_slices, d_slice = kProdGroups % P.n_slices;
+    int slot = group / P.n_slices, slice = group % P.n_slices, st = group, par = 1;  // (n_stages is at least kProdGroups)
+    const bool brings_weights = warp % kStepWarps == 0 && lane == 0;
+    int slot_k = 0, filled = 0;
+    bool ok = true, bad = false, fresh = true;
+    const unsigned char *const col = P.in_split + j * 16;
+    int rows[NI];
+    for (;;) {
+      if (fresh) {
         const int si = slot % kSlots;
+        // (A warp comes by every slot, or by every second one with one slice: it has seen the slot kSlots before this one
+        // filled, so the parity cannot be that of an earlier round.)
         if (!mbar_wait(&C.s_full[si], (slot / kSlots) & 1)) {
           ok = false;
           break;
         }
-        const int k = C.slot_k[si];
-        mbar_arrive(&C.s_empty[si]);
-        if (k < 0) break;
-        const unsigned char *src = P.wprep + (size_t)(k == kNoRules ? 0 : k) * P.n_slices * w_bytes;
-        for (int s = 0; s < P.n_slices; ++s) {
-          if (!mbar_wait(&C.empty[st], par) || *abort) {
-            ok = false;
-            break;
-          }
-          if (!(P.drop && blockIdx.x == 0 && filled == 0)) {
-            mbar_expect_tx(&C.full[st], w_bytes);
-            bulk_copy_g2s(smem0 + (unsigned)st * stage_bytes + Shape::A_BYTES, src + (size_t)s * w_bytes, w_bytes, &C.full[st]);
-          }
-          ++filled;
-          if (++st == P.n_stages) st = 0, par ^= 1;
+        slot_k = C.slot_k[si];
+        if (slot_k < 0 || *abort) break;
+        const int4 *ent = reinterpret_cast<const int4 *>(entries + si * kRows + row0);
+#pragma unroll
+        for (int i = 0; i < NI; i += 4) {
+          const int4 e4 = ent[i / 4];
+          rows[i] = e4.x, rows[i + 1] = e4.y, rows[i + 2] = e4.z, rows[i + 3] = e4.w;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&C.s_empty[si]);
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+          if (slot_k == kNoRules) rows[i] = -1;
+          bad |= rows[i] >= (int)P.n_in;
         }
       }
-      if (!ok) {  // slabs in flight must land before the CTA's shared memory goes away
-        *abort = 1;
-        for (int i = 0; i < P.n_stages; ++i) {
-          const long long uses = (filled + P.n_stages - 1 - i) / P.n_stages;
-          if (uses > 0) mbar_wait(&C.full[i], (unsigned)((uses - 1) & 1));
-        }
+      if (!mbar_wait(&C.empty[st], par)) {  // (the first round passes)
+        ok = false;
+        break;
       }
+      const unsigned dst = lane_dst + (unsigned)st * stage_bytes;
+      if (brings_weights && !(P.drop && blockIdx.x == 0 && group == 0 && filled == 0)) {
+        const unsigned char *w = P.wprep + ((size_t)(slot_k == kNoRules ? 0 : slot_k) * P.n_slices + slice) * w_bytes;
+        mbar_expect_tx(&C.full[st], w_bytes);
+        bulk_copy_g2s(smem0 + (unsigned)st * stage_bytes + Shape::A_BYTES, w, w_bytes, &C.full[st]);
+      }
+      ++filled;
+      const unsigned char *src = col + slice * (SP * 2 * PARTS);
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        const bool hit = (unsigned)rows[i] < (unsigned)P.n_in;
+        const unsigned swizzle = (PP == 8 ? i & 7 : i >> 1 & 3) * 16;
+        cp_async16((dst ^ swizzle) + i * Shape::ROW, src + (size_t)(unsigned)(hit ? rows[i] : 0) * P.row_bytes, hit ? 16u : 0u);
+      }
+      cp_async_arrive(&C.full[st]);
+      slot += d_slot, slice += d_slice;
+      fresh = d_slot > 0;
+      if (slice >= P.n_slices) slice -= P.n_slices, ++slot, fresh = true;
+      st += kProdGroups;
+      if (st >= P.n_stages) st -= P.n_stages, par ^= 1;
+    }
+    if (bad) atomicOr(P.flags, FLAG_BAD_ROW);
+    asm volatile("cp.async.wait_all;" ::: "memory");  // they must land before the CTA's shared memory goes away
+    if (!ok) {
+      *abort = 1;
+      if (brings_weights)  // and so must the slabs
+        for (int i = max(0, filled - (P.n_stages + 1) / kProdGroups); i < filled; ++i) {
+          const int n = group + i * kProdGroups;
+          mbar_wait(&C.full[n % P.n_stages], (n / P.n_stages) & 1);
+        }
     }
   } else if (warp == kMma) {
     // ==================================== MMA issue =============================================
-    // The whole warp runs the loop and one elected lane issues: with warp-uniform control flow and operands (votes and
-    // reductions instead of loaded flags) the descriptors stay in uniform registers.  Issued from inside a lane == 0
-    // branch every instruction cost 200 to 260 cycles of moves and address arithmetic, four to eight times its own.
+    // The whole warp runs the loop and one elected lane issues, by a predicate (mma_bf16_if).
     const unsigned id_all = tile_idesc(joint ? 2 * P.coutp : P.coutp), id_one = tile_idesc(P.coutp);
     const unsigned long long a_desc = rows_desc<Shape::ROW>(smem0, 0);
     const unsigned long long w_desc = smem_desc(smem0 + Shape::A_BYTES, 128, SP / 8 * 128);
@@ -265,48 +276,53 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     const unsigned stage_step = stage_bytes >> 4, wm_step = w_part >> 4;
     const int items = (int)my_items, n_stages = P.n_stages, coutp = P.coutp;
     int st = 0, par = 0, buf = 0, buf_par = 1;
-    unsigned at = 0, d = tmem;
+    unsigned d = tmem;
     bool ok = true;
-    const bool leader = elect_one();
-    int offsets_next = item_offsets(P, item_of(0));
+    const unsigned lead = elect_one() ? 1u : 0u;
+    bool ready = false;  // the stage at hand, looked at while the instructions of the one before it were issued
     for (int i = 0; i < items && ok; ++i) {
-      const int steps = __reduce_max_sync(0xffffffffu, max(1, offsets_next)) * P.n_slices;
-      offsets_next = item_offsets(P, item_of(i + 1));
+      const int ri = i % kRecords;
+      if (!mbar_wait_warp(&C.r_full[ri], (i / kRecords) & 1)) {
+        ok = false;
+        break;
+      }
+      const int steps = __reduce_max_sync(0xffffffffu, C.record[ri].steps);
+      if (lead) mbar_arrive(&C.r_empty[ri]);
       // the item's accumulator must have been drained
       if (!mbar_wait_warp(&C.acc_empty[buf], buf_par) || __any_sync(0xffffffffu, *abort != 0)) {
         ok = false;
         break;
       }
       for (int s = 0; s < steps; ++s) {
-        if (!mbar_wait_warp(&C.full[st], par)) {
+        if (!ready && !mbar_wait_warp(&C.full[st], par)) {
           ok = false;
           break;
         }
-        if (leader) {
-          // order the copied rows (acquired through the barrier) before the tensor core's async-proxy reads; done
-          // here, not by the producers: their fence would wait for the copies they have just started
-          fence_proxy_async_smem();
-          tc_fence_after();
+        const int st1 = st + 1 == n_stages ? 0 : st + 1, par1 = st1 ? par : par ^ 1;
+        const unsigned seen = mbar_test(&C.full[st1], par1);
+        // order the copied rows (acquired through the barrier) before the tensor core's async-proxy reads; done
+        // here, not by the producers: their fence would wait for the copies they have just started
+        fence_proxy_async_smem();
+        tc_fence_after();
+        const unsigned at = (unsigned)st * stage_step;
 #pragma unroll
-          for (int jj = 0; jj < SP / 16; ++jj) {
-            const unsigned ah = a0 + at + jj * 2, am = ah + SP / 8, wh = w0 + at + jj * 16;
-            if (jj == 0) mma_bf16(d, ah, a_hi, wh, w_hi, joint ? id_all : id_one, (unsigned)s);
-            else mma_bf16_acc(d, ah, a_hi, wh, w_hi, joint ? id_all : id_one);
-            if (TERMS == 3) {
-              if (joint) {
-                mma_bf16_acc(d + coutp, am, a_hi, wh, w_hi, id_one);
-              } else {
-                mma_bf16_acc(d, ah, a_hi, wh + wm_step, w_hi, id_one);
-                mma_bf16_acc(d, am, a_hi, wh, w_hi, id_one);
-              }
+        for (int jj = 0; jj < SP / 16; ++jj) {
+          const unsigned ah = a0 + at + jj * 2, am = ah + SP / 8, wh = w0 + at + jj * 16;
+          if (jj == 0) mma_bf16_if(lead, d, ah, a_hi, wh, w_hi, joint ? id_all : id_one, (unsigned)s);
+          else mma_bf16_acc_if(lead, d, ah, a_hi, wh, w_hi, joint ? id_all : id_one);
+          if (TERMS == 3) {
+            if (joint) {
+              mma_bf16_acc_if(lead, d + coutp, am, a_hi, wh, w_hi, id_one);
+            } else {
+              mma_bf16_acc_if(lead, d, ah, a_hi, wh + wm_step, w_hi, id_one);
+              mma_bf16_acc_if(lead, d, am, a_hi, wh, w_hi, id_one);
             }
           }
-          tc_commit(&C.empty[st]);
-          if (s == steps - 1) tc_commit(&C.acc_full[buf]);
         }
-        __syncwarp();
-        at += stage_step;
-        if (++st == n_stages) st = 0, par ^= 1, at = 0;
+        tc_commit_if(lead, &C.empty[st]);
+        if (s == steps - 1) tc_commit_if(lead, &C.acc_full[buf]);
+        st = st1, par = par1;
+        ready = __all_sync(0xffffffffu, seen != 0);
       }
       d += dcols;
       if (++buf == n_acc) buf = 0, buf_par ^= 1, d = tmem;
@@ -317,29 +333,31 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     if (lane == 0) {
       int slot = 0;
       bool ok = true;
-      unsigned b_next[4];
-      auto fetch = [&](long long item) {
-#pragma unroll
-        for (int w = 0; w < 4; ++w)
-          b_next[w] = item < P.n_items && w < P.words ? __ldg(P.tile_bits + item_tile(P, item) * P.words + w) : 0u;
-      };
-      fetch(item_of(0));
+      Tiles tiles(P);
       for (long long it = 0; it < my_items && ok; ++it) {
-        const long long item = item_of(it);
         unsigned u[4];
 #pragma unroll
-        for (int w = 0; w < 4; ++w) u[w] = b_next[w];
-        fetch(item_of(it + 1));
-        const int *src = P.packed + item_tile(P, item) * P.K * kRows;
+        for (int w = 0; w < 4; ++w) u[w] = tiles.mask[w];
+        const int tile = tiles.tile, part = P.n_split == 1 ? 0 : (int)item_of(it) % P.n_split;
+        const int *src = P.packed + (long long)tile * P.K * kRows;
+        tiles.advance(P, it);
+        int offsets = __popc(u[0]) + __popc(u[1]) + __popc(u[2]) + __popc(u[3]);
         if (P.n_split > 1) {
-          const int total = __popc(u[0]) + __popc(u[1]) + __popc(u[2]) + __popc(u[3]), part = (int)(item % P.n_split);
-          const int first = total * part / P.n_split;
-          keep_range(u, first, total * (part + 1) / P.n_split);
+          const int first = offsets * part / P.n_split, last = offsets * (part + 1) / P.n_split;
+          keep_range(u, first, last);
           src += first * kRows;
+          offsets = last - first;
         }
         // a tile (or part) without any rule still gets one step, of weights and rows of zeros
-        bool none = (u[0] | u[1] | u[2] | u[3]) == 0;
+        const bool none = offsets == 0;
         if (none) u[0] = 1u;
+        const int ri = (int)it % kRecords;
+        if (!mbar_wait(&C.r_empty[ri], (((int)it / kRecords) + 1) & 1)) {
+          ok = false;
+          break;
+        }
+        C.record[ri] = Ctl::Record{max(1, offsets) * P.n_slices, tile, part, tiles.tile};
+        mbar_arrive(&C.r_full[ri]);
 #pragma unroll 1
         for (int w = 0; w < 4 && ok; ++w) {
           unsigned m = u[0];
@@ -361,8 +379,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
         }
       }
       const int filled = slot;
-      // every producer warp finds its next step in a slot that ends it
-      const int ends = (min(kProdWarps, P.n_stages) - 1) / P.n_slices + 1;
+      // every producing warp finds its next step in a slot that ends it
+      const int ends = (kProdGroups - 1) / P.n_slices + 1;
       for (int i = 0; i < ends && ok; ++i, ++slot) {
         const int si = slot % kSlots;
         if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1)) {
@@ -386,11 +404,20 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     const int nc = P.cout;
     float4 *my_epi = reinterpret_cast<float4 *>(epi + quad * kEpiBytes);
     int buf = 0, buf_par = 0;
-    for (long long it = 0; it < my_items; ++it) {
-      const long long item = item_of(it), t = item_tile(P, item);
-      const int part = (int)(item % P.n_split);
-      const int orow = __ldg(P.order + t * kRows + quad * 32 + lane);
+    int next_orow = 0;  // this lane's row of the next item: asked for an item ahead
+    for (int it = 0; it < (int)my_items; ++it) {
+      const int ri = it % kRecords;
       int got = 1;
+      if (lane == 0) got = mbar_wait(&C.r_full[ri], (it / kRecords) & 1) ? 1 : 0;
+      if (!__shfl_sync(0xffffffffu, got, 0)) {
+        *abort = 1;
+        break;
+      }
+      const Ctl::Record R = C.record[ri];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&C.r_empty[ri]);
+      const int orow = it ? next_orow : __ldg(P.order + (long long)R.tile * kRows + quad * 32 + lane);
+      next_orow = __ldg(P.order + (long long)R.next_tile * kRows + quad * 32 + lane);
       if (lane == 0) got = (!*abort && mbar_wait(&C.acc_full[buf], buf_par)) ? 1 : 0;
       got = __shfl_sync(0xffffffffu, got, 0);
       if (!got) {
@@ -399,33 +426,22 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
       }
       tc_fence_after();
       const unsigned base = tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(buf * dcols);
-      // where rows lane / 4, + 8, + 16, + 24 of the warp go: this lane's four planes of them, or (OUT_SPLIT, which is short of
-      // registers) the row.  Two CTAs of 15 warps have 64 registers a thread, and which form fits them was measured: 32 planes
-      // on 200 k rows 51 us in both kernels, 56 with rows and eight columns at a time where nothing is split; 160 planes on
-      // 3 k rows 24 us, 26 with rows and sixteen columns.
-      long long at[4];
+      // where rows lane / 4, + 8, + 16, + 24 of the warp go: rows of the result, or of the partial sums
       int to[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int r = __shfl_sync(0xffffffffu, orow, i * 8 + (lane >> 2));
-        if (OUT_SPLIT) to[i] = r;
-        else at[i] = r < 0 ? -1 : (P.n_split > 1 ? ((long long)part * P.n_tiles + t) * kRows + quad * 32 + i * 8 + (lane >> 2) : r) * nc + (lane & 3) * 4;
+        to[i] = __shfl_sync(0xffffffffu, orow, i * 8 + (lane >> 2));
+        if (!OUT_SPLIT && P.n_split > 1 && to[i] >= 0) to[i] = (R.part * (int)P.n_tiles + R.tile) * kRows + quad * 32 + i * 8 + (lane >> 2);
       }
       for (int c0 = 0; c0 < nc; c0 += 16) {
-        constexpr int kCols = OUT_SPLIT ? 8 : 16;
 #pragma unroll
-        for (int half = 0; half < 16; half += kCols) {
-          unsigned a[kCols], b[kCols];
-          if constexpr (OUT_SPLIT) {
-            tmem_ld8_nowait(base + c0 + half, a);
-            if (joint) tmem_ld8_nowait(base + P.coutp + c0 + half, b);
-          } else {
-            tmem_ld16_nowait(base + c0, a);
-            if (joint) tmem_ld16_nowait(base + P.coutp + c0, b);
-          }
+        for (int half = 0; half < 16; half += 8) {
+          unsigned a[8], b[8];
+          tmem_ld8_nowait(base + c0 + half, a);
+          if (joint) tmem_ld8_nowait(base + P.coutp + c0 + half, b);
           tmem_wait_ld();
 #pragma unroll
-          for (int e = 0; e < kCols; e += 4) {
+          for (int e = 0; e < 8; e += 4) {
             float4 v;
             v.x = __uint_as_float(a[e]), v.y = __uint_as_float(a[e + 1]), v.z = __uint_as_float(a[e + 2]), v.w = __uint_as_float(a[e + 3]);
             if (joint) {
@@ -445,11 +461,15 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
             sc = __ldg(reinterpret_cast<const float4 *>(P.bn_scale + c));
             sh = __ldg(reinterpret_cast<const float4 *>(P.bn_shift + c));
           }
+          float4 vs[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int row = i * 8 + (lane >> 2);
-            float4 v = my_epi[row * 4 + ((lane & 3) ^ ((row >> 1) & 3))];
-            if (OUT_SPLIT ? to[i] < 0 : at[i] < 0) continue;
+            vs[i] = my_epi[row * 4 + ((lane & 3) ^ ((row >> 1) & 3))];
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float4 v = vs[i];
             if (finish && P.bias) v.x += bias.x, v.y += bias.y, v.z += bias.z, v.w += bias.w;
             if (finish && P.bn_scale) {  // separate multiply and add, as the stand-alone BatchNorm kernel rounds them
               v.x = __fadd_rn(__fmul_rn(v.x, sc.x), sh.x), v.y = __fadd_rn(__fmul_rn(v.y, sc.y), sh.y);
@@ -457,7 +477,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
               v.x *= v.x > 0.f ? 1.f : P.leak, v.y *= v.y > 0.f ? 1.f : P.leak;
               v.z *= v.z > 0.f ? 1.f : P.leak, v.w *= v.w > 0.f ? 1.f : P.leak;
             }
-            *reinterpret_cast<float4 *>(P.out + (OUT_SPLIT ? (long long)to[i] * nc + c : at[i] + c0)) = v;
+            if (to[i] < 0) continue;
+            *reinterpret_cast<float4 *>(P.out + (long long)to[i] * nc + c) = v;
             if (OUT_SPLIT) {
               uint2 h, m;
               split_bf16_pair(v.x, v.y, h.x, m.x);
@@ -732,7 +753,7 @@ int conv_forward_tile(const float *in, long long n_in, float *out, long long n_o
   g_drop_arrival = 0;
   const double w_bytes = (double)coutp * SP * 2 * parts, a_bytes = kRows * SP * 2.0 * parts;
   const char *e = getenv("SCN_TILE_SPLIT");
-  P.n_split = e ? std::max(1, atoi(e)) : split_parts(P.n_tiles, ord.one_offset ? 1 : K, n_slices, (a_bytes + w_bytes) / 32.0, cout, n_sm);
+  P.n_split = e ? std::max(1, std::min<int>(atoi(e), (int)((1ll << 31) / (P.n_tiles * kRows) - 1))) : split_parts(P.n_tiles, ord.one_offset ? 1 : K, n_slices, (a_bytes + w_bytes) / 32.0, cout, n_sm);
   P.out_split = P.n_split > 1 ? nullptr : out_split;
   if (P.n_split > 1) SCN_TRY(tmp.get(&P.out, (size_t)P.n_split * P.n_tiles * kRows * cout * sizeof(float)));
   const auto launch = terms == 3 ? (SP == 32 ? launch_tile<3, 32> : launch_tile<3, 16>) : (SP == 64 ? launch_tile<1, 64> : launch_tile<1, 32>);

@@ -53,6 +53,16 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long *bar) {
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+// Has the phase completed?  (does not wait)
+__device__ __forceinline__ unsigned mbar_test(unsigned long long *bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return done;
+}
 // Bounded wait: returns false if the phase did not complete within the iteration limit.
 __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned parity) {
   unsigned addr = smem_u32(bar);
@@ -165,6 +175,31 @@ __device__ __forceinline__ bool mbar_wait_warp(unsigned long long *bar, unsigned
     if (__all_sync(0xffffffffu, done != 0)) return true;
   }
   return false;
+}
+// D[128 x N] (+)= A * B; descriptors as (low, high) words.  The whole warp comes here with the same operands and the lane whose
+// `lead` is set issues: a predicate instead of a branch, so that the descriptors are made in uniform registers.  Four
+// instructions and their commit take 38 + 20 cycles of the warp like this, 135 + 57 inside a branch of one lane.
+__device__ __forceinline__ void mma_bf16_if(unsigned lead, unsigned d, unsigned a_lo, unsigned a_hi, unsigned b_lo, unsigned b_hi,
+                                            unsigned idesc, unsigned accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\tsetp.ne.u32 e, %7, 0;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void mma_bf16_acc_if(unsigned lead, unsigned d, unsigned a_lo, unsigned a_hi, unsigned b_lo, unsigned b_hi,
+                                                unsigned idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\tsetp.ne.u32 e, %6, 0;\n\t"
+      "setp.eq.u32 p, 0, 0;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_if(unsigned lead, unsigned long long *bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.u32 e, %1, 0;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(lead)
+      : "memory");
 }
 // D[128 x N] (+)= A * B; descriptors as (low, high) words
 __device__ __forceinline__ void mma_bf16(unsigned d, unsigned a_lo, unsigned a_hi, unsigned b_lo, unsigned b_hi,
