@@ -18,20 +18,24 @@
 // weights, and where a sum could overflow the kernel multiplies plain fp32 values instead (slow_items).  So it does where the
 // largest products are near the lower end, where k_conv_fma's own rounding of subnormal sums is kept.
 //
-// Roles (20 or 16 warps, one CTA per SM, persistent), as in k_conv_tile but for the drain:
-//   entries     one thread: a slot per (tile, filter offset with a rule), 512 bytes of input rows from the packed table
-//   producers   8 (4) warps, a step each: 128 rows of 192 bytes ([32 h | 32 m] and [32 l]) by 16-byte cp.async
-//   weights     one thread: one bulk copy of [W_h | W_m | W_l] per step
+// Roles (19 or 15 warps, one CTA per SM, persistent), as in k_conv_tile but for the drain:
+//   entries     one thread: a record per item, a slot per (tile, filter offset with a rule), 512 bytes of input rows from the table
+//   producers   8 (4) warps, four to a step: 128 rows of 192 bytes ([32 h | 32 m] and [32 l]) by 16-byte cp.async; the first
+//               lane of a step's warps orders its [W_h | W_m | W_l], one bulk copy
 //   MMA         two warps; up to 64 output planes three instructions per 16 input planes, h (W_h | W_m | W_l), m (W_h | W_m), l W_h, into
 //               three column ranges; above that six into one: the drain waits for what it reads beside the tensor core's own
 //               traffic, 1 100 cycles per step of 96 planes with two ranges, more than the step's 700 of instructions
 //   drain       8 warps, a row and half of the planes per lane: TMEM -> registers after every step, and after the tile's
 //               last one through shared memory -> bias -> optional BatchNorm -> 16-byte stores, four lanes per row
-// Bound by the copies into shared memory, 24 KB of rows and 6 (32 output planes) to 24 KB (128) of weights per step at about
-// 32 bytes per cycle and SM, against 336 to 768 cycles of tensor work; as multiply-adds the same step is 1 024 to 4 096 cycles
-// of the whole FMA pipe.  Rows split once per call, not once per gather: with fp32 rows (16 KB per step) split by the
-// producers on their way through registers a step took twice as long (32 -> 32 planes on 200 k rows 157 us against 88 when both
-// forms were there, 96 -> 96 682 against 309; 85 and 281 since).
+// Bound by shared memory from 96 planes on: a step of 96 planes writes 42 KB of rows and weights and its instructions read 84 KB,
+// 1 008 cycles of 128 bytes (1 070 measured); below that by the way from an instruction through the drain back to its
+// accumulator (64 planes, two accumulators of three ranges: 1 030 cycles where shared memory takes 672; 32 planes 880, 528).  As
+// multiply-adds the same step is 1 024 to 4 096 cycles of the whole FMA pipe.  That way is why the barriers of the next step
+// are looked at while this one is under way and why the loads of a row's stores come before its branches: with a wait, a look at the
+// abort flag and a role for the weights in every step, 200 k rows: 32 -> 32 planes 103 us, 92 now; 64 -> 64 229, 207; 96 -> 96
+// 373, 325; 128 -> 128 527, 455; a Deconvolution 128 -> 96 to 43 k rows 28, 17.  (Three loads of 16 columns under one wait
+// do not fit the registers of 64 planes: 216.)  Rows split once per call, not once per gather: with fp32 rows (16 KB per step) split
+// by the producers on their way through registers a step took twice as long.
 //
 // Every wait is bounded; on expiry the role raises the abort flag, everybody leaves, tensor memory is freed and
 // the host sees FLAG_TC_TIMEOUT through scn_md_poll_errors.
@@ -49,7 +53,7 @@ namespace {
 
 constexpr int kRows = kOrderTile;
 constexpr int kDrainWarps = 8, kMmaWarps = 2;
-constexpr int kSlots = 8;  // offsets the entries run ahead; at least the producing warps (the slots that end the work)
+constexpr int kSlots = 8;  // offsets the entries run ahead; even, so that a producing warp comes by every slot or every second
 constexpr int kMaxStages = 12;
 constexpr int kEpiBytes = 32 * 64;   // per drain warp: 32 rows x 16 planes on their way from lanes to whole lines
 constexpr int kScale = 24;           // of rows and of weights, as a power of two
@@ -74,7 +78,7 @@ struct SixParams {
   int K, n_slices, log2_terms;  // log2_terms: of the products of a sum, rounded up
   int n_stages;
   long long n_tiles, n_items;
-  int n_split;
+  int n_split, per_tile;  // parts of a tile's offsets; items of a tile (parts x column blocks)
   // for slow_items: the operands as they are
   const float *in, *in_b, *weight, *pre_scale, *pre_shift;
   float pre_leak;
@@ -84,25 +88,28 @@ struct SixParams {
 };
 
 // Warps by role.  With 64 planes per drain lane (and weights that leave room for four stages) fewer producers, for
-// 128 registers a thread.  (Two producing warps per step there: 96 -> 96 planes on 200 k rows 331 us, 288 with one.)
+// 128 registers a thread.
 template <int NA>
 struct SixWarps {
-  static constexpr int PROD = NA == 64 ? 4 : 8;
-  static constexpr int DRAIN0 = PROD, MMA = DRAIN0 + kDrainWarps, WGT = MMA + kMmaWarps, ENTRIES = WGT + 1, THREADS = (ENTRIES + 1) * 32;
+  static constexpr int PROD = NA == 64 ? 4 : 8, GROUPS = PROD / kStepWarps;
+  static constexpr int DRAIN0 = PROD, MMA = DRAIN0 + kDrainWarps, ENTRIES = MMA + kMmaWarps, THREADS = (ENTRIES < 15 ? 16 : ENTRIES + 1) * 32;  // (slow_items has 512 threads)
 };
 
 template <int SP>
 struct SixShape {
   static constexpr unsigned HM = SP * 4, L = SP * 2;  // bytes of a row of a stage: [h | m], and [l]
   static constexpr unsigned A_BYTES = kRows * (HM + L);
-  static constexpr int PIECES = HM / 16, NI = kRows / (32 / PIECES);  // 16-byte pieces per row, rows per lane
-  static constexpr int L_PIECES = L / 16, L_NI = kRows / (32 / L_PIECES);
+  static constexpr int PIECES = HM / 16, NI = 32 / (32 / PIECES);  // 16-byte pieces per row, rows per lane (a warp has 32 rows)
+  static constexpr int L_PIECES = L / 16, L_NI = 32 / (32 / L_PIECES);
+  static_assert(NI == 2 * L_NI, "a lane's rows for [l] are half of those for [h | m]");
   static_assert(HM == 128 || HM == 64, "swizzled rows");
 };
 
 struct Ctl {
   unsigned long long full[kMaxStages], empty[kMaxStages];  // rows and weights landed; MMAs done
   unsigned long long s_full[kSlots], s_empty[kSlots], acc_full[4], acc_empty[4];
+  unsigned long long r_full[kRecords], r_empty[kRecords];
+  ItemRecord record[kRecords];  // part: the item within its tile
   int slot_k[kSlots];  // filter offset + (column block << 10); -1: no more work; + kNoRules: offset 0 with rows of zeros
   unsigned tmem, range[2];
   int abort;
@@ -116,15 +123,6 @@ __device__ __forceinline__ Item item_at(const SixParams &P, long long item) {
   const int per = P.n_split * P.n_cb, rest = (int)(item % per);
   const long long i = item / per;
   return Item{P.by_work ? (long long)__ldg(P.by_work + i) : P.n_tiles - 1 - i, rest / P.n_cb, rest % P.n_cb};
-}
-
-// filter offsets of an item: those of its tile, or its share of them when the offsets are divided
-__device__ __forceinline__ int item_offsets(const SixParams &P, long long item) {
-  if (item >= P.n_items) return 0;
-  const Item I = item_at(P, item);
-  int total = 0;
-  for (int w = 0; w < P.words; ++w) total += __popc(__ldg(P.tile_bits + I.tile * P.words + w));
-  return total * (I.part + 1) / P.n_split - total * I.part / P.n_split;
 }
 
 // Where a row of an item's result goes.
@@ -332,7 +330,7 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
   SCN_GRID_WAIT();
   using Shape = SixShape<SP>;
   using Warps = SixWarps<NA>;
-  constexpr int kProdWarps = Warps::PROD, kDrain0 = Warps::DRAIN0, kMma = Warps::MMA, kWgt = Warps::WGT, kEntries = Warps::ENTRIES;
+  constexpr int kProdWarps = Warps::PROD, kDrain0 = Warps::DRAIN0, kMma = Warps::MMA, kEntries = Warps::ENTRIES, kProdGroups = Warps::GROUPS;
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const unsigned w_part = (unsigned)P.cb * SP * 2, w_bytes = w_part * 3;
@@ -351,12 +349,16 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
   if (tid < 2) C.range[tid] = 0;
   if (tid == 0) {
     for (int i = 0; i < P.n_stages; ++i) {
-      mbar_init(&C.full[i], 32 + 1);  // the producing warp's lanes and the weights
+      mbar_init(&C.full[i], kStepWarps * 32 + 1);  // the lanes of the producing warps, and the weights
       mbar_init(&C.empty[i], kMmaWarps);
     }
     for (int i = 0; i < kSlots; ++i) {
       mbar_init(&C.s_full[i], 1);
-      mbar_init(&C.s_empty[i], P.n_slices + 1);    // a producer warp per slice, and the weights
+      mbar_init(&C.s_empty[i], kStepWarps * min(P.n_slices, kProdGroups));  // the producing warps that come by
+    }
+    for (int i = 0; i < kRecords; ++i) {
+      mbar_init(&C.r_full[i], 1);
+      mbar_init(&C.r_empty[i], kDrainWarps + kMmaWarps);
     }
     for (int i = 0; i < 4; ++i) {
       mbar_init(&C.acc_full[i], 1);
@@ -386,113 +388,92 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
   }
   if (warp < kProdWarps) {
     // ==================================== producers =============================================
-    // this lane's 16-byte piece of the rows q NI .. q NI + NI - 1, for [h | m] and again for [l]
+    // Group g of four warps takes the steps g, g + kProdGroups, ...; a warp copies 32 rows of a step, a lane one 16-byte piece of
+    // [h | m] of the rows q NI .. q NI + NI - 1 of them and one of [l] of half of these.  The input rows of the next step are in
+    // registers before its stage is free.
     const int j = lane % Shape::PIECES, q = lane / Shape::PIECES, lj = lane % Shape::L_PIECES, lq = lane / Shape::L_PIECES;
-    const int hm_row = q * Shape::NI, l_row = lq * Shape::L_NI;
-    const unsigned hm_dst = (unsigned)hm_row * Shape::HM + (unsigned)j * 16;
-    const unsigned l_dst = kRows * Shape::HM + (unsigned)l_row * Shape::L + (unsigned)lj * 16;
-    // No more warps than stages: a warp at step n has seen the consumption of step n - active - n_stages, and its wait
-    // below can tell step n - n_stages from the one a round earlier only if that one is not later than this.
-    const int active = min(kProdWarps, P.n_stages);
-    const int d_slot = active / P.n_slices, d_slice = active % P.n_slices;
-    const int d_round = active / P.n_stages, d_st = active % P.n_stages;
-    int slot = warp / P.n_slices, slice = warp % P.n_slices;
-    int round = warp / P.n_stages, st = warp % P.n_stages;
-    bool ok = true, bad = false;
-    while (warp < active) {
-      const int si = slot % kSlots;
-      if (!mbar_wait(&C.s_full[si], (slot / kSlots) & 1)) {
-        ok = false;
-        break;
-      }
-      const int slot_k = C.slot_k[si];
-      if (slot_k < 0 || *abort) break;
-      const int rows_in = slot_k >= kNoRules ? 0 : (int)P.n_in;  // entries below it are rows
-      const int4 *ent = reinterpret_cast<const int4 *>(entries + si * kRows + hm_row);
-      const int4 *l_ent = reinterpret_cast<const int4 *>(entries + si * kRows + l_row);
-      if (!mbar_wait(&C.empty[st], (round + 1) & 1)) {  // (the first round passes)
-        ok = false;
-        break;
-      }
-      const unsigned stage = smem0 + (unsigned)st * stage_bytes;
-      const unsigned char *col = P.in_split + slice * (SP * 6);
-#pragma unroll
-      for (int i = 0; i < Shape::NI; i += 4) {
-        const int4 e4 = ent[i / 4];
-        const int v[4] = {e4.x, e4.y, e4.z, e4.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const bool hit = (unsigned)v[e] < (unsigned)rows_in;
-          bad |= v[e] >= (int)P.n_in && slot_k < kNoRules;
-          const unsigned swizzle = (Shape::HM == 128 ? (i + e) & 7 : ((i + e) >> 1) & 3) * 16;  // (hm_row is a multiple of eight)
-          cp_async16(((stage + hm_dst) ^ swizzle) + (i + e) * Shape::HM, col + j * 16 + (size_t)(unsigned)(hit ? v[e] : 0) * P.row_bytes, hit ? 16u : 0u);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < Shape::L_NI; i += 4) {
-        const int4 e4 = l_ent[i / 4];
-        const int v[4] = {e4.x, e4.y, e4.z, e4.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const bool hit = (unsigned)v[e] < (unsigned)rows_in;
-          const unsigned swizzle = (Shape::L == 64 ? ((i + e) >> 1) & 3 : ((i + e) >> 2) & 1) * 16;
-          cp_async16(((stage + l_dst) ^ swizzle) + (i + e) * Shape::L, col + SP * 4 + lj * 16 + (size_t)(unsigned)(hit ? v[e] : 0) * P.row_bytes, hit ? 16u : 0u);
-        }
-      }
-      cp_async_arrive(&C.full[st]);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&C.s_empty[si]);
-      slot += d_slot, slice += d_slice;
-      if (slice >= P.n_slices) slice -= P.n_slices, ++slot;
-      round += d_round, st += d_st;
-      if (st >= P.n_stages) st -= P.n_stages, ++round;
-    }
-    if (bad) atomicOr(P.flags, FLAG_BAD_ROW);
-    asm volatile("cp.async.wait_all;" ::: "memory");  // they must land before the CTA's shared memory goes away
-    if (!ok) *abort = 1;
-  } else if (warp == kWgt) {
-    // ==================================== weights ===============================================
-    if (lane == 0) {
-      int st = 0, par = 1;
-      long long filled = 0;
-      bool ok = true;
-      for (int slot = 0; ok; ++slot) {
+    const int group = warp / kStepWarps, row0 = warp % kStepWarps * 32 + q * Shape::NI, l_row0 = warp % kStepWarps * 32 + lq * Shape::L_NI;
+    // (where a 16-byte chunk c of row r goes: rows_desc; rows of 128 bytes come in eights, of 64 in fours, of 32 in twos)
+    const unsigned hm_dst = smem0 + (unsigned)row0 * Shape::HM + (unsigned)((Shape::HM == 128 ? j : j ^ (q & 1) * 2) * 16);
+    const unsigned l_dst = smem0 + kRows * Shape::HM + (unsigned)l_row0 * Shape::L +
+                           (unsigned)((Shape::L == 64 ? lj ^ (lq & 1) * 2 : lj ^ (lq >> 1 & 1)) * 16);
+    const int d_slot = kProdGroups / P.n_slices, d_slice = kProdGroups % P.n_slices;
+    int slot = group / P.n_slices, slice = group % P.n_slices, st = group, par = 1;  // (n_stages is at least kProdGroups)
+    const bool brings_weights = warp % kStepWarps == 0 && lane == 0;
+    int slot_k = 0, filled = 0;
+    bool ok = true, bad = false, fresh = true;
+    int rows[Shape::NI];
+    for (;;) {
+      if (fresh) {
         const int si = slot % kSlots;
+        // (A warp comes by every slot, or by every second one with one slice: it has seen the slot kSlots before this one
+        // filled, so the parity cannot be that of an earlier round.)
         if (!mbar_wait(&C.s_full[si], (slot / kSlots) & 1)) {
           ok = false;
           break;
         }
-        const int slot_k = C.slot_k[si];
-        mbar_arrive(&C.s_empty[si]);
-        if (slot_k < 0) break;
+        slot_k = C.slot_k[si];
+        if (slot_k < 0 || *abort) break;
+        const int *ent = entries + si * kRows + row0;
+#pragma unroll
+        for (int i = 0; i < Shape::NI; i += 4) {
+          const int4 e4 = *reinterpret_cast<const int4 *>(ent + i);
+          rows[i] = e4.x, rows[i + 1] = e4.y, rows[i + 2] = e4.z, rows[i + 3] = e4.w;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&C.s_empty[si]);
+#pragma unroll
+        for (int i = 0; i < Shape::NI; ++i) {
+          if (slot_k >= kNoRules) rows[i] = -1;
+          bad |= rows[i] >= (int)P.n_in;
+        }
+      }
+      if (!mbar_wait(&C.empty[st], par)) {  // (the first round passes)
+        ok = false;
+        break;
+      }
+      const unsigned at = (unsigned)st * stage_bytes;
+      if (brings_weights && !(P.drop && blockIdx.x == 0 && group == 0 && filled == 0)) {
         const int k = slot_k & 1023, block = slot_k >> 10 & 1;
-        const unsigned char *src = P.wprep + (size_t)(k * P.n_cb + block) * P.n_slices * w_bytes;
-        for (int s = 0; s < P.n_slices; ++s) {
-          if (!mbar_wait(&C.empty[st], par) || *abort) {
-            ok = false;
-            break;
-          }
-          if (!(P.drop && blockIdx.x == 0 && filled == 0)) {
-            mbar_expect_tx(&C.full[st], w_bytes);
-            bulk_copy_g2s(smem0 + (unsigned)st * stage_bytes + Shape::A_BYTES, src + (size_t)s * w_bytes, w_bytes, &C.full[st]);
-          }
-          ++filled;
-          if (++st == P.n_stages) st = 0, par ^= 1;
-        }
+        mbar_expect_tx(&C.full[st], w_bytes);
+        bulk_copy_g2s(smem0 + at + Shape::A_BYTES, P.wprep + ((size_t)(k * P.n_cb + block) * P.n_slices + slice) * w_bytes, w_bytes, &C.full[st]);
       }
-      if (!ok) {  // slabs in flight must land before the CTA's shared memory goes away
-        *abort = 1;
-        for (int i = 0; i < P.n_stages; ++i) {
-          const long long uses = (filled + P.n_stages - 1 - i) / P.n_stages;
-          if (uses > 0) mbar_wait(&C.full[i], (unsigned)((uses - 1) & 1));
-        }
+      ++filled;
+      const unsigned char *col = P.in_split + slice * (SP * 6) + j * 16, *l_col = P.in_split + slice * (SP * 6) + SP * 4 + lj * 16;
+#pragma unroll
+      for (int i = 0; i < Shape::NI; ++i) {
+        const bool hit = (unsigned)rows[i] < (unsigned)P.n_in;
+        const unsigned swizzle = (Shape::HM == 128 ? i & 7 : i >> 1 & 3) * 16;
+        cp_async16(((hm_dst + at) ^ swizzle) + i * Shape::HM, col + (size_t)(unsigned)(hit ? rows[i] : 0) * P.row_bytes, hit ? 16u : 0u);
       }
+#pragma unroll
+      for (int i = 0; i < Shape::L_NI; ++i) {
+        const int row = lq & 1 ? rows[Shape::L_NI + i] : rows[i];
+        const bool hit = (unsigned)row < (unsigned)P.n_in;
+        const unsigned swizzle = (Shape::L == 64 ? i >> 1 & 3 : i >> 2 & 1) * 16;
+        cp_async16(((l_dst + at) ^ swizzle) + i * Shape::L, l_col + (size_t)(unsigned)(hit ? row : 0) * P.row_bytes, hit ? 16u : 0u);
+      }
+      cp_async_arrive(&C.full[st]);
+      slot += d_slot, slice += d_slice;
+      fresh = d_slot > 0;
+      if (slice >= P.n_slices) slice -= P.n_slices, ++slot, fresh = true;
+      st += kProdGroups;
+      if (st >= P.n_stages) st -= P.n_stages, par ^= 1;
+    }
+    if (bad) atomicOr(P.flags, FLAG_BAD_ROW);
+    asm volatile("cp.async.wait_all;" ::: "memory");  // they must land before the CTA's shared memory goes away
+    if (!ok) {
+      *abort = 1;
+      if (brings_weights)  // and so must the slabs
+        for (int i = max(0, filled - (P.n_stages + kProdGroups - 1) / kProdGroups); i < filled; ++i) {
+          const int n = group + i * kProdGroups;
+          mbar_wait(&C.full[n % P.n_stages], (n / P.n_stages) & 1);
+        }
     }
   } else if (warp < kMma + kMmaWarps && warp >= kMma) {
     // ==================================== MMA issue =============================================
     // Two warps take the accumulators in turn: what one spends on barriers passes while the other's instructions run (U-Net
-    // of two rooms 2 985 -> 2 950 us).  The whole warp runs the loop and one elected lane issues: with warp-uniform control
-    // flow and operands the descriptors stay in uniform registers.
+    // of two rooms 2 985 -> 2 950 us).  The whole warp runs the loop and one elected lane issues, by a predicate (mma_bf16_if).
     const unsigned id1 = tile_idesc(P.cb), id2 = tile_idesc(kJoint ? 2 * P.cb : 16), id3 = tile_idesc(kJoint ? 3 * P.cb : 16);
     const unsigned long long a_desc = rows_desc<Shape::HM>(smem0, 0), l_desc = rows_desc<Shape::L>(smem0, kRows * Shape::HM);
     const unsigned long long w_desc = smem_desc(smem0 + Shape::A_BYTES, 128, SP / 8 * 128);
@@ -501,72 +482,77 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
     const unsigned stage_step = stage_bytes >> 4, wm_step = w_part >> 4;
     const int items = (int)my_items, n_stages = P.n_stages, cb = P.cb;
     int st = 0, par = 0, buf = 0, buf_par = 1;
-    unsigned at = 0, d = tmem;
+    unsigned d = tmem;
     bool ok = true;
-    const bool leader = elect_one();
+    const unsigned lead = elect_one() ? 1u : 0u;
     bool mine = warp == kMma;  // the next accumulator is this warp's
-    int offsets_next = item_offsets(P, item_of(0));
+    bool ready = false, acc_ready = false;  // the stage and the accumulator at hand, looked at a step earlier
     for (int i = 0; i < items && ok; ++i) {
-      const int steps = __reduce_max_sync(0xffffffffu, max(1, offsets_next)) * P.n_slices;
-      offsets_next = item_offsets(P, item_of(i + 1));
+      const int ri = i % kRecords;
+      if (!mbar_wait_warp(&C.r_full[ri], (i / kRecords) & 1)) {
+        ok = false;
+        break;
+      }
+      const int steps = __reduce_max_sync(0xffffffffu, C.record[ri].steps);
+      if (lead) mbar_arrive(&C.r_empty[ri]);
       for (int s = 0; s < steps; ++s) {
         const bool opens = s % kGroup == 0, closes = s % kGroup == kGroup - 1 || s == steps - 1;
         // the accumulator must have been drained
-        if (opens && mine && (!mbar_wait_warp(&C.acc_empty[buf], buf_par) || __any_sync(0xffffffffu, *abort != 0))) {
+        if (opens && mine && !acc_ready && (__any_sync(0xffffffffu, *abort != 0) || !mbar_wait_warp(&C.acc_empty[buf], buf_par))) {
           ok = false;
           break;
         }
-        if (!mbar_wait_warp(&C.full[st], par)) {
+        if (!ready && !mbar_wait_warp(&C.full[st], par)) {
           ok = false;
           break;
         }
+        const int st1 = st + 1 == n_stages ? 0 : st + 1, par1 = st1 ? par : par ^ 1;
+        const int buf1 = !closes ? buf : buf + 1 == n_acc ? 0 : buf + 1, buf_par1 = closes && buf1 == 0 ? buf_par ^ 1 : buf_par;
+        const unsigned seen = mbar_test(&C.full[st1], par1), acc_seen = mbar_test(&C.acc_empty[buf1], buf_par1);
         // (the other warp's steps too, and a stage goes when both have been here: neither can fall a round behind, or run a round
         // ahead, where a phase's parity is that of another)
         if (!mine) {
-          if (leader) mbar_arrive(&C.empty[st]);
-        } else if (leader) {
+          if (lead) mbar_arrive(&C.empty[st]);
+        } else {
           // order the copied rows (acquired through the barrier) before the tensor core's async-proxy reads
           fence_proxy_async_smem();
           tc_fence_after();
+          const unsigned at = (unsigned)st * stage_step;
           if (kJoint) {
 #pragma unroll
             for (int jj = 0; jj < SP / 16; ++jj) {
               const unsigned ah = a0 + at + jj * 2, am = ah + SP / 8, al = l0 + at + jj * 2, wh = w0 + at + jj * 16;
-              if (jj == 0) mma_bf16(d, ah, a_hi, wh, w_hi, id3, opens ? 0u : 1u);
-              else mma_bf16_acc(d, ah, a_hi, wh, w_hi, id3);
-              mma_bf16_acc(d + cb, am, a_hi, wh, w_hi, id2);
-              mma_bf16_acc(d + 2 * cb, al, l_hi, wh, w_hi, id1);
+              if (jj == 0) mma_bf16_if(lead, d, ah, a_hi, wh, w_hi, id3, opens ? 0u : 1u);
+              else mma_bf16_acc_if(lead, d, ah, a_hi, wh, w_hi, id3);
+              mma_bf16_acc_if(lead, d + cb, am, a_hi, wh, w_hi, id2);
+              mma_bf16_acc_if(lead, d + 2 * cb, al, l_hi, wh, w_hi, id1);
             }
           } else {
             const unsigned wm = wm_step, wl = 2 * wm_step;
 #pragma unroll
             for (int jj = 0; jj < SP / 16; ++jj) {  // 2^-16 of a product, 2^-8, then the large ones
               const unsigned ah = a0 + at + jj * 2, am = ah + SP / 8, al = l0 + at + jj * 2, wh = w0 + at + jj * 16;
-              if (jj == 0) mma_bf16(d, al, l_hi, wh, w_hi, id1, 0u);
-              else mma_bf16_acc(d, al, l_hi, wh, w_hi, id1);
-              mma_bf16_acc(d, ah, a_hi, wh + wl, w_hi, id1);
-              mma_bf16_acc(d, am, a_hi, wh + wm, w_hi, id1);
+              if (jj == 0) mma_bf16_if(lead, d, al, l_hi, wh, w_hi, id1, 0u);
+              else mma_bf16_acc_if(lead, d, al, l_hi, wh, w_hi, id1);
+              mma_bf16_acc_if(lead, d, ah, a_hi, wh + wl, w_hi, id1);
+              mma_bf16_acc_if(lead, d, am, a_hi, wh + wm, w_hi, id1);
             }
 #pragma unroll
             for (int jj = 0; jj < SP / 16; ++jj) {
               const unsigned ah = a0 + at + jj * 2, am = ah + SP / 8, wh = w0 + at + jj * 16;
-              mma_bf16_acc(d, am, a_hi, wh, w_hi, id1);
-              mma_bf16_acc(d, ah, a_hi, wh + wm, w_hi, id1);
+              mma_bf16_acc_if(lead, d, am, a_hi, wh, w_hi, id1);
+              mma_bf16_acc_if(lead, d, ah, a_hi, wh + wm, w_hi, id1);
             }
 #pragma unroll
-            for (int jj = 0; jj < SP / 16; ++jj) mma_bf16_acc(d, a0 + at + jj * 2, a_hi, w0 + at + jj * 16, w_hi, id1);
+            for (int jj = 0; jj < SP / 16; ++jj) mma_bf16_acc_if(lead, d, a0 + at + jj * 2, a_hi, w0 + at + jj * 16, w_hi, id1);
           }
-          tc_commit(&C.empty[st]);
-          if (closes) tc_commit(&C.acc_full[buf]);
+          tc_commit_if(lead, &C.empty[st]);
+          if (closes) tc_commit_if(lead, &C.acc_full[buf]);
         }
-        __syncwarp();
-        at += stage_step;
-        if (++st == n_stages) st = 0, par ^= 1, at = 0;
-        if (closes) {
-          mine = !mine;
-          d += dcols;
-          if (++buf == n_acc) buf = 0, buf_par ^= 1, d = tmem;
-        }
+        st = st1, par = par1;
+        ready = __all_sync(0xffffffffu, seen != 0), acc_ready = __all_sync(0xffffffffu, acc_seen != 0);
+        if (closes) mine = !mine;
+        buf = buf1, buf_par = buf_par1, d = tmem + (unsigned)(buf * dcols);
       }
     }
     if (!ok) *abort = 1;
@@ -575,21 +561,31 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
     if (lane == 0) {
       int slot = 0;
       bool ok = true;
+      Tiles<SixParams> tiles(P);
       for (long long it = 0; it < my_items && ok; ++it) {
-        const Item I = item_at(P, item_of(it));
         unsigned u[4];
 #pragma unroll
-        for (int w = 0; w < 4; ++w) u[w] = w < P.words ? __ldg(P.tile_bits + I.tile * P.words + w) : 0u;
-        const int *src = P.packed + I.tile * P.K * kRows;
+        for (int w = 0; w < 4; ++w) u[w] = tiles.mask[w];
+        const int tile = tiles.tile, within = P.per_tile == 1 ? 0 : (int)item_of(it) % P.per_tile, part = within / P.n_cb, block = within - part * P.n_cb;
+        const int *src = P.packed + (long long)tile * P.K * kRows;
+        tiles.advance(P, it);
+        int offsets = __popc(u[0]) + __popc(u[1]) + __popc(u[2]) + __popc(u[3]);
         if (P.n_split > 1) {
-          const int total = __popc(u[0]) + __popc(u[1]) + __popc(u[2]) + __popc(u[3]);
-          const int first = total * I.part / P.n_split;
-          keep_range(u, first, total * (I.part + 1) / P.n_split);
+          const int first = offsets * part / P.n_split, last = offsets * (part + 1) / P.n_split;
+          keep_range(u, first, last);
           src += first * kRows;
+          offsets = last - first;
         }
         // a tile (or part) without any rule still gets one step, of weights and rows of zeros
-        const bool none = (u[0] | u[1] | u[2] | u[3]) == 0;
+        const bool none = offsets == 0;
         if (none) u[0] = 1u;
+        const int ri = (int)it % kRecords;
+        if (!mbar_wait(&C.r_empty[ri], (((int)it / kRecords) + 1) & 1)) {
+          ok = false;
+          break;
+        }
+        C.record[ri] = ItemRecord{max(1, offsets) * P.n_slices, tile, within, tiles.tile};
+        mbar_arrive(&C.r_full[ri]);
 #pragma unroll 1
         for (int w = 0; w < 4 && ok; ++w) {
           unsigned m = u[0];
@@ -600,7 +596,7 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
               ok = false;
               break;
             }
-            C.slot_k[si] = (none ? kNoRules : w * 32 + __ffs(m) - 1) + (I.block << 10);
+            C.slot_k[si] = (none ? kNoRules : w * 32 + __ffs(m) - 1) + (block << 10);
             if (none) {
               mbar_arrive(&C.s_full[si]);
             } else {
@@ -611,8 +607,8 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
         }
       }
       const int filled = slot;
-      // every producer warp finds its next step in a slot that ends it
-      const int ends = (min(kProdWarps, P.n_stages) - 1) / P.n_slices + 1;
+      // every producing warp finds its next step in a slot that ends it
+      const int ends = (kProdGroups - 1) / P.n_slices + 1;
       for (int i = 0; i < ends && ok; ++i, ++slot) {
         const int si = slot % kSlots;
         if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1)) {
@@ -630,7 +626,7 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
         }
       }
     }
-  } else {
+  } else if (warp < kMma) {
     // ==================================== drain =================================================
     const int quad = warp & 3, half = (warp - kDrain0) >> 2;
     const int units = P.cb / 16, first_unit = half ? (units + 1) / 2 : 0, my_units = half ? units / 2 : (units + 1) / 2;
@@ -639,18 +635,26 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
     const int nc = P.cout, cb = P.cb;
     int buf = 0, buf_par = 0;
     bool ok = true;
-    int offsets_next = item_offsets(P, item_of(0));
-    for (long long it = 0; it < my_items && ok; ++it) {
-      const long long item = item_of(it);
-      const Item I = item_at(P, item);
-      const int orow = __ldg(P.order + I.tile * kRows + quad * 32 + lane);
-      const int groups = (__reduce_max_sync(0xffffffffu, max(1, offsets_next)) * P.n_slices + kGroup - 1) / kGroup;
-      offsets_next = item_offsets(P, item_of(it + 1));
+    int next_orow = 0;  // this lane's row of the next item: asked for an item ahead
+    bool ready = false;  // the accumulator at hand, looked at while the one before it was read
+    for (int it = 0; it < (int)my_items && ok; ++it) {
+      const int ri = it % kRecords;
+      if (!mbar_wait_warp(&C.r_full[ri], (it / kRecords) & 1)) {
+        ok = false;
+        break;
+      }
+      const ItemRecord R = C.record[ri];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&C.r_empty[ri]);
+      const int groups = (__reduce_max_sync(0xffffffffu, R.steps) + kGroup - 1) / kGroup;
+      const Item I{R.tile, R.part / P.n_cb, R.part % P.n_cb};
+      const int orow = it ? next_orow : __ldg(P.order + I.tile * kRows + quad * 32 + lane);
+      next_orow = __ldg(P.order + (long long)R.next_tile * kRows + quad * 32 + lane);
       float acc[NA];
 #pragma unroll
       for (int e = 0; e < NA; ++e) acc[e] = 0.f;
       for (int s = 0; s < groups; ++s) {
-        if (!mbar_wait_warp(&C.acc_full[buf], buf_par) || __any_sync(0xffffffffu, *abort != 0)) {
+        if (!ready && (__any_sync(0xffffffffu, *abort != 0) || !mbar_wait_warp(&C.acc_full[buf], buf_par))) {
           ok = false;
           break;
         }
@@ -683,12 +687,16 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
         __syncwarp();
         if (lane == 0) mbar_arrive(&C.acc_empty[buf]);
         if (++buf == n_acc) buf = 0, buf_par ^= 1;
+        ready = __all_sync(0xffffffffu, mbar_test(&C.acc_full[buf], buf_par) != 0);
       }
       if (!ok) break;
       // where rows lane / 4, + 8, + 16, + 24 of the warp go
       int to[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) to[i] = __shfl_sync(0xffffffffu, orow, i * 8 + (lane >> 2));
+      for (int i = 0; i < 4; ++i) {
+        to[i] = __shfl_sync(0xffffffffu, orow, i * 8 + (lane >> 2));
+        if (P.n_split > 1 && to[i] >= 0) to[i] = (I.part * (int)P.n_tiles + R.tile) * kRows + quad * 32 + i * 8 + (lane >> 2);
+      }
 #pragma unroll
       for (int u = 0; u < NA / 16; ++u)
         if (u < my_units) {
@@ -698,13 +706,29 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
           __syncwarp();
           const int c = I.block * cb + (first_unit + u) * 16 + (lane & 3) * 4;
           if (c < nc) {
+            const bool finish = P.n_split == 1;
+            float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), sc = bias, sh = bias, v[4];
+            if (finish && P.bias) bias = __ldg(reinterpret_cast<const float4 *>(P.bias + c));
+            if (finish && P.bn_scale) {
+              sc = make_float4(__ldg(P.bn_scale + c), __ldg(P.bn_scale + c + 1), __ldg(P.bn_scale + c + 2), __ldg(P.bn_scale + c + 3));
+              sh = make_float4(__ldg(P.bn_shift + c), __ldg(P.bn_shift + c + 1), __ldg(P.bn_shift + c + 2), __ldg(P.bn_shift + c + 3));
+            }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const int row = i * 8 + (lane >> 2);
-              float4 v = my_epi[row * 4 + ((lane & 3) ^ ((row >> 1) & 3))];
-              if (to[i] < 0) continue;
-              v.x = finished(P, v.x, c), v.y = finished(P, v.y, c + 1), v.z = finished(P, v.z, c + 2), v.w = finished(P, v.w, c + 3);
-              *reinterpret_cast<float4 *>(result_row(P, I, quad * 32 + row, to[i]) + c) = v;
+              v[i] = my_epi[row * 4 + ((lane & 3) ^ ((row >> 1) & 3))];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float *y = &v[i].x;
+              if (finish && P.bias) v[i].x += bias.x, v[i].y += bias.y, v[i].z += bias.z, v[i].w += bias.w;
+              if (finish && P.bn_scale) {  // separate multiply and add, as the stand-alone BatchNorm kernel rounds them
+                v[i].x = __fadd_rn(__fmul_rn(v[i].x, sc.x), sh.x), v[i].y = __fadd_rn(__fmul_rn(v[i].y, sc.y), sh.y);
+                v[i].z = __fadd_rn(__fmul_rn(v[i].z, sc.z), sh.z), v[i].w = __fadd_rn(__fmul_rn(v[i].w, sc.w), sh.w);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) y[e] *= y[e] > 0.f ? 1.f : P.leak;
+              }
+              if (to[i] >= 0) *reinterpret_cast<float4 *>(P.out + to[i] * (long long)nc + c) = v[i];
             }
           }
           __syncwarp();
@@ -822,7 +846,8 @@ int launch_six(SixParams &P, int n_sm, int dev, cudaStream_t stream) {
   static_assert(SixWarps<NA>::THREADS >= kFmaGroups * kFmaGroup, "slow_items");
   SCN_REQUIRE((size_t)P.n_stages * stage + fixed - sizeof(Ctl) >= sizeof(float) * kFmaGroups * kFmaShare, SCN_ERR_UNSUPPORTED,
               "k_conv_six: %d stages of %zu bytes", P.n_stages, stage);
-  P.n_items = P.n_tiles * P.n_split * P.n_cb;
+  P.per_tile = P.n_split * P.n_cb;
+  P.n_items = P.n_tiles * P.per_tile;
   SCN_LAUNCH(kernel, (unsigned)std::min<long long>(P.n_items, (long long)n_sm), SixWarps<NA>::THREADS, kSmemBudget, stream, P);
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
@@ -849,33 +874,39 @@ extern thread_local int g_drop_arrival;  // test hook (conv_tc.cu)
 
 // Which fp32 convolutions run here instead of on k_conv_fma (which is left for few output planes on many rows, whose
 // multiply-adds cost less than six bytes per input value and rule, and for little work, where its one launch is the shorter
-// chain).  One layer, us on this kernel / on k_conv_fma.  27 offsets, submanifold, rows scattered over a surface; the error of
-// each against float64 (2-norm, products of mixed sign):
-//                 16->16    16->32    24->32    32->32     64->64      96->96      160->160      error (96->96)
-//   600 rows      -         -         14.3/11.9 13.7/12.3  16.0/12.5   19.2/15.4   22.1/25.9     0.8e-7 / 2.0e-7
-//   1 000         14.6/11.2 14.1/11.6 14.1/12.1 14.3/13.1  16.6/14.3   20.0/24.3   24.1/47.2     0.9e-7 / 2.6e-7
-//   2 000         14.6/11.7 15.3/12.4 15.3/13.4 14.6/14.4  17.9/26.1   23.3/50.9   37.1/101.3    0.9e-7 / 3.4e-7
-//   9 000         -         21.2/19.8 19.2/22.3 19.2/25.3  28.8/59.5   42.7/123    92.9/329      1.0e-7 / 3.5e-7
-//   30 000        21/29     22/38     25/45     25/52      46/122      66/250      164/719       1.1e-7 / 5.3e-7
-//   200 000       63/57     66/80     83/100    85/118     180/370     281/932     709/2 622     1.2e-7 / 5.4e-7
-//   1 600 000     446/403   434/591   584/727   589/856
-// The same on sphere shells, whose rows are closer together (k_conv_fma packs rows from 2 048 on):
-//                 32->32     64->64     64->96     96->96     128->128
-//   500 rows      13.5/11.0  16.2/13.3  17.8/15.6  18.8/19.2  21.0/22.5
-//   1 000         13.6/12.1  16.8/17.4  18.4/23.6  19.9/31.2  21.4/38.2
-//   2 000         13.7/9.3   16.2/14.6  18.5/17.3  19.0/22.1  22.5/31.9
-//   3 000         14.7/18.0  19.2/34.4  21.6/40.6  24.7/55.7  30.8/82.0
-// Other filters:
+// chain).  One layer, us of its launches on this kernel / on k_conv_fma.  27 offsets, submanifold, sphere shells; the error of each
+// against float64 (2-norm, products of mixed sign):
+//                 16->16     16->32     32->32     64->64     96->96     160->160       error (96->96)
+//   600 rows      13.1/10.4  13.1/10.7  14.2/11.6  16.1/16.0  18.4/24.7  21.2/46.1      0.8e-7 / 2.0e-7
+//   1 000         13.3/10.6  13.4/11.2  13.7/12.5  16.1/18.0  18.9/31.8  23.8/62.4      0.9e-7 / 2.6e-7
+//   2 000         13.7/11.9  13.7/12.6  14.1/14.6  16.8/26.6  22.3/53.2  36.2/110       0.9e-7 / 3.4e-7
+//   9 000         16.3/14.9  17.4/18.7  18.4/23.4  29.1/60.6  41.5/127   92.0/327       1.0e-7 / 3.5e-7
+//   30 000        20.3/32.3  21.4/42.5  26.4/59.5  53.6/141   81.8/317   222/859        1.1e-7 / 5.3e-7
+//   200 000       72/97      78/135     102/200    231/603    359/1 549  1 005/4 178    1.2e-7 / 5.4e-7
+// Other filters (measured when this kernel took 10 to 18 % longer up to 64 planes):
 //   3-D shapes, 99 000 rows, 27 offsets: 8->16 45/42, 16->16 45/51, 32->16 57/67, 16->32 45/63
 //   2-D strokes, 91 000 rows, 9 offsets: 16->16 28/21, 32->16 33/27, 16->32 28/26, 24->32 34/31, 32->32 34/37
 //   2-D, 25 offsets, 31 500 rows: 16->32 26/37, 32->32 29/51, 64->64 56/129; 4-D, 81 offsets, 60 000 rows: 32->32 76/221
 //   3 / 2, 27 offsets, 26 700 rows: 16->32 22/30, 32->32 27/40, 64->64 52/99, 128->128 115/361
-// Windows side by side (filter = stride), where a fine row has one rule and K * rows * planes says less about the work (2 / 2; 2^4 offsets alike):
-//   Convolution   32->48   64->64    96->64    64->96    96->96    128->128     Deconvolution  64->64    64->128  96->96   128->96  128->128  160->128
-//   1 800 rows    14/10    15/11     17/15     17/15     18/20     22/24        6 000 rows     12/11     15/11    14/12    15/15    17/16     17/18
-//   5 800         15/18    19/24     23/31     21/25     24/33     28/52        20 000         18/13     24/17    22/18    24/22    27/27     28/33
-//   60 000        35/38    57/67     76/97     65/97     83/138    112/182      60 000         29/29     41/40    39/42    41/51    48/67     50/79
-//   150 000       79/70    124/118   168/165   137/197   182/278   246/399      200 000        70/58     107/108  96/121   103/152  124/178   133/213
+// Windows side by side (filter = stride), where a fine row has one rule (2 / 2; fine rows; a Convolution's coarse rows):
+//   Deconvolution 32->16     32->32     48->32     64->32     64->48     96->48     64->64     96->96     128->128
+//   4 000 rows                                                                      10.6/10.4  11.3/9.8   12.5/15.1
+//   15 000                                                                          11.0/11.0  12.0/14.7  13.7/21.3
+//   25 000        10.5/5.2   10.8/7.4   11.9/8.9   11.8/9.7   12.8/13.3  14.6/17.1  13.7/13.5
+//   100 000       15.9/10.4  16.8/16.3  20.0/19.5  20.3/22.0  23.4/31.4  27.6/42.3  25.0/31.6
+//   200 000       22.2/15.7  23.4/24.6  28.8/30.2  30.7/34.3  36.2/55.3  44.7/73.6  39.1/56.0
+//   400 000                             52/58      55/67                            71/113     97/242     134/341
+//   1 600 000     119/116    141/189    175/220    193/244    230/410    299/535    243/412
+//   error         0.5/1.0e-7 0.5/1.0e-7 0.5/1.3e-7 0.5/1.4e-7 0.5/1.4e-7 0.6/1.8e-7 0.5/1.4e-7
+//   Convolution   32->48     32->64     64->64     96->64     64->96     96->96     128->128
+//   1 500 rows    12.4/9.9              14.8/11.8  16.1/14.6  15.1/13.1  17.1/16.3  17.7/22.0
+//   4 000         12.7/18.2             16.2/19.2  18.4/31.8  17.1/21.8  19.7/30.1  23.4/47.3
+//   16 000        16.5/23.2             22.3/31.7  28.1/43.7  23.8/46.5  30.2/62.9  38.4/90.3
+//   54 000        25.5/38.1  28.1/39.8  50.3/61.3
+//   118 000       49/54                 87/95      124/132    91/159     129/224    177/321
+//   463 000       165/191    173/192    307/321
+// (The lines for windows side by side were drawn when this kernel took 10 to 40 % longer on them: every one of them that comes
+// here gains, and Deconvolutions of 70 M multiply-adds, or Convolutions to 64 planes on more rows, would.)
 // Its error is the smaller one, or the same, for every shape and table that comes here, 8 to 256 planes, products of mixed
 // and of one sign, rows behind a ReLU (16->32 on 9 000 rows of one sign, where k_conv_fma's sums are in parts: 6.5e-8 and
 // 6.1e-8, so not here).
@@ -921,7 +952,7 @@ int conv_forward_six(const float *in, long long n_in, float *out, long long n_ou
   const double chunk = cb <= 64 ? std::max(56.0, 1.5 * cb) + std::max(56.0, 1.0 * cb) + 56 : 6 * std::max(56.0, 0.5 * cb);
   const double step = std::max((kRows * SP * 6.0 + cb * SP * 6.0) / 32.0, chunk * SP / 16);
   const char *e = getenv("SCN_SIX_SPLIT");
-  const int n_split = e ? std::max(1, std::min(atoi(e), 64)) : split_parts(ord.n_tiles, n_cb, ord.one_offset ? 1 : K, n_slices, step, cout, n_sm);
+  const int n_split = e ? (int)std::max<long long>(1, std::min<long long>({atoi(e), 64, (1ll << 31) / (ord.n_tiles * kRows) - 1})) : split_parts(ord.n_tiles, n_cb, ord.one_offset ? 1 : K, n_slices, step, cout, n_sm);
   if (tmp.get(&image, image_bytes + sizeof(unsigned) * kRangeWords) != SCN_OK ||  // (multiples of 16)
       tmp.get(&rows, rows_bytes + sizeof(unsigned) * kRangeWords) != SCN_OK ||
       (n_split > 1 && tmp.get(&partial, (size_t)n_split * ord.n_tiles * kRows * cout * sizeof(float)) != SCN_OK)) {

@@ -59,12 +59,11 @@ namespace scn {
 namespace {
 
 constexpr int kRows = kOrderTile;  // rows of a tile = MMA M
-constexpr int kProdWarps = 8, kStepWarps = 4, kProdGroups = kProdWarps / kStepWarps;
+constexpr int kProdWarps = 8, kProdGroups = kProdWarps / kStepWarps;
 constexpr int kEpi0 = kProdWarps, kMma = kProdWarps + 4, kEntries = kMma + 1;
 constexpr int kThreads = (kProdWarps + 6) * 32;
 constexpr int kSlots = 8;       // offsets the entries run ahead; even, so that a producing warp comes by every slot or every second
 constexpr int kMaxStages = 12;
-constexpr int kRecords = 4;     // items the entries run ahead of the epilogue
 constexpr int kEpiBytes = 32 * 64;  // per epilogue warp: 32 rows x 16 planes on their way from TMEM lanes to whole lines
 
 struct TileParams {
@@ -83,7 +82,7 @@ struct TileParams {
   int K, n_slices;
   int n_stages, tmem_cols;
   long long n_tiles, n_items;
-  int n_split;
+  int n_split, per_tile;      // parts of a tile's offsets; items of a tile (the same)
   unsigned char *out_split;  // (optional, n_split 1) the result once more as split rows, slices of out_sp planes
   int out_sp;
   int drop;         // test hook: leave out one barrier arrival of the first CTA
@@ -105,43 +104,10 @@ struct Ctl {
   unsigned long long full[kMaxStages], empty[kMaxStages];  // rows and weights landed; MMAs done
   unsigned long long s_full[kSlots], s_empty[kSlots], acc_full[4], acc_empty[4];
   unsigned long long r_full[kRecords], r_empty[kRecords];
-  struct Record {
-    int steps, tile, part, next_tile;  // of an item; the tile of the item behind it
-  } record[kRecords];
+  ItemRecord record[kRecords];
   int slot_k[kSlots];  // filter offset of the slot; -1: no more work; kNoRules: offset 0 with rows of zeros
   unsigned tmem;
   int abort;
-};
-
-// The tile of an item: the tiles with the most offsets first (packed tiles come in ascending order of their masks, so from
-// the back where they have not been sorted by work).  Past the last item any tile.
-__device__ __forceinline__ int item_tile(const TileParams &P, long long item) {
-  if (item >= P.n_items) return 0;
-  const int i = P.n_split == 1 ? (int)item : (int)item / P.n_split;
-  return P.by_work ? __ldg(P.by_work + i) : (int)P.n_tiles - 1 - i;
-}
-
-// The tiles of a CTA's items in turn: the tile of an item is asked for three items ahead and its mask of offsets one ahead, so
-// that neither trip to memory is waited for between two tiles.
-struct Tiles {
-  int tile, next, next2;
-  unsigned mask[4], next_mask[4];
-  __device__ __forceinline__ void fetch(const TileParams &P, int t, unsigned (&m)[4]) {
-#pragma unroll
-    for (int w = 0; w < 4; ++w) m[w] = w < P.words ? __ldg(P.tile_bits + (long long)t * P.words + w) : 0u;
-  }
-  __device__ __forceinline__ explicit Tiles(const TileParams &P) {
-    tile = item_tile(P, item_of(0)), next = item_tile(P, item_of(1)), next2 = item_tile(P, item_of(2));
-    fetch(P, tile, mask);
-    fetch(P, next, next_mask);
-  }
-  // from item `it` to the one behind it
-  __device__ __forceinline__ void advance(const TileParams &P, long long it) {
-    tile = next, next = next2, next2 = item_tile(P, item_of(it + 3));
-#pragma unroll
-    for (int w = 0; w < 4; ++w) mask[w] = next_mask[w];
-    fetch(P, next, next_mask);
-  }
 };
 
 template <int TERMS, int SP, bool OUT_SPLIT>
@@ -260,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     if (!ok) {
       *abort = 1;
       if (brings_weights)  // and so must the slabs
-        for (int i = max(0, filled - (P.n_stages + 1) / kProdGroups); i < filled; ++i) {
+        for (int i = max(0, filled - (P.n_stages + kProdGroups - 1) / kProdGroups); i < filled; ++i) {
           const int n = group + i * kProdGroups;
           mbar_wait(&C.full[n % P.n_stages], (n / P.n_stages) & 1);
         }
@@ -333,7 +299,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     if (lane == 0) {
       int slot = 0;
       bool ok = true;
-      Tiles tiles(P);
+      Tiles<TileParams> tiles(P);
       for (long long it = 0; it < my_items && ok; ++it) {
         unsigned u[4];
 #pragma unroll
@@ -356,7 +322,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
           ok = false;
           break;
         }
-        C.record[ri] = Ctl::Record{max(1, offsets) * P.n_slices, tile, part, tiles.tile};
+        C.record[ri] = ItemRecord{max(1, offsets) * P.n_slices, tile, part, tiles.tile};
         mbar_arrive(&C.r_full[ri]);
 #pragma unroll 1
         for (int w = 0; w < 4 && ok; ++w) {
@@ -413,7 +379,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
         *abort = 1;
         break;
       }
-      const Ctl::Record R = C.record[ri];
+      const ItemRecord R = C.record[ri];
       __syncwarp();
       if (lane == 0) mbar_arrive(&C.r_empty[ri]);
       const int orow = it ? next_orow : __ldg(P.order + (long long)R.tile * kRows + quad * 32 + lane);
@@ -630,7 +596,8 @@ int launch_tile_as(TileParams &P, int n_sm, int dev, cudaStream_t stream) {
   P.tmem_cols = 512 / ctas;
   P.n_stages = (int)std::min<size_t>(kMaxStages, (smem - fixed) / stage);
   SCN_REQUIRE(P.n_stages >= 2, SCN_ERR_UNSUPPORTED, "tile kernel: %d output planes do not fit shared memory", P.cout);
-  P.n_items = P.n_tiles * P.n_split;
+  P.per_tile = P.n_split;
+  P.n_items = P.n_tiles * P.per_tile;
   SCN_LAUNCH(kernel, (unsigned)std::min<long long>(P.n_items, (long long)n_sm * ctas), kThreads, smem, stream, P);
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;

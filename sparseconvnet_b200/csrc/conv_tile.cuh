@@ -52,4 +52,46 @@ __device__ __forceinline__ long long items_here(long long n_items) {
   const long long full = n_items / gridDim.x;
   return full + (item_of(full) < n_items ? 1 : 0);
 }
+
+constexpr int kStepWarps = 4;  // producing warps of a step: 32 rows each
+constexpr int kRecords = 4;    // items the entries run ahead of the roles that store results
+
+// What the roles behind the entries have to know of an item: its steps, its tile (the last one too, so that the rows of the
+// item behind it can be asked for early), which part of the tile's offsets or which column block it is.
+struct ItemRecord {
+  int steps, tile, part, next_tile;
+};
+
+// The tile of an item: the tiles with the most offsets first (packed tiles come in ascending order of their masks, so from
+// the back where they have not been sorted by work).  Past the last item any tile.
+template <class Params>
+__device__ __forceinline__ int item_tile(const Params &P, long long item) {
+  if (item >= P.n_items) return 0;
+  const int i = P.per_tile == 1 ? (int)item : (int)item / P.per_tile;
+  return P.by_work ? __ldg(P.by_work + i) : (int)P.n_tiles - 1 - i;
+}
+
+// The tiles of a CTA's items in turn: the tile of an item is asked for three items ahead and its mask of offsets one ahead, so
+// that neither trip to memory is waited for between two tiles.
+template <class Params>
+struct Tiles {
+  int tile, next, next2;
+  unsigned mask[4], next_mask[4];
+  __device__ __forceinline__ void fetch(const Params &P, int t, unsigned (&m)[4]) {
+#pragma unroll
+    for (int w = 0; w < 4; ++w) m[w] = w < P.words ? __ldg(P.tile_bits + (long long)t * P.words + w) : 0u;
+  }
+  __device__ __forceinline__ explicit Tiles(const Params &P) {
+    tile = item_tile(P, item_of(0)), next = item_tile(P, item_of(1)), next2 = item_tile(P, item_of(2));
+    fetch(P, tile, mask);
+    fetch(P, next, next_mask);
+  }
+  // from item `it` to the one behind it
+  __device__ __forceinline__ void advance(const Params &P, long long it) {
+    tile = next, next = next2, next2 = item_tile(P, item_of(it + 3));
+#pragma unroll
+    for (int w = 0; w < 4; ++w) mask[w] = next_mask[w];
+    fetch(P, next, next_mask);
+  }
+};
 }  // namespace scn
