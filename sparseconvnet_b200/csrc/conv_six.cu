@@ -561,7 +561,8 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
     if (lane == 0) {
       int slot = 0;
       bool ok = true;
-      Tiles<SixParams> tiles(P);
+      Tiles<SixParams> tiles;
+      tiles.start(P);
       for (long long it = 0; it < my_items && ok; ++it) {
         unsigned u[4];
 #pragma unroll

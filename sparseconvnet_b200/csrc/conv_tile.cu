@@ -39,7 +39,9 @@
 //               cycles from the first copy to the last, during which the stage waits.)
 //   MMA         one warp
 //   epilogue    4 warps: tcgen05.ld (a lane holds a row) -> shared memory, 16 planes at a time -> bias -> optional
-//               BatchNorm scale / shift / leaky ReLU -> 16-byte stores, four lanes per row.  (Stored straight from the TMEM
+//               BatchNorm scale / shift / leaky ReLU -> 16-byte stores, four lanes per row.  A CTA's last item is stored by the
+//               producers as well, a third of the columns for every four warps: 224 planes on 1.4 k rows 19.6 us, 18.2 (with the
+//               entries' first loads made before the CTA is set up).  (Stored straight from the TMEM
 //               lanes every instruction touched 32 lines: a fifth of the cycles in which the gather could have issued.)
 //
 // With fewer tiles than SMs the offsets of a tile are divided over n_split items whose partial sums are added in a
@@ -60,10 +62,12 @@ namespace {
 
 constexpr int kRows = kOrderTile;  // rows of a tile = MMA M
 constexpr int kProdWarps = 8, kProdGroups = kProdWarps / kStepWarps;
-constexpr int kEpi0 = kProdWarps, kMma = kProdWarps + 4, kEntries = kMma + 1;
+constexpr int kMma = kProdWarps + 4, kEntries = kMma + 1;
 constexpr int kThreads = (kProdWarps + 6) * 32;
+constexpr int kStoreSets = 1 + kProdGroups;  // of four warps that store a CTA's last item
 constexpr int kSlots = 8;       // offsets the entries run ahead; even, so that a producing warp comes by every slot or every second
 constexpr int kMaxStages = 12;
+constexpr int kBarriers = 2 * kMaxStages + 2 * kSlots + 8 + 2 * kRecords;
 constexpr int kEpiBytes = 32 * 64;  // per epilogue warp: 32 rows x 16 planes on their way from TMEM lanes to whole lines
 
 struct TileParams {
@@ -105,10 +109,85 @@ struct Ctl {
   unsigned long long s_full[kSlots], s_empty[kSlots], acc_full[4], acc_empty[4];
   unsigned long long r_full[kRecords], r_empty[kRecords];
   ItemRecord record[kRecords];
+  int total_steps;     // of the CTA, when the slots end
   int slot_k[kSlots];  // filter offset of the slot; -1: no more work; kNoRules: offset 0 with rows of zeros
   unsigned tmem;
   int abort;
 };
+
+// Columns first, first + step, ..., 16 at a time, of the 32 rows that lanes of `quad` hold: tensor memory -> shared memory -> bias
+// -> BatchNorm -> the result (and its split form), four lanes per row.  `base`: the accumulator at this quarter of the lanes.
+template <int PARTS, bool OUT_SPLIT>
+__device__ __forceinline__ void store_columns(const TileParams &P, bool joint, unsigned base, const ItemRecord &R, int orow, int quad,
+                                              int lane, float4 *my_epi, int first, int step) {
+  const int nc = P.cout;
+  // where rows lane / 4, + 8, + 16, + 24 of the warp go: rows of the result, or of the partial sums
+  int to[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    to[i] = __shfl_sync(0xffffffffu, orow, i * 8 + (lane >> 2));
+    if (!OUT_SPLIT && P.n_split > 1 && to[i] >= 0) to[i] = (R.part * (int)P.n_tiles + R.tile) * kRows + quad * 32 + i * 8 + (lane >> 2);
+  }
+  for (int c0 = first; c0 < nc; c0 += step) {
+#pragma unroll
+    for (int half = 0; half < 16; half += 8) {
+      unsigned a[8], b[8];
+      tmem_ld8_nowait(base + c0 + half, a);
+      if (joint) tmem_ld8_nowait(base + P.coutp + c0 + half, b);
+      tmem_wait_ld();
+#pragma unroll
+      for (int e = 0; e < 8; e += 4) {
+        float4 v;
+        v.x = __uint_as_float(a[e]), v.y = __uint_as_float(a[e + 1]), v.z = __uint_as_float(a[e + 2]), v.w = __uint_as_float(a[e + 3]);
+        if (joint) {
+          v.x += __uint_as_float(b[e]), v.y += __uint_as_float(b[e + 1]);
+          v.z += __uint_as_float(b[e + 2]), v.w += __uint_as_float(b[e + 3]);
+        }
+        my_epi[lane * 4 + (((half + e) >> 2) ^ ((lane >> 1) & 3))] = v;
+      }
+    }
+    __syncwarp();
+    const int c = c0 + (lane & 3) * 4;
+    if (c < nc) {
+      float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), sc = bias, sh = bias;
+      const bool finish = OUT_SPLIT || P.n_split == 1;
+      if (finish && P.bias) bias = __ldg(reinterpret_cast<const float4 *>(P.bias + c));
+      if (finish && P.bn_scale) {
+        sc = __ldg(reinterpret_cast<const float4 *>(P.bn_scale + c));
+        sh = __ldg(reinterpret_cast<const float4 *>(P.bn_shift + c));
+      }
+      float4 vs[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = i * 8 + (lane >> 2);
+        vs[i] = my_epi[row * 4 + ((lane & 3) ^ ((row >> 1) & 3))];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float4 v = vs[i];
+        if (finish && P.bias) v.x += bias.x, v.y += bias.y, v.z += bias.z, v.w += bias.w;
+        if (finish && P.bn_scale) {  // separate multiply and add, as the stand-alone BatchNorm kernel rounds them
+          v.x = __fadd_rn(__fmul_rn(v.x, sc.x), sh.x), v.y = __fadd_rn(__fmul_rn(v.y, sc.y), sh.y);
+          v.z = __fadd_rn(__fmul_rn(v.z, sc.z), sh.z), v.w = __fadd_rn(__fmul_rn(v.w, sc.w), sh.w);
+          v.x *= v.x > 0.f ? 1.f : P.leak, v.y *= v.y > 0.f ? 1.f : P.leak;
+          v.z *= v.z > 0.f ? 1.f : P.leak, v.w *= v.w > 0.f ? 1.f : P.leak;
+        }
+        if (to[i] < 0) continue;
+        *reinterpret_cast<float4 *>(P.out + (long long)to[i] * nc + c) = v;
+        if (OUT_SPLIT) {
+          uint2 h, m;
+          split_bf16_pair(v.x, v.y, h.x, m.x);
+          split_bf16_pair(v.z, v.w, h.y, m.y);
+          const int slice = c0 & -P.out_sp;  // (16, 32 or 64 planes)
+          unsigned char *q = P.out_split + ((long long)to[i] * nc + slice) * (2 * PARTS) + (c - slice) * 2;
+          *reinterpret_cast<uint2 *>(q) = h;
+          if (PARTS == 2) *reinterpret_cast<uint2 *>(q + P.out_sp * 2) = m;
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
 
 template <int TERMS, int SP, bool OUT_SPLIT>
 __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
@@ -129,26 +208,21 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
   const int dcols = ((joint ? 2 : 1) * P.coutp + 31) & ~31;
   const int n_acc = min(4, P.tmem_cols / dcols);
 
-  if (tid == 0) {
-    for (int i = 0; i < P.n_stages; ++i) {
-      mbar_init(&C.full[i], kStepWarps * 32 + 1);  // the lanes of the producing warps, and the weights
-      mbar_init(&C.empty[i], 1);
-    }
-    for (int i = 0; i < kSlots; ++i) {
-      mbar_init(&C.s_full[i], 1);
-      mbar_init(&C.s_empty[i], kStepWarps * min(P.n_slices, kProdGroups));  // the producing warps that come by
-    }
-    for (int i = 0; i < kRecords; ++i) {
-      mbar_init(&C.r_full[i], 1);
-      mbar_init(&C.r_empty[i], 4 + 1);  // the epilogue's warps and the issuing one
-    }
-    for (int i = 0; i < 4; ++i) {
-      mbar_init(&C.acc_full[i], 1);
-      mbar_init(&C.acc_empty[i], 4);
-    }
-    C.abort = 0;
+  if (tid < kBarriers) {  // a thread per barrier, in the order of Ctl
+    const int i = tid - 2 * kMaxStages, j = i - 2 * kSlots;
+    const unsigned arrivals = tid < kMaxStages ? kStepWarps * 32 + 1  // full: the lanes of the producing warps, and the weights
+                              : i < kSlots     ? 1                    // empty, s_full
+                              : j < 0          ? kStepWarps * min(P.n_slices, kProdGroups)  // s_empty: the producing warps that come by
+                              : j < 4          ? 1                                          // acc_full
+                              : j < 8          ? 4                                          // acc_empty
+                              : j < 8 + kRecords ? 1                                        // r_full
+                                                 : 4 + 1;  // r_empty: the epilogue's warps and the issuing one
+    mbar_init(&C.full[0] + tid, arrivals);
+    if (tid == 0) C.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  Tiles<TileParams> tiles;
+  if (tid == kEntries * 32) tiles.start(P);  // (on its way while tensor memory is had)
   if (warp == kMma) tmem_alloc(&C.tmem, (unsigned)P.tmem_cols);
   tc_fence_before();
   __syncthreads();
@@ -181,7 +255,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
           break;
         }
         slot_k = C.slot_k[si];
-        if (slot_k < 0 || *abort) break;
+        if (slot_k < 0) break;
+        if (*abort) {
+          ok = false;
+          break;
+        }
         const int4 *ent = reinterpret_cast<const int4 *>(entries + si * kRows + row0);
 #pragma unroll
         for (int i = 0; i < NI; i += 4) {
@@ -230,6 +308,23 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
           const int n = group + i * kProdGroups;
           mbar_wait(&C.full[n % P.n_stages], (n / P.n_stages) & 1);
         }
+    } else if (!*abort) {
+      // The CTA's last item: these warps store two thirds of its columns, through the ring, which nothing reads any more when
+      // the last step has been consumed.  (The step before it first, whose parity cannot be an earlier round's: this
+      // warp has seen the consumption of the one n_stages before either.)
+      const int last = (int)my_items - 1, n = C.total_steps, quad = warp & 3;
+      const ItemRecord R = C.record[last % kRecords];
+      const int orow = __ldg(P.order + (long long)R.tile * kRows + quad * 32 + lane);
+      if ((n < 2 || mbar_wait(&C.empty[(n - 2) % P.n_stages], ((n - 2) / P.n_stages) & 1)) &&
+          mbar_wait(&C.empty[(n - 1) % P.n_stages], ((n - 1) / P.n_stages) & 1)) {
+        __syncwarp();
+        tc_fence_after();
+        store_columns<PARTS, OUT_SPLIT>(P, joint, tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(last % n_acc * dcols), R, orow, quad,
+                                        lane, reinterpret_cast<float4 *>(smem + warp * kEpiBytes), 16 * (1 + group), 16 * kStoreSets);
+        tc_fence_before();
+      } else {
+        *abort = 1;
+      }
     }
   } else if (warp == kMma) {
     // ==================================== MMA issue =============================================
@@ -299,7 +394,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     if (lane == 0) {
       int slot = 0;
       bool ok = true;
-      Tiles<TileParams> tiles(P);
       for (long long it = 0; it < my_items && ok; ++it) {
         unsigned u[4];
 #pragma unroll
@@ -347,6 +441,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
       const int filled = slot;
       // every producing warp finds its next step in a slot that ends it
       const int ends = (kProdGroups - 1) / P.n_slices + 1;
+      C.total_steps = filled * P.n_slices;
       for (int i = 0; i < ends && ok; ++i, ++slot) {
         const int si = slot % kSlots;
         if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1)) {
@@ -367,7 +462,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
   } else {
     // ==================================== epilogue ==============================================
     const int quad = warp & 3;
-    const int nc = P.cout;
     float4 *my_epi = reinterpret_cast<float4 *>(epi + quad * kEpiBytes);
     int buf = 0, buf_par = 0;
     int next_orow = 0;  // this lane's row of the next item: asked for an item ahead
@@ -391,73 +485,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
         break;
       }
       tc_fence_after();
-      const unsigned base = tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(buf * dcols);
-      // where rows lane / 4, + 8, + 16, + 24 of the warp go: rows of the result, or of the partial sums
-      int to[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        to[i] = __shfl_sync(0xffffffffu, orow, i * 8 + (lane >> 2));
-        if (!OUT_SPLIT && P.n_split > 1 && to[i] >= 0) to[i] = (R.part * (int)P.n_tiles + R.tile) * kRows + quad * 32 + i * 8 + (lane >> 2);
-      }
-      for (int c0 = 0; c0 < nc; c0 += 16) {
-#pragma unroll
-        for (int half = 0; half < 16; half += 8) {
-          unsigned a[8], b[8];
-          tmem_ld8_nowait(base + c0 + half, a);
-          if (joint) tmem_ld8_nowait(base + P.coutp + c0 + half, b);
-          tmem_wait_ld();
-#pragma unroll
-          for (int e = 0; e < 8; e += 4) {
-            float4 v;
-            v.x = __uint_as_float(a[e]), v.y = __uint_as_float(a[e + 1]), v.z = __uint_as_float(a[e + 2]), v.w = __uint_as_float(a[e + 3]);
-            if (joint) {
-              v.x += __uint_as_float(b[e]), v.y += __uint_as_float(b[e + 1]);
-              v.z += __uint_as_float(b[e + 2]), v.w += __uint_as_float(b[e + 3]);
-            }
-            my_epi[lane * 4 + (((half + e) >> 2) ^ ((lane >> 1) & 3))] = v;
-          }
-        }
-        __syncwarp();
-        const int c = c0 + (lane & 3) * 4;
-        if (c < nc) {
-          float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), sc = bias, sh = bias;
-          const bool finish = OUT_SPLIT || P.n_split == 1;
-          if (finish && P.bias) bias = __ldg(reinterpret_cast<const float4 *>(P.bias + c));
-          if (finish && P.bn_scale) {
-            sc = __ldg(reinterpret_cast<const float4 *>(P.bn_scale + c));
-            sh = __ldg(reinterpret_cast<const float4 *>(P.bn_shift + c));
-          }
-          float4 vs[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int row = i * 8 + (lane >> 2);
-            vs[i] = my_epi[row * 4 + ((lane & 3) ^ ((row >> 1) & 3))];
-          }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            float4 v = vs[i];
-            if (finish && P.bias) v.x += bias.x, v.y += bias.y, v.z += bias.z, v.w += bias.w;
-            if (finish && P.bn_scale) {  // separate multiply and add, as the stand-alone BatchNorm kernel rounds them
-              v.x = __fadd_rn(__fmul_rn(v.x, sc.x), sh.x), v.y = __fadd_rn(__fmul_rn(v.y, sc.y), sh.y);
-              v.z = __fadd_rn(__fmul_rn(v.z, sc.z), sh.z), v.w = __fadd_rn(__fmul_rn(v.w, sc.w), sh.w);
-              v.x *= v.x > 0.f ? 1.f : P.leak, v.y *= v.y > 0.f ? 1.f : P.leak;
-              v.z *= v.z > 0.f ? 1.f : P.leak, v.w *= v.w > 0.f ? 1.f : P.leak;
-            }
-            if (to[i] < 0) continue;
-            *reinterpret_cast<float4 *>(P.out + (long long)to[i] * nc + c) = v;
-            if (OUT_SPLIT) {
-              uint2 h, m;
-              split_bf16_pair(v.x, v.y, h.x, m.x);
-              split_bf16_pair(v.z, v.w, h.y, m.y);
-              const int slice = c0 & -P.out_sp;  // (16, 32 or 64 planes)
-              unsigned char *q = P.out_split + ((long long)to[i] * nc + slice) * (2 * PARTS) + (c - slice) * 2;
-              *reinterpret_cast<uint2 *>(q) = h;
-              if (PARTS == 2) *reinterpret_cast<uint2 *>(q + P.out_sp * 2) = m;
-            }
-          }
-        }
-        __syncwarp();
-      }
+      store_columns<PARTS, OUT_SPLIT>(P, joint, tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(buf * dcols), R, orow, quad, lane, my_epi,
+                                      0, it == (int)my_items - 1 ? 16 * kStoreSets : 16);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&C.acc_empty[buf]);

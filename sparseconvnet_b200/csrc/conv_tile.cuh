@@ -81,7 +81,7 @@ struct Tiles {
 #pragma unroll
     for (int w = 0; w < 4; ++w) m[w] = w < P.words ? __ldg(P.tile_bits + (long long)t * P.words + w) : 0u;
   }
-  __device__ __forceinline__ explicit Tiles(const Params &P) {
+  __device__ __forceinline__ void start(const Params &P) {
     tile = item_tile(P, item_of(0)), next = item_tile(P, item_of(1)), next2 = item_tile(P, item_of(2));
     fetch(P, tile, mask);
     fetch(P, next, next_mask);
