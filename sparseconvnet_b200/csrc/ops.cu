@@ -61,10 +61,11 @@ __global__ void k_output_features(const float *__restrict__ in, float *__restric
 // BatchNorm + leaky ReLU (CPU/BatchNormalization.cpp:12-62)
 // ------------------------------------------------------------------------------------------
 
-// per-plane sum and sum of squares; grid.x tiles planes by 32, grid.y splits the rows
+// per-plane sum and sum of squares; grid.x tiles planes by 32, grid.y splits the rows in chunks, whose sums are added in a
+// fixed order (bn_total)
 __global__ void __launch_bounds__(256)
 k_bn_stats(const float *__restrict__ in, long long n_rows, int C, long long in_stride,
-           double *__restrict__ sums /* [2][C] */) {
+           double *__restrict__ partial /* [2][C][chunks] */) {
   SCN_GRID_WAIT();
   __shared__ float sh_s[8][33], sh_q[8][33];
   int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
@@ -85,15 +86,16 @@ k_bn_stats(const float *__restrict__ in, long long n_rows, int C, long long in_s
       ds += sh_s[j][lane];
       dq += sh_q[j][lane];
     }
-    atomicAdd(&sums[c], ds);
-    atomicAdd(&sums[C + c], dq);
+    partial[(long long)c * gridDim.y + blockIdx.y] = ds;
+    partial[(long long)(C + c) * gridDim.y + blockIdx.y] = dq;
   }
 }
 
-// The same for rows of whole 16-byte pieces: eight lanes per row and 32 planes, 32 rows per pass of the block, two passes
-// in flight.  Bound by HBM: the 14 layers of a U-Net training step on 400 k points 165 us (198 with one value per load).
+// The same for rows of whole 16-byte pieces: eight lanes per row and 32 planes, 32 rows per pass of the block, four passes
+// in flight.  Bound by HBM.  (With the blocks' sums added by atomics, up to 1 184 of them to the same 64 doubles, and two passes
+// in flight, 400 k rows of 32 planes took 16.5 us, 12.6 now, and the 14 layers of a U-Net training step 162 us with their memsets, 120.)
 __global__ void __launch_bounds__(256)
-k_bn_stats4(const float *__restrict__ in, int n_rows, int C, int in_stride, double *__restrict__ sums /* [2][C] */) {
+k_bn_stats4(const float *__restrict__ in, int n_rows, int C, int in_stride, double *__restrict__ partial /* [2][C][chunks] */) {
   SCN_GRID_WAIT();
   __shared__ float sh[2][8][33];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
@@ -108,12 +110,15 @@ k_bn_stats4(const float *__restrict__ in, int n_rows, int C, int in_stride, doub
       s[0] += v.x, s[1] += v.y, s[2] += v.z, s[3] += v.w;
       z[0] += v.x * v.x, z[1] += v.y * v.y, z[2] += v.z * v.z, z[3] += v.w * v.w;
     };
-    for (; r < n_rows - step; r += 2 * step, p += 2 * hop) {
-      const float4 a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p + hop));
+    auto ld = [](const float *q) { return __ldg(reinterpret_cast<const float4 *>(q)); };
+    for (; r < n_rows - 3ll * step; r += 4 * step, p += 4 * hop) {
+      const float4 a = ld(p), b = ld(p + hop), d = ld(p + 2 * hop), e = ld(p + 3 * hop);
       add(a);
       add(b);
+      add(d);
+      add(e);
     }
-    if (r < n_rows) add(__ldg(reinterpret_cast<const float4 *>(p)));
+    for (; r < n_rows; r += step, p += hop) add(ld(p));
   }
 #pragma unroll
   for (int e = 0; e < 4; ++e) {  // the four rows of a warp
@@ -133,38 +138,70 @@ k_bn_stats4(const float *__restrict__ in, int n_rows, int C, int in_stride, doub
     double t = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) t += sh[wy][j][lane];
-    atomicAdd(&sums[wy * C + col], t);
+    partial[(long long)(wy * C + col) * gridDim.y + blockIdx.y] = t;
   }
 }
 
-static void launch_bn_stats(const float *in, long long n_rows, int C, long long in_stride, double *sums, cudaStream_t stream) {
+static int launch_bn_stats(const float *in, long long n_rows, int C, long long in_stride, Scratch &tmp, double **partial, int *chunks,
+                           cudaStream_t stream) {
   const unsigned gx = (unsigned)ceil_div(C, 32);
-  if (C % 4 == 0 && in_stride % 4 == 0 && (uintptr_t)in % 16 == 0 && n_rows < (1 << 30) && in_stride < (1 << 20)) {
-    const unsigned gy = (unsigned)std::max<long long>(1, std::min<long long>(ceil_div(n_rows, 64), 148 * 8 / gx));
-    SCN_LAUNCH(k_bn_stats4, dim3(gx, gy), 256, 0, stream, in, (int)n_rows, C, (int)in_stride, sums);
-  } else {
-    const unsigned gy = (unsigned)std::min<long long>(ceil_div(n_rows, 64), 1024);
-    SCN_LAUNCH(k_bn_stats, dim3(gx, gy), 256, 0, stream, in, n_rows, C, in_stride, sums);
+  const bool pieces = C % 4 == 0 && in_stride % 4 == 0 && (uintptr_t)in % 16 == 0 && n_rows < (1 << 30) && in_stride < (1 << 20);
+  const unsigned gy = (unsigned)std::max<long long>(1, std::min<long long>(ceil_div(n_rows, 64), pieces ? 148 * 8 / gx : 1024));
+  SCN_TRY(tmp.get(partial, sizeof(double) * 2 * (size_t)C * gy));
+  *chunks = (int)gy;
+  if (pieces)
+    SCN_LAUNCH(k_bn_stats4, dim3(gx, gy), 256, 0, stream, in, (int)n_rows, C, (int)in_stride, *partial);
+  else
+    SCN_LAUNCH(k_bn_stats, dim3(gx, gy), 256, 0, stream, in, n_rows, C, in_stride, *partial);
+  return SCN_OK;
+}
+
+// The chunk sums of plane c, added by one warp in a fixed order (lane l takes chunks l, l + 32, ..., then the lanes); eight
+// loads of each on their way.  (One at a time, the chunks of a plane 2 C doubles apart: 11 to 14 us for 1 024 chunks, 4 now.)
+__device__ __forceinline__ void bn_total(const double *__restrict__ partial /* [2][C][chunks] */, int chunks, int C, int c, double &s,
+                                         double &q) {
+  const int lane = threadIdx.x & 31;
+  const double *ps = partial + (long long)c * chunks, *pq = partial + (long long)(C + c) * chunks;
+  s = q = 0.0;
+  for (int i = lane; i < chunks; i += 256) {
+    double a[8], b[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const bool here = i + e * 32 < chunks;
+      a[e] = here ? __ldg(ps + i + e * 32) : 0.0;
+      b[e] = here ? __ldg(pq + i + e * 32) : 0.0;
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s += a[e], q += b[e];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    q += __shfl_xor_sync(0xffffffffu, q, o);
   }
 }
 
 // Turns either running statistics (eval) or batch sums (train) into saveMean / saveInvStd and
 // updates the running statistics in training mode: momentum weighs the OLD value, the
-// normalising variance is biased, the running variance unbiased (CPU/BatchNormalization.cpp:32-46).
-__global__ void k_bn_finalize(int C, long long n_rows, const double *__restrict__ sums,
-                              float *save_mean, float *save_invstd, float *running_mean,
-                              float *running_var, float eps, float momentum, int train,
-                              int count_follows_sums) {
+// normalising variance is biased, the running variance unbiased (CPU/BatchNormalization.cpp:32-46).  One warp per plane.
+__global__ void __launch_bounds__(256)
+k_bn_finalize(int C, long long n_rows, const double *__restrict__ partial /* [2][C][chunks] */, int chunks,
+              float *save_mean, float *save_invstd, float *running_mean,
+              float *running_var, float eps, float momentum, int train,
+              int count_follows_sums) {
   SCN_GRID_WAIT();
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (c >= C) return;
   if (count_follows_sums) {  // the row count of all devices, summed along with the array
-    n_rows = (long long)sums[2 * C];
+    n_rows = (long long)partial[2 * C];
     if (n_rows == 0) return;
   }
+  double sum = 0.0, squares = 0.0;
+  if (train) bn_total(partial, chunks, C, c, sum, squares);
+  if ((threadIdx.x & 31) != 0) return;
   if (train) {
-    double mean = sums[c] / (double)n_rows;
-    double ss = sums[C + c] - mean * mean * (double)n_rows;
+    double mean = sum / (double)n_rows;
+    double ss = squares - mean * mean * (double)n_rows;
     save_mean[c] = (float)mean;
     running_mean[c] = momentum * running_mean[c] + (1 - momentum) * (float)mean;
     running_var[c] = momentum * running_var[c] + (1 - momentum) * (float)(ss / (double)(n_rows - 1));
@@ -242,7 +279,7 @@ __global__ void __launch_bounds__(256)
 k_bn_back_sums(const float *__restrict__ in, const float *__restrict__ out, const float *__restrict__ d_out,
                long long n_rows, int C, long long in_stride, long long out_stride,
                const float *__restrict__ mean, float leak, long long chunk_rows,
-               double *__restrict__ partial /* [chunks][2][C] */) {
+               double *__restrict__ partial /* [2][C][chunks] */) {
   SCN_GRID_WAIT();
   __shared__ double sh_s[8][33], sh_q[8][33];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
@@ -284,8 +321,8 @@ k_bn_back_sums(const float *__restrict__ in, const float *__restrict__ out, cons
       ts += sh_s[i][lane];
       tq += sh_q[i][lane];
     }
-    partial[((long long)blockIdx.y * 2 + 0) * C + c] = ts;
-    partial[((long long)blockIdx.y * 2 + 1) * C + c] = tq;
+    partial[(long long)c * gridDim.y + blockIdx.y] = ts;
+    partial[(long long)(C + c) * gridDim.y + blockIdx.y] = tq;
   }
 }
 
@@ -294,7 +331,7 @@ k_bn_back_sums(const float *__restrict__ in, const float *__restrict__ out, cons
 __global__ void __launch_bounds__(256)
 k_bn_back_sums4(const float *__restrict__ in, const float *__restrict__ out, const float *__restrict__ d_out, int n_rows, int C,
                 int in_stride, int out_stride, const float *__restrict__ mean, float leak, int chunk_rows,
-                double *__restrict__ partial /* [chunks][2][C] */) {
+                double *__restrict__ partial /* [2][C][chunks] */) {
   SCN_GRID_WAIT();
   __shared__ double sh[2][8][33];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
@@ -344,7 +381,7 @@ k_bn_back_sums4(const float *__restrict__ in, const float *__restrict__ out, con
     double t = 0.0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) t += sh[wy][i][lane];
-    partial[((long long)blockIdx.y * 2 + wy) * C + col] = t;
+    partial[(long long)(wy * C + col) * gridDim.y + blockIdx.y] = t;
   }
 }
 
@@ -359,21 +396,6 @@ static void launch_bn_back_sums(const float *in, const float *out, const float *
     SCN_LAUNCH(k_bn_back_sums, grid, 256, 0, stream, in, out, d_out, n_rows, C, in_stride, out_stride, mean, leak, chunk_rows, partial);
 }
 
-// the chunk sums of plane c, added by one warp in a fixed order (lane l takes chunks l, l + 32, ..., then the lanes)
-__device__ __forceinline__ void bn_back_total(const double *__restrict__ partial, int chunks, int C, int c, double &s, double &q) {
-  const int lane = threadIdx.x & 31;
-  s = q = 0.0;
-  for (int i = lane; i < chunks; i += 32) {
-    s += partial[((long long)i * 2 + 0) * C + c];
-    q += partial[((long long)i * 2 + 1) * C + c];
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s += __shfl_xor_sync(0xffffffffu, s, o);
-    q += __shfl_xor_sync(0xffffffffu, q, o);
-  }
-}
-
 // one warp per plane (a thread per plane that walked up to 1024 chunks on its own took 57 us, as long as the passes over
 // the rows)
 __global__ void __launch_bounds__(256)
@@ -384,7 +406,7 @@ k_bn_back_finalize(const double *__restrict__ partial, int chunks, int C, long l
   const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (c >= C) return;
   double s, q;
-  bn_back_total(partial, chunks, C, c, s, q);
+  bn_total(partial, chunks, C, c, s, q);
   if ((threadIdx.x & 31) != 0) return;
   const float is = invstd[c];
   if (d_bias) d_bias[c] = (float)s;
@@ -401,7 +423,7 @@ k_bn_back_reduce(const double *__restrict__ partial, int chunks, int C, double *
   const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (c >= C) return;
   double s, q;
-  bn_back_total(partial, chunks, C, c, s, q);
+  bn_total(partial, chunks, C, c, s, q);
   if ((threadIdx.x & 31) != 0) return;
   sums[c] = s;
   sums[C + c] = q;
@@ -768,14 +790,13 @@ int scn_batchnorm_forward(const float *in_features, float *out_features, int64_t
   SCN_REQUIRE(in_stride >= n_planes && out_stride >= n_planes, SCN_ERR_BAD_ARG, "row stride below n_planes");
   if (n_rows == 0) return SCN_OK;
   SCN_REQUIRE(in_features && out_features, SCN_ERR_BAD_ARG, "null features");
-  double *sums = nullptr;
+  Scratch tmp(stream);
   if (train) {
-    SCN_TRY(device_alloc((void **)&sums, sizeof(double) * 2 * n_planes, stream));
-    SCN_CUDA_CHECK(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * n_planes, stream));
-    launch_bn_stats(in_features, n_rows, n_planes, in_stride, sums, stream);
+    double *partial = nullptr;
+    int chunks = 0;
+    SCN_TRY(launch_bn_stats(in_features, n_rows, n_planes, in_stride, tmp, &partial, &chunks, stream));
+    SCN_LAUNCH(k_bn_finalize, (unsigned)ceil_div(n_planes, 8), 256, 0, stream, n_planes, n_rows, partial, chunks, save_mean, save_invstd, running_mean, running_var, (float)eps, (float)momentum, train, 0);
   }
-  if (train)
-    SCN_LAUNCH(k_bn_finalize, (unsigned)ceil_div(n_planes, 128), 128, 0, stream, n_planes, n_rows, sums, save_mean, save_invstd, running_mean, running_var, (float)eps, (float)momentum, train, 0);
   const float *rm = train ? nullptr : running_mean, *rv = train ? nullptr : running_var;
   bool vec4 = (n_planes % 4 == 0) && (in_stride % 4 == 0) && (out_stride % 4 == 0) &&
               ((uintptr_t)in_features % 16 == 0) && ((uintptr_t)out_features % 16 == 0);
@@ -787,7 +808,6 @@ int scn_batchnorm_forward(const float *in_features, float *out_features, int64_t
   else
     SCN_LAUNCH(k_bn_apply<1>, blocks, 256, smem, stream, in_features, out_features, n_rows, n_planes, in_stride, out_stride, save_mean, save_invstd, rm, rv, (float)eps, weight, bias, (float)leakiness);
   SCN_CUDA_CHECK(cudaGetLastError());
-  if (sums) SCN_TRY(device_free(sums, stream));
   return SCN_OK;
 }
 
@@ -933,10 +953,16 @@ int scn_batchnorm_moments(const float *in_features, int64_t n_rows, int n_planes
   SCN_REQUIRE(n_planes >= 1 && n_planes <= 4096, SCN_ERR_UNSUPPORTED, "n_planes %d unsupported", n_planes);
   SCN_REQUIRE(sums && n_rows >= 0, SCN_ERR_BAD_ARG, "null sums or negative row count");
   SCN_REQUIRE(in_stride >= n_planes, SCN_ERR_BAD_ARG, "row stride below n_planes");
-  SCN_CUDA_CHECK(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * n_planes, stream));
-  if (n_rows == 0) return SCN_OK;
+  if (n_rows == 0) {
+    SCN_CUDA_CHECK(cudaMemsetAsync(sums, 0, sizeof(double) * 2 * n_planes, stream));
+    return SCN_OK;
+  }
   SCN_REQUIRE(in_features, SCN_ERR_BAD_ARG, "null features");
-  launch_bn_stats(in_features, n_rows, n_planes, in_stride, sums, stream);
+  Scratch tmp(stream);
+  double *partial = nullptr;
+  int chunks = 0;
+  SCN_TRY(launch_bn_stats(in_features, n_rows, n_planes, in_stride, tmp, &partial, &chunks, stream));
+  SCN_LAUNCH(k_bn_back_reduce, (unsigned)ceil_div(n_planes, 8), 256, 0, stream, partial, chunks, n_planes, sums);
   SCN_CUDA_CHECK(cudaGetLastError());
   return SCN_OK;
 }
@@ -953,7 +979,7 @@ int scn_batchnorm_forward_moments(const float *in_features, float *out_features,
   SCN_REQUIRE(n_rows >= 0 && (n_rows_total < 0 || n_rows_total >= n_rows), SCN_ERR_BAD_ARG,
               "total row count below this device's");
   if (n_rows_total == 0) return SCN_OK;
-  SCN_LAUNCH(k_bn_finalize, (unsigned)ceil_div(n_planes, 128), 128, 0, stream, n_planes, (long long)n_rows_total, sums, save_mean, save_invstd, running_mean, running_var, (float)eps, (float)momentum, 1, n_rows_total < 0 ? 1 : 0);
+  SCN_LAUNCH(k_bn_finalize, (unsigned)ceil_div(n_planes, 8), 256, 0, stream, n_planes, (long long)n_rows_total, sums, 1, save_mean, save_invstd, running_mean, running_var, (float)eps, (float)momentum, 1, n_rows_total < 0 ? 1 : 0);
   if (n_rows > 0) {
     SCN_REQUIRE(in_features && out_features, SCN_ERR_BAD_ARG, "null features");
     launch_bn_apply(in_features, out_features, n_rows, n_planes, in_stride, out_stride, save_mean, save_invstd, weight, bias, (float)leakiness, stream);
