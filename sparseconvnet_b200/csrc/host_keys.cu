@@ -2,8 +2,9 @@
 //
 // A point arrives as dim + 1 64-bit integers in pageable memory.  Copied as they are (32 bytes a point in 3-D, through the
 // driver's staging buffers at 12.5 GB/s, with the host held until the stream reaches the copy) 400 k points were 1.0 ms of
-// a training step's 9.5.  Here a few host threads check and pack each point into the 8 bytes the site table stores anyway
-// (bound by reading the coordinates once), and the insert kernel reads those across the bus: a quarter of the bytes, no staging.
+// a training step's 9.5.  Here a few host threads check and pack each point into the site table's key (bound by reading the
+// coordinates once), and the insert kernel reads those bytes of the keys that are in use across the bus: 4 to 6 instead of 32, no
+// staging.
 #include <stdlib.h>
 
 #include <algorithm>
@@ -112,16 +113,34 @@ PinnedPool &pinned_pool() {
   return *p;
 }
 
-template <int DIM>
+// what a packed key is written to
+struct WholeKeys {
+  unsigned long long *keys;
+  void put(long long i, unsigned long long key) { keys[i] = key; }
+  unsigned long long any() const { return 0; }
+};
+struct KeyBytes {
+  NarrowKeys keys;
+  unsigned long long all = 0;
+  void put(long long i, unsigned long long key) {
+    keys.low[i] = (unsigned)key;
+    keys.high[0][i] = (unsigned char)(key >> 32);
+    keys.high[1][i] = (unsigned char)(key >> 40);
+    all |= key;
+  }
+  unsigned long long any() const { return all; }
+};
+
+template <int DIM, class Keys>
 void pack_rows(const KeyLayout &L, const long long *coords, long long first, long long last, int ncols, long long bl_length,
-               unsigned long long *keys, int &samples, bool &bad) {
+               Keys &keys, int &samples, bool &bad) {
   const int dim = DIM ? DIM : L.dim;
   long long most = -1;
   bool wrong = false;
   for (long long i = first; i < last; ++i) {
     const long long *c = coords + i * ncols;
     if (bl_length > 0 && c[0] < 0) {  // empty slot of the batch x length array
-      keys[i] = kEmptyKey;
+      keys.put(i, kEmptyKey);
       continue;
     }
     const long long bl = bl_length > 0 ? i / bl_length : (ncols > dim ? c[dim] : 0);
@@ -132,7 +151,7 @@ void pack_rows(const KeyLayout &L, const long long *coords, long long first, lon
       key |= (unsigned long long)c[d] << L.shift[d];
     }
     wrong |= !ok;
-    keys[i] = key;
+    keys.put(i, key);
     most = std::max(most, bl);
   }
   samples = wrong ? 0 : (int)(most + 1);
@@ -187,18 +206,21 @@ void pinned_trim() {
   for (auto &b : idle) cudaFreeHost(b.p);
 }
 
-// keys[i] of every row (the empty key for an empty slot); *samples = batch indices in use; *bad: some row lies outside.
-void pack_keys(const KeyLayout &L, const long long *coords, long long n, int ncols, long long bl_length,
-               unsigned long long *keys, int *samples, bool *bad) {
+namespace {
+template <class Keys>
+void pack_all(const KeyLayout &L, const long long *coords, long long n, int ncols, long long bl_length, const Keys &to, int *samples,
+              bool *bad, unsigned long long *any) {
   // pieces of 16 k points (~30 us each): below two of them waking a helper costs more than it saves
   constexpr long long kPiece = 16384;
   const int pieces = (int)ceil_div(n, kPiece);
   std::atomic<int> most{0};
   std::atomic<bool> wrong{false};
+  std::atomic<unsigned long long> bits{0};
   Helpers::get().run(pieces, [&](int i) {
     const long long first = i * kPiece, last = std::min(n, first + kPiece);
     int s = 0;
     bool b = false;
+    Keys keys = to;
     switch (L.dim) {
       case 2: pack_rows<2>(L, coords, first, last, ncols, bl_length, keys, s, b); break;
       case 3: pack_rows<3>(L, coords, first, last, ncols, bl_length, keys, s, b); break;
@@ -206,12 +228,25 @@ void pack_keys(const KeyLayout &L, const long long *coords, long long n, int nco
       default: pack_rows<0>(L, coords, first, last, ncols, bl_length, keys, s, b);
     }
     if (b) wrong.store(true);
+    bits.fetch_or(keys.any());
     int was = most.load();
     while (s > was && !most.compare_exchange_weak(was, s)) {
     }
   });
   *samples = most.load();
   *bad = wrong.load();
+  if (any) *any = bits.load();
+}
+}  // namespace
+
+// keys[i] of every row (the empty key for an empty slot); *samples = batch indices in use; *bad: some row lies outside.
+void pack_keys(const KeyLayout &L, const long long *coords, long long n, int ncols, long long bl_length,
+               unsigned long long *keys, int *samples, bool *bad) {
+  pack_all(L, coords, n, ncols, bl_length, WholeKeys{keys}, samples, bad, nullptr);
+}
+void pack_keys(const KeyLayout &L, const long long *coords, long long n, int ncols, const NarrowKeys &keys, int *samples, bool *bad,
+               unsigned long long *any) {
+  pack_all(L, coords, n, ncols, 0, KeyBytes{keys}, samples, bad, any);
 }
 
 }  // namespace scn

@@ -155,5 +155,12 @@ void pinned_release(void *p, size_t bytes);
 void pinned_trim();
 void pack_keys(const KeyLayout &L, const long long *coords, long long n, int ncols, long long bl_length,
                unsigned long long *keys, int *samples, bool *bad);
+// ... in bytes of their own: bits 0 to 31, 32 to 39, 40 to 47 of every key; *any: the bits that some key has
+struct NarrowKeys {
+  unsigned *low;
+  unsigned char *high[2];
+};
+void pack_keys(const KeyLayout &L, const long long *coords, long long n, int ncols, const NarrowKeys &keys, int *samples, bool *bad,
+               unsigned long long *any);
 
 }  // namespace scn

@@ -30,3 +30,17 @@ def test_host_coordinate_out_of_range(row, value):
     coords[row, 1] = value
     with pytest.raises(RuntimeError, match="outside the spatial size"):
         _locations(scn, 3, coords, 40, 3)
+
+
+# keys of 30 to 33 bits, 36 to 39, 42 to 45, and more than 48, which travel whole; one piece and more
+@pytest.mark.parametrize("size", [1000, 4096, 16000, 65000])
+@pytest.mark.parametrize("n,batch", [(1, 1), (1025, 8), (16383, 2), (33793, 5)])
+@pytest.mark.parametrize("mode", [0, 3])
+def test_keys_by_their_bytes(n, batch, size, mode):
+    import sparseconvnet_b200 as scn
+    g = torch.Generator().manual_seed(n)
+    coords = torch.randint(0, size, (n, 4), generator=g)
+    coords[:, 3] = torch.randint(0, batch, (n,), generator=g)
+    coords[n // 2:] = coords[:n - n // 2].clone()  # every site twice
+    for a, b in zip(_locations(scn, 3, coords, size, mode), _locations(scn, 3, coords.cuda(), size, mode)):
+        assert torch.equal(a, b)
