@@ -508,11 +508,20 @@ k_tile_sum(const float4 *__restrict__ partial, int n_split, long long n_pos, int
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_pos * cout4) return;
   const int c = (int)(i % cout4);
+  const long long step = n_pos * cout4;
+  // the first four parts and the row on their way together (a place without a row has room for parts as well)
+  float4 v[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) v[p] = p < n_split ? __ldg(partial + p * step + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   const long long r = order ? __ldg(order + i / cout4) : i / cout4;
   if (r < 0 || r >= n_out) return;
-  float4 q = __ldg(partial + i);
-  for (int p = 1; p < n_split; ++p) {
-    const float4 a = __ldg(partial + (long long)p * n_pos * cout4 + i);
+  float4 q = v[0];
+#pragma unroll
+  for (int p = 1; p < 4; ++p)
+    if (p < n_split) q.x += v[p].x, q.y += v[p].y, q.z += v[p].z, q.w += v[p].w;
+#pragma unroll 4
+  for (int p = 4; p < n_split; ++p) {
+    const float4 a = __ldg(partial + p * step + i);
     q.x += a.x, q.y += a.y, q.z += a.z, q.w += a.w;
   }
   if (bias) {

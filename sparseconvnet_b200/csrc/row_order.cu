@@ -179,13 +179,37 @@ k_order_scatter(const KEY *__restrict__ keys, const int *__restrict__ rows_in, l
   }
 }
 
-// Levels too small to sort: the identity order, its tiles and their entries in one launch, one block per tile.
+// Levels too small to sort: the identity order, its tiles and their entries in one launch, one block per tile.  Bound by trips to
+// memory one behind the other: with at most 32 offsets a row's entries are asked for at once and stay in registers (2.8 us for
+// 27 offsets on 6 k rows; 5.8 when they were read nine at a time, twice).
+template <bool ONE_WORD>
 __global__ void __launch_bounds__(kTile)
 k_order_plain(const int *__restrict__ nbr, long long n, int K, int words, int *__restrict__ order,
               unsigned *__restrict__ tile_bits, int *__restrict__ packed) {
   SCN_GRID_WAIT();
   __shared__ unsigned bits[4];
   const long long t = blockIdx.x, p = t * kTile + threadIdx.x;
+  if (ONE_WORD) {
+    int v[32];
+#pragma unroll
+    for (int k = 0; k < 32; ++k) v[k] = k < K && p < n ? __ldg(nbr + (long long)k * n + p) : -1;
+    if (threadIdx.x < 4) bits[threadIdx.x] = 0;
+    order[p] = p < n ? (int)p : -1;
+    __syncthreads();
+    unsigned mine = 0;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) mine |= v[k] >= 0 ? 1u << k : 0u;
+    const unsigned seen = __reduce_or_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31) == 0) atomicOr(&bits[0], seen);
+    __syncthreads();
+    const unsigned all = bits[0];
+    if (threadIdx.x == 0) tile_bits[t] = all;
+    int *dst = packed + t * K * kTile + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 32; ++k)
+      if (all >> k & 1u) dst[__popc(all & ((1u << k) - 1u)) * kTile] = v[k];
+    return;
+  }
   if (threadIdx.x < 4) bits[threadIdx.x] = 0;
   order[p] = p < n ? (int)p : -1;
   __syncthreads();
@@ -574,7 +598,7 @@ int rulebook_row_order(const Rulebook &rb, const int *table, long long n, RowOrd
   long long least = 8192;
   if (const char *e = getenv("SCN_ORDER_MIN_ROWS")) least = atoll(e);
   if (st == SCN_OK && n < least) {
-    SCN_LAUNCH(k_order_plain, (unsigned)o.n_tiles, kTile, 0, stream, table, n, K, o.words, o.order, o.tile_bits, o.packed);
+    SCN_LAUNCH((K <= 32 ? k_order_plain<true> : k_order_plain<false>), (unsigned)o.n_tiles, kTile, 0, stream, table, n, K, o.words, o.order, o.tile_bits, o.packed);
     if (cudaGetLastError() != cudaSuccess) {
       set_error("row order: launch failed");
       st = SCN_ERR_CUDA;

@@ -255,3 +255,28 @@ def test_scale_and_shift_anywhere(n, cin, cout, precision, cuda):
             assert torch.equal(out, results[0][0]) and torch.equal(both, results[0][1])
     finally:
         scn.set_precision("fp32")
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 3000])
+@pytest.mark.parametrize("dim,filter_size", [(1, 1), (3, 3), (1, 31), (2, 5), (1, 33), (2, 7)])
+def test_rows_in_their_own_order(n, dim, filter_size, cuda):
+    """Tiles of levels too small to sort, up to 32 offsets (one word of a mask) and above: against float64."""
+    import sparseconvnet_b200 as scn
+    coords = _points(n, dim, 8192 if dim == 1 else 200 if dim == 2 else 40, n)
+    torch.manual_seed(n)
+    layer = scn.SubmanifoldConvolution(dim, 16, 16, filter_size, True).to(cuda)
+    size = torch.LongTensor([8192 if dim == 1 else 200 if dim == 2 else 40] * dim)
+    try:
+        scn.set_precision("tf32x3")
+        with torch.no_grad():
+            x = scn.InputLayer(dim, size, mode=0)([torch.from_numpy(coords), torch.randn(len(coords), 16, device=cuda)])
+            y = layer(x).features
+            x.metadata.poll_errors()
+            want = torch.zeros(len(coords), 16, dtype=torch.float64, device=cuda) + layer.bias.double()
+            for r, w in zip(x.metadata.rulebook(0, size, [filter_size] * dim, None), layer.weight.double()[:, 0]):
+                r = r.long().to(cuda)
+                want.index_add_(0, r[:, 1], x.features.double()[r[:, 0]] @ w)
+            # (three bf16 terms of a product: 2^-16 of it is left out at most)
+            assert float((y.double() - want).norm() / want.norm()) <= 2.0 ** -16
+    finally:
+        scn.set_precision("fp32")
