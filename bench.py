@@ -44,11 +44,11 @@ UNIT = "voxels/s"
 TRAFFIC_RATIO = {"k_conv_tile": 0.27}
 # (bound reported for the kernel, what the ncu captures show as its limiter)
 LIMITS = {
-    "k_conv_tile": ("hbm", "the gather of whole rows from L2 into shared memory by 16-byte cp.async (ncu, 4-room case): LSU "
-                           "wavefronts 39 % of peak on average and up to 53 %, tensor pipe 25 % (43 % on the widest levels), "
-                           "issue slots 28 %; DRAM sees 0.27 of the algorithmic bytes"),
-    "k_conv_six": ("hbm", "the copies of rows and weights into shared memory, 30 to 48 KB per step of 128 rows and 32 planes, and "
-                          "the drain of the step's sums beside the tensor core"),
+    "k_conv_tile": ("hbm", "the chain of barriers between copies and instructions, a step of 128 rows at a time (ncu, layers on "
+                           "200 k rows): tensor pipe 20 to 72 % active for 32 to 128 planes, issue slots 57 to 40 %, shared memory "
+                           "banks 39 to 56 %, L2 37 to 56 bytes per cycle and SM; DRAM sees 0.27 of the algorithmic bytes"),
+    "k_conv_six": ("hbm", "the way from a step's instructions through the drain of its sums to the next one (ncu, layers on 200 k "
+                          "rows): tensor pipe 21 to 73 % active for 32 to 128 planes, issue slots 64 to 46 %"),
 }
 # what `dtype` says for each arithmetic mode: the type the path computes in, kernel by kernel
 DTYPE_LABEL = {

@@ -27,15 +27,14 @@
 //               traffic, 1 100 cycles per step of 96 planes with two ranges, more than the step's 700 of instructions
 //   drain       8 warps, a row and half of the planes per lane: TMEM -> registers after every step, and after the tile's
 //               last one through shared memory -> bias -> optional BatchNorm -> 16-byte stores, four lanes per row
-// Bound by shared memory from 96 planes on: a step of 96 planes writes 42 KB of rows and weights and its instructions read 84 KB,
-// 1 008 cycles of 128 bytes (1 070 measured); below that by the way from an instruction through the drain back to its
-// accumulator (64 planes, two accumulators of three ranges: 1 030 cycles where shared memory takes 672; 32 planes 880, 528).  As
-// multiply-adds the same step is 1 024 to 4 096 cycles of the whole FMA pipe.  That way is why the barriers of the next step
-// are looked at while this one is under way and why the loads of a row's stores come before its branches: with a wait, a look at the
-// abort flag and a role for the weights in every step, 200 k rows: 32 -> 32 planes 103 us, 92 now; 64 -> 64 229, 207; 96 -> 96
-// 373, 325; 128 -> 128 527, 455; a Deconvolution 128 -> 96 to 43 k rows 28, 17.  (Three loads of 16 columns under one wait
-// do not fit the registers of 64 planes: 216.)  Rows split once per call, not once per gather: with fp32 rows (16 KB per step) split
-// by the producers on their way through registers a step took twice as long.
+// Tensor pipe active 73 % for 128 output planes, 54 for 96 (200 k rows, 1 050 and 1 070 cycles per step); below that no unit is near
+// its peak: 64 planes 38 % beside 64 % of the issue slots and 1 030 cycles per step, 32 planes 21 and 59 %, 880 cycles.  As multiply-adds
+// the same step is 1 024 to 4 096 cycles of the whole FMA pipe.  The barriers of the next step are looked at while this one is
+// under way and the loads of a row's stores come before its branches: with a wait, a look at the abort flag and a role for the
+// weights in every step, 200 k rows: 32 -> 32 planes 103 us, 92 now; 64 -> 64 229, 207; 96 -> 96 373, 325; 128 -> 128 527, 455; a
+// Deconvolution 128 -> 96 to 43 k rows 28, 17.  (64 planes: three loads of 16 columns under one wait do not fit the registers, 216;
+// two column ranges and with them four accumulators 204; sixteen drain warps 207.)  Rows split once per call, not once per gather:
+// with fp32 rows (16 KB per step) split by the producers on their way through registers a step took twice as long.
 //
 // Every wait is bounded; on expiry the role raises the abort flag, everybody leaves, tensor memory is freed and
 // the host sees FLAG_TC_TIMEOUT through scn_md_poll_errors.

@@ -17,16 +17,15 @@
 //     since the reads count: U-Net on eight rooms 6095 -> 6034 us, on one room 1912 -> 1884.  The small terms are no longer cut
 //     off against the large ones, so the error against float64 fell: 128 -> 128 planes on 60 k rows 6.6e-6 -> 4.7e-6, of one
 //     sign 6.9e-6 -> 3.7e-6; smaller for every shape of 80 to 128 planes.)
-//   * What bounds it is shared memory, 128 bytes per cycle and SM: a step of 32 -> 32 planes writes 16 KB of rows and 4 KB of
-//     weights and its four instructions read 22 KB, 336 cycles (416 for 64 -> 64, 496 for 96 -> 96, 576 for 128 -> 128), against
-//     176, 224, 304 and 384 cycles of tensor work.  L2 is not the limit: 16-byte cp.async gathers of rows that lie in L2 reach
-//     75 bytes per cycle and SM, twice what a step needs.
-//   * So that shared memory is busy all the time no role may take longer per step than that, and every barrier, load and store
-//     of shared memory waits 100 to 200 cycles behind the copies.  With a thread of its own for the weights (two waits, a
-//     load, an arrival and the copy per step: 1 050 cycles) and instructions issued inside a branch of one lane (descriptors moved
-//     into uniform registers one by one: 135 cycles per four instructions, 38 with a predicate) the same tiles took, 8 rooms:
-//     32 -> 32 planes 253 us, now 202; 64 -> 64 145, 132; 96 -> 96 98, 88; 128 -> 128 83, 70; 224 -> 224 on 1.4 k rows 22.6, 19.6;
-//     4-D 64 -> 64 bf16 778, 671.
+//   * A step's work is small beside the barriers around it, so what bounds it is the longest chain of any one role: 224 to 384 cycles
+//     of tensor instructions, 336 (32 -> 32 planes: 20 KB written, 22 read) to 576 (128 -> 128) cycles of shared memory at 128
+//     bytes; L2 gives 75 bytes per cycle and SM to 16-byte cp.async gathers of rows that lie in it, a step takes 37 to 56.  Every
+//     wait, load and store of shared memory stands 100 to 200 cycles behind the copies.  With a thread of its own for the
+//     weights (two waits, a load, an arrival and the copy per step: 1 050 cycles) and instructions issued inside a branch of
+//     one lane (descriptors moved into uniform registers one by one: 135 cycles per four instructions, 38 with a predicate) the
+//     same tiles took, 8 rooms: 32 -> 32 planes 253 us, now 207; 64 -> 64 145, 134; 96 -> 96 98, 88; 128 -> 128 83, 69;
+//     224 -> 224 on 1.4 k rows 22.6, 18.2; 4-D 64 -> 64 bf16 778, 676.  Now, 200 k rows: tensor pipe active 20, 41, 54, 72 % for 32,
+//     64, 96, 128 planes, shared memory banks 22 + 17 to 33 + 24 % (read + written), issue slots 57, 56, 42, 40 %.
 //
 // Roles (14 warps, one or two CTAs per SM, persistent).  A step is one filter offset of one tile and SP input planes; the
 // steps of a CTA are numbered through all its tiles and step n uses stage n % n_stages of one ring.
