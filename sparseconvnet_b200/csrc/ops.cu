@@ -327,7 +327,7 @@ k_bn_back_sums(const float *__restrict__ in, const float *__restrict__ out, cons
 }
 
 // The same for rows of whole 16-byte pieces: eight lanes per row and 32 planes, two rows of a lane in flight.  Bound by HBM
-// and the conversions to double: the 14 layers of a U-Net training step on 400 k points 338 us (469 with one value per load).
+// (sums in fp32 would save 3 %): the 14 layers of a U-Net training step on 400 k points 293 us (469 with one value per load).
 __global__ void __launch_bounds__(256)
 k_bn_back_sums4(const float *__restrict__ in, const float *__restrict__ out, const float *__restrict__ d_out, int n_rows, int C,
                 int in_stride, int out_stride, const float *__restrict__ mean, float leak, int chunk_rows,
@@ -383,6 +383,14 @@ k_bn_back_sums4(const float *__restrict__ in, const float *__restrict__ out, con
     for (int i = 0; i < 8; ++i) t += sh[wy][i][lane];
     partial[(long long)(wy * C + col) * gridDim.y + blockIdx.y] = t;
   }
+}
+
+// Chunks of at least 64 rows, at most as many blocks as are on the SMs at once (four each: 59 and 64 registers a thread).  With up
+// to 1 024 chunks of at least 256 rows a layer's blocks took one and a half waves to two, and levels of 10 k rows had too
+// few: the 14 layers of a U-Net training step on 400 k points 329 -> 293 us, their k_bn_back_finalize 43 -> 38, the seven on
+// 93 k and fewer pixels 44 -> 28 (k_bn_back_finalize there 15 -> 18).
+static int bn_back_chunks(long long n_rows, int C) {
+  return (int)std::max<long long>(1, std::min<long long>(ceil_div(n_rows, 64), 148 * 4 / ceil_div(C, 32)));
 }
 
 static void launch_bn_back_sums(const float *in, const float *out, const float *d_out, long long n_rows, int C, long long in_stride,
@@ -919,7 +927,7 @@ int scn_batchnorm_backward(const float *in_features, float *d_in_features, const
     return SCN_OK;
   }
   SCN_REQUIRE(in_features && d_in_features && out_features && d_out_features, SCN_ERR_BAD_ARG, "null features");
-  const int chunks = (int)std::max<long long>(1, std::min<long long>(1024, n_rows / 256));
+  const int chunks = bn_back_chunks(n_rows, n_planes);
   const long long chunk_rows = ceil_div(n_rows, chunks);
   double *partial = nullptr;
   float *coef = nullptr;
@@ -1000,7 +1008,7 @@ int scn_batchnorm_backward_sums(const float *in_features, const float *out_featu
     return SCN_OK;
   }
   SCN_REQUIRE(in_features && out_features && d_out_features, SCN_ERR_BAD_ARG, "null features");
-  const int chunks = (int)std::max<long long>(1, std::min<long long>(1024, n_rows / 256));
+  const int chunks = bn_back_chunks(n_rows, n_planes);
   const long long chunk_rows = ceil_div(n_rows, chunks);
   double *partial = nullptr;
   SCN_TRY(device_alloc((void **)&partial, sizeof(double) * 2 * (size_t)chunks * n_planes, stream));
