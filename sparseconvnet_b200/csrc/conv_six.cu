@@ -110,6 +110,7 @@ struct Ctl {
   unsigned long long r_full[kRecords], r_empty[kRecords];
   ItemRecord record[kRecords];  // part: the item within its tile
   int slot_k[kSlots];  // filter offset + (column block << 10); -1: no more work; + kNoRules: offset 0 with rows of zeros
+  OrderedCopies ordered;
   unsigned tmem, range[2];
   int abort;
 };
@@ -461,14 +462,8 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
     }
     if (bad) atomicOr(P.flags, FLAG_BAD_ROW);
     asm volatile("cp.async.wait_all;" ::: "memory");  // they must land before the CTA's shared memory goes away
-    if (!ok) {
-      *abort = 1;
-      if (brings_weights)  // and so must the slabs
-        for (int i = max(0, filled - (P.n_stages + kProdGroups - 1) / kProdGroups); i < filled; ++i) {
-          const int n = group + i * kProdGroups;
-          mbar_wait(&C.full[n % P.n_stages], (n / P.n_stages) & 1);
-        }
-    }
+    if (brings_weights) C.ordered.slabs[group] = filled;
+    if (!ok) *abort = 1;
   } else if (warp < kMma + kMmaWarps && warp >= kMma) {
     // ==================================== MMA issue =============================================
     // Two warps take the accumulators in turn: what one spends on barriers passes while the other's instructions run (U-Net
@@ -606,7 +601,6 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
           }
         }
       }
-      const int filled = slot;
       // every producing warp finds its next step in a slot that ends it
       const int ends = (kProdGroups - 1) / P.n_slices + 1;
       for (int i = 0; i < ends && ok; ++i, ++slot) {
@@ -618,13 +612,8 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
         C.slot_k[si] = -1;
         mbar_arrive(&C.s_full[si]);
       }
-      if (!ok) {  // copies in flight must land before the CTA's shared memory goes away
-        *abort = 1;
-        for (int i = 0; i < kSlots; ++i) {
-          const int uses = (filled + kSlots - 1 - i) / kSlots;
-          if (uses > 0) mbar_wait(&C.s_full[i], (unsigned)((uses - 1) & 1));
-        }
-      }
+      C.ordered.slots = slot;
+      if (!ok) *abort = 1;
     }
   } else if (warp < kMma) {
     // ==================================== drain =================================================
@@ -738,7 +727,11 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
   }
   tc_fence_before();
   __syncthreads();
-  if (*abort && tid == 0) atomicOr(P.flags, FLAG_TC_TIMEOUT);
+  if (*abort) {
+    if (tid == 0) atomicOr(P.flags, FLAG_TC_TIMEOUT);
+    land_copies<kSlots>(C, P.n_stages, kProdGroups);
+  }
+  __syncwarp();
   if (warp == kMma) tmem_dealloc(tmem, 512);
 }
 

@@ -110,6 +110,7 @@ struct Ctl {
   ItemRecord record[kRecords];
   int total_steps;     // of the CTA, when the slots end
   int slot_k[kSlots];  // filter offset of the slot; -1: no more work; kNoRules: offset 0 with rows of zeros
+  OrderedCopies ordered;
   unsigned tmem;
   int abort;
 };
@@ -300,13 +301,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     }
     if (bad) atomicOr(P.flags, FLAG_BAD_ROW);
     asm volatile("cp.async.wait_all;" ::: "memory");  // they must land before the CTA's shared memory goes away
+    if (brings_weights) C.ordered.slabs[group] = filled;
     if (!ok) {
       *abort = 1;
-      if (brings_weights)  // and so must the slabs
-        for (int i = max(0, filled - (P.n_stages + kProdGroups - 1) / kProdGroups); i < filled; ++i) {
-          const int n = group + i * kProdGroups;
-          mbar_wait(&C.full[n % P.n_stages], (n / P.n_stages) & 1);
-        }
     } else if (!*abort) {
       // The CTA's last item: these warps store two thirds of its columns, through the ring, which nothing reads any more when
       // the last step has been consumed.  (The step before it first, whose parity cannot be an earlier round's: this
@@ -437,10 +434,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
           }
         }
       }
-      const int filled = slot;
       // every producing warp finds its next step in a slot that ends it
       const int ends = (kProdGroups - 1) / P.n_slices + 1;
-      C.total_steps = filled * P.n_slices;
+      C.total_steps = slot * P.n_slices;
       for (int i = 0; i < ends && ok; ++i, ++slot) {
         const int si = slot % kSlots;
         if (!mbar_wait(&C.s_empty[si], ((slot / kSlots) + 1) & 1)) {
@@ -450,13 +446,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
         C.slot_k[si] = -1;
         mbar_arrive(&C.s_full[si]);
       }
-      if (!ok) {  // copies in flight must land before the CTA's shared memory goes away
-        *abort = 1;
-        for (int i = 0; i < kSlots; ++i) {
-          const int uses = (filled + kSlots - 1 - i) / kSlots;
-          if (uses > 0) mbar_wait(&C.s_full[i], (unsigned)((uses - 1) & 1));
-        }
-      }
+      C.ordered.slots = slot;
+      if (!ok) *abort = 1;
     }
   } else {
     // ==================================== epilogue ==============================================
@@ -494,7 +485,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
   }
   tc_fence_before();
   __syncthreads();
-  if (*abort && tid == 0) atomicOr(P.flags, FLAG_TC_TIMEOUT);
+  if (*abort) {
+    if (tid == 0) atomicOr(P.flags, FLAG_TC_TIMEOUT);
+    land_copies<kSlots>(C, P.n_stages, kProdGroups);
+  }
+  __syncwarp();
   if (warp == kMma) tmem_dealloc(tmem, (unsigned)P.tmem_cols);
 }
 

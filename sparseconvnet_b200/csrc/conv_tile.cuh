@@ -94,4 +94,37 @@ struct Tiles {
     fetch(P, next, next_mask);
   }
 };
+
+// What the bulk copies of a CTA have been ordered for, left by the threads that order them when they leave their loops.
+struct OrderedCopies {
+  int slots;     // by the entries, the slots that end the work among them
+  int slabs[2];  // weights of the steps g, g + groups, ... by group g of the producing warps
+};
+
+// The last step of those that use stage `st` whose slab has been ordered, -1: none.  (The ones before it have been consumed: an order
+// waits for that.)
+__host__ __device__ inline int last_slab(const int *slabs, int groups, int n_stages, int st) {
+  int last = -1;
+  for (int g = 0; g < groups; ++g)
+    for (int i = slabs[g] - 1; i >= 0 && i >= slabs[g] - n_stages; --i)
+      if ((g + i * groups) % n_stages == st) {
+        if (g + i * groups > last) last = g + i * groups;
+        break;
+      }
+  return last;
+}
+
+// A CTA whose roles left early, whichever of them and on whichever way: its bulk copies must land before its shared memory goes
+// away.  All threads come here behind the block's last barrier, when nobody orders any more; one waits for each stage and each slot.
+template <int SLOTS, class Control>
+__device__ __forceinline__ void land_copies(Control &C, int n_stages, int groups) {
+  const int st = threadIdx.x, si = (int)threadIdx.x - 32;
+  if (st < n_stages) {
+    const int step = last_slab(C.ordered.slabs, groups, n_stages, st);
+    if (step >= 0) mbar_wait(&C.full[st], (unsigned)(step / n_stages & 1));
+  } else if (si >= 0 && si < SLOTS) {
+    const int uses = (C.ordered.slots + SLOTS - 1 - si) / SLOTS;
+    if (uses > 0) mbar_wait(&C.s_full[si], (unsigned)((uses - 1) & 1));
+  }
+}
 }  // namespace scn

@@ -1,8 +1,13 @@
-"""What a launch through SCN_LAUNCH relies on, checked in the sources: every kernel's first statement waits for the kernel
-before it."""
+"""What the kernels rely on, checked in the sources: every kernel's first statement waits for the kernel before it; the kernels on
+row tiles end well when a wait has run out."""
+import ctypes
 import glob
 import os
+import random
 import re
+import subprocess
+
+import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sparseconvnet_b200", "csrc")
 
@@ -32,3 +37,50 @@ def test_every_kernel_waits_first():
                     waiting.add(name.group(1))
     assert len(defined) > 60
     assert defined == waiting, sorted(defined - waiting)
+
+
+TILE_KERNELS = ["conv_tile.cu", "conv_six.cu"]
+
+
+def _source(name):
+    return re.sub(r"//.*", "", open(os.path.join(CSRC, name)).read())
+
+
+@pytest.mark.parametrize("name", TILE_KERNELS)
+def test_bulk_copies_land_on_every_way_out(name):
+    """Whatever made a role leave, and when: behind the block's last barrier the abort flag alone decides whether the bulk copies are
+    waited for, and both roles that order them have said which, unconditionally."""
+    text = _source(name)
+    end = text[text.rindex("__syncthreads();", 0, text.index("tmem_dealloc(tmem")):text.index("tmem_dealloc(tmem")]
+    assert re.search(r"if \(\*abort\) \{[^}]*land_copies<kSlots>\(C, P\.n_stages, kProdGroups\);\s*\}", end)
+    assert re.search(r"\n    if \(brings_weights\) C\.ordered\.slabs\[group\] = filled;", text)
+    assert re.search(r"\n      C\.ordered\.slots = slot;", text)
+    assert text.count("bulk_copy_g2s(") == 2
+
+
+def test_last_slab(tmp_path):
+    """The slab that a stage may still be waiting for, against a ring played step by step: two groups of warps, or one, order
+    weights when a stage is free, steps are consumed in their turn, and everybody stops at some point."""
+    text = _source("conv_tile.cuh")
+    at = text.index("__host__ __device__ inline int last_slab")
+    body = text[at:text.index("\n}\n", at) + 3].replace("__host__ __device__ inline", 'extern "C"')
+    src, lib = tmp_path / "last_slab.cpp", tmp_path / "last_slab.so"
+    src.write_text(body)
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-shared", "-fPIC", "-o", str(lib), str(src)])
+    last_slab = ctypes.CDLL(str(lib)).last_slab
+    rng = random.Random(5)
+    for groups in (1, 2):
+        for stages in range(2, 13):
+            for _ in range(60):
+                ordered, consumed, total = [0] * groups, 0, rng.randrange(0, 40)
+                for _ in range(rng.randrange(0, 120)):
+                    g = rng.randrange(groups + 1)
+                    if g == groups:  # the next step has been consumed, if it is there
+                        consumed += consumed // groups < ordered[consumed % groups]
+                    elif (step := g + ordered[g] * groups) < total and step - stages < consumed:
+                        ordered[g] += 1
+                steps = {g + i * groups for g in range(groups) for i in range(ordered[g])}
+                for st in range(stages):
+                    mine = [n for n in steps if n % stages == st]
+                    assert last_slab((ctypes.c_int * 2)(*ordered), groups, stages, st) == max(mine, default=-1)
+                    assert all(n < consumed for n in mine if n != max(mine))  # the others need no waiting for
