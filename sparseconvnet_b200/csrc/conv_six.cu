@@ -390,7 +390,8 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
     // ==================================== producers =============================================
     // Group g of four warps takes the steps g, g + kProdGroups, ...; a warp copies 32 rows of a step, a lane one 16-byte piece of
     // [h | m] of the rows q NI .. q NI + NI - 1 of them and one of [l] of half of these.  The input rows of the next step are in
-    // registers before its stage is free.
+    // registers before its stage is free.  A warp leaves as a whole: what its lanes do together has no limit to its wait for one
+    // that has gone.
     const int j = lane % Shape::PIECES, q = lane / Shape::PIECES, lj = lane % Shape::L_PIECES, lq = lane / Shape::L_PIECES;
     const int group = warp / kStepWarps, row0 = warp % kStepWarps * 32 + q * Shape::NI, l_row0 = warp % kStepWarps * 32 + lq * Shape::L_NI;
     // (where a 16-byte chunk c of row r goes: rows_desc; rows of 128 bytes come in eights, of 64 in fours, of 32 in twos)
@@ -408,12 +409,10 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
         const int si = slot % kSlots;
         // (A warp comes by every slot, or by every second one with one slice: it has seen the slot kSlots before this one
         // filled, so the parity cannot be that of an earlier round.)
-        if (!mbar_wait(&C.s_full[si], (slot / kSlots) & 1)) {
-          ok = false;
-          break;
-        }
+        ok = mbar_wait_warp(&C.s_full[si], (slot / kSlots) & 1, abort);
+        if (!ok) break;
         slot_k = C.slot_k[si];
-        if (slot_k < 0 || *abort) break;
+        if (slot_k < 0) break;
         const int *ent = entries + si * kRows + row0;
 #pragma unroll
         for (int i = 0; i < Shape::NI; i += 4) {
@@ -428,10 +427,8 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
           bad |= rows[i] >= (int)P.n_in;
         }
       }
-      if (!mbar_wait(&C.empty[st], par)) {  // (the first round passes)
-        ok = false;
-        break;
-      }
+      ok = mbar_wait_warp(&C.empty[st], par, abort);  // (the first round passes)
+      if (!ok) break;
       const unsigned at = (unsigned)st * stage_bytes;
       if (brings_weights && !(P.drop && blockIdx.x == 0 && group == 0 && filled == 0)) {
         const int k = slot_k & 1023, block = slot_k >> 10 & 1;

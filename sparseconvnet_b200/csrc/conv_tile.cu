@@ -234,7 +234,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
   if (warp < kProdWarps) {
     // ==================================== producers =============================================
     // Group g of four warps takes the steps g, g + 2, ...; a warp copies 32 rows of a step, a lane one 16-byte piece of the
-    // rows q NI .. q NI + NI - 1 of them.  The input rows of the next step are in registers before its stage is free.
+    // rows q NI .. q NI + NI - 1 of them.  The input rows of the next step are in registers before its stage is free.  A warp leaves
+    // as a whole: what its lanes do together has no limit to its wait for one that has gone.
     const int j = lane % PP, q = lane / PP, group = warp / kStepWarps, row0 = warp % kStepWarps * 32 + q * NI;
     // (ROW 128: rows come in eights, chunk j of row r is stored at j ^ (r & 7); ROW 64: in fours, at j ^ ((r >> 1) & 3))
     const unsigned lane_dst = smem0 + (unsigned)row0 * Shape::ROW + (unsigned)((PP == 8 ? j : j ^ (q & 1) * 2) * 16);
@@ -250,16 +251,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
         const int si = slot % kSlots;
         // (A warp comes by every slot, or by every second one with one slice: it has seen the slot kSlots before this one
         // filled, so the parity cannot be that of an earlier round.)
-        if (!mbar_wait(&C.s_full[si], (slot / kSlots) & 1)) {
-          ok = false;
-          break;
-        }
+        ok = mbar_wait_warp(&C.s_full[si], (slot / kSlots) & 1, abort);
+        if (!ok) break;
         slot_k = C.slot_k[si];
         if (slot_k < 0) break;
-        if (*abort) {
-          ok = false;
-          break;
-        }
         const int4 *ent = reinterpret_cast<const int4 *>(entries + si * kRows + row0);
 #pragma unroll
         for (int i = 0; i < NI; i += 4) {
@@ -274,10 +269,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
           bad |= rows[i] >= (int)P.n_in;
         }
       }
-      if (!mbar_wait(&C.empty[st], par)) {  // (the first round passes)
-        ok = false;
-        break;
-      }
+      ok = mbar_wait_warp(&C.empty[st], par, abort);  // (the first round passes)
+      if (!ok) break;
       const unsigned dst = lane_dst + (unsigned)st * stage_bytes;
       if (brings_weights && !(P.drop && blockIdx.x == 0 && group == 0 && filled == 0)) {
         const unsigned char *w = P.wprep + ((size_t)(slot_k == kNoRules ? 0 : slot_k) * P.n_slices + slice) * w_bytes;
@@ -304,16 +297,15 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     if (brings_weights) C.ordered.slabs[group] = filled;
     if (!ok) {
       *abort = 1;
-    } else if (!*abort) {
+    } else if (!__any_sync(0xffffffffu, *abort != 0)) {
       // The CTA's last item: these warps store two thirds of its columns, through the ring, which nothing reads any more when
       // the last step has been consumed.  (The step before it first, whose parity cannot be an earlier round's: this
       // warp has seen the consumption of the one n_stages before either.)
       const int last = (int)my_items - 1, n = C.total_steps, quad = warp & 3;
       const ItemRecord R = C.record[last % kRecords];
       const int orow = __ldg(P.order + (long long)R.tile * kRows + quad * 32 + lane);
-      if ((n < 2 || mbar_wait(&C.empty[(n - 2) % P.n_stages], ((n - 2) / P.n_stages) & 1)) &&
-          mbar_wait(&C.empty[(n - 1) % P.n_stages], ((n - 1) / P.n_stages) & 1)) {
-        __syncwarp();
+      if ((n < 2 || mbar_wait_warp(&C.empty[(n - 2) % P.n_stages], ((n - 2) / P.n_stages) & 1, abort)) &&
+          mbar_wait_warp(&C.empty[(n - 1) % P.n_stages], ((n - 1) / P.n_stages) & 1, abort)) {
         tc_fence_after();
         store_columns<PARTS, OUT_SPLIT>(P, joint, tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(last % n_acc * dcols), R, orow, quad,
                                         lane, reinterpret_cast<float4 *>(smem + warp * kEpiBytes), 16 * (1 + group), 16 * kStoreSets);

@@ -176,6 +176,21 @@ __device__ __forceinline__ bool mbar_wait_warp(unsigned long long *bar, unsigned
   }
   return false;
 }
+// The same for a warp that also leaves when another role has given up; the flag is looked at only where the phase is not there yet.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long *bar, unsigned parity, const volatile int *abort) {
+  const unsigned addr = smem_u32(bar);
+  for (unsigned it = 0; it < kWaitLimit; ++it) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (__all_sync(0xffffffffu, done != 0)) return true;
+    if (__any_sync(0xffffffffu, *abort != 0)) return false;
+  }
+  return false;
+}
 // D[128 x N] (+)= A * B; descriptors as (low, high) words.  The whole warp comes here with the same operands and the lane whose
 // `lead` is set issues: a predicate instead of a branch, so that the descriptors are made in uniform registers.  Four
 // instructions and their commit take 38 + 20 cycles of the warp like this, 135 + 57 inside a branch of one lane.

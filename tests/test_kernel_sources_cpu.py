@@ -58,6 +58,24 @@ def test_bulk_copies_land_on_every_way_out(name):
     assert text.count("bulk_copy_g2s(") == 2
 
 
+def _role(text, name):
+    return re.search(r"// =+ %s =+\n(.*?)(?=// =====|\n__global__)" % name, text, re.S).group(1)
+
+
+def _decided_by_lanes(text):
+    """Waits and looks at the abort flag in `text` whose outcome may differ between the lanes of a warp."""
+    looks = re.sub(r"__(any|all)_sync\(0xffffffffu, [^;]*?\*abort != 0\)", "", re.sub(r"\*abort = 1", "", re.sub(r"//.*", "", text)))
+    return re.findall(r"\bmbar_wait\(|\*abort", looks)
+
+
+@pytest.mark.parametrize("name", TILE_KERNELS)
+@pytest.mark.parametrize("role", ["producers", "MMA issue"])
+def test_warps_leave_as_a_whole(name, role):
+    """Behind a wait that can run out, or the abort flag, all lanes of a warp go the same way: the collectives that follow
+    (__syncwarp, shuffles, tcgen05.ld) would wait without limit for a lane that has left."""
+    assert not _decided_by_lanes(_role(open(os.path.join(CSRC, name)).read(), role))
+
+
 def test_last_slab(tmp_path):
     """The slab that a stage may still be waiting for, against a ring played step by step: two groups of warps, or one, order
     weights when a stage is free, steps are consumed in their turn, and everybody stops at some point."""
