@@ -449,20 +449,16 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
     int next_orow = 0;  // this lane's row of the next item: asked for an item ahead
     for (int it = 0; it < (int)my_items; ++it) {
       const int ri = it % kRecords;
-      int got = 1;
-      if (lane == 0) got = mbar_wait(&C.r_full[ri], (it / kRecords) & 1) ? 1 : 0;
-      if (!__shfl_sync(0xffffffffu, got, 0)) {
+      if (!mbar_wait_warp(&C.r_full[ri], (it / kRecords) & 1, abort)) {
         *abort = 1;
         break;
       }
-      const ItemRecord R = C.record[ri];
+      const ItemRecord R = C.record[ri];  // (each lane has seen the phase: a shuffle of one lane's answer orders no memory)
       __syncwarp();
       if (lane == 0) mbar_arrive(&C.r_empty[ri]);
       const int orow = it ? next_orow : __ldg(P.order + (long long)R.tile * kRows + quad * 32 + lane);
       next_orow = __ldg(P.order + (long long)R.next_tile * kRows + quad * 32 + lane);
-      if (lane == 0) got = (!*abort && mbar_wait(&C.acc_full[buf], buf_par)) ? 1 : 0;
-      got = __shfl_sync(0xffffffffu, got, 0);
-      if (!got) {
+      if (!mbar_wait_warp(&C.acc_full[buf], buf_par, abort)) {
         *abort = 1;
         break;
       }

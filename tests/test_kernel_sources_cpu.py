@@ -59,7 +59,7 @@ def test_bulk_copies_land_on_every_way_out(name):
 
 
 def _role(text, name):
-    return re.search(r"// =+ %s =+\n(.*?)(?=// =====|\n__global__)" % name, text, re.S).group(1)
+    return re.search(r"// =+ %s =+\n(.*?)(?=// =====|\n  __syncthreads)" % name, text, re.S).group(1)
 
 
 def _decided_by_lanes(text):
@@ -68,11 +68,12 @@ def _decided_by_lanes(text):
     return re.findall(r"\bmbar_wait\(|\*abort", looks)
 
 
-@pytest.mark.parametrize("name", TILE_KERNELS)
-@pytest.mark.parametrize("role", ["producers", "MMA issue"])
+@pytest.mark.parametrize("name,role", [(name, role) for name, stores in zip(TILE_KERNELS, ("epilogue", "drain"))
+                                       for role in ("producers", "MMA issue", stores)])
 def test_warps_leave_as_a_whole(name, role):
     """Behind a wait that can run out, or the abort flag, all lanes of a warp go the same way: the collectives that follow
-    (__syncwarp, shuffles, tcgen05.ld) would wait without limit for a lane that has left."""
+    (__syncwarp, shuffles, tcgen05.ld) would wait without limit for a lane that has left.  And all of them have seen the phase:
+    one lane's wait and a shuffle order nothing for the others."""
     assert not _decided_by_lanes(_role(open(os.path.join(CSRC, name)).read(), role))
 
 
