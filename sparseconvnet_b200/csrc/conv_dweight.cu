@@ -227,16 +227,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
     bool bad = false, ok = true;
     int slot = 0, s_par = 0, n_g = 0, n_t = 0;  // of the slot: first G piece, tile
     for (;;) {
-      if (!mbar_wait(&C.s_full[slot], s_par) || *abort) {
-        ok = false;
-        break;
-      }
+      ok = mbar_wait_warp(&C.s_full[slot], s_par, abort);
+      if (!ok) break;
       const int job = C.job[slot];
       if (job == kEnd) break;
       const int *row = rows + slot * kRows;
       if (job == kTRows) {
         const int tb = n_t & 1;
-        ok = mbar_wait(&C.t_empty[tb], (unsigned)((n_t >> 1) + 1) & 1);
+        ok = mbar_wait_warp(&C.t_empty[tb], (unsigned)((n_t >> 1) + 1) & 1, abort);
         if (!ok) break;
         bad |= copy_rows<PT, S::T_PIECE>(t_dst + tb * S::T_BYTES, kAtom, row + warp * S::T_PIECE, t_src, t_bytes, (int)P.n_t, lane);
         cp_async_arrive(&C.t_full[tb]);
@@ -244,7 +242,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
       } else {
         const int q = (warp - n_g) & (kLoadWarps - 1);  // the piece of the job that is this warp's
         if (q < S::PIECES) {
-          ok = mbar_wait(&C.empty[warp / S::PIECES], (unsigned)((n_g + q) / S::STAGES + 1) & 1);
+          ok = mbar_wait_warp(&C.empty[warp / S::PIECES], (unsigned)((n_g + q) / S::STAGES + 1) & 1, abort);
           if (!ok) break;
           bad |= copy_rows<PG, S::G_PIECE>(g_dst, S::G_ATOM, row + q * S::G_PIECE, g_src, g_bytes, (int)P.n_g, lane);
           cp_async_arrive(&C.full[warp / S::PIECES]);

@@ -69,7 +69,8 @@ def _decided_by_lanes(text):
 
 
 @pytest.mark.parametrize("name,role", [(name, role) for name, stores in zip(TILE_KERNELS, ("epilogue", "drain"))
-                                       for role in ("producers", "MMA issue", stores)])
+                                       for role in ("producers", "MMA issue", stores)] +
+                         [("conv_dweight.cu", role) for role in ("rows", "MMA issue")])
 def test_warps_leave_as_a_whole(name, role):
     """Behind a wait that can run out, or the abort flag, all lanes of a warp go the same way: the collectives that follow
     (__syncwarp, shuffles, tcgen05.ld) would wait without limit for a lane that has left.  And all of them have seen the phase:
