@@ -36,8 +36,7 @@
 #include <atomic>
 #include <utility>
 
-#include "metadata.cuh"
-#include "tc_ptx.cuh"
+#include "conv_tile.cuh"
 
 namespace scn {
 
@@ -170,7 +169,7 @@ struct Ctl {
   unsigned long long full[2], empty[2], t_full[2], t_empty[2], s_full[kSlots], s_empty[kSlots], done;
   int job[kSlots];  // index of the offset in the group; kTRows; kEnd
   unsigned tmem, used;
-  int abort;
+  int abort, slots;  // slots: filled by the jobs
 };
 
 template <int PT, int PG>
@@ -316,15 +315,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
           ++it;
         }
       }
-      const int filled = n;
       if (ok) put(kEnd, nullptr);
-      if (!ok) {  // copies in flight must land before the CTA's shared memory goes away
-        *abort = 1;
-        for (int i = 0; i < kSlots; ++i) {
-          const int uses = (filled + kSlots - 1 - i) / kSlots;
-          if (uses > 0) mbar_wait(&C.s_full[i], (unsigned)((uses - 1) & 1));
-        }
-      }
+      C.slots = n;
+      if (!ok) *abort = 1;
     }
     __syncwarp();  // the other lanes must not go ahead: waiting for `done` they would hold up lane 0
   } else {
@@ -457,7 +450,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_dweight_tile(const __grid_const
   }
   tc_fence_before();
   __syncthreads();
-  if (*abort && tid == 0) atomicOr(P.flags, FLAG_TC_TIMEOUT);
+  if (*abort) {
+    if (tid == 0) atomicOr(P.flags, FLAG_TC_TIMEOUT);
+    land_slots(C.s_full, C.slots);
+  }
+  __syncwarp();
   if (warp == kMma) tmem_dealloc(tmem, 512);
 }
 

@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(SixWarps<NA>::THREADS, 1) k_conv_six(const __g
   __syncthreads();
   if (*abort) {
     if (tid == 0) atomicOr(P.flags, FLAG_TC_TIMEOUT);
-    land_copies<kSlots>(C, P.n_stages, kProdGroups);
+    land_copies(C, P.n_stages, kProdGroups);
   }
   __syncwarp();
   if (warp == kMma) tmem_dealloc(tmem, 512);

@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_tile(TileParams P) {
   __syncthreads();
   if (*abort) {
     if (tid == 0) atomicOr(P.flags, FLAG_TC_TIMEOUT);
-    land_copies<kSlots>(C, P.n_stages, kProdGroups);
+    land_copies(C, P.n_stages, kProdGroups);
   }
   __syncwarp();
   if (warp == kMma) tmem_dealloc(tmem, (unsigned)P.tmem_cols);

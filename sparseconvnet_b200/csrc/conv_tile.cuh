@@ -115,16 +115,18 @@ __host__ __device__ inline int last_slab(const int *slabs, int groups, int n_sta
 }
 
 // A CTA whose roles left early, whichever of them and on whichever way: its bulk copies must land before its shared memory goes
-// away.  All threads come here behind the block's last barrier, when nobody orders any more; one waits for each stage and each slot.
-template <int SLOTS, class Control>
+// away.  All threads come here behind the block's last barrier, when nobody orders any more; one waits for each slot and each stage.
+template <int SLOTS>
+__device__ __forceinline__ void land_slots(unsigned long long (&s_full)[SLOTS], int slots) {
+  const int si = threadIdx.x, uses = (slots + SLOTS - 1 - si) / SLOTS;
+  if (si < SLOTS && uses > 0) mbar_wait(&s_full[si], (unsigned)((uses - 1) & 1));
+}
+template <class Control>
 __device__ __forceinline__ void land_copies(Control &C, int n_stages, int groups) {
-  const int st = threadIdx.x, si = (int)threadIdx.x - 32;
-  if (st < n_stages) {
-    const int step = last_slab(C.ordered.slabs, groups, n_stages, st);
-    if (step >= 0) mbar_wait(&C.full[st], (unsigned)(step / n_stages & 1));
-  } else if (si >= 0 && si < SLOTS) {
-    const int uses = (C.ordered.slots + SLOTS - 1 - si) / SLOTS;
-    if (uses > 0) mbar_wait(&C.s_full[si], (unsigned)((uses - 1) & 1));
-  }
+  land_slots(C.s_full, C.ordered.slots);
+  const int st = (int)threadIdx.x - 32;
+  if (st < 0 || st >= n_stages) return;
+  const int step = last_slab(C.ordered.slabs, groups, n_stages, st);
+  if (step >= 0) mbar_wait(&C.full[st], (unsigned)(step / n_stages & 1));
 }
 }  // namespace scn

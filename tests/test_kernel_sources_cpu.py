@@ -46,16 +46,18 @@ def _source(name):
     return re.sub(r"//.*", "", open(os.path.join(CSRC, name)).read())
 
 
-@pytest.mark.parametrize("name", TILE_KERNELS)
-def test_bulk_copies_land_on_every_way_out(name):
+@pytest.mark.parametrize("name,wait,said", [
+    (name, r"land_copies\(C, P\.n_stages, kProdGroups\)", [r"\n    if \(brings_weights\) C\.ordered\.slabs\[group\] = filled;",
+                                                           r"\n      C\.ordered\.slots = slot;"]) for name in TILE_KERNELS] +
+    [("conv_dweight.cu", r"land_slots\(C\.s_full, C\.slots\)", [r"\n      C\.slots = n;"])])
+def test_bulk_copies_land_on_every_way_out(name, wait, said):
     """Whatever made a role leave, and when: behind the block's last barrier the abort flag alone decides whether the bulk copies are
-    waited for, and both roles that order them have said which, unconditionally."""
+    waited for, and every role that orders them has said which, unconditionally."""
     text = _source(name)
     end = text[text.rindex("__syncthreads();", 0, text.index("tmem_dealloc(tmem")):text.index("tmem_dealloc(tmem")]
-    assert re.search(r"if \(\*abort\) \{[^}]*land_copies<kSlots>\(C, P\.n_stages, kProdGroups\);\s*\}", end)
-    assert re.search(r"\n    if \(brings_weights\) C\.ordered\.slabs\[group\] = filled;", text)
-    assert re.search(r"\n      C\.ordered\.slots = slot;", text)
-    assert text.count("bulk_copy_g2s(") == 2
+    assert re.search(r"if \(\*abort\) \{[^}]*%s;\s*\}" % wait, end)
+    assert all(re.search(s, text) for s in said)
+    assert text.count("bulk_copy_g2s(") == len(said)
 
 
 def _role(text, name):
