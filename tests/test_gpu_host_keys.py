@@ -32,7 +32,7 @@ def test_host_coordinate_out_of_range(row, value):
         _locations(scn, 3, coords, 40, 3)
 
 
-# keys of 30 to 33 bits, 36 to 39, 42 to 45, and more than 48, which travel whole; one piece and more
+# keys of 30 to 33 bits, 36 to 39, 42 to 45, and more than 48 by the coordinates alone, which travel whole; one piece and more
 @pytest.mark.parametrize("size", [1000, 4096, 16000, 65000])
 @pytest.mark.parametrize("n,batch", [(1, 1), (1025, 8), (16383, 2), (33793, 5)])
 @pytest.mark.parametrize("mode", [0, 3])
@@ -43,4 +43,19 @@ def test_keys_by_their_bytes(n, batch, size, mode):
     coords[:, 3] = torch.randint(0, batch, (n,), generator=g)
     coords[n // 2:] = coords[:n - n // 2].clone()  # every site twice
     for a, b in zip(_locations(scn, 3, coords, size, mode), _locations(scn, 3, coords.cuda(), size, mode)):
+        assert torch.equal(a, b)
+
+
+# One point alone has bits of its key from 48 on, or 47 as the last one without: coordinates of 42 bits, the batch above them.  The
+# last point is one that is looked at before the keys are packed, the one before it is not.
+@pytest.mark.parametrize("batch", [63, 64, 1 << 14, (1 << 21) - 1])
+@pytest.mark.parametrize("row", [19998, 19999])
+@pytest.mark.parametrize("mode", [0, 3])
+def test_keys_wide_by_their_batch(row, batch, mode):
+    import sparseconvnet_b200 as scn
+    coords = torch.randint(0, 16000, (20000, 4), generator=torch.Generator().manual_seed(batch))
+    coords[:, 3] = torch.arange(20000) // 10000
+    coords[9000:10000] = coords[:1000].clone()
+    coords[row, 3] = batch
+    for a, b in zip(_locations(scn, 3, coords, 16000, mode), _locations(scn, 3, coords.cuda(), 16000, mode)):
         assert torch.equal(a, b)
