@@ -61,31 +61,39 @@ __global__ void k_output_features(const float *__restrict__ in, float *__restric
 // BatchNorm + leaky ReLU (CPU/BatchNormalization.cpp:12-62)
 // ------------------------------------------------------------------------------------------
 
-// per-plane sum and sum of squares; grid.x tiles planes by 32, grid.y splits the rows in chunks, whose sums are added in a
-// fixed order (bn_total)
+// per-plane sum and sum of squares; grid.x tiles planes by 32, the rows are split in chunks, block y takes chunk y (SEVERAL: and
+// y + grid.y, ...); the blocks' sums are added in a fixed order (bn_total)
+template <bool SEVERAL>
 __global__ void __launch_bounds__(256)
-k_bn_stats(const float *__restrict__ in, long long n_rows, int C, long long in_stride,
-           double *__restrict__ partial /* [2][C][chunks] */) {
+k_bn_stats(const float *__restrict__ in, long long n_rows, int C, long long in_stride, int chunks,
+           double *__restrict__ partial /* [2][C][gridDim.y] */) {
   SCN_GRID_WAIT();
   __shared__ float sh_s[8][33], sh_q[8][33];
   int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
   int c = blockIdx.x * 32 + lane;
-  float s = 0.f, q = 0.f;
-  if (c < C)
-    for (long long r = (long long)blockIdx.y * 8 + wy; r < n_rows; r += (long long)gridDim.y * 8) {
-      float v = in[r * in_stride + c];
-      s += v;
-      q += v * v;
-    }
-  sh_s[wy][lane] = s;
-  sh_q[wy][lane] = q;
-  __syncthreads();
+  double ds = 0, dq = 0;
+  int chunk = blockIdx.y;
+  do {
+    float s = 0.f, q = 0.f;
+    if (c < C)
+#pragma unroll 4
+      for (long long r = (long long)chunk * 8 + wy; r < n_rows; r += (long long)(SEVERAL ? chunks : gridDim.y) * 8) {
+        float v = in[r * in_stride + c];
+        s += v;
+        q += v * v;
+      }
+    if (SEVERAL) __syncthreads();
+    sh_s[wy][lane] = s;
+    sh_q[wy][lane] = q;
+    __syncthreads();
+    if (wy == 0 && c < C)
+      for (int j = 0; j < 8; ++j) {
+        ds += sh_s[j][lane];
+        dq += sh_q[j][lane];
+      }
+    chunk += gridDim.y;
+  } while (SEVERAL && chunk < chunks);
   if (wy == 0 && c < C) {
-    double ds = 0, dq = 0;
-    for (int j = 0; j < 8; ++j) {
-      ds += sh_s[j][lane];
-      dq += sh_q[j][lane];
-    }
     partial[(long long)c * gridDim.y + blockIdx.y] = ds;
     partial[(long long)(C + c) * gridDim.y + blockIdx.y] = dq;
   }
@@ -146,13 +154,16 @@ static int launch_bn_stats(const float *in, long long n_rows, int C, long long i
                            cudaStream_t stream) {
   const unsigned gx = (unsigned)ceil_div(C, 32);
   const bool pieces = C % 4 == 0 && in_stride % 4 == 0 && (uintptr_t)in % 16 == 0 && n_rows < (1 << 30) && in_stride < (1 << 20);
-  const unsigned gy = (unsigned)std::max<long long>(1, std::min<long long>(ceil_div(n_rows, 64), pieces ? 148 * 8 / gx : 1024));
+  const int split = (int)std::max<long long>(1, std::min<long long>(ceil_div(n_rows, 64), pieces ? 148 * 8 / gx : 1024));
+  // What the blocks leave takes 0.6 MB at most, without the pieces 8: with more than 512 planes a block takes several chunks there
+  // (4 095 planes on 65 k rows: 67 MB with a block for each, 288 us, 257 now).
+  const unsigned gy = (unsigned)(pieces ? split : std::min(split, (1 << 19) / C));
   SCN_TRY(tmp.get(partial, sizeof(double) * 2 * (size_t)C * gy));
   *chunks = (int)gy;
   if (pieces)
     SCN_LAUNCH(k_bn_stats4, dim3(gx, gy), 256, 0, stream, in, (int)n_rows, C, (int)in_stride, *partial);
   else
-    SCN_LAUNCH(k_bn_stats, dim3(gx, gy), 256, 0, stream, in, n_rows, C, in_stride, *partial);
+    SCN_LAUNCH(((int)gy < split ? k_bn_stats<true> : k_bn_stats<false>), dim3(gx, gy), 256, 0, stream, in, n_rows, C, in_stride, split, *partial);
   return SCN_OK;
 }
 

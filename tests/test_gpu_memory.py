@@ -212,3 +212,24 @@ def test_weight_gradient_scratch_is_bounded(cuda):
         want = f[r[:, 0]].double().t() @ g[r[:, 1]].double()
         assert float((dw[k, 0] - want).norm() / want.norm()) <= 1e-5
     x.metadata.poll_errors()
+
+
+def test_batchnorm_scratch_is_bounded(cuda):
+    """Statistics of 4 095 planes on 65 k rows, 1 024 chunks: what a chunk leaves is 16 bytes a plane, 67 MB if each left its own.
+    A chunk's fp32 sums are of eight rows at most (eight roundings, and one of a square), and added in double."""
+    from sparseconvnet_b200._lib import check, lib
+    for n, planes in ((65536, 4095), (65535, 515), (700, 4095), (1, 2049)):
+        torch.manual_seed(planes)
+        x, sums = torch.randn(n, planes, device=cuda), torch.empty(2 * planes + 1, dtype=torch.float64, device=cuda)
+        torch.cuda.synchronize()
+        check(lib.scn_trim_memory(0))
+        before = _used()[0]
+        check(lib.scn_batchnorm_moments(x.data_ptr(), n, planes, planes, sums.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        assert _used()[0] - before <= 40 << 20
+        for got, power in ((sums[:planes], 1), (sums[planes:2 * planes], 2)):
+            want, scale = (torch.zeros(planes, dtype=torch.float64, device=cuda) for _ in range(2))
+            for part in x.split(8192):
+                want += (part.double() ** power).sum(0)
+                scale += (part.double() ** power).abs().sum(0)
+            assert bool(((got - want).abs() <= 9 * 2.0 ** -24 * scale).all())
