@@ -99,9 +99,10 @@ k_bn_stats(const float *__restrict__ in, long long n_rows, int C, long long in_s
   }
 }
 
-// The same for rows of whole 16-byte pieces: eight lanes per row and 32 planes, 32 rows per pass of the block, four passes
-// in flight.  Bound by HBM.  (With the blocks' sums added by atomics, up to 1 184 of them to the same 64 doubles, and two passes
-// in flight, 400 k rows of 32 planes took 16.5 us, 12.6 now, and the 14 layers of a U-Net training step 162 us with their memsets, 120.)
+// The same for rows of whole 16-byte pieces: eight lanes per row and 32 planes, 32 rows per pass of the block, two passes
+// in flight.  Bound by HBM.  The 14 layers of a U-Net training step on 400 k points: 111 us; 144 and 18 of memsets with the blocks' sums
+// added by atomics, up to 1 184 of them to the same 64 doubles; 121 with four passes in flight, whose last rows go one at a time (the
+// call on 100 k rows of 96 planes 32 -> 26 us, on 1.6 M of 64 219 -> 211).
 __global__ void __launch_bounds__(256)
 k_bn_stats4(const float *__restrict__ in, int n_rows, int C, int in_stride, double *__restrict__ partial /* [2][C][chunks] */) {
   SCN_GRID_WAIT();
@@ -119,14 +120,12 @@ k_bn_stats4(const float *__restrict__ in, int n_rows, int C, int in_stride, doub
       z[0] += v.x * v.x, z[1] += v.y * v.y, z[2] += v.z * v.z, z[3] += v.w * v.w;
     };
     auto ld = [](const float *q) { return __ldg(reinterpret_cast<const float4 *>(q)); };
-    for (; r < n_rows - 3ll * step; r += 4 * step, p += 4 * hop) {
-      const float4 a = ld(p), b = ld(p + hop), d = ld(p + 2 * hop), e = ld(p + 3 * hop);
+    for (; r < n_rows - step; r += 2 * step, p += 2 * hop) {
+      const float4 a = ld(p), b = ld(p + hop);
       add(a);
       add(b);
-      add(d);
-      add(e);
     }
-    for (; r < n_rows; r += step, p += hop) add(ld(p));
+    if (r < n_rows) add(ld(p));
   }
 #pragma unroll
   for (int e = 0; e < 4; ++e) {  // the four rows of a warp
@@ -194,7 +193,8 @@ __device__ __forceinline__ void bn_total(const double *__restrict__ partial /* [
 
 // Turns either running statistics (eval) or batch sums (train) into saveMean / saveInvStd and
 // updates the running statistics in training mode: momentum weighs the OLD value, the
-// normalising variance is biased, the running variance unbiased (CPU/BatchNormalization.cpp:32-46).  One warp per plane.
+// normalising variance is biased, the running variance unbiased (CPU/BatchNormalization.cpp:32-46).  One warp per plane: 53 us for the
+// 14 layers (40 when atomics had added the sums; a block per plane, all chunks at once, made no call shorter).
 __global__ void __launch_bounds__(256)
 k_bn_finalize(int C, long long n_rows, const double *__restrict__ partial /* [2][C][chunks] */, int chunks,
               float *save_mean, float *save_invstd, float *running_mean,
@@ -338,7 +338,7 @@ k_bn_back_sums(const float *__restrict__ in, const float *__restrict__ out, cons
 }
 
 // The same for rows of whole 16-byte pieces: eight lanes per row and 32 planes, two rows of a lane in flight.  Bound by HBM
-// (sums in fp32 would save 3 %): the 14 layers of a U-Net training step on 400 k points 293 us (469 with one value per load).
+// (sums in fp32 would save 3 %): the 14 layers of a U-Net training step on 400 k points 296 us (469 with one value per load).
 __global__ void __launch_bounds__(256)
 k_bn_back_sums4(const float *__restrict__ in, const float *__restrict__ out, const float *__restrict__ d_out, int n_rows, int C,
                 int in_stride, int out_stride, const float *__restrict__ mean, float leak, int chunk_rows,
@@ -396,9 +396,9 @@ k_bn_back_sums4(const float *__restrict__ in, const float *__restrict__ out, con
   }
 }
 
-// Chunks of at least 64 rows, at most as many blocks as are on the SMs at once (four each: 59 and 64 registers a thread).  With up
+// Chunks of 33 rows or more, at most as many blocks as are on the SMs at once (four each: 59 and 64 registers a thread).  With up
 // to 1 024 chunks of at least 256 rows a layer's blocks took one and a half waves to two, and levels of 10 k rows had too
-// few: the 14 layers of a U-Net training step on 400 k points 329 -> 293 us, their k_bn_back_finalize 43 -> 38, the seven on
+// few: the 14 layers of a U-Net training step on 400 k points 331 -> 296 us, their k_bn_back_finalize 43 -> 38, the seven on
 // 93 k and fewer pixels 44 -> 28 (k_bn_back_finalize there 15 -> 18).
 static int bn_back_chunks(long long n_rows, int C) {
   return (int)std::max<long long>(1, std::min<long long>(ceil_div(n_rows, 64), 148 * 4 / ceil_div(C, 32)));
