@@ -27,11 +27,11 @@
 //               traffic, 1 100 cycles per step of 96 planes with two ranges, more than the step's 700 of instructions
 //   drain       8 warps, a row and half of the planes per lane: TMEM -> registers after every step, and after the tile's
 //               last one through shared memory -> bias -> optional BatchNorm -> 16-byte stores, four lanes per row
-// Tensor pipe active 73 % for 128 output planes, 54 for 96 (200 k rows, 1 050 and 1 070 cycles per step); below that no unit is near
-// its peak: 64 planes 38 % beside 64 % of the issue slots and 1 030 cycles per step, 32 planes 21 and 59 %, 880 cycles.  As multiply-adds
+// Tensor pipe active 74 % for 128 output planes, 54 for 96 (200 k rows, 1 050 and 1 070 cycles per step); below that no unit is near
+// its peak: 64 planes 38 % beside 64 % of the issue slots and 1 030 cycles per step, 32 planes 22 and 60 %, 880 cycles.  As multiply-adds
 // the same step is 1 024 to 4 096 cycles of the whole FMA pipe.  The barriers of the next step are looked at while this one is
 // under way and the loads of a row's stores come before its branches: with a wait, a look at the abort flag and a role for the
-// weights in every step, 200 k rows: 32 -> 32 planes 103 us, 92 now; 64 -> 64 229, 207; 96 -> 96 373, 325; 128 -> 128 527, 455; a
+// weights in every step, 200 k rows: 32 -> 32 planes 102 us, 89 now; 64 -> 64 229, 205; 96 -> 96 372, 318; 128 -> 128 525, 445; a
 // Deconvolution 128 -> 96 to 43 k rows 28, 17.  (64 planes: three loads of 16 columns under one wait do not fit the registers, 216;
 // two column ranges and with them four accumulators 204; sixteen drain warps 207.)  Rows split once per call, not once per gather:
 // with fp32 rows (16 KB per step) split by the producers on their way through registers a step took twice as long.
@@ -844,7 +844,9 @@ int launch_six(SixParams &P, int n_sm, int dev, cudaStream_t stream) {
 }
 
 // Into how many parts a tile's offsets are divided: as in conv_tile.cu, the smallest estimate of (waves of items) x (steps of
-// an item) in SM cycles, plus, with more than one part, the partial sums' traffic and the second launch.
+// an item) in SM cycles, plus, with more than one part, the partial sums' traffic and the second launch.  The constants are empirical
+// here too: against 1 to 16 parts on 36 layers of U-Nets within 5 % of the best on 32; 256 -> 128 planes on 57 k rows 266 us (one part:
+// 234), 192 -> 96 on 18.6 k 103 (four: 94), 64 -> 32 on 40 k 41.5 (three: 38.8), 192 -> 224 strided 18.5 (four: 17.5).
 int split_parts(long long n_tiles, int n_cb, int K, int n_slices, double step_cycles, int cout, int n_sm) {
   const double offsets = n_tiles >= 2 * n_sm ? 0.5 * K : 0.75 * K;
   double best = 0;
@@ -873,30 +875,31 @@ extern thread_local int g_drop_arrival;  // test hook (conv_tc.cu)
 //   9 000         16.3/14.9  17.4/18.7  18.4/23.4  29.1/60.6  41.5/127   92.0/327       1.0e-7 / 3.5e-7
 //   30 000        20.3/32.3  21.4/42.5  26.4/59.5  53.6/141   81.8/317   222/859        1.1e-7 / 5.3e-7
 //   200 000       72/97      78/135     102/200    231/603    359/1 549  1 005/4 178    1.2e-7 / 5.4e-7
-// Other filters (measured when this kernel took 10 to 18 % longer up to 64 planes):
-//   3-D shapes, 99 000 rows, 27 offsets: 8->16 45/42, 16->16 45/51, 32->16 57/67, 16->32 45/63
-//   2-D strokes, 91 000 rows, 9 offsets: 16->16 28/21, 32->16 33/27, 16->32 28/26, 24->32 34/31, 32->32 34/37
-//   2-D, 25 offsets, 31 500 rows: 16->32 26/37, 32->32 29/51, 64->64 56/129; 4-D, 81 offsets, 60 000 rows: 32->32 76/221
-//   3 / 2, 27 offsets, 26 700 rows: 16->32 22/30, 32->32 27/40, 64->64 52/99, 128->128 115/361
+// Other filters:
+//   3-D shapes, 99 000 rows, 27 offsets: 8->16 37/42, 16->16 37/51, 32->16 46/69, 16->32 40/64
+//   2-D strokes, 92 000 rows, 9 offsets: 16->16 21/20, 32->16 25/27, 16->32 23/26, 24->32 27/32, 32->32 27/38
+//   2-D, 25 offsets, 32 000 rows: 16->32 24/40, 32->32 30/57, 64->64 61/143; 4-D, 81 offsets, 60 000 rows: 32->32 72/226
+//   3 / 2, 27 offsets, 48 000 rows: 16->32 27/42, 32->32 35/58, 64->64 69/152, 128->128 143/536
 // Windows side by side (filter = stride), where a fine row has one rule (2 / 2; fine rows; a Convolution's coarse rows):
 //   Deconvolution 32->16     32->32     48->32     64->32     64->48     96->48     64->64     96->96     128->128
-//   4 000 rows                                                                      10.6/10.4  11.3/9.8   12.5/15.1
-//   15 000                                                                          11.0/11.0  12.0/14.7  13.7/21.3
-//   25 000        10.5/5.2   10.8/7.4   11.9/8.9   11.8/9.7   12.8/13.3  14.6/17.1  13.7/13.5
-//   100 000       15.9/10.4  16.8/16.3  20.0/19.5  20.3/22.0  23.4/31.4  27.6/42.3  25.0/31.6
-//   200 000       22.2/15.7  23.4/24.6  28.8/30.2  30.7/34.3  36.2/55.3  44.7/73.6  39.1/56.0
-//   400 000                             52/58      55/67                            71/113     97/242     134/341
-//   1 600 000     119/116    141/189    175/220    193/244    230/410    299/535    243/412
+//   4 000 rows                                                                      10.4/10.3  11.2/10.0  12.4/15.1
+//   15 000                                                                          10.9/11.1  12.0/14.9  13.9/21.5
+//   25 000        10.2/5.2   10.4/7.5   11.7/8.9   11.8/9.7   12.6/13.3  14.5/17.1  13.6/13.4
+//   100 000       15.9/10.9  16.8/16.6  20.2/19.9  21.4/22.1  24.5/31.5  29.1/42.1  26.8/31.9
+//   200 000       22.5/15.8  23.6/24.8  29.1/30.2  31.3/34.2  36.0/55.1  44.1/73.4  39.6/56.6
+//   400 000                             53/59      56/69                            72/113     100/242    142/340
+//   1 600 000     118/118    142/191    175/222    193/246    230/413    296/536    240/414
 //   error         0.5/1.0e-7 0.5/1.0e-7 0.5/1.3e-7 0.5/1.4e-7 0.5/1.4e-7 0.6/1.8e-7 0.5/1.4e-7
 //   Convolution   32->48     32->64     64->64     96->64     64->96     96->96     128->128
-//   1 500 rows    12.4/9.9              14.8/11.8  16.1/14.6  15.1/13.1  17.1/16.3  17.7/22.0
-//   4 000         12.7/18.2             16.2/19.2  18.4/31.8  17.1/21.8  19.7/30.1  23.4/47.3
-//   16 000        16.5/23.2             22.3/31.7  28.1/43.7  23.8/46.5  30.2/62.9  38.4/90.3
-//   54 000        25.5/38.1  28.1/39.8  50.3/61.3
-//   118 000       49/54                 87/95      124/132    91/159     129/224    177/321
-//   463 000       165/191    173/192    307/321
-// (The lines for windows side by side were drawn when this kernel took 10 to 40 % longer on them: every one of them that comes
-// here gains, and Deconvolutions of 70 M multiply-adds, or Convolutions to 64 planes on more rows, would.)
+//   1 100 rows    12.2/9.6              14.5/9.4   15.8/14.4  15.4/10.9  16.9/14.8  17.1/20.0
+//   5 400         12.7/18.3             16.6/23.0  19.3/31.9  17.5/24.7  20.9/33.0  25.6/66.2
+//   21 000        16.8/23.1             22.3/30.6  28.5/40.0  24.3/48.2  31.0/68.6  38.7/92.7
+//   55 000        26.6/38.7  28.7/40.3  50.7/63.7
+//   109 000       48/53                 84/97      119/134    87/158     123/224    166/311
+//   463 000       166/192    176/192    308/321
+// (The lines are from a form of this kernel that took 10 to 40 % longer.  What comes here gains; some of what stays away would gain too:
+// 8 -> 16 planes on 99 000 rows of shapes 11 %, 24 -> 32 with 9 offsets 17 %, Deconvolutions to 48 planes and more up to 45 %,
+// Convolutions to 64 planes on more than 90 000 rows 4 to 13 %.)
 // Its error is the smaller one, or the same, for every shape and table that comes here, 8 to 256 planes, products of mixed
 // and of one sign, rows behind a ReLU (16->32 on 9 000 rows of one sign, where k_conv_fma's sums are in parts: 6.5e-8 and
 // 6.1e-8, so not here).

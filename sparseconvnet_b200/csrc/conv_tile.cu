@@ -19,13 +19,13 @@
 //     sign 6.9e-6 -> 3.7e-6; smaller for every shape of 80 to 128 planes.)
 //   * A step's work is small beside the barriers around it, so what bounds it is the longest chain of any one role: 224 to 384 cycles
 //     of tensor instructions, 336 (32 -> 32 planes: 20 KB written, 22 read) to 576 (128 -> 128) cycles of shared memory at 128
-//     bytes; L2 gives 75 bytes per cycle and SM to 16-byte cp.async gathers of rows that lie in it, a step takes 37 to 56.  Every
+//     bytes; L2 gives 75 bytes per cycle and SM to 16-byte cp.async gathers of rows that lie in it, a step takes 39 to 58.  Every
 //     wait, load and store of shared memory stands 100 to 200 cycles behind the copies.  With a thread of its own for the
 //     weights (two waits, a load, an arrival and the copy per step: 1 050 cycles) and instructions issued inside a branch of
 //     one lane (descriptors moved into uniform registers one by one: 135 cycles per four instructions, 38 with a predicate) the
-//     same tiles took, 8 rooms: 32 -> 32 planes 253 us, now 207; 64 -> 64 145, 134; 96 -> 96 98, 88; 128 -> 128 83, 69;
-//     224 -> 224 on 1.4 k rows 22.6, 18.2; 4-D 64 -> 64 bf16 778, 676.  Now, 200 k rows: tensor pipe active 20, 41, 54, 72 % for 32,
-//     64, 96, 128 planes, shared memory banks 22 + 17 to 33 + 24 % (read + written), issue slots 57, 56, 42, 40 %.
+//     same tiles took, 8 rooms: 32 -> 32 planes 252 us, now 198; 64 -> 64 144, 128; 96 -> 96 98, 84; 128 -> 128 82, 66;
+//     224 -> 224 on 1.4 k rows 22.6, 17.6; 4-D 64 -> 64 bf16 774, 643.  Now, 200 k rows: tensor pipe active 22, 44, 57, 76 % for 32,
+//     64, 96, 128 planes, shared memory banks 23 + 17 to 34 + 25 % (read + written), issue slots 55, 52, 40, 39 %.
 //
 // Roles (14 warps, one or two CTAs per SM, persistent).  A step is one filter offset of one tile and SP input planes; the
 // steps of a CTA are numbered through all its tiles and step n uses stage n % n_stages of one ring.
@@ -649,8 +649,11 @@ bool conv_tile_supported(const float *in, const float *in_b, int planes_a, const
 }
 
 // Into how many parts a tile's offsets are divided: the smallest estimate of (waves of items) x (steps of an item),
-// plus, with more than one part, the partial sums' traffic and the second launch.  In SM cycles; a step is bound by its
-// 16 KB of gathered rows at 32 bytes per cycle or by its weight slab, an item also costs the fill and drain of the rings.
+// plus, with more than one part, the partial sums' traffic and the second launch.  In SM cycles: a step counts as its bytes (rows and
+// weights) at 32 per cycle, an item's fill and drain as 2 500, for one CTA per SM.  The constants are empirical and older than the
+// kernel's present form, whose steps take 39 to 58 bytes per cycle.  What they choose, measured against 1 to 16 parts on 48 layers of
+// U-Nets, 40 to 57 k rows, 32 to 448 planes: within 5 % of the best on 42; 64 -> 64 planes on 10.7 k rows 20.8 us (three parts: 16.1);
+// 160 -> 160 and 320 -> 160 on 22 k 61 and 107 (57 and 101); three strided layers 11 to 13 (one microsecond less).
 static int split_parts(long long n_tiles, int K, int n_slices, double step_cycles, int cout, int n_sm) {
   const double offsets = n_tiles >= 2 * n_sm ? 0.5 * K : 0.75 * K;  // sorted tiles of a large level meet fewer
   double best = 0;
