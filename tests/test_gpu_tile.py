@@ -280,3 +280,33 @@ def test_rows_in_their_own_order(n, dim, filter_size, cuda):
             assert float((y.double() - want).norm() / want.norm()) <= 2.0 ** -16
     finally:
         scn.set_precision("fp32")
+
+
+# one slice and several, one accumulator range and three, one and two CTAs per SM, offsets divided and not, few stages and many
+@pytest.mark.parametrize("precision,cin,cout,n", [
+    ("tf32x3", 32, 32, 20000), ("tf32x3", 224, 224, 700), ("bf16", 64, 64, 9000), ("fp32", 16, 32, 20000), ("fp32", 64, 64, 9000),
+    ("fp32", 160, 160, 3000)])
+def test_giving_up_in_every_form(precision, cin, cout, n, cuda):
+    """One barrier arrival left out in k_conv_tile's or k_conv_six's first CTA, at a step from which all its roles run dry: the kernel
+    ends by itself, the host learns of it, and nothing of it is left for the next call."""
+    import sparseconvnet_b200 as scn
+    from sparseconvnet_b200._lib import ScnError, lib
+    coords = _points(n, 3, 200, n)
+    layer = scn.SubmanifoldConvolution(3, cin, cout, 3, True).to(cuda)
+    try:
+        scn.set_precision(precision)
+        with torch.no_grad():
+            x = scn.InputLayer(3, 200, mode=3)([torch.from_numpy(coords), torch.randn(len(coords), cin, device=cuda)])
+            good = layer(x).features
+            assert lib.scn_last_conv_kernel() == (8 if precision == "fp32" else 6)
+            x.metadata.poll_errors()
+            assert lib.scn_test_drop_barrier_arrival() == 0
+            layer(x)
+            torch.cuda.synchronize()
+            with pytest.raises(ScnError, match="bounded wait"):
+                x.metadata.poll_errors()
+            for _ in range(3):
+                assert torch.equal(layer(x).features, good)
+            x.metadata.poll_errors()
+    finally:
+        scn.set_precision("fp32")
